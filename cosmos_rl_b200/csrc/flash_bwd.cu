@@ -1,23 +1,31 @@
 // Varlen causal flash-attention backward on tcgen05 / TMEM / TMA (head_dim 128, GQA, packed sequences).
 //
-// One CTA owns one (sequence, 128-key block, kv head): K and V tiles stay in shared memory, dK and dV accumulate
-// in TMEM over every query head of the GQA group and every 64-query block that can see the key block, and are
-// written once as bf16 (no atomics, no per-head partial sums). Per (query head, 64-query block) iteration i:
-//     S^T  = K Q^T                 M=keys(128) N=queries(64) K=d     TMEM S[i&1]   (64 columns)
-//     dP^T = V dO^T                M=keys      N=queries     K=d     TMEM dP[i&1]  (64 columns)
-//     P^T  = exp2(S^T c - lse),  dS^T = P^T o (dP^T - delta) * scale   8 softmax warps, thread = key row x 32 queries;
-//                                                                      both written to smem as bf16 [keys x queries]
-//     dV  += P^T dO                M=keys N=d K=queries(64)          dO tile re-read as MN-major B
-//     dK  += dS^T Q                M=keys N=d K=queries              Q  tile re-read as MN-major B
-//     dQ^T = K^T dS^T              M=d N=queries K=keys              K tile as MN-major A, dS^T smem as MN-major B;
-//                                                                    written over dP[i&1], which is dead by then
-// Q/dO tiles and the S/dP accumulators are double-buffered: the TMA loads and the first two MMAs of iteration i+1
-// run while the softmax warps work on iteration i, and the dQ^T drain of iteration i-1 (coalesced fp32 atomics:
-// a warp adds 32 consecutive head-dim elements of one query) runs while the tensor core does the three MMAs of
-// iteration i. A tile loaded by TMA as rows of 128 bytes (SW128) serves both as a K-major operand (rows = M/N) and
-// as an MN-major operand (rows = contraction), so nothing is transposed or loaded twice.
-// delta = rowsum(O o dO) comes from a small pre-pass. All waits are bounded; a failed wait never leaves a loop that
-// contains a named barrier early.
+// Two kernels, each owning its outputs, so nothing is accumulated through memory (no fp32 dQ buffer, no atomics, the
+// same bits on every run):
+//
+//   dQ     one CTA = (sequence, 128-query block, query head); loops over the 128-key blocks it can see
+//          S  = Q K^T          M=queries N=keys K=d        TMEM S[j&1]
+//          dP = dO V^T         M=queries N=keys K=d        TMEM dP
+//          dS = exp2(S c - lse) o (dP - delta)             softmax warps, bf16 into the columns of dP
+//          dQ += dS K          M=queries N=d K=keys        A = dS out of TMEM, B = the K tile read MN-major
+//          delta = rowsum(O o dO) of its rows is formed first and left in memory for the second kernel.
+//   dK, dV one CTA = (sequence, 128-key block, kv head); loops over the query heads of its GQA group and the
+//          128-query blocks that can see the key block
+//          S^T  = K Q^T        M=keys N=queries K=d        TMEM S
+//          dP^T = V dO^T       M=keys N=queries K=d        TMEM dP
+//          P^T, dS^T           softmax warps, bf16 into the columns of S and dP
+//          dV += P^T dO        M=keys N=d K=queries        A out of TMEM, B = the dO tile read MN-major
+//          dK += dS^T Q        M=keys N=d K=queries        A out of TMEM, B = the Q tile read MN-major
+//
+// S and dP are formed twice (7 products of 128 x 128 x 128 per tile pair instead of 5). That is the cheaper side: a
+// product of two shared-memory operands reads 64 KB for 512 tensor-core cycles, which is all the 128 B per cycle that
+// shared memory gives, and in the one-kernel form the transposed dS and the fp32 dQ tile go through shared memory and
+// L2 as well. With P and dS taken from TMEM the five products per tile of the two accumulations need 32 KB each.
+// The tensor core runs the products in the order in which the one issuing thread gives them; a product that
+// overwrites the columns of an operand of the product before it (S over P, dP over dS) relies on that order.
+// Timing: profiles/flash_attention_B16_L4096.md.
+// Roles of both: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 softmax (two per TMEM lane quadrant, 64 columns
+// each). All waits are bounded; on a timeout a status code is recorded and the CTA leaves with its TMEM freed.
 // Replaces flash_attn's varlen backward (cosmos_rl/policy/kernel/modeling_utils.py:65-173).
 #include "sm100.cuh"
 #include "gemm_core.cuh"
@@ -25,91 +33,156 @@
 
 namespace b200 {
 
-constexpr int FB_BK = 128;                           // keys per CTA
-constexpr int FB_BQ = 64;                            // queries per iteration
+constexpr int FB_B = 128;                            // queries / keys per block
 constexpr int FB_D = 128;
-constexpr int FB_KV_TILE = FB_BK * FB_D * 2;         // 32 KiB
-constexpr int FB_Q_TILE = FB_BQ * FB_D * 2;          // 16 KiB
-constexpr int FB_P_TILE = FB_BK * FB_BQ * 2;         // 16 KiB
-constexpr int FB_SMEM = 2 * FB_KV_TILE + 4 * FB_Q_TILE + 2 * FB_P_TILE + 1024 /*lse, delta x2*/ + 256 + 1024;
-constexpr int FB_THREADS = 320;                      // TMA warp, MMA warp, 8 softmax warps (two per TMEM lane quadrant)
+constexpr int FB_TILE = FB_B * FB_D * 2;             // 32 KiB, two boxes of 128 rows x 64 elements
+constexpr int FB_STATS = 2 * 2 * FB_B * 4;           // dK/dV kernel: lse and delta of two query blocks
+constexpr int FB_SMEM = 6 * FB_TILE + FB_STATS + 256 + 1024;
+constexpr int FB_THREADS = 320;                      // TMA warp, MMA warp, 8 softmax warps
 constexpr float FB_LOG2E = 1.4426950408889634f;
 
 struct FbParams {
   const int* cu_q;
   const int* cu_k;
-  const float* lse;      // [hq, Tq]
-  const float* delta;    // [hq, Tq]
-  float* dq_accum;       // [Tq, hq, d] fp32, zero-initialised
-  __nv_bfloat16* dk;     // [Tk, hkv, d]
+  const float* lse;            // [hq, Tq]
+  float* delta;                // [hq, Tq]; written by the dQ kernel, read by the dK/dV kernel
+  const __nv_bfloat16* out;    // [Tq, hq, d] of the forward pass
+  const __nv_bfloat16* dout;
+  __nv_bfloat16* dq;           // [Tq, hq, d]
+  __nv_bfloat16* dk;           // [Tk, hkv, d]
   __nv_bfloat16* dv;
-  long long lddk, lddv;  // token strides (elements)
-  int hq, hkv, Tq, causal;
+  long long ldo, lddo, lddq, lddk, lddv;  // token strides (elements)
+  int B, hq, hkv, Tq, causal;
   float scale, scale_log2;
   uint32_t* status;
 };
 
-__device__ __forceinline__ float fb_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
+// Whole-warp bounded wait; on a timeout records `code`, raises the CTA's abort flag and returns false in every lane.
+__device__ __forceinline__ bool fb_wait(uint64_t* bar, uint32_t parity, uint32_t code, uint32_t* status,
+                                        volatile uint32_t* abort_flag) {
+  const bool ok = mbar_wait(bar, parity);
+  if (!ok) {
+    atomicCAS(status, ST_OK, code);
+    *abort_flag = 1;
+  }
+  return __all_sync(0xffffffffu, ok);
 }
 
-#define FB_FAIL(code)                         \
-  {                                           \
+// The same for the single thread of the producer / issuer roles.
+#define FB_WAIT1(bar, parity, code)           \
+  if (!mbar_wait(bar, parity)) {              \
     atomicCAS(p.status, ST_OK, code);         \
     *abort_flag = 1;                          \
     break;                                    \
   }
 
+__device__ __forceinline__ void fb_load_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
+  tma_load_2d(dst, tm, bar, col, row);
+  tma_load_2d(dst + FB_TILE / 2, tm, bar, col + 64, row);
+}
+
+// D[128, 128] = A[128, 128] * B[128, 128]^T of two K-major shared-memory tiles
+__device__ __forceinline__ void fb_mma_ss(uint32_t tmem_d, uint32_t a, uint32_t b) {
+  constexpr uint32_t idesc = umma_idesc_bf16_f32(128, 128);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t off = (k >> 2) * (FB_TILE / 2) + (k & 3) * 32;
+    umma_bf16_ss(tmem_d, umma_desc_kmajor_sw128(a + off), umma_desc_kmajor_sw128(b + off), idesc, k > 0 ? 1u : 0u);
+  }
+}
+
+// D[128, 128] += A[128, 128] * B[128, 128] with A in TMEM (contraction elements 0..63 in columns [0, 32), 64..127 in
+// columns [64, 96)) and B a shared-memory tile whose rows are the contraction index
+__device__ __forceinline__ void fb_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, bool first) {
+  constexpr uint32_t idesc = umma_idesc_bf16_f32(128, 128) | (1u << 16);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    umma_bf16_ts(tmem_d, tmem_a + (k >> 2) * 64 + (k & 3) * 8, umma_desc_mnmajor_sw128(b + k * 2048, FB_TILE / 2), idesc,
+                 (first && k == 0) ? 0u : 1u);
+}
+
+// 64 fp32 columns of this thread's accumulator row, times `mul`, as bf16 to global memory
+__device__ __forceinline__ void fb_store_row(uint32_t taddr, bool zero, float mul, __nv_bfloat16* dst, bool live) {
+#pragma unroll 1
+  for (int c = 0; c < 64; c += 32) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(taddr + c, r);
+    tmem_ld_wait();
+    if (live) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          o[j] = zero ? 0u : pack_bf16x2(__uint_as_float(r[8 * g + 2 * j]) * mul, __uint_as_float(r[8 * g + 2 * j + 1]) * mul);
+        *reinterpret_cast<uint4*>(dst + c + 8 * g) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// dQ (and delta)
+// ---------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(FB_THREADS, 1)
-flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, FbParams p) {
-  const int b = blockIdx.z, hk = blockIdx.y, kb = blockIdx.x;
+flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, FbParams p) {
+  const int heads = p.hq * p.B, nblk = gridDim.x / heads;
+  const int hb = blockIdx.x % heads, h = hb % p.hq, b = hb / p.hq;
+  const int qb = nblk - 1 - blockIdx.x / heads;        // under the causal mask late query blocks see most keys: first
   const int q_beg = p.cu_q[b], len_q = p.cu_q[b + 1] - q_beg;
   const int k_beg = p.cu_k[b], len_k = p.cu_k[b + 1] - k_beg;
-  const int kv0 = kb * FB_BK;
-  if (kv0 >= len_k) return;
+  const int q0 = qb * FB_B;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (qb == 0) {
+    // tokens outside every sequence have no gradient
+    const int head = b == 0 ? q_beg : 0, tail = b == p.B - 1 ? p.cu_q[p.B] : p.Tq;
+    for (int t = warp; t < head; t += FB_THREADS / 32)
+      *reinterpret_cast<uint2*>(p.dq + (long long)t * p.lddq + h * FB_D + lane * 4) = make_uint2(0u, 0u);
+    for (int t = tail + warp; t < p.Tq; t += FB_THREADS / 32)
+      *reinterpret_cast<uint2*>(p.dq + (long long)t * p.lddq + h * FB_D + lane * 4) = make_uint2(0u, 0u);
+  }
+  if (q0 >= len_q) return;
   const int shift = len_k - len_q;
-  const int G = p.hq / p.hkv;
-  const int nqb = (len_q + FB_BQ - 1) / FB_BQ;
-  int qb_first = 0;
-  if (p.causal && kv0 - shift > 0) qb_first = (kv0 - shift) / FB_BQ;
-  const int per_head = nqb > qb_first ? nqb - qb_first : 0;
-  const int n_iter = per_head * G;
+  int kv_end = p.causal ? min(len_k, q0 + FB_B + shift) : len_k;
+  if (kv_end < 0) kv_end = 0;
+  const int n = (kv_end + FB_B - 1) / FB_B;
+  const int hk = h / (p.hq / p.hkv);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* k_sh = smem;
-  uint8_t* v_sh = smem + FB_KV_TILE;
-  uint8_t* q_sh = smem + 2 * FB_KV_TILE;                    // [2]
-  uint8_t* do_sh = q_sh + 2 * FB_Q_TILE;                    // [2]
-  uint8_t* pt_sh = do_sh + 2 * FB_Q_TILE;
-  uint8_t* ds_sh = pt_sh + FB_P_TILE;
-  float* lse_sh = reinterpret_cast<float*>(ds_sh + FB_P_TILE);   // [2][64] lse * log2(e)
-  float* dlt_sh = lse_sh + 2 * FB_BQ;                             // [2][64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(lse_sh) + 1024);
-  uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;     // [2]
-  uint64_t* qdo_empty = bars + 3;    // [2]
-  uint64_t* sdp_ready = bars + 5;    // [2]
-  uint64_t* pds_ready = bars + 7;
-  uint64_t* mma3_done = bars + 8;
-  uint64_t* dq_drained = bars + 9;   // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint8_t* q_sh = smem;
+  uint8_t* do_sh = smem + FB_TILE;
+  uint8_t* k_sh = smem + 2 * FB_TILE;                  // [2]
+  uint8_t* v_sh = smem + 4 * FB_TILE;                  // [2]
+  float* delta_sh = reinterpret_cast<float*>(smem + 6 * FB_TILE);   // [128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * FB_TILE + FB_STATS);
+  uint64_t* q_full = bars;
+  uint64_t* do_full = bars + 1;
+  uint64_t* k_full = bars + 2;     // [2]
+  uint64_t* v_full = bars + 4;     // [2]
+  uint64_t* k_empty = bars + 6;    // [2]
+  uint64_t* v_empty = bars + 8;    // [2]
+  uint64_t* s_ready = bars + 10;   // [2]
+  uint64_t* dp_ready = bars + 12;
+  uint64_t* ds_ready = bars + 13;
+  uint64_t* done = bars + 14;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
+    mbar_init(q_full, 1);
+    mbar_init(do_full, 1);
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&qdo_full[s], 1);
-      mbar_init(&qdo_empty[s], 1);
-      mbar_init(&sdp_ready[s], 1);
-      mbar_init(&dq_drained[s], 8);
+      mbar_init(&k_full[s], 1);
+      mbar_init(&v_full[s], 1);
+      mbar_init(&k_empty[s], 1);
+      mbar_init(&v_empty[s], 1);
+      mbar_init(&s_ready[s], 1);
     }
-    mbar_init(pds_ready, 8);
-    mbar_init(mma3_done, 1);
+    mbar_init(dp_ready, 1);
+    mbar_init(ds_ready, 8);
+    mbar_init(done, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tm_q);
@@ -125,213 +198,431 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // columns: S[2] 0..127, dP[2] (later dQ^T) 128..255, dV 256..383, dK 384..511
-  const uint32_t tm_dv = tmem_base + 256, tm_dk = tmem_base + 384;
+  // columns: S[2] 0..255, dP (then dS) 256..383, dQ 384..511
+  const uint32_t tm_dp = tmem_base + 256, tm_dq = tmem_base + 384;
 
   if (warp == 0) {
-    // ------------------------------------------------ TMA producer
-    if (lane == 0 && n_iter > 0) {
-      mbar_arrive_expect_tx(kv_full, 2 * FB_KV_TILE);
-      tma_load_2d(k_sh, &tm_k, kv_full, hk * FB_D, k_beg + kv0);
-      tma_load_2d(k_sh + FB_KV_TILE / 2, &tm_k, kv_full, hk * FB_D + 64, k_beg + kv0);
-      tma_load_2d(v_sh, &tm_v, kv_full, hk * FB_D, k_beg + kv0);
-      tma_load_2d(v_sh + FB_KV_TILE / 2, &tm_v, kv_full, hk * FB_D + 64, k_beg + kv0);
-      for (int i = 0; i < n_iter && !*abort_flag; ++i) {
-        const int s = i & 1;
-        const int h = hk * G + i / per_head, qb = qb_first + i % per_head;
-        if (!mbar_wait(&qdo_empty[s], ((i >> 1) & 1) ^ 1)) FB_FAIL(ST_TIMEOUT_EMPTY)
-        const int row = q_beg + qb * FB_BQ;
-        mbar_arrive_expect_tx(&qdo_full[s], 2 * FB_Q_TILE);
-        tma_load_2d(q_sh + s * FB_Q_TILE, &tm_q, &qdo_full[s], h * FB_D, row);
-        tma_load_2d(q_sh + s * FB_Q_TILE + FB_Q_TILE / 2, &tm_q, &qdo_full[s], h * FB_D + 64, row);
-        tma_load_2d(do_sh + s * FB_Q_TILE, &tm_do, &qdo_full[s], h * FB_D, row);
-        tma_load_2d(do_sh + s * FB_Q_TILE + FB_Q_TILE / 2, &tm_do, &qdo_full[s], h * FB_D + 64, row);
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------ MMA issuer
-    if (lane == 0 && n_iter > 0) {
-      constexpr uint32_t id_s = umma_idesc_bf16_f32(128, FB_BQ);                                 // both K-major
-      constexpr uint32_t id_dkv = umma_idesc_bf16_f32(128, FB_D) | (1u << 16);                   // B MN-major
-      constexpr uint32_t id_dq = umma_idesc_bf16_f32(128, FB_BQ) | (1u << 15) | (1u << 16);      // A, B MN-major
-      const uint32_t k_a = smem_u32(k_sh), v_a = smem_u32(v_sh), pt_a = smem_u32(pt_sh), ds_a = smem_u32(ds_sh);
-      auto issue_sdp = [&](int i) -> bool {   // S^T(i), dP^T(i)
-        const int s = i & 1;
-        if (!mbar_wait(&qdo_full[s], (i >> 1) & 1)) return false;
-        // dP[s] still holds dQ^T of iteration i-2 until the softmax warps have drained it
-        if (i >= 2 && !mbar_wait(&dq_drained[s], ((i - 2) >> 1) & 1)) return false;
-        tc_fence_after_sync();
-        const uint32_t q_a = smem_u32(q_sh + s * FB_Q_TILE), do_a = smem_u32(do_sh + s * FB_Q_TILE);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_bf16_ss(tmem_base + s * FB_BQ, umma_desc_kmajor_sw128(k_a + (k >> 2) * (FB_KV_TILE / 2) + (k & 3) * 32),
-                       umma_desc_kmajor_sw128(q_a + (k >> 2) * (FB_Q_TILE / 2) + (k & 3) * 32), id_s, k > 0 ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          umma_bf16_ss(tmem_base + 128 + s * FB_BQ,
-                       umma_desc_kmajor_sw128(v_a + (k >> 2) * (FB_KV_TILE / 2) + (k & 3) * 32),
-                       umma_desc_kmajor_sw128(do_a + (k >> 2) * (FB_Q_TILE / 2) + (k & 3) * 32), id_s, k > 0 ? 1u : 0u);
-        tc_commit(&sdp_ready[s]);
-        return true;
-      };
+    if (lane == 0 && n > 0) {
       do {
-        if (!mbar_wait(kv_full, 0)) FB_FAIL(ST_TIMEOUT_FULL)
-        if (!issue_sdp(0)) FB_FAIL(ST_TIMEOUT_FULL)
-        for (int i = 0; i < n_iter; ++i) {
-          const int s = i & 1;
-          if (i + 1 < n_iter && !issue_sdp(i + 1)) FB_FAIL(ST_TIMEOUT_FULL)
-          if (!mbar_wait(pds_ready, i & 1)) FB_FAIL(ST_TIMEOUT_TMEM_EMPTY)
-          tc_fence_after_sync();
-          const uint32_t q_a = smem_u32(q_sh + s * FB_Q_TILE), do_a = smem_u32(do_sh + s * FB_Q_TILE);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)   // dV += P^T dO      (K = 64 queries)
-            umma_bf16_ss(tm_dv, umma_desc_kmajor_sw128(pt_a + k * 32), umma_desc_mnmajor_sw128(do_a + k * 2048, FB_Q_TILE / 2),
-                         id_dkv, (i > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)   // dK += dS^T Q
-            umma_bf16_ss(tm_dk, umma_desc_kmajor_sw128(ds_a + k * 32), umma_desc_mnmajor_sw128(q_a + k * 2048, FB_Q_TILE / 2),
-                         id_dkv, (i > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-          for (int k = 0; k < 8; ++k)   // dQ^T = K^T dS^T   (K = 128 keys), over dP[s]
-            umma_bf16_ss(tmem_base + 128 + s * FB_BQ, umma_desc_mnmajor_sw128(k_a + k * 2048, FB_KV_TILE / 2),
-                         umma_desc_mnmajor_sw128(ds_a + k * 2048, FB_P_TILE), id_dq, k > 0 ? 1u : 0u);
-          tc_commit(&qdo_empty[s]);
-          tc_commit(mma3_done);
+        mbar_arrive_expect_tx(q_full, FB_TILE);
+        fb_load_tile(q_sh, &tm_q, q_full, h * FB_D, q_beg + q0);
+        for (int j = 0; j < n && !*abort_flag; ++j) {
+          const int s = j & 1, row = k_beg + j * FB_B;
+          const uint32_t ph = ((j >> 1) & 1) ^ 1;
+          FB_WAIT1(&k_empty[s], ph, ST_TIMEOUT_EMPTY)
+          mbar_arrive_expect_tx(&k_full[s], FB_TILE);
+          fb_load_tile(k_sh + s * FB_TILE, &tm_k, &k_full[s], hk * FB_D, row);
+          if (j == 0) {
+            mbar_arrive_expect_tx(do_full, FB_TILE);
+            fb_load_tile(do_sh, &tm_do, do_full, h * FB_D, q_beg + q0);
+          }
+          FB_WAIT1(&v_empty[s], ph, ST_TIMEOUT_EMPTY)
+          mbar_arrive_expect_tx(&v_full[s], FB_TILE);
+          fb_load_tile(v_sh + s * FB_TILE, &tm_v, &v_full[s], hk * FB_D, row);
         }
       } while (false);
     }
+  } else if (warp == 1) {
+    if (lane == 0 && n > 0) {
+      const uint32_t q_a = smem_u32(q_sh), do_a = smem_u32(do_sh);
+      do {
+        FB_WAIT1(q_full, 0, ST_TIMEOUT_FULL)
+        FB_WAIT1(&k_full[0], 0, ST_TIMEOUT_FULL)
+        tc_fence_after_sync();
+        fb_mma_ss(tmem_base, q_a, smem_u32(k_sh));
+        tc_commit(&s_ready[0]);
+        FB_WAIT1(do_full, 0, ST_TIMEOUT_FULL)
+        FB_WAIT1(&v_full[0], 0, ST_TIMEOUT_FULL)
+        tc_fence_after_sync();
+        fb_mma_ss(tm_dp, do_a, smem_u32(v_sh));
+        tc_commit(dp_ready);
+        tc_commit(&v_empty[0]);
+        for (int j = 0; j < n; ++j) {
+          const int s = j & 1, s1 = s ^ 1;
+          const uint32_t ph1 = ((j + 1) >> 1) & 1;
+          if (j + 1 < n) {   // S of the next block: its buffer was read before dS(j-1) was announced
+            FB_WAIT1(&k_full[s1], ph1, ST_TIMEOUT_FULL)
+            tc_fence_after_sync();
+            fb_mma_ss(tmem_base + s1 * 128, q_a, smem_u32(k_sh + s1 * FB_TILE));
+            tc_commit(&s_ready[s1]);
+          }
+          FB_WAIT1(ds_ready, j & 1, ST_TIMEOUT_TMEM_EMPTY)
+          tc_fence_after_sync();
+          fb_mma_ts(tm_dq, tm_dp, smem_u32(k_sh + s * FB_TILE), j == 0);
+          tc_commit(&k_empty[s]);
+          if (j + 1 < n) {
+            FB_WAIT1(&v_full[s1], ph1, ST_TIMEOUT_FULL)
+            tc_fence_after_sync();
+            fb_mma_ss(tm_dp, do_a, smem_u32(v_sh + s1 * FB_TILE));
+            tc_commit(dp_ready);
+            tc_commit(&v_empty[s1]);
+          }
+        }
+        if (!*abort_flag) tc_commit(done);
+      } while (false);
+    }
   } else {
-    // ------------------------------------------------ softmax / dS / drains (warps 2..9)
-    // warp -> (TMEM lane quadrant, half of the 64 query columns). S^T / dP^T rows are keys, dQ^T rows are head-dim.
     const int quad = warp & 3;
-    const int chalf = (warp - 2) >> 2;
+    const int c0 = ((warp - 2) >> 2) * 64;               // first key column of this warp
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    const int c0 = chalf * 32;                           // first query column of this warp
+    const int q_idx = q0 + row;
+    const bool live = q_idx < len_q;
+    const int k_limit = p.causal ? min(len_k, q_idx + shift + 1) : len_k;   // keys [0, k_limit) are visible
+    // delta of 16 of the quadrant's 32 rows per warp: a row is one coalesced 256-byte read of O and of dO, and the sixteen
+    // sums are reduced together (each shuffle step halves the rows that a lane carries)
+    {
+      float v[16];
+      uint2 o2[16], g2[16];
+      const int half = (warp - 2) >> 2;
+      // rows past the end are read at the last row and dropped: no branch keeps the 32 loads apart
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const long long t = q_beg + min(q0 + quad * 32 + half * 16 + i, len_q - 1);
+        o2[i] = *reinterpret_cast<const uint2*>(p.out + t * p.ldo + h * FB_D + lane * 4);
+        g2[i] = *reinterpret_cast<const uint2*>(p.dout + t * p.lddo + h * FB_D + lane * 4);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].x));
+        const float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].y));
+        const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].x));
+        const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].y));
+        v[i] = (x0.x * y0.x + x0.y * y0.y) + (x1.x * y1.x + x1.y * y1.y);
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) {   // lane distance 2 w: w rows stay with each lane
+        const bool hi = lane & (2 * w);
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+          const float send = hi ? v[i] : v[i + w], keep = hi ? v[i + w] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * w);
+        }
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      const int r = half * 16 + (lane >> 1), qi = q0 + quad * 32 + r;
+      if ((lane & 1) == 0) {
+        delta_sh[quad * 32 + r] = qi < len_q ? v[0] : 0.f;
+        if (qi < len_q) p.delta[(long long)h * p.Tq + q_beg + qi] = v[0];
+      }
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");   // the two warps of this quadrant
+    }
+    const float delta = delta_sh[row];
+    const float nlse = live ? -p.lse[(long long)h * p.Tq + q_beg + q_idx] * FB_LOG2E : -INFINITY;
+    const float2 c2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(nlse, nlse);
+    const float2 nd2 = make_float2(-delta, -delta);
+    bool ok = true;
+    for (int j = 0; j < n; ++j) {
+      const int s = j & 1;
+      if (!(ok = fb_wait(&s_ready[s], (j >> 1) & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+      tc_fence_after_sync();
+      float2 e[32];
+      const int key0 = j * FB_B + c0;
+      const bool need_mask = key0 + 64 > k_limit;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tmem_base + s * 128 + lane_addr + c0 + half * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 x = fma2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), c2, nl2);
+          e[half * 16 + i] = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+        }
+      }
+      if (need_mask) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          if (key0 + 2 * i >= k_limit) e[i].x = 0.f;
+          if (key0 + 2 * i + 1 >= k_limit) e[i].y = 0.f;
+        }
+      }
+      if (!(ok = fb_wait(dp_ready, j & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+      tc_fence_after_sync();
+      uint32_t ds[32];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tm_dp + lane_addr + c0 + half * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 v = mul2(e[half * 16 + i],
+                                add2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), nd2));
+          ds[half * 16 + i] = pack_bf16x2(v.x, v.y);
+        }
+      }
+      tmem_st_32x32b_x32(tm_dp + lane_addr + c0, ds);   // over the first half of the columns just read
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_ready);
+    }
+    if (ok && n > 0) ok = fb_wait(done, 0, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag);
+    if (ok) {
+      tc_fence_after_sync();
+      fb_store_row(tm_dq + lane_addr + c0, n == 0, p.scale, p.dq + (long long)(q_beg + q_idx) * p.lddq + h * FB_D + c0, live);
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag && threadIdx.x == 0) {
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);     // copies already issued land before shared memory is released
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// dK, dV
+// ---------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(FB_THREADS, 1)
+flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, FbParams p) {
+  const int heads = p.hkv * p.B;
+  const int hb = blockIdx.x % heads, hk = hb % p.hkv, b = hb / p.hkv;
+  const int kv0 = blockIdx.x / heads * FB_B;            // early key blocks are seen by most queries: first
+  const int q_beg = p.cu_q[b], len_q = p.cu_q[b + 1] - q_beg;
+  const int k_beg = p.cu_k[b], len_k = p.cu_k[b + 1] - k_beg;
+  if (kv0 >= len_k) return;
+  const int shift = len_k - len_q;
+  const int G = p.hq / p.hkv;
+  const int nqb = (len_q + FB_B - 1) / FB_B;
+  int qb_first = 0;
+  if (p.causal && kv0 - shift > 0) qb_first = (kv0 - shift) / FB_B;
+  const int per_head = nqb > qb_first ? nqb - qb_first : 0;
+  const int n = per_head * G;
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* k_sh = smem;
+  uint8_t* v_sh = smem + FB_TILE;
+  uint8_t* q_sh = smem + 2 * FB_TILE;                   // [2]
+  uint8_t* do_sh = smem + 4 * FB_TILE;                  // [2]
+  float* lse_sh = reinterpret_cast<float*>(smem + 6 * FB_TILE);   // [2][128] -lse * log2(e)
+  float* dlt_sh = lse_sh + 2 * FB_B;                              // [2][128] -delta
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * FB_TILE + FB_STATS);
+  uint64_t* k_full = bars;
+  uint64_t* v_full = bars + 1;
+  uint64_t* q_full = bars + 2;     // [2] Q tile and the statistics of its rows
+  uint64_t* do_full = bars + 4;    // [2]
+  uint64_t* q_empty = bars + 6;    // [2]
+  uint64_t* do_empty = bars + 8;   // [2]
+  uint64_t* st_empty = bars + 10;  // [2] statistics read by the softmax warps
+  uint64_t* s_ready = bars + 12;
+  uint64_t* dp_ready = bars + 13;
+  uint64_t* p_ready = bars + 14;
+  uint64_t* ds_ready = bars + 15;
+  uint64_t* done = bars + 16;
+  uint64_t* st_full = bars + 17;   // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&do_full[s], 1);
+      mbar_init(&q_empty[s], 1);
+      mbar_init(&do_empty[s], 1);
+      mbar_init(&st_empty[s], 8);
+      mbar_init(&st_full[s], 1);
+    }
+    mbar_init(s_ready, 1);
+    mbar_init(dp_ready, 1);
+    mbar_init(p_ready, 8);
+    mbar_init(ds_ready, 8);
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+    tma_prefetch_desc(&tm_do);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  // columns: S (then P) 0..127, dP (then dS) 128..255, dV 256..383, dK 384..511
+  const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128, tm_dv = tmem_base + 256, tm_dk = tmem_base + 384;
+
+  if (warp == 0) {
+    // the whole warp: lane 0 issues the tile loads, all lanes fetch the 128 rows' lse and delta with plain loads
+    // (their addresses have no 16-byte alignment, so they cannot be a bulk copy)
+    for (int i = 0; i < n && !*abort_flag; ++i) {
+      const int s = i & 1;
+      const uint32_t ph = ((i >> 1) & 1) ^ 1;
+      const int h = hk * G + i / per_head, qr = (qb_first + i % per_head) * FB_B;
+      float ls[4], dl[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int qi = qr + lane + 32 * j;
+        const long long at = (long long)h * p.Tq + q_beg + qi;
+        ls[j] = qi < len_q ? -p.lse[at] * FB_LOG2E : -INFINITY;
+        dl[j] = qi < len_q ? -p.delta[at] : 0.f;
+      }
+      if (!fb_wait(&q_empty[s], ph, ST_TIMEOUT_EMPTY, p.status, abort_flag)) break;
+      if (lane == 0) {
+        if (i == 0) {
+          mbar_arrive_expect_tx(k_full, FB_TILE);
+          fb_load_tile(k_sh, &tm_k, k_full, hk * FB_D, k_beg + kv0);
+        }
+        mbar_arrive_expect_tx(&q_full[s], FB_TILE);
+        fb_load_tile(q_sh + s * FB_TILE, &tm_q, &q_full[s], h * FB_D, q_beg + qr);
+        if (i == 0) {
+          mbar_arrive_expect_tx(v_full, FB_TILE);
+          fb_load_tile(v_sh, &tm_v, v_full, hk * FB_D, k_beg + kv0);
+        }
+      }
+      if (!fb_wait(&do_empty[s], ph, ST_TIMEOUT_EMPTY, p.status, abort_flag)) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&do_full[s], FB_TILE);
+        fb_load_tile(do_sh + s * FB_TILE, &tm_do, &do_full[s], h * FB_D, q_beg + qr);
+      }
+      if (!fb_wait(&st_empty[s], ph, ST_TIMEOUT_EMPTY, p.status, abort_flag)) break;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        lse_sh[s * FB_B + lane + 32 * j] = ls[j];
+        dlt_sh[s * FB_B + lane + 32 * j] = dl[j];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&st_full[s]);
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && n > 0) {
+      const uint32_t k_a = smem_u32(k_sh), v_a = smem_u32(v_sh);
+      do {
+        FB_WAIT1(k_full, 0, ST_TIMEOUT_FULL)
+        FB_WAIT1(&q_full[0], 0, ST_TIMEOUT_FULL)
+        tc_fence_after_sync();
+        fb_mma_ss(tm_s, k_a, smem_u32(q_sh));
+        tc_commit(s_ready);
+        FB_WAIT1(v_full, 0, ST_TIMEOUT_FULL)
+        FB_WAIT1(&do_full[0], 0, ST_TIMEOUT_FULL)
+        tc_fence_after_sync();
+        fb_mma_ss(tm_dp, v_a, smem_u32(do_sh));
+        tc_commit(dp_ready);
+        for (int i = 0; i < n; ++i) {
+          const int s = i & 1, s1 = s ^ 1;
+          const uint32_t ph1 = ((i + 1) >> 1) & 1;
+          FB_WAIT1(p_ready, i & 1, ST_TIMEOUT_TMEM_EMPTY)
+          tc_fence_after_sync();
+          fb_mma_ts(tm_dv, tm_s, smem_u32(do_sh + s * FB_TILE), i == 0);      // dV += P^T dO
+          tc_commit(&do_empty[s]);
+          if (i + 1 < n) {
+            FB_WAIT1(&q_full[s1], ph1, ST_TIMEOUT_FULL)
+            tc_fence_after_sync();
+            fb_mma_ss(tm_s, k_a, smem_u32(q_sh + s1 * FB_TILE));              // S^T of the next block, over P^T
+            tc_commit(s_ready);
+          }
+          FB_WAIT1(ds_ready, i & 1, ST_TIMEOUT_TMEM_EMPTY)
+          tc_fence_after_sync();
+          fb_mma_ts(tm_dk, tm_dp, smem_u32(q_sh + s * FB_TILE), i == 0);      // dK += dS^T Q
+          tc_commit(&q_empty[s]);
+          if (i + 1 < n) {
+            FB_WAIT1(&do_full[s1], ph1, ST_TIMEOUT_FULL)
+            tc_fence_after_sync();
+            fb_mma_ss(tm_dp, v_a, smem_u32(do_sh + s1 * FB_TILE));            // dP^T of the next block, over dS^T
+            tc_commit(dp_ready);
+          }
+        }
+        if (!*abort_flag) tc_commit(done);
+      } while (false);
+    }
+  } else {
+    // rows (TMEM lanes) are keys, columns are queries: the statistics of a column come from shared memory
+    const int quad = warp & 3;
+    const int c0 = ((warp - 2) >> 2) * 64;
+    const int row = quad * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     const int key = kv0 + row;
     const bool key_ok = key < len_k;
     const int q_min = p.causal ? key - shift : -(1 << 30);   // visible iff q >= key - shift
-    const int tid = threadIdx.x - 64;                    // 0..255
+    const float2 c2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
-    auto load_stats = [&](int i, float& l, float& dl) {  // threads 0..63: statistics of query (i, tid)
-      const int ph = per_head > 0 ? per_head : 1;
-      const int h = hk * G + i / ph, qi = (qb_first + i % ph) * FB_BQ + tid;
-      const long long o = (long long)h * p.Tq + q_beg + qi;
-      const bool live = tid < FB_BQ && i < n_iter && qi < len_q;
-      l = live ? p.lse[o] * FB_LOG2E : INFINITY;
-      dl = live ? p.delta[o] : 0.f;
-    };
-    auto drain_dq = [&](int j) {                         // dQ^T of iteration j: lanes = head-dim, columns = queries
-      const int s = j & 1;
-      const int h = hk * G + j / per_head, q0 = (qb_first + j % per_head) * FB_BQ;
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_base + 128 + s * FB_BQ + lane_addr + c0, r);
-      tmem_ld_wait();
-      float* dst = p.dq_accum + ((long long)(q_beg + q0 + c0) * p.hq + h) * FB_D + row;
+    for (int i = 0; i < n; ++i) {
+      const int s = i & 1;
+      const int qc0 = (qb_first + i % per_head) * FB_B + c0;   // first query of this warp's columns
+      if (!(ok = fb_wait(&st_full[s], (i >> 1) & 1, ST_TIMEOUT_FULL, p.status, abort_flag))) break;
+      if (!(ok = fb_wait(s_ready, i & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+      tc_fence_after_sync();
+      const float4* nl = reinterpret_cast<const float4*>(lse_sh + s * FB_B + c0);
+      const float4* nd = reinterpret_cast<const float4*>(dlt_sh + s * FB_B + c0);
+      float2 e[32];
 #pragma unroll
-      for (int c = 0; c < 32; ++c)
-        if (q0 + c0 + c < len_q) atomicAdd(dst + (long long)c * p.hq * FB_D, __uint_as_float(r[c]));
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tm_s + lane_addr + c0 + half * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const float4 l4 = nl[half * 8 + g];
+          const float2 x = fma2(make_float2(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1])), c2, make_float2(l4.x, l4.y));
+          const float2 y = fma2(make_float2(__uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3])), c2, make_float2(l4.z, l4.w));
+          e[half * 16 + 2 * g] = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+          e[half * 16 + 2 * g + 1] = make_float2(exp2_approx(y.x), exp2_approx(y.y));
+        }
+      }
+      if (qc0 < q_min || qc0 + 64 > len_q) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          if (qc0 + 2 * c < q_min || qc0 + 2 * c >= len_q) e[c].x = 0.f;
+          if (qc0 + 2 * c + 1 < q_min || qc0 + 2 * c + 1 >= len_q) e[c].y = 0.f;
+        }
+      }
+      {
+        uint32_t pk[32];
+#pragma unroll
+        for (int c = 0; c < 32; ++c) pk[c] = pack_bf16x2(e[c].x, e[c].y);
+        tmem_st_32x32b_x32(tm_s + lane_addr + c0, pk);
+        tmem_st_wait();
+      }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&dq_drained[s]);
-    };
-    float l_next, d_next;
-    load_stats(0, l_next, d_next);
-    for (int i = 0; i < n_iter; ++i) {                   // never left early (named barrier inside)
-      const int s = i & 1;
-      const int q0 = (qb_first + i % per_head) * FB_BQ;
-      if (tid < FB_BQ) { lse_sh[s * FB_BQ + tid] = l_next; dlt_sh[s * FB_BQ + tid] = d_next; }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (*abort_flag) ok = false;
-      load_stats(i + 1, l_next, d_next);                 // prefetch for the next iteration
-      if (ok && !mbar_wait(&sdp_ready[s], (i >> 1) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
-      ok = __all_sync(0xffffffffu, ok);                  // tcgen05.ld below is warp-collective
-      uint32_t pp[16], dd[16];
-      if (ok) {
-        tc_fence_after_sync();
-        uint32_t rs[32], rd[32];
-        tmem_ld_32x32b_x32(tmem_base + s * FB_BQ + lane_addr + c0, rs);
-        tmem_ld_32x32b_x32(tmem_base + 128 + s * FB_BQ + lane_addr + c0, rd);
+      if (lane == 0) mbar_arrive(p_ready);
+      if (!(ok = fb_wait(dp_ready, i & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+      tc_fence_after_sync();
+      uint32_t ds[32];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tm_dp + lane_addr + c0 + half * 32, r);
         tmem_ld_wait();
-        const bool need_mask = !key_ok || (q0 < q_min) || (q0 + FB_BQ > len_q);
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          float pv[2], dv2[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int qc = c0 + c + u;
-            float pe = fb_exp2(fmaf(__uint_as_float(rs[c + u]), p.scale_log2, -lse_sh[s * FB_BQ + qc]));
-            if (need_mask && (!key_ok || q0 + qc < q_min || q0 + qc >= len_q)) pe = 0.f;
-            pv[u] = pe;
-            dv2[u] = pe * (__uint_as_float(rd[c + u]) - dlt_sh[s * FB_BQ + qc]) * p.scale;
-          }
-          pp[c >> 1] = pack_bf16x2(pv[0], pv[1]);
-          dd[c >> 1] = pack_bf16x2(dv2[0], dv2[1]);
+        for (int g = 0; g < 8; ++g) {
+          const float4 d4 = nd[half * 8 + g];
+          const float2 x = mul2(e[half * 16 + 2 * g], add2(make_float2(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1])), make_float2(d4.x, d4.y)));
+          const float2 y = mul2(e[half * 16 + 2 * g + 1], add2(make_float2(__uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3])), make_float2(d4.z, d4.w)));
+          ds[half * 16 + 2 * g] = pack_bf16x2(x.x, x.y);
+          ds[half * 16 + 2 * g + 1] = pack_bf16x2(y.x, y.y);
         }
-        tc_fence_before_sync();
       }
-      // P^T / dS^T of the previous iteration are still being read by its three MMAs until mma3_done(i-1)
-      if (ok && i > 0 && !mbar_wait(mma3_done, (i - 1) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        const int off = row * 128;
-        const int chunk0 = c0 >> 3;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int sw = ((chunk0 + g) ^ (row & 7)) << 4;
-          *reinterpret_cast<uint4*>(pt_sh + off + sw) = make_uint4(pp[4 * g], pp[4 * g + 1], pp[4 * g + 2], pp[4 * g + 3]);
-          *reinterpret_cast<uint4*>(ds_sh + off + sw) = make_uint4(dd[4 * g], dd[4 * g + 1], dd[4 * g + 2], dd[4 * g + 3]);
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pds_ready);
-        // while the tensor core runs the three MMAs of iteration i: drain dQ^T of iteration i-1
-        if (i > 0) {
-          tc_fence_after_sync();
-          drain_dq(i - 1);
-        }
+      tmem_st_32x32b_x32(tm_dp + lane_addr + c0, ds);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&st_empty[s]);
+        mbar_arrive(ds_ready);
       }
     }
-    // ---- last dQ^T, then dK, dV of the key block
-    if (n_iter > 0) {
-      if (ok && !mbar_wait(mma3_done, (n_iter - 1) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        tc_fence_after_sync();
-        drain_dq(n_iter - 1);
-      }
+    if (ok && n > 0) ok = fb_wait(done, 0, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag);
+    if (ok) {
+      tc_fence_after_sync();
+      fb_store_row(tm_dk + lane_addr + c0, n == 0, p.scale, p.dk + (long long)(k_beg + key) * p.lddk + hk * FB_D + c0, key_ok);
+      fb_store_row(tm_dv + lane_addr + c0, n == 0, 1.f, p.dv + (long long)(k_beg + key) * p.lddv + hk * FB_D + c0, key_ok);
     }
-    if (ok) {                                            // loads by every lane, stores by rows inside the sequence
-      __nv_bfloat16* dkr = p.dk + (long long)(k_beg + key) * p.lddk + hk * FB_D;
-      __nv_bfloat16* dvr = p.dv + (long long)(k_beg + key) * p.lddv + hk * FB_D;
-#pragma unroll 1
-      for (int c = chalf * 64; c < chalf * 64 + 64; c += 32) {
-        uint32_t a[32], bb[32];
-        if (n_iter > 0) {
-          tmem_ld_32x32b_x32(tm_dk + lane_addr + c, a);
-          tmem_ld_32x32b_x32(tm_dv + lane_addr + c, bb);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) { a[j] = 0u; bb[j] = 0u; }
-        }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 o;
-          o.x = pack_bf16x2(__uint_as_float(a[8 * g + 0]), __uint_as_float(a[8 * g + 1]));
-          o.y = pack_bf16x2(__uint_as_float(a[8 * g + 2]), __uint_as_float(a[8 * g + 3]));
-          o.z = pack_bf16x2(__uint_as_float(a[8 * g + 4]), __uint_as_float(a[8 * g + 5]));
-          o.w = pack_bf16x2(__uint_as_float(a[8 * g + 6]), __uint_as_float(a[8 * g + 7]));
-          if (key_ok) *reinterpret_cast<uint4*>(dkr + c + 8 * g) = o;
-          o.x = pack_bf16x2(__uint_as_float(bb[8 * g + 0]), __uint_as_float(bb[8 * g + 1]));
-          o.y = pack_bf16x2(__uint_as_float(bb[8 * g + 2]), __uint_as_float(bb[8 * g + 3]));
-          o.z = pack_bf16x2(__uint_as_float(bb[8 * g + 4]), __uint_as_float(bb[8 * g + 5]));
-          o.w = pack_bf16x2(__uint_as_float(bb[8 * g + 6]), __uint_as_float(bb[8 * g + 7]));
-          if (key_ok) *reinterpret_cast<uint4*>(dvr + c + 8 * g) = o;
-        }
-      }
-    }
-    tc_fence_before_sync();
   }
 
   tc_fence_before_sync();
@@ -346,60 +637,40 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
 }
 
-// delta[h, t] = sum_d O[t, h, d] * dO[t, h, d]; one warp per (t, h)
-__global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                                   float* __restrict__ delta, int T, int hq, long long ldo, long long lddo) {
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= (long long)T * hq) return;
-  const int t = (int)(w / hq), h = (int)(w % hq);
-  const uint2 a = *reinterpret_cast<const uint2*>(o + t * ldo + h * FB_D + lane * 4);
-  const uint2 b = *reinterpret_cast<const uint2*>(dout + t * lddo + h * FB_D + lane * 4);
-  const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&a);
-  const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&b);
-  float s = 0.f;
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const float2 x = __bfloat1622float2(ah[j]), y = __bfloat1622float2(bh[j]);
-    s += x.x * y.x + x.y * y.y;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) delta[(long long)h * T + t] = s;
-}
-
 }  // namespace b200
 
-// Gradients of b200_flash_fwd. dq_accum [Tq, hq, 128] fp32 must be zero on entry and holds dQ on return;
-// dk / dv [Tk, hkv, 128] bf16 are overwritten; delta [hq, Tq] fp32 is scratch. max_k bounds the grid.
+// Gradients of b200_flash_fwd: dq [Tq, hq, 128], dk / dv [Tk, hkv, 128] bf16 are overwritten (rows of dq outside every
+// sequence are zeroed); delta [hq, Tq] fp32 is scratch. max_q / max_k bound the grids.
 extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout,
-                              const float* lse, float* dq_accum, void* dk, void* dv, float* delta, const int* cu_q,
+                              const float* lse, void* dq, void* dk, void* dv, float* delta, const int* cu_q,
                               const int* cu_k, int B, int Tq, int Tk, int hq, int hkv, int d, long long ldq,
-                              long long ldk, long long ldv, long long ldo, long long lddo, long long lddk,
-                              long long lddv, int max_k, int causal, float scale, uint32_t* status,
-                              cudaStream_t stream) {
+                              long long ldk, long long ldv, long long ldo, long long lddo, long long lddq,
+                              long long lddk, long long lddv, int max_q, int max_k, int causal, float scale,
+                              uint32_t* status, cudaStream_t stream) {
   using namespace b200;
   if (B <= 0 || Tq <= 0 || Tk <= 0) return 0;
   if (d != FB_D || hkv <= 0 || hq % hkv || (ldq & 7) || (ldk & 7) || (ldv & 7) || (ldo & 3) || (lddo & 7) ||
-      (lddk & 7) || (lddv & 7) || max_k <= 0)
+      (lddq & 7) || (lddk & 7) || (lddv & 7) || max_q <= 0 || max_k <= 0 || ((uintptr_t)out & 7) || ((uintptr_t)dq & 15) ||
+      ((uintptr_t)dk & 15) || ((uintptr_t)dv & 15))
     return B200_ERR_ARG;
+  const long long grid_q = (long long)((max_q + FB_B - 1) / FB_B) * hq * B, grid_k = (long long)((max_k + FB_B - 1) / FB_B) * hkv * B;
+  if (grid_q > 0x7fffffff || grid_k > 0x7fffffff) return B200_ERR_TOO_LARGE;
   CUtensorMap tm_q, tm_k, tm_v, tm_do;
-  if (make_tmap_2d(&tm_q, q, Tq, (uint64_t)hq * FB_D, ldq, FB_BQ, 64, 2)) return B200_ERR_TENSORMAP;
-  if (make_tmap_2d(&tm_k, k, Tk, (uint64_t)hkv * FB_D, ldk, FB_BK, 64, 2)) return B200_ERR_TENSORMAP;
-  if (make_tmap_2d(&tm_v, v, Tk, (uint64_t)hkv * FB_D, ldv, FB_BK, 64, 2)) return B200_ERR_TENSORMAP;
-  if (make_tmap_2d(&tm_do, dout, Tq, (uint64_t)hq * FB_D, lddo, FB_BQ, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_q, q, Tq, (uint64_t)hq * FB_D, ldq, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_k, k, Tk, (uint64_t)hkv * FB_D, ldk, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_v, v, Tk, (uint64_t)hkv * FB_D, ldv, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_do, dout, Tq, (uint64_t)hq * FB_D, lddo, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(flash_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(flash_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM) != cudaSuccess)
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  const long long warps = (long long)Tq * hq;
-  flash_delta_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, stream>>>(
-      (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, Tq, hq, ldo, lddo);
-  FbParams p{cu_q, cu_k, lse, delta, dq_accum, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, lddk, lddv, hq, hkv, Tq, causal,
-             scale, scale * FB_LOG2E, status};
-  dim3 grid((max_k + FB_BK - 1) / FB_BK, hkv, B);
-  flash_bwd_kernel<<<grid, FB_THREADS, FB_SMEM, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
+  FbParams p{cu_q, cu_k, lse, delta, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dq,
+             (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, causal, scale,
+             scale * FB_LOG2E, status};
+  flash_bwd_dq_kernel<<<(unsigned)grid_q, FB_THREADS, FB_SMEM, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
+  flash_bwd_dkdv_kernel<<<(unsigned)grid_k, FB_THREADS, FB_SMEM, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
