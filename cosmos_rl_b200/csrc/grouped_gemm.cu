@@ -18,68 +18,85 @@
 namespace b200 {
 
 struct GroupedParams {
-  void* C;
-  long long ldc;
-  long long c_batch_stride;   // wgrad: elements between dW[e] and dW[e+1]
+  const CUtensorMap* tm_out;  // output as [batches, rows, N] (batches = experts for wgrad, else 1): boxes of 32 rows x 128 bytes
+  const __nv_bfloat16* old;   // bf16 output that is accumulated into: its values are added in fp32 before the one rounding
+  long long ld_old, batch_old;
   int N;                      // output columns
   int rows_limit;             // fwd/dgrad: allocated rows of C; wgrad: output rows per expert
-  int out_fp32, accumulate, bn;
+  int out_fp32, accumulate, bn, batched;
   const int* tile_expert;     // [max_tiles] expert of each 128-row tile (fwd/dgrad)
   const int* expert_offsets;  // [E + 1] padded row offsets (wgrad)
   const int* n_tiles;         // [1] number of 128-row tiles in use
   int num_experts;
-  int K;                      // contraction length (fwd/dgrad)
 };
 
+// Each warp turns its 32 accumulator rows into slabs of 32 rows x 128 bytes in swizzled shared memory and hands them to
+// TMA stores (reduce-adds when an fp32 result is accumulated), which clip rows and columns outside the output. The weight
+// gradient is bound by these stores: an expert of 256 tokens has four contraction blocks per 64 KB of output.
 struct GroupedEpilogue {
   using Params = GroupedParams;
-  __device__ __forceinline__ void tile_begin(const Params&, const TileInfo&, int) {}
-  __device__ __forceinline__ void tile_end(const Params&, const TileInfo&, int) {}
-  __device__ __forceinline__ void finish(const Params&) {}
-  __device__ __forceinline__ void chunk(const Params& p, const TileInfo& t, int row, int col0, const float (&v)[32]) {
-    // forward / dgrad: batch offset is zero and m_blk indexes the padded token rows;
-    // wgrad: m_blk indexes rows of dW[e] and the expert selects the slice.
-    char* base = reinterpret_cast<char*>(p.C) + (long long)(p.c_batch_stride ? t.batch : 0) * p.c_batch_stride *
-                                                    (p.out_fp32 ? 4 : 2);
-    StoreEpilogue_store(base, p.ldc, p.rows_limit, p.N, p.out_fp32, p.accumulate, (long long)t.m_blk * GEMM_BM + row,
-                        t.n_blk * p.bn + col0, v);
+  static constexpr bool CUSTOM_TILE = true;
+  uint32_t slab_idx = 0;
+  __device__ __forceinline__ void finish(const Params&) {
+    if ((threadIdx.x & 31) == 0) tma_store_wait<0>();
   }
-  static __device__ __forceinline__ void StoreEpilogue_store(void* C, long long ldc, long long M, int N, int out_fp32,
-                                                             int accumulate, long long r, int c,
-                                                             const float (&v)[32]) {
-    if (r >= M || c >= N) return;
-    if (out_fp32) {
-      float* dst = reinterpret_cast<float*>(C) + r * ldc + c;
-      for (int i = 0; i < 32 && c + i < N; ++i) dst[i] = accumulate ? dst[i] + v[i] : v[i];
-    } else {
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + r * ldc + c;
-      if (c + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+  __device__ __forceinline__ void tile(const Params& p, const TileInfo& t, int, uint32_t taddr, uint8_t* epi_smem) {
+    const int lane = threadIdx.x & 31, quad = (threadIdx.x >> 5) & 3;
+    uint8_t* slab0 = epi_smem + quad * 8192;
+    const uint32_t sw = (uint32_t)(lane & 7);   // 128-byte swizzle: 16-byte chunk j of row r sits at chunk j ^ (r & 7)
+    const int row0 = t.m_blk * GEMM_BM + quad * 32;
+    const int batch = p.batched ? t.batch : 0;
+    const int slab_cols = p.out_fp32 ? 32 : 64;
+#pragma unroll 1
+    for (int c = 0; c < p.bn; c += slab_cols) {
+      const int gc = t.n_blk * p.bn + c;
+      if (gc >= p.N) break;
+      uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
+      if (lane == 0) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
+      __syncwarp();
+      uint8_t* my_row = slab + lane * 128;
+      uint32_t r[2][32];
+      tmem_ld_32x32b_x32(taddr + c, r[0]);
+      if (!p.out_fp32) tmem_ld_32x32b_x32(taddr + c + 32, r[1]);
+      tmem_ld_wait();
+      if (t.num_kb == 0) {   // an expert without rows
 #pragma unroll
-        for (int i = 0; i < 32; i += 8) {
-          float w[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) w[j] = v[i + j];
-          if (accumulate) {
-            uint4 old = *reinterpret_cast<uint4*>(dst + i);
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&old);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float2 f = __bfloat1622float2(h[j]);
-              w[2 * j] += f.x;
-              w[2 * j + 1] += f.y;
-            }
-          }
-          uint4 o;
-          o.x = pack_bf16x2(w[0], w[1]);
-          o.y = pack_bf16x2(w[2], w[3]);
-          o.z = pack_bf16x2(w[4], w[5]);
-          o.w = pack_bf16x2(w[6], w[7]);
-          *reinterpret_cast<uint4*>(dst + i) = o;
-        }
-      } else {
-        for (int i = 0; i < 32 && c + i < N; ++i)
-          dst[i] = __float2bfloat16(accumulate ? __bfloat162float(dst[i]) + v[i] : v[i]);
+        for (int j = 0; j < 32; ++j) r[0][j] = r[1][j] = 0u;
       }
+      if (p.old != nullptr && row0 + lane < p.rows_limit) {
+        const __nv_bfloat16* o = p.old + batch * p.batch_old + (long long)(row0 + lane) * p.ld_old + gc;
+#pragma unroll
+        for (int j = 0; j < 64; ++j)
+          if (gc + j < p.N) r[j >> 5][j & 31] = __float_as_uint(__uint_as_float(r[j >> 5][j & 31]) + __bfloat162float(o[j]));
+      }
+      if (p.out_fp32) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<uint4*>(my_row + ((((uint32_t)j) ^ sw) << 4)) =
+              make_uint4(r[0][4 * j], r[0][4 * j + 1], r[0][4 * j + 2], r[0][4 * j + 3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t(&v)[32] = r[j >> 2];
+          const int k = (j & 3) * 8;
+          uint4 o;
+          o.x = pack_bf16x2(__uint_as_float(v[k]), __uint_as_float(v[k + 1]));
+          o.y = pack_bf16x2(__uint_as_float(v[k + 2]), __uint_as_float(v[k + 3]));
+          o.z = pack_bf16x2(__uint_as_float(v[k + 4]), __uint_as_float(v[k + 5]));
+          o.w = pack_bf16x2(__uint_as_float(v[k + 6]), __uint_as_float(v[k + 7]));
+          *reinterpret_cast<uint4*>(my_row + ((((uint32_t)j) ^ sw) << 4)) = o;
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (row0 < p.rows_limit) {
+          if (p.accumulate && p.out_fp32) tma_reduce_add_3d(p.tm_out, slab, gc, row0, batch);
+          else tma_store_3d(p.tm_out, slab, gc, row0, batch);
+        }
+        tma_store_commit();
+      }
+      ++slab_idx;
     }
   }
 };
@@ -140,28 +157,54 @@ struct ExpertWgradSchedule {
 constexpr int GG_BN = 256, GG_STAGES = 4;
 
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-grouped_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
-                   int K, GroupedParams ep, uint32_t* status) {
+grouped_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmC, int M, int N, int K, GroupedParams ep, uint32_t* status) {
+  ep.tm_out = &tmC;
   gemm_mainloop<GG_BN, GG_STAGES, GroupedEpilogue, TokenTileSchedule, GemmTraits<false, false, false, true>>(
       &tmA, &tmB, M, N, K, ep, status);
 }
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-grouped_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
-                     int K, GroupedParams ep, uint32_t* status) {
+grouped_dgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, int M, int N, int K, GroupedParams ep, uint32_t* status) {
+  ep.tm_out = &tmC;
   gemm_mainloop<GG_BN, GG_STAGES, GroupedEpilogue, TokenTileSchedule, GemmTraits<false, true, false, true>>(
       &tmA, &tmB, M, N, K, ep, status);
 }
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
-                     int K, GroupedParams ep, uint32_t* status) {
+grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, int M, int N, int K, GroupedParams ep, uint32_t* status) {
+  ep.tm_out = &tmC;
   gemm_mainloop<GG_BN, GG_STAGES, GroupedEpilogue, ExpertWgradSchedule, GemmTraits<true, true>>(&tmA, &tmB, M, N, K,
                                                                                                   ep, status);
+}
+
+// [batches, rows, cols] output, boxes of 32 rows x 128 bytes, 128-byte swizzle
+static int make_tmap_grouped_out(CUtensorMap* out, const void* ptr, uint64_t batches, uint64_t rows, uint64_t cols,
+                                 uint64_t ld, uint64_t ld_batch, int fp32) {
+  PFN_encodeTiled enc = get_encode_tiled();
+  if (!enc) { last_tmap_error() = 1 << 24; return -1; }
+  const uint64_t eb = fp32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(ptr) & 15) || ((ld * eb) & 15) || ((ld_batch * eb) & 15)) {
+    last_tmap_error() = (2 << 24) | 0x40000;
+    return -2;
+  }
+  cuuint64_t gdim[3] = {cols, rows, batches};
+  cuuint64_t gstr[2] = {ld * eb, ld_batch * eb};
+  cuuint32_t box[3] = {(cuuint32_t)(128 / eb), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = encode_with_context([&] {
+    return enc(out, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr),
+               gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
+  if (r != CUDA_SUCCESS) last_tmap_error() = (3 << 24) | 0x40000 | (int)r;
+  return r == CUDA_SUCCESS ? 0 : -3;
 }
 
 template <class Kern>
 static int set_smem(Kern k, bool& done) {
   if (!done) {
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<GG_BN, GG_STAGES>::TOTAL) !=
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI) !=
         cudaSuccess)
       return B200_ERR_LAUNCH;
     done = true;
@@ -180,22 +223,23 @@ int b200_grouped_gemm(const void* X, const void* W, void* Y, int max_rows, int N
                       int accumulate, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (max_rows <= 0 || N <= 0 || K <= 0 || (ldx & 7) || (max_rows % GEMM_BM)) return B200_ERR_ARG;
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
+  if (make_tmap_grouped_out(&tmC, Y, 1, max_rows, N, ldy, (uint64_t)max_rows * ldy, 0)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmA, X, max_rows, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   static bool s0 = false, s1 = false;
-  GroupedParams ep{Y, ldy, 0, N, max_rows, 0, accumulate, GG_BN, tile_expert, nullptr, n_tiles, num_experts, K};
+  GroupedParams ep{nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, n_tiles, num_experts};
   const int grid = num_sms;
   if (mode == 0) {
     if (make_tmap_3d(&tmB, W, num_experts, N, K, K, (uint64_t)N * K, GG_BN, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
     if (set_smem(grouped_fwd_kernel, s0)) return B200_ERR_LAUNCH;
-    grouped_fwd_kernel<<<grid, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL, stream>>>(tmA, tmB, max_rows, N, K, ep,
-                                                                                          status);
+    grouped_fwd_kernel<<<grid, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, max_rows, N,
+                                                                                                   K, ep, status);
   } else {
     // W[e] stored [K(contraction), N(out)]: MN-major B, boxes of 64 contraction rows x 64 output columns
     if (make_tmap_3d(&tmB, W, num_experts, K, N, N, (uint64_t)N * K, 64, 64, 2)) return B200_ERR_TENSORMAP;
     if (set_smem(grouped_dgrad_kernel, s1)) return B200_ERR_LAUNCH;
-    grouped_dgrad_kernel<<<grid, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL, stream>>>(tmA, tmB, max_rows, N, K,
-                                                                                            ep, status);
+    grouped_dgrad_kernel<<<grid, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, max_rows,
+                                                                                                     N, K, ep, status);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
@@ -206,15 +250,16 @@ int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, in
                        uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (max_rows <= 0 || N <= 0 || K <= 0 || (lddy & 7) || (ldx & 7)) return B200_ERR_ARG;
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
+  if (make_tmap_grouped_out(&tmC, dW, num_experts, N, K, K, (uint64_t)N * K, out_fp32)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmA, dY, max_rows, N, lddy, 64, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, X, max_rows, K, ldx, 64, 64, 2)) return B200_ERR_TENSORMAP;
   static bool s2 = false;
   if (set_smem(grouped_wgrad_kernel, s2)) return B200_ERR_LAUNCH;
-  GroupedParams ep{dW, K, (long long)N * K, K, N, out_fp32, accumulate, GG_BN, nullptr, expert_offsets, nullptr,
-                   num_experts, 0};
-  grouped_wgrad_kernel<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL, stream>>>(tmA, tmB, N, K, 0, ep,
-                                                                                            status);
+  GroupedParams ep{nullptr, accumulate && !out_fp32 ? (const __nv_bfloat16*)dW : nullptr, K, (long long)N * K, K, N, out_fp32,
+                   accumulate, GG_BN, 1, nullptr, expert_offsets, nullptr, num_experts};
+  grouped_wgrad_kernel<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, N, K,
+                                                                                                     0, ep, status);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 

@@ -891,3 +891,22 @@ def test_activation_offload_prefetches_and_keeps_gradients():
     for a, p in zip(ref, net.parameters()):
         assert torch.allclose(a, p.grad, rtol=1e-4, atol=1e-4)
     assert torch.allclose(gx, x.grad, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_grouped_wgrad_accumulates(fp32):
+    from cosmos_rl_b200.ops import moe
+    torch.manual_seed(39)
+    T, E, N, K = 200, 3, 136, 264
+    idx = torch.randint(0, 2, (T, 1), device=DEV, dtype=torch.int32)                # the last expert has no rows
+    disp = moe._Dispatch(idx, E)
+    rows = [torch.zeros(disp.max_rows, n, dtype=torch.bfloat16, device=DEV) for n in (N, K)]
+    off = disp.offsets.tolist()
+    for r in rows:
+        for e in range(E):
+            r[off[e]:off[e + 1]] = _bf16(off[e + 1] - off[e], r.shape[1])
+    out = _bf16(E, N, K).to(torch.float32 if fp32 else torch.bfloat16)
+    want = out.double() + torch.stack([rows[0][off[e]:off[e + 1]].double().t() @ rows[1][off[e]:off[e + 1]].double() for e in range(E)])
+    moe._grouped_wgrad(rows[0], rows[1], disp, out, True)
+    native.read_status(out.device)
+    assert torch.allclose(out.double(), want, rtol=1e-5 if fp32 else 2 ** -8, atol=1e-3)
