@@ -60,13 +60,16 @@ struct TileInfo {
 // and gives up (abort) when it returns false (used to wait for operand rows that another GPU is still sending).
 // B_TWO_BOXES (K-major 2-D B only): the B tile is fetched as two boxes of BN / 2 rows starting at rows t.b_mn0 and
 // t.b_mn1 (gate and up rows of a fused gate/up weight, so that one accumulator row holds both).
+// L2_PREFETCH (B not MN-major, 2-D): before the CTA waits for the previous kernel of the stream it brings the first
+// ep.prefetch_kb contraction blocks of its B tiles into L2. The schedule's init() may then read nothing but Params.
 template <bool A_MN_ = false, bool B_MN_ = false, bool A_3D_ = false, bool B_3D_ = false, int SIDE_WARPS_ = 0,
-          bool PRODUCER_HOOK_ = false, bool B_TWO_BOXES_ = false>
+          bool PRODUCER_HOOK_ = false, bool B_TWO_BOXES_ = false, bool L2_PREFETCH_ = false>
 struct GemmTraits {
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_, A_3D = A_3D_, B_3D = B_3D_;
   static constexpr int SIDE_WARPS = SIDE_WARPS_;
   static constexpr bool PRODUCER_HOOK = PRODUCER_HOOK_;
   static constexpr bool B_TWO_BOXES = B_TWO_BOXES_;
+  static constexpr bool L2_PREFETCH = L2_PREFETCH_;
 };
 
 // An epilogue that declares `static constexpr bool CUSTOM_TILE = true` reads its accumulator itself:
@@ -135,6 +138,21 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
   constexpr uint32_t TMEM_COLS = (2 * BN <= 32) ? 32 : (2 * BN <= 64) ? 64 : (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
 
   pdl_launch_dependents();
+  if constexpr (Traits::L2_PREFETCH) {
+    if (threadIdx.x == GEMM_THREADS - 32 && ep.prefetch_kb > 0) {
+      Sched ps;
+      ps.init(M, N, K, BN, ep);
+      TileInfo t;
+      int left = ep.prefetch_kb;
+      for (int it = 0; left > 0 && ps.get(it, t); ++it) {
+        if (t.m_blk != 0) continue;   // row blocks share their slice of B: one of them fetches it
+        for (int kb = 0; kb < t.num_kb && left > 0; ++kb, --left) {
+          tma_prefetch_2d(tmB, t.k0 + kb * GEMM_BK, t.b_mn0);
+          if constexpr (Traits::B_TWO_BOXES) tma_prefetch_2d(tmB, t.k0 + kb * GEMM_BK, t.b_mn1);
+        }
+      }
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);

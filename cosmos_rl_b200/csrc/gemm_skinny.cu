@@ -34,6 +34,7 @@ struct SkinnyParams {
   int M, N;                   // N = columns of the output (for SwiGLU: the intermediate size)
   int splits;
   int up_row0;                // SwiGLU: first "up" row of W
+  int prefetch_kb;            // contraction blocks a CTA brings into L2 before it waits for the previous kernel
 };
 
 template <int BN, bool SWIGLU>
@@ -166,7 +167,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   ep.tm_out = &tmO;
   if (threadIdx.x == 0) tma_prefetch_desc(&tmO);
   gemm_mainloop<BN, SkinnyCfg<BN>::STAGES, SkinnyEpilogue<BN, SWIGLU>, SkinnySchedule<BN, SWIGLU>,
-                GemmTraits<false, false, false, false, 0, false, SWIGLU>>(&tmA, &tmB, M, N, K, ep, status);
+                GemmTraits<false, false, false, false, 0, false, SWIGLU, true>>(&tmA, &tmB, M, N, K, ep, status);
 }
 
 // fp32 [splits, M, N] partials: boxes of 32 rows x 32 columns, 128-byte swizzle
@@ -238,11 +239,34 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   }
 }
 
+// Sum over the splits of four neighbouring columns. The first eight partials are loaded before any is used: with one
+// item a thread, the latency of one round trip to L2 is what these kernels cost.
+constexpr int SPLIT_BATCH = 8;
+struct SplitSum {
+  float4 t[SPLIT_BATCH];
+  __device__ __forceinline__ void load(const float* p, long long stride, int splits) {
+#pragma unroll
+    for (int s = 0; s < SPLIT_BATCH; ++s)
+      if (s < splits) t[s] = *reinterpret_cast<const float4*>(p + s * stride);
+  }
+  __device__ __forceinline__ float4 sum(const float* p, long long stride, int splits) const {
+    float4 a = t[0];
+#pragma unroll
+    for (int s = 1; s < SPLIT_BATCH; ++s)
+      if (s < splits) { a.x += t[s].x; a.y += t[s].y; a.z += t[s].z; a.w += t[s].w; }
+    for (int s = SPLIT_BATCH; s < splits; ++s) {
+      const float4 v = *reinterpret_cast<const float4*>(p + s * stride);
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    return a;
+  }
+};
+
 // One CTA per row: res_out = sum_s ws[s, r, :] (+ res_in);  y = res_out * rsqrt(mean(res_out^2) + eps) * w.
-// The row (H <= RN_MAX_H fp32 values) is kept in registers between the two passes.
-constexpr int RN_THREADS = 256;
-constexpr int RN_VPT = 8;  // float4 per thread -> H <= 256 * 8 * 4 = 8192
-__global__ void __launch_bounds__(RN_THREADS)
+// Four columns a thread, VPT times (H <= 1024 * VPT * 4); the row stays in registers between the two passes.
+constexpr int RN_MAX_THREADS = 1024;
+template <int VPT>
+__global__ void __launch_bounds__(RN_MAX_THREADS)
 splitk_reduce_residual_rmsnorm_kernel(const float* __restrict__ ws, int splits, int M, int H,
                                       const __nv_bfloat16* __restrict__ res_in, const __nv_bfloat16* __restrict__ w,
                                       float eps, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y) {
@@ -250,24 +274,24 @@ splitk_reduce_residual_rmsnorm_kernel(const float* __restrict__ ws, int splits, 
   pdl_wait();
   const int r = blockIdx.x;
   const int n4 = H / 4;
-  float4 v[RN_VPT];
+  const long long split_stride = (long long)M * H;
+  float4 v[VPT];
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < RN_VPT; ++j) {
-    const int c4 = threadIdx.x + j * RN_THREADS;
+  for (int j = 0; j < VPT; ++j) {
+    const int c4 = threadIdx.x + j * blockDim.x;
     v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c4 < n4) {
-      float4 acc = *reinterpret_cast<const float4*>(ws + (long long)r * H + c4 * 4);
-#pragma unroll 4
-      for (int s = 1; s < splits; ++s) {
-        const float4 t = *reinterpret_cast<const float4*>(ws + ((long long)s * M + r) * H + c4 * 4);
-        acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
-      }
+      const float* p = ws + (long long)r * H + c4 * 4;
+      SplitSum sum;
+      sum.load(p, split_stride, splits);
+      uint2 rr = make_uint2(0u, 0u);
+      if (res_in) rr = *reinterpret_cast<const uint2*>(res_in + (long long)r * H + c4 * 4);
+      float4 acc = sum.sum(p, split_stride, splits);
       if (res_in) {
-        const uint2 rr = *reinterpret_cast<const uint2*>(res_in + (long long)r * H + c4 * 4);
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rr.x));
-        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rr.y));
-        acc.x += a.x; acc.y += a.y; acc.z += b.x; acc.w += b.y;
+        const float2 ra = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rr.x));
+        const float2 rb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&rr.y));
+        acc.x += ra.x; acc.y += ra.y; acc.z += rb.x; acc.w += rb.y;
       }
       // the residual stream is stored in bf16; normalise what is stored
       uint2 o;
@@ -280,18 +304,18 @@ splitk_reduce_residual_rmsnorm_kernel(const float* __restrict__ ws, int splits, 
       ss += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
     }
   }
-  __shared__ float red[RN_THREADS / 32];
+  __shared__ float red[RN_MAX_THREADS / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float tot = 0.f;
+  float tot = (threadIdx.x & 31) < (blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.f;
 #pragma unroll
-  for (int i = 0; i < RN_THREADS / 32; ++i) tot += red[i];
+  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   const float rstd = rsqrtf(tot / (float)H + eps);
 #pragma unroll
-  for (int j = 0; j < RN_VPT; ++j) {
-    const int c4 = threadIdx.x + j * RN_THREADS;
+  for (int j = 0; j < VPT; ++j) {
+    const int c4 = threadIdx.x + j * blockDim.x;
     if (c4 < n4) {
       const uint2 ww = *reinterpret_cast<const uint2*>(w + c4 * 4);
       const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ww.x));
@@ -304,11 +328,12 @@ splitk_reduce_residual_rmsnorm_kernel(const float* __restrict__ ws, int splits, 
   }
 }
 
-// One CTA per token row of the fused qkv projection ([hq + 2 hkv] heads of d = 128): sums the split-K partials,
-// adds the bias, rotates q and k (rotate-half RoPE at positions[r]), writes q [B, hq * d] and puts the K row and the
-// V row of every kv head into the paged cache [pages, 2, hkv, page, d] at slot_mapping[r] (V slab transposed to
-// [d, page] when v_transposed). A negative slot skips the cache write (padded batch rows).
-__global__ void __launch_bounds__(256)
+// The fused qkv projection ([hq + 2 hkv] heads of d): sums the split-K partials, adds the bias, rotates q and k
+// (rotate-half RoPE at positions[r]), writes q [B, hq * d] and puts the K row and the V row of every kv head into the
+// paged cache [pages, 2, hkv, page, d] at slot_mapping[r] (V slab transposed to [d, page] when v_transposed). A negative
+// slot skips the cache write (padded batch rows). grid (row, part of the row); one thread = (head, four rotation pairs).
+constexpr int QR_THREADS = 128;
+__global__ void __launch_bounds__(QR_THREADS)
 splitk_reduce_qkv_rope_append_kernel(const float* __restrict__ ws, int splits, int M, int hq, int hkv, int d,
                                      const void* bias, int bias_bf16, const long long* __restrict__ positions,
                                      const int* __restrict__ slot_mapping, float log2_theta,
@@ -320,75 +345,65 @@ splitk_reduce_qkv_rope_append_kernel(const float* __restrict__ ws, int splits, i
   const int half = d >> 1;
   const int q4 = half >> 2;  // groups of four rotation pairs per head
   const int N = (hq + 2 * hkv) * d;
-  const int heads = hq + 2 * hkv;
-  const float pos = (float)positions[r];
+  const int idx = blockIdx.y * QR_THREADS + threadIdx.x;
+  if (idx >= (hq + 2 * hkv) * q4) return;
+  const int h = idx / q4, i0 = (idx % q4) * 4;
+  const int c0 = h * d + i0, c1 = c0 + half;
+  const long long split_stride = (long long)M * N;
+  const float* p0 = ws + (long long)r * N + c0;
+  const float* p1 = p0 + half;
+  SplitSum s0, s1;
+  s0.load(p0, split_stride, splits);
+  s1.load(p1, split_stride, splits);
   const int slot = slot_mapping[r];
-  const int page = slot >= 0 ? slot / page_size : 0, off = slot >= 0 ? slot % page_size : 0;
-  const long long slab = (long long)page_size * d;
-  // one thread per (head, four rotation pairs): 16-byte loads of the partial sums. When the block size is a multiple
-  // of d / 8 a thread keeps the same pair indices for every head it visits and evaluates their sines once.
-  const bool fixed_i = (blockDim.x % q4) == 0;
   float sn[4], cs[4];
-  if (fixed_i) {
-    const int i0 = (threadIdx.x % q4) * 4;
+  if (h < hq + hkv) {   // while the partial sums are on their way
+    const float pos = (float)positions[r];
 #pragma unroll
     for (int j = 0; j < 4; ++j) sincosf(pos * exp2f(-(2.0f * (float)(i0 + j) / (float)d) * log2_theta), &sn[j], &cs[j]);
   }
-  const float* row0 = ws + (long long)r * N;
-  const long long split_stride = (long long)M * N;
-#pragma unroll 2
-  for (int idx = threadIdx.x; idx < heads * q4; idx += blockDim.x) {
-    const int h = idx / q4, i0 = (idx % q4) * 4;
-    const int c0 = h * d + i0, c1 = c0 + half;
-    float4 a4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = a4;
-#pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
-      const float4 x = *reinterpret_cast<const float4*>(row0 + s * split_stride + c0);
-      const float4 y = *reinterpret_cast<const float4*>(row0 + s * split_stride + c1);
-      a4.x += x.x; a4.y += x.y; a4.z += x.z; a4.w += x.w;
-      b4.x += y.x; b4.y += y.y; b4.z += y.z; b4.w += y.w;
-    }
-    float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
-    if (bias) {
+  const float4 a4 = s0.sum(p0, split_stride, splits), b4 = s1.sum(p1, split_stride, splits);
+  float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+  if (bias) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        a[j] += bias_at(bias, bias_bf16, c0 + j);
-        b[j] += bias_at(bias, bias_bf16, c1 + j);
-      }
+    for (int j = 0; j < 4; ++j) {
+      a[j] += bias_at(bias, bias_bf16, c0 + j);
+      b[j] += bias_at(bias, bias_bf16, c1 + j);
     }
+  }
+  if (h < hq + hkv) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // the unfused path rounds the projection to bf16 before rotating; do the same
+      const float x = __bfloat162float(__float2bfloat16(a[j])), y = __bfloat162float(__float2bfloat16(b[j]));
+      a[j] = x * cs[j] - y * sn[j];
+      b[j] = y * cs[j] + x * sn[j];
+    }
+  }
+  uint2 oa, ob;
+  oa.x = pack_bf16x2(a[0], a[1]); oa.y = pack_bf16x2(a[2], a[3]);
+  ob.x = pack_bf16x2(b[0], b[1]); ob.y = pack_bf16x2(b[2], b[3]);
+  if (h < hq) {
+    *reinterpret_cast<uint2*>(q_out + (long long)r * hq * d + c0) = oa;
+    *reinterpret_cast<uint2*>(q_out + (long long)r * hq * d + c1) = ob;
+  } else if (slot >= 0) {
+    const int page = slot / page_size, off = slot % page_size;
+    const long long slab = (long long)page_size * d;
     if (h < hq + hkv) {
+      __nv_bfloat16* kd = cache + ((long long)(page * 2 + 0) * hkv + (h - hq)) * slab + (long long)off * d;
+      *reinterpret_cast<uint2*>(kd + i0) = oa;
+      *reinterpret_cast<uint2*>(kd + i0 + half) = ob;
+    } else {
+      __nv_bfloat16* vd = cache + ((long long)(page * 2 + 1) * hkv + (h - hq - hkv)) * slab;
+      if (v_transposed) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        // the unfused path rounds the projection to bf16 before rotating; do the same
-        const float x = __bfloat162float(__float2bfloat16(a[j])), y = __bfloat162float(__float2bfloat16(b[j]));
-        if (!fixed_i) sincosf(pos * exp2f(-(2.0f * (float)(i0 + j) / (float)d) * log2_theta), &sn[j], &cs[j]);
-        a[j] = x * cs[j] - y * sn[j];
-        b[j] = y * cs[j] + x * sn[j];
-      }
-    }
-    uint2 oa, ob;
-    oa.x = pack_bf16x2(a[0], a[1]); oa.y = pack_bf16x2(a[2], a[3]);
-    ob.x = pack_bf16x2(b[0], b[1]); ob.y = pack_bf16x2(b[2], b[3]);
-    if (h < hq) {
-      *reinterpret_cast<uint2*>(q_out + (long long)r * hq * d + c0) = oa;
-      *reinterpret_cast<uint2*>(q_out + (long long)r * hq * d + c1) = ob;
-    } else if (slot >= 0) {
-      if (h < hq + hkv) {
-        __nv_bfloat16* kd = cache + ((long long)(page * 2 + 0) * hkv + (h - hq)) * slab + (long long)off * d;
-        *reinterpret_cast<uint2*>(kd + i0) = oa;
-        *reinterpret_cast<uint2*>(kd + i0 + half) = ob;
-      } else {
-        __nv_bfloat16* vd = cache + ((long long)(page * 2 + 1) * hkv + (h - hq - hkv)) * slab;
-        if (v_transposed) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            vd[(long long)(i0 + j) * page_size + off] = __float2bfloat16(a[j]);
-            vd[(long long)(i0 + j + half) * page_size + off] = __float2bfloat16(b[j]);
-          }
-        } else {
-          *reinterpret_cast<uint2*>(vd + (long long)off * d + i0) = oa;
-          *reinterpret_cast<uint2*>(vd + (long long)off * d + i0 + half) = ob;
+        for (int j = 0; j < 4; ++j) {
+          vd[(long long)(i0 + j) * page_size + off] = __float2bfloat16(a[j]);
+          vd[(long long)(i0 + j + half) * page_size + off] = __float2bfloat16(b[j]);
         }
+      } else {
+        *reinterpret_cast<uint2*>(vd + (long long)off * d + i0) = oa;
+        *reinterpret_cast<uint2*>(vd + (long long)off * d + i0 + half) = ob;
       }
     }
   }
@@ -458,7 +473,7 @@ int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, 
   if (make_tmap_2d(&tmA, x, M, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, W, n_rows_w, K, ldw, swiglu ? bn / 2 : bn, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (ws ? make_tmap_ws(&tmO, ws, splits, M, N) : make_tmap_out16(&tmO, out, M, N, ldo)) return B200_ERR_TENSORMAP;
-  SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, up_row0};
+  SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, up_row0, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
   if (bn == 256) {
     if (swiglu) return launch_skinny<256, true>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
     return launch_skinny<256, false>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
@@ -479,10 +494,13 @@ int b200_splitk_reduce(const float* ws, int splits, int M, int N, const void* bi
 int b200_splitk_reduce_residual_rmsnorm(const float* ws, int splits, int M, int H, const void* res_in, const void* w,
                                         float eps, void* res_out, void* y, cudaStream_t stream) {
   using namespace b200;
-  if (M <= 0 || H <= 0 || (H & 3) || H > RN_THREADS * RN_VPT * 4 || splits < 1) return B200_ERR_ARG;
-  return launch_pdl(splitk_reduce_residual_rmsnorm_kernel, dim3(M), dim3(RN_THREADS), 0, stream, ws, splits, M, H,
-                    (const __nv_bfloat16*)res_in, (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)res_out,
-                    (__nv_bfloat16*)y) == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  if (M <= 0 || H <= 0 || (H & 3) || H > RN_MAX_THREADS * 2 * 4 || splits < 1) return B200_ERR_ARG;
+  const int n4 = H / 4, vpt = n4 <= RN_MAX_THREADS ? 1 : 2;
+  const int threads = ((n4 + vpt - 1) / vpt + 31) / 32 * 32;
+  auto kern = vpt == 1 ? splitk_reduce_residual_rmsnorm_kernel<1> : splitk_reduce_residual_rmsnorm_kernel<2>;
+  return launch_pdl(kern, dim3(M), dim3(threads), 0, stream, ws, splits, M, H, (const __nv_bfloat16*)res_in,
+                    (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)res_out, (__nv_bfloat16*)y) == cudaSuccess
+             ? 0 : B200_ERR_LAUNCH;
 }
 
 int b200_splitk_reduce_qkv_rope_append(const float* ws, int splits, int M, int hq, int hkv, int d, const void* bias,
@@ -490,7 +508,9 @@ int b200_splitk_reduce_qkv_rope_append(const float* ws, int splits, int M, int h
                                        float theta, void* q_out, void* cache, int page_size, int v_transposed,
                                        cudaStream_t stream) {
   if (M <= 0 || hq <= 0 || hkv <= 0 || d <= 0 || (d & 7) || splits < 1) return B200_ERR_ARG;
-  return b200::launch_pdl(b200::splitk_reduce_qkv_rope_append_kernel, dim3(M), dim3(192), 0, stream, ws, splits, M, hq,
+  const int items = (hq + 2 * hkv) * (d / 8);
+  return b200::launch_pdl(b200::splitk_reduce_qkv_rope_append_kernel,
+                          dim3(M, (items + b200::QR_THREADS - 1) / b200::QR_THREADS), dim3(b200::QR_THREADS), 0, stream, ws, splits, M, hq,
                           hkv, d, bias, bias_bf16, positions, slot_mapping, log2f(theta), (__nv_bfloat16*)q_out,
                           (__nv_bfloat16*)cache, page_size, v_transposed) == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }

@@ -14,9 +14,12 @@
 //   warp 0   : TMA producer (Q tile per item, K / V^T slabs per page through a 3-stage ring)
 //   warp 1   : MMA issuer (one thread), owns the TMEM allocation (S^T: 16 columns, O^T: 16 columns)
 //   warps 2-5: softmax. Thread <-> TMEM lane: a token row of S^T, a head-dim row of O^T. Column (head)
-//              maxima / sums over the 128 tokens go through warp shuffles and a small shared array; P is
-//              written to shared memory in the swizzled K-major layout the second MMA reads; O^T is
-//              rescaled in TMEM (tcgen05.ld / st) when the running maximum moves.
+//              maxima over the 128 tokens go through warp shuffles and a small shared array; P is
+//              written to shared memory in the swizzled K-major layout the second MMA reads.
+// What bounds the kernel besides HBM is the softmax chain of one tile after another, so that chain is kept short: the
+// eight column maxima are reduced together (nine shuffles, each step halving the heads a lane carries), the sums
+// stay per thread until the end of the item, one named barrier a tile, and the running maximum only moves when it
+// grows by more than 2^8, so that O^T is rarely rescaled in TMEM and the chain does not wait for the previous PV.
 // Every mbarrier wait is bounded; on a timeout the kernel records a status code, frees TMEM and returns.
 #include "sm100.cuh"
 #include "gemm_core.cuh"
@@ -35,6 +38,7 @@ constexpr int PDT_P_BYTES = 2 * PDT_N * 64 * 2;             // two 16 x 64-token
 constexpr int PDT_SMEM = PDT_STAGES * PDT_STAGE_BYTES + 2 * PDT_Q_BYTES + 2 * PDT_P_BYTES + 1024 /*barriers, reductions*/ + 1024;
 constexpr int PDT_THREADS = 192;
 constexpr float PDT_LOG2E = 1.4426950408889634f;
+constexpr float PDT_RESCALE_TAU = 8.0f;
 
 struct PdtParams {
   const int* block_table;
@@ -50,7 +54,41 @@ struct PdtParams {
   int max_shared, ns_total;
 };
 
-__device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// Reduces v[0..7] over the 32 lanes of the warp; lane l ends up with the result of head (l >> 2).
+template <class Op>
+__device__ __forceinline__ float reduce_heads(const float (&v)[8], int lane, Op op) {
+  float a[4], b[2];
+  const bool hi16 = lane & 16, hi8 = lane & 8, hi4 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float send = hi16 ? v[i] : v[i + 4], keep = hi16 ? v[i + 4] : v[i];
+    a[i] = op(keep, __shfl_xor_sync(0xffffffffu, send, 16));
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float send = hi8 ? a[i] : a[i + 2], keep = hi8 ? a[i + 2] : a[i];
+    b[i] = op(keep, __shfl_xor_sync(0xffffffffu, send, 8));
+  }
+  float r = op(hi4 ? b[1] : b[0], __shfl_xor_sync(0xffffffffu, hi4 ? b[0] : b[1], 4));
+  r = op(r, __shfl_xor_sync(0xffffffffu, r, 2));
+  return op(r, __shfl_xor_sync(0xffffffffu, r, 1));
+}
+
+// Barrier of the four softmax warps; true when `ok` is true in all of them, so that they leave their loops together.
+__device__ __forceinline__ bool softmax_bar(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 1, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}\n"
+      : "=r"(all)
+      : "r"((uint32_t)ok)
+      : "memory");
+  return all != 0;
+}
 
 __global__ void __launch_bounds__(PDT_THREADS, 1)
 paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __grid_constant__ CUtensorMap tm_q,
@@ -70,7 +108,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   uint64_t* o_ready = p_ready + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_ready + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  float* red = reinterpret_cast<float*>(tmem_slot + 2);  // [2][4 warps][8 heads]
+  float* red = reinterpret_cast<float*>(bars + 24);      // [2 buffers][4 warps][8 heads], 16-byte aligned
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.hq / p.hkv;
@@ -243,7 +281,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     uint32_t item_it = 0, tile_it = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok && !*abort_flag; item += gridDim.x) {
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       int b, h, split, t0, t1;
       item_range(item, b, h, split, t0, t1);
       const int ntiles = (t1 - t0 + PDT_PAGE - 1) / PDT_PAGE;
@@ -268,48 +306,50 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
       for (int g = 0; g < 8; ++g) { m_run[g] = -INFINITY; l_run[g] = 0.f; }
       for (int j = 0; j < ntiles; ++j, ++tile_it) {
         const uint32_t tb = tile_it & 1;
-        if (!mbar_wait(&s_ready[tb], (tile_it >> 1) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; break; }
-        tc_fence_after_sync();
-        uint32_t sr[16];
-        tmem_ld_32x32b_x16(tmem_base + tb * 16 + lane_addr, sr);
-        tmem_ld_wait();
+        if (ok && !mbar_wait(&s_ready[tb], (tile_it >> 1) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
+        ok = __all_sync(0xffffffffu, ok);
         const bool valid = (t0 + j * PDT_PAGE + row) < t1;
-        float s[8], wmax[8];
+        float s[8];
+        if (ok) {
+          tc_fence_after_sync();
+          uint32_t sr[16];
+          tmem_ld_32x32b_x16(tmem_base + tb * 16 + lane_addr, sr);
+          tmem_ld_wait();
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          s[g] = valid ? __uint_as_float(sr[g]) * p.scale_log2 : -INFINITY;
-          float v = s[g];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-          wmax[g] = v;
+          for (int g = 0; g < 8; ++g) s[g] = valid ? __uint_as_float(sr[g]) * p.scale_log2 : -INFINITY;
+          const float wmax = reduce_heads(s, lane, [](float x, float y) { return fmaxf(x, y); });
+          if ((lane & 3) == 0) red[tb * 32 + quad * 8 + (lane >> 2)] = wmax;
         }
-        if (lane == 0) {
+        ok = softmax_bar(ok);
+        if (!ok) break;
+        float corr[8], pv[8];
+        bool grow = false;      // the same in all 128 threads
 #pragma unroll
-          for (int g = 0; g < 8; ++g) red[quad * 8 + g] = wmax[g];
+        for (int h4 = 0; h4 < 2; ++h4) {
+          const float4* rd = reinterpret_cast<const float4*>(red + tb * 32 + h4 * 4);
+          const float4 w0 = rd[0], w1 = rd[2], w2 = rd[4], w3 = rd[6];
+          const float tmax[4] = {fmaxf(fmaxf(w0.x, w1.x), fmaxf(w2.x, w3.x)), fmaxf(fmaxf(w0.y, w1.y), fmaxf(w2.y, w3.y)),
+                                 fmaxf(fmaxf(w0.z, w1.z), fmaxf(w2.z, w3.z)), fmaxf(fmaxf(w0.w, w1.w), fmaxf(w2.w, w3.w))};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int g = h4 * 4 + i;
+            corr[g] = 1.f;
+            if (tmax[i] > m_run[g] + PDT_RESCALE_TAU || (m_run[g] == -INFINITY && tmax[i] != -INFINITY)) {
+              corr[g] = exp2f(m_run[g] - tmax[i]);
+              m_run[g] = tmax[i];
+              grow = true;
+            }
+            pv[g] = (valid && m_run[g] != -INFINITY) ? exp2f(s[g] - m_run[g]) : 0.f;
+            l_run[g] = l_run[g] * corr[g] + pv[g];
+          }
         }
-        softmax_bar();
-        float corr[8], pv[8], wsum[8];
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          float tmax = fmaxf(fmaxf(red[g], red[8 + g]), fmaxf(red[16 + g], red[24 + g]));
-          float nm = fmaxf(m_run[g], tmax);
-          corr[g] = (nm == -INFINITY) ? 1.f : exp2f(m_run[g] - nm);
-          pv[g] = (valid && nm != -INFINITY) ? exp2f(s[g] - nm) : 0.f;
-          m_run[g] = nm;
-          float v = pv[g];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          wsum[g] = v;
-        }
-        if (lane == 0) {
-#pragma unroll
-          for (int g = 0; g < 8; ++g) red[32 + quad * 8 + g] = wsum[g];
-        }
-        // The P tile written two tiles ago and the running output are in use until the PV product of the previous
-        // tile has finished (kvempty of its ring stage).
-        if (tile_it > 0) {
-          const uint32_t pt = tile_it - 1;
+        // The P buffer written two tiles ago must have been read by its PV product; before O^T is rescaled the product
+        // of the previous tile must have finished too (kvempty of the tile's ring stage, in order).
+        const uint32_t behind = grow && j > 0 ? 1 : 2;
+        if (tile_it >= behind) {
+          const uint32_t pt = tile_it - behind;
           if (!mbar_wait(&kvempty[pt % PDT_STAGES], (pt / PDT_STAGES) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
+          ok = __all_sync(0xffffffffu, ok);
           tc_fence_after_sync();
         }
         // P[head g][token row] -> shared memory, K-major rows of 64 tokens (128 bytes), 128-byte swizzle
@@ -325,8 +365,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
             }
           }
         }
-        // rescale the running output (a head-dim row per thread, one column per head)
-        if (j > 0) {
+        if (grow && j > 0 && ok) {   // rescale the running output (a head-dim row per thread, one column per head)
           uint32_t orr[16];
           tmem_ld_32x32b_x16(tmem_o + lane_addr, orr);
           tmem_ld_wait();
@@ -335,19 +374,25 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
           tmem_st_32x32b_x16(tmem_o + lane_addr, orr);
           tmem_st_wait();
         }
-        softmax_bar();
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          l_run[g] = l_run[g] * corr[g] + (red[32 + g] + red[40 + g] + red[48 + g] + red[56 + g]);
         fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[tb]);
-        if (!ok) break;
+        if (lane == 0) mbar_arrive(&p_ready[tb]);   // after a failed wait the next barrier ends the loop
       }
       if (!ok) break;
       // ---- item epilogue
-      if (!mbar_wait(o_ready, item_it & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; break; }
+      // the sums over the 128 tokens, through the buffer that the last tile's maxima did not use
+      {
+        float* sums = red + (tile_it & 1) * 32;   // tile_it is already one past the last tile
+        const float wsum = reduce_heads(l_run, lane, [](float x, float y) { return x + y; });
+        if ((lane & 3) == 0) sums[quad * 8 + (lane >> 2)] = wsum;
+        ok = softmax_bar(ok);
+        if (!ok) break;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) l_run[g] = (sums[g] + sums[8 + g]) + (sums[16 + g] + sums[24 + g]);
+      }
+      if (!mbar_wait(o_ready, item_it & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
+      ok = __all_sync(0xffffffffu, ok);
       tc_fence_after_sync();
       float o[8];
       {
@@ -362,6 +407,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
       for (int g = 0; g < 8; ++g) {
         if (g < G) {
           const long long head = (long long)b * p.hq + h * G + g;
+          if (!ok) continue;
           if (p.nsplit == 1 && !p.prefix_pages) {
             p.out[head * PDT_D + row] = __float2bfloat16(l_run[g] > 0.f ? o[g] / l_run[g] : 0.f);
           } else {
@@ -373,7 +419,8 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
           }
         }
       }
-      softmax_bar();  // `red` and TMEM reads are done before the next item starts overwriting
+      // `red` and TMEM reads are done before the next item starts overwriting
+      ok = softmax_bar(ok && !*abort_flag);
       ++item_it;
     }
   }

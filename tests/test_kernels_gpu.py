@@ -910,3 +910,26 @@ def test_grouped_wgrad_accumulates(fp32):
     moe._grouped_wgrad(rows[0], rows[1], disp, out, True)
     native.read_status(out.device)
     assert torch.allclose(out.double(), want, rtol=1e-5 if fp32 else 2 ** -8, atol=1e-3)
+
+
+@pytest.mark.parametrize("growth", [0.0, 60.0, -60.0])
+def test_paged_decode_running_maximum(growth):
+    """Scores that rise or fall by many powers of two from page to page; lengths around the page size."""
+    torch.manual_seed(33)
+    hq, hkv, d, P, B = 14, 2, 128, 128, 5
+    lens = torch.tensor([1, 128, 129, 640, 1000], dtype=torch.int32, device=DEV)
+    pages = 8
+    table = (torch.arange(B * pages, device=DEV, dtype=torch.int32) + 1).view(B, pages)
+    cache = torch.zeros(B * pages + 1, 2, hkv, P, d, dtype=torch.bfloat16, device=DEV)
+    ramp = torch.linspace(0, growth, pages * P, device=DEV) / math.sqrt(d)
+    for b in range(B):
+        L = int(lens[b])
+        t = torch.arange(L, device=DEV)
+        k = (0.3 * torch.randn(L, hkv, d, device=DEV) + ramp[:L, None, None]).to(torch.bfloat16)
+        F.kv_append(k, _bf16(L, hkv, d), cache, (table[b, t // P].long() * P + t % P).to(torch.int32), v_transposed=True)
+    q = torch.ones(B, hq, d, device=DEV).to(torch.bfloat16)
+    ref = R.paged_decode(q.cpu(), cache.cpu(), table.cpu(), lens.cpu(), v_transposed=True)
+    for nsplit in (1, 3):
+        out = F.paged_decode(q, cache, table, lens, nsplit=nsplit, v_transposed=True)
+        native.read_status(q.device)
+        assert (out.float().cpu() - ref.float()).abs().max() < 3e-2, nsplit
