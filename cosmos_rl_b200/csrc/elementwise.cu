@@ -42,6 +42,8 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
+// Makes the compiler unpack `u` again after this point instead of keeping the eight fp32 values alive in registers.
+__device__ __forceinline__ void keep_packed(uint4& u) { asm volatile("" : "+r"(u.x), "+r"(u.y), "+r"(u.z), "+r"(u.w)); }
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   uint4 u;
   __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&u);
@@ -51,188 +53,226 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// RMSNorm forward: one CTA per row, row cached in registers (H <= 256*8*MAXV)
+// RMSNorm. A row is spread over one CTA (VPT 16-byte vectors a thread); a CTA works on ROWS rows at a time so that the
+// loads of all of them are in flight before the first sum is needed, and one barrier pair serves all their sums.
 // ------------------------------------------------------------------------------------------------
-constexpr int NORM_THREADS = 256;
-constexpr int NORM_MAXV = 4;
+constexpr int NORM_MAX_THREADS = 512;
+constexpr int NORM_MAX_H = NORM_MAX_THREADS * 8 * 2;
+constexpr int RMSNORM_WS_ROWS = 296;   // persistent blocks of the backward pass, two per SM
 
-__global__ void __launch_bounds__(NORM_THREADS)
+// sums of ROWS values over the block, the result in every thread; `sh` holds [ROWS][16] and is reused by the next call
+// only after another barrier of the caller's loop (two buffers alternate)
+template <int ROWS>
+__device__ __forceinline__ void block_sums(float (&v)[ROWS], float (*sh)[16]) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    v[r] = warp_sum(v[r]);
+    if (l == 0) sh[r][w] = v[r];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) v[r] = warp_sum(l < nw ? sh[r][l] : 0.f);
+}
+
+template <int VPT, int ROWS>
+__global__ void __launch_bounds__(NORM_MAX_THREADS)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                   __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int H, float eps) {
-  __shared__ float sh[32];
-  const long long row = blockIdx.x;
+                   __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int T, int H, float eps) {
+  __shared__ float sh[ROWS][16];
   const int nvec = H >> 3;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-  const uint4* rr = res ? reinterpret_cast<const uint4*>(res + row * H) : nullptr;
-  uint4* ro = res_out ? reinterpret_cast<uint4*>(res_out + row * H) : nullptr;
-  float cache[NORM_MAXV][8];
-  float ss = 0.f;
+  const long long row0 = (long long)blockIdx.x * ROWS;
+  uint4 h[ROWS][VPT];
 #pragma unroll
-  for (int i = 0; i < NORM_MAXV; ++i) {
-    int v = threadIdx.x + i * NORM_THREADS;
-    if (v < nvec) {
-      float f[8];
-      unpack8(xr[v], f);
-      if (rr) {
-        float g[8];
-        unpack8(rr[v], g);
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
+      h[r][i] = make_uint4(0u, 0u, 0u, 0u);
+      if (v < nvec && row0 + r < T) h[r][i] = reinterpret_cast<const uint4*>(x + (row0 + r) * H)[v];
+    }
+  if (res) {
+    uint4 q[ROWS][VPT];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        q[r][i] = make_uint4(0u, 0u, 0u, 0u);
+        if (v < nvec && row0 + r < T) q[r][i] = reinterpret_cast<const uint4*>(res + (row0 + r) * H)[v];
+      }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        float f[8], g[8];
+        unpack8(h[r][i], f);
+        unpack8(q[r][i], g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] += g[j];
-        uint4 h = pack8(f);
-        unpack8(h, f);  // the norm sees the bf16-rounded residual stream
-        if (ro) ro[v] = h;
+        h[r][i] = pack8(f);   // the norm sees the bf16-rounded residual stream
+        if (res_out && v < nvec && row0 + r < T) reinterpret_cast<uint4*>(res_out + (row0 + r) * H)[v] = h[r][i];
       }
+  }
+  float ss[ROWS];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        cache[i][j] = f[j];
-        ss += f[j] * f[j];
-      }
+  for (int r = 0; r < ROWS; ++r) {
+    ss[r] = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      float f[8];
+      unpack8(h[r][i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss[r] += f[j] * f[j];
     }
   }
-  ss = block_sum<NORM_THREADS>(ss, sh);
-  const float rstd = rsqrtf(ss / (float)H + eps);
-  if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  uint4* yr = reinterpret_cast<uint4*>(y + row * H);
+  block_sums<ROWS>(ss, sh);
 #pragma unroll
-  for (int i = 0; i < NORM_MAXV; ++i) {
-    int v = threadIdx.x + i * NORM_THREADS;
-    if (v < nvec) {
-      float g[8], o[8];
-      unpack8(wr[v], g);
+  for (int r = 0; r < ROWS; ++r) {
+    ss[r] = rsqrtf(ss[r] / (float)H + eps);
+    if (threadIdx.x == 0 && rstd_out && row0 + r < T) rstd_out[row0 + r] = ss[r];
+  }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = cache[i][j] * rstd * g[j];
-      yr[v] = pack8(o);
+  for (int i = 0; i < VPT; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v >= nvec) continue;
+    float g[8];
+    unpack8(reinterpret_cast<const uint4*>(w)[v], g);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      float f[8], o[8];
+      unpack8(h[r][i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = f[j] * ss[r] * g[j];
+      if (row0 + r < T) reinterpret_cast<uint4*>(y + (row0 + r) * H)[v] = pack8(o);
     }
   }
 }
 
-// RMSNorm backward. CTA b handles rows b, b+grid, ...; dw partial sums stay in registers.
-__global__ void __launch_bounds__(NORM_THREADS)
+// RMSNorm backward of wide rows: dx (+ dres) and the weight gradient in one pass over dy and x. Persistent CTAs walk
+// groups of ROWS rows; a thread keeps the weight-gradient sums of its own columns in registers and writes them once, to
+// its block's row of dw_partial (null: no weight gradient).
+template <int VPT, int ROWS, int MIN_CTAS>
+__global__ void __launch_bounds__(NORM_MAX_THREADS, MIN_CTAS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                   float* __restrict__ dw_partial, int T, int H) {
-  __shared__ float sh[32];
+                   float* __restrict__ dw_partial, long long T, int H) {
+  __shared__ float sh[2][ROWS][16];
   const int nvec = H >> 3;
-  float dw[NORM_MAXV][8];
-  float wv[NORM_MAXV][8];
+  uint4 wv[VPT];
+  float dw[VPT][8];
 #pragma unroll
-  for (int i = 0; i < NORM_MAXV; ++i) {
-    int v = threadIdx.x + i * NORM_THREADS;
+  for (int i = 0; i < VPT; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    wv[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (v < nvec) wv[i] = reinterpret_cast<const uint4*>(w)[v];
 #pragma unroll
     for (int j = 0; j < 8; ++j) dw[i][j] = 0.f;
-    if (v < nvec) unpack8(reinterpret_cast<const uint4*>(w)[v], wv[i]);
   }
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
-    const uint4* dyr = reinterpret_cast<const uint4*>(dy + row * H);
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-    const float rs = rstd[row];
-    float xh[NORM_MAXV][8], dxh[NORM_MAXV][8];
-    float dot = 0.f;
+  int buf = 0;
+  for (long long row0 = (long long)blockIdx.x * ROWS; row0 < T; row0 += (long long)gridDim.x * ROWS, buf ^= 1) {
+    uint4 a[ROWS][VPT], b[ROWS][VPT];
+    float rs[ROWS], dot[ROWS];
 #pragma unroll
-    for (int i = 0; i < NORM_MAXV; ++i) {
-      int v = threadIdx.x + i * NORM_THREADS;
-      if (v < nvec) {
-        float a[8], b[8];
-        unpack8(dyr[v], a);
-        unpack8(xr[v], b);
+    for (int r = 0; r < ROWS; ++r) {
+      const bool in = row0 + r < T;
+      rs[r] = in ? rstd[row0 + r] : 0.f;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        a[r][i] = b[r][i] = make_uint4(0u, 0u, 0u, 0u);
+        if (in && v < nvec) {
+          a[r][i] = reinterpret_cast<const uint4*>(dy + (row0 + r) * H)[v];
+          b[r][i] = reinterpret_cast<const uint4*>(x + (row0 + r) * H)[v];
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      dot[r] = 0.f;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        float fa[8], fb[8], g[8];
+        unpack8(a[r][i], fa);
+        unpack8(b[r][i], fb);
+        unpack8(wv[i], g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] = b[j] * rs;
-          dxh[i][j] = a[j] * wv[i][j];
-          dw[i][j] += a[j] * xh[i][j];
-          dot += dxh[i][j] * xh[i][j];
+          const float xh = fb[j] * rs[r];
+          dw[i][j] += fa[j] * xh;
+          dot[r] += fa[j] * g[j] * xh;
         }
       }
     }
-    dot = block_sum<NORM_THREADS>(dot, sh) / (float)H;
-    uint4* dxr = reinterpret_cast<uint4*>(dx + row * H);
-    const uint4* drr = dres ? reinterpret_cast<const uint4*>(dres + row * H) : nullptr;
+    uint4 d[ROWS][VPT];   // in flight across the barrier
 #pragma unroll
-    for (int i = 0; i < NORM_MAXV; ++i) {
-      int v = threadIdx.x + i * NORM_THREADS;
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        d[r][i] = make_uint4(0u, 0u, 0u, 0u);
+        if (dres && row0 + r < T && v < nvec) d[r][i] = reinterpret_cast<const uint4*>(dres + (row0 + r) * H)[v];
+      }
+    block_sums<ROWS>(dot, sh[buf]);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      dot[r] /= (float)H;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        float fa[8], fb[8], g[8], o[8];
+        keep_packed(a[r][i]);
+        keep_packed(b[r][i]);
+        keep_packed(wv[i]);
+        unpack8(a[r][i], fa);
+        unpack8(b[r][i], fb);
+        unpack8(wv[i], g);
+        unpack8(d[r][i], o);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += rs[r] * (fa[j] * g[j] - fb[j] * rs[r] * dot[r]);
+        if (row0 + r < T && v < nvec) reinterpret_cast<uint4*>(dx + (row0 + r) * H)[v] = pack8(o);
+      }
+    }
+  }
+  if (dw_partial) {
+    float4* out = reinterpret_cast<float4*>(dw_partial + (long long)blockIdx.x * H);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
       if (v < nvec) {
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (dxh[i][j] - xh[i][j] * dot);
-        if (drr) {
-          float r[8];
-          unpack8(drr[v], r);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += r[j];
-        }
-        dxr[v] = pack8(o);
+        out[2 * v] = make_float4(dw[i][0], dw[i][1], dw[i][2], dw[i][3]);
+        out[2 * v + 1] = make_float4(dw[i][4], dw[i][5], dw[i][6], dw[i][7]);
       }
-    }
-  }
-  float* out = dw_partial + (long long)blockIdx.x * H;
-#pragma unroll
-  for (int i = 0; i < NORM_MAXV; ++i) {
-    int v = threadIdx.x + i * NORM_THREADS;
-    if (v < nvec) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) out[v * 8 + j] = dw[i][j];
     }
   }
 }
 
-// ---- RMSNorm backward, split in two bandwidth-shaped kernels ---------------------------------------------
-// dx: fully parallel over rows (one CTA per row for wide rows, one warp per row for narrow rows such as the
-// per-head q/k norms), no weight-gradient state in registers. dw: column strips, each warp streams a strip of
-// rows for 256 columns and the strips meet in one fp32 atomicAdd per column.
-__global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_dx_row_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                      const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, int H) {
-  __shared__ float sh[32];
-  const long long row = blockIdx.x;
-  const int nvec = H >> 3;
-  const uint4* dyr = reinterpret_cast<const uint4*>(dy + row * H);
-  const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  const float rs = rstd[row];
-  float xh[NORM_MAXV][8], dxh[NORM_MAXV][8];
-  float dot = 0.f;
-#pragma unroll
-  for (int i = 0; i < NORM_MAXV; ++i) {
-    int v = threadIdx.x + i * NORM_THREADS;
-    if (v < nvec) {
-      float a[8], b[8], g[8];
-      unpack8(dyr[v], a);
-      unpack8(xr[v], b);
-      unpack8(wr[v], g);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        xh[i][j] = b[j] * rs;
-        dxh[i][j] = a[j] * g[j];
-        dot += dxh[i][j] * xh[i][j];
-      }
-    }
+// dw[c] = sum of the rows of partial [rows, H], as bf16: a warp takes every eighth row of 32 columns
+__global__ void __launch_bounds__(256)
+rmsnorm_dw_sum_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, int rows, int H) {
+  __shared__ float sh[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (c < H) {
+#pragma unroll 8
+    for (int r = warp; r < rows; r += 8) s += partial[(long long)r * H + c];
   }
-  dot = block_sum<NORM_THREADS>(dot, sh) / (float)H;
-  uint4* dxr = reinterpret_cast<uint4*>(dx + row * H);
-  const uint4* drr = dres ? reinterpret_cast<const uint4*>(dres + row * H) : nullptr;
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && c < H) {
 #pragma unroll
-  for (int i = 0; i < NORM_MAXV; ++i) {
-    int v = threadIdx.x + i * NORM_THREADS;
-    if (v < nvec) {
-      float o[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = rs * (dxh[i][j] - xh[i][j] * dot);
-      if (drr) {
-        float r[8];
-        unpack8(drr[v], r);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += r[j];
-      }
-      dxr[v] = pack8(o);
-    }
+    for (int w = 1; w < 8; ++w) s += sh[w][lane];
+    dw[c] = __float2bfloat16(s);
   }
 }
 
-// narrow rows (H <= 1024, H % 8 == 0): one warp per row, up to 4 vectors per lane
+// ---- RMSNorm backward of narrow rows (H <= 1024, the per-head q/k norms): two bandwidth-shaped kernels -----
+// dx: one warp per row. dw: column strips, each block streams a strip of rows for 256 columns into the strip's row of
+// dw_partial.
+// H % 8 == 0, up to 4 vectors per lane
 __global__ void __launch_bounds__(256)
 rmsnorm_dx_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
@@ -283,10 +323,10 @@ rmsnorm_dx_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
   }
 }
 
-// dw[c] += sum_t dy[t,c] * x[t,c] * rstd[t]; grid (ceil(H/256), row strips), 8 warps per CTA split the strip
+// dw_partial[strip, c] = sum_t dy[t,c] * x[t,c] * rstd[t] over the strip; grid (ceil(H/256), row strips), 8 warps per CTA split the strip
 __global__ void __launch_bounds__(256)
 rmsnorm_dw_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                  const float* __restrict__ rstd, float* __restrict__ dw, long long T, int H) {
+                  const float* __restrict__ rstd, float* __restrict__ dw_partial, long long T, int H) {
   __shared__ float sh[8][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = blockIdx.x * 256 + lane * 8;
@@ -311,7 +351,7 @@ rmsnorm_dw_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __r
     float s = 0.f;
 #pragma unroll
     for (int wv = 0; wv < 8; ++wv) s += sh[wv][threadIdx.x];
-    atomicAdd(&dw[c], s);
+    dw_partial[(long long)blockIdx.y * H + c] = s;
   }
 }
 
@@ -533,6 +573,16 @@ __global__ void clip_coef_kernel(const float* sumsq, float max_norm, float* coef
   *coef = c < 1.f ? c : 1.f;
 }
 
+// threads of a CTA and vectors per thread for a row of H elements
+struct NormShape {
+  int vpt, threads;
+  explicit NormShape(int H) {
+    const int nvec = H >> 3;
+    vpt = nvec <= NORM_MAX_THREADS ? 1 : 2;
+    threads = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
+  }
+};
+
 inline int ok() { return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH; }
 
 }  // namespace
@@ -542,45 +592,51 @@ extern "C" {
 int b200_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* residual_out, float* rstd,
                      int T, int H, float eps, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if ((H & 7) || H > NORM_THREADS * 8 * NORM_MAXV) return B200_ERR_ARG;
-  rmsnorm_fwd_kernel<<<T, NORM_THREADS, 0, stream>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
-      (__nv_bfloat16*)residual_out, rstd, H, eps);
+  if ((H & 7) || H > NORM_MAX_H) return B200_ERR_ARG;
+  const NormShape n(H);
+  // two rows a CTA once every SM has several CTAs of work anyway
+  const int rows = T >= 148 * 8 ? 2 : 1;
+  const unsigned grid = (unsigned)((T + rows - 1) / rows);
+  auto go = [&](auto kern) {
+    kern<<<grid, n.threads, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w,
+                                         (__nv_bfloat16*)y, (__nv_bfloat16*)residual_out, rstd, T, H, eps);
+  };
+  if (n.vpt == 1) rows == 2 ? go(rmsnorm_fwd_kernel<1, 2>) : go(rmsnorm_fwd_kernel<1, 1>);
+  else rows == 2 ? go(rmsnorm_fwd_kernel<2, 2>) : go(rmsnorm_fwd_kernel<2, 1>);
   return ok();
 }
 
-int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                     float* dw_partial, int n_partial, int T, int H, cudaStream_t stream) {
-  if (T <= 0) return 0;
-  if ((H & 7) || H > NORM_THREADS * 8 * NORM_MAXV || n_partial <= 0) return B200_ERR_ARG;
-  rmsnorm_bwd_kernel<<<n_partial, NORM_THREADS, 0, stream>>>(
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
-      (__nv_bfloat16*)dx, dw_partial, T, H);
-  return ok();
-}
-
-// dx (+ dres) and dw (fp32, ACCUMULATED into dw_accum, which the caller zeroes or reuses across micro-batches)
+// dx (+ dres) and dw (bf16; null: no weight gradient). ws: fp32 scratch of RMSNORM_WS_ROWS * max(H, 1024) elements.
 int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                      float* dw_accum, long long T, int H, cudaStream_t stream) {
-  if (T <= 0) return 0;
-  if ((H & 7) || H > NORM_THREADS * 8 * NORM_MAXV) return B200_ERR_ARG;
-  if (H <= 1024)
+                      void* dw, float* ws, long long T, int H, cudaStream_t stream) {
+  if (T <= 0) return dw ? (cudaMemsetAsync(dw, 0, (size_t)H * 2, stream) == cudaSuccess ? 0 : B200_ERR_RUNTIME) : 0;
+  if ((H & 7) || H > NORM_MAX_H || (dw && !ws)) return B200_ERR_ARG;
+  if (!dw) ws = nullptr;
+  int rows = 0;   // of partial weight gradients
+  if (H <= 1024) {
     rmsnorm_dx_warp_kernel<<<(unsigned)((T + 7) / 8), 256, 0, stream>>>(
         (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
         (__nv_bfloat16*)dx, T, H);
-  else
-    rmsnorm_dx_row_kernel<<<(unsigned)T, NORM_THREADS, 0, stream>>>(
-        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
-        (__nv_bfloat16*)dx, H);
-  if (dw_accum) {
-    const int col_blocks = (H + 255) / 256;
-    long long strips = (148 * 8 + col_blocks - 1) / col_blocks;
-    if (strips > (T + 63) / 64) strips = (T + 63) / 64;
-    if (strips < 1) strips = 1;
-    dim3 grid(col_blocks, (unsigned)strips);
-    rmsnorm_dw_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd, dw_accum, T,
-                                                H);
+    if (dw) {
+      const int col_blocks = (H + 255) / 256;
+      long long strips = RMSNORM_WS_ROWS * 4 / col_blocks;   // col_blocks * 256 <= 1024 columns of the scratch
+      if (strips > (T + 63) / 64) strips = (T + 63) / 64;
+      rows = (int)strips;
+      rmsnorm_dw_kernel<<<dim3(col_blocks, rows), 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
+                                                                    rstd, ws, T, H);
+    }
+  } else {
+    const NormShape n(H);
+    auto go = [&](auto kern, int group, int ctas) {
+      const long long groups = (T + group - 1) / group;
+      rows = (int)(groups < ctas ? groups : ctas);
+      kern<<<rows, n.threads, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+                                           rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, ws, T, H);
+    };
+    if (n.vpt == 1) go(rmsnorm_bwd_kernel<1, 2, 2>, 2, RMSNORM_WS_ROWS);
+    else go(rmsnorm_bwd_kernel<2, 2, 1>, 2, RMSNORM_WS_ROWS / 2);
   }
+  if (dw) rmsnorm_dw_sum_kernel<<<(H + 31) / 32, 256, 0, stream>>>(ws, (__nv_bfloat16*)dw, rows, H);
   return ok();
 }
 

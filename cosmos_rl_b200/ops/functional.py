@@ -15,7 +15,7 @@ import torch
 
 from . import native, reference
 
-_N_PARTIAL_NORM = 296  # CTAs (2 per SM) that accumulate RMSNorm weight-gradient partials
+_NORM_WS_ROWS = 296  # rows of partial weight gradients that the RMSNorm backward needs room for
 
 
 def _c(t: torch.Tensor) -> torch.Tensor:
@@ -56,12 +56,15 @@ class _RMSNorm(torch.autograd.Function):
         dy2 = _c(dy).view(-1, H)
         dres2 = _c(dres_out).view(-1, H) if dres_out is not None else None
         dx = torch.empty_like(h)
-        dw = torch.zeros(H, dtype=torch.float32, device=h.device)
+        dw = ws = None
+        if ctx.needs_input_grad[1]:
+            dw = torch.empty(H, dtype=torch.bfloat16, device=h.device)
+            ws = torch.empty(_NORM_WS_ROWS * max(H, 1024), dtype=torch.float32, device=h.device)
         native.check(native.lib().b200_rmsnorm_bwd2(native.ptr(dy2), native.ptr(h), native.ptr(weight),
                                                     native.ptr(rstd), native.ptr(dres2), native.ptr(dx),
-                                                    native.ptr(dw), T, H, native.stream()), "rmsnorm_bwd")
+                                                    native.ptr(dw), native.ptr(ws), T, H, native.stream()), "rmsnorm_bwd")
         dxv = dx.view(ctx.shape)
-        return dxv, dw.to(weight.dtype), None, (dxv if ctx.has_res else None)
+        return dxv, dw, None, (dxv if ctx.has_res else None)
 
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: Optional[torch.Tensor] = None):

@@ -933,3 +933,23 @@ def test_paged_decode_running_maximum(growth):
         out = F.paged_decode(q, cache, table, lens, nsplit=nsplit, v_transposed=True)
         native.read_status(q.device)
         assert (out.float().cpu() - ref.float()).abs().max() < 3e-2, nsplit
+
+
+@pytest.mark.parametrize("T,H", [(1, 1032), (2, 2048), (3, 4096), (1185, 4104), (1184, 5120), (7, 128)])
+def test_rmsnorm_row_groups(T, H):
+    """One row, an odd number of rows, one and two vectors a thread, and more row groups than persistent blocks."""
+    torch.manual_seed(34)
+    x, w, res, gy, gr = _bf16(T, H), _bf16(H), _bf16(T, H), _bf16(T, H), _bf16(T, H)
+    a = [t.clone().requires_grad_(True) for t in (x, w, res)]
+    y, ro = F.rms_norm(a[0], a[1], 1e-6, a[2])
+    got = torch.autograd.grad([y, ro], a, [gy, gr])
+    assert torch.equal(ro, (x.float() + res.float()).to(torch.bfloat16))
+    h = ro.double().requires_grad_(True)
+    wd = w.double().requires_grad_(True)
+    yr = h * torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-6) * wd
+    dh, dw = torch.autograd.grad(yr, [h, wd], gy.double())
+    # one bf16 rounding of the result is 2^-9 of it; the weight gradient sums T terms in fp32
+    assert torch.allclose(y.double(), yr, rtol=2 ** -8, atol=1e-6)
+    assert torch.allclose(got[0].double(), dh + gr.double(), rtol=2 ** -8, atol=1e-4)
+    assert torch.equal(got[0], got[2])
+    assert torch.allclose(got[1].double(), dw, rtol=2 ** -8, atol=1e-5 * T + 1e-5)
