@@ -85,6 +85,8 @@ int b200_moe_offsets(const int* counts, int E, int* offsets, int* tile_expert, i
                      int max_tiles, cudaStream_t stream);
 int b200_moe_permute(const void* x, const int* idx, const int* offsets, int* cursor, int* row_map, void* xp, int T,
                      int k, int H, cudaStream_t stream);
+// clears the rows of xp between each expert's last token and the end of its last 128-row tile
+int b200_moe_zero_padding(const int* counts, const int* offsets, void* xp, int E, int H, cudaStream_t stream);
 int b200_moe_scatter_scaled(const void* src, const float* probs, const int* row_map, void* dst, int T, int k, int H,
                             cudaStream_t stream);
 int b200_moe_combine(const void* y, const float* probs, const int* row_map, void* out, int T, int k, int H,
@@ -108,8 +110,10 @@ int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float*
 int b200_colsum_f32(const float* partial, float* out, int rows, int cols, int accumulate, cudaStream_t stream);
 int b200_rope_inplace(void* q, void* k, const long long* positions, int T, int hq, int hkv, int d, long long q_stride,
                       long long k_stride, float theta, int backward, cudaStream_t stream);
-int b200_swiglu_fwd(const void* gate_up, void* out, long long T, int I, cudaStream_t stream);
-int b200_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long T, int I, cudaStream_t stream);
+// row_tiles (device, nullable): only the first row_tiles[0] * 128 of the T rows are in use.
+int b200_swiglu_fwd(const void* gate_up, void* out, long long T, int I, const int* row_tiles, cudaStream_t stream);
+int b200_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long T, int I, const int* row_tiles,
+                    cudaStream_t stream);
 
 // ---- optimizer -----------------------------------------------------------------------------------------
 // Flat fused AdamW on fp32 master weights with bf16 (or fp32) grads; writes the bf16 compute copy.

@@ -441,43 +441,78 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __
 // ------------------------------------------------------------------------------------------------
 // SwiGLU on a fused [T, 2I] gate|up projection
 // ------------------------------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T,
-                                  int I) {
-  const int nvec = I >> 3;
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= T * nvec) return;
-  const long long t = idx / nvec;
-  const int v = (int)(idx % nvec);
-  const uint4* g = reinterpret_cast<const uint4*>(gu + t * 2 * I);
-  const uint4* u = reinterpret_cast<const uint4*>(gu + t * 2 * I + I);
-  float a[8], b[8], o[8];
-  unpack8(g[v], a);
-  unpack8(u[v], b);
+// A thread works on SWIGLU_ITEMS vectors of 8 columns whose loads are all in flight before the first is used; the
+// position is found with 32-bit divisions unless the tensor is too large for them. row_tiles (nullable, device): only
+// the first row_tiles[0] * 128 rows are in use.
+constexpr int SWIGLU_ITEMS = 2;
+template <class Index>
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I,
+                  const int* __restrict__ row_tiles) {
+  const Index nvec = I >> 3;
+  const Index total = (Index)(row_tiles ? min((long long)row_tiles[0] * 128, T) : T) * nvec;
+  const Index first = (Index)blockIdx.x * (256 * SWIGLU_ITEMS) + threadIdx.x;
+  uint4 g[SWIGLU_ITEMS], u[SWIGLU_ITEMS];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) o[j] = a[j] / (1.f + __expf(-a[j])) * b[j];
-  reinterpret_cast<uint4*>(out + t * I)[v] = pack8(o);
+  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
+    const Index idx = first + k * 256;
+    if (idx >= total) continue;
+    const Index t = idx / nvec, v = idx - t * nvec;
+    const uint4* row = reinterpret_cast<const uint4*>(gu + (long long)t * 2 * I);
+    g[k] = row[v];
+    u[k] = row[nvec + v];
+  }
+#pragma unroll
+  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
+    const Index idx = first + k * 256;
+    if (idx >= total) continue;
+    float a[8], b[8], o[8];
+    unpack8(g[k], a);
+    unpack8(u[k], b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = a[j] / (1.f + __expf(-a[j])) * b[j];
+    reinterpret_cast<uint4*>(out)[idx] = pack8(o);
+  }
 }
 
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ dgu, long long T, int I) {
-  const int nvec = I >> 3;
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= T * nvec) return;
-  const long long t = idx / nvec;
-  const int v = (int)(idx % nvec);
-  float a[8], b[8], d[8], dg[8], du[8];
-  unpack8(reinterpret_cast<const uint4*>(gu + t * 2 * I)[v], a);
-  unpack8(reinterpret_cast<const uint4*>(gu + t * 2 * I + I)[v], b);
-  unpack8(reinterpret_cast<const uint4*>(dout + t * I)[v], d);
+template <class Index>
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ gu,
+                  __nv_bfloat16* __restrict__ dgu, long long T, int I, const int* __restrict__ row_tiles) {
+  const Index nvec = I >> 3;
+  const Index total = (Index)(row_tiles ? min((long long)row_tiles[0] * 128, T) : T) * nvec;
+  const Index first = (Index)blockIdx.x * (256 * SWIGLU_ITEMS) + threadIdx.x;
+  uint4 g[SWIGLU_ITEMS], u[SWIGLU_ITEMS], dd[SWIGLU_ITEMS];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float s = 1.f / (1.f + __expf(-a[j]));
-    float silu = a[j] * s;
-    dg[j] = d[j] * b[j] * (s + silu * (1.f - s));
-    du[j] = d[j] * silu;
+  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
+    const Index idx = first + k * 256;
+    if (idx >= total) continue;
+    const Index t = idx / nvec, v = idx - t * nvec;
+    const uint4* row = reinterpret_cast<const uint4*>(gu + (long long)t * 2 * I);
+    g[k] = row[v];
+    u[k] = row[nvec + v];
+    dd[k] = reinterpret_cast<const uint4*>(dout)[idx];
   }
-  reinterpret_cast<uint4*>(dgu + t * 2 * I)[v] = pack8(dg);
-  reinterpret_cast<uint4*>(dgu + t * 2 * I + I)[v] = pack8(du);
+#pragma unroll
+  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
+    const Index idx = first + k * 256;
+    if (idx >= total) continue;
+    const Index t = idx / nvec, v = idx - t * nvec;
+    float a[8], b[8], d[8], dg[8], du[8];
+    unpack8(g[k], a);
+    unpack8(u[k], b);
+    unpack8(dd[k], d);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float s = 1.f / (1.f + __expf(-a[j]));
+      float silu = a[j] * s;
+      dg[j] = d[j] * b[j] * (s + silu * (1.f - s));
+      du[j] = d[j] * silu;
+    }
+    uint4* row = reinterpret_cast<uint4*>(dgu + (long long)t * 2 * I);
+    row[v] = pack8(dg);
+    row[nvec + v] = pack8(du);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -664,21 +699,24 @@ int b200_rope_inplace(void* q, void* k, const long long* positions, int T, int h
   return ok();
 }
 
-int b200_swiglu_fwd(const void* gate_up, void* out, long long T, int I, cudaStream_t stream) {
+int b200_swiglu_fwd(const void* gate_up, void* out, long long T, int I, const int* row_tiles, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (I & 7) return B200_ERR_ARG;
-  long long n = T * (I / 8);
-  swiglu_fwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)gate_up,
-                                                                    (__nv_bfloat16*)out, T, I);
+  const long long n = T * (I / 8), per = 256 * SWIGLU_ITEMS;
+  auto kern = n < (1ll << 32) - 2 * per ? swiglu_fwd_kernel<uint32_t> : swiglu_fwd_kernel<unsigned long long>;
+  kern<<<(unsigned)((n + per - 1) / per), 256, 0, stream>>>((const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, T, I,
+                                                            row_tiles);
   return ok();
 }
 
-int b200_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long T, int I, cudaStream_t stream) {
+int b200_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long T, int I, const int* row_tiles,
+                    cudaStream_t stream) {
   if (T <= 0) return 0;
   if (I & 7) return B200_ERR_ARG;
-  long long n = T * (I / 8);
-  swiglu_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
-      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)dgate_up, T, I);
+  const long long n = T * (I / 8), per = 256 * SWIGLU_ITEMS;
+  auto kern = n < (1ll << 32) - 2 * per ? swiglu_bwd_kernel<uint32_t> : swiglu_bwd_kernel<unsigned long long>;
+  kern<<<(unsigned)((n + per - 1) / per), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate_up,
+                                                            (__nv_bfloat16*)dgate_up, T, I, row_tiles);
   return ok();
 }
 

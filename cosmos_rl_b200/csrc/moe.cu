@@ -71,94 +71,170 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int T, int E
 }
 
 // ---- offsets: one block; padded exclusive scan + tile -> expert table --------------------------------
-__global__ void offsets_kernel(const int* __restrict__ counts, int E, int* __restrict__ offsets,
-                               int* __restrict__ tile_expert, int* __restrict__ n_tiles, int* __restrict__ cursor,
-                               int max_tiles) {
-  if (threadIdx.x != 0) return;
-  int off = 0;
-  for (int e = 0; e < E; ++e) {
-    offsets[e] = off;
-    cursor[e] = 0;
-    const int padded = (counts[e] + MOE_ALIGN - 1) / MOE_ALIGN * MOE_ALIGN;
-    for (int t = off / MOE_ALIGN; t < (off + padded) / MOE_ALIGN && t < max_tiles; ++t) tile_expert[t] = e;
-    off += padded;
+constexpr int OFF_THREADS = 256;
+__global__ void __launch_bounds__(OFF_THREADS)
+offsets_kernel(const int* __restrict__ counts, int E, int* __restrict__ offsets, int* __restrict__ tile_expert,
+               int* __restrict__ n_tiles, int* __restrict__ cursor, int max_tiles) {
+  __shared__ int warp_tot[OFF_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;   // tiles of the experts before this round of the loop
+  for (int e0 = 0; e0 < E; e0 += OFF_THREADS) {
+    const int e = e0 + threadIdx.x;
+    const int tiles = e < E ? (counts[e] + MOE_ALIGN - 1) / MOE_ALIGN : 0;
+    int incl = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    int before = base;
+    for (int w = 0; w < warp; ++w) before += warp_tot[w];
+    for (int w = 0; w < OFF_THREADS / 32; ++w) base += warp_tot[w];
+    __syncthreads();
+    if (e < E) {
+      const int first = before + incl - tiles;
+      offsets[e] = first * MOE_ALIGN;
+      cursor[e] = 0;
+      for (int t = first; t < first + tiles && t < max_tiles; ++t) tile_expert[t] = e;
+    }
   }
-  offsets[E] = off;
-  n_tiles[0] = min(off / MOE_ALIGN, max_tiles);
+  if (threadIdx.x == 0) {
+    offsets[E] = base * MOE_ALIGN;
+    n_tiles[0] = min(base, max_tiles);
+  }
 }
 
-// ---- permute: claim a slot per (token, choice), copy the row -------------------------------------------
-__global__ void permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx,
-                               const int* __restrict__ offsets, int* __restrict__ cursor, int* __restrict__ row_map,
-                               __nv_bfloat16* __restrict__ xp, int T, int k, int H) {
-  const int pair = blockIdx.x;  // one block per (token, choice)
-  if (pair >= T * k) return;
-  __shared__ int pos_sh;
-  if (threadIdx.x == 0) {
-    const int e = idx[pair];
-    pos_sh = offsets[e] + atomicAdd(&cursor[e], 1);
-    row_map[pair] = pos_sh;
+// ---- rows of the expert-sorted buffer. One block per token; a thread moves 16 bytes of the token's row at a time and
+// touches all k choices with it, so the token's own row is read once and the k rows are in flight together. ---------
+constexpr int ROW_MAX_THREADS = 256;
+
+// permute: claim a slot per (token, choice), copy the row
+__global__ void __launch_bounds__(ROW_MAX_THREADS)
+permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx, const int* __restrict__ offsets,
+               int* __restrict__ cursor, int* __restrict__ row_map, __nv_bfloat16* __restrict__ xp, int k, int H) {
+  extern __shared__ int pos_sh[];
+  const long long t = blockIdx.x;
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    const int e = idx[t * k + j];
+    pos_sh[j] = row_map[t * k + j] = offsets[e] + atomicAdd(&cursor[e], 1);
   }
   __syncthreads();
-  const uint4* src = reinterpret_cast<const uint4*>(x + (long long)(pair / k) * H);
-  uint4* dst = reinterpret_cast<uint4*>(xp + (long long)pos_sh * H);
-  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) dst[i] = src[i];
+  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+    const uint4 v = reinterpret_cast<const uint4*>(x + t * H)[i];
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) reinterpret_cast<uint4*>(xp + (long long)pos_sh[j] * H)[i] = v;
+  }
 }
 
-// gather rows through an existing row_map (backward of combine: dy[pos] = prob * dout[t])
-__global__ void scatter_scaled_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ probs,
-                                      const int* __restrict__ row_map, __nv_bfloat16* __restrict__ dst, int T, int k,
-                                      int H) {
-  const int pair = blockIdx.x;
-  if (pair >= T * k) return;
-  const float p = probs ? probs[pair] : 1.f;
-  const __nv_bfloat162* s = reinterpret_cast<const __nv_bfloat162*>(src + (long long)(pair / k) * H);
-  __nv_bfloat162* d = reinterpret_cast<__nv_bfloat162*>(dst + (long long)row_map[pair] * H);
-  for (int i = threadIdx.x; i < H / 2; i += blockDim.x) {
-    float2 f = __bfloat1622float2(s[i]);
-    d[i] = __floats2bfloat162_rn(f.x * p, f.y * p);
+// the rows between an expert's last token and the end of its last tile: the GEMMs contract over them
+__global__ void __launch_bounds__(ROW_MAX_THREADS)
+zero_padding_kernel(const int* __restrict__ counts, const int* __restrict__ offsets, __nv_bfloat16* __restrict__ xp,
+                    int H) {
+  const int e = blockIdx.x;
+  for (int r = offsets[e] + counts[e] + blockIdx.y; r < offsets[e + 1]; r += gridDim.y)
+    for (int i = threadIdx.x; i < H / 8; i += blockDim.x)
+      reinterpret_cast<uint4*>(xp + (long long)r * H)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(p[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 u;
+  __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  return u;
+}
+
+// spread rows through an existing row_map (backward of combine: dy[pos] = prob * dout[t])
+__global__ void __launch_bounds__(ROW_MAX_THREADS)
+scatter_scaled_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ probs,
+                      const int* __restrict__ row_map, __nv_bfloat16* __restrict__ dst, int k, int H) {
+  const long long t = blockIdx.x;
+  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+    float f[8];
+    unpack8(reinterpret_cast<const uint4*>(src + t * H)[i], f);
+#pragma unroll 4
+    for (int j = 0; j < k; ++j) {
+      const float p = probs ? probs[t * k + j] : 1.f;
+      float o[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) o[c] = f[c] * p;
+      reinterpret_cast<uint4*>(dst + (long long)row_map[t * k + j] * H)[i] = pack8(o);
+    }
   }
 }
 
 // ---- combine: out[t] = sum_j prob[t,j] * y[row_map[t,j]]  (probs null: plain sum) ------------------------
-__global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ probs,
-                               const int* __restrict__ row_map, __nv_bfloat16* __restrict__ out, int T, int k, int H) {
-  const int t = blockIdx.x;
-  if (t >= T) return;
-  for (int i = threadIdx.x; i < H / 2; i += blockDim.x) {
-    float ax = 0.f, ay = 0.f;
+__global__ void __launch_bounds__(ROW_MAX_THREADS)
+combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ probs, const int* __restrict__ row_map,
+               __nv_bfloat16* __restrict__ out, int k, int H) {
+  const long long t = blockIdx.x;
+  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
     for (int j = 0; j < k; ++j) {
       const float p = probs ? probs[t * k + j] : 1.f;
-      float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(y + (long long)row_map[t * k + j] * H)[i]);
-      ax += p * f.x;
-      ay += p * f.y;
+      float f[8];
+      unpack8(reinterpret_cast<const uint4*>(y + (long long)row_map[t * k + j] * H)[i], f);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) a[c] += p * f[c];
     }
-    reinterpret_cast<__nv_bfloat162*>(out + (long long)t * H)[i] = __floats2bfloat162_rn(ax, ay);
+    reinterpret_cast<uint4*>(out + t * H)[i] = pack8(a);
   }
 }
 
-// dprob[t,j] = <dout[t], y[row_map[t,j]]>
-__global__ void combine_dprob_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
-                                     const int* __restrict__ row_map, float* __restrict__ dprob, int T, int k, int H) {
-  const int pair = blockIdx.x;
-  if (pair >= T * k) return;
-  __shared__ float sh[32];
-  const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(dout + (long long)(pair / k) * H);
-  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(y + (long long)row_map[pair] * H);
-  float s = 0.f;
-  for (int i = threadIdx.x; i < H / 2; i += blockDim.x) {
-    float2 f = __bfloat1622float2(a[i]), g = __bfloat1622float2(b[i]);
-    s += f.x * g.x + f.y * g.y;
-  }
+// dprob[t,j] = <dout[t], y[row_map[t,j]]>, eight choices at a time
+__global__ void __launch_bounds__(ROW_MAX_THREADS)
+combine_dprob_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
+                     const int* __restrict__ row_map, float* __restrict__ dprob, int k, int H) {
+  __shared__ float sh[ROW_MAX_THREADS / 32][8];
+  const long long t = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int j0 = 0; j0 < k; j0 += 8) {
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
+      float f[8];
+      unpack8(reinterpret_cast<const uint4*>(dout + t * H)[i], f);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (blockDim.x + 31) / 32; ++w) t += sh[w];
-    dprob[pair] = t;
+      for (int j = 0; j < 8; ++j) {
+        if (j0 + j < k) {
+          float g[8];
+          unpack8(reinterpret_cast<const uint4*>(y + (long long)row_map[t * k + j0 + j] * H)[i], g);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) s[j] += f[c] * g[c];
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+      if (lane == 0) sh[warp][j] = s[j];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 && j0 + (int)threadIdx.x < k) {
+      float r = 0.f;
+      for (int w = 0; w < (int)blockDim.x / 32; ++w) r += sh[w][threadIdx.x];
+      dprob[t * k + j0 + threadIdx.x] = r;
+    }
+    __syncthreads();
   }
+}
+
+// threads of a block that moves rows of H elements
+inline int row_threads(int H) {
+  const int t = (H / 8 + 31) / 32 * 32;
+  return t < ROW_MAX_THREADS ? t : ROW_MAX_THREADS;
 }
 
 inline int ok() { return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH; }
@@ -177,39 +253,49 @@ int b200_moe_route_topk(const float* logits, int T, int E, int k, int renorm, fl
 
 int b200_moe_offsets(const int* counts, int E, int* offsets, int* tile_expert, int* n_tiles, int* cursor,
                      int max_tiles, cudaStream_t stream) {
-  offsets_kernel<<<1, 32, 0, stream>>>(counts, E, offsets, tile_expert, n_tiles, cursor, max_tiles);
+  offsets_kernel<<<1, OFF_THREADS, 0, stream>>>(counts, E, offsets, tile_expert, n_tiles, cursor, max_tiles);
   return ok();
 }
 
 int b200_moe_permute(const void* x, const int* idx, const int* offsets, int* cursor, int* row_map, void* xp, int T,
                      int k, int H, cudaStream_t stream) {
   if (T <= 0) return 0;
+  if ((H & 7) || k <= 0 || k > 4096) return B200_ERR_ARG;
+  permute_kernel<<<T, row_threads(H), k * sizeof(int), stream>>>((const __nv_bfloat16*)x, idx, offsets, cursor, row_map,
+                                                                 (__nv_bfloat16*)xp, k, H);
+  return ok();
+}
+
+int b200_moe_zero_padding(const int* counts, const int* offsets, void* xp, int E, int H, cudaStream_t stream) {
+  if (E <= 0) return 0;
   if (H & 7) return B200_ERR_ARG;
-  permute_kernel<<<T * k, 128, 0, stream>>>((const __nv_bfloat16*)x, idx, offsets, cursor, row_map,
-                                            (__nv_bfloat16*)xp, T, k, H);
+  zero_padding_kernel<<<dim3(E, E < 64 ? 32 : 16), row_threads(H), 0, stream>>>(counts, offsets, (__nv_bfloat16*)xp, H);
   return ok();
 }
 
 int b200_moe_scatter_scaled(const void* src, const float* probs, const int* row_map, void* dst, int T, int k, int H,
                             cudaStream_t stream) {
   if (T <= 0) return 0;
-  scatter_scaled_kernel<<<T * k, 128, 0, stream>>>((const __nv_bfloat16*)src, probs, row_map, (__nv_bfloat16*)dst, T,
-                                                   k, H);
+  if (H & 7) return B200_ERR_ARG;
+  scatter_scaled_kernel<<<T, row_threads(H), 0, stream>>>((const __nv_bfloat16*)src, probs, row_map, (__nv_bfloat16*)dst,
+                                                          k, H);
   return ok();
 }
 
 int b200_moe_combine(const void* y, const float* probs, const int* row_map, void* out, int T, int k, int H,
                      cudaStream_t stream) {
   if (T <= 0) return 0;
-  combine_kernel<<<T, 256, 0, stream>>>((const __nv_bfloat16*)y, probs, row_map, (__nv_bfloat16*)out, T, k, H);
+  if (H & 7) return B200_ERR_ARG;
+  combine_kernel<<<T, row_threads(H), 0, stream>>>((const __nv_bfloat16*)y, probs, row_map, (__nv_bfloat16*)out, k, H);
   return ok();
 }
 
 int b200_moe_combine_dprob(const void* dout, const void* y, const int* row_map, float* dprob, int T, int k, int H,
                            cudaStream_t stream) {
   if (T <= 0) return 0;
-  combine_dprob_kernel<<<T * k, 128, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)y, row_map, dprob,
-                                                  T, k, H);
+  if (H & 7) return B200_ERR_ARG;
+  combine_dprob_kernel<<<T, row_threads(H), 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)y, row_map,
+                                                         dprob, k, H);
   return ok();
 }
 

@@ -174,7 +174,7 @@ class _SwiGLU(torch.autograd.Function):
         gu = _c(gate_up).view(-1, I2)
         out = torch.empty(gu.shape[0], I2 // 2, dtype=gu.dtype, device=gu.device)
         native.check(native.lib().b200_swiglu_fwd(native.ptr(gu), native.ptr(out), gu.shape[0], I2 // 2,
-                                                  native.stream()), "swiglu_fwd")
+                                                  None, native.stream()), "swiglu_fwd")
         ctx.save_for_backward(gu)
         ctx.shape = gate_up.shape
         return out.view(*gate_up.shape[:-1], I2 // 2)
@@ -185,7 +185,7 @@ class _SwiGLU(torch.autograd.Function):
         d2 = _c(dout).view(-1, gu.shape[1] // 2)
         dgu = torch.empty_like(gu)
         native.check(native.lib().b200_swiglu_bwd(native.ptr(d2), native.ptr(gu), native.ptr(dgu), gu.shape[0],
-                                                  gu.shape[1] // 2, native.stream()), "swiglu_bwd")
+                                                  gu.shape[1] // 2, None, native.stream()), "swiglu_bwd")
         return dgu.view(ctx.shape)
 
 

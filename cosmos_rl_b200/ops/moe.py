@@ -91,6 +91,26 @@ class _Dispatch:
                      "moe_offsets")
 
 
+    def zero_padding(self, buf: torch.Tensor) -> None:
+        """Clears the rows of an expert-sorted buffer that fill up each expert's last tile."""
+        native.check(native.lib().b200_moe_zero_padding(native.ptr(self.counts), native.ptr(self.offsets),
+                                                        native.ptr(buf), self.E, buf.shape[1], native.stream()),
+                     "moe_zero_padding")
+
+
+def _rows16(x: torch.Tensor) -> torch.Tensor:
+    """Contiguous rows that start on 16-byte boundaries."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
+def _swiglu_rows(h1: torch.Tensor, disp: _Dispatch) -> torch.Tensor:
+    out = torch.empty(h1.shape[0], h1.shape[1] // 2, dtype=h1.dtype, device=h1.device)
+    native.check(native.lib().b200_swiglu_fwd(native.ptr(h1), native.ptr(out), h1.shape[0], h1.shape[1] // 2,
+                                              native.ptr(disp.n_tiles), native.stream()), "swiglu_fwd")
+    return out
+
+
 def _grouped(x, w, disp: _Dispatch, mode: int, n_out: int) -> torch.Tensor:
     K = x.shape[1]
     y = torch.empty(disp.max_rows, n_out, dtype=torch.bfloat16, device=x.device)
@@ -122,12 +142,14 @@ class _MoEExperts(torch.autograd.Function):
         k = idx.shape[1]
         L = native.lib()
         disp = _Dispatch(idx, E, counts)
-        xp = torch.zeros(disp.max_rows, H, dtype=torch.bfloat16, device=x.device)
-        native.check(L.b200_moe_permute(native.ptr(x.contiguous()), native.ptr(idx), native.ptr(disp.offsets),
+        # rows of the permuted buffers beyond the last tile in use are never read and stay uninitialised
+        xp = torch.empty(disp.max_rows, H, dtype=torch.bfloat16, device=x.device)
+        disp.zero_padding(xp)
+        native.check(L.b200_moe_permute(native.ptr(_rows16(x)), native.ptr(idx), native.ptr(disp.offsets),
                                         native.ptr(disp.cursor), native.ptr(disp.row_map), native.ptr(xp), T, k, H,
                                         native.stream()), "moe_permute")
         h1 = _grouped(xp, w_gate_up, disp, 0, I2)
-        act = F.swiglu(h1)
+        act = _swiglu_rows(h1, disp)
         y = _grouped(act, w_down, disp, 0, H)
         out = torch.empty(T, H, dtype=torch.bfloat16, device=x.device)
         probs = probs.float().contiguous()
@@ -145,20 +167,21 @@ class _MoEExperts(torch.autograd.Function):
         H = xp.shape[1]
         I2 = h1.shape[1]
         L = native.lib()
-        dout = dout.contiguous()
+        dout = _rows16(dout)
         dprob = torch.empty(T, k, dtype=torch.float32, device=dout.device)
         native.check(L.b200_moe_combine_dprob(native.ptr(dout), native.ptr(y), native.ptr(disp.row_map),
                                               native.ptr(dprob), T, k, H, native.stream()), "moe_dprob")
-        dy = torch.zeros(disp.max_rows, H, dtype=torch.bfloat16, device=dout.device)
+        dy = torch.empty(disp.max_rows, H, dtype=torch.bfloat16, device=dout.device)
+        disp.zero_padding(dy)
         native.check(L.b200_moe_scatter_scaled(native.ptr(dout), native.ptr(probs), native.ptr(disp.row_map),
                                                native.ptr(dy), T, k, H, native.stream()), "moe_scatter")
-        act = F.swiglu(h1)                                  # recomputed: cheaper than keeping [Mp, I] alive
+        act = _swiglu_rows(h1, disp)                        # recomputed: cheaper than keeping [Mp, I] alive
         dact = _grouped(dy, w_down, disp, 1, I2 // 2)       # dY . W_down[e]   (W_down [E, H, I])
         dw_down = torch.empty_like(w_down)
         _grouped_wgrad(dy, act, disp, dw_down, False)
         dh1 = torch.empty_like(h1)
         native.check(L.b200_swiglu_bwd(native.ptr(dact), native.ptr(h1), native.ptr(dh1), h1.shape[0], I2 // 2,
-                                       native.stream()), "swiglu_bwd")
+                                       native.ptr(disp.n_tiles), native.stream()), "swiglu_bwd")
         dxp = _grouped(dh1, w_gate_up, disp, 1, H)          # dH1 . W_gu[e]     (W_gu [E, 2I, H])
         dw_gu = torch.empty_like(w_gate_up)
         _grouped_wgrad(dh1, xp, disp, dw_gu, False)

@@ -74,8 +74,8 @@ _SIGS = {
     "b200_colsum_f32": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "b200_rope_inplace": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_float,
                           c_int, c_void_p],
-    "b200_swiglu_fwd": [c_void_p, c_void_p, c_longlong, c_int, c_void_p],
-    "b200_swiglu_bwd": [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p],
+    "b200_swiglu_fwd": [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p],
+    "b200_swiglu_bwd": [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p],
     "b200_adamw": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_float, c_float, c_float,
                    c_float, c_float, c_float, c_float, c_void_p, c_void_p],
     "b200_sumsq": [c_void_p, c_int, c_longlong, c_void_p, c_void_p],
@@ -106,6 +106,7 @@ _SIGS = {
     "b200_moe_route_topk": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "b200_moe_offsets": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "b200_moe_permute": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "b200_moe_zero_padding": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "b200_moe_scatter_scaled": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "b200_moe_combine": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "b200_moe_combine_dprob": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
