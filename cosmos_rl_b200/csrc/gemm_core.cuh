@@ -24,9 +24,11 @@ constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;  // 64 bf16 = 128 bytes = one swizzle row
 constexpr int GEMM_THREADS = 192;
 
-template <int BN, int STAGES>
+// A_ROWS < 128: only that many rows of the A tile are fetched and kept (a problem with few rows); the MMA then reads
+// whatever follows them for the other rows, whose results nobody stores.
+template <int BN, int STAGES, int A_ROWS = GEMM_BM>
 struct GemmSmem {
-  static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
+  static constexpr int A_BYTES = A_ROWS * GEMM_BK * 2;
   static constexpr int B_BYTES = BN * GEMM_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int BAR_BYTES = 256;
@@ -62,14 +64,20 @@ struct TileInfo {
 // t.b_mn1 (gate and up rows of a fused gate/up weight, so that one accumulator row holds both).
 // L2_PREFETCH (B not MN-major, 2-D): before the CTA waits for the previous kernel of the stream it brings the first
 // ep.prefetch_kb contraction blocks of its B tiles into L2. The schedule's init() may then read nothing but Params.
+// A_ROWS (A K-major, 2-D): see GemmSmem; the tensor map's box has that many rows.
+// DYN_N (B K-major): a tile has ep.b_rows <= BN rows of B (a multiple of 16), chosen at launch; the boxes of B have
+// ep.b_rows rows, or ep.b_rows / 2 with B_TWO_BOXES.
 template <bool A_MN_ = false, bool B_MN_ = false, bool A_3D_ = false, bool B_3D_ = false, int SIDE_WARPS_ = 0,
-          bool PRODUCER_HOOK_ = false, bool B_TWO_BOXES_ = false, bool L2_PREFETCH_ = false>
+          bool PRODUCER_HOOK_ = false, bool B_TWO_BOXES_ = false, bool L2_PREFETCH_ = false, int A_ROWS_ = GEMM_BM,
+          bool DYN_N_ = false>
 struct GemmTraits {
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_, A_3D = A_3D_, B_3D = B_3D_;
   static constexpr int SIDE_WARPS = SIDE_WARPS_;
   static constexpr bool PRODUCER_HOOK = PRODUCER_HOOK_;
   static constexpr bool B_TWO_BOXES = B_TWO_BOXES_;
   static constexpr bool L2_PREFETCH = L2_PREFETCH_;
+  static constexpr int A_ROWS = A_ROWS_;
+  static constexpr bool DYN_N = DYN_N_;
 };
 
 // An epilogue that declares `static constexpr bool CUSTOM_TILE = true` reads its accumulator itself:
@@ -123,7 +131,8 @@ struct RasterSchedule {
 template <int BN, int STAGES, class Epi, class Sched, class Traits = GemmTraits<>>
 __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, int M, int N, int K,
                                               const typename Epi::Params& ep, uint32_t* status) {
-  using SM = GemmSmem<BN, STAGES>;
+  using SM = GemmSmem<BN, STAGES, Traits::A_ROWS>;
+  static_assert(SM::A_BYTES % 1024 == 0 && SM::STAGE_BYTES >= GEMM_BM * GEMM_BK * 2, "the A tile's rows lie in its stage");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * SM::STAGE_BYTES);
@@ -201,7 +210,13 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
           uint8_t* sa = smem + stage * SM::STAGE_BYTES;
           uint8_t* sb = sa + SM::A_BYTES;
           const int k = t.k0 + kb * GEMM_BK;
-          mbar_arrive_expect_tx(&full_bar[stage], SM::STAGE_BYTES);
+          uint32_t b_half = SM::B_BYTES / 2;   // B_TWO_BOXES: bytes of one box
+          if constexpr (Traits::DYN_N) {
+            b_half = ep.b_rows * (GEMM_BK * 2 / 2);
+            mbar_arrive_expect_tx(&full_bar[stage], SM::A_BYTES + 2 * b_half);
+          } else {
+            mbar_arrive_expect_tx(&full_bar[stage], SM::STAGE_BYTES);
+          }
           if constexpr (!Traits::A_MN) {
             if constexpr (Traits::A_3D) tma_load_3d(sa, tmA, &full_bar[stage], k, t.a_mn0, t.batch);
             else tma_load_2d(sa, tmA, &full_bar[stage], k, t.a_mn0);
@@ -214,7 +229,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
           }
           if constexpr (Traits::B_TWO_BOXES) {
             tma_load_2d(sb, tmB, &full_bar[stage], k, t.b_mn0);
-            tma_load_2d(sb + SM::B_BYTES / 2, tmB, &full_bar[stage], k, t.b_mn1);
+            tma_load_2d(sb + b_half, tmB, &full_bar[stage], k, t.b_mn1);
           } else if constexpr (!Traits::B_MN) {
             if constexpr (Traits::B_3D) tma_load_3d(sb, tmB, &full_bar[stage], k, t.b_mn0, t.batch);
             else tma_load_2d(sb, tmB, &full_bar[stage], k, t.b_mn0);
@@ -232,8 +247,8 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
     if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16_f32(GEMM_BM, BN) | (Traits::A_MN ? (1u << 15) : 0u) |
-                                 (Traits::B_MN ? (1u << 16) : 0u);
+      uint32_t idesc = umma_idesc_bf16_f32(GEMM_BM, BN) | (Traits::A_MN ? (1u << 15) : 0u) | (Traits::B_MN ? (1u << 16) : 0u);
+      if constexpr (Traits::DYN_N) idesc = umma_idesc_bf16_f32(GEMM_BM, ep.b_rows);
       uint32_t stage = 0, phase = 0;
       uint32_t acc = 0, acc_phase = 0;
       TileInfo t;

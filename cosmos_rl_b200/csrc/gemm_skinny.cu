@@ -18,12 +18,17 @@
 
 namespace b200 {
 
-// Tile widths: 128 columns (6 stages) when the contraction has to be split to occupy the machine, 256 columns (4
-// stages) when the column tiles alone do: a wider tile re-reads the activation rows half as often, and with 128
-// rows per tile that traffic out of L2 is as large as the weight stream itself.
-template <int BN>
+// Tile widths: 128 columns when the contraction has to be split to occupy the machine, 256 columns when the column
+// tiles alone do: a wider tile re-reads the activation rows half as often, and with 128 rows per tile that traffic out
+// of L2 is as large as the weight stream itself. Up to 16 or 64 rows only those rows are kept per stage and the room
+// goes into more stages, i.e. more of the weight stream in flight.
+template <int BN, int A_ROWS>
 struct SkinnyCfg {
-  static constexpr int STAGES = BN == 256 ? 4 : 6;
+  static constexpr int STAGES = BN == 256 ? (A_ROWS == 16 ? 5 : 4) : (A_ROWS == 16 ? 10 : A_ROWS == 64 ? 8 : 6);
+  static constexpr int ROW_STORE_STAGES = A_ROWS == 16 ? 6 : A_ROWS == 64 ? 5 : 4;   // 256 wide, no store staging
+  static constexpr int SMEM_LIMIT = 227 * 1024;
+  static_assert(GemmSmem<BN, STAGES, A_ROWS>::TOTAL_WITH_EPI <= SMEM_LIMIT, "shared memory");
+  static_assert(GemmSmem<256, ROW_STORE_STAGES, A_ROWS>::TOTAL <= SMEM_LIMIT, "shared memory");
 };
 
 struct SkinnyParams {
@@ -33,17 +38,20 @@ struct SkinnyParams {
   int to_ws;                  // 1: fp32 partials through the 3-D map; 0: bf16 result through the 2-D map
   int M, N;                   // N = columns of the output (for SwiGLU: the intermediate size)
   int splits;
+  __nv_bfloat16* out;         // direct output of the row-store epilogue
+  long long ldo;
   int up_row0;                // SwiGLU: first "up" row of W
+  int b_rows;                 // rows of W per tile (BN, or the width chosen at launch)
   int prefetch_kb;            // contraction blocks a CTA brings into L2 before it waits for the previous kernel
 };
 
 template <int BN, bool SWIGLU>
 struct SkinnySchedule {
-  int num_m, num_n, splits, num_kb, total, up_row0;
+  int num_m, num_n, splits, num_kb, total, up_row0, out_bn;
   __device__ __forceinline__ void init(int M, int N, int K, int, const SkinnyParams& p) {
     num_m = (M + GEMM_BM - 1) / GEMM_BM;
-    constexpr int OUT_BN = SWIGLU ? BN / 2 : BN;
-    num_n = (p.N + OUT_BN - 1) / OUT_BN;
+    out_bn = SWIGLU ? p.b_rows / 2 : BN;
+    num_n = (p.N + out_bn - 1) / out_bn;
     splits = p.splits;
     num_kb = (K + GEMM_BK - 1) / GEMM_BK;
     total = num_m * num_n * splits;
@@ -62,8 +70,8 @@ struct SkinnySchedule {
     const int kb1 = (int)(((long long)(s + 1) * num_kb) / splits);
     t.a_mn0 = t.m_blk * GEMM_BM;
     if (SWIGLU) {
-      t.b_mn0 = t.n_blk * (BN / 2);
-      t.b_mn1 = up_row0 + t.n_blk * (BN / 2);
+      t.b_mn0 = t.n_blk * out_bn;
+      t.b_mn1 = up_row0 + t.n_blk * out_bn;
     } else {
       t.b_mn0 = t.n_blk * BN;
       t.b_mn1 = 0;
@@ -92,6 +100,7 @@ struct SkinnyEpilogue {
     uint8_t* slab0 = epi_smem + quad * 8192;
     const uint32_t sw = (uint32_t)(lane & 7);
     const int row0 = t.m_blk * GEMM_BM + quad * 32;
+    if (row0 >= p.M) return;
     const int slab_cols = p.to_ws ? 32 : 64;
 #pragma unroll 1
     for (int c = 0; c < OUT_BN; c += slab_cols) {
@@ -160,14 +169,66 @@ struct SkinnyEpilogue {
   }
 };
 
-template <int BN, bool SWIGLU>
+// SwiGLU tiles of any width (a multiple of 8 columns): a tile's edge need not be a multiple of a store box, so rows are
+// written with plain 16-byte stores.
+struct SwigluRowsEpilogue {
+  using Params = SkinnyParams;
+  static constexpr bool CUSTOM_TILE = true;
+  __device__ __forceinline__ void finish(const Params&) {}
+  __device__ __forceinline__ void tile(const Params& p, const TileInfo& t, int row, uint32_t taddr, uint8_t*) {
+    const int width = p.b_rows / 2, r = t.m_blk * GEMM_BM + row, gc0 = t.n_blk * width;
+    if (r - (int)(threadIdx.x & 31) >= p.M) return;   // none of the warp's rows
+    __nv_bfloat16* dst = p.out + (long long)r * p.ldo + gc0;
+#pragma unroll 1
+    for (int c = 0; c < width; c += 16) {
+      uint32_t a[16], u[16];
+      tmem_ld_32x32b_x16(taddr + c, a);
+      tmem_ld_32x32b_x16(taddr + width + c, u);
+      tmem_ld_wait();
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float g = __uint_as_float(a[j]);
+        v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
+      }
+      if (r >= p.M) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int cc = c + 8 * h;
+        if (cc >= width) continue;
+        if (gc0 + cc + 8 <= p.N) {
+          uint4 o;
+          o.x = pack_bf16x2(v[8 * h], v[8 * h + 1]);
+          o.y = pack_bf16x2(v[8 * h + 2], v[8 * h + 3]);
+          o.z = pack_bf16x2(v[8 * h + 4], v[8 * h + 5]);
+          o.w = pack_bf16x2(v[8 * h + 6], v[8 * h + 7]);
+          *reinterpret_cast<uint4*>(dst + cc) = o;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (gc0 + cc + j < p.N) dst[cc + j] = __float2bfloat16(v[8 * h + j]);
+        }
+      }
+    }
+  }
+};
+
+template <int BN, bool SWIGLU, int A_ROWS>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmO, int M, int N, int K, SkinnyParams ep, uint32_t* status) {
   ep.tm_out = &tmO;
   if (threadIdx.x == 0) tma_prefetch_desc(&tmO);
-  gemm_mainloop<BN, SkinnyCfg<BN>::STAGES, SkinnyEpilogue<BN, SWIGLU>, SkinnySchedule<BN, SWIGLU>,
-                GemmTraits<false, false, false, false, 0, false, SWIGLU, true>>(&tmA, &tmB, M, N, K, ep, status);
+  gemm_mainloop<BN, SkinnyCfg<BN, A_ROWS>::STAGES, SkinnyEpilogue<BN, SWIGLU>, SkinnySchedule<BN, SWIGLU>,
+                GemmTraits<false, false, false, false, 0, false, SWIGLU, true, A_ROWS>>(&tmA, &tmB, M, N, K, ep, status);
+}
+
+template <int A_ROWS>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_skinny_swiglu_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
+                               int N, int K, SkinnyParams ep, uint32_t* status) {
+  gemm_mainloop<256, SkinnyCfg<256, A_ROWS>::ROW_STORE_STAGES, SwigluRowsEpilogue, SkinnySchedule<256, true>,
+                GemmTraits<false, false, false, false, 0, false, true, true, A_ROWS, true>>(&tmA, &tmB, M, N, K, ep, status);
 }
 
 // fp32 [splits, M, N] partials: boxes of 32 rows x 32 columns, 128-byte swizzle
@@ -422,24 +483,58 @@ static int skinny_bn(int M, int N, int swiglu, int num_sms) {
   return tiles256 >= 2 * num_sms ? 256 : 128;
 }
 
-template <int BN, bool SWIGLU>
+// SwiGLU: columns per tile when every SM gets one tile of that width, or 0 when fixed 64-column tiles are as good. Tiles
+// of 64 columns cost whole rounds: 14336 columns are 224 tiles, two rounds of 148 SMs for 1.5 rounds of work, while
+// 104-column tiles are one round of 138.
+static int swiglu_width(int M, int N, int num_sms) {
+  const int num_m = (M + b200::GEMM_BM - 1) / b200::GEMM_BM;
+  if (num_m > num_sms) return 0;
+  const int per_sm = num_sms / num_m;                       // column tiles that fit in one round
+  const int w = ((N + per_sm - 1) / per_sm + 7) / 8 * 8;
+  const int rounds64 = (num_m * ((N + 63) / 64) + num_sms - 1) / num_sms;
+  return w <= 128 && w < 64 * rounds64 * 0.95f ? w : 0;
+}
+
+template <class Kern>
+static int launch_skinny_kernel(Kern kern, bool& attr_set, int smem, int units, int num_sms) {
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
+    attr_set = true;
+  }
+  return units < num_sms ? units : num_sms;   // grid
+}
+
+template <int BN, bool SWIGLU, int A_ROWS>
 static int launch_skinny(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmO, int M, int N, int K,
                          const b200::SkinnyParams& ep, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
-  using SM = GemmSmem<BN, SkinnyCfg<BN>::STAGES>;
-  auto kern = gemm_skinny_kernel<BN, SWIGLU>;
+  using SM = GemmSmem<BN, SkinnyCfg<BN, A_ROWS>::STAGES, A_ROWS>;
+  auto kern = gemm_skinny_kernel<BN, SWIGLU, A_ROWS>;
   static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL_WITH_EPI) != cudaSuccess)
-      return B200_ERR_LAUNCH;
-    attr_set = true;
-  }
   constexpr int OUT_BN = SWIGLU ? BN / 2 : BN;
   const int units = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + OUT_BN - 1) / OUT_BN) * ep.splits;
-  const int grid = units < num_sms ? units : num_sms;
+  const int grid = launch_skinny_kernel(kern, attr_set, SM::TOTAL_WITH_EPI, units, num_sms);
+  if (grid < 0) return B200_ERR_LAUNCH;
   return launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), SM::TOTAL_WITH_EPI, stream, tmA, tmB, tmO, M, N, K, ep,
                     status) == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
+
+template <int A_ROWS>
+static int launch_swiglu_rows(const CUtensorMap& tmA, const CUtensorMap& tmB, int M, int N, int K,
+                              const b200::SkinnyParams& ep, uint32_t* status, int num_sms, cudaStream_t stream) {
+  using namespace b200;
+  using SM = GemmSmem<256, SkinnyCfg<256, A_ROWS>::ROW_STORE_STAGES, A_ROWS>;
+  auto kern = gemm_skinny_swiglu_rows_kernel<A_ROWS>;
+  static bool attr_set = false;
+  const int width = ep.b_rows / 2, units = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + width - 1) / width);
+  const int grid = launch_skinny_kernel(kern, attr_set, SM::TOTAL, units, num_sms);
+  if (grid < 0) return B200_ERR_LAUNCH;
+  return launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), SM::TOTAL, stream, tmA, tmB, M, N, K, ep, status) == cudaSuccess
+             ? 0 : B200_ERR_LAUNCH;
+}
+
+// rows of the A tile that are kept in shared memory
+static int skinny_a_rows(int M) { return M <= 16 ? 16 : M <= 64 ? 64 : b200::GEMM_BM; }
 
 extern "C" {
 
@@ -468,18 +563,27 @@ int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, 
   if (splits > 1 && (!ws || swiglu)) return B200_ERR_ARG;
   if (!ws && !out) return B200_ERR_ARG;
   const int n_rows_w = swiglu ? up_row0 + N : N;
-  const int bn = skinny_bn(M, N, swiglu, num_sms);
+  const int width = swiglu ? swiglu_width(M, N, num_sms) : 0;
+  const int bn = width ? 256 : skinny_bn(M, N, swiglu, num_sms);
+  const int b_rows = width ? 2 * width : bn, a_rows = skinny_a_rows(M);
   CUtensorMap tmA, tmB, tmO;
-  if (make_tmap_2d(&tmA, x, M, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
-  if (make_tmap_2d(&tmB, W, n_rows_w, K, ldw, swiglu ? bn / 2 : bn, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tmA, x, M, K, ldx, a_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tmB, W, n_rows_w, K, ldw, swiglu ? b_rows / 2 : b_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (ws ? make_tmap_ws(&tmO, ws, splits, M, N) : make_tmap_out16(&tmO, out, M, N, ldo)) return B200_ERR_TENSORMAP;
-  SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, up_row0, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
-  if (bn == 256) {
-    if (swiglu) return launch_skinny<256, true>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
-    return launch_skinny<256, false>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
-  }
-  if (swiglu) return launch_skinny<128, true>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
-  return launch_skinny<128, false>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
+  SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, (__nv_bfloat16*)out, ldo, up_row0,
+                  b_rows, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
+  auto launch = [&](auto rows) -> int {
+    constexpr int R = decltype(rows)::value;
+    if (width) return launch_swiglu_rows<R>(tmA, tmB, M, N, K, ep, status, num_sms, stream);
+    if (bn == 256)
+      return swiglu ? launch_skinny<256, true, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream)
+                    : launch_skinny<256, false, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
+    return swiglu ? launch_skinny<128, true, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream)
+                  : launch_skinny<128, false, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
+  };
+  if (a_rows == 16) return launch(std::integral_constant<int, 16>{});
+  if (a_rows == 64) return launch(std::integral_constant<int, 64>{});
+  return launch(std::integral_constant<int, GEMM_BM>{});
 }
 
 int b200_splitk_reduce(const float* ws, int splits, int M, int N, const void* bias, int bias_bf16, void* out,

@@ -976,3 +976,31 @@ def test_moe_experts_padding_and_many_choices(T, H, I, E, k):
     assert torch.allclose(out.float(), ref, rtol=3e-2, atol=3e-2 * ref.abs().max().item())
     for a, b in zip(got, want):
         assert torch.allclose(a.float(), b, rtol=5e-2, atol=5e-2 * b.abs().max().item())
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 64, 65, 129, 256])
+@pytest.mark.parametrize("I,K", [(14336, 512), (18944, 128), (1000, 520), (64, 64)])
+def test_skinny_swiglu_tile_widths(M, I, K):
+    """Row counts around the kept A rows (16, 64, 128) and column counts that take both kinds of tiles."""
+    torch.manual_seed(35)
+    x, w = _bf16(M, K), _bf16(2 * I, K, scale=0.05)
+    z = F.skinny_gate_up_swiglu(x, w)
+    native.read_status(x.device)
+    gu = x.float() @ w.float().t()
+    ref = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+    # fp32 sums of K products, rounded once to bf16
+    assert torch.allclose(z.float(), ref, rtol=2 ** -8, atol=1e-4 * math.sqrt(K)), (z.float() - ref).abs().max()
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 64, 65])
+@pytest.mark.parametrize("N,K", [(4096, 2048), (6144, 1032), (32000, 512), (72, 64)])
+def test_skinny_kept_rows(M, N, K):
+    torch.manual_seed(36)
+    x, w, res = _bf16(M, K), _bf16(N, K, scale=0.05), _bf16(M, N)
+    y = F.gemm_skinny(x, w)
+    ref = x.float() @ w.float().t()
+    assert torch.allclose(y.float(), ref, rtol=2 ** -8, atol=1e-4 * math.sqrt(K))
+    if N <= 8192:
+        _, r = F.skinny_linear_residual_rmsnorm(x, w, res, torch.ones(N, dtype=torch.bfloat16, device=DEV), 1e-6)
+        assert torch.allclose(r.float(), ref + res.float(), rtol=2 ** -8, atol=1e-4 * math.sqrt(K))
+    native.read_status(x.device)
