@@ -1004,3 +1004,45 @@ def test_skinny_kept_rows(M, N, K):
         _, r = F.skinny_linear_residual_rmsnorm(x, w, res, torch.ones(N, dtype=torch.bfloat16, device=DEV), 1e-6)
         assert torch.allclose(r.float(), ref + res.float(), rtol=2 ** -8, atol=1e-4 * math.sqrt(K))
     native.read_status(x.device)
+
+
+# ------------------------------------------------------------------------------------------------ edges of tiles
+@pytest.mark.parametrize("lens,hq,hkv,causal", [([127], 3, 1, True), ([128, 129], 2, 2, True), ([255, 256, 257, 1], 4, 2, True),
+                                                ([385], 7, 1, True), ([127, 1, 130], 2, 1, False), ([513, 64], 2, 2, False)])
+def test_flash_attention_tile_edges(lens, hq, hkv, causal):
+    """Sequence lengths around one and two tiles of queries and keys: forward and gradients against fp32, the same bits on
+    a second run, and a zero query gradient for tokens that belong to no sequence."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(31)
+    d, T = 128, sum(lens) + 3                                       # three tokens after the last sequence
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    q, k, v, go = _bf16(T, hq, d), _bf16(T, hkv, d), _bf16(T, hkv, d), _bf16(T, hq, d)
+    scale, n = 1.0 / math.sqrt(d), sum(lens)
+    out, lse = attention.flash_fwd(q, k, v, cu, cu, max(lens), scale, causal)
+    grads = attention.flash_bwd(go, q, k, v, out, lse, cu, max(lens), scale, causal=causal)
+    again = attention.flash_bwd(go, q, k, v, out, lse, cu, max(lens), scale, causal=causal)
+    native.read_status(q.device)
+    assert torch.equal(grads[0], again[0]) and all(torch.equal(a[:n], b[:n]) for a, b in zip(grads[1:], again[1:]))
+    assert not grads[0][n:].any()
+    rq, rk, rv = (t.float().requires_grad_(True) for t in (q, k, v))
+    ref = R.varlen_attention(rq, rk, rv, cu, scale, causal=causal)
+    ref.backward(go.float())
+    # bf16 rounds the result (2^-9 of it) and P / dS on the way (2^-9 of sums of about unit terms)
+    assert torch.allclose(out[:n].float(), ref[:n], atol=2e-2, rtol=2e-2)
+    for got, want in zip(grads, (rq.grad, rk.grad, rv.grad)):
+        assert (got[:n].float() - want[:n]).abs().max() <= 3e-2 * want.abs().max() + 2e-2
+
+
+def test_flash_attention_scores_that_grow_along_the_keys():
+    """Running maximum that moves in every key block (the accumulator is rescaled) and probabilities that underflow."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(32)
+    L, h, d = 700, 2, 128
+    q = torch.ones(L, h, d, device=DEV).to(torch.bfloat16)
+    k = (torch.linspace(0, 40, L, device=DEV)[:, None, None] + torch.zeros(L, h, d, device=DEV)).to(torch.bfloat16)
+    v = _bf16(L, h, d)
+    cu = torch.tensor([0, L], dtype=torch.int32, device=DEV)
+    out, _ = attention.flash_fwd(q, k, v, cu, cu, L, 1.0 / math.sqrt(d), True)
+    native.read_status(q.device)
+    ref = R.varlen_attention(q.float(), k.float(), v.float(), cu, 1.0 / math.sqrt(d))
+    assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2), (out.float() - ref).abs().max()
