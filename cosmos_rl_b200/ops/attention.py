@@ -13,6 +13,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import native
+from .functional import needs_graph
 
 
 def native_flash_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
@@ -53,6 +54,12 @@ class _FlashAttn(torch.autograd.Function):
                          max_k=ctx.max_k, causal=ctx.causal) + (None, None, None, None, None, None)
 
 
+def _attend(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal):
+    if not needs_graph(q, k, v):
+        return flash_fwd(q, k, v, cu_q, cu_k, max_q, scale, causal)[0]
+    return _FlashAttn.apply(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal)
+
+
 def flash_attention(q, k, v, cu_q, cu_k, max_q: int, scale: Optional[float] = None, max_k: Optional[int] = None,
                     causal: bool = True):
     """Differentiable attention over packed sequences. Causal: the queries of a sequence are aligned to the end of
@@ -62,7 +69,7 @@ def flash_attention(q, k, v, cu_q, cu_k, max_q: int, scale: Optional[float] = No
     i32 = lambda t: t if t.dtype == torch.int32 else t.to(torch.int32)
     if max_k is None:
         max_k = int((cu_k[1:] - cu_k[:-1]).max().item()) if cu_k is not cu_q else max_q
-    return _FlashAttn.apply(q, k, v, i32(cu_q), i32(cu_k), int(max_q), int(max_k), scale, bool(causal))
+    return _attend(q, k, v, i32(cu_q), i32(cu_k), int(max_q), int(max_k), scale, bool(causal))
 
 
 def flash_bwd(dout, q, k, v, out, lse, cu, max_seqlen: int, scale: float, cu_k=None, max_k=None,
@@ -99,7 +106,7 @@ def full_attention_cuda(q, k, v, cu_q, cu_k, max_q: int, max_k: int, scale: Opti
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     i32 = lambda t: t if t.dtype == torch.int32 else t.to(torch.int32)
     if native_flash_supported(q, k, v):
-        return _FlashAttn.apply(q, k, v, i32(cu_q), i32(cu_k), int(max_q), int(max_k), scale, False)
+        return _attend(q, k, v, i32(cu_q), i32(cu_k), int(max_q), int(max_k), scale, False)
     from flash_attn import flash_attn_varlen_func
     return flash_attn_varlen_func(q, k, v, i32(cu_q), i32(cu_k), max_q, max_k, dropout_p=0.0, softmax_scale=scale,
                                   causal=False)
@@ -110,7 +117,7 @@ def varlen_attention_cuda(q, k, v, cu_seqlens, max_seqlen: int, scale: Optional[
     scale = scale if scale is not None else 1.0 / math.sqrt(d)
     cu = cu_seqlens if cu_seqlens.dtype == torch.int32 else cu_seqlens.to(torch.int32)
     if native_flash_supported(q, k, v):
-        return _FlashAttn.apply(q, k, v, cu, cu, int(max_seqlen), int(max_seqlen), scale)
+        return _attend(q, k, v, cu, cu, int(max_seqlen), int(max_seqlen), scale, True)
     from flash_attn import flash_attn_varlen_func
     return flash_attn_varlen_func(q, k, v, cu, cu, max_seqlen, max_seqlen, dropout_p=0.0, softmax_scale=scale,
                                   causal=True)

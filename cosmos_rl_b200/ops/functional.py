@@ -12,6 +12,7 @@ import os
 from typing import Optional, Tuple
 
 import torch
+from torch.autograd import forward_ad
 
 from . import native, reference
 
@@ -22,9 +23,28 @@ def _c(t: torch.Tensor) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+def needs_graph(*tensors: Optional[torch.Tensor]) -> bool:
+    """Whether a call has to go through its autograd function: one of the inputs records a gradient, or forward-mode
+    derivatives are being taken (which the functions refuse). Inference calls skip the function's bookkeeping."""
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t is not None and t.requires_grad:
+                return True
+    return forward_ad._current_level >= 0
+
+
 # --------------------------------------------------------------------------------------------------
 # RMSNorm
 # --------------------------------------------------------------------------------------------------
+def _rmsnorm_fwd(x2, weight, eps, res2, rstd):
+    y = torch.empty_like(x2)
+    res_out = torch.empty_like(x2) if res2 is not None else None
+    native.check(native.lib().b200_rmsnorm_fwd(native.ptr(x2), native.ptr(res2), native.ptr(weight), native.ptr(y),
+                                               native.ptr(res_out), native.ptr(rstd), x2.shape[0], x2.shape[1], eps,
+                                               native.stream()), "rmsnorm_fwd")
+    return y, res_out
+
+
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps, residual):
@@ -33,13 +53,8 @@ class _RMSNorm(torch.autograd.Function):
         x2 = _c(x).view(-1, H)
         T = x2.shape[0]
         res2 = _c(residual).view(-1, H) if residual is not None else None
-        y = torch.empty_like(x2)
-        res_out = torch.empty_like(x2) if residual is not None else None
         rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-        L = native.lib()
-        native.check(L.b200_rmsnorm_fwd(native.ptr(x2), native.ptr(res2), native.ptr(weight), native.ptr(y),
-                                        native.ptr(res_out), native.ptr(rstd), T, H, eps, native.stream()),
-                     "rmsnorm_fwd")
+        y, res_out = _rmsnorm_fwd(x2, weight, eps, res2, rstd)
         h = res_out if residual is not None else x2
         ctx.save_for_backward(h, weight, rstd)
         ctx.has_res = residual is not None
@@ -72,6 +87,11 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual:
     if x.is_cuda:
         if x.dtype != torch.bfloat16:
             raise TypeError("rms_norm on CUDA expects bf16 activations")
+        if not needs_graph(x, weight, residual):
+            shape, H = x.shape, x.shape[-1]
+            y, res_out = _rmsnorm_fwd(_c(x).view(-1, H), weight, eps,
+                                      _c(residual).view(-1, H) if residual is not None else None, None)
+            return y.view(shape), res_out.view(shape) if res_out is not None else None
         return _RMSNorm.apply(x, weight, eps, residual)
     return reference.rms_norm(x, weight, eps, residual)
 
@@ -167,14 +187,19 @@ def rope_qkv_(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: 
 # --------------------------------------------------------------------------------------------------
 # SwiGLU
 # --------------------------------------------------------------------------------------------------
+def _swiglu_fwd(gu):
+    out = torch.empty(gu.shape[0], gu.shape[1] // 2, dtype=gu.dtype, device=gu.device)
+    native.check(native.lib().b200_swiglu_fwd(native.ptr(gu), native.ptr(out), gu.shape[0], gu.shape[1] // 2, None,
+                                              native.stream()), "swiglu_fwd")
+    return out
+
+
 class _SwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate_up):
         I2 = gate_up.shape[-1]
         gu = _c(gate_up).view(-1, I2)
-        out = torch.empty(gu.shape[0], I2 // 2, dtype=gu.dtype, device=gu.device)
-        native.check(native.lib().b200_swiglu_fwd(native.ptr(gu), native.ptr(out), gu.shape[0], I2 // 2,
-                                                  None, native.stream()), "swiglu_fwd")
+        out = _swiglu_fwd(gu)
         ctx.save_for_backward(gu)
         ctx.shape = gate_up.shape
         return out.view(*gate_up.shape[:-1], I2 // 2)
@@ -191,6 +216,9 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     if gate_up.is_cuda:
+        if not needs_graph(gate_up):
+            I2 = gate_up.shape[-1]
+            return _swiglu_fwd(_c(gate_up).view(-1, I2)).view(*gate_up.shape[:-1], I2 // 2)
         return _SwiGLU.apply(gate_up)
     return reference.swiglu(gate_up)
 

@@ -145,8 +145,15 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (without building a ``torch.cuda.Stream`` for each launch)."""
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 LAUNCHES = [0]  # launcher calls into libb200rl since import (CUDA-graph replays add their captured count)
