@@ -27,7 +27,7 @@ constexpr int G2_BM = 256;      // rows of the pair's tile
 constexpr int G2_BK = 64;
 constexpr int G2_THREADS = 192;
 
-enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1 };
+enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2 };
 
 template <int BN, int STAGES>
 struct Gemm2Smem {
@@ -39,6 +39,40 @@ struct Gemm2Smem {
   static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING_BYTES + BAR_BYTES + 1024;
 };
 
+// G2_EPI_DLOGITS: the accumulator is a tile of logits (before the temperature) and the result is their gradient, see
+// dlogit_of. Arrays of one value a row; g_ent and ent may be null.
+struct DlogitsParams {
+  const long long* labels;
+  const float* lse;
+  const float* g_lp;
+  const float* g_ent;
+  const float* ent;
+  int v0;             // vocabulary index of column 0
+  float inv_temp;
+};
+
+// Gradient of g_lp * logprob + g_ent * entropy with respect to one logit (a = the product before the temperature), without
+// the label's own term.
+struct DlogitsRow {
+  float lse, glp, gent, ent;
+  long long label;
+  __device__ __forceinline__ void load(const DlogitsParams& p, long long r) {
+    lse = p.lse[r];
+    glp = p.g_lp[r];
+    gent = p.g_ent ? p.g_ent[r] : 0.f;
+    ent = p.ent ? p.ent[r] : 0.f;
+    label = p.labels[r];
+    if (label < 0) glp = 0.f;
+  }
+  __device__ __forceinline__ float of(float a, float inv_temp, bool is_label) const {
+    const float x = a * inv_temp;
+    const float pr = __expf(x - lse);
+    float g = -glp * pr - gent * pr * (x - lse + ent);
+    if (is_label) g += glp;
+    return g * inv_temp;
+  }
+};
+
 struct Gemm2Params {
   const void* bias;  // [N] added to every row (nullable); bf16 when bias_bf16 else fp32
   int bias_bf16;
@@ -46,6 +80,7 @@ struct Gemm2Params {
   int accumulate;    // C += result (TMA reduce-add)
   int up_row0;       // G2_EPI_SWIGLU: first row of the "up" half inside B (= intermediate size)
   int group_m;       // raster: tiles of this many 256-row blocks share their B columns in time
+  DlogitsParams dl;  // G2_EPI_DLOGITS
 };
 
 // tile index -> (m_blk, n_blk): groups of `G` row blocks sweep all column blocks before the next group starts, so
@@ -231,6 +266,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
       const int row0 = m_blk * G2_BM + (int)cta_rank * G2_BM_CTA + quad * 32;  // first row of this warp's slabs
       const int col_base = n_blk * OUT_BN;
+      DlogitsRow dlr;
+      if constexpr (EPI == G2_EPI_DLOGITS) dlr.load(ep.dl, min(row0 + lane, M - 1));
       // a slab = 32 rows x 128 bytes of C: 64 bf16 or 32 fp32 columns
       const int slab_cols = ep.out_fp32 ? 32 : 64;
 #pragma unroll 1
@@ -256,6 +293,11 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
               const float g = __uint_as_float(r[j]);
               v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
             }
+          } else if constexpr (EPI == G2_EPI_DLOGITS) {
+            tmem_ld_wait();
+            const long long off = dlr.label - (ep.dl.v0 + col_base + cc);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = dlr.of(__uint_as_float(r[j]), ep.dl.inv_temp, (long long)j == off);
           } else {
             tmem_ld_wait();
 #pragma unroll

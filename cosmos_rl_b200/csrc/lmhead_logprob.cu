@@ -9,6 +9,7 @@
 // to a [T, nsplit, 4] fp32 scratch that b200_logprob_combine reduces.
 // Backward: the logits tile is recomputed on the tensor cores and the epilogue emits
 // d(loss)/d(logits) in bf16 for a vocabulary chunk; the two remaining GEMMs are plain ones.
+#include "gemm_2cta_launch.cuh"
 #include "gemm_core.cuh"
 #include "api.h"
 
@@ -145,30 +146,18 @@ __global__ void logprob_combine_kernel(const float* __restrict__ partial, const 
 // ---------------------------------------------------------------------------------------------
 // backward: dlogits chunk
 // ---------------------------------------------------------------------------------------------
+// single-CTA form, for up to 128 rows (the pair form is an epilogue of gemm_2cta.cuh)
 struct DlogitsEpilogue {
   struct Params {
-    const long long* labels;
-    const float* lse;
-    const float* g_lp;
-    const float* g_ent;   // may be null
-    const float* ent;     // may be null
+    DlogitsParams dl;
     __nv_bfloat16* out;
     long long ldd;
-    int T, Vc, v0;
-    float inv_temp;
+    int T, Vc;
   };
-  float lse_r, glp, gent, ent_r;
-  long long label;
+  DlogitsRow st;
   __device__ __forceinline__ void tile_begin(const Params& p, const TileInfo& t, int row) {
-    long long r = (long long)t.m_blk * GEMM_BM + row;
-    if (r < p.T) {
-      lse_r = p.lse[r];
-      glp = p.g_lp[r];
-      gent = p.g_ent ? p.g_ent[r] : 0.f;
-      ent_r = p.ent ? p.ent[r] : 0.f;
-      label = p.labels[r];
-      if (label < 0) { glp = 0.f; }
-    }
+    const long long r = (long long)t.m_blk * GEMM_BM + row;
+    if (r < p.T) st.load(p.dl, r);
   }
   __device__ __forceinline__ void chunk(const Params& p, const TileInfo& t, int row, int col0,
                                         const float (&v)[32]) {
@@ -176,15 +165,9 @@ struct DlogitsEpilogue {
     const int c = t.n_blk * LP_BN + col0;
     if (r >= p.T || c >= p.Vc) return;
     float o[32];
-    const long long off = label - (long long)(p.v0 + c);
+    const long long off = st.label - (long long)(p.dl.v0 + c);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      float x = v[i] * p.inv_temp;
-      float pr = __expf(x - lse_r);
-      float g = -glp * pr - gent * pr * (x - lse_r + ent_r);
-      if ((long long)i == off) g += glp;
-      o[i] = g * p.inv_temp;
-    }
+    for (int i = 0; i < 32; ++i) o[i] = st.of(v[i], p.dl.inv_temp, (long long)i == off);
     __nv_bfloat16* dst = p.out + r * p.ldd + c;
     if (c + 32 <= p.Vc && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
 #pragma unroll
@@ -253,8 +236,16 @@ int b200_lmhead_dlogits(const void* hidden, const void* weight, const long long*
                         float inv_temperature, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (T <= 0 || Vc <= 0 || H <= 0 || (H & 7) || v0 < 0 || v0 + Vc > V) return B200_ERR_ARG;
-  CUtensorMap tmA, tmB;
   const __nv_bfloat16* wchunk = reinterpret_cast<const __nv_bfloat16*>(weight) + (long long)v0 * ldw;
+  const DlogitsParams dl{labels, lse, g_logprob, g_entropy, entropy, v0, inv_temperature};
+  // The logits are formed at the rate of the dense GEMM: CTA pairs once there are rows for their 256-row tiles (2048 x
+  // 16384 x 3584: 147 us against 182 us with one CTA a tile, whose operand traffic bounds it).
+  if (T > 128 && !(reinterpret_cast<uintptr_t>(dlogits) & 15) && !(ldd & 7)) {
+    const Gemm2Params ep{nullptr, 0, 0, 0, 0, 8, dl};
+    return launch_gemm2<256, 6, false, false, G2_EPI_DLOGITS>(hidden, wchunk, dlogits, T, Vc, H, ldh, ldw, ldd, ep, status,
+                                                              num_sms, stream);
+  }
+  CUtensorMap tmA, tmB;
   if (make_tmap_2d(&tmA, hidden, T, H, ldh, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, wchunk, Vc, H, ldw, LP_BN, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   using SM = GemmSmem<LP_BN, LP_STAGES>;
@@ -265,8 +256,7 @@ int b200_lmhead_dlogits(const void* hidden, const void* weight, const long long*
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  DlogitsEpilogue::Params ep{labels, lse, g_logprob, g_entropy, entropy, (__nv_bfloat16*)dlogits, ldd, T, Vc, v0,
-                             inv_temperature};
+  DlogitsEpilogue::Params ep{dl, (__nv_bfloat16*)dlogits, ldd, T, Vc};
   int tiles = ((T + GEMM_BM - 1) / GEMM_BM) * ((Vc + LP_BN - 1) / LP_BN);
   int grid = tiles < num_sms ? tiles : num_sms;
   lmhead_dlogits_kernel<<<grid, GEMM_THREADS, SM::TOTAL, stream>>>(tmA, tmB, T, Vc, H, ep, status);
