@@ -6,10 +6,13 @@
 //
 // The tensor core cannot apply a different fp32 scale per 128-wide slice of K inside one accumulation, so the
 // kernel accumulates in two levels: each 128-deep k-block (four kind::f8f6f4 MMAs of K = 32 on a 128 x 128 tile)
-// goes into one of two TMEM buffers with accumulate = 0; eight promotion warps (two per TMEM lane quadrant, 64
+// goes into one of four TMEM buffers with accumulate = 0; eight promotion warps (two per TMEM lane quadrant, 64
 // columns each) read the finished buffer, multiply by the block's scale product and add into fp32 registers while
-// the tensor core is already filling the other buffer. Operands arrive by TMA (128-byte swizzle, a 128-byte row =
-// 128 fp8 elements) through a 6-stage ring. Persistent CTAs, bounded waits.
+// the tensor core is already filling the others. A k-block is 256 tensor-core cycles and 64 issue slots a scheduler of
+// packed multiply-adds, so what counts is that the promotion's TMEM round trip is off the chain: all of a warp's
+// columns are loaded at once and three further buffers are in flight meanwhile (4096 x 37888 x 3584: 880 us, 892 us with
+// two buffers and two loads; CTA pairs on 256-row tiles measured 1110 us). Operands arrive by TMA (128-byte swizzle, a
+// 128-byte row = 128 fp8 elements) through a 6-stage ring. Persistent CTAs, bounded waits.
 #include "gemm_core.cuh"
 #include "api.h"
 
@@ -17,6 +20,7 @@ namespace b200 {
 
 constexpr int F8_BM = 128, F8_BN = 128, F8_BK = 128;
 constexpr int F8_STAGES = 6;
+constexpr int F8_BUFS = 4;                                   // TMEM accumulators of 128 columns: all 512
 constexpr int F8_STAGE_BYTES = (F8_BM + F8_BN) * F8_BK;     // 32 KiB
 constexpr int F8_SMEM = F8_STAGES * F8_STAGE_BYTES + 256 + 1024;
 constexpr int F8_THREADS = 64 + 256;                         // TMA warp, MMA warp, 8 promotion warps
@@ -30,15 +34,35 @@ struct F8Params {
   uint32_t* status;
 };
 
+// 64 columns of one result row as bf16
+__device__ __forceinline__ void f8_store_row(const F8Params& p, long long row, int col0, const float2 (&acc)[32]) {
+  __nv_bfloat16* dst = p.C + row * p.ldc + col0;
+#pragma unroll
+  for (int c = 0; c < 64; c += 8) {
+    if (col0 + c + 8 <= p.N) {
+      uint4 o;
+      o.x = pack_bf16x2(acc[c / 2].x, acc[c / 2].y);
+      o.y = pack_bf16x2(acc[c / 2 + 1].x, acc[c / 2 + 1].y);
+      o.z = pack_bf16x2(acc[c / 2 + 2].x, acc[c / 2 + 2].y);
+      o.w = pack_bf16x2(acc[c / 2 + 3].x, acc[c / 2 + 3].y);
+      *reinterpret_cast<uint4*>(dst + c) = o;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col0 + c + j < p.N) dst[c + j] = __float2bfloat16(j & 1 ? acc[(c + j) / 2].y : acc[(c + j) / 2].x);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, F8Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + F8_STAGES * F8_STAGE_BYTES);
   uint64_t* empty_bar = full_bar + F8_STAGES;
-  uint64_t* pfull = empty_bar + F8_STAGES;    // [2] partial accumulator ready
-  uint64_t* pempty = pfull + 2;               // [2] partial accumulator consumed (8 warps)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pempty + 2);
+  uint64_t* pfull = empty_bar + F8_STAGES;    // [BUFS] partial accumulator ready
+  uint64_t* pempty = pfull + F8_BUFS;         // [BUFS] partial accumulator consumed (8 warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pempty + F8_BUFS);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -47,7 +71,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < F8_BUFS; ++a) {
       mbar_init(&pfull[a], 1);
       mbar_init(&pempty[a], 8);
     }
@@ -57,7 +81,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     tma_prefetch_desc(&tmB);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 256);
+    tmem_alloc(tmem_slot, F8_BUFS * F8_BN);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -100,7 +124,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       bool ok = true;
       for (int i = blockIdx.x; i < total && ok && !*abort_flag; i += gridDim.x) {
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const uint32_t buf = it & 1, bph = (it >> 1) & 1;
+          const uint32_t buf = it % F8_BUFS, bph = (it / F8_BUFS) & 1;
           if (!mbar_wait(&pempty[buf], bph ^ 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_EMPTY); *abort_flag = 1; ok = false; break; }
           if (!mbar_wait(&full_bar[stage], phase)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_FULL); *abort_flag = 1; ok = false; break; }
           tc_fence_after_sync();
@@ -128,47 +152,47 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const long long grow = (long long)m_blk * F8_BM + row;
       const float* sa_row = p.sa + (grow < p.M ? grow : 0) * p.ldsa;
       const float* sb_row = p.sb + (long long)n_blk * p.ldsb;
-      float acc[64];
+      float2 acc[32];
 #pragma unroll
-      for (int c = 0; c < 64; ++c) acc[c] = 0.f;
-      float s_next = sa_row[0] * sb_row[0];
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
-        const uint32_t buf = it & 1, bph = (it >> 1) & 1;
-        const float s = s_next;
-        if (kb + 1 < num_kb) s_next = sa_row[kb + 1] * sb_row[kb + 1];
-        if (!mbar_wait(&pfull[buf], bph)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after_sync();
+      for (int c = 0; c < 32; ++c) acc[c] = make_float2(0.f, 0.f);
+      // the scales of four k-blocks are fetched four k-blocks ahead (a round trip to L2 is longer than one k-block)
+      float nxt[4];
+      auto fetch = [&](int kb) {
 #pragma unroll
-        for (int c = 0; c < 64; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(tmem_base + buf * F8_BN + lane_addr + chalf * 64 + c, r);
+        for (int u = 0; u < 4; ++u) nxt[u] = kb + u < num_kb ? sa_row[kb + u] * sb_row[kb + u] : 0.f;
+      };
+      fetch(0);
+      for (int kb0 = 0; kb0 < num_kb && ok; kb0 += 4) {
+        float cur[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
+        fetch(kb0 + 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (kb0 + u >= num_kb) break;
+          const uint32_t buf = it % F8_BUFS, bph = (it / F8_BUFS) & 1;
+          ++it;
+          if (!mbar_wait(&pfull[buf], bph)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_TMEM_FULL); *abort_flag = 1; ok = false; }
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after_sync();
+          uint32_t r[2][32];
+          tmem_ld_32x32b_x32(tmem_base + buf * F8_BN + lane_addr + chalf * 64, r[0]);
+          tmem_ld_32x32b_x32(tmem_base + buf * F8_BN + lane_addr + chalf * 64 + 32, r[1]);
           tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&pempty[buf]);   // the values are in registers
+          const float2 s = make_float2(cur[u], cur[u]);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[c + j] = fmaf(s, __uint_as_float(r[j]), acc[c + j]);
+          for (int c = 0; c < 32; ++c)
+            acc[c] = fma2(s, make_float2(__uint_as_float(r[c >> 4][2 * (c & 15)]), __uint_as_float(r[c >> 4][2 * (c & 15) + 1])),
+                          acc[c]);
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&pempty[buf]);
       }
       if (!ok) break;
       if (grow < p.M) {
-        const int col0 = n_blk * F8_BN + chalf * 64;
-        __nv_bfloat16* dst = p.C + grow * p.ldc + col0;
-#pragma unroll
-        for (int c = 0; c < 64; c += 8) {
-          if (col0 + c + 8 <= p.N) {
-            uint4 o;
-            o.x = pack_bf16x2(acc[c], acc[c + 1]);
-            o.y = pack_bf16x2(acc[c + 2], acc[c + 3]);
-            o.z = pack_bf16x2(acc[c + 4], acc[c + 5]);
-            o.w = pack_bf16x2(acc[c + 6], acc[c + 7]);
-            *reinterpret_cast<uint4*>(dst + c) = o;
-          } else {
-            for (int j = 0; j < 8 && col0 + c + j < p.N; ++j) dst[c + j] = __float2bfloat16(acc[c + j]);
-          }
-        }
+        f8_store_row(p, grow, n_blk * F8_BN + chalf * 64, acc);
       }
     }
   }
@@ -181,7 +205,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, F8_BUFS * F8_BN);
   }
 }
 

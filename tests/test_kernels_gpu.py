@@ -63,6 +63,21 @@ def test_fused_logprob_fwd_bwd(T, V, H, temp):
     assert torch.allclose(w.grad.float(), wr.grad, rtol=5e-2, atol=5e-2 * wr.grad.abs().max().item())
 
 
+@pytest.mark.parametrize("R_,C,off", [(1, 128, 0), (3, 200, 0), (17, 1032, 0), (5, 130, 1), (65, 4096, 0)])
+def test_quant_fp8_rows_match_reference_bit_for_bit(R_, C, off):
+    """Ragged last blocks, and rows that start off the 16-byte grid."""
+    torch.manual_seed(37)
+    w = _bf16(R_, C + off + 7)[:, off:off + C]
+    q, s = F.quant_fp8_block(w, 1)
+    nb = (C + 127) // 128
+    pad = torch.zeros(R_, nb * 128, device=DEV)
+    pad[:, :C] = w.float()
+    scale = pad.view(R_, nb, 128).abs().amax(-1).clamp_min(1e-12) / torch.tensor(448.0, device=DEV)
+    assert torch.equal(s, scale)
+    want = (pad.view(R_, nb, 128) * (1.0 / scale)[:, :, None]).view(R_, -1)[:, :C].to(torch.float8_e4m3fn)
+    assert torch.equal(q.view(torch.uint8), want.view(torch.uint8))
+
+
 @pytest.mark.parametrize("T,H", [(33, 256), (1000, 3584), (64, 8192)])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_rmsnorm(T, H, with_res):
