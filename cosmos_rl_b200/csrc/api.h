@@ -44,6 +44,10 @@ int b200_gemm_skinny_splits(int M, int N, int K, int swiglu, int num_sms);
 int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, int N, int K, long long ldx,
                      long long ldw, long long ldo, const void* bias, int bias_bf16, int swiglu, int up_row0,
                      int splits, uint32_t* status, int num_sms, cudaStream_t stream);
+// out [M, N] bf16 = x W^T (+ bias): chooses the split and reduces it in the same call
+int b200_skinny_linear(const void* x, const void* W, const void* bias, int bias_bf16, void* out, float* ws,
+                       long long ws_floats, int M, int N, int K, long long ldx, long long ldw, long long ldo,
+                       uint32_t* status, int num_sms, cudaStream_t stream);
 int b200_splitk_reduce(const float* ws, int splits, int M, int N, const void* bias, int bias_bf16, void* out,
                        long long ldo, cudaStream_t stream);
 // res_out = sum(ws) (+ res_in);  y = rmsnorm(res_out) * w   (bf16 rows of H <= 8192 values)

@@ -595,6 +595,19 @@ int b200_splitk_reduce(const float* ws, int splits, int M, int N, const void* bi
                           (__nv_bfloat16*)out, ldo) == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 
+// y [M, N] bf16 = x W^T (+ bias) in one call: the split is chosen here and reduced when there is one. ws: fp32 scratch of
+// ws_floats elements (splits * M * N are used).
+int b200_skinny_linear(const void* x, const void* W, const void* bias, int bias_bf16, void* out, float* ws,
+                       long long ws_floats, int M, int N, int K, long long ldx, long long ldw, long long ldo,
+                       uint32_t* status, int num_sms, cudaStream_t stream) {
+  const int splits = b200_gemm_skinny_splits(M, N, K, 0, num_sms);
+  if (splits == 1)
+    return b200_gemm_skinny(x, W, out, nullptr, M, N, K, ldx, ldw, ldo, bias, bias_bf16, 0, 0, 1, status, num_sms, stream);
+  if ((long long)splits * M * N > ws_floats) return B200_ERR_TOO_LARGE;
+  const int rc = b200_gemm_skinny(x, W, nullptr, ws, M, N, K, ldx, ldw, 0, nullptr, 0, 0, 0, splits, status, num_sms, stream);
+  return rc ? rc : b200_splitk_reduce(ws, splits, M, N, bias, bias_bf16, out, ldo, stream);
+}
+
 int b200_splitk_reduce_residual_rmsnorm(const float* ws, int splits, int M, int H, const void* res_in, const void* w,
                                         float eps, void* res_out, void* y, cudaStream_t stream) {
   using namespace b200;

@@ -406,14 +406,19 @@ def _skinny_launch(x2, weight, N, swiglu, out, use_ws, bias=None):
 def gemm_skinny(x2: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x2 [M <= 256, K] @ weight [N, K]^T (+ bias)`` in bf16 on the weight-streaming kernel."""
-    M, N = x2.shape[0], weight.shape[0]
+    (M, K), N = x2.shape, weight.shape[0]
+    assert x2.is_cuda and x2.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and M <= _SKINNY_MAX_M
+    assert x2.stride(-1) == 1 and weight.stride(-1) == 1
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x2.device)
-    ws, splits = _skinny_launch(x2, weight, N, False, out, False, bias)
-    if ws is not None:
-        native.check(native.lib().b200_splitk_reduce(native.ptr(ws), splits, M, N, native.ptr(bias),
-                                                     1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
-                                                     native.ptr(out), out.stride(0), native.stream()), "splitk_reduce")
+    dev, strm = x2.device.index, native.stream()
+    ws = _skinny_workspace(x2.device)
+    native.check(native.lib().b200_skinny_linear(x2.data_ptr(), weight.data_ptr(), native.ptr(bias),
+                                                 1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
+                                                 out.data_ptr(), ws.data_ptr(), _SKINNY_WS_FLOATS, M, N, K,
+                                                 x2.stride(0), weight.stride(0), out.stride(0),
+                                                 native.status_word(x2.device).data_ptr(), native.num_sms(dev), strm),
+                 "gemm_skinny")
     return out
 
 

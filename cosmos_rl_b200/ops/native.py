@@ -57,6 +57,8 @@ _SIGS = {
     "b200_gemm_skinny_splits": [c_int, c_int, c_int, c_int, c_int],
     "b200_gemm_skinny": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                          c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
+    "b200_skinny_linear": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int,
+                           c_longlong, c_longlong, c_longlong, c_void_p, c_int, c_void_p],
     "b200_splitk_reduce": [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_longlong, c_void_p],
     "b200_splitk_reduce_residual_rmsnorm": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p,
                                             c_void_p, c_void_p],
