@@ -3,7 +3,9 @@
 // Two kernels, each owning its outputs, so nothing is accumulated through memory (no fp32 dQ buffer, no atomics, the
 // same bits on every run):
 //
-//   dQ     one CTA = (sequence, 128-query block, query head); loops over the 128-key blocks it can see
+//   dQ     one item = (sequence, 128-query block, query head); loops over the 128-key blocks it can see. One CTA per SM
+//          works through items (flash_sched.cuh): loads and the first products of the next one run under the end of this
+//          one.
 //          S  = Q K^T          M=queries N=keys K=d        TMEM S[j&1]
 //          dP = dO V^T         M=queries N=keys K=d        TMEM dP
 //          dS = exp2(S c - lse) o (dP - delta)             softmax warps, bf16 into the columns of dP
@@ -28,6 +30,7 @@
 // each). All waits are bounded; on a timeout a status code is recorded and the CTA leaves with its TMEM freed.
 // Replaces flash_attn's varlen backward (cosmos_rl/policy/kernel/modeling_utils.py:65-173).
 #include "sm100.cuh"
+#include "flash_sched.cuh"
 #include "gemm_core.cuh"
 #include "api.h"
 
@@ -37,7 +40,9 @@ constexpr int FB_B = 128;                            // queries / keys per block
 constexpr int FB_D = 128;
 constexpr int FB_TILE = FB_B * FB_D * 2;             // 32 KiB, two boxes of 128 rows x 64 elements
 constexpr int FB_STATS = 2 * 2 * FB_B * 4;           // dK/dV kernel: lse and delta of two query blocks
-constexpr int FB_SMEM = 6 * FB_TILE + FB_STATS + 256 + 1024;
+constexpr int FB_SMEM = 6 * FB_TILE + FB_STATS + 256 + 1024;          // dK/dV kernel
+constexpr int FB_OUT_BYTES = 8 * 4096;                                // dQ kernel: epilogue staging, 4 KB a warp
+constexpr int FB_SMEM_DQ = 6 * FB_TILE + FB_OUT_BYTES + 512 + 1024;
 constexpr int FB_THREADS = 320;                      // TMA warp, MMA warp, 8 softmax warps
 constexpr float FB_LOG2E = 1.4426950408889634f;
 
@@ -53,6 +58,7 @@ struct FbParams {
   __nv_bfloat16* dv;
   long long ldo, lddo, lddq, lddk, lddv;  // token strides (elements)
   int B, hq, hkv, Tq, causal;
+  int levels_q;                // 128-query blocks of the longest sequence
   float scale, scale_log2;
   uint32_t* status;
 };
@@ -91,8 +97,8 @@ __device__ __forceinline__ void fb_mma_ss(uint32_t tmem_d, uint32_t a, uint32_t 
   }
 }
 
-// D[128, 128] += A[128, 128] * B[128, 128] with A in TMEM (contraction elements 0..63 in columns [0, 32), 64..127 in
-// columns [64, 96)) and B a shared-memory tile whose rows are the contraction index
+// D[128, 128] += A[128, 128] * B[128, 128] with A in TMEM (contraction elements 0..63 as bf16 pairs in columns [0, 32),
+// 64..127 in columns [64, 96)) and B a shared-memory tile whose rows are the contraction index
 __device__ __forceinline__ void fb_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, bool first) {
   constexpr uint32_t idesc = umma_idesc_bf16_f32(128, 128) | (1u << 16);
 #pragma unroll
@@ -101,92 +107,95 @@ __device__ __forceinline__ void fb_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint
                  (first && k == 0) ? 0u : 1u);
 }
 
-// 64 fp32 columns of this thread's accumulator row (+ `add`, one float every 128), times `mul`, as bf16 to global memory
-__device__ __forceinline__ void fb_store_row(uint32_t taddr, bool zero, float mul, __nv_bfloat16* dst, bool live,
-                                             const float* add = nullptr) {
-#pragma unroll 1
-  for (int c = 0; c < 64; c += 32) {
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(taddr + c, r);
-    tmem_ld_wait();
-    float v[32];
+// 64 fp32 accumulator columns of the warp's 32 rows (+ `add`, this thread's row, one float every 128), times `mul`, as bf16
+// to global memory: through 4 KB of shared memory, so that the warp writes whole 128-byte lines. `live`: rows to write.
+__device__ __forceinline__ void fb_store_rows(uint32_t taddr, bool zero, float mul, uint8_t* stage, __nv_bfloat16* dst,
+                                              long long ld, int live, const float* add = nullptr) {
+  const int lane = threadIdx.x & 31;
+  uint32_t r[2][32];
+  tmem_ld_32x32b_x32(taddr, r[0]);
+  tmem_ld_32x32b_x32(taddr + 32, r[1]);
+  tmem_ld_wait();
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = zero ? 0.f : __uint_as_float(r[j]);
-    if (add) {
+  for (int g = 0; g < 8; ++g) {
+    uint32_t o[4];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] += add[(c + j) * FB_B];
-    }
-    if (live) {
+    for (int j = 0; j < 4; ++j) {
+      float v[2];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(v[8 * g + 2 * j] * mul, v[8 * g + 2 * j + 1] * mul);
-        *reinterpret_cast<uint4*>(dst + c + 8 * g) = make_uint4(o[0], o[1], o[2], o[3]);
+      for (int u = 0; u < 2; ++u) {
+        const int c = 8 * g + 2 * j + u;
+        v[u] = zero ? 0.f : __uint_as_float(r[c >> 5][c & 31]);
+        if (add) v[u] += add[c * FB_B];
       }
+      o[j] = pack_bf16x2(v[0] * mul, v[1] * mul);
     }
+    *reinterpret_cast<uint4*>(stage + lane * 128 + ((g ^ (lane & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
   }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {   // four rows a step, eight lanes each
+    const int rr = 4 * i + (lane >> 3), g = lane & 7;
+    const uint4 o = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((g ^ (rr & 7)) << 4));
+    if (rr < live) *reinterpret_cast<uint4*>(dst + rr * ld + 8 * g) = o;
+  }
+  __syncwarp();                   // before the staging rows are written again
 }
 
 // ---------------------------------------------------------------------------------------------------------------
 // dQ (and delta)
 // ---------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ int fb_key_blocks(const FlashItem& w, int causal) {
+  const int end = causal ? min(w.len_k, w.row0 + FB_B + w.len_k - w.len_q) : w.len_k;
+  return end > 0 ? (end + FB_B - 1) / FB_B : 0;
+}
+
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, FbParams p) {
-  const int heads = p.hq * p.B, nblk = gridDim.x / heads;
-  const int hb = blockIdx.x % heads, h = hb % p.hq, b = hb / p.hq;
-  const int qb = nblk - 1 - blockIdx.x / heads;        // under the causal mask late query blocks see most keys: first
-  const int q_beg = p.cu_q[b], len_q = p.cu_q[b + 1] - q_beg;
-  const int k_beg = p.cu_k[b], len_k = p.cu_k[b + 1] - k_beg;
-  const int q0 = qb * FB_B;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (qb == 0) {
-    // tokens outside every sequence have no gradient
-    const int head = b == 0 ? q_beg : 0, tail = b == p.B - 1 ? p.cu_q[p.B] : p.Tq;
-    for (int t = warp; t < head; t += FB_THREADS / 32)
-      *reinterpret_cast<uint2*>(p.dq + (long long)t * p.lddq + h * FB_D + lane * 4) = make_uint2(0u, 0u);
-    for (int t = tail + warp; t < p.Tq; t += FB_THREADS / 32)
-      *reinterpret_cast<uint2*>(p.dq + (long long)t * p.lddq + h * FB_D + lane * 4) = make_uint2(0u, 0u);
-  }
-  if (q0 >= len_q) return;
-  const int shift = len_k - len_q;
-  int kv_end = p.causal ? min(len_k, q0 + FB_B + shift) : len_k;
-  if (kv_end < 0) kv_end = 0;
-  const int n = (kv_end + FB_B - 1) / FB_B;
-  const int hk = h / (p.hq / p.hkv);
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_sh = smem;
   uint8_t* do_sh = smem + FB_TILE;
   uint8_t* k_sh = smem + 2 * FB_TILE;                  // [2]
   uint8_t* v_sh = smem + 4 * FB_TILE;                  // [2]
-  float* delta_sh = reinterpret_cast<float*>(smem + 6 * FB_TILE);   // [128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * FB_TILE + FB_STATS);
+  uint8_t* out_sh = smem + 6 * FB_TILE;                // [8 warps][32 rows][128 bytes]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_sh + FB_OUT_BYTES);
   uint64_t* q_full = bars;
-  uint64_t* do_full = bars + 1;
-  uint64_t* k_full = bars + 2;     // [2]
-  uint64_t* v_full = bars + 4;     // [2]
-  uint64_t* k_empty = bars + 6;    // [2]
-  uint64_t* v_empty = bars + 8;    // [2]
-  uint64_t* s_ready = bars + 10;   // [2]
-  uint64_t* dp_ready = bars + 12;
-  uint64_t* ds_ready = bars + 13;
-  uint64_t* done = bars + 14;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* q_empty = bars + 1;
+  uint64_t* do_full = bars + 2;
+  uint64_t* do_empty = bars + 3;
+  uint64_t* k_full = bars + 4;     // [2]
+  uint64_t* v_full = bars + 6;     // [2]
+  uint64_t* k_empty = bars + 8;    // [2]
+  uint64_t* v_empty = bars + 10;   // [2]
+  uint64_t* s_ready = bars + 12;   // [2]
+  uint64_t* dp_ready = bars + 14;
+  uint64_t* ds_ready = bars + 15;
+  uint64_t* done = bars + 16;
+  uint64_t* item_full = bars + 17;   // [2] slots of the work queue
+  uint64_t* item_empty = bars + 19;  // [2] read by the MMA thread and the eight softmax warps
+  FlashItem* items = reinterpret_cast<FlashItem*>(bars + 22);   // [2]
+  // bars + 30: 16 bytes and bars + 21: barrier of cluster launch control
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
+    mbar_init(q_empty, 1);
     mbar_init(do_full, 1);
+    mbar_init(do_empty, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&k_full[s], 1);
       mbar_init(&v_full[s], 1);
       mbar_init(&k_empty[s], 1);
       mbar_init(&v_empty[s], 1);
       mbar_init(&s_ready[s], 1);
+      mbar_init(&item_full[s], 1);
+      mbar_init(&item_empty[s], 9);
     }
+    mbar_init(bars + 21, 1);
     mbar_init(dp_ready, 1);
     mbar_init(ds_ready, 8);
     mbar_init(done, 1);
@@ -209,170 +218,235 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t tm_dp = tmem_base + 256, tm_dq = tmem_base + 384;
 
   if (warp == 0) {
-    if (lane == 0 && n > 0) {
-      do {
-        mbar_arrive_expect_tx(q_full, FB_TILE);
-        fb_load_tile(q_sh, &tm_q, q_full, h * FB_D, q_beg + q0);
-        for (int j = 0; j < n && !*abort_flag; ++j) {
-          const int s = j & 1, row = k_beg + j * FB_B;
-          const uint32_t ph = ((j >> 1) & 1) ^ 1;
-          FB_WAIT1(&k_empty[s], ph, ST_TIMEOUT_EMPTY)
-          mbar_arrive_expect_tx(&k_full[s], FB_TILE);
-          fb_load_tile(k_sh + s * FB_TILE, &tm_k, &k_full[s], hk * FB_D, row);
-          if (j == 0) {
-            mbar_arrive_expect_tx(do_full, FB_TILE);
-            fb_load_tile(do_sh, &tm_do, do_full, h * FB_D, q_beg + q0);
-          }
-          FB_WAIT1(&v_empty[s], ph, ST_TIMEOUT_EMPTY)
-          mbar_arrive_expect_tx(&v_full[s], FB_TILE);
-          fb_load_tile(v_sh + s * FB_TILE, &tm_v, &v_full[s], hk * FB_D, row);
+    // ---- scheduler and TMA producer (whole warp, lane 0 issues)
+    FlashWork work;
+    work.list.init(p.cu_q, p.B, FB_B, p.hq, p.levels_q, !p.causal);
+    work.init(reinterpret_cast<uint4*>(bars + 30), bars + 21);
+    uint32_t kv = 0, nq = 0;   // key blocks and Q tiles so far
+    bool ok = true;
+    auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
+      if (lane == 0) {
+        mbar_arrive_expect_tx(bar, FB_TILE);
+        fb_load_tile(dst, tm, bar, col, row);
+      }
+    };
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return fb_wait(bar, parity, ST_TIMEOUT_EMPTY, p.status, abort_flag); };
+    for (uint32_t it = 0; ok; ++it) {
+      const uint32_t slot = it & 1;
+      FlashItem w;
+      int block = 0;
+      w.head = w.b = 0;
+      w.valid = work.next(w.b, block, w.head);
+      if (w.valid < 0) {
+        atomicCAS(p.status, ST_OK, ST_TIMEOUT_EMPTY);
+        *abort_flag = 1;
+        break;
+      }
+      w.q_beg = w.len_q = w.k_beg = w.len_k = w.row0 = 0;
+      if (w.valid) {
+        w.q_beg = p.cu_q[w.b];
+        w.len_q = p.cu_q[w.b + 1] - w.q_beg;
+        w.k_beg = p.cu_k[w.b];
+        w.len_k = p.cu_k[w.b + 1] - w.k_beg;
+        w.row0 = block * FB_B;
+      }
+      if (!(ok = wait(&item_empty[slot], ((it >> 1) & 1) ^ 1))) break;
+      if (lane == 0) {
+        items[slot] = w;
+        mbar_arrive(&item_full[slot]);
+      }
+      if (!w.valid) break;
+      const int n = fb_key_blocks(w, p.causal), hk = w.head / (p.hq / p.hkv), qrow = w.q_beg + w.row0;
+      for (int j = 0; j < n; ++j, ++kv) {
+        if (j + 2 >= n) work.request();   // the answer comes while the last blocks wait for their buffers
+        const uint32_t s = kv & 1, ph = ((kv >> 1) & 1) ^ 1;
+        const int row = w.k_beg + j * FB_B;
+        if (j == 0) {
+          if (!(ok = wait(q_empty, (nq & 1) ^ 1))) break;
+          load(q_sh, &tm_q, q_full, w.head * FB_D, qrow);
         }
-      } while (false);
+        if (!(ok = wait(&k_empty[s], ph))) break;
+        load(k_sh + s * FB_TILE, &tm_k, &k_full[s], hk * FB_D, row);
+        if (j == 0) {
+          if (!(ok = wait(do_empty, (nq & 1) ^ 1))) break;
+          load(do_sh, &tm_do, do_full, w.head * FB_D, qrow);
+          ++nq;
+        }
+        if (!(ok = wait(&v_empty[s], ph))) break;
+        load(v_sh + s * FB_TILE, &tm_v, &v_full[s], hk * FB_D, row);
+      }
+    }
+    work.finish();
+    // the tensor core's last arrivals on these barriers land before the CTA's shared memory is released
+    if (ok) ok = wait(q_empty, (nq & 1) ^ 1) && wait(do_empty, (nq & 1) ^ 1);
+    for (int i = 0; i < 2 && ok; ++i, ++kv) {
+      const uint32_t s = kv & 1, ph = ((kv >> 1) & 1) ^ 1;
+      ok = wait(&k_empty[s], ph) && wait(&v_empty[s], ph);
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (lane == 0) {
       const uint32_t q_a = smem_u32(q_sh), do_a = smem_u32(do_sh);
-      do {
-        FB_WAIT1(q_full, 0, ST_TIMEOUT_FULL)
-        FB_WAIT1(&k_full[0], 0, ST_TIMEOUT_FULL)
+      uint32_t kv = 0, nq = 0;
+      for (uint32_t it = 0; !*abort_flag; ++it) {
+        const uint32_t slot = it & 1;
+        FB_WAIT1(&item_full[slot], (it >> 1) & 1, ST_TIMEOUT_FULL)
+        const FlashItem w = items[slot];
+        mbar_arrive(&item_empty[slot]);
+        if (!w.valid) break;
+        const int n = fb_key_blocks(w, p.causal);
+        if (n == 0) continue;
+        FB_WAIT1(q_full, nq & 1, ST_TIMEOUT_FULL)
+        FB_WAIT1(&k_full[kv & 1], (kv >> 1) & 1, ST_TIMEOUT_FULL)
         tc_fence_after_sync();
-        fb_mma_ss(tmem_base, q_a, smem_u32(k_sh));
-        tc_commit(&s_ready[0]);
-        FB_WAIT1(do_full, 0, ST_TIMEOUT_FULL)
-        FB_WAIT1(&v_full[0], 0, ST_TIMEOUT_FULL)
+        fb_mma_ss(tmem_base + (kv & 1) * 128, q_a, smem_u32(k_sh + (kv & 1) * FB_TILE));
+        tc_commit(&s_ready[kv & 1]);
+        if (n == 1) tc_commit(q_empty);
+        FB_WAIT1(do_full, nq & 1, ST_TIMEOUT_FULL)
+        FB_WAIT1(&v_full[kv & 1], (kv >> 1) & 1, ST_TIMEOUT_FULL)
+        ++nq;
         tc_fence_after_sync();
-        fb_mma_ss(tm_dp, do_a, smem_u32(v_sh));
+        fb_mma_ss(tm_dp, do_a, smem_u32(v_sh + (kv & 1) * FB_TILE));
         tc_commit(dp_ready);
-        tc_commit(&v_empty[0]);
-        for (int j = 0; j < n; ++j) {
-          const int s = j & 1, s1 = s ^ 1;
-          const uint32_t ph1 = ((j + 1) >> 1) & 1;
-          if (j + 1 < n) {   // S of the next block: its buffer was read before dS(j-1) was announced
+        tc_commit(&v_empty[kv & 1]);
+        if (n == 1) tc_commit(do_empty);
+        for (int j = 0; j < n && !*abort_flag; ++j, ++kv) {
+          const uint32_t s = kv & 1, s1 = s ^ 1, ph1 = ((kv + 1) >> 1) & 1;
+          const uint32_t k_a = smem_u32(k_sh + s * FB_TILE);
+          if (j + 1 < n) {   // S of the next block: its buffer was read before dS of the block before this one was announced
             FB_WAIT1(&k_full[s1], ph1, ST_TIMEOUT_FULL)
             tc_fence_after_sync();
             fb_mma_ss(tmem_base + s1 * 128, q_a, smem_u32(k_sh + s1 * FB_TILE));
             tc_commit(&s_ready[s1]);
+            if (j + 2 == n) tc_commit(q_empty);
           }
-          FB_WAIT1(ds_ready, j & 1, ST_TIMEOUT_TMEM_EMPTY)
+          // dS also says that the previous item's dQ has been read, which the first product of an item overwrites
+          FB_WAIT1(ds_ready, kv & 1, ST_TIMEOUT_TMEM_EMPTY)
           tc_fence_after_sync();
-          fb_mma_ts(tm_dq, tm_dp, smem_u32(k_sh + s * FB_TILE), j == 0);
+          fb_mma_ts(tm_dq, tm_dp, k_a, j == 0);
           tc_commit(&k_empty[s]);
           if (j + 1 < n) {
             FB_WAIT1(&v_full[s1], ph1, ST_TIMEOUT_FULL)
             tc_fence_after_sync();
-            fb_mma_ss(tm_dp, do_a, smem_u32(v_sh + s1 * FB_TILE));
+            fb_mma_ss(tm_dp, do_a, smem_u32(v_sh + s1 * FB_TILE));   // dP of the next block, over dS
             tc_commit(dp_ready);
             tc_commit(&v_empty[s1]);
+            if (j + 2 == n) tc_commit(do_empty);
           }
         }
         if (!*abort_flag) tc_commit(done);
-      } while (false);
+      }
     }
   } else {
     const int quad = warp & 3;
-    const int c0 = ((warp - 2) >> 2) * 64;               // first key column of this warp
+    const int half_id = (warp - 2) >> 2;
+    const int c0 = half_id * 64;                         // first key column of this warp
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    const int q_idx = q0 + row;
-    const bool live = q_idx < len_q;
-    const int k_limit = p.causal ? min(len_k, q_idx + shift + 1) : len_k;   // keys [0, k_limit) are visible
-    // delta of 16 of the quadrant's 32 rows per warp: a row is one coalesced 256-byte read of O and of dO, and the sixteen
-    // sums are reduced together (each shuffle step halves the rows that a lane carries)
-    {
-      float v[16];
-      uint2 o2[16], g2[16];
-      const int half = (warp - 2) >> 2;
-      // rows past the end are read at the last row and dropped: no branch keeps the 32 loads apart
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const long long t = q_beg + min(q0 + quad * 32 + half * 16 + i, len_q - 1);
-        o2[i] = *reinterpret_cast<const uint2*>(p.out + t * p.ldo + h * FB_D + lane * 4);
-        g2[i] = *reinterpret_cast<const uint2*>(p.dout + t * p.lddo + h * FB_D + lane * 4);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].x));
-        const float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].y));
-        const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].x));
-        const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].y));
-        v[i] = (x0.x * y0.x + x0.y * y0.y) + (x1.x * y1.x + x1.y * y1.y);
-      }
-#pragma unroll
-      for (int w = 8; w > 0; w >>= 1) {   // lane distance 2 w: w rows stay with each lane
-        const bool hi = lane & (2 * w);
-#pragma unroll
-        for (int i = 0; i < w; ++i) {
-          const float send = hi ? v[i] : v[i + w], keep = hi ? v[i + w] : v[i];
-          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * w);
-        }
-      }
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-      const int r = half * 16 + (lane >> 1), qi = q0 + quad * 32 + r;
-      if ((lane & 1) == 0) {
-        delta_sh[quad * 32 + r] = qi < len_q ? v[0] : 0.f;
-        if (qi < len_q) p.delta[(long long)h * p.Tq + q_beg + qi] = v[0];
-      }
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");   // the two warps of this quadrant
-    }
-    const float delta = delta_sh[row];
-    const float nlse = live ? -p.lse[(long long)h * p.Tq + q_beg + q_idx] * FB_LOG2E : -INFINITY;
-    const float2 c2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(nlse, nlse);
-    const float2 nd2 = make_float2(-delta, -delta);
+    uint8_t* stage = out_sh + (warp - 2) * 4096;
+    const float2 c2 = make_float2(p.scale_log2, p.scale_log2);
+    uint32_t kv = 0, finished = 0;
     bool ok = true;
-    for (int j = 0; j < n; ++j) {
-      const int s = j & 1;
-      if (!(ok = fb_wait(&s_ready[s], (j >> 1) & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
-      tc_fence_after_sync();
-      float2 e[32];
-      const int key0 = j * FB_B + c0;
-      const bool need_mask = key0 + 64 > k_limit;
-      uint32_t rs[2][32];
-      tmem_ld_32x32b_x32(tmem_base + s * 128 + lane_addr + c0, rs[0]);
-      tmem_ld_32x32b_x32(tmem_base + s * 128 + lane_addr + c0 + 32, rs[1]);
-      tmem_ld_wait();
+    for (uint32_t it = 0; ok; ++it) {
+      const uint32_t slot = it & 1;
+      if (!(ok = fb_wait(&item_full[slot], (it >> 1) & 1, ST_TIMEOUT_FULL, p.status, abort_flag))) break;
+      const FlashItem& w = items[slot];                  // read where it is needed: registers are short in the loop
+      if (!w.valid) break;
+      const int n = fb_key_blocks(w, p.causal);
+      const int q_idx = w.row0 + row;
+      const bool live = q_idx < w.len_q;
+      const int k_limit = p.causal ? min(w.len_k, q_idx + w.len_k - w.len_q + 1) : w.len_k;   // keys [0, k_limit) are visible
+      const long long at = (long long)w.head * p.Tq + w.q_beg + q_idx;
+      const float nlse = live ? -p.lse[at] * FB_LOG2E : -INFINITY;
+      // delta of the quadrant's 32 rows: a row is one coalesced 256-byte read of O and of dO; the sums of 32 rows are
+      // reduced together (each shuffle step halves the rows that a lane carries) and row r ends up in lane r. Rows past
+      // the end are read at the last row and dropped: no branch keeps the loads apart.
+      float delta;
+      {
+        float v[32];
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const uint32_t(&r)[32] = rs[half];
+        for (int i0 = 0; i0 < 32; i0 += 16) {
+          uint2 o2[16], g2[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float2 x = fma2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), c2, nl2);
-          e[half * 16 + i] = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+          for (int i = 0; i < 16; ++i) {
+            const long long t = w.q_beg + min(w.row0 + quad * 32 + i0 + i, w.len_q - 1);
+            o2[i] = *reinterpret_cast<const uint2*>(p.out + t * p.ldo + w.head * FB_D + lane * 4);
+            g2[i] = *reinterpret_cast<const uint2*>(p.dout + t * p.lddo + w.head * FB_D + lane * 4);
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].x));
+            const float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].y));
+            const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].x));
+            const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].y));
+            v[i0 + i] = (x0.x * y0.x + x0.y * y0.y) + (x1.x * y1.x + x1.y * y1.y);
+          }
         }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {   // lane distance d: d rows stay with each lane
+          const bool hi = lane & d;
+#pragma unroll
+          for (int i = 0; i < d; ++i) {
+            const float send = hi ? v[i] : v[i + d], keep = hi ? v[i + d] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+          }
+        }
+        delta = v[0];
       }
-      if (need_mask) {
+      if (live && half_id == 0) p.delta[at] = delta;
+      const float2 nl2 = make_float2(nlse, nlse), nd2 = make_float2(-delta, -delta);
+      for (int j = 0; j < n; ++j, ++kv) {
+        const uint32_t s = kv & 1;
+        if (!(ok = fb_wait(&s_ready[s], (kv >> 1) & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+        tc_fence_after_sync();
+        float2 e[32];
+        const int key0 = j * FB_B + c0;
+        uint32_t rs[2][32];
+        tmem_ld_32x32b_x32(tmem_base + s * 128 + lane_addr + c0, rs[0]);
+        tmem_ld_32x32b_x32(tmem_base + s * 128 + lane_addr + c0 + 32, rs[1]);
+        tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          if (key0 + 2 * i >= k_limit) e[i].x = 0.f;
-          if (key0 + 2 * i + 1 >= k_limit) e[i].y = 0.f;
+          const uint32_t(&r)[32] = rs[i >> 4];
+          const float2 x = fma2(make_float2(__uint_as_float(r[2 * (i & 15)]), __uint_as_float(r[2 * (i & 15) + 1])), c2, nl2);
+          e[i] = make_float2(exp2_approx(x.x), exp2_approx(x.y));
         }
-      }
-      if (!(ok = fb_wait(dp_ready, j & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
-      tc_fence_after_sync();
-      uint32_t ds[32];
-      uint32_t rp[2][32];
-      tmem_ld_32x32b_x32(tm_dp + lane_addr + c0, rp[0]);
-      tmem_ld_32x32b_x32(tm_dp + lane_addr + c0 + 32, rp[1]);
-      tmem_ld_wait();
+        if (key0 + 64 > k_limit) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const uint32_t(&r)[32] = rp[half];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float2 v = mul2(e[half * 16 + i],
-                                add2(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), nd2));
-          ds[half * 16 + i] = pack_bf16x2(v.x, v.y);
+          for (int i = 0; i < 32; ++i) {
+            if (key0 + 2 * i >= k_limit) e[i].x = 0.f;
+            if (key0 + 2 * i + 1 >= k_limit) e[i].y = 0.f;
+          }
         }
+        if (!(ok = fb_wait(dp_ready, kv & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+        tc_fence_after_sync();
+        uint32_t ds[32], rp[2][32];
+        tmem_ld_32x32b_x32(tm_dp + lane_addr + c0, rp[0]);
+        tmem_ld_32x32b_x32(tm_dp + lane_addr + c0 + 32, rp[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const uint32_t(&r)[32] = rp[i >> 4];
+          const float2 v = mul2(e[i], add2(make_float2(__uint_as_float(r[2 * (i & 15)]), __uint_as_float(r[2 * (i & 15) + 1])), nd2));
+          ds[i] = pack_bf16x2(v.x, v.y);
+        }
+        tmem_st_32x32b_x32(tm_dp + lane_addr + c0, ds);   // over the first half of the columns just read
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ds_ready);
       }
-      tmem_st_32x32b_x32(tm_dp + lane_addr + c0, ds);   // over the first half of the columns just read
-      tmem_st_wait();
-      tc_fence_before_sync();
+      if (!ok) break;
+      if (n > 0) {
+        if (!(ok = fb_wait(done, finished & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
+        ++finished;
+        tc_fence_after_sync();
+      }
+      const int first = w.row0 + quad * 32;
+      fb_store_rows(tm_dq + lane_addr + c0, n == 0, p.scale, stage,
+                    p.dq + (long long)(w.q_beg + first) * p.lddq + w.head * FB_D + c0, p.lddq, w.len_q - first);
+      tc_fence_before_sync();                            // dQ has been read: the next item's first product overwrites it
       __syncwarp();
-      if (lane == 0) mbar_arrive(ds_ready);
-    }
-    if (ok && n > 0) ok = fb_wait(done, 0, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag);
-    if (ok) {
-      tc_fence_after_sync();
-      fb_store_row(tm_dq + lane_addr + c0, n == 0, p.scale, p.dq + (long long)(q_beg + q_idx) * p.lddq + h * FB_D + c0, live);
+      if (lane == 0) mbar_arrive(&item_empty[slot]);
     }
   }
 
@@ -402,6 +476,15 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int kv0 = block / heads * FB_B;                 // early key blocks are seen by most queries: first
   const int q_beg = p.cu_q[b], len_q = p.cu_q[b + 1] - q_beg;
   const int k_beg = p.cu_k[b], len_k = p.cu_k[b + 1] - k_beg;
+  {
+    // queries outside every sequence have no gradient (here, because every CTA of this grid runs)
+    const int head = p.cu_q[0], tail = p.cu_q[p.B], outside = head + max(p.Tq - tail, 0);
+    for (long long i = (long long)blockIdx.x * FB_THREADS + threadIdx.x; i < (long long)outside * p.hq * (FB_D / 4);
+         i += (long long)gridDim.x * FB_THREADS) {
+      const int e = (int)(i % (p.hq * (FB_D / 4))), k = (int)(i / (p.hq * (FB_D / 4)));
+      *reinterpret_cast<uint2*>(p.dq + (long long)(k < head ? k : tail + k - head) * p.lddq + e * 4) = make_uint2(0u, 0u);
+    }
+  }
   if (kv0 >= len_k) return;
   const int shift = len_k - len_q;
   const int G = p.hq / p.hkv;
@@ -529,7 +612,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tc_fence_after_sync();
         fb_mma_ss(tm_dp, v_a, smem_u32(do_sh));
         tc_commit(dp_ready);
-        for (int i = 0; i < n; ++i) {
+        for (int i = 0; i < n && !*abort_flag; ++i) {
           const int s = i & 1, s1 = s ^ 1;
           const uint32_t ph1 = ((i + 1) >> 1) & 1;
           FB_WAIT1(p_ready, i & 1, ST_TIMEOUT_TMEM_EMPTY)
@@ -655,11 +738,12 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
 
   // ---- results of the key block; after a failed wait nothing is written
-  const int quad = warp & 3, c0 = ((warp - 2) >> 2) * 64, row = quad * 32 + lane, key = kv0 + row;
+  const int quad = warp & 3, c0 = ((warp - 2) >> 2) * 64, row = quad * 32 + lane;
   const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-  const bool key_ok = key < len_k;
-  __nv_bfloat16* dk_row = p.dk + (long long)(k_beg + key) * p.lddk + hk * FB_D + c0;
-  __nv_bfloat16* dv_row = p.dv + (long long)(k_beg + key) * p.lddv + hk * FB_D + c0;
+  __nv_bfloat16* dk_dst = p.dk + (long long)(k_beg + kv0 + quad * 32) * p.lddk + hk * FB_D + c0;
+  __nv_bfloat16* dv_dst = p.dv + (long long)(k_beg + kv0 + quad * 32) * p.lddv + hk * FB_D + c0;
+  uint8_t* stage = do_sh + (warp - 2) * 4096;   // the dO tiles are no longer read
+  const int live = len_k - (kv0 + quad * 32);
   if constexpr (SPLIT == 2) {
     // The Q tiles' 64 KB receive the peer's partial sums as [column][row]. Both CTAs' loops have ended before either
     // writes, and every thread takes part in the cluster barriers whatever happened before.
@@ -680,12 +764,12 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     cluster_sync_all();
     if (warp >= 2 && ok) {
       const float* add = reinterpret_cast<const float*>(q_sh) + c0 * FB_B + row;
-      if (rank == 0) fb_store_row(tm_dk + lane_addr + c0, n == 0, p.scale, dk_row, key_ok, add);
-      else fb_store_row(tm_dv + lane_addr + c0, n == 0, 1.f, dv_row, key_ok, add);
+      if (rank == 0) fb_store_rows(tm_dk + lane_addr + c0, n == 0, p.scale, stage, dk_dst, p.lddk, live, add);
+      else fb_store_rows(tm_dv + lane_addr + c0, n == 0, 1.f, stage, dv_dst, p.lddv, live, add);
     }
   } else if (warp >= 2 && ok) {
-    fb_store_row(tm_dk + lane_addr + c0, n == 0, p.scale, dk_row, key_ok);
-    fb_store_row(tm_dv + lane_addr + c0, n == 0, 1.f, dv_row, key_ok);
+    fb_store_rows(tm_dk + lane_addr + c0, n == 0, p.scale, stage, dk_dst, p.lddk, live);
+    fb_store_rows(tm_dv + lane_addr + c0, n == 0, 1.f, stage, dv_dst, p.lddv, live);
   }
 
   tc_fence_before_sync();
@@ -716,8 +800,9 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
       (lddq & 7) || (lddk & 7) || (lddv & 7) || max_q <= 0 || max_k <= 0 || ((uintptr_t)out & 7) || ((uintptr_t)dq & 15) ||
       ((uintptr_t)dk & 15) || ((uintptr_t)dv & 15))
     return B200_ERR_ARG;
-  const long long grid_q = (long long)((max_q + FB_B - 1) / FB_B) * hq * B, grid_k = (long long)((max_k + FB_B - 1) / FB_B) * hkv * B;
-  if (grid_q > 0x7fffffff || grid_k > 0x7fffffff) return B200_ERR_TOO_LARGE;
+  const int levels_q = (max_q + FB_B - 1) / FB_B;
+  const long long items_q = flash_items(B, Tq, max_q, FB_B, hq), grid_k = (long long)((max_k + FB_B - 1) / FB_B) * hkv * B;
+  if (grid_k > 0x7fffffff || items_q > 0x7fffffff) return B200_ERR_TOO_LARGE;
   CUtensorMap tm_q, tm_k, tm_v, tm_do;
   if (make_tmap_2d(&tm_q, q, Tq, (uint64_t)hq * FB_D, ldq, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tm_k, k, Tk, (uint64_t)hkv * FB_D, ldk, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
@@ -725,16 +810,16 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
   if (make_tmap_2d(&tm_do, dout, Tq, (uint64_t)hq * FB_D, lddo, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM) != cudaSuccess ||
+    if (cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM_DQ) != cudaSuccess ||
         cudaFuncSetAttribute(flash_bwd_dkdv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(flash_bwd_dkdv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM) != cudaSuccess)
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
   FbParams p{cu_q, cu_k, lse, delta, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dq,
-             (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, causal, scale,
+             (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, causal, levels_q, scale,
              scale * FB_LOG2E, status};
-  flash_bwd_dq_kernel<<<(unsigned)grid_q, FB_THREADS, FB_SMEM, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
+  flash_bwd_dq_kernel<<<(unsigned)items_q, FB_THREADS, FB_SMEM_DQ, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
   // Few key blocks leave SMs idle behind the one with the most queries: share each between two CTAs while there are fewer
   // than three per SM. (Seven packed sequences of 640 to 1536 tokens, 28 / 4 heads: 336 blocks, the longest 84 iterations
   // against 69 per SM on average.)

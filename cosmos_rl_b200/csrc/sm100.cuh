@@ -104,6 +104,39 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   }
 }
 
+// Registers a thread of the executing warpgroup, all of whose warps run this; the sum over the block's warpgroups stays
+// within what it was launched with.
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// ---------------------------------------------------------------------------
+// Cluster launch control: a running CTA takes over the next CTA of the grid that has not started. The answer is 16 bytes
+// of shared memory, announced on an mbarrier as 16 transaction bytes; after a refusal no further request may be made.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void clc_try_cancel(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// true: block `x` will not start by itself
+__device__ __forceinline__ bool clc_answer(const void* answer, uint32_t& x) {
+  uint32_t got, first = 0;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(got), "+r"(first)
+      : "r"(smem_u32(answer))
+      : "memory");
+  x = first;
+  return got != 0;
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -487,6 +520,11 @@ __device__ __forceinline__ float exp2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

@@ -63,6 +63,26 @@ def test_fused_logprob_fwd_bwd(T, V, H, temp):
     assert torch.allclose(w.grad.float(), wr.grad, rtol=5e-2, atol=5e-2 * wr.grad.abs().max().item())
 
 
+@pytest.mark.parametrize("T,V,H", [(128, 520, 64), (129, 264, 64), (255, 1000, 72), (385, 8, 128)])
+def test_logit_gradient_tiles(T, V, H):
+    torch.manual_seed(61)
+    h, w = _bf16(T, H).requires_grad_(True), _bf16(V, H, scale=0.1).requires_grad_(True)
+    labels = torch.randint(0, V, (T,), device=DEV)
+    labels[::5] = -100
+    g1, g2 = torch.randn(T, device=DEV), torch.randn(T, device=DEV)
+    lp, ent = F.fused_logprob(h, w, labels, 0.9)
+    (lp * g1 + ent * g2).sum().backward()
+    native.read_status(h.device)
+    hr, wr = h.detach().double(), w.detach().double()
+    logits = (hr @ wr.t() / 0.9).requires_grad_(True)
+    lsm = torch.log_softmax(logits, -1)
+    picked = torch.where(labels >= 0, lsm.gather(1, labels.clamp_min(0)[:, None])[:, 0], 0.0)
+    (picked * g1 - (lsm.exp() * lsm).sum(-1) * g2).sum().backward()
+    d = logits.grad / 0.9   # kept as bf16: each entry is off by 2^-9 of itself, as is the result; fp32 sums: the floor
+    for grad, ref, size in ((h.grad, d @ wr, d.abs() @ wr.abs()), (w.grad, d.t() @ hr, d.abs().t() @ hr.abs())):
+        assert ((grad.double() - ref).abs() <= 2.0 ** -8 * (size + ref.abs()) + 1e-5).all()
+
+
 @pytest.mark.parametrize("R_,C,off", [(1, 128, 0), (3, 200, 0), (17, 1032, 0), (5, 130, 1), (65, 4096, 0)])
 def test_quant_fp8_rows_match_reference_bit_for_bit(R_, C, off):
     """Ragged last blocks, and rows that start off the 16-byte grid."""
@@ -1044,6 +1064,29 @@ def test_flash_attention_tile_edges(lens, hq, hkv, causal):
     ref.backward(go.float())
     # bf16 rounds the result (2^-9 of it) and P / dS on the way (2^-9 of sums of about unit terms)
     assert torch.allclose(out[:n].float(), ref[:n], atol=2e-2, rtol=2e-2)
+    for got, want in zip(grads, (rq.grad, rk.grad, rv.grad)):
+        assert (got[:n].float() - want[:n]).abs().max() <= 3e-2 * want.abs().max() + 2e-2
+
+
+@pytest.mark.parametrize("causal,max_q", [(True, 299), (True, 700), (False, 700)])
+def test_flash_attention_many_sequences(causal, max_q):
+    """More items than SMs over more sequences than one warp-wide step of the work list covers, empty ones among them, and
+    a bound on the length that no sequence reaches."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(62)
+    lens = [(37 * i) % 300 for i in range(70)]
+    d, hq, hkv, T = 128, 16, 4, sum(lens) + 5
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    q, k, v, go = _bf16(T, hq, d), _bf16(T, hkv, d), _bf16(T, hkv, d), _bf16(T, hq, d)
+    scale, n = 1.0 / math.sqrt(d), sum(lens)
+    out, lse = attention.flash_fwd(q, k, v, cu, cu, max_q, scale, causal)
+    grads = attention.flash_bwd(go, q, k, v, out, lse, cu, max_q, scale, causal=causal)
+    native.read_status(q.device)
+    assert not grads[0][n:].any()
+    rq, rk, rv = (t.float().requires_grad_(True) for t in (q, k, v))
+    ref = R.varlen_attention(rq, rk, rv, cu, scale, causal=causal)
+    ref.backward(go.float())
+    assert torch.allclose(out[:n].float(), ref[:n], atol=2e-2, rtol=2e-2)   # as in the test above
     for got, want in zip(grads, (rq.grad, rk.grad, rv.grad)):
         assert (got[:n].float() - want[:n]).abs().max() <= 3e-2 * want.abs().max() + 2e-2
 
