@@ -89,8 +89,9 @@ int b200_moe_offsets(const int* counts, int E, int* offsets, int* tile_expert, i
                      int max_tiles, cudaStream_t stream);
 int b200_moe_permute(const void* x, const int* idx, const int* offsets, int* cursor, int* row_map, void* xp, int T,
                      int k, int H, cudaStream_t stream);
-// clears the rows of xp between each expert's last token and the end of its last 128-row tile
-int b200_moe_zero_padding(const int* counts, const int* offsets, void* xp, int E, int H, cudaStream_t stream);
+// clears the rows of xp between an expert's last filled row (filled: rows claimed by the permutation, its cursor) and the
+// next expert's first; none at or past max_rows
+int b200_moe_zero_padding(const int* filled, const int* offsets, void* xp, int E, int max_rows, int H, cudaStream_t stream);
 int b200_moe_scatter_scaled(const void* src, const float* probs, const int* row_map, void* dst, int T, int k, int H,
                             cudaStream_t stream);
 int b200_moe_combine(const void* y, const float* probs, const int* row_map, void* out, int T, int k, int H,

@@ -128,12 +128,12 @@ permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx,
   }
 }
 
-// the rows between an expert's last token and the end of its last tile: the GEMMs contract over them
+// the rows between an expert's last filled row and the next expert's first: the GEMMs contract over them
 __global__ void __launch_bounds__(ROW_MAX_THREADS)
-zero_padding_kernel(const int* __restrict__ counts, const int* __restrict__ offsets, __nv_bfloat16* __restrict__ xp,
-                    int H) {
-  const int e = blockIdx.x;
-  for (int r = offsets[e] + counts[e] + blockIdx.y; r < offsets[e + 1]; r += gridDim.y)
+zero_padding_kernel(const int* __restrict__ filled, const int* __restrict__ offsets, __nv_bfloat16* __restrict__ xp,
+                    int max_rows, int H) {
+  const int e = blockIdx.x, end = min(offsets[e + 1], max_rows);   // counts that are only an upper bound may add up to more
+  for (int r = offsets[e] + filled[e] + blockIdx.y; r < end; r += gridDim.y)
     for (int i = threadIdx.x; i < H / 8; i += blockDim.x)
       reinterpret_cast<uint4*>(xp + (long long)r * H)[i] = make_uint4(0u, 0u, 0u, 0u);
 }
@@ -266,10 +266,10 @@ int b200_moe_permute(const void* x, const int* idx, const int* offsets, int* cur
   return ok();
 }
 
-int b200_moe_zero_padding(const int* counts, const int* offsets, void* xp, int E, int H, cudaStream_t stream) {
+int b200_moe_zero_padding(const int* filled, const int* offsets, void* xp, int E, int max_rows, int H, cudaStream_t stream) {
   if (E <= 0) return 0;
   if (H & 7) return B200_ERR_ARG;
-  zero_padding_kernel<<<dim3(E, E < 64 ? 32 : 16), row_threads(H), 0, stream>>>(counts, offsets, (__nv_bfloat16*)xp, H);
+  zero_padding_kernel<<<dim3(E, E < 64 ? 32 : 16), row_threads(H), 0, stream>>>(filled, offsets, (__nv_bfloat16*)xp, max_rows, H);
   return ok();
 }
 

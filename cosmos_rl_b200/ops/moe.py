@@ -79,7 +79,6 @@ class _Dispatch:
         if counts is None:
             counts = torch.zeros(E, dtype=torch.int32, device=dev)
             counts.index_add_(0, idx.flatten().long(), torch.ones(T * k, dtype=torch.int32, device=dev))
-        self.counts = counts
         self.offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
         self.tile_expert = torch.zeros(self.max_tiles, dtype=torch.int32, device=dev)
         self.n_tiles = torch.empty(1, dtype=torch.int32, device=dev)
@@ -90,12 +89,13 @@ class _Dispatch:
                                                    native.ptr(self.cursor), self.max_tiles, native.stream()),
                      "moe_offsets")
 
-
     def zero_padding(self, buf: torch.Tensor) -> None:
-        """Clears the rows of an expert-sorted buffer that fill up each expert's last tile."""
-        native.check(native.lib().b200_moe_zero_padding(native.ptr(self.counts), native.ptr(self.offsets),
-                                                        native.ptr(buf), self.E, buf.shape[1], native.stream()),
-                     "moe_zero_padding")
+        """Clears the rows of an expert-sorted buffer that no (token, choice) fills. After the permutation ``cursor`` holds
+        how many rows each expert got; the caller's histogram is read for the offsets only, since the caller may clear or
+        refill it before backward runs."""
+        native.check(native.lib().b200_moe_zero_padding(native.ptr(self.cursor), native.ptr(self.offsets),
+                                                        native.ptr(buf), self.E, buf.shape[0], buf.shape[1],
+                                                        native.stream()), "moe_zero_padding")
 
 
 def _rows16(x: torch.Tensor) -> torch.Tensor:
@@ -144,10 +144,10 @@ class _MoEExperts(torch.autograd.Function):
         disp = _Dispatch(idx, E, counts)
         # rows of the permuted buffers beyond the last tile in use are never read and stay uninitialised
         xp = torch.empty(disp.max_rows, H, dtype=torch.bfloat16, device=x.device)
-        disp.zero_padding(xp)
         native.check(L.b200_moe_permute(native.ptr(_rows16(x)), native.ptr(idx), native.ptr(disp.offsets),
                                         native.ptr(disp.cursor), native.ptr(disp.row_map), native.ptr(xp), T, k, H,
                                         native.stream()), "moe_permute")
+        disp.zero_padding(xp)
         h1 = _grouped(xp, w_gate_up, disp, 0, I2)
         act = _swiglu_rows(h1, disp)
         y = _grouped(act, w_down, disp, 0, H)

@@ -1104,3 +1104,64 @@ def test_flash_attention_scores_that_grow_along_the_keys():
     native.read_status(q.device)
     ref = R.varlen_attention(q.float(), k.float(), v.float(), cu, 1.0 / math.sqrt(d))
     assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2), (out.float() - ref).abs().max()
+
+
+# ------------------------------------------------------------------------------------------------ what memory held before
+@pytest.fixture
+def dirty_allocations(monkeypatch):
+    """New tensors hold NaN, as memory that the allocator hands out again may."""
+    for name in ("empty", "empty_like"):
+        def dirty(*args, _plain=getattr(torch, name), **kw):
+            t = _plain(*args, **kw)
+            return t.fill_(float("nan")) if t.is_floating_point() else t
+        monkeypatch.setattr(torch, name, dirty)
+
+
+def _moe_case(T, H, I, E, k):
+    return [t.requires_grad_(True) for t in (_bf16(T, H), torch.rand(T, k, device=DEV), _bf16(E, 2 * I, H, scale=0.05),
+                                             _bf16(E, H, I, scale=0.05))]
+
+
+def _check_moe(out, args, idx):
+    from cosmos_rl_b200.ops import moe
+    g = _bf16(*out.shape)
+    got = torch.autograd.grad(out, args, g)
+    native.read_status(out.device)
+    ref_in = [t.detach().float().requires_grad_(True) for t in args]
+    ref = moe.moe_experts_reference(ref_in[0], ref_in[1], idx, ref_in[2], ref_in[3])
+    want = torch.autograd.grad(ref, ref_in, g.float())
+    assert torch.allclose(out.float(), ref, rtol=3e-2, atol=3e-2 * ref.abs().max().item())
+    for a, b in zip(got, want):
+        assert torch.allclose(a.float(), b, rtol=5e-2, atol=5e-2 * b.abs().max().item())
+
+
+def test_moe_experts_counts_buffer_used_again_before_backward(dirty_allocations):
+    """One histogram buffer, cleared and filled again for the next call while the first call's backward is still to come."""
+    from cosmos_rl_b200.ops import moe
+    torch.manual_seed(71)
+    T, E, k = 200, 6, 2
+    counts, calls = torch.zeros(E, dtype=torch.int32, device=DEV), []
+    for favoured in (0, 3):                                          # other experts are the long ones in the second call
+        logits = torch.randn(T, E, device=DEV)
+        logits[:, favoured] += 6.0
+        counts.zero_()
+        probs, idx = moe.route_topk(logits, k, counts=counts)
+        args = _moe_case(T, 256, 128, E, k)
+        args[1] = probs.requires_grad_(True)
+        calls.append((moe.moe_experts(args[0], args[1], idx, args[2], args[3], counts), args, idx))
+    for call in calls:
+        _check_moe(*call)
+
+
+@pytest.mark.parametrize("spare", [0, 5000])
+def test_moe_experts_counts_above_what_the_choices_hold(dirty_allocations, spare):
+    """An upper bound instead of the histogram: whole tiles, and for the last experts (which no token chooses) more rows than
+    the permuted buffers have."""
+    from cosmos_rl_b200.ops import moe
+    torch.manual_seed(72)
+    T, E, k = 150, 4, 1
+    args = _moe_case(T, 256, 128, E, k)
+    idx = torch.randint(0, 2, (T, k), device=DEV, dtype=torch.int32)
+    counts = (torch.bincount(idx.flatten().long(), minlength=E) + 127) // 128 * 128
+    counts[2:] = 64 + spare
+    _check_moe(moe.moe_experts(args[0], args[1], idx, args[2], args[3], counts.to(torch.int32)), args, idx)
