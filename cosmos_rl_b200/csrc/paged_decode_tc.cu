@@ -18,8 +18,9 @@
 //              written to shared memory in the swizzled K-major layout the second MMA reads.
 // What bounds the kernel besides HBM is the softmax chain of one tile after another, so that chain is kept short: the
 // eight column maxima are reduced together (nine shuffles, each step halving the heads a lane carries), the sums
-// stay per thread until the end of the item, one named barrier a tile, and the running maximum only moves when it
-// grows by more than 2^8, so that O^T is rarely rescaled in TMEM and the chain does not wait for the previous PV.
+// stay per thread until the end of the item, one named barrier a tile, and O^T is rescaled in TMEM (after the previous
+// PV) only when a running maximum has moved. The maximum is exact: the largest probability is 1, which bf16 holds. (A
+// maximum that lags by up to 2^8 rounds it like any other: error of peaked heads against 64 bits 2.18e-3, 1.74e-3 so.)
 // Every mbarrier wait is bounded; on a timeout the kernel records a status code, frees TMEM and returns.
 #include "sm100.cuh"
 #include "gemm_core.cuh"
@@ -38,7 +39,6 @@ constexpr int PDT_P_BYTES = 2 * PDT_N * 64 * 2;             // two 16 x 64-token
 constexpr int PDT_SMEM = PDT_STAGES * PDT_STAGE_BYTES + 2 * PDT_Q_BYTES + 2 * PDT_P_BYTES + 1024 /*barriers, reductions*/ + 1024;
 constexpr int PDT_THREADS = 192;
 constexpr float PDT_LOG2E = 1.4426950408889634f;
-constexpr float PDT_RESCALE_TAU = 8.0f;
 
 struct PdtParams {
   const int* block_table;
@@ -334,7 +334,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
           for (int i = 0; i < 4; ++i) {
             const int g = h4 * 4 + i;
             corr[g] = 1.f;
-            if (tmax[i] > m_run[g] + PDT_RESCALE_TAU || (m_run[g] == -INFINITY && tmax[i] != -INFINITY)) {
+            if (tmax[i] > m_run[g]) {
               corr[g] = exp2f(m_run[g] - tmax[i]);
               m_run[g] = tmax[i];
               grow = true;

@@ -1165,3 +1165,26 @@ def test_moe_experts_counts_above_what_the_choices_hold(dirty_allocations, spare
     counts = (torch.bincount(idx.flatten().long(), minlength=E) + 127) // 128 * 128
     counts[2:] = 64 + spare
     _check_moe(moe.moe_experts(args[0], args[1], idx, args[2], args[3], counts.to(torch.int32)), args, idx)
+
+
+@pytest.mark.parametrize("nsplit", [1, 2])
+def test_paged_decode_largest_probability_is_not_rounded(nsplit):
+    """Only the key with the largest score has values (ones): the result is 1 / sum, rounded once, wherever that key lies."""
+    torch.manual_seed(78)
+    B, h, d, P, L = 32, 4, 128, 128, 700
+    pages = (L + P - 1) // P
+    table = (torch.arange(B * pages, device=DEV, dtype=torch.int32) + 1).view(B, pages)
+    lens = torch.full((B,), L, dtype=torch.int32, device=DEV)
+    cache = _bf16(B * pages + 1, 2, h, P, d)
+    q = _bf16(B, h, d)
+    k = cache[1:, 0].view(B, pages, h, P, d).transpose(1, 2).reshape(B, h, pages * P, d)[:, :, :L].double()
+    s = torch.einsum("bhd,bhkd->bhk", q.double(), k) / math.sqrt(d)
+    top = s.argmax(-1)
+    cache[:, 1] = 0
+    b, hh = torch.meshgrid(torch.arange(B, device=DEV), torch.arange(h, device=DEV), indexing="ij")
+    cache[table.long().gather(1, (top // P)), 1, hh, :, top % P] = 1
+    out = F.paged_decode(q, cache, table, lens, nsplit=nsplit, v_transposed=True)
+    native.read_status(q.device)
+    want = (s - s.amax(-1, keepdim=True)).exp().sum(-1).reciprocal().to(torch.bfloat16)
+    # fp32 scores and sums are off by about 1e-6 of the result, a rounding step is 2^-8 of it: next to none may round otherwise
+    assert (out != want[..., None]).any(-1).float().mean() <= 0.02
