@@ -164,7 +164,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           for (int c = 0; c < 4; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (kbase + c * 32 + i >= k_limit) r[c][i] = 0xff800000u;   // -infinity
+              if (kbase + c * 32 + i >= k_limit) r[c][i] = 0xff800000u;   // -infinity; the scale is positive
         }
         float mx4[4];
 #pragma unroll
@@ -431,6 +431,26 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
 }  // namespace b200
 
+#include "flash_fwd_tile.cuh"
+
+namespace b200 {
+
+// One tile a CTA (flash_fwd_tile.cuh); the grid covers the longest sequence's blocks for every sequence.
+template <bool POSITIVE>
+static int launch_fwd_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const FaParams& p,
+                           int max_q, cudaStream_t stream) {
+  auto kern = flash_fwd_tile_kernel<POSITIVE>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM) != cudaSuccess) return B200_ERR_LAUNCH;
+    attr_set = true;
+  }
+  kern<<<dim3((max_q + FA_B - 1) / FA_B, p.hq, p.B), FT_THREADS, FT_SMEM, stream>>>(tm_q, tm_k, tm_v, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+}
+
+}  // namespace b200
+
 // q [Tq, hq, 128], k / v [Tk, hkv, 128] bf16 with token strides ldq / ldk / ldv (elements, multiples of 8);
 // out [Tq, hq, 128] with token stride ldo; lse [hq, Tq] fp32. cu_q / cu_k: int32 [B + 1] on the device.
 // max_q: longest query segment (bounds the grid). Sequences need len_k >= len_q when causal.
@@ -449,13 +469,15 @@ extern "C" int b200_flash_fwd(const void* q, const void* k, const void* v, void*
   if (make_tmap_2d(&tm_q, q, Tq, (uint64_t)hq * FA_D, ldq, FA_B, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tm_k, k, Tk, (uint64_t)hkv * FA_D, ldk, FA_B, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tm_v, v, Tk, (uint64_t)hkv * FA_D, ldv, FA_B, 64, 2)) return B200_ERR_TENSORMAP;
+  const FaParams p{cu_q, cu_k, (__nv_bfloat16*)out, lse, ldo, B, hq, hkv, Tq, causal, levels, scale * FA_LOG2E, status};
+  // flash_fwd_kernel hides keys before the scale is applied, which takes a positive one
+  if (!(scale > 0.f)) return launch_fwd_tile<false>(tm_q, tm_k, tm_v, p, max_q, stream);
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(flash_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM) != cudaSuccess)
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  FaParams p{cu_q, cu_k, (__nv_bfloat16*)out, lse, ldo, B, hq, hkv, Tq, causal, levels, scale * FA_LOG2E, status};
   flash_fwd_kernel<<<(unsigned)items, FA_THREADS, FA_SMEM, stream>>>(tm_q, tm_k, tm_v, p);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }

@@ -1188,3 +1188,25 @@ def test_paged_decode_largest_probability_is_not_rounded(nsplit):
     want = (s - s.amax(-1, keepdim=True)).exp().sum(-1).reciprocal().to(torch.bfloat16)
     # fp32 scores and sums are off by about 1e-6 of the result, a rounding step is 2^-8 of it: next to none may round otherwise
     assert (out != want[..., None]).any(-1).float().mean() <= 0.02
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.03, -1.0 / math.sqrt(128)])
+@pytest.mark.parametrize("lens,causal", [([300, 17, 129, 256], True), ([300, 130], False)])
+def test_flash_attention_scale_of_zero_or_less(scale, lens, causal):
+    """Partly visible key blocks at a scale of zero (the mean of the visible values) and below it, forward and gradients."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(73)
+    d, hq, hkv, T = 128, 4, 2, sum(lens)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    q, k, v, go = _bf16(T, hq, d), _bf16(T, hkv, d), _bf16(T, hkv, d), _bf16(T, hq, d)
+    out, lse = attention.flash_fwd(q, k, v, cu, cu, max(lens), scale, causal)
+    grads = attention.flash_bwd(go, q, k, v, out, lse, cu, max(lens), scale, causal=causal)
+    native.read_status(q.device)
+    rq, rk, rv = (t.float().requires_grad_(True) for t in (q, k, v))
+    ref, ref_lse = R.varlen_attention(rq, rk, rv, cu, scale, causal=causal, return_lse=True)
+    ref.backward(go.float())
+    # bf16 rounds the result (2^-9 of it) and P / dS on the way (2^-9 of sums of about unit terms); lse is fp32 throughout
+    assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2)
+    assert torch.allclose(lse, ref_lse, atol=1e-3, rtol=1e-4)
+    for got, want in zip(grads, (rq.grad, rk.grad, rv.grad)):
+        assert (got.float() - want).abs().max() <= 3e-2 * want.abs().max() + 2e-2
