@@ -795,7 +795,14 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
                               long long lddk, long long lddv, int max_q, int max_k, int causal, float scale,
                               uint32_t* status, cudaStream_t stream) {
   using namespace b200;
-  if (B <= 0 || Tq <= 0 || Tk <= 0) return 0;
+  if (B <= 0 || Tq <= 0 || Tk <= 0) {   // nothing attends to anything
+    auto clear = [&](void* g, long long ld, int rows, int heads) {
+      return rows <= 0 || heads <= 0 ||
+             cudaMemset2DAsync(g, (size_t)ld * 2, 0, (size_t)heads * FB_D * 2, (size_t)rows, stream) == cudaSuccess;
+    };
+    if (d != FB_D) return B200_ERR_ARG;
+    return clear(dq, lddq, Tq, hq) && clear(dk, lddk, Tk, hkv) && clear(dv, lddv, Tk, hkv) ? 0 : B200_ERR_RUNTIME;
+  }
   if (d != FB_D || hkv <= 0 || hq % hkv || (ldq & 7) || (ldk & 7) || (ldv & 7) || (ldo & 3) || (lddo & 7) ||
       (lddq & 7) || (lddk & 7) || (lddv & 7) || max_q <= 0 || max_k <= 0 || ((uintptr_t)out & 7) || ((uintptr_t)dq & 15) ||
       ((uintptr_t)dk & 15) || ((uintptr_t)dv & 15))

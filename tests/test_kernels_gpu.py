@@ -1210,3 +1210,17 @@ def test_flash_attention_scale_of_zero_or_less(scale, lens, causal):
     assert torch.allclose(lse, ref_lse, atol=1e-3, rtol=1e-4)
     for got, want in zip(grads, (rq.grad, rk.grad, rv.grad)):
         assert (got.float() - want).abs().max() <= 3e-2 * want.abs().max() + 2e-2
+
+
+def test_flash_attention_gradients_with_nothing_to_attend_to(dirty_allocations):
+    """No sequences, no keys, no queries: every gradient that has rows is zero."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(74)
+    d, hq, hkv, T = 128, 2, 1, 96
+    q, k, out, go = _bf16(T, hq, d), _bf16(T, hkv, d), _bf16(T, hq, d), _bf16(T, hq, d)
+    for nq, nk, cu, cu_k in ((T, T, [0], [0]), (T, 0, [0, T], [0, 0]), (0, T, [0, 0], [0, T])):
+        cu, cu_k = (torch.tensor(c, dtype=torch.int32, device=DEV) for c in (cu, cu_k))
+        grads = attention.flash_bwd(go[:nq], q[:nq], k[:nk], k[:nk], out[:nq], torch.zeros(hq, nq, device=DEV), cu, T, 0.1,
+                                    cu_k=cu_k, max_k=T, causal=False)
+        assert [len(g) for g in grads] == [nq, nk, nk]
+        assert all(torch.equal(g, torch.zeros_like(g)) for g in grads)
