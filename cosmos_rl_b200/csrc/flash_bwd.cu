@@ -57,7 +57,7 @@ struct FbParams {
   __nv_bfloat16* dk;           // [Tk, hkv, d]
   __nv_bfloat16* dv;
   long long ldo, lddo, lddq, lddk, lddv;  // token strides (elements)
-  int B, hq, hkv, Tq, causal;
+  int B, hq, hkv, Tq, Tk, causal;
   int levels_q;                // 128-query blocks of the longest sequence
   float scale, scale_log2;
   uint32_t* status;
@@ -462,6 +462,16 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   }
 }
 
+// rows [0, head) and [tail, T) of a gradient [T, heads, d], by the whole grid
+__device__ __forceinline__ void fb_clear_outside(__nv_bfloat16* g, long long ld, int heads, int head, int tail, int T) {
+  const int vec = heads * (FB_D / 4), outside = head + max(T - tail, 0);
+  for (long long i = (long long)blockIdx.x * FB_THREADS + threadIdx.x; i < (long long)outside * vec;
+       i += (long long)gridDim.x * FB_THREADS) {
+    const int e = (int)(i % vec), k = (int)(i / vec);
+    *reinterpret_cast<uint2*>(g + (long long)(k < head ? k : tail + k - head) * ld + e * 4) = make_uint2(0u, 0u);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // dK, dV. SPLIT = 2: a cluster of two CTAs shares a key block, each taking half of its (head, query block) iterations; at
 // the end they exchange partial sums through distributed shared memory, the first CTA finishing dK and the second dV.
@@ -476,15 +486,10 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int kv0 = block / heads * FB_B;                 // early key blocks are seen by most queries: first
   const int q_beg = p.cu_q[b], len_q = p.cu_q[b + 1] - q_beg;
   const int k_beg = p.cu_k[b], len_k = p.cu_k[b + 1] - k_beg;
-  {
-    // queries outside every sequence have no gradient (here, because every CTA of this grid runs)
-    const int head = p.cu_q[0], tail = p.cu_q[p.B], outside = head + max(p.Tq - tail, 0);
-    for (long long i = (long long)blockIdx.x * FB_THREADS + threadIdx.x; i < (long long)outside * p.hq * (FB_D / 4);
-         i += (long long)gridDim.x * FB_THREADS) {
-      const int e = (int)(i % (p.hq * (FB_D / 4))), k = (int)(i / (p.hq * (FB_D / 4)));
-      *reinterpret_cast<uint2*>(p.dq + (long long)(k < head ? k : tail + k - head) * p.lddq + e * 4) = make_uint2(0u, 0u);
-    }
-  }
+  // tokens outside every sequence have no gradient (here, because every CTA of this grid runs)
+  fb_clear_outside(p.dq, p.lddq, p.hq, p.cu_q[0], p.cu_q[p.B], p.Tq);
+  fb_clear_outside(p.dk, p.lddk, p.hkv, p.cu_k[0], p.cu_k[p.B], p.Tk);
+  fb_clear_outside(p.dv, p.lddv, p.hkv, p.cu_k[0], p.cu_k[p.B], p.Tk);
   if (kv0 >= len_k) return;
   const int shift = len_k - len_q;
   const int G = p.hq / p.hkv;
@@ -786,8 +791,8 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
 }  // namespace b200
 
-// Gradients of b200_flash_fwd: dq [Tq, hq, 128], dk / dv [Tk, hkv, 128] bf16 are overwritten (rows of dq outside every
-// sequence are zeroed); delta [hq, Tq] fp32 is scratch. max_q / max_k bound the grids.
+// Gradients of b200_flash_fwd: dq [Tq, hq, 128], dk / dv [Tk, hkv, 128] bf16 are overwritten (rows outside every sequence
+// are zeroed); delta [hq, Tq] fp32 is scratch. max_q / max_k bound the grids.
 extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout,
                               const float* lse, void* dq, void* dk, void* dv, float* delta, const int* cu_q,
                               const int* cu_k, int B, int Tq, int Tk, int hq, int hkv, int d, long long ldq,
@@ -824,8 +829,8 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
     attr_set = true;
   }
   FbParams p{cu_q, cu_k, lse, delta, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dq,
-             (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, causal, levels_q, scale,
-             scale * FB_LOG2E, status};
+             (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, Tk, causal, levels_q,
+             scale, scale * FB_LOG2E, status};
   flash_bwd_dq_kernel<<<(unsigned)items_q, FB_THREADS, FB_SMEM_DQ, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
   // Few key blocks leave SMs idle behind the one with the most queries: share each between two CTAs while there are fewer
   // than three per SM. (Seven packed sequences of 640 to 1536 tokens, 28 / 4 heads: 336 blocks, the longest 84 iterations

@@ -1224,3 +1224,20 @@ def test_flash_attention_gradients_with_nothing_to_attend_to(dirty_allocations):
                                     cu_k=cu_k, max_k=T, causal=False)
         assert [len(g) for g in grads] == [nq, nk, nk]
         assert all(torch.equal(g, torch.zeros_like(g)) for g in grads)
+
+
+@pytest.mark.parametrize("hkv,bound", [(1, 130), (4, 16384)])   # a key block shared by two CTAs, or by one
+def test_flash_attention_gradients_of_tokens_outside_the_sequences(dirty_allocations, hkv, bound):
+    """Tokens before the first and after the last sequence: zero gradients of queries, keys and values, as the one packed
+    tensor that they are slices of needs them."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(75)
+    d, hq, head, lens, tail = 128, 4, 5, [130, 64], 140
+    T = head + sum(lens) + tail
+    cu = torch.tensor([head] + list(head + torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    q, k, v, go = _bf16(T, hq, d), _bf16(T, hkv, d), _bf16(T, hkv, d), _bf16(T, hq, d)
+    out, lse = attention.flash_fwd(q, k, v, cu, cu, max(lens), 0.1)
+    grads = attention.flash_bwd(go, q, k, v, out, lse, cu, bound, 0.1)
+    native.read_status(q.device)
+    for g in grads:
+        assert not g[:head].any() and not g[T - tail:].any() and torch.isfinite(g.float()).all()
