@@ -379,8 +379,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready[tb]);   // after a failed wait the next barrier ends the loop
       }
-      if (!ok) break;
-      // ---- item epilogue
+      // ---- item epilogue, which a warp enters after a failed wait too: the others are at its barrier or on their way there
       // the sums over the 128 tokens, through the buffer that the last tile's maxima did not use
       {
         float* sums = red + (tile_it & 1) * 32;   // tile_it is already one past the last tile
