@@ -21,3 +21,13 @@ def test_decode_softmax_warps_leave_their_loops_together():
     for line in lines:
         if line.startswith(("for (", "while (")):
             assert "abort_flag" not in line, line
+
+
+def test_local_arrays_read_as_vectors_are_aligned():
+    """An array of 2-byte values that is read as one 16-byte vector says so in its declaration: as long as it lives in
+    registers nothing depends on it, but in local memory the load would be misaligned."""
+    for path in sorted(CSRC.glob("*.cu*")):
+        src = path.read_text()
+        for name in set(re.findall(r"\*reinterpret_cast<(?:const )?uint4\*>\((\w+)\)", src)):
+            for decl in re.findall(r"^.*\b__nv_bfloat16 %s\[\d+\];" % re.escape(name), src, flags=re.M):
+                assert "alignas(16)" in decl, (path.name, decl.strip())

@@ -1241,3 +1241,19 @@ def test_flash_attention_gradients_of_tokens_outside_the_sequences(dirty_allocat
     native.read_status(q.device)
     for g in grads:
         assert not g[:head].any() and not g[T - tail:].any() and torch.isfinite(g.float()).all()
+
+
+@pytest.mark.parametrize("R_,C,off", [(128, 128, 0), (130, 200, 0), (5, 130, 1), (257, 264, 3)])
+def test_quant_fp8_weight_blocks_match_reference_bit_for_bit(R_, C, off):
+    """Ragged last blocks, and rows that start off the 16-byte grid."""
+    torch.manual_seed(77)
+    w = _bf16(R_, C + off + 7)[:, off:off + C]
+    q, s = F.quant_fp8_block(w, 128)
+    nr, nc = (R_ + 127) // 128, (C + 127) // 128
+    pad = torch.zeros(nr * 128, nc * 128, device=DEV)
+    pad[:R_, :C] = w.float()
+    blocks = pad.view(nr, 128, nc, 128)
+    scale = blocks.abs().amax((1, 3)).clamp_min(1e-12) / torch.tensor(448.0, device=DEV)
+    assert torch.equal(s, scale)
+    want = (blocks * (1.0 / scale)[:, None, :, None]).view(nr * 128, -1)[:R_, :C].to(torch.float8_e4m3fn)
+    assert torch.equal(q.view(torch.uint8), want.view(torch.uint8))
