@@ -11,6 +11,7 @@
 #define B200_ERR_LAUNCH (-3)
 #define B200_ERR_TOO_LARGE (-4)
 #define B200_ERR_RUNTIME (-5)
+#define B200_NEED_WORKSPACE 1   // nothing was launched: the same call needs its scratch buffer
 
 #ifdef __cplusplus
 extern "C" {
@@ -44,7 +45,7 @@ int b200_gemm_skinny_splits(int M, int N, int K, int swiglu, int num_sms);
 int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, int N, int K, long long ldx,
                      long long ldw, long long ldo, const void* bias, int bias_bf16, int swiglu, int up_row0,
                      int splits, uint32_t* status, int num_sms, cudaStream_t stream);
-// out [M, N] bf16 = x W^T (+ bias): chooses the split and reduces it in the same call
+// out [M, N] bf16 = x W^T (+ bias): chooses the split and reduces it in the same call (ws null: B200_NEED_WORKSPACE if split)
 int b200_skinny_linear(const void* x, const void* W, const void* bias, int bias_bf16, void* out, float* ws,
                        long long ws_floats, int M, int N, int K, long long ldx, long long ldw, long long ldo,
                        uint32_t* status, int num_sms, cudaStream_t stream);

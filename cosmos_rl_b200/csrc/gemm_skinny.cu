@@ -596,13 +596,15 @@ int b200_splitk_reduce(const float* ws, int splits, int M, int N, const void* bi
 }
 
 // y [M, N] bf16 = x W^T (+ bias) in one call: the split is chosen here and reduced when there is one. ws: fp32 scratch of
-// ws_floats elements (splits * M * N are used).
+// ws_floats elements (splits * M * N are used); null with ws_floats 0 until a shape is split, which then returns
+// B200_NEED_WORKSPACE without having launched anything.
 int b200_skinny_linear(const void* x, const void* W, const void* bias, int bias_bf16, void* out, float* ws,
                        long long ws_floats, int M, int N, int K, long long ldx, long long ldw, long long ldo,
                        uint32_t* status, int num_sms, cudaStream_t stream) {
   const int splits = b200_gemm_skinny_splits(M, N, K, 0, num_sms);
   if (splits == 1)
     return b200_gemm_skinny(x, W, out, nullptr, M, N, K, ldx, ldw, ldo, bias, bias_bf16, 0, 0, 1, status, num_sms, stream);
+  if (ws == nullptr) return B200_NEED_WORKSPACE;
   if ((long long)splits * M * N > ws_floats) return B200_ERR_TOO_LARGE;
   const int rc = b200_gemm_skinny(x, W, nullptr, ws, M, N, K, ldx, ldw, 0, nullptr, 0, 0, 0, splits, status, num_sms, stream);
   return rc ? rc : b200_splitk_reduce(ws, splits, M, N, bias, bias_bf16, out, ldo, stream);

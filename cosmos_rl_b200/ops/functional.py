@@ -412,13 +412,18 @@ def gemm_skinny(x2: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x2.device)
     dev, strm = x2.device.index, native.stream()
-    ws = _skinny_workspace(x2.device)
-    native.check(native.lib().b200_skinny_linear(x2.data_ptr(), weight.data_ptr(), native.ptr(bias),
-                                                 1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
-                                                 out.data_ptr(), ws.data_ptr(), _SKINNY_WS_FLOATS, M, N, K,
-                                                 x2.stride(0), weight.stride(0), out.stride(0),
-                                                 native.status_word(x2.device).data_ptr(), native.num_sms(dev), strm),
-                 "gemm_skinny")
+
+    def call(ws):
+        return native.lib().b200_skinny_linear(x2.data_ptr(), weight.data_ptr(), native.ptr(bias),
+                                               1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
+                                               out.data_ptr(), native.ptr(ws), 0 if ws is None else _SKINNY_WS_FLOATS, M, N,
+                                               K, x2.stride(0), weight.stride(0), out.stride(0),
+                                               native.status_word(x2.device).data_ptr(), native.num_sms(dev), strm)
+
+    rc = call(_skinny_ws.get((dev, strm)))
+    if rc == native.NEED_WORKSPACE:     # the first shape on this stream whose contraction is split
+        rc = call(_skinny_workspace(x2.device))
+    native.check(rc, "gemm_skinny")
     return out
 
 

@@ -165,6 +165,9 @@ def add_launches(n: int) -> None:
     LAUNCHES[0] += n
 
 
+NEED_WORKSPACE = 1      # a launcher's answer: nothing was launched, the same call needs its scratch buffer
+
+
 def check(rc: int, what: str) -> None:
     LAUNCHES[0] += 1
     if rc != 0:

@@ -1257,3 +1257,26 @@ def test_quant_fp8_weight_blocks_match_reference_bit_for_bit(R_, C, off):
     assert torch.equal(s, scale)
     want = (blocks * (1.0 / scale)[:, None, :, None]).view(nr * 128, -1)[:R_, :C].to(torch.float8_e4m3fn)
     assert torch.equal(q.view(torch.uint8), want.view(torch.uint8))
+
+
+def test_skinny_workspace_only_where_there_is_a_split():
+    torch.manual_seed(76)
+    x, wide, x2, narrow = _bf16(3, 512), _bf16(32000, 512, scale=0.05), _bf16(3, 4096), _bf16(512, 4096, scale=0.05)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    key = (x.device.index, s.cuda_stream)
+    F._skinny_ws.pop(key, None)
+    with torch.cuda.stream(s):
+        y = F.gemm_skinny(x, wide)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):                         # a first call inside a capture keeps nothing of its pool
+            z = F.gemm_skinny(x, wide)
+        assert key not in F._skinny_ws
+        g.replay()
+        t = F.gemm_skinny(x2, narrow)
+        assert key in F._skinny_ws
+    s.synchronize()
+    native.read_status(x.device)
+    assert torch.equal(y, z)
+    for out, a, w in ((y, x, wide), (t, x2, narrow)):               # fp32 sums of K products, rounded once to bf16
+        assert torch.allclose(out.float(), a.float() @ w.float().t(), rtol=2 ** -8, atol=1e-4 * math.sqrt(a.shape[1]))
