@@ -191,7 +191,7 @@ int b200_paged_decode_static(const void* q, const void* cache, const int* block_
 int b200_flash_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* cu_q,
                    const int* cu_k, int B, int Tq, int Tk, int hq, int hkv, int d, long long ldq, long long ldk,
                    long long ldv, long long ldo, int max_q, int causal, float scale, uint32_t* status,
-                   cudaStream_t stream);
+                   int num_sms, cudaStream_t stream);
 
 // Gradients of b200_flash_fwd (flash_bwd.cu). dq [Tq,hq,d], dk/dv [Tk,hkv,d] bf16 are overwritten; delta [hq,Tq] fp32 is
 // scratch. max_q / max_k: longest query / key segment (bound the grids).

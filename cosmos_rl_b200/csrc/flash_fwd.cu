@@ -1,7 +1,7 @@
 // Varlen (packed) causal flash-attention forward on tcgen05 / TMEM / TMA for head_dim 128, GQA.
 //
-// One CTA per SM works through items (sequence, 256 queries, query head), see flash_sched.cuh; an item is two tiles of 128
-// queries that share every K / V tile. Per tile t and 128-key block j:
+// CTAs take items (sequence, 256 queries, query head) one after the other, see flash_sched.cuh; an item is two tiles of 128
+// queries that share every K / V tile. Calls of few tiles take the one-tile form in flash_fwd_tile.cuh. Per tile t and 128-key block j:
 //     S_t  = Q_t K_j^T          tcgen05.mma M=128 (queries) N=128 (keys) K=128 (d), both operands K-major (TMA, SW128)
 //     P_t  = exp2(S_t*c - m)    one thread per query row (TMEM lane) holds the whole row in registers: no shuffles, no
 //                               shared memory; P goes back as bf16 over the columns of S_t
@@ -457,7 +457,7 @@ static int launch_fwd_tile(const CUtensorMap& tm_q, const CUtensorMap& tm_k, con
 extern "C" int b200_flash_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* cu_q,
                               const int* cu_k, int B, int Tq, int Tk, int hq, int hkv, int d, long long ldq,
                               long long ldk, long long ldv, long long ldo, int max_q, int causal, float scale,
-                              uint32_t* status, cudaStream_t stream) {
+                              uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (B <= 0 || Tq <= 0) return 0;
   if (d != FA_D || hkv <= 0 || hq % hkv || (ldq & 7) || (ldk & 7) || (ldv & 7) || (ldo & 7) || max_q <= 0)
@@ -472,6 +472,13 @@ extern "C" int b200_flash_fwd(const void* q, const void* k, const void* v, void*
   const FaParams p{cu_q, cu_k, (__nv_bfloat16*)out, lse, ldo, B, hq, hkv, Tq, causal, levels, scale * FA_LOG2E, status};
   // flash_fwd_kernel hides keys before the scale is applied, which takes a positive one
   if (!(scale > 0.f)) return launch_fwd_tile<false>(tm_q, tm_k, tm_v, p, max_q, stream);
+  // While every tile of 128 queries has an SM of its own, the time is that of one tile's chain, and the one-tile form has the
+  // shorter one: two warps a row, S of the next block under the softmax of this one, no queue before the first load. One
+  // sequence of 200 tokens, 32 heads: 8.2 us, 12.0 us in the other form; 512 queries on 8192 keys, 28 heads: 100 and 126;
+  // 1152 tokens, 16 heads (144 tiles): 19.7 and 23.3. Beyond one round of CTAs two tiles that share K and V win: 1300 tokens,
+  // 16 heads (176 tiles): 28.4 and 27.2; 1024 tokens, 28 heads (224 tiles): 29.5 and 23.6.
+  if ((long long)((max_q + FA_B - 1) / FA_B) * hq * B <= num_sms)
+    return launch_fwd_tile<true>(tm_q, tm_k, tm_v, p, max_q, stream);
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(flash_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FA_SMEM) != cudaSuccess)

@@ -1,5 +1,5 @@
-// Forward attention with one tile of 128 queries a CTA, the form for a scale of zero or less (see flash_fwd.cu for the other
-// form, the layouts and the roles in common).
+// Forward attention with one tile of 128 queries a CTA: the form for calls that have an SM for every tile, and for a scale of
+// zero or less (see flash_fwd.cu for the other form, the layouts, and why the line lies there).
 //
 // One CTA = one (sequence, 128-query block, query head). Per 128-key block j:
 //     S_j = Q K_j^T            S is double-buffered in TMEM, so the tensor core forms S_{j+1} under the softmax of S_j

@@ -35,7 +35,8 @@ def flash_fwd(q, k, v, cu_q, cu_k, max_q: int, scale: float, causal: bool = True
     native.check(native.lib().b200_flash_fwd(
         native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(out), native.ptr(lse), native.ptr(cu_q),
         native.ptr(cu_k), cu_q.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0), v.stride(0), out.stride(0),
-        int(max_q), 1 if causal else 0, float(scale), native.ptr(st), native.stream()), "flash_fwd")
+        int(max_q), 1 if causal else 0, float(scale), native.ptr(st), native.num_sms(q.device.index), native.stream()),
+        "flash_fwd")
     return out, lse
 
 

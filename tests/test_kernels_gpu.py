@@ -1280,3 +1280,31 @@ def test_skinny_workspace_only_where_there_is_a_split():
     assert torch.equal(y, z)
     for out, a, w in ((y, x, wide), (t, x2, narrow)):               # fp32 sums of K products, rounded once to bf16
         assert torch.allclose(out.float(), a.float() @ w.float().t(), rtol=2 ** -8, atol=1e-4 * math.sqrt(a.shape[1]))
+
+
+@pytest.mark.parametrize("hq,hkv,causal", [(4, 2, True), (7, 1, True), (4, 4, False)])
+def test_flash_attention_forward_forms_agree(hq, hkv, causal):
+    """A sequence alone has an SM for each of its tiles, packed with others it has not: the two forms of the forward on the
+    same rows, sliced out of one packed tensor, with as many keys as queries and with more."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(79)
+    d, scale = 128, 1.0 / math.sqrt(128)
+    lens = [1, 64, 127, 128, 129, 255, 256, 257, 385, 40] * 3
+    more = [0, 5, 128, 300, 0, 1, 255, 0, 127, 0] * 3               # keys before the first query
+    lk = [a + b for a, b in zip(lens, more)]
+    T, Tk = sum(lens), sum(lk)
+    q = _bf16(T, (hq + 3) * d)[:, d:(hq + 1) * d].unflatten(-1, (hq, d))
+    kv = _bf16(Tk, 2 * hkv * d)
+    k, v = kv[:, :hkv * d].unflatten(-1, (hkv, d)), kv[:, hkv * d:].unflatten(-1, (hkv, d))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    cq, ck = i32([0] + list(torch.tensor(lens).cumsum(0))), i32([0] + list(torch.tensor(lk).cumsum(0)))
+    assert sum((n + 127) // 128 for n in lens) * hq > native.num_sms(0) >= (max(lens) + 127) // 128 * hq
+    out, lse = attention.flash_fwd(q, k, v, cq, ck, max(lens), scale, causal)
+    ref, ref_lse = R.varlen_attention(q.float(), k.float(), v.float(), cq, scale, causal, ck, return_lse=True)
+    for i, n in enumerate(lens):
+        r, c = slice(int(cq[i]), int(cq[i + 1])), slice(int(ck[i]), int(ck[i + 1]))
+        one, one_lse = attention.flash_fwd(q[r], k[c], v[c], i32([0, n]), i32([0, lk[i]]), n, scale, causal)
+        for got, got_lse in ((out[r], lse[:, r]), (one, one_lse)):
+            assert torch.allclose(got.float(), ref[r], atol=2e-2, rtol=2e-2)     # bf16 result and probabilities
+            assert torch.allclose(got_lse, ref_lse[:, r], atol=1e-3, rtol=1e-4)
+    native.read_status(q.device)
