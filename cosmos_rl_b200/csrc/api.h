@@ -199,7 +199,7 @@ int b200_flash_bwd(const void* q, const void* k, const void* v, const void* out,
                    void* dq, void* dk, void* dv, float* delta, const int* cu_q, const int* cu_k, int B, int Tq, int Tk,
                    int hq, int hkv, int d, long long ldq, long long ldk, long long ldv, long long ldo, long long lddo,
                    long long lddq, long long lddk, long long lddv, int max_q, int max_k, int causal, float scale,
-                   uint32_t* status, cudaStream_t stream);
+                   uint32_t* status, int num_sms, cudaStream_t stream);
 
 // ---- quantisation ----------------------------------------------------------------------------------------------
 // bf16 [R, C] -> e4m3 [R, C] with one fp32 scale per 128 x 128 block (weights) or per 1 x 128 (activations).

@@ -471,6 +471,15 @@ __device__ __forceinline__ void fb_clear_outside(__nv_bfloat16* g, long long ld,
     *reinterpret_cast<uint2*>(g + (long long)(k < head ? k : tail + k - head) * ld + e * 4) = make_uint2(0u, 0u);
   }
 }
+// tokens outside every sequence have no gradient; in a kernel all of whose CTAs run
+__device__ __forceinline__ void fb_clear_all_outside(const FbParams& p) {
+  const int q0 = p.cu_q[0], q1 = p.cu_q[p.B], k0 = p.cu_k[0], k1 = p.cu_k[p.B];
+  if (q0 > 0 || q1 < p.Tq) fb_clear_outside(p.dq, p.lddq, p.hq, q0, q1, p.Tq);
+  if (k0 > 0 || k1 < p.Tk) {
+    fb_clear_outside(p.dk, p.lddk, p.hkv, k0, k1, p.Tk);
+    fb_clear_outside(p.dv, p.lddv, p.hkv, k0, k1, p.Tk);
+  }
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 // dK, dV. SPLIT = 2: a cluster of two CTAs shares a key block, each taking half of its (head, query block) iterations; at
@@ -486,10 +495,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int kv0 = block / heads * FB_B;                 // early key blocks are seen by most queries: first
   const int q_beg = p.cu_q[b], len_q = p.cu_q[b + 1] - q_beg;
   const int k_beg = p.cu_k[b], len_k = p.cu_k[b + 1] - k_beg;
-  // tokens outside every sequence have no gradient (here, because every CTA of this grid runs)
-  fb_clear_outside(p.dq, p.lddq, p.hq, p.cu_q[0], p.cu_q[p.B], p.Tq);
-  fb_clear_outside(p.dk, p.lddk, p.hkv, p.cu_k[0], p.cu_k[p.B], p.Tk);
-  fb_clear_outside(p.dv, p.lddv, p.hkv, p.cu_k[0], p.cu_k[p.B], p.Tk);
+  fb_clear_all_outside(p);
   if (kv0 >= len_k) return;
   const int shift = len_k - len_q;
   const int G = p.hq / p.hkv;
@@ -791,6 +797,29 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
 }  // namespace b200
 
+#include "flash_bwd_short.cuh"
+
+namespace b200 {
+
+static int launch_bwd_short(const void* q, const void* k, const void* v, const FbParams& p, long long ldq, long long ldk,
+                            long long ldv, cudaStream_t stream) {
+  CUtensorMap tm_q, tm_k, tm_v, tm_do;
+  if (make_tmap_2d(&tm_q, q, p.Tq, (uint64_t)p.hq * FB_D, ldq, FS_BQ, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_k, k, p.Tk, (uint64_t)p.hkv * FB_D, ldk, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_v, v, p.Tk, (uint64_t)p.hkv * FB_D, ldv, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tm_do, p.dout, p.Tq, (uint64_t)p.hq * FB_D, p.lddo, FS_BQ, 64, 2)) return B200_ERR_TENSORMAP;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(flash_bwd_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FS_SMEM) != cudaSuccess)
+      return B200_ERR_LAUNCH;
+    attr_set = true;
+  }
+  flash_bwd_short_kernel<<<(unsigned)(p.B * p.hkv), FB_THREADS, FS_SMEM, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+}
+
+}  // namespace b200
+
 // Gradients of b200_flash_fwd: dq [Tq, hq, 128], dk / dv [Tk, hkv, 128] bf16 are overwritten (rows outside every sequence
 // are zeroed); delta [hq, Tq] fp32 is scratch. max_q / max_k bound the grids.
 extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout,
@@ -798,7 +827,7 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
                               const int* cu_k, int B, int Tq, int Tk, int hq, int hkv, int d, long long ldq,
                               long long ldk, long long ldv, long long ldo, long long lddo, long long lddq,
                               long long lddk, long long lddv, int max_q, int max_k, int causal, float scale,
-                              uint32_t* status, cudaStream_t stream) {
+                              uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (B <= 0 || Tq <= 0 || Tk <= 0) {   // nothing attends to anything
     auto clear = [&](void* g, long long ld, int rows, int heads) {
@@ -815,6 +844,17 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
   const int levels_q = (max_q + FB_B - 1) / FB_B;
   const long long items_q = flash_items(B, Tq, max_q, FB_B, hq), grid_k = (long long)((max_k + FB_B - 1) / FB_B) * hkv * B;
   if (grid_k > 0x7fffffff || items_q > 0x7fffffff) return B200_ERR_TOO_LARGE;
+  const FbParams p{cu_q, cu_k, lse, delta, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dq,
+                   (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, Tk, causal, levels_q,
+                   scale, scale * FB_LOG2E, status};
+  // One kernel over short sequences: it has half the prologues of the two below, which is what such calls cost, but walks
+  // the G query heads of a kv head one after the other. 256 sequences of 20 tokens, 28 / 4 heads: 241 us, with the two 407;
+  // one of 64 tokens, 16 / 16 heads: 10.6 and 18.4. For one or two heads a group always; for more once two fifths of the SMs
+  // have a CTA (16 x 20 tokens, 28 / 4 heads: 33.6 and 40.2; 8 x 20: 33.4 and 31.3). More than 64 queries are two iterations
+  // a head, which pays for one head only (8 x 128 tokens, 16 / 16 heads: 15.7 and 28.9; 32 x 128, 4 / 2 heads: 25.5 and 19.8).
+  const int G = hq / hkv;
+  if (max_k <= FB_B && (max_q <= FS_BQ ? G <= 2 || 5LL * B * hkv >= 2LL * num_sms : max_q <= FB_B && G == 1))
+    return launch_bwd_short(q, k, v, p, ldq, ldk, ldv, stream);
   CUtensorMap tm_q, tm_k, tm_v, tm_do;
   if (make_tmap_2d(&tm_q, q, Tq, (uint64_t)hq * FB_D, ldq, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tm_k, k, Tk, (uint64_t)hkv * FB_D, ldk, FB_B, 64, 2)) return B200_ERR_TENSORMAP;
@@ -828,14 +868,11 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  FbParams p{cu_q, cu_k, lse, delta, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dq,
-             (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ldo, lddo, lddq, lddk, lddv, B, hq, hkv, Tq, Tk, causal, levels_q,
-             scale, scale * FB_LOG2E, status};
   flash_bwd_dq_kernel<<<(unsigned)items_q, FB_THREADS, FB_SMEM_DQ, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
   // Few key blocks leave SMs idle behind the one with the most queries: share each between two CTAs while there are fewer
   // than three per SM. (Seven packed sequences of 640 to 1536 tokens, 28 / 4 heads: 336 blocks, the longest 84 iterations
   // against 69 per SM on average.)
-  if (grid_k < 3 * 148) {
+  if (grid_k < 3LL * num_sms) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * grid_k));
     cfg.blockDim = dim3(FB_THREADS);

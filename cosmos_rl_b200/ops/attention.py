@@ -89,7 +89,7 @@ def flash_bwd(dout, q, k, v, out, lse, cu, max_seqlen: int, scale: float, cu_k=N
         native.ptr(dq), native.ptr(dk), native.ptr(dv), native.ptr(delta), native.ptr(cu), native.ptr(cu_k),
         cu.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0), v.stride(0), out.stride(0), dout.stride(0),
         dq.stride(0), dk.stride(0), dv.stride(0), int(max_seqlen), int(max_k if max_k is not None else max_seqlen),
-        1 if causal else 0, float(scale), native.ptr(st), native.stream()), "flash_bwd")
+        1 if causal else 0, float(scale), native.ptr(st), native.num_sms(q.device.index), native.stream()), "flash_bwd")
     return dq, dk, dv
 
 
