@@ -871,8 +871,13 @@ extern "C" int b200_flash_bwd(const void* q, const void* k, const void* v, const
   flash_bwd_dq_kernel<<<(unsigned)items_q, FB_THREADS, FB_SMEM_DQ, stream>>>(tm_q, tm_k, tm_v, tm_do, p);
   // Few key blocks leave SMs idle behind the one with the most queries: share each between two CTAs while there are fewer
   // than three per SM. (Seven packed sequences of 640 to 1536 tokens, 28 / 4 heads: 336 blocks, the longest 84 iterations
-  // against 69 per SM on average.)
-  if (grid_k < 3LL * num_sms) {
+  // against 69 per SM on average.) A CTA costs about six iterations before and after its loop, so blocks of few iterations
+  // are shared only where the longest alone takes longer than all of them with that cost twice: 8 x 600 tokens, 4 / 2 heads
+  // (80 blocks of 2 to 10) 35.9 us, not shared 41.0; 8 x 129 tokens, 16 / 16 heads (256 of 1 and 2) 54.4 and 34.5; 64 x 129,
+  // 4 / 2 heads 70.0 and 52.4.
+  const long long longest = (long long)G * ((max_q + FB_B - 1) / FB_B);   // iterations of a block that every query sees
+  const long long mean2 = causal ? longest + G : 2 * longest;             // twice the mean
+  if (grid_k < 3LL * num_sms && (longest >= 12 || 2 * (6 + longest) * num_sms > grid_k * (24 + mean2))) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * grid_k));
     cfg.blockDim = dim3(FB_THREADS);
