@@ -441,20 +441,19 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __
 // ------------------------------------------------------------------------------------------------
 // SwiGLU on a fused [T, 2I] gate|up projection
 // ------------------------------------------------------------------------------------------------
-// A thread works on SWIGLU_ITEMS vectors of 8 columns whose loads are all in flight before the first is used; the
-// position is found with 32-bit divisions unless the tensor is too large for them. row_tiles (nullable, device): only
-// the first row_tiles[0] * 128 rows are in use.
-constexpr int SWIGLU_ITEMS = 2;
-template <class Index>
+// Positions are found with 32-bit divisions unless the tensor is too large for them. row_tiles (nullable, device): only the
+// first row_tiles[0] * 128 rows are in use. A thread of the forward works on ITEMS vectors of 8 columns whose loads are all in
+// flight before the first is used.
+template <class Index, int ITEMS>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I,
                   const int* __restrict__ row_tiles) {
   const Index nvec = I >> 3;
   const Index total = (Index)(row_tiles ? min((long long)row_tiles[0] * 128, T) : T) * nvec;
-  const Index first = (Index)blockIdx.x * (256 * SWIGLU_ITEMS) + threadIdx.x;
-  uint4 g[SWIGLU_ITEMS], u[SWIGLU_ITEMS];
+  const Index first = (Index)blockIdx.x * (256 * ITEMS) + threadIdx.x;
+  uint4 g[ITEMS], u[ITEMS];
 #pragma unroll
-  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
+  for (int k = 0; k < ITEMS; ++k) {
     const Index idx = first + k * 256;
     if (idx >= total) continue;
     const Index t = idx / nvec, v = idx - t * nvec;
@@ -463,7 +462,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
     u[k] = row[nvec + v];
   }
 #pragma unroll
-  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
+  for (int k = 0; k < ITEMS; ++k) {
     const Index idx = first + k * 256;
     if (idx >= total) continue;
     float a[8], b[8], o[8];
@@ -481,38 +480,25 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
                   __nv_bfloat16* __restrict__ dgu, long long T, int I, const int* __restrict__ row_tiles) {
   const Index nvec = I >> 3;
   const Index total = (Index)(row_tiles ? min((long long)row_tiles[0] * 128, T) : T) * nvec;
-  const Index first = (Index)blockIdx.x * (256 * SWIGLU_ITEMS) + threadIdx.x;
-  uint4 g[SWIGLU_ITEMS], u[SWIGLU_ITEMS], dd[SWIGLU_ITEMS];
+  const Index idx = (Index)blockIdx.x * 256 + threadIdx.x;
+  if (idx >= total) return;
+  const Index t = idx / nvec, v = idx - t * nvec;
+  const uint4* in = reinterpret_cast<const uint4*>(gu + (long long)t * 2 * I);
+  const uint4 g = in[v], u = in[nvec + v], dd = reinterpret_cast<const uint4*>(dout)[idx];
+  float a[8], b[8], d[8], dg[8], du[8];
+  unpack8(g, a);
+  unpack8(u, b);
+  unpack8(dd, d);
 #pragma unroll
-  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
-    const Index idx = first + k * 256;
-    if (idx >= total) continue;
-    const Index t = idx / nvec, v = idx - t * nvec;
-    const uint4* row = reinterpret_cast<const uint4*>(gu + (long long)t * 2 * I);
-    g[k] = row[v];
-    u[k] = row[nvec + v];
-    dd[k] = reinterpret_cast<const uint4*>(dout)[idx];
+  for (int j = 0; j < 8; ++j) {
+    float s = 1.f / (1.f + __expf(-a[j]));
+    float silu = a[j] * s;
+    dg[j] = d[j] * b[j] * (s + silu * (1.f - s));
+    du[j] = d[j] * silu;
   }
-#pragma unroll
-  for (int k = 0; k < SWIGLU_ITEMS; ++k) {
-    const Index idx = first + k * 256;
-    if (idx >= total) continue;
-    const Index t = idx / nvec, v = idx - t * nvec;
-    float a[8], b[8], d[8], dg[8], du[8];
-    unpack8(g[k], a);
-    unpack8(u[k], b);
-    unpack8(dd[k], d);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float s = 1.f / (1.f + __expf(-a[j]));
-      float silu = a[j] * s;
-      dg[j] = d[j] * b[j] * (s + silu * (1.f - s));
-      du[j] = d[j] * silu;
-    }
-    uint4* row = reinterpret_cast<uint4*>(dgu + (long long)t * 2 * I);
-    row[v] = pack8(dg);
-    row[nvec + v] = pack8(du);
-  }
+  uint4* out = reinterpret_cast<uint4*>(dgu + (long long)t * 2 * I);
+  out[v] = pack8(dg);
+  out[nvec + v] = pack8(du);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -702,8 +688,13 @@ int b200_rope_inplace(void* q, void* k, const long long* positions, int T, int h
 int b200_swiglu_fwd(const void* gate_up, void* out, long long T, int I, const int* row_tiles, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (I & 7) return B200_ERR_ARG;
-  const long long n = T * (I / 8), per = 256 * SWIGLU_ITEMS;
-  auto kern = n < (1ll << 32) - 2 * per ? swiglu_fwd_kernel<uint32_t> : swiglu_fwd_kernel<unsigned long long>;
+  // Two vectors a thread once they fill the machine several times over: 2000 x 14336 32.2 us, with one 33.6; 1000 x 14336 16.0
+  // and 16.1. Below that more threads hide more: 57 x 768 2.7 and 2.1.
+  const long long n = T * (I / 8);
+  const int items = n >= (3ll << 19) ? 2 : 1, per = 256 * items;
+  auto kern = n >= (1ll << 32) - 1024 ? swiglu_fwd_kernel<unsigned long long, 2>
+              : items == 2            ? swiglu_fwd_kernel<uint32_t, 2>
+                                      : swiglu_fwd_kernel<uint32_t, 1>;
   kern<<<(unsigned)((n + per - 1) / per), 256, 0, stream>>>((const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, T, I,
                                                             row_tiles);
   return ok();
@@ -713,10 +704,11 @@ int b200_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long 
                     cudaStream_t stream) {
   if (T <= 0) return 0;
   if (I & 7) return B200_ERR_ARG;
-  const long long n = T * (I / 8), per = 256 * SWIGLU_ITEMS;
-  auto kern = n < (1ll << 32) - 2 * per ? swiglu_bwd_kernel<uint32_t> : swiglu_bwd_kernel<unsigned long long>;
-  kern<<<(unsigned)((n + per - 1) / per), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate_up,
-                                                            (__nv_bfloat16*)dgate_up, T, I, row_tiles);
+  // One vector a thread (8192 x 18944: 223 us, with two 241; 57 x 768: 2.3 and 3.1)
+  const long long n = T * (I / 8);
+  auto kern = n >= (1ll << 32) - 512 ? swiglu_bwd_kernel<unsigned long long> : swiglu_bwd_kernel<uint32_t>;
+  kern<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate_up,
+                                                        (__nv_bfloat16*)dgate_up, T, I, row_tiles);
   return ok();
 }
 

@@ -1339,3 +1339,19 @@ def test_flash_attention_backward_forms_agree(dirty_allocations, hq, hkv, longes
         for got, want in zip(grads, (rq.grad, rk.grad, rv.grad)):
             # bf16 rounds P, dS and the result; queries, keys and values of no sequence have a gradient of zero
             assert (got.float() - want).abs().max() <= 3e-2 * want.abs().max() + 2e-2
+
+
+@pytest.mark.parametrize("T,I", [(1, 8), (57, 776), (1535, 8192), (1536, 8192)])
+def test_swiglu_vectors_a_thread(T, I):
+    """The smallest call, ragged last blocks, and both sides of the size from which a thread takes two vectors."""
+    torch.manual_seed(81)
+    gu, g = _bf16(T, 2 * I), _bf16(T, I)
+    x = gu.clone().requires_grad_(True)
+    y = F.swiglu(x)
+    dx, = torch.autograd.grad(y, x, g)
+    a, b = gu.double().chunk(2, -1)
+    s = torch.sigmoid(a)
+    # one bf16 rounding of the result; the exponential is good to 2^-21 of its argument
+    assert torch.allclose(y.double(), a * s * b, rtol=2 ** -8, atol=1e-5)
+    want = torch.cat([g.double() * b * (s + a * s * (1 - s)), g.double() * a * s], -1)
+    assert torch.allclose(dx.double(), want, rtol=2 ** -8, atol=1e-5)
