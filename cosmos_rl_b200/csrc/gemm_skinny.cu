@@ -300,22 +300,22 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   }
 }
 
-// Sum over the splits of four neighbouring columns. The first eight partials are loaded before any is used: with one
-// item a thread, the latency of one round trip to L2 is what these kernels cost.
-constexpr int SPLIT_BATCH = 8;
+// Sum over the splits of four neighbouring columns. The first BATCH partials are loaded before any is used: with one item a
+// thread, the latency of one round trip to L2 is what these kernels cost.
+template <int BATCH>
 struct SplitSum {
-  float4 t[SPLIT_BATCH];
+  float4 t[BATCH];
   __device__ __forceinline__ void load(const float* p, long long stride, int splits) {
 #pragma unroll
-    for (int s = 0; s < SPLIT_BATCH; ++s)
+    for (int s = 0; s < BATCH; ++s)
       if (s < splits) t[s] = *reinterpret_cast<const float4*>(p + s * stride);
   }
   __device__ __forceinline__ float4 sum(const float* p, long long stride, int splits) const {
     float4 a = t[0];
 #pragma unroll
-    for (int s = 1; s < SPLIT_BATCH; ++s)
+    for (int s = 1; s < BATCH; ++s)
       if (s < splits) { a.x += t[s].x; a.y += t[s].y; a.z += t[s].z; a.w += t[s].w; }
-    for (int s = SPLIT_BATCH; s < splits; ++s) {
+    for (int s = BATCH; s < splits; ++s) {
       const float4 v = *reinterpret_cast<const float4*>(p + s * stride);
       a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
     }
@@ -324,10 +324,10 @@ struct SplitSum {
 };
 
 // One CTA per row: res_out = sum_s ws[s, r, :] (+ res_in);  y = res_out * rsqrt(mean(res_out^2) + eps) * w.
-// Four columns a thread, VPT times (H <= 1024 * VPT * 4); the row stays in registers between the two passes.
+// Four columns a thread, VPT times (H <= MAX_THREADS * VPT * 4); the row stays in registers between the two passes.
 constexpr int RN_MAX_THREADS = 1024;
-template <int VPT>
-__global__ void __launch_bounds__(RN_MAX_THREADS)
+template <int VPT, int MAX_THREADS, int MIN_CTAS>
+__global__ void __launch_bounds__(MAX_THREADS, MIN_CTAS)
 splitk_reduce_residual_rmsnorm_kernel(const float* __restrict__ ws, int splits, int M, int H,
                                       const __nv_bfloat16* __restrict__ res_in, const __nv_bfloat16* __restrict__ w,
                                       float eps, __nv_bfloat16* __restrict__ res_out, __nv_bfloat16* __restrict__ y) {
@@ -344,7 +344,7 @@ splitk_reduce_residual_rmsnorm_kernel(const float* __restrict__ ws, int splits, 
     v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c4 < n4) {
       const float* p = ws + (long long)r * H + c4 * 4;
-      SplitSum sum;
+      SplitSum<VPT <= 2 ? 8 : 2> sum;
       sum.load(p, split_stride, splits);
       uint2 rr = make_uint2(0u, 0u);
       if (res_in) rr = *reinterpret_cast<const uint2*>(res_in + (long long)r * H + c4 * 4);
@@ -413,7 +413,7 @@ splitk_reduce_qkv_rope_append_kernel(const float* __restrict__ ws, int splits, i
   const long long split_stride = (long long)M * N;
   const float* p0 = ws + (long long)r * N + c0;
   const float* p1 = p0 + half;
-  SplitSum s0, s1;
+  SplitSum<8> s0, s1;
   s0.load(p0, split_stride, splits);
   s1.load(p1, split_stride, splits);
   const int slot = slot_mapping[r];
@@ -614,9 +614,14 @@ int b200_splitk_reduce_residual_rmsnorm(const float* ws, int splits, int M, int 
                                         float eps, void* res_out, void* y, cudaStream_t stream) {
   using namespace b200;
   if (M <= 0 || H <= 0 || (H & 3) || H > RN_MAX_THREADS * 2 * 4 || splits < 1) return B200_ERR_ARG;
-  const int n4 = H / 4, vpt = n4 <= RN_MAX_THREADS ? 1 : 2;
+  // A CTA of so many threads has an SM to itself. With more rows than SMs that is two rounds, so long rows (of which there are
+  // at most two splits then) take a quarter of the threads there and two rows share an SM: projection and reduction of 256 x
+  // 8192 (K 4096) 29.3 us, with half the threads 33.3; 256 x 6144 27.7 and 30.0.
+  const int n4 = H / 4, vpt = n4 <= RN_MAX_THREADS ? 1 : M > 148 ? 4 : 2;
   const int threads = ((n4 + vpt - 1) / vpt + 31) / 32 * 32;
-  auto kern = vpt == 1 ? splitk_reduce_residual_rmsnorm_kernel<1> : splitk_reduce_residual_rmsnorm_kernel<2>;
+  auto kern = vpt == 1   ? splitk_reduce_residual_rmsnorm_kernel<1, RN_MAX_THREADS, 1>
+              : vpt == 2 ? splitk_reduce_residual_rmsnorm_kernel<2, RN_MAX_THREADS, 1>
+                         : splitk_reduce_residual_rmsnorm_kernel<4, RN_MAX_THREADS / 2, 2>;
   return launch_pdl(kern, dim3(M), dim3(threads), 0, stream, ws, splits, M, H, (const __nv_bfloat16*)res_in,
                     (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)res_out, (__nv_bfloat16*)y) == cudaSuccess
              ? 0 : B200_ERR_LAUNCH;

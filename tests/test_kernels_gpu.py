@@ -1355,3 +1355,17 @@ def test_swiglu_vectors_a_thread(T, I):
     assert torch.allclose(y.double(), a * s * b, rtol=2 ** -8, atol=1e-5)
     want = torch.cat([g.double() * b * (s + a * s * (1 - s)), g.double() * a * s], -1)
     assert torch.allclose(dx.double(), want, rtol=2 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("M", [148, 149, 256])
+@pytest.mark.parametrize("N,K", [(4096, 256), (4100, 320), (5120, 1032), (8192, 64)])
+def test_skinny_residual_norm_rows_that_share_an_sm(M, N, K):
+    torch.manual_seed(82)
+    x, w, res, nw = _bf16(M, K), _bf16(N, K, scale=0.05), _bf16(M, N), _bf16(N)
+    y, r = F.skinny_linear_residual_rmsnorm(x, w, res, nw, 1e-6)
+    native.read_status(x.device)
+    want = x.double() @ w.double().t() + res.double()
+    assert torch.allclose(r.double(), want, rtol=2 ** -8, atol=1e-4 * math.sqrt(K))       # fp32 sums, rounded once to bf16
+    h = r.double()                                                                        # the norm sees what is stored
+    assert torch.allclose(y.double(), h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * nw.double(), rtol=2 ** -8,
+                          atol=1e-6)
