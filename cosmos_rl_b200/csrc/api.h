@@ -113,7 +113,6 @@ int b200_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y
 // dx (+ dres), dw [H] bf16 (nullable); ws: fp32 scratch of 296 * max(H, 1024) elements (unused without dw)
 int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                       void* dw, float* ws, long long T, int H, cudaStream_t stream);
-int b200_colsum_f32(const float* partial, float* out, int rows, int cols, int accumulate, cudaStream_t stream);
 int b200_rope_inplace(void* q, void* k, const long long* positions, int T, int hq, int hkv, int d, long long q_stride,
                       long long k_stride, float theta, int backward, cudaStream_t stream);
 // row_tiles (device, nullable): only the first row_tiles[0] * 128 of the T rows are in use.

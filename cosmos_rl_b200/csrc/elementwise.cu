@@ -355,15 +355,6 @@ rmsnorm_dw_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __r
   }
 }
 
-__global__ void colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows, int cols,
-                              int accumulate) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += partial[(long long)r * cols + c];
-  out[c] = accumulate ? out[c] + s : s;
-}
-
 // ------------------------------------------------------------------------------------------------
 // RoPE (rotate-half convention), in place, cos/sin evaluated in fp32 from the integer position
 // ------------------------------------------------------------------------------------------------
@@ -658,11 +649,6 @@ int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float*
     else go(rmsnorm_bwd_kernel<2, 2, 1>, 2, RMSNORM_WS_ROWS / 2);
   }
   if (dw) rmsnorm_dw_sum_kernel<<<(H + 31) / 32, 256, 0, stream>>>(ws, (__nv_bfloat16*)dw, rows, H);
-  return ok();
-}
-
-int b200_colsum_f32(const float* partial, float* out, int rows, int cols, int accumulate, cudaStream_t stream) {
-  colsum_kernel<<<(cols + 255) / 256, 256, 0, stream>>>(partial, out, rows, cols, accumulate);
   return ok();
 }
 

@@ -1,10 +1,10 @@
 // Varlen causal flash-attention backward on tcgen05 / TMEM / TMA (head_dim 128, GQA, packed sequences).
 //
-// Two kernels, each owning its outputs, so nothing is accumulated through memory (no fp32 dQ buffer, no atomics, the
+// Two kernels (short sequences: one, flash_bwd_short.cuh), each owning its outputs, so nothing is accumulated through memory (no fp32 dQ buffer, no atomics, the
 // same bits on every run):
 //
-//   dQ     one item = (sequence, 128-query block, query head); loops over the 128-key blocks it can see. One CTA per SM
-//          works through items (flash_sched.cuh): loads and the first products of the next one run under the end of this
+//   dQ     one item = (sequence, 128-query block, query head); loops over the 128-key blocks it can see. CTAs take items
+//          one after the other (flash_sched.cuh): loads and the first products of the next one run under the end of this
 //          one.
 //          S  = Q K^T          M=queries N=keys K=d        TMEM S[j&1]
 //          dP = dO V^T         M=queries N=keys K=d        TMEM dP
@@ -25,7 +25,6 @@
 // L2 as well. With P and dS taken from TMEM the five products per tile of the two accumulations need 32 KB each.
 // The tensor core runs the products in the order in which the one issuing thread gives them; a product that
 // overwrites the columns of an operand of the product before it (S over P, dP over dS) relies on that order.
-// Timing: profiles/flash_attention_B16_L4096.md.
 // Roles of both: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 softmax (two per TMEM lane quadrant, 64 columns
 // each). All waits are bounded; on a timeout a status code is recorded and the CTA leaves with its TMEM freed.
 // Replaces flash_attn's varlen backward (cosmos_rl/policy/kernel/modeling_utils.py:65-173).

@@ -24,7 +24,6 @@ struct StoreEpilogue {
     store_chunk(p.C, p.ldc, p.M, p.N, p.out_fp32, p.accumulate, (long long)t.m_blk * GEMM_BM + row,
                 t.n_blk * p.bn + col0, v);
   }
-  // shared with the grouped GEMM epilogue
   static __device__ __forceinline__ void store_chunk(void* C, long long ldc, long long M, int N, int out_fp32,
                                                      int accumulate, long long r, int c, const float (&v)[32]) {
     if (r >= M || c >= N) return;

@@ -485,7 +485,9 @@ static int skinny_bn(int M, int N, int swiglu, int num_sms) {
 
 // SwiGLU: columns per tile when every SM gets one tile of that width, or 0 when fixed 64-column tiles are as good. Tiles
 // of 64 columns cost whole rounds: 14336 columns are 224 tiles, two rounds of 148 SMs for 1.5 rounds of work, while
-// 104-column tiles are one round of 138.
+// 104-column tiles are one round of 138 (16 to 128 rows x 4096: 46 to 49 us, in 64-column tiles 52 to 55; 12288 columns: 40 to
+// 42 and 51 to 53). A width that saves less than a twentieth loses to the store boxes of the fixed tiles: 18944 columns, where
+// it would be 128 in one round instead of 64 in two, 16 rows x 3584: 50.8 us, fixed 47.5.
 static int swiglu_width(int M, int N, int num_sms) {
   const int num_m = (M + b200::GEMM_BM - 1) / b200::GEMM_BM;
   if (num_m > num_sms) return 0;
@@ -570,6 +572,9 @@ int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, 
   if (make_tmap_2d(&tmA, x, M, K, ldx, a_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, W, n_rows_w, K, ldw, swiglu ? b_rows / 2 : b_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (ws ? make_tmap_ws(&tmO, ws, splits, M, N) : make_tmap_out16(&tmO, out, M, N, ldo)) return B200_ERR_TENSORMAP;
+  // Blocks of weights that a CTA brings into L2 ahead of its predecessor's end: a decode block of five sequences (8B) takes
+  // 135.5 us without, 131.7 with half or all of this, 134.4 with twice as much; at 128 sequences (7B) 180.2, 179.7, 180.3 and
+  // 182.3: more than the pipeline's own depth competes with the kernel that still runs.
   SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, (__nv_bfloat16*)out, ldo, up_row0,
                   b_rows, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
   auto launch = [&](auto rows) -> int {

@@ -146,7 +146,7 @@ __global__ void logprob_combine_kernel(const float* __restrict__ partial, const 
 // ---------------------------------------------------------------------------------------------
 // backward: dlogits chunk
 // ---------------------------------------------------------------------------------------------
-// single-CTA form, for up to 128 rows (the pair form is an epilogue of gemm_2cta.cuh)
+// single-CTA form, for up to 128 rows and for results off the 16-byte grid (the pair form is an epilogue of gemm_2cta.cuh)
 struct DlogitsEpilogue {
   struct Params {
     DlogitsParams dl;

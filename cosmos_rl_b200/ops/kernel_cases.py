@@ -362,7 +362,7 @@ def case_flash(iters, B=16, L=4096, library=True):
     out, lse = attention.flash_fwd(q, k, v, cu, cu, L, 1.0 / math.sqrt(d))
     go = torch.randn_like(out)
     t = timed(lambda: attention.flash_bwd(go, q, k, v, out, lse, cu, L, 1.0 / math.sqrt(d)), iters)
-    report(f"flash_bwd tcgen05 (same shape, incl. delta pre-pass and dQ cast)", t, flops=2.5 * flops)
+    report(f"flash_bwd tcgen05 (same shape)", t, flops=2.5 * flops)
     if library:
         t = timed(lambda: attention.flash_bwd_library(go, q, k, v, out, lse, cu, L, 1.0 / math.sqrt(d)), iters)
         report(f"flash_attn library bwd (same shape)", t, flops=2.5 * flops)
