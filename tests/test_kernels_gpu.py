@@ -1369,3 +1369,22 @@ def test_skinny_residual_norm_rows_that_share_an_sm(M, N, K):
     h = r.double()                                                                        # the norm sees what is stored
     assert torch.allclose(y.double(), h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * nw.double(), rtol=2 ** -8,
                           atol=1e-6)
+
+
+@pytest.mark.parametrize("h", [2, 40])                              # an SM for every tile of queries, and fewer
+def test_flash_attention_running_maximum_in_both_forms(h):
+    """Scores that grow along the keys by more than the maximum may lag, so the accumulator is rescaled in every key block."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(83)
+    L, d = 700, 128
+    q = torch.ones(L, h, d, device=DEV).to(torch.bfloat16)
+    k = (torch.linspace(0, 40, L, device=DEV)[:, None, None] + torch.zeros(L, h, d, device=DEV)).to(torch.bfloat16)
+    v = _bf16(L, h, d)
+    cu = torch.tensor([0, L], dtype=torch.int32, device=DEV)
+    assert ((L + 127) // 128 * h <= native.num_sms(0)) == (h == 2)
+    for causal in (True, False):
+        out, lse = attention.flash_fwd(q, k, v, cu, cu, L, 1.0 / math.sqrt(d), causal)
+        native.read_status(q.device)
+        ref, ref_lse = R.varlen_attention(q.float(), k.float(), v.float(), cu, 1.0 / math.sqrt(d), causal, return_lse=True)
+        assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2)      # bf16 result and probabilities
+        assert torch.allclose(lse, ref_lse, atol=1e-2, rtol=1e-4)
