@@ -224,7 +224,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     uint32_t kv = 0, nq = 0;   // key blocks and Q tiles so far
     bool ok = true;
     auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar, FB_TILE);
         fb_load_tile(dst, tm, bar, col, row);
       }
@@ -283,7 +283,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       ok = wait(&k_empty[s], ph) && wait(&v_empty[s], ph);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t q_a = smem_u32(q_sh), do_a = smem_u32(do_sh);
       uint32_t kv = 0, nq = 0;
       for (uint32_t it = 0; !*abort_flag; ++it) {
@@ -582,7 +582,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         dl[j] = qi < len_q ? -p.delta[at] : 0.f;
       }
       if (!fb_wait(&q_empty[s], ph, ST_TIMEOUT_EMPTY, p.status, abort_flag)) break;
-      if (lane == 0) {
+      if (elect_one()) {
         if (i == 0) {
           mbar_arrive_expect_tx(k_full, FB_TILE);
           fb_load_tile(k_sh, &tm_k, k_full, hk * FB_D, k_beg + kv0);
@@ -595,7 +595,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
       }
       if (!fb_wait(&do_empty[s], ph, ST_TIMEOUT_EMPTY, p.status, abort_flag)) break;
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_arrive_expect_tx(&do_full[s], FB_TILE);
         fb_load_tile(do_sh + s * FB_TILE, &tm_do, &do_full[s], h * FB_D, q_beg + qr);
       }
@@ -609,7 +609,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       if (lane == 0) mbar_arrive(&st_full[s]);
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && elect_one()) {
       const uint32_t k_a = smem_u32(k_sh), v_a = smem_u32(v_sh);
       do {
         FB_WAIT1(k_full, 0, ST_TIMEOUT_FULL)

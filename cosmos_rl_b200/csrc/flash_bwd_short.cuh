@@ -100,7 +100,7 @@ flash_bwd_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       mbar_arrive_expect_tx(kv_full, 2 * FB_TILE);
       tma_load_2d(k_sh, &tm_k, kv_full, hk * FB_D, k_beg);
       tma_load_2d(k_sh + FB_TILE / 2, &tm_k, kv_full, hk * FB_D + 64, k_beg);
@@ -123,7 +123,7 @@ flash_bwd_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && elect_one()) {
       constexpr uint32_t id_s = umma_idesc_bf16_f32(128, FS_BQ);                                 // both K-major
       constexpr uint32_t id_dkv = umma_idesc_bf16_f32(128, FB_D) | (1u << 16);                   // B MN-major
       constexpr uint32_t id_dq = umma_idesc_bf16_f32(128, FS_BQ) | (1u << 15) | (1u << 16);      // A, B MN-major

@@ -284,7 +284,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         return __all_sync(0xffffffffu, w);
       };
       auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_arrive_expect_tx(bar, FA_TILE);
           tma_load_2d(dst, tm, bar, col, row);
           tma_load_2d(dst + FA_TILE / 2, tm, bar, col + 64, row);
@@ -345,7 +345,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     } else if (warp == 1) {
       // ------------------------------------------------ MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc_s = umma_idesc_bf16_f32(FA_B, FA_B);
         constexpr uint32_t idesc_o = umma_idesc_bf16_f32(FA_B, FA_D) | (1u << 16);   // B (= V) is MN-major
         uint32_t kv = 0, nq[2] = {0, 0}, np[2] = {0, 0};

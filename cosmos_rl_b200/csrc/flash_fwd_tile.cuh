@@ -88,7 +88,7 @@ flash_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (lane == 0 && n > 0) {
+    if (n > 0 && elect_one()) {
       mbar_arrive_expect_tx(qfull, FA_TILE);
       tma_load_2d(q_sh, &tm_q, qfull, h * FA_D, q_beg + q0);
       tma_load_2d(q_sh + FA_TILE / 2, &tm_q, qfull, h * FA_D + 64, q_beg + q0);
@@ -111,7 +111,7 @@ flash_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0 && n > 0) {
+    if (n > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16_f32(FA_B, FA_B);
       constexpr uint32_t idesc_o = umma_idesc_bf16_f32(FA_B, FA_D) | (1u << 16);   // B (= V) is MN-major
       const uint32_t q_addr = smem_u32(q_sh), p_addr = smem_u32(p_sh);

@@ -153,7 +153,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int i = cluster_id; i < total && ok && !*abort_flag; i += num_clusters) {
@@ -207,7 +207,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) --------------------------
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc =
           umma_idesc_bf16_f32(G2_BM, BN) | (A_MN ? (1u << 15) : 0u) | (B_MN ? (1u << 16) : 0u);
       uint32_t stage = 0, phase = 0;
@@ -274,7 +274,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       for (int c = 0; c < OUT_BN; c += slab_cols) {
         uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
         // the store issued two slabs ago has finished reading this buffer
-        if (lane == 0) tma_store_wait_read<1>();
+        if (elect_one()) tma_store_wait_read<1>();
         __syncwarp();
         uint8_t* my_row = slab + lane * 128;
 #pragma unroll
@@ -332,7 +332,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
           const int gc = col_base + c;
           if (gc < n_cols && row0 < M) {
             if (ep.accumulate) tma_reduce_add_2d(tmC, slab, gc, row0);
@@ -347,7 +347,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
-    if (lane == 0) tma_store_wait<0>();
+    if (elect_one()) tma_store_wait<0>();
   }
 
   // ------------------------------ teardown ------------------------------------

@@ -191,7 +191,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       TileInfo t;
       for (int it = 0; sched.get(it, t) && !*abort_flag; ++it) {
@@ -246,7 +246,7 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t idesc = umma_idesc_bf16_f32(GEMM_BM, BN) | (Traits::A_MN ? (1u << 15) : 0u) | (Traits::B_MN ? (1u << 16) : 0u);
       if constexpr (Traits::DYN_N) idesc = umma_idesc_bf16_f32(GEMM_BM, ep.b_rows);
       uint32_t stage = 0, phase = 0;

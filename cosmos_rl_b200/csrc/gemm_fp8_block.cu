@@ -103,7 +103,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       for (int i = blockIdx.x; i < total && !*abort_flag; i += gridDim.x) {
         int m_blk, n_blk;
@@ -119,7 +119,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_e4m3_f32(F8_BM, F8_BN);
       uint32_t stage = 0, phase = 0, it = 0;
       bool ok = true;

@@ -91,7 +91,7 @@ struct SkinnyEpilogue {
   static constexpr bool CUSTOM_TILE = true;
   uint32_t slab_idx = 0;
   __device__ __forceinline__ void finish(const Params&) {
-    if ((threadIdx.x & 31) == 0) tma_store_wait<0>();
+    if (elect_one()) tma_store_wait<0>();
   }
   __device__ __forceinline__ void tile(const Params& p, const TileInfo& t, int row, uint32_t taddr, uint8_t* epi_smem) {
     constexpr int OUT_BN = SWIGLU ? BN / 2 : BN;
@@ -105,7 +105,7 @@ struct SkinnyEpilogue {
 #pragma unroll 1
     for (int c = 0; c < OUT_BN; c += slab_cols) {
       uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
-      if (lane == 0) tma_store_wait_read<1>();  // the store issued two slabs ago has finished reading this buffer
+      if (elect_one()) tma_store_wait_read<1>();  // the store issued two slabs ago has finished reading this buffer
       __syncwarp();
       uint8_t* my_row = slab + lane * 128;
 #pragma unroll
@@ -156,7 +156,7 @@ struct SkinnyEpilogue {
       }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         const int gc = t.n_blk * OUT_BN + c;
         if (gc < p.N && row0 < p.M) {
           if (p.to_ws) tma_store_3d(p.tm_out, slab, gc, row0, t.batch);

@@ -38,7 +38,7 @@ struct GroupedEpilogue {
   static constexpr bool CUSTOM_TILE = true;
   uint32_t slab_idx = 0;
   __device__ __forceinline__ void finish(const Params&) {
-    if ((threadIdx.x & 31) == 0) tma_store_wait<0>();
+    if (elect_one()) tma_store_wait<0>();
   }
   __device__ __forceinline__ void tile(const Params& p, const TileInfo& t, int, uint32_t taddr, uint8_t* epi_smem) {
     const int lane = threadIdx.x & 31, quad = (threadIdx.x >> 5) & 3;
@@ -52,7 +52,7 @@ struct GroupedEpilogue {
       const int gc = t.n_blk * p.bn + c;
       if (gc >= p.N) break;
       uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
-      if (lane == 0) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
+      if (elect_one()) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
       __syncwarp();
       uint8_t* my_row = slab + lane * 128;
       uint32_t r[2][32];
@@ -89,7 +89,7 @@ struct GroupedEpilogue {
       }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         if (row0 < p.rows_limit) {
           if (p.accumulate && p.out_fp32) tma_reduce_add_3d(p.tm_out, slab, gc, row0, batch);
           else tma_store_3d(p.tm_out, slab, gc, row0, batch);

@@ -169,7 +169,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t kv_it = 0, item_it = 0;
       // work items with an empty token range are skipped by every role (item_it counts the others)
       for (int item = blockIdx.x; item < n_items && !*abort_flag; item += gridDim.x) {
@@ -206,7 +206,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     // ------------------------------------------------ MMA issuer
     // S^T of tile t+1 (also the first tile of the next work item) is issued before the softmax warps have finished
     // tile t: S, P and the query tile are double-buffered, so the K.Q^T product never waits for the softmax.
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16_f32(128, PDT_N);
       uint32_t kv_it = 0, item_it = 0;
       const uint32_t q_base = smem_u32(q_sh), p_base = smem_u32(p_sh);
@@ -542,7 +542,7 @@ paged_prefix_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base + 128;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t q_bytes = 2u * (uint32_t)rows_used * 128u;
       mbar_arrive_expect_tx(qk_full, q_bytes + PDT_SLAB_BYTES);
       tma_load_3d(q_sh, &tm_q3, qk_full, 0, hk * G, s0);
@@ -556,7 +556,7 @@ paged_prefix_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
       tma_load_2d(v_sh + PDT_SLAB_BYTES / 2, &tm_cache, v_full, 64, vrow);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16_f32(128, 128);
       const uint32_t q_a = smem_u32(q_sh), k_a = smem_u32(k_sh), v_a = smem_u32(v_sh), p_a = smem_u32(p_sh);
       do {
