@@ -14,10 +14,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
 // How many CTA pairs can be resident at once (asked once per kernel and device; <= num_sms / 2).
 template <class Kern>
-static int max_pairs(Kern kern, int smem_bytes, int num_sms) {
+static int max_pairs(Kern kern, int smem_bytes, int num_sms, int threads = G2_THREADS) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (num_sms / 2), 1, 1);
-  cfg.blockDim = dim3(G2_THREADS, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem_bytes;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;

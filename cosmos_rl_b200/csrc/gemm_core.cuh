@@ -64,12 +64,13 @@ struct TileInfo {
 // t.b_mn1 (gate and up rows of a fused gate/up weight, so that one accumulator row holds both).
 // L2_PREFETCH (B not MN-major, 2-D): before the CTA waits for the previous kernel of the stream it brings the first
 // ep.prefetch_kb contraction blocks of its B tiles into L2. The schedule's init() may then read nothing but Params.
-// A_ROWS (A K-major, 2-D): see GemmSmem; the tensor map's box has that many rows.
+// A_ROWS (A K-major, 2-D): see GemmSmem; the tensor map's box has that many rows, or with DYN_A the number chosen at launch
+// (ep.a_bytes a stage).
 // DYN_N (B K-major): a tile has ep.b_rows <= BN rows of B (a multiple of 16), chosen at launch; the boxes of B have
 // ep.b_rows rows, or ep.b_rows / 2 with B_TWO_BOXES.
 template <bool A_MN_ = false, bool B_MN_ = false, bool A_3D_ = false, bool B_3D_ = false, int SIDE_WARPS_ = 0,
           bool PRODUCER_HOOK_ = false, bool B_TWO_BOXES_ = false, bool L2_PREFETCH_ = false, int A_ROWS_ = GEMM_BM,
-          bool DYN_N_ = false>
+          bool DYN_N_ = false, bool DYN_A_ = false>
 struct GemmTraits {
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_, A_3D = A_3D_, B_3D = B_3D_;
   static constexpr int SIDE_WARPS = SIDE_WARPS_;
@@ -78,6 +79,7 @@ struct GemmTraits {
   static constexpr bool L2_PREFETCH = L2_PREFETCH_;
   static constexpr int A_ROWS = A_ROWS_;
   static constexpr bool DYN_N = DYN_N_;
+  static constexpr bool DYN_A = DYN_A_;
 };
 
 // An epilogue that declares `static constexpr bool CUSTOM_TILE = true` reads its accumulator itself:
@@ -213,10 +215,10 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
           uint32_t b_half = SM::B_BYTES / 2;   // B_TWO_BOXES: bytes of one box
           if constexpr (Traits::DYN_N) {
             b_half = ep.b_rows * (GEMM_BK * 2 / 2);
-            mbar_arrive_expect_tx(&full_bar[stage], SM::A_BYTES + 2 * b_half);
-          } else {
-            mbar_arrive_expect_tx(&full_bar[stage], SM::STAGE_BYTES);
           }
+          uint32_t a_bytes = SM::A_BYTES;
+          if constexpr (Traits::DYN_A) a_bytes = ep.a_bytes;
+          mbar_arrive_expect_tx(&full_bar[stage], a_bytes + 2 * b_half);
           if constexpr (!Traits::A_MN) {
             if constexpr (Traits::A_3D) tma_load_3d(sa, tmA, &full_bar[stage], k, t.a_mn0, t.batch);
             else tma_load_2d(sa, tmA, &full_bar[stage], k, t.a_mn0);

@@ -31,6 +31,10 @@ struct SkinnyCfg {
   static_assert(GemmSmem<256, ROW_STORE_STAGES, A_ROWS>::TOTAL <= SMEM_LIMIT, "shared memory");
 };
 
+// Gate value of accumulator rows that belong to no row of x and are not stored. What they hold (zeros, whatever follows the
+// tile) sends the whole warp through the division's path for special operands: gate/up of 14336 x 4096, 5 rows 57.6 us, 45.
+constexpr float SKINNY_NO_ROW = 1.f;
+
 struct SkinnyParams {
   const CUtensorMap* tm_out;  // bf16 [M, N] (direct output) or fp32 [splits, M, N] (partials), boxes of 32 rows x 128 bytes
   const void* bias;           // [N], nullable (direct output only; the reduce kernels add it otherwise)
@@ -42,6 +46,7 @@ struct SkinnyParams {
   long long ldo;
   int up_row0;                // SwiGLU: first "up" row of W
   int b_rows;                 // rows of W per tile (BN, or the width chosen at launch)
+  int a_bytes;                // bytes of A a stage: the rows that are fetched
   int prefetch_kb;            // contraction blocks a CTA brings into L2 before it waits for the previous kernel
 };
 
@@ -121,7 +126,7 @@ struct SkinnyEpilogue {
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            const float g = __uint_as_float(a[j]);
+            const float g = row0 + lane < p.M ? __uint_as_float(a[j]) : SKINNY_NO_ROW;
             v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
           }
         } else {
@@ -188,7 +193,7 @@ struct SwigluRowsEpilogue {
       float v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const float g = __uint_as_float(a[j]);
+        const float g = r < p.M ? __uint_as_float(a[j]) : SKINNY_NO_ROW;
         v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
       }
       if (r >= p.M) continue;
@@ -220,7 +225,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   ep.tm_out = &tmO;
   if (threadIdx.x == 0) tma_prefetch_desc(&tmO);
   gemm_mainloop<BN, SkinnyCfg<BN, A_ROWS>::STAGES, SkinnyEpilogue<BN, SWIGLU>, SkinnySchedule<BN, SWIGLU>,
-                GemmTraits<false, false, false, false, 0, false, SWIGLU, true, A_ROWS>>(&tmA, &tmB, M, N, K, ep, status);
+                GemmTraits<false, false, false, false, 0, false, SWIGLU, true, A_ROWS, false, true>>(&tmA, &tmB, M, N, K, ep, status);
 }
 
 template <int A_ROWS>
@@ -228,7 +233,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_skinny_swiglu_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
                                int N, int K, SkinnyParams ep, uint32_t* status) {
   gemm_mainloop<256, SkinnyCfg<256, A_ROWS>::ROW_STORE_STAGES, SwigluRowsEpilogue, SkinnySchedule<256, true>,
-                GemmTraits<false, false, false, false, 0, false, true, true, A_ROWS, true>>(&tmA, &tmB, M, N, K, ep, status);
+                GemmTraits<false, false, false, false, 0, false, true, true, A_ROWS, true, true>>(&tmA, &tmB, M, N, K, ep, status);
 }
 
 // fp32 [splits, M, N] partials: boxes of 32 rows x 32 columns, 128-byte swizzle
@@ -568,15 +573,17 @@ int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, 
   const int width = swiglu ? swiglu_width(M, N, num_sms) : 0;
   const int bn = width ? 256 : skinny_bn(M, N, swiglu, num_sms);
   const int b_rows = width ? 2 * width : bn, a_rows = skinny_a_rows(M);
+  // Exactly the rows there are: a row of a box that lies outside the tensor takes longer than one that is fetched.
+  const int box_rows = M < a_rows ? M : a_rows;
   CUtensorMap tmA, tmB, tmO;
-  if (make_tmap_2d(&tmA, x, M, K, ldx, a_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tmA, x, M, K, ldx, box_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, W, n_rows_w, K, ldw, swiglu ? b_rows / 2 : b_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (ws ? make_tmap_ws(&tmO, ws, splits, M, N) : make_tmap_out16(&tmO, out, M, N, ldo)) return B200_ERR_TENSORMAP;
   // Blocks of weights that a CTA brings into L2 ahead of its predecessor's end: a decode block of five sequences (8B) takes
   // 135.5 us without, 131.7 with half or all of this, 134.4 with twice as much; at 128 sequences (7B) 180.2, 179.7, 180.3 and
   // 182.3: more than the pipeline's own depth competes with the kernel that still runs.
   SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, (__nv_bfloat16*)out, ldo, up_row0,
-                  b_rows, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
+                  b_rows, box_rows * GEMM_BK * 2, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
   auto launch = [&](auto rows) -> int {
     constexpr int R = decltype(rows)::value;
     if (width) return launch_swiglu_rows<R>(tmA, tmB, M, N, K, ep, status, num_sms, stream);

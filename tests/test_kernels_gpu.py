@@ -543,6 +543,45 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
+# one row; K of one block, of less than one, of 4 n + 1 blocks; columns that end inside 16 bytes; CTA pairs (enough tiles for
+# two rounds of single CTAs) with ragged rows and columns, and with more tiles than pairs
+@pytest.mark.parametrize("M,N,K", [(1, 264, 128), (3, 5, 144), (1, 4096, 640), (127, 1001, 112), (129, 19000, 128),
+                                   (257, 19197, 656), (2000, 12300, 400)])
+def test_gemm_fp8_block_forms(M, N, K):
+    torch.manual_seed(M)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    aq, sa = F.quant_fp8_block(a, 1)
+    bq, sb = F.quant_fp8_block(b, 128)
+    out = torch.full((M + 1, (N + 7) // 8 * 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    F.gemm_fp8_block(aq, sa, bq, sb, out=out[:M, :N])
+    torch.cuda.synchronize()
+    assert native.read_status(a.device) == 0
+    ref = R.dequant_fp8_block(aq, sa, 1, 128).double() @ R.dequant_fp8_block(bq, sb, 128, 128).double().t()
+    # one rounding to bf16 (2^-9) and the fp32 sums of K products, which a 64-bit sum bounds by 2^-24 K |a| |b|
+    bound = ref.abs() * 2.0 ** -8 + 2.0 ** -20 * K ** 0.5 * (a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=1)) + 1e-6
+    assert ((out[:M, :N].double() - ref).abs() <= bound).all()
+    assert (out[M] == 7.0).all() and (out[:M, N:] == 7.0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 13, 33, 127, 129])
+@pytest.mark.parametrize("inter,K", [(1536, 512), (14336, 256)])
+def test_gate_up_rows_that_fill_no_box(M, inter, K):
+    """Row counts between the sizes of the activation tiles: boxes of exactly those rows, and nothing of the accumulator's
+    other rows reaches the result."""
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2 * inter, K, device="cuda") * 0.05).to(torch.bfloat16)
+    got = F.skinny_gate_up_swiglu(x, w)
+    torch.cuda.synchronize()
+    assert native.read_status(x.device) == 0
+    h = x.double() @ w.double().t()
+    ref = torch.nn.functional.silu(h[:, :inter]) * h[:, inter:]
+    assert (got.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() + 1e-5   # one rounding, fp32 sums
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("hq,hkv,n", [(28, 4, 4), (8, 8, 8), (64, 8, 3), (28, 4, 8)])
 def test_paged_decode_shared_prefix_groups(hq, hkv, n):
     """Groups of n sequences share their first pages; the prefix pass + suffix pass + merge must equal plain
