@@ -11,6 +11,10 @@
 //          dS = exp2(S c - lse) o (dP - delta)             softmax warps, bf16 into the columns of dP
 //          dQ += dS K          M=queries N=d K=keys        A = dS out of TMEM, B = the K tile read MN-major
 //          delta = rowsum(O o dO) of its rows is formed first and left in memory for the second kernel.
+//          K has three slots: a block is needed from S until dQ, and with two the load of block j + 1 starts when dQ of block
+//          j - 1 is through and S of j + 1 waits for it (3600 and 2340 tokens, 16 heads, no mask: 296 us, 244 with
+//          three; 16384 tokens, 32 heads: 2874 and 2494). The
+//          result passes through the K slot that the item read last, since there is no room for staging of its own.
 //   dK, dV one CTA = (sequence, 128-key block, kv head); loops over the query heads of its GQA group and the
 //          128-query blocks that can see the key block
 //          S^T  = K Q^T        M=keys N=queries K=d        TMEM S
@@ -40,8 +44,7 @@ constexpr int FB_D = 128;
 constexpr int FB_TILE = FB_B * FB_D * 2;             // 32 KiB, two boxes of 128 rows x 64 elements
 constexpr int FB_STATS = 2 * 2 * FB_B * 4;           // dK/dV kernel: lse and delta of two query blocks
 constexpr int FB_SMEM = 6 * FB_TILE + FB_STATS + 256 + 1024;          // dK/dV kernel
-constexpr int FB_OUT_BYTES = 8 * 4096;                                // dQ kernel: epilogue staging, 4 KB a warp
-constexpr int FB_SMEM_DQ = 6 * FB_TILE + FB_OUT_BYTES + 512 + 1024;
+constexpr int FB_SMEM_DQ = 7 * FB_TILE + 512 + 1024;                  // dQ kernel: Q, dO, K x3, V x2
 constexpr int FB_THREADS = 320;                      // TMA warp, MMA warp, 8 softmax warps
 constexpr float FB_LOG2E = 1.4426950408889634f;
 
@@ -156,27 +159,26 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_sh = smem;
   uint8_t* do_sh = smem + FB_TILE;
-  uint8_t* k_sh = smem + 2 * FB_TILE;                  // [2]
-  uint8_t* v_sh = smem + 4 * FB_TILE;                  // [2]
-  uint8_t* out_sh = smem + 6 * FB_TILE;                // [8 warps][32 rows][128 bytes]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(out_sh + FB_OUT_BYTES);
+  uint8_t* k_sh = smem + 2 * FB_TILE;                  // [3]
+  uint8_t* v_sh = smem + 5 * FB_TILE;                  // [2]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * FB_TILE);
   uint64_t* q_full = bars;
   uint64_t* q_empty = bars + 1;
   uint64_t* do_full = bars + 2;
   uint64_t* do_empty = bars + 3;
-  uint64_t* k_full = bars + 4;     // [2]
-  uint64_t* v_full = bars + 6;     // [2]
-  uint64_t* k_empty = bars + 8;    // [2]
-  uint64_t* v_empty = bars + 10;   // [2]
-  uint64_t* s_ready = bars + 12;   // [2]
-  uint64_t* dp_ready = bars + 14;
-  uint64_t* ds_ready = bars + 15;
-  uint64_t* done = bars + 16;
-  uint64_t* item_full = bars + 17;   // [2] slots of the work queue
-  uint64_t* item_empty = bars + 19;  // [2] read by the MMA thread and the eight softmax warps
-  FlashItem* items = reinterpret_cast<FlashItem*>(bars + 22);   // [2]
-  // bars + 30: 16 bytes and bars + 21: barrier of cluster launch control
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
+  uint64_t* k_full = bars + 4;       // [3]
+  uint64_t* v_full = bars + 7;       // [2]
+  uint64_t* k_empty = bars + 9;      // [3]
+  uint64_t* v_empty = bars + 12;     // [2]
+  uint64_t* s_ready = bars + 14;     // [2]
+  uint64_t* dp_ready = bars + 16;
+  uint64_t* ds_ready = bars + 17;
+  uint64_t* done = bars + 18;
+  uint64_t* item_full = bars + 19;   // [2] slots of the work queue
+  uint64_t* item_empty = bars + 21;  // [2] read by the MMA thread and the eight softmax warps
+  FlashItem* items = reinterpret_cast<FlashItem*>(bars + 24);   // [2]
+  // bars + 32: 16 bytes and bars + 23: barrier of cluster launch control
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 34);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -185,16 +187,18 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     mbar_init(q_empty, 1);
     mbar_init(do_full, 1);
     mbar_init(do_empty, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < 3; ++s) {
       mbar_init(&k_full[s], 1);
-      mbar_init(&v_full[s], 1);
       mbar_init(&k_empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 1);
       mbar_init(&s_ready[s], 1);
       mbar_init(&item_full[s], 1);
       mbar_init(&item_empty[s], 9);
     }
-    mbar_init(bars + 21, 1);
+    mbar_init(bars + 23, 1);
     mbar_init(dp_ready, 1);
     mbar_init(ds_ready, 8);
     mbar_init(done, 1);
@@ -220,7 +224,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     // ---- scheduler and TMA producer (whole warp, lane 0 issues)
     FlashWork work;
     work.list.init(p.cu_q, p.B, FB_B, p.hq, p.levels_q, !p.causal);
-    work.init(reinterpret_cast<uint4*>(bars + 30), bars + 21);
+    work.init(reinterpret_cast<uint4*>(bars + 32), bars + 23);
     uint32_t kv = 0, nq = 0;   // key blocks and Q tiles so far
     bool ok = true;
     auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
@@ -258,14 +262,16 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const int n = fb_key_blocks(w, p.causal), hk = w.head / (p.hq / p.hkv), qrow = w.q_beg + w.row0;
       for (int j = 0; j < n; ++j, ++kv) {
         if (j + 2 >= n) work.request();   // the answer comes while the last blocks wait for their buffers
-        const uint32_t s = kv & 1, ph = ((kv >> 1) & 1) ^ 1;
+        const uint32_t s = kv & 1, ph = ((kv >> 1) & 1) ^ 1, ks = kv % 3;
         const int row = w.k_beg + j * FB_B;
         if (j == 0) {
           if (!(ok = wait(q_empty, (nq & 1) ^ 1))) break;
           load(q_sh, &tm_q, q_full, w.head * FB_D, qrow);
         }
-        if (!(ok = wait(&k_empty[s], ph))) break;
-        load(k_sh + s * FB_TILE, &tm_k, &k_full[s], hk * FB_D, row);
+        // the third block goes where the previous item's result passes through on its way out
+        if (j == 2 && it > 0 && !(ok = wait(&item_empty[slot ^ 1], ((it - 1) >> 1) & 1))) break;
+        if (!(ok = wait(&k_empty[ks], (kv / 3 & 1) ^ 1))) break;
+        load(k_sh + ks * FB_TILE, &tm_k, &k_full[ks], hk * FB_D, row);
         if (j == 0) {
           if (!(ok = wait(do_empty, (nq & 1) ^ 1))) break;
           load(do_sh, &tm_do, do_full, w.head * FB_D, qrow);
@@ -278,10 +284,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     work.finish();
     // the tensor core's last arrivals on these barriers land before the CTA's shared memory is released
     if (ok) ok = wait(q_empty, (nq & 1) ^ 1) && wait(do_empty, (nq & 1) ^ 1);
-    for (int i = 0; i < 2 && ok; ++i, ++kv) {
-      const uint32_t s = kv & 1, ph = ((kv >> 1) & 1) ^ 1;
-      ok = wait(&k_empty[s], ph) && wait(&v_empty[s], ph);
-    }
+    for (int i = 0; i < 3 && ok; ++i, ++kv)
+      ok = wait(&k_empty[kv % 3], (kv / 3 & 1) ^ 1) && (i == 2 || wait(&v_empty[kv & 1], ((kv >> 1) & 1) ^ 1));
   } else if (warp == 1) {
     if (elect_one()) {
       const uint32_t q_a = smem_u32(q_sh), do_a = smem_u32(do_sh);
@@ -295,9 +299,9 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int n = fb_key_blocks(w, p.causal);
         if (n == 0) continue;
         FB_WAIT1(q_full, nq & 1, ST_TIMEOUT_FULL)
-        FB_WAIT1(&k_full[kv & 1], (kv >> 1) & 1, ST_TIMEOUT_FULL)
+        FB_WAIT1(&k_full[kv % 3], kv / 3 & 1, ST_TIMEOUT_FULL)
         tc_fence_after_sync();
-        fb_mma_ss(tmem_base + (kv & 1) * 128, q_a, smem_u32(k_sh + (kv & 1) * FB_TILE));
+        fb_mma_ss(tmem_base + (kv & 1) * 128, q_a, smem_u32(k_sh + kv % 3 * FB_TILE));
         tc_commit(&s_ready[kv & 1]);
         if (n == 1) tc_commit(q_empty);
         FB_WAIT1(do_full, nq & 1, ST_TIMEOUT_FULL)
@@ -310,11 +314,12 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         if (n == 1) tc_commit(do_empty);
         for (int j = 0; j < n && !*abort_flag; ++j, ++kv) {
           const uint32_t s = kv & 1, s1 = s ^ 1, ph1 = ((kv + 1) >> 1) & 1;
-          const uint32_t k_a = smem_u32(k_sh + s * FB_TILE);
+          const uint32_t ks = kv % 3, ks1 = (kv + 1) % 3;
+          const uint32_t k_a = smem_u32(k_sh + ks * FB_TILE);
           if (j + 1 < n) {   // S of the next block: its buffer was read before dS of the block before this one was announced
-            FB_WAIT1(&k_full[s1], ph1, ST_TIMEOUT_FULL)
+            FB_WAIT1(&k_full[ks1], (kv + 1) / 3 & 1, ST_TIMEOUT_FULL)
             tc_fence_after_sync();
-            fb_mma_ss(tmem_base + s1 * 128, q_a, smem_u32(k_sh + s1 * FB_TILE));
+            fb_mma_ss(tmem_base + s1 * 128, q_a, smem_u32(k_sh + ks1 * FB_TILE));
             tc_commit(&s_ready[s1]);
             if (j + 2 == n) tc_commit(q_empty);
           }
@@ -322,7 +327,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           FB_WAIT1(ds_ready, kv & 1, ST_TIMEOUT_TMEM_EMPTY)
           tc_fence_after_sync();
           fb_mma_ts(tm_dq, tm_dp, k_a, j == 0);
-          tc_commit(&k_empty[s]);
+          tc_commit(&k_empty[ks]);
           if (j + 1 < n) {
             FB_WAIT1(&v_full[s1], ph1, ST_TIMEOUT_FULL)
             tc_fence_after_sync();
@@ -341,7 +346,6 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int c0 = half_id * 64;                         // first key column of this warp
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    uint8_t* stage = out_sh + (warp - 2) * 4096;
     const float2 c2 = make_float2(p.scale_log2, p.scale_log2);
     uint32_t kv = 0, finished = 0;
     bool ok = true;
@@ -440,9 +444,12 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         ++finished;
         tc_fence_after_sync();
       }
+      // the rows leave through the K slot of the item's last block, or of the one before it if it has none
+      uint8_t* stage = k_sh + (kv + 2) % 3 * FB_TILE + (warp - 2) * 4096;
       const int first = w.row0 + quad * 32;
       fb_store_rows(tm_dq + lane_addr + c0, n == 0, p.scale, stage,
                     p.dq + (long long)(w.q_beg + first) * p.lddq + w.head * FB_D + c0, p.lddq, w.len_q - first);
+      fence_proxy_async_smem();                          // a TMA load overwrites the staging rows
       tc_fence_before_sync();                            // dQ has been read: the next item's first product overwrites it
       __syncwarp();
       if (lane == 0) mbar_arrive(&item_empty[slot]);
