@@ -8,13 +8,15 @@
 //          one.
 //          S  = Q K^T          M=queries N=keys K=d        TMEM S[j&1]
 //          dP = dO V^T         M=queries N=keys K=d        TMEM dP
-//          dS = exp2(S c - lse) o (dP - delta)             softmax warps, bf16 into the columns of dP
+//          dS = exp2(S c - lse) o (dP - delta)             softmax warps, bf16 into the columns of S
 //          dQ += dS K          M=queries N=d K=keys        A = dS out of TMEM, B = the K tile read MN-major
 //          delta = rowsum(O o dO) of its rows is formed first and left in memory for the second kernel.
 //          K has three slots: a block is needed from S until dQ, and with two the load of block j + 1 starts when dQ of block
 //          j - 1 is through and S of j + 1 waits for it (3600 and 2340 tokens, 16 heads, no mask: 296 us, 244 with
-//          three; 16384 tokens, 32 heads: 2874 and 2494). The
-//          result passes through the K slot that the item read last, since there is no room for staging of its own.
+//          three). The result passes through the K slot that the item read last, since there is no room for staging of
+//          its own. dS goes into the columns of its S, so that dP of the next block is formed as soon as this one's is in
+//          registers and S two blocks ahead; the loop is then bound by the softmax warps (4096 tokens, 16 heads: 92.5 us with
+//          dS over dP, 91.2).
 //   dK, dV one CTA = (sequence, 128-key block, kv head); loops over the query heads of its GQA group and the
 //          128-query blocks that can see the key block
 //          S^T  = K Q^T        M=keys N=queries K=d        TMEM S
@@ -28,7 +30,9 @@
 // shared memory gives, and in the one-kernel form the transposed dS and the fp32 dQ tile go through shared memory and
 // L2 as well. With P and dS taken from TMEM the five products per tile of the two accumulations need 32 KB each.
 // The tensor core runs the products in the order in which the one issuing thread gives them; a product that
-// overwrites the columns of an operand of the product before it (S over P, dP over dS) relies on that order.
+// overwrites the columns of an operand of the product before it (S over P or dS, dP over dS) relies on that order. In the
+// dK/dV kernel the chain P, dV, S of the next block, exponentials is what is left (3100 cycles an iteration, 2048 of them
+// products); S and dP changing places, with P and dS in the columns of S and the next S under dS, gave the same time.
 // Roles of both: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 softmax (two per TMEM lane quadrant, 64 columns
 // each). All waits are bounded; on a timeout a status code is recorded and the CTA leaves with its TMEM freed.
 // Replaces flash_attn's varlen backward (cosmos_rl/policy/kernel/modeling_utils.py:65-173).
@@ -47,6 +51,10 @@ constexpr int FB_SMEM = 6 * FB_TILE + FB_STATS + 256 + 1024;          // dK/dV k
 constexpr int FB_SMEM_DQ = 7 * FB_TILE + 512 + 1024;                  // dQ kernel: Q, dO, K x3, V x2
 constexpr int FB_THREADS = 320;                      // TMA warp, MMA warp, 8 softmax warps
 constexpr float FB_LOG2E = 1.4426950408889634f;
+// One pair of exponentials in so many runs on the fp32 pipe (exp2_poly2): the two warps of a scheduler are in their exponentials
+// at the same time, 1050 cycles of 1024 that the special-function unit needs for 128 x 128. us with none, a sixth, a quarter, a
+// third and half of them there, 3600 and 2340 tokens, 16 heads, no mask: dQ 195, 191, 193, 193, 195; dK/dV 274, 264, 264, 266, 269.
+constexpr int FB_POLY_DQ = 6, FB_POLY_KV = 4;
 
 struct FbParams {
   const int* cu_q;
@@ -174,6 +182,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* dp_ready = bars + 16;
   uint64_t* ds_ready = bars + 17;
   uint64_t* done = bars + 18;
+  uint64_t* dp_free = bars + 36;     // dP has been read
   uint64_t* item_full = bars + 19;   // [2] slots of the work queue
   uint64_t* item_empty = bars + 21;  // [2] read by the MMA thread and the eight softmax warps
   FlashItem* items = reinterpret_cast<FlashItem*>(bars + 24);   // [2]
@@ -201,6 +210,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     mbar_init(bars + 23, 1);
     mbar_init(dp_ready, 1);
     mbar_init(ds_ready, 8);
+    mbar_init(dp_free, 8);
     mbar_init(done, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -217,7 +227,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // columns: S[2] 0..255, dP (then dS) 256..383, dQ 384..511
+  // columns: S[2] (then dS) 0..255, dP 256..383, dQ 384..511
   const uint32_t tm_dp = tmem_base + 256, tm_dq = tmem_base + 384;
 
   if (warp == 0) {
@@ -312,29 +322,36 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_commit(dp_ready);
         tc_commit(&v_empty[kv & 1]);
         if (n == 1) tc_commit(do_empty);
+        if (n > 1) {
+          FB_WAIT1(&k_full[(kv + 1) % 3], (kv + 1) / 3 & 1, ST_TIMEOUT_FULL)
+          tc_fence_after_sync();
+          fb_mma_ss(tmem_base + ((kv + 1) & 1) * 128, q_a, smem_u32(k_sh + (kv + 1) % 3 * FB_TILE));
+          tc_commit(&s_ready[(kv + 1) & 1]);
+          if (n == 2) tc_commit(q_empty);
+        }
         for (int j = 0; j < n && !*abort_flag; ++j, ++kv) {
-          const uint32_t s = kv & 1, s1 = s ^ 1, ph1 = ((kv + 1) >> 1) & 1;
-          const uint32_t ks = kv % 3, ks1 = (kv + 1) % 3;
-          const uint32_t k_a = smem_u32(k_sh + ks * FB_TILE);
-          if (j + 1 < n) {   // S of the next block: its buffer was read before dS of the block before this one was announced
-            FB_WAIT1(&k_full[ks1], (kv + 1) / 3 & 1, ST_TIMEOUT_FULL)
+          const uint32_t s = kv & 1, s1 = s ^ 1, ks = kv % 3;
+          if (j + 1 < n) {   // dP of the next block, once this one's is in registers
+            FB_WAIT1(dp_free, kv & 1, ST_TIMEOUT_TMEM_EMPTY)
+            FB_WAIT1(&v_full[s1], ((kv + 1) >> 1) & 1, ST_TIMEOUT_FULL)
             tc_fence_after_sync();
-            fb_mma_ss(tmem_base + s1 * 128, q_a, smem_u32(k_sh + ks1 * FB_TILE));
-            tc_commit(&s_ready[s1]);
-            if (j + 2 == n) tc_commit(q_empty);
+            fb_mma_ss(tm_dp, do_a, smem_u32(v_sh + s1 * FB_TILE));
+            tc_commit(dp_ready);
+            tc_commit(&v_empty[s1]);
+            if (j + 2 == n) tc_commit(do_empty);
           }
           // dS also says that the previous item's dQ has been read, which the first product of an item overwrites
           FB_WAIT1(ds_ready, kv & 1, ST_TIMEOUT_TMEM_EMPTY)
           tc_fence_after_sync();
-          fb_mma_ts(tm_dq, tm_dp, k_a, j == 0);
+          fb_mma_ts(tm_dq, tmem_base + s * 128, smem_u32(k_sh + ks * FB_TILE), j == 0);
           tc_commit(&k_empty[ks]);
-          if (j + 1 < n) {
-            FB_WAIT1(&v_full[s1], ph1, ST_TIMEOUT_FULL)
+          if (j + 2 < n) {   // S of the block after the next, over dS of this one
+            const uint32_t ks2 = (kv + 2) % 3;
+            FB_WAIT1(&k_full[ks2], (kv + 2) / 3 & 1, ST_TIMEOUT_FULL)
             tc_fence_after_sync();
-            fb_mma_ss(tm_dp, do_a, smem_u32(v_sh + s1 * FB_TILE));   // dP of the next block, over dS
-            tc_commit(dp_ready);
-            tc_commit(&v_empty[s1]);
-            if (j + 2 == n) tc_commit(do_empty);
+            fb_mma_ss(tmem_base + s * 128, q_a, smem_u32(k_sh + ks2 * FB_TILE));
+            tc_commit(&s_ready[s]);
+            if (j + 3 == n) tc_commit(q_empty);
           }
         }
         if (!*abort_flag) tc_commit(done);
@@ -411,7 +428,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int i = 0; i < 32; ++i) {
           const uint32_t(&r)[32] = rs[i >> 4];
           const float2 x = fma2(make_float2(__uint_as_float(r[2 * (i & 15)]), __uint_as_float(r[2 * (i & 15) + 1])), c2, nl2);
-          e[i] = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+          e[i] = i % FB_POLY_DQ == FB_POLY_DQ - 1 ? exp2_poly2(x) : make_float2(exp2_approx(x.x), exp2_approx(x.y));
         }
         if (key0 + 64 > k_limit) {
 #pragma unroll
@@ -426,13 +443,16 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tmem_ld_32x32b_x32(tm_dp + lane_addr + c0, rp[0]);
         tmem_ld_32x32b_x32(tm_dp + lane_addr + c0 + 32, rp[1]);
         tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dp_free);
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const uint32_t(&r)[32] = rp[i >> 4];
           const float2 v = mul2(e[i], add2(make_float2(__uint_as_float(r[2 * (i & 15)]), __uint_as_float(r[2 * (i & 15) + 1])), nd2));
           ds[i] = pack_bf16x2(v.x, v.y);
         }
-        tmem_st_32x32b_x32(tm_dp + lane_addr + c0, ds);   // over the first half of the columns just read
+        tmem_st_32x32b_x32(tmem_base + s * 128 + lane_addr + c0, ds);   // over the first half of this warp's columns of S
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
@@ -688,7 +708,8 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             const float2 x = fma2(make_float2(__uint_as_float(r[4 * g + 2 * u]), __uint_as_float(r[4 * g + 2 * u + 1])), c2, nl[g]);
-            e[2 * hf + u][g] = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+            e[2 * hf + u][g] = (2 * g + u) % FB_POLY_KV == FB_POLY_KV - 1 ? exp2_poly2(x)
+                                                                          : make_float2(exp2_approx(x.x), exp2_approx(x.y));
           }
       }
       // a query sees a key iff q >= key - shift (causal); queries past the end have no probabilities

@@ -8,9 +8,10 @@
 //     O_t += P_t V_j            A = P_t out of TMEM, B = V MN-major, so the [token, d] layout is used as stored
 // While the softmax warps of one tile work, the tensor core runs the two products of the other. Reading P out of TMEM
 // and sharing K / V between the tiles leaves 192 KB of shared-memory reads per key block for 2048 tensor-core cycles.
-// The softmax chain of a tile is what bounds a long item. (A quarter of the exponentials on the fp32 pipe instead of the
-// special-function unit, and P handed over in halves, both measured nothing: 1.96 and 1.89 ms against 1.87 ms for one
-// sequence of 16384 tokens, 32 heads.) A short item is bound by what surrounds the loop, so items follow each other
+// The softmax chain of a tile is what bounds a long item (2400 cycles; the products of both tiles take 2048). A quarter of the
+// exponentials runs on the fp32 pipe instead of the special-function unit: 3600 and 2340 tokens, 16 heads, no mask: 154 us, none
+// 159, a third 153, half 171. (P handed over in halves measured nothing: 1.89 ms against 1.87 ms for one sequence of 16384
+// tokens, 32 heads.) A short item is bound by what surrounds the loop, so items follow each other
 // without a break: loads and the first S of the next one run under the epilogue of this one.
 // O stays in TMEM for the whole item and is rescaled lazily: the running maximum only moves when it grows by more than
 // 2^8, so the TMEM read-modify-write of O is rare. S_t(j+1) is issued after P_t(j) V_j by the same thread and the tensor
@@ -38,6 +39,7 @@ constexpr int FA_THREADS = 384;
 constexpr float FA_LOG2E = 1.4426950408889634f;
 constexpr float FA_LN2 = 0.6931471805599453f;
 constexpr float FA_RESCALE_TAU = 8.0f;
+constexpr int FA_POLY = 4;                         // one pair of exponentials in so many runs on the fp32 pipe
 
 struct FaParams {
   const int* cu_q;
@@ -204,7 +206,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const float2 x = fma2(make_float2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), c2, nm2);
-              const float2 e = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+              const float2 e = i % FA_POLY == FA_POLY - 1 ? exp2_poly2(x) : make_float2(exp2_approx(x.x), exp2_approx(x.y));
               sum[c] = add2(sum[c], e);
               pk[(c & 1) * 16 + i] = pack_bf16x2(e.x, e.y);
             }

@@ -543,6 +543,44 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("n,hq,hkv", [(129, 4, 2), (700, 16, 4), (1200, 16, 16)])
+def test_attention_far_apart_scores(n, hq, hkv, causal):
+    """Scores that lie hundreds apart, so that most probabilities are below the smallest normal number, and a NaN key: it reaches
+    every query that sees it and no other."""
+    torch.manual_seed(n)
+    d = 128
+    q = (torch.randn(n, hq, d, device="cuda") * 6).to(torch.bfloat16).requires_grad_(True)
+    k = (torch.randn(n, hkv, d, device="cuda") * 6).to(torch.bfloat16).requires_grad_(True)
+    v = torch.randn(n, hkv, d, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    cu = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    go = torch.randn(n, hq, d, device="cuda").to(torch.bfloat16)
+
+    def run(q, k, v):
+        return F.varlen_attention(q, k, v, cu, n) if causal else F.full_attention(q, k, v, cu, cu, n, n)
+    out = run(q, k, v)
+    out.backward(go)
+    rq, rk, rv = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    s = torch.einsum("qhd,khd->hqk", rq, rk.repeat_interleave(hq // hkv, 1)) / math.sqrt(d)
+    if causal:
+        s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    assert (s.detach()[:, -1].amax(-1) - s.detach()[:, -1].median(-1).values).min() > 64
+    ref = torch.einsum("hqk,khd->qhd", s.softmax(-1), rv.repeat_interleave(hq // hkv, 1))
+    ref.backward(go.double())
+    # P, dS and the results are rounded to bf16 (2^-9 each); scores of 36 sqrt(d) carry 2^-24 of that into the exponent
+    for got, want in ((out, ref), (q.grad, rq.grad), (k.grad, rk.grad), (v.grad, rv.grad)):
+        assert (got.double() - want).norm() <= 2.0 ** -6 * want.norm()
+    bad = k.detach().clone()
+    bad[n // 2, 0, 5] = float("nan")
+    with torch.no_grad():
+        hit = run(q.detach(), bad, v.detach()).isnan().any(-1)      # [n, hq]
+    want = torch.zeros_like(hit)
+    want[n // 2 if causal else 0:, : hq // hkv] = True
+    assert torch.equal(hit, want)
+    assert native.read_status(q.device) == 0
+
+
+@pytest.mark.gpu
 # one row; K of one block, of less than one, of 4 n + 1 blocks; columns that end inside 16 bytes; CTA pairs (enough tiles for
 # two rounds of single CTAs) with ragged rows and columns, and with more tiles than pairs
 @pytest.mark.parametrize("M,N,K", [(1, 264, 128), (3, 5, 144), (1, 4096, 640), (127, 1001, 112), (129, 19000, 128),
