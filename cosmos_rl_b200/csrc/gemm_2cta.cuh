@@ -13,6 +13,14 @@
 // 32-row x 128-byte slabs into swizzled staging buffers and hand them to TMA stores (or TMA reduce-adds when
 // the result is accumulated into C). TMA clips rows and columns outside C, so no edge code exists.
 //
+// Last round. Tiles rarely fill their last round of CTA pairs, and calls of few rows have fewer tiles than pairs. If at most
+// half of the pairs would have a tile in that round, its tiles come first, each cut along the contraction into as many equal
+// shares as there are pairs for. Shares go to a workspace as fp32 and are added by a small kernel behind this one, in the order
+// of the contraction. The pairs of one share index walk the same blocks of A and B at the same time; shares of any size, which
+// would fill every pair, do not, and read the operands from HBM again and again (1003 x 4096 x 28672: 167 us uncut, 247). A
+// sum by the warp that arrives last, instead of a kernel, reads the shares one after the other (100 x 4096 x 14336: 91 us
+// uncut, 42 with it, 34).
+//
 // Barriers (per CTA unless stated): full[s] (leader's is the one in use; loads of both CTAs complete on it),
 // empty[s] (the leader's tcgen05.commit arrives on both CTAs'), tfull[a] (same), tempty[a] (leader's; the 8
 // epilogue warps of the pair arrive on it). Every wait is bounded; on a timeout the kernel records a status
@@ -80,7 +88,45 @@ struct Gemm2Params {
   int accumulate;    // C += result (TMA reduce-add)
   int up_row0;       // G2_EPI_SWIGLU: first row of the "up" half inside B (= intermediate size)
   int group_m;       // raster: tiles of this many 256-row blocks share their B columns in time
+  int a_bytes;       // bytes of A that the leader fetches a stage: all its 128 rows, or those there are
+  int rest, splits;  // tiles 0 .. rest - 1 are cut into `splits` shares along the contraction (see "Last round"), 0: none
+  float* ws;         // shares, [pairs][256][BN]
   DlogitsParams dl;  // G2_EPI_DLOGITS
+};
+
+// What a pair works on, one unit after the other: its share of a cut tile, then whole tiles.
+struct G2Unit {
+  int tile, kb0, kb1;
+  bool cut;
+};
+struct G2Work {
+  int pair, pairs, rest, splits, total, num_kb;
+  __device__ __forceinline__ void init(int rest_, int splits_, int total_, int num_kb_) {
+    pair = blockIdx.x >> 1;
+    pairs = gridDim.x >> 1;
+    rest = rest_;
+    splits = splits_;
+    total = total_;
+    num_kb = num_kb_;
+  }
+  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
+    u.cut = false;
+    u.kb0 = 0;
+    u.kb1 = num_kb;
+    if (pair < rest * splits) {
+      if (it == 0) {
+        const int s = pair / rest;   // share s of tile t belongs to pair s * rest + t
+        u.tile = pair - s * rest;
+        u.cut = true;
+        u.kb0 = s * num_kb / splits;
+        u.kb1 = (s + 1) * num_kb / splits;
+        return true;
+      }
+      --it;
+    }
+    u.tile = rest + pair + it * pairs;
+    return u.tile < total;
+  }
 };
 
 // tile index -> (m_blk, n_blk): groups of `G` row blocks sweep all column blocks before the next group starts, so
@@ -97,7 +143,8 @@ __device__ __forceinline__ void g2_tile_coords(int i, int num_m, int num_n, int 
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
 __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmC,
-                                               int M, int N, int K, const Gemm2Params& ep, uint32_t* status) {
+                                               const CUtensorMap* tmW, int M, int N, int K, const Gemm2Params& ep,
+                                               uint32_t* status) {
   using SM = Gemm2Smem<BN, STAGES>;
   static_assert(BN == 128 || BN == 256, "BN");
   extern __shared__ uint8_t smem_raw[];
@@ -147,25 +194,28 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   const int num_n = (n_cols + OUT_BN - 1) / OUT_BN;
   const int total = num_m * num_n;
   const int num_kb = (K + G2_BK - 1) / G2_BK;
-  const int cluster_id = blockIdx.x >> 1;
-  const int num_clusters = gridDim.x >> 1;
   const int G = ep.group_m > 0 ? ep.group_m : 8;
+  G2Work work;
+  work.init(EPI == G2_EPI_STORE ? ep.rest : 0, ep.splits, total, num_kb);
+  G2Unit unit;
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
     if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int i = cluster_id; i < total && ok && !*abort_flag; i += num_clusters) {
+      for (int it = 0; work.get(it, unit) && ok && !*abort_flag; ++it) {
         int m_blk, n_blk;
-        g2_tile_coords(i, num_m, num_n, G, m_blk, n_blk);
+        g2_tile_coords(unit.tile, num_m, num_n, G, m_blk, n_blk);
+        // rows of A that lie outside the tensor are not fetched: it takes longer than fetching rows that exist
+        const bool peer_rows = m_blk * G2_BM + G2_BM_CTA < M;
         const int a_row0 = m_blk * G2_BM + (int)cta_rank * G2_BM_CTA;
         // rows of B that this CTA feeds: its half of the tile's columns; with the SwiGLU epilogue the leader
         // feeds the gate rows and the other CTA the matching up rows, so a thread sees both in its TMEM lane
         int b_row0;
         if constexpr (EPI == G2_EPI_SWIGLU) b_row0 = n_blk * (BN / 2) + (cta_rank ? ep.up_row0 : 0);
         else b_row0 = n_blk * BN + (int)cta_rank * (BN / 2);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = unit.kb0; kb < unit.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
             atomicCAS(status, ST_OK, ST_TIMEOUT_EMPTY);
             *abort_flag = 1;
@@ -175,9 +225,10 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
           uint8_t* sa = smem + stage * SM::STAGE_BYTES;
           uint8_t* sb = sa + SM::A_BYTES;
           const int k = kb * G2_BK;
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * SM::STAGE_BYTES);
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * SM::B_BYTES + ep.a_bytes + (peer_rows ? SM::A_BYTES : 0));
           const uint32_t bar = mapa_shared(smem_u32(&full_bar[stage]), 0);
-          if constexpr (!A_MN) {
+          if (!leader && !peer_rows) {
+          } else if constexpr (!A_MN) {
             tma_load_2d_pair(sa, tmA, bar, k, a_row0);
           } else {
 #pragma unroll
@@ -213,7 +264,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       uint32_t stage = 0, phase = 0;
       uint32_t acc = 0, acc_phase = 0;
       bool ok = true;
-      for (int i = cluster_id; i < total && ok && !*abort_flag; i += num_clusters) {
+      for (int it = 0; work.get(it, unit) && ok && !*abort_flag; ++it) {
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1)) {
           atomicCAS(status, ST_OK, ST_TIMEOUT_TMEM_EMPTY);
           *abort_flag = 1;
@@ -221,7 +272,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         }
         tc_fence_after_sync();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = unit.kb0; kb < unit.kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase)) {
             atomicCAS(status, ST_OK, ST_TIMEOUT_FULL);
             *abort_flag = 1;
@@ -235,7 +286,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
           for (int k = 0; k < G2_BK / 16; ++k) {
             uint64_t ad = A_MN ? umma_desc_mnmajor_sw128(sa + k * 2048, 8192) : umma_desc_kmajor_sw128(sa + k * 32);
             uint64_t bd = B_MN ? umma_desc_mnmajor_sw128(sb + k * 2048, 8192) : umma_desc_kmajor_sw128(sb + k * 32);
-            umma_bf16_ss_pair(tmem_d, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_bf16_ss_pair(tmem_d, ad, bd, idesc, (kb > unit.kb0 || k > 0) ? 1u : 0u);
           }
           tc_commit_pair(&empty_bar[stage], 3);  // frees this stage in both CTAs once the MMAs retire
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -254,9 +305,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
     uint32_t acc = 0, acc_phase = 0;
     uint32_t slab_idx = 0;
     const uint32_t sw = (uint32_t)(lane & 7);  // 128-byte swizzle: 16-byte chunk j of row r sits at chunk j ^ (r & 7)
-    for (int i = cluster_id; i < total && !*abort_flag; i += num_clusters) {
+    for (int it = 0; work.get(it, unit) && !*abort_flag; ++it) {
       int m_blk, n_blk;
-      g2_tile_coords(i, num_m, num_n, G, m_blk, n_blk);
+      g2_tile_coords(unit.tile, num_m, num_n, G, m_blk, n_blk);
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
         atomicCAS(status, ST_OK, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
@@ -266,10 +317,12 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
       const int row0 = m_blk * G2_BM + (int)cta_rank * G2_BM_CTA + quad * 32;  // first row of this warp's slabs
       const int col_base = n_blk * OUT_BN;
+      const bool cut = EPI == G2_EPI_STORE && unit.cut;             // fp32 into the pair's part of the workspace
+      const bool out_fp32 = cut || ep.out_fp32;
       DlogitsRow dlr;
       if constexpr (EPI == G2_EPI_DLOGITS) dlr.load(ep.dl, min(row0 + lane, M - 1));
       // a slab = 32 rows x 128 bytes of C: 64 bf16 or 32 fp32 columns
-      const int slab_cols = ep.out_fp32 ? 32 : 64;
+      const int slab_cols = out_fp32 ? 32 : 64;
 #pragma unroll 1
       for (int c = 0; c < OUT_BN; c += slab_cols) {
         uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
@@ -279,7 +332,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         uint8_t* my_row = slab + lane * 128;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          if (ep.out_fp32 && h == 1) break;
+          if (out_fp32 && h == 1) break;
           const int cc = c + h * 32;  // 32 accumulator columns [cc, cc + 32)
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + cc, r);
@@ -302,7 +355,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            if (ep.bias != nullptr) {
+            if (ep.bias != nullptr && !cut) {
               const int gc = col_base + cc;
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
@@ -312,7 +365,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
               }
             }
           }
-          if (ep.out_fp32) {
+          if (out_fp32) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {  // 8 chunks of 4 floats
               float4 o = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -335,7 +388,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         if (elect_one()) {
           const int gc = col_base + c;
           if (gc < n_cols && row0 < M) {
-            if (ep.accumulate) tma_reduce_add_2d(tmC, slab, gc, row0);
+            if (cut) tma_store_2d(tmW, slab, c, work.pair * G2_BM + (row0 - m_blk * G2_BM));
+            else if (ep.accumulate) tma_reduce_add_2d(tmC, slab, gc, row0);
             else tma_store_2d(tmC, slab, gc, row0);
           }
           tma_store_commit();

@@ -8,8 +8,77 @@ namespace b200 {
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, Gemm2Params ep, uint32_t* status) {
-  gemm2_mainloop<BN, STAGES, A_MN, B_MN, EPI>(&tmA, &tmB, &tmC, M, N, K, ep, status);
+                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, int M, int N, int K,
+                  Gemm2Params ep, uint32_t* status) {
+  gemm2_mainloop<BN, STAGES, A_MN, B_MN, EPI>(&tmA, &tmB, &tmC, &tmW, M, N, K, ep, status);
+}
+
+// C of the cut tiles: the sum of their shares (+ bias) (+ C). A warp has one row of a tile, a lane eight columns; rows of C
+// start on 16-byte boundaries. Grid (rest, 256 / 8).
+template <int BN>
+__global__ void __launch_bounds__(256)
+gemm2_sum_shares_kernel(const float* __restrict__ ws, void* __restrict__ C, long long ldc, int M, int N, Gemm2Params ep) {
+  pdl_wait();
+  const int num_m = (M + G2_BM - 1) / G2_BM, num_n = (N + BN - 1) / BN;
+  int m_blk, n_blk;
+  g2_tile_coords(blockIdx.x, num_m, num_n, ep.group_m > 0 ? ep.group_m : 8, m_blk, n_blk);
+  const int r = blockIdx.y * 8 + (threadIdx.x >> 5);
+  const long long row = (long long)m_blk * G2_BM + r;
+  if (row >= M) return;
+#pragma unroll
+  for (int c = (threadIdx.x & 31) * 8; c < BN; c += 256) {
+    const int col = n_blk * BN + c;
+    if (col >= N) continue;
+    const float* p = ws + ((long long)blockIdx.x * G2_BM + r) * BN + c;
+    const long long step = (long long)ep.rest * G2_BM * BN;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float4 x[8][2];
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (s < ep.splits) {
+        x[s][0] = *reinterpret_cast<const float4*>(p + s * step);
+        x[s][1] = *reinterpret_cast<const float4*>(p + s * step + 4);
+      }
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (s < ep.splits) {
+        v[0] += x[s][0].x; v[1] += x[s][0].y; v[2] += x[s][0].z; v[3] += x[s][0].w;
+        v[4] += x[s][1].x; v[5] += x[s][1].y; v[6] += x[s][1].z; v[7] += x[s][1].w;
+      }
+    if (ep.bias != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col + j < N)
+          v[j] += ep.bias_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(ep.bias)[col + j])
+                               : reinterpret_cast<const float*>(ep.bias)[col + j];
+    }
+    if (ep.out_fp32) {
+      float* dst = reinterpret_cast<float*>(C) + row * ldc + col;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col + j < N) dst[j] = ep.accumulate ? dst[j] + v[j] : v[j];
+    } else {
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + row * ldc + col;
+      if (col + 8 <= N) {
+        if (ep.accumulate) {
+          const uint4 old = *reinterpret_cast<const uint4*>(dst);
+          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&old);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __bfloat1622float2(h[j]);
+            v[2 * j] += f.x;
+            v[2 * j + 1] += f.y;
+          }
+        }
+        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                                    pack_bf16x2(v[6], v[7]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (col + j < N) dst[j] = __float2bfloat16(ep.accumulate ? __bfloat162float(dst[j]) + v[j] : v[j]);
+      }
+    }
+  }
 }
 
 // How many CTA pairs can be resident at once (asked once per kernel and device; <= num_sms / 2).
@@ -34,16 +103,30 @@ static int max_pairs(Kern kern, int smem_bytes, int num_sms, int threads = G2_TH
   return n < num_sms / 2 ? n : num_sms / 2;
 }
 
+// Contraction blocks that a cut has to save a pair: the shares' way through memory and the kernel that adds them. Weight
+// gradients, us, uncut and cut: 1500 tokens (24 blocks), 6144 x 4096 57 and 61; 2048 tokens (32 blocks) 74 and 77. Of 64 blocks
+// and more every cut pays: 300 x 4096 x 28672 141 and 89, 1500 x 4096 x 14336 149 and 125, 1500 x 4096 x 4096 49 and 44.
+constexpr int G2_CUT_BLOCKS = 30;
+// Scratch of a launch whose last round is cut (Gemm2Params::ws) for `num_sms` SMs.
+constexpr long long g2_ws_floats(int num_sms) { return (long long)(num_sms / 2) * G2_BM * 256; }
+
+// Tiles of the last round that are cut along the contraction, into how many shares; 0: none.
+inline int g2_rest(long long tiles, int pairs, int num_kb, int& splits) {
+  const int rest = (int)(tiles % pairs);
+  splits = rest > 0 ? pairs / rest : 0;
+  if (splits > 8) splits = 8;
+  if (splits > num_kb / 8) splits = num_kb / 8;
+  if (splits < 2 || num_kb - num_kb / splits < G2_CUT_BLOCKS) return splits = 0;
+  return rest;
+}
+
+// allow_cut: a launch that would gain from a workspace and has none (ep.ws null) returns B200_NEED_WORKSPACE
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
 static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                        long long ldc, const Gemm2Params& ep, uint32_t* status, int num_sms, cudaStream_t stream) {
-  CUtensorMap tmA, tmB, tmC;
-  if (A_MN ? make_tmap_2d(&tmA, A, K, M, lda, 64, 64, 2) : make_tmap_2d(&tmA, A, M, K, lda, G2_BM_CTA, G2_BK, 2))
-    return B200_ERR_TENSORMAP;
-  if (B_MN ? make_tmap_2d(&tmB, B, K, N, ldb, 64, 64, 2) : make_tmap_2d(&tmB, B, N, K, ldb, BN / 2, G2_BK, 2))
-    return B200_ERR_TENSORMAP;
+                        long long ldc, Gemm2Params ep, uint32_t* status, int num_sms, cudaStream_t stream,
+                        bool allow_cut = false) {
+  CUtensorMap tmA, tmB, tmC, tmW;
   const int n_cols = EPI == G2_EPI_SWIGLU ? N / 2 : N;
-  if (make_tmap_out(&tmC, C, M, n_cols, ldc, ep.out_fp32)) return B200_ERR_TENSORMAP;
   using SM = Gemm2Smem<BN, STAGES>;
   auto kern = gemm2_bf16_kernel<BN, STAGES, A_MN, B_MN, EPI>;
   static int pairs[16] = {0};  // per device
@@ -59,9 +142,25 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   int np = pairs[dev];
   if (num_sms / 2 < np) np = num_sms / 2;  // the caller may reserve SMs for kernels on other streams
   if (np < 1) np = 1;
-  const int grid = 2 * (tiles < np ? tiles : np);
-  kern<<<grid, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, M, N, K, ep, status);
-  return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  ep.rest = EPI == G2_EPI_STORE && allow_cut ? g2_rest(tiles, np, (K + G2_BK - 1) / G2_BK, ep.splits) : (ep.splits = 0);
+  if (ep.rest > 0 && ep.ws == nullptr) return B200_NEED_WORKSPACE;
+  const int a_rows = !A_MN && M < G2_BM_CTA ? M : G2_BM_CTA;
+  ep.a_bytes = a_rows * G2_BK * 2;
+  if (A_MN ? make_tmap_2d(&tmA, A, K, M, lda, 64, 64, 2) : make_tmap_2d(&tmA, A, M, K, lda, a_rows, G2_BK, 2))
+    return B200_ERR_TENSORMAP;
+  if (B_MN ? make_tmap_2d(&tmB, B, K, N, ldb, 64, 64, 2) : make_tmap_2d(&tmB, B, N, K, ldb, BN / 2, G2_BK, 2))
+    return B200_ERR_TENSORMAP;
+  if (make_tmap_out(&tmC, C, M, n_cols, ldc, ep.out_fp32)) return B200_ERR_TENSORMAP;
+  tmW = tmC;
+  if (ep.rest > 0 && make_tmap_out(&tmW, ep.ws, (uint64_t)np * G2_BM, BN, BN, 1)) return B200_ERR_TENSORMAP;
+  const int grid = 2 * (ep.rest > 0 || tiles >= np ? np : tiles);
+  kern<<<grid, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, tmW, M, N, K, ep, status);
+  if (cudaGetLastError() != cudaSuccess) return B200_ERR_LAUNCH;
+  if constexpr (EPI == G2_EPI_STORE)
+    if (ep.rest > 0 && launch_pdl(gemm2_sum_shares_kernel<BN>, dim3(ep.rest, G2_BM / 8), dim3(256), 0, stream,
+                                  (const float*)ep.ws, C, ldc, M, N, ep) != cudaSuccess)
+      return B200_ERR_LAUNCH;
+  return 0;
 }
 
 }  // namespace b200

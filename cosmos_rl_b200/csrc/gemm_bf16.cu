@@ -119,7 +119,7 @@ static int dispatch_bn(const void* A, const void* B, void* C, int M, int N, int 
 
 template <bool A_MN, bool B_MN>
 static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                          long long ldc, const Gemm2Params& ep, int epi, uint32_t* status, int num_sms,
+                          long long ldc, const Gemm2Params& ep, int epi, bool cut, uint32_t* status, int num_sms,
                           cudaStream_t stream) {
   if (epi == G2_EPI_SWIGLU) {
     if constexpr (!A_MN && !B_MN)
@@ -128,13 +128,21 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
       return B200_ERR_ARG;
   }
   if (N > 128)
-    return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream);
-  return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream);
+    return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
+  return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
 }
 
 static bool pair_kernel_usable(const void* C, int M, long long ldc, int out_fp32) {
   const int eb = out_fp32 ? 4 : 2;
   return M > 128 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ((ldc * eb) & 15) == 0;
+}
+
+// Up to 128 rows the pair kernel is the faster one when all its tiles run at once, with or without a cut (100 rows, us, single
+// CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56). It is usable where the
+// rows of C are whole 16 bytes, which is what its stores write.
+static bool pair_kernel_for_few_rows(const void* C, int M, int N, long long ldc, int out_fp32, int num_sms) {
+  return M <= 128 && (N + 255) / 256 <= num_sms / 2 && pair_kernel_usable(C, 129, ldc, out_fp32) &&
+         ((N * (out_fp32 ? 4 : 2)) & 15) == 0;
 }
 
 }  // namespace b200
@@ -147,32 +155,46 @@ static bool pair_kernel_usable(const void* C, int M, long long ldc, int out_fp32
 // (reason << 24) | CUresult of the last tensor-map encode that failed in this process (0: none); see gemm_core.cuh
 extern "C" int b200_last_tmap_error() { return b200::last_tmap_error(); }
 
-extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+// cut: a call whose tiles leave half of their last round of CTA pairs idle cuts it along the contraction. ws: scratch for that
+// (b200_gemm_ws_floats); null: such a call returns B200_NEED_WORKSPACE and has launched nothing.
+extern "C" int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                                  long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate,
-                                 const void* bias, int bias_bf16, int epilogue, int up_row0, int path,
+                                 const void* bias, int bias_bf16, int epilogue, int up_row0, int path, int cut, float* ws,
                                  uint32_t* status, int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return B200_ERR_ARG;
   // TMA needs 16-byte aligned row strides; MN-major tiles are fetched in 64-element columns
   if ((lda & 7) || (ldb & 7)) return B200_ERR_ARG;
   using namespace b200;
-  const bool want_pair = path != 1 && pair_kernel_usable(C, M, ldc, out_fp32);
+  const bool want_pair = path != 1 && (pair_kernel_usable(C, M, ldc, out_fp32) ||
+                                       (cut && pair_kernel_for_few_rows(C, M, N, ldc, out_fp32, num_sms)));
   if (epilogue == G2_EPI_SWIGLU || bias != nullptr || path == 2) {
     // epilogues that only the CTA-pair kernel has
     if (!pair_kernel_usable(C, 129, ldc, out_fp32)) return B200_ERR_ARG;
     if (epilogue == G2_EPI_SWIGLU && (a_mn || b_mn || (N & 1) || accumulate)) return B200_ERR_ARG;
   }
   if (want_pair || epilogue == G2_EPI_SWIGLU || bias != nullptr || path == 2) {
-    Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, {}};
-    if (!a_mn && !b_mn) return dispatch_gemm2<false, false>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, status, num_sms, stream);
-    if (!a_mn && b_mn) return dispatch_gemm2<false, true>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, status, num_sms, stream);
-    if (a_mn && b_mn) return dispatch_gemm2<true, true>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, status, num_sms, stream);
-    return dispatch_gemm2<true, false>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, status, num_sms, stream);
+    Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, {}};
+    if (!a_mn && !b_mn) return dispatch_gemm2<false, false>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
+    if (!a_mn && b_mn) return dispatch_gemm2<false, true>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
+    if (a_mn && b_mn) return dispatch_gemm2<true, true>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
+    return dispatch_gemm2<true, false>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
   }
   if (!a_mn && !b_mn) return dispatch_bn<false, false>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
   if (!a_mn && b_mn) return dispatch_bn<false, true>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
   if (a_mn && b_mn) return dispatch_bn<true, true>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
   return dispatch_bn<true, false>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
 }
+
+extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                                 long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate,
+                                 const void* bias, int bias_bf16, int epilogue, int up_row0, int path,
+                                 uint32_t* status, int num_sms, cudaStream_t stream) {
+  return b200_gemm_bf16_ws(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, bias, bias_bf16, epilogue, up_row0,
+                           path, 0, nullptr, status, num_sms, stream);
+}
+
+// Scratch of b200_gemm_bf16_ws, in elements.
+extern "C" long long b200_gemm_ws_floats(int num_sms) { return b200::g2_ws_floats(num_sms); }
 
 extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                               long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate,

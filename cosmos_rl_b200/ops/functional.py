@@ -262,14 +262,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = Fals
         out = torch.empty(M, N // 2 if swiglu else N, dtype=out_dtype, device=a.device)
     if bias is not None:
         assert bias.is_contiguous() and bias.numel() == N and bias.dtype in (torch.bfloat16, torch.float32)
-    st = native.status_word(a.device)
     dev = a.device.index if a.device.index is not None else torch.cuda.current_device()
-    native.check(native.lib().b200_gemm_bf16_ex(native.ptr(a), native.ptr(b), native.ptr(out), M, N, K, a.stride(0),
-                                                b.stride(0), out.stride(0), int(a_mn), int(b_mn),
-                                                1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0,
-                                                native.ptr(bias), 1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
-                                                1 if swiglu else 0, N // 2 if swiglu else 0, path,
-                                                native.ptr(st), native.num_sms(dev), native.stream()), "gemm_bf16")
+    sms, strm, L = native.num_sms(dev), native.stream(), native.lib()
+
+    def call(ws):
+        return L.b200_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                                   int(a_mn), int(b_mn), 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0,
+                                   native.ptr(bias), 1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
+                                   1 if swiglu else 0, N // 2 if swiglu else 0, path, 1, native.ptr(ws),
+                                   native.status_word(a.device).data_ptr(), sms, strm)
+
+    rc = call(None)
+    if rc == native.NEED_WORKSPACE:     # the last round of tiles is cut along the contraction
+        rc = call(torch.empty(L.b200_gemm_ws_floats(sms), dtype=torch.float32, device=a.device))
+    native.check(rc, "gemm_bf16")
     return out
 
 

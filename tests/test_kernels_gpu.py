@@ -543,6 +543,37 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
+# (rows, columns, contraction): one tile and few rows; ragged everything; 128-wide tiles; one tile past a full round; two shares
+# of uneven length; a contraction too short to be cut
+@pytest.mark.parametrize("M,N,K", [(3, 256, 4096), (127, 1032, 4200), (129, 520, 8200), (300, 104, 4096), (1300, 3840, 4104),
+                                   (900, 2304, 4160), (256, 512, 512)])
+@pytest.mark.parametrize("out_dtype,accumulate,bias,mn", [(torch.bfloat16, False, True, False), (torch.float32, True, False, False),
+                                                          (torch.bfloat16, True, False, True)])
+def test_gemm_cut_last_round(M, N, K, out_dtype, accumulate, bias, mn):
+    torch.manual_seed(M + N)
+    a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    bv = torch.randn(N, device="cuda").to(torch.bfloat16) if bias else None
+    if mn and M % 8:
+        pytest.skip("rows of a transposed operand are 16 bytes")
+    buf = torch.randn(M + 1, N, device="cuda").to(out_dtype)
+    out, before = buf[:M], buf.clone()
+    ops = (a.t().contiguous(), b.t().contiguous()) if mn else (a, b)
+    F.gemm(*ops, a_mn=mn, b_mn=mn, out=out, accumulate=accumulate, bias=bv)
+    torch.cuda.synchronize()
+    assert native.read_status(a.device) == 0
+    ref = a.double() @ b.double().t() + (bv.double() if bias else 0) + (before[:M].double() if accumulate else 0)
+    # fp32 sums of K products, and for bf16 one rounding of the product and one of the sum with what was there
+    bound = 2.0 ** -20 * K ** 0.5 * a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=1) / K ** 0.5 + 1e-5
+    if out_dtype == torch.bfloat16:
+        bound = bound + 2.0 ** -8 * ref.abs() + (2.0 ** -8 * (ref - before[:M].double()).abs() if accumulate else 0)
+    assert ((out.double() - ref).abs() <= bound).all()
+    assert torch.equal(buf[M], before[M])
+    again = before.clone()
+    F.gemm(*ops, a_mn=mn, b_mn=mn, out=again[:M], accumulate=accumulate, bias=bv)
+    assert torch.equal(again, buf)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("n,hq,hkv", [(129, 4, 2), (700, 16, 4), (1200, 16, 16)])
 def test_attention_far_apart_scores(n, hq, hkv, causal):
