@@ -35,7 +35,7 @@ constexpr int G2_BM = 256;      // rows of the pair's tile
 constexpr int G2_BK = 64;
 constexpr int G2_THREADS = 192;
 
-enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2 };
+enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3 };
 
 template <int BN, int STAGES>
 struct Gemm2Smem {
@@ -92,41 +92,10 @@ struct Gemm2Params {
   int rest, splits;  // tiles 0 .. rest - 1 are cut into `splits` shares along the contraction (see "Last round"), 0: none
   float* ws;         // shares, [pairs][256][BN]
   DlogitsParams dl;  // G2_EPI_DLOGITS
-};
-
-// What a pair works on, one unit after the other: its share of a cut tile, then whole tiles.
-struct G2Unit {
-  int tile, kb0, kb1;
-  bool cut;
-};
-struct G2Work {
-  int pair, pairs, rest, splits, total, num_kb;
-  __device__ __forceinline__ void init(int rest_, int splits_, int total_, int num_kb_) {
-    pair = blockIdx.x >> 1;
-    pairs = gridDim.x >> 1;
-    rest = rest_;
-    splits = splits_;
-    total = total_;
-    num_kb = num_kb_;
-  }
-  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
-    u.cut = false;
-    u.kb0 = 0;
-    u.kb1 = num_kb;
-    if (pair < rest * splits) {
-      if (it == 0) {
-        const int s = pair / rest;   // share s of tile t belongs to pair s * rest + t
-        u.tile = pair - s * rest;
-        u.cut = true;
-        u.kb0 = s * num_kb / splits;
-        u.kb1 = (s + 1) * num_kb / splits;
-        return true;
-      }
-      --it;
-    }
-    u.tile = rest + pair + it * pairs;
-    return u.tile < total;
-  }
+  // G2_EPI_EXPERTS: C is [experts, M, N], and expert e contracts over rows [offsets[e], offsets[e + 1]) of A and B (multiples
+  // of 64; both MN-major)
+  const int* offsets;
+  int experts;
 };
 
 // tile index -> (m_blk, n_blk): groups of `G` row blocks sweep all column blocks before the next group starts, so
@@ -140,6 +109,71 @@ __device__ __forceinline__ void g2_tile_coords(int i, int num_m, int num_n, int 
   m_blk = first_m + r % gsz;
   n_blk = r / gsz;
 }
+
+// What a pair works on, one unit after the other: its share of a cut tile, then whole tiles.
+struct G2Unit {
+  int m_blk, n_blk, batch, kb0, kb1;
+  bool cut;
+};
+struct G2Work {
+  int pair, pairs, rest, splits, num_m, num_n, G, total, num_kb;
+  __device__ __forceinline__ void init(const Gemm2Params& ep, bool may_cut, int num_m_, int num_n_, int num_kb_) {
+    pair = blockIdx.x >> 1;
+    pairs = gridDim.x >> 1;
+    rest = may_cut ? ep.rest : 0;
+    splits = ep.splits;
+    num_m = num_m_;
+    num_n = num_n_;
+    G = ep.group_m > 0 ? ep.group_m : 8;
+    total = num_m * num_n;
+    num_kb = num_kb_;
+  }
+  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
+    u.cut = false;
+    u.batch = 0;
+    u.kb0 = 0;
+    u.kb1 = num_kb;
+    if (pair < rest * splits) {
+      if (it == 0) {
+        const int s = pair / rest;   // share s of tile t belongs to pair s * rest + t
+        g2_tile_coords(pair - s * rest, num_m, num_n, G, u.m_blk, u.n_blk);
+        u.cut = true;
+        u.kb0 = s * num_kb / splits;
+        u.kb1 = (s + 1) * num_kb / splits;
+        return true;
+      }
+      --it;
+    }
+    const int tile = rest + pair + it * pairs;
+    if (tile >= total) return false;
+    g2_tile_coords(tile, num_m, num_n, G, u.m_blk, u.n_blk);
+    return true;
+  }
+};
+
+// G2_EPI_EXPERTS: all tiles of an expert's weight gradient, expert by expert
+struct G2ExpertWork {
+  int num_n, per_expert, total;
+  const int* offsets;
+  __device__ __forceinline__ void init(const Gemm2Params& ep, bool, int num_m, int num_n_, int) {
+    num_n = num_n_;
+    per_expert = num_m * num_n_;
+    total = per_expert * ep.experts;
+    offsets = ep.offsets;
+  }
+  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
+    const int i = (blockIdx.x >> 1) + it * (gridDim.x >> 1);
+    if (i >= total) return false;
+    u.batch = i / per_expert;
+    const int r = i - u.batch * per_expert;
+    u.m_blk = r / num_n;
+    u.n_blk = r - u.m_blk * num_n;
+    u.kb0 = offsets[u.batch] / G2_BK;
+    u.kb1 = offsets[u.batch + 1] / G2_BK;
+    u.cut = false;
+    return true;
+  }
+};
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
 __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmC,
@@ -192,11 +226,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   constexpr int OUT_BN = (EPI == G2_EPI_SWIGLU) ? BN / 2 : BN;  // columns of C per tile
   const int n_cols = (EPI == G2_EPI_SWIGLU) ? N / 2 : N;        // columns of C
   const int num_n = (n_cols + OUT_BN - 1) / OUT_BN;
-  const int total = num_m * num_n;
-  const int num_kb = (K + G2_BK - 1) / G2_BK;
-  const int G = ep.group_m > 0 ? ep.group_m : 8;
-  G2Work work;
-  work.init(EPI == G2_EPI_STORE ? ep.rest : 0, ep.splits, total, num_kb);
+  std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork, G2Work> work;
+  work.init(ep, EPI == G2_EPI_STORE, num_m, num_n, (K + G2_BK - 1) / G2_BK);
   G2Unit unit;
 
   if (warp == 0) {
@@ -205,8 +236,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int it = 0; work.get(it, unit) && ok && !*abort_flag; ++it) {
-        int m_blk, n_blk;
-        g2_tile_coords(unit.tile, num_m, num_n, G, m_blk, n_blk);
+        const int m_blk = unit.m_blk, n_blk = unit.n_blk;
         // rows of A that lie outside the tensor are not fetched: it takes longer than fetching rows that exist
         const bool peer_rows = m_blk * G2_BM + G2_BM_CTA < M;
         const int a_row0 = m_blk * G2_BM + (int)cta_rank * G2_BM_CTA;
@@ -306,8 +336,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
     uint32_t slab_idx = 0;
     const uint32_t sw = (uint32_t)(lane & 7);  // 128-byte swizzle: 16-byte chunk j of row r sits at chunk j ^ (r & 7)
     for (int it = 0; work.get(it, unit) && !*abort_flag; ++it) {
-      int m_blk, n_blk;
-      g2_tile_coords(unit.tile, num_m, num_n, G, m_blk, n_blk);
+      const int m_blk = unit.m_blk, n_blk = unit.n_blk;
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
         atomicCAS(status, ST_OK, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
@@ -330,12 +359,21 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         if (elect_one()) tma_store_wait_read<1>();
         __syncwarp();
         uint8_t* my_row = slab + lane * 128;
+        // The slab's accumulators, all on their way before the first is used: results of short contractions are bound by the
+        // epilogue (28672 x 4096 over 64 rows: 70 us, 54). Two warps a quadrant in place of a stage: 45 there, but 73 and 69
+        // over 300 rows.
+        uint32_t plain[2][32];
+        if constexpr (EPI == G2_EPI_STORE || EPI == G2_EPI_EXPERTS) {
+          tmem_ld_32x32b_x32(taddr + c, plain[0]);
+          if (!out_fp32) tmem_ld_32x32b_x32(taddr + c + 32, plain[1]);
+          tmem_ld_wait();
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (out_fp32 && h == 1) break;
           const int cc = c + h * 32;  // 32 accumulator columns [cc, cc + 32)
           uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + cc, r);
+          if constexpr (EPI == G2_EPI_SWIGLU || EPI == G2_EPI_DLOGITS) tmem_ld_32x32b_x32(taddr + cc, r);
           float v[32];
           if constexpr (EPI == G2_EPI_SWIGLU) {
             uint32_t u[32];
@@ -352,9 +390,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = dlr.of(__uint_as_float(r[j]), ep.dl.inv_temp, (long long)j == off);
           } else {
-            tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            for (int j = 0; j < 32; ++j) v[j] = EPI == G2_EPI_EXPERTS && unit.kb0 == unit.kb1 ? 0.f : __uint_as_float(plain[h][j]);
             if (ep.bias != nullptr && !cut) {
               const int gc = col_base + cc;
 #pragma unroll
@@ -388,7 +425,10 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         if (elect_one()) {
           const int gc = col_base + c;
           if (gc < n_cols && row0 < M) {
-            if (cut) tma_store_2d(tmW, slab, c, work.pair * G2_BM + (row0 - m_blk * G2_BM));
+            if constexpr (EPI == G2_EPI_EXPERTS) {
+              if (ep.accumulate) tma_reduce_add_3d(tmC, slab, gc, row0, unit.batch);
+              else tma_store_3d(tmC, slab, gc, row0, unit.batch);
+            } else if (cut) tma_store_2d(tmW, slab, c, (int)(blockIdx.x >> 1) * G2_BM + (row0 - m_blk * G2_BM));
             else if (ep.accumulate) tma_reduce_add_2d(tmC, slab, gc, row0);
             else tma_store_2d(tmC, slab, gc, row0);
           }

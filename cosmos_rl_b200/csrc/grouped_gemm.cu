@@ -13,6 +13,7 @@
 // Tile counts and expert boundaries are read from device memory (tile_expert / expert_offsets / n_tiles), so
 // no host synchronisation sits between routing and the expert GEMMs.
 #include "gemm_core.cuh"
+#include "gemm_2cta_launch.cuh"
 #include "api.h"
 
 namespace b200 {
@@ -254,6 +255,34 @@ int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, in
   if (make_tmap_grouped_out(&tmC, dW, num_experts, N, K, K, (uint64_t)N * K, out_fp32)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmA, dY, max_rows, N, lddy, 64, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, X, max_rows, K, ldx, 64, 64, 2)) return B200_ERR_TENSORMAP;
+  // CTA pairs on 256 x 256 tiles once every pair has one: the single CTAs are bound by operands out of L2 (4.9 blocks of 48 KB
+  // for 64 KB of result, 4096 tokens on 128 experts), and a pair fetches two thirds of that. us, single CTAs and pairs, 1536 x
+  // 2048 a gradient: 256 rows for each of 128 experts 290 and 260, 512 rows 465 and 400, 2048 rows for each of 16 165 and 143;
+  // few rows are bound by the epilogue, of which a pair has the less: 44 rows 190 and 216, 6 rows 166 and 191. max_rows is what
+  // there is room for, up to 128 rows an expert more than there are. A bf16 result that is added to keeps its one rounding in
+  // the other kernel.
+  const long long pair_tiles = (long long)num_experts * ((N + G2_BM - 1) / G2_BM) * ((K + 255) / 256);
+  if (!(accumulate && !out_fp32) && num_sms >= 2 && pair_tiles >= num_sms / 2 &&
+      pair_tiles < (1ll << 31) && max_rows >= 320ll * num_experts) {
+    auto kern = gemm2_bf16_kernel<256, 6, true, true, G2_EPI_EXPERTS>;
+    using SM = Gemm2Smem<256, 6>;
+    static int pairs[16] = {0};   // per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return B200_ERR_RUNTIME;
+    if (pairs[dev] == 0) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL) != cudaSuccess) return B200_ERR_LAUNCH;
+      pairs[dev] = max_pairs(kern, SM::TOTAL, num_sms);
+    }
+    Gemm2Params ep2{};
+    ep2.out_fp32 = out_fp32;
+    ep2.accumulate = accumulate;
+    ep2.a_bytes = SM::A_BYTES;
+    ep2.offsets = expert_offsets;
+    ep2.experts = num_experts;
+    const int np = pairs[dev] < num_sms / 2 ? pairs[dev] : num_sms / 2;
+    kern<<<2 * np, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, tmC, N, K, 0, ep2, status);
+    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  }
   static bool s2 = false;
   if (set_smem(grouped_wgrad_kernel, s2)) return B200_ERR_LAUNCH;
   GroupedParams ep{nullptr, accumulate && !out_fp32 ? (const __nv_bfloat16*)dW : nullptr, K, (long long)N * K, K, N, out_fp32,

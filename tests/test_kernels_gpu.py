@@ -543,6 +543,33 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
+# ragged result rows and columns; experts without rows; fp32 sums; too few rows for CTA pairs
+@pytest.mark.parametrize("E,N,K,rows", [(10, 1032, 520, [128, 0, 640, 384, 0, 256, 1024, 128, 512, 768]),
+                                        (6, 1536, 768, [512] * 6), (40, 256, 520, [128] * 40)])
+@pytest.mark.parametrize("out_dtype,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_grouped_wgrad_forms(E, N, K, rows, out_dtype, accumulate):
+    torch.manual_seed(E)
+    off = torch.tensor([0] + rows, device="cuda").cumsum(0).to(torch.int32)
+    Mp = int(off[-1])
+    dy, x = torch.randn(Mp, N, device="cuda").to(torch.bfloat16), torch.randn(Mp, K, device="cuda").to(torch.bfloat16)
+    out = torch.randn(E, N, K, device="cuda").to(out_dtype)
+    before = out.double()
+    native.check(native.lib().b200_grouped_wgrad(native.ptr(dy), native.ptr(x), native.ptr(out), Mp, N, K, E, N, K,
+                                                 native.ptr(off), int(out_dtype == torch.float32), int(accumulate),
+                                                 native.ptr(native.status_word(x.device)), native.num_sms(0),
+                                                 native.stream()), "grouped_wgrad")
+    torch.cuda.synchronize()
+    assert native.read_status(x.device) == 0
+    for e in range(E):
+        a, b = dy[off[e]:off[e + 1]].double(), x[off[e]:off[e + 1]].double()
+        ref = a.t() @ b + (before[e] if accumulate else 0)
+        bound = 2.0 ** -20 * a.norm(dim=0)[:, None] * b.norm(dim=0) + 1e-5      # fp32 sums
+        if out_dtype == torch.bfloat16:
+            bound = bound + 2.0 ** -8 * ref.abs()                              # and one rounding
+        assert ((out[e].double() - ref).abs() <= bound).all(), e
+
+
+@pytest.mark.gpu
 # (rows, columns, contraction): one tile and few rows; ragged everything; 128-wide tiles; one tile past a full round; two shares
 # of uneven length; a contraction too short to be cut
 @pytest.mark.parametrize("M,N,K", [(3, 256, 4096), (127, 1032, 4200), (129, 520, 8200), (300, 104, 4096), (1300, 3840, 4104),
