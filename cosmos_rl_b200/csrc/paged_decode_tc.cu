@@ -10,7 +10,11 @@
 // so both contractions take K-major operands straight from TMA (128-byte swizzle):
 //   S^T[token, head] = K[token, :] . Q[head, :]        M = 128 tokens, N = 16 (G <= 8 heads, padded), K = d
 //   O^T[d, head]    += V^T[d, token] . P[head, token]   M = 128 (d),    N = 16,                        K = tokens
-// One work item = (sequence, kv head, split). Persistent CTAs (one per SM) walk the items.
+// One work item = (sequence, kv head, split). Persistent CTAs (one per SM) walk the items. When there are more items than CTAs
+// they are listed by the length of their sequence, the longest first, and dealt out forwards and backwards in turn: an SM
+// that gets the longest of one round gets the shortest of the next. 128 sequences of 384 to 1536 tokens, 4 kv heads: the
+// busiest SM has 31.6 pages' work instead of 42.6 in the order of the sequences, the mean is 28.5: 61
+// and 65 us; 64 sequences of 1000 to 4000 tokens, 8 kv heads: 120 and 133.
 //   warp 0   : TMA producer (Q tile per item, K / V^T slabs per page through a 3-stage ring)
 //   warp 1   : MMA issuer (one thread), owns the TMEM allocation (S^T: 16 columns, O^T: 16 columns)
 //   warps 2-5: softmax. Thread <-> TMEM lane: a token row of S^T, a head-dim row of O^T. Column (head)
@@ -36,8 +40,9 @@ constexpr int PDT_SLAB_BYTES = PDT_PAGE * PDT_D * 2;        // 32 KiB
 constexpr int PDT_STAGE_BYTES = 2 * PDT_SLAB_BYTES;         // K + V^T
 constexpr int PDT_Q_BYTES = 2 * PDT_N * 64 * 2;             // two 16 x 64 boxes
 constexpr int PDT_P_BYTES = 2 * PDT_N * 64 * 2;             // two 16 x 64-token halves
-constexpr int PDT_SMEM = PDT_STAGES * PDT_STAGE_BYTES + 2 * PDT_Q_BYTES + 2 * PDT_P_BYTES + 1024 /*barriers, reductions*/ + 1024;
+constexpr int PDT_SMEM = PDT_STAGES * PDT_STAGE_BYTES + 2 * PDT_Q_BYTES + 2 * PDT_P_BYTES + 2048 /*barriers, reductions, order*/ + 1024;
 constexpr int PDT_THREADS = 192;
+constexpr int PDT_SORT_MAX = 256;  // sequences that are sorted: each CTA compares all of them with each other
 constexpr float PDT_LOG2E = 1.4426950408889634f;
 
 struct PdtParams {
@@ -109,6 +114,8 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_ready + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* red = reinterpret_cast<float*>(bars + 24);      // [2 buffers][4 warps][8 heads], 16-byte aligned
+  uint16_t* pages_sh = reinterpret_cast<uint16_t*>(red + 64);   // [PDT_SORT_MAX] pages of each sequence
+  uint8_t* order = reinterpret_cast<uint8_t*>(pages_sh + PDT_SORT_MAX);   // [PDT_SORT_MAX] sequences by length
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.hq / p.hkv;
@@ -147,12 +154,39 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   const uint32_t tmem_o = tmem_base + 32;   // S^T: columns [0,16) and [16,32) (even / odd tile); O^T: [32,48)
   pdl_wait();  // the set-up above is CTA-local; queries, cache pages and lengths are global memory
 
+  const bool sorted = n_items > (int)gridDim.x && p.B <= PDT_SORT_MAX;
+  if (sorted) {
+    for (int b = threadIdx.x; b < PDT_SORT_MAX; b += PDT_THREADS) {
+      int pages = 0;
+      if (b < p.B) pages = (p.seq_lens[b] + PDT_PAGE - 1) / PDT_PAGE - (p.prefix_pages ? p.prefix_pages[b] : 0);
+      pages_sh[b] = (uint16_t)min(max(pages, 0), 65535);
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < p.B; b += PDT_THREADS) {
+      const int mine = pages_sh[b];
+      int rank = 0;
+#pragma unroll 4
+      for (int o = 0; o < p.B; o += 4) {   // past the end there is nothing longer
+        const ushort4 x = *reinterpret_cast<const ushort4*>(pages_sh + o);
+        rank += (x.x > mine || (x.x == mine && o < b)) + (x.y > mine || (x.y == mine && o + 1 < b)) +
+                (x.z > mine || (x.z == mine && o + 2 < b)) + (x.w > mine || (x.w == mine && o + 3 < b));
+      }
+      order[rank] = (uint8_t)b;
+    }
+    __syncthreads();
+  }
+  // the k-th item of this CTA; rises with k
+  auto nth = [&](int k) -> int {
+    const int c = sorted && (k & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+    return k * (int)gridDim.x + c;
+  };
   // item -> (b, h, split) and its token range, identical in every role
   auto item_range = [&](int item, int& b, int& h, int& split, int& t0, int& t1) {
     split = item % p.nsplit;
     int bh = item / p.nsplit;
     h = bh % p.hkv;
     b = bh / p.hkv;
+    if (sorted) b = order[b];
     const int len = p.seq_lens[b];
     const int tb = p.prefix_pages ? min(p.prefix_pages[b] * PDT_PAGE, len) : 0;
     int chunk = (len - tb + p.nsplit - 1) / p.nsplit;
@@ -172,7 +206,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     if (elect_one()) {
       uint32_t kv_it = 0, item_it = 0;
       // work items with an empty token range are skipped by every role (item_it counts the others)
-      for (int item = blockIdx.x; item < n_items && !*abort_flag; item += gridDim.x) {
+      for (int k = 0, item = nth(0); item < n_items && !*abort_flag; item = nth(++k)) {
         int b, h, split, t0, t1;
         item_range(item, b, h, split, t0, t1);
         const int ntiles = (t1 - t0 + PDT_PAGE - 1) / PDT_PAGE;
@@ -236,7 +270,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
         }
       };
       bool ok = true, s_issued = false;
-      for (int item = blockIdx.x; item < n_items && ok && !*abort_flag; item += gridDim.x) {
+      for (int k = 0, item = nth(0); item < n_items && ok && !*abort_flag; item = nth(++k)) {
         const int ntiles = item_tiles(item);
         if (ntiles == 0) continue;
         const uint32_t qs = item_it & 1;
@@ -252,9 +286,9 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
           if (j + 1 < ntiles) {
             if (!mma1(kv_it + 1, item_it)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_FULL); *abort_flag = 1; ok = false; break; }
           } else {
-            int nxt = item + gridDim.x;
-            while (nxt < n_items && item_tiles(nxt) == 0) nxt += gridDim.x;
-            if (nxt < n_items) {
+            int after = k + 1;
+            while (nth(after) < n_items && item_tiles(nth(after)) == 0) ++after;
+            if (nth(after) < n_items) {
               if (!mbar_wait(&qfull[(item_it + 1) & 1], ((item_it + 1) >> 1) & 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_FULL); *abort_flag = 1; ok = false; break; }
               tc_fence_after_sync();
               if (!mma1(kv_it + 1, item_it + 1)) { atomicCAS(p.status, ST_OK, ST_TIMEOUT_FULL); *abort_flag = 1; ok = false; break; }
@@ -281,7 +315,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     uint32_t item_it = 0, tile_it = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+    for (int k = 0, item = nth(0); item < n_items && ok; item = nth(++k)) {
       int b, h, split, t0, t1;
       item_range(item, b, h, split, t0, t1);
       const int ntiles = (t1 - t0 + PDT_PAGE - 1) / PDT_PAGE;

@@ -381,6 +381,35 @@ def test_rope_separate_qk_autograd_on_views():
 
 
 @pytest.mark.gpu
+# more items than SMs, listed by length: the most sequences that are sorted and one more, equal and empty ones among them
+@pytest.mark.parametrize("B,hq,hkv,nsplit", [(256, 7, 1, 1), (257, 4, 2, 1), (75, 8, 4, 2), (149, 2, 1, 1)])
+def test_paged_decode_many_uneven_sequences(B, hq, hkv, nsplit):
+    torch.manual_seed(B)
+    lens = torch.randint(1, 500, (B,), dtype=torch.int32)
+    lens[::9], lens[1::9], lens[B // 2] = 129, 128, 0
+    lens[-1] = 1100
+    per = (lens + 127) // 128
+    pages, width = int(per.sum()) + 1, int(per.max()) + 1
+    table = torch.zeros(B, width, dtype=torch.int32)
+    order = torch.randperm(pages - 1).int() + 1
+    at = 0
+    for b in range(B):
+        table[b, :per[b]] = order[at:at + per[b]]
+        at += int(per[b])
+    cache = torch.randn(pages, 2, hkv, 128, 128).to(torch.bfloat16).cuda()
+    q = torch.randn(B, hq, 128).to(torch.bfloat16).cuda()
+    out = F.paged_decode(q, cache, table.cuda(), lens.cuda(), nsplit=nsplit, v_transposed=True)
+    torch.cuda.synchronize()
+    assert native.read_status(q.device) == 0
+    some = lens.nonzero().flatten()
+    ref = R.paged_decode(q.cpu()[some], cache.cpu(), table[some], lens[some], v_transposed=True)
+    # probabilities and the result are rounded to bf16 (2^-9 each)
+    assert (out.cpu()[some].float() - ref.float()).norm() <= 2.0 ** -7 * ref.float().norm()
+    assert (out.cpu()[some].float() - ref.float()).abs().max() <= 2.0 ** -6 * ref.float().abs().max()
+    assert (out.cpu()[lens == 0] == 0).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("over", [
     {}, {"kl_beta": 0.05}, {"kl_beta": 0.05, "unbiased_kl_estimate": True}, {"aipo_rho": 1.1},
     {"use_decoupled_loss": True, "behav_imp_weight_cap": 1.3, "kl_beta": 0.01},
