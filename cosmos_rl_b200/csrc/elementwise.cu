@@ -434,7 +434,9 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __
 // ------------------------------------------------------------------------------------------------
 // Positions are found with 32-bit divisions unless the tensor is too large for them. row_tiles (nullable, device): only the
 // first row_tiles[0] * 128 rows are in use. A thread of the forward works on ITEMS vectors of 8 columns whose loads are all in
-// flight before the first is used.
+// flight before the first is used. The quotient is a product with the correctly rounded reciprocal: a division by 1 + e^-x takes
+// more instructions, and its path for special operands where x is zero (padding rows). 8192 x 18944: 162 us, 153; all zero
+// 299 and 152.
 template <class Index, int ITEMS>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I,
@@ -460,7 +462,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
     unpack8(g[k], a);
     unpack8(u[k], b);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = a[j] / (1.f + __expf(-a[j])) * b[j];
+    for (int j = 0; j < 8; ++j) o[j] = a[j] * __frcp_rn(1.f + __expf(-a[j])) * b[j];
     reinterpret_cast<uint4*>(out)[idx] = pack8(o);
   }
 }

@@ -127,7 +127,14 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
     else
       return B200_ERR_ARG;
   }
-  if (N > 128)
+  // 128-wide tiles, whose product takes 0.6 of the time of a 256-wide one, where those would fill more than half of one round of
+  // pairs (so that it is not cut) and these one round and at most a third of the next, which is cut then. us, 256 and 128 wide:
+  // 700 x 3584 x 18944 (42 tiles) 99 and 80, 600 x 4096 x 14336 (48) 79 and 70; 1003 x 4096 x 14336 (64) 84 and 91.
+  const int pairs = num_sms / 2, num_m = (M + G2_BM - 1) / G2_BM;
+  const long long wide = (long long)num_m * ((N + 255) / 256), narrow = (long long)num_m * ((N + 127) / 128);
+  const bool two_rounds = cut && wide <= pairs && 2 * wide > pairs && narrow > pairs && 3 * (narrow - pairs) <= pairs &&
+                          K >= 64 * G2_BK;
+  if (N > 128 && !two_rounds)
     return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
   return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
 }
