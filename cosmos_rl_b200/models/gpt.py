@@ -199,6 +199,9 @@ class Attention(nn.Module):
             q, k = F.apply_rope(q, k, positions, self.theta)
             return q, k, v.reshape(T, hkv, d)
         qkv = F.rope_qkv_(qkv, positions, hq, hkv, d, self.theta)
+        if qkv.is_contiguous() and not F.needs_graph(qkv):     # the same views with fewer calls
+            heads = qkv.view(T, hq + 2 * hkv, d)
+            return heads[:, :hq], heads[:, hq: hq + hkv], heads[:, hq + hkv:]
         q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=-1)
         return q.unflatten(-1, (hq, d)), k.unflatten(-1, (hkv, d)), v.unflatten(-1, (hkv, d))
 

@@ -31,12 +31,11 @@ def flash_fwd(q, k, v, cu_q, cu_k, max_q: int, scale: float, causal: bool = True
     Tk, hkv = k.shape[0], k.shape[1]
     out = torch.empty(Tq, hq, d, dtype=q.dtype, device=q.device)
     lse = torch.empty(hq, Tq, dtype=torch.float32, device=q.device)
-    st = native.status_word(q.device)
     native.check(native.lib().b200_flash_fwd(
-        native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(out), native.ptr(lse), native.ptr(cu_q),
-        native.ptr(cu_k), cu_q.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0), v.stride(0), out.stride(0),
-        int(max_q), 1 if causal else 0, float(scale), native.ptr(st), native.num_sms(q.device.index), native.stream()),
-        "flash_fwd")
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), cu_q.data_ptr(), cu_k.data_ptr(),
+        cu_q.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0), v.stride(0), hq * d, int(max_q),
+        1 if causal else 0, float(scale), native.status_word(q.device).data_ptr(), native.num_sms(q.device.index),
+        native.stream()), "flash_fwd")
     return out, lse
 
 

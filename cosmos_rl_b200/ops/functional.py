@@ -23,6 +23,13 @@ def _c(t: torch.Tensor) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous ``[rows, last dimension]``; a tensor that is that already is not viewed again, which costs a small call as
+    much as its launch."""
+    t = _c(t)
+    return t if t.dim() == 2 else t.view(-1, t.shape[-1])
+
+
 def needs_graph(*tensors: Optional[torch.Tensor]) -> bool:
     """Whether a call has to go through its autograd function: one of the inputs records a gradient, or forward-mode
     derivatives are being taken (which the functions refuse). Inference calls skip the function's bookkeeping."""
@@ -39,9 +46,10 @@ def needs_graph(*tensors: Optional[torch.Tensor]) -> bool:
 def _rmsnorm_fwd(x2, weight, eps, res2, rstd):
     y = torch.empty_like(x2)
     res_out = torch.empty_like(x2) if res2 is not None else None
-    native.check(native.lib().b200_rmsnorm_fwd(native.ptr(x2), native.ptr(res2), native.ptr(weight), native.ptr(y),
-                                               native.ptr(res_out), native.ptr(rstd), x2.shape[0], x2.shape[1], eps,
-                                               native.stream()), "rmsnorm_fwd")
+    T, H = x2.shape
+    native.check(native.lib().b200_rmsnorm_fwd(x2.data_ptr(), native.ptr(res2), weight.data_ptr(), y.data_ptr(),
+                                               native.ptr(res_out), native.ptr(rstd), T, H, eps, native.stream()),
+                 "rmsnorm_fwd")
     return y, res_out
 
 
@@ -88,10 +96,10 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual:
         if x.dtype != torch.bfloat16:
             raise TypeError("rms_norm on CUDA expects bf16 activations")
         if not needs_graph(x, weight, residual):
-            shape, H = x.shape, x.shape[-1]
-            y, res_out = _rmsnorm_fwd(_c(x).view(-1, H), weight, eps,
-                                      _c(residual).view(-1, H) if residual is not None else None, None)
-            return y.view(shape), res_out.view(shape) if res_out is not None else None
+            y, res_out = _rmsnorm_fwd(_rows(x), weight, eps, _rows(residual) if residual is not None else None, None)
+            if x.dim() == 2:
+                return y, res_out
+            return y.view(x.shape), res_out.view(x.shape) if res_out is not None else None
         return _RMSNorm.apply(x, weight, eps, residual)
     return reference.rms_norm(x, weight, eps, residual)
 
@@ -174,8 +182,12 @@ def rope_qkv_(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: 
         positions = positions.to(torch.int64)
         if torch.is_grad_enabled() and qkv.requires_grad:
             return _RoPEQKV.apply(qkv, positions, hq, hkv, d, theta)
-        q = qkv[:, : hq * d].unflatten(-1, (hq, d))
-        k = qkv[:, hq * d: (hq + hkv) * d].unflatten(-1, (hkv, d))
+        if qkv.shape[1] == (hq + 2 * hkv) * d and qkv.is_contiguous():
+            heads = qkv.view(qkv.shape[0], hq + 2 * hkv, d)
+            q, k = heads[:, :hq], heads[:, hq: hq + hkv]
+        else:
+            q = qkv[:, : hq * d].unflatten(-1, (hq, d))
+            k = qkv[:, hq * d: (hq + hkv) * d].unflatten(-1, (hkv, d))
         _rope_native(q, k, positions, theta, False)
         return qkv
     T = qkv.shape[0]
@@ -217,8 +229,8 @@ class _SwiGLU(torch.autograd.Function):
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     if gate_up.is_cuda:
         if not needs_graph(gate_up):
-            I2 = gate_up.shape[-1]
-            return _swiglu_fwd(_c(gate_up).view(-1, I2)).view(*gate_up.shape[:-1], I2 // 2)
+            out = _swiglu_fwd(_rows(gate_up))
+            return out if gate_up.dim() == 2 else out.view(*gate_up.shape[:-1], out.shape[1])
         return _SwiGLU.apply(gate_up)
     return reference.swiglu(gate_up)
 
@@ -329,8 +341,8 @@ def linear_tc(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
         if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or
                                         (bias is not None and bias.requires_grad)):
             return _LinearTC.apply(x, weight, bias)
-        x2 = _c(x).view(-1, x.shape[-1])
-        return linear_infer(x2, weight, bias).view(*x.shape[:-1], weight.shape[0])
+        y = linear_infer(_rows(x), weight, bias)
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], weight.shape[0])
     return torch.nn.functional.linear(x, weight, bias)
 
 
