@@ -44,6 +44,7 @@ int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K
                       int bias_bf16, int epilogue, int up_row0, int path, int cut, float* ws, uint32_t* status,
                       int num_sms, cudaStream_t stream);
 long long b200_gemm_ws_floats(int num_sms);
+int b200_gemm_cuts(int M, int N, int K, int num_sms);   // whether such a call will want it, by its sizes
 
 // Weight-streaming GEMM for decode-sized batches (M <= 256) and the reductions that finish a decode-layer step
 // (gemm_skinny.cu). x [M, K] bf16, W [rows, K] bf16. ws == NULL: out (bf16) = x W^T (+ bias), splits = 1; swiglu: W is a

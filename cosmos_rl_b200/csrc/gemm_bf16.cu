@@ -117,6 +117,15 @@ static int dispatch_bn(const void* A, const void* B, void* C, int M, int N, int 
   return launch_gemm<128, 6, A_MN, B_MN>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
 }
 
+// 128-wide tiles, whose product takes 0.6 of the time of a 256-wide one, where those would fill more than half of one round of
+// pairs (so that it is not cut) and these one round and at most a third of the next, which is cut then. us, 256 and 128 wide:
+// 700 x 3584 x 18944 (42 tiles) 99 and 80, 600 x 4096 x 14336 (48) 79 and 70; 1003 x 4096 x 14336 (64) 84 and 91.
+static bool narrow_tiles(int M, int N, int K, int pairs) {
+  const int num_m = (M + G2_BM - 1) / G2_BM;
+  const long long wide = (long long)num_m * ((N + 255) / 256), narrow = (long long)num_m * ((N + 127) / 128);
+  return wide <= pairs && 2 * wide > pairs && narrow > pairs && 3 * (narrow - pairs) <= pairs && K >= 64 * G2_BK;
+}
+
 template <bool A_MN, bool B_MN>
 static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                           long long ldc, const Gemm2Params& ep, int epi, bool cut, uint32_t* status, int num_sms,
@@ -127,14 +136,7 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
     else
       return B200_ERR_ARG;
   }
-  // 128-wide tiles, whose product takes 0.6 of the time of a 256-wide one, where those would fill more than half of one round of
-  // pairs (so that it is not cut) and these one round and at most a third of the next, which is cut then. us, 256 and 128 wide:
-  // 700 x 3584 x 18944 (42 tiles) 99 and 80, 600 x 4096 x 14336 (48) 79 and 70; 1003 x 4096 x 14336 (64) 84 and 91.
-  const int pairs = num_sms / 2, num_m = (M + G2_BM - 1) / G2_BM;
-  const long long wide = (long long)num_m * ((N + 255) / 256), narrow = (long long)num_m * ((N + 127) / 128);
-  const bool two_rounds = cut && wide <= pairs && 2 * wide > pairs && narrow > pairs && 3 * (narrow - pairs) <= pairs &&
-                          K >= 64 * G2_BK;
-  if (N > 128 && !two_rounds)
+  if (N > 128 && !(cut && narrow_tiles(M, N, K, num_sms / 2)))
     return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
   return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
 }
@@ -198,6 +200,16 @@ extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, i
                                  uint32_t* status, int num_sms, cudaStream_t stream) {
   return b200_gemm_bf16_ws(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, bias, bias_bf16, epilogue, up_row0,
                            path, 0, nullptr, status, num_sms, stream);
+}
+
+// Whether a call of b200_gemm_bf16_ws with `cut` will want its workspace, by the sizes alone and if every pair of SMs can be
+// had: a caller that asks saves the call that only finds out.
+extern "C" int b200_gemm_cuts(int M, int N, int K, int num_sms) {
+  using namespace b200;
+  if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2) return 0;
+  const int bn = N > 128 && !narrow_tiles(M, N, K, num_sms / 2) ? 256 : 128;
+  int splits = 0;
+  return g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), num_sms / 2, (K + G2_BK - 1) / G2_BK, splits) > 0;
 }
 
 // Scratch of b200_gemm_bf16_ws, in elements.

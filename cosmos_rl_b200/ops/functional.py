@@ -7,6 +7,7 @@ activations are ``[T, ...]`` with ``T`` the total number of tokens of the micro-
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -256,6 +257,16 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     return out
 
 
+@functools.lru_cache(maxsize=4096)
+def _gemm_cuts(M: int, N: int, K: int, sms: int) -> bool:
+    return native.lib().b200_gemm_cuts(M, N, K, sms) != 0
+
+
+@functools.lru_cache(maxsize=8)
+def _gemm_ws_floats(sms: int) -> int:
+    return native.lib().b200_gemm_ws_floats(sms)
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16, accumulate: bool = False,
          bias: Optional[torch.Tensor] = None, swiglu: bool = False, path: int = 0) -> torch.Tensor:
@@ -284,9 +295,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = Fals
                                    1 if swiglu else 0, N // 2 if swiglu else 0, path, 1, native.ptr(ws),
                                    native.status_word(a.device).data_ptr(), sms, strm)
 
-    rc = call(None)
-    if rc == native.NEED_WORKSPACE:     # the last round of tiles is cut along the contraction
-        rc = call(torch.empty(L.b200_gemm_ws_floats(sms), dtype=torch.float32, device=a.device))
+    def scratch():      # the last round of tiles is cut along the contraction
+        return torch.empty(_gemm_ws_floats(sms), dtype=torch.float32, device=a.device)
+
+    rc = call(scratch() if not swiglu and _gemm_cuts(M, N, K, sms) else None)
+    if rc == native.NEED_WORKSPACE:
+        rc = call(scratch())
     native.check(rc, "gemm_bf16")
     return out
 

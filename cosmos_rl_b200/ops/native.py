@@ -58,6 +58,7 @@ _SIGS = {
                           c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                           c_int, c_void_p],
     "b200_gemm_ws_floats": [c_int],
+    "b200_gemm_cuts": [c_int, c_int, c_int, c_int],
     "b200_gemm_skinny_splits": [c_int, c_int, c_int, c_int, c_int],
     "b200_gemm_skinny": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                          c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
