@@ -31,3 +31,29 @@ def test_local_arrays_read_as_vectors_are_aligned():
         for name in set(re.findall(r"\*reinterpret_cast<(?:const )?uint4\*>\((\w+)\)", src)):
             for decl in re.findall(r"^.*\b__nv_bfloat16 %s\[\d+\];" % re.escape(name), src, flags=re.M):
                 assert "alignas(16)" in decl, (path.name, decl.strip())
+
+
+def test_rms_norm_refuses_a_residual_of_other_rows(monkeypatch):
+    """The kernel reads as many residual rows as there are activations: a residual whose values do not make rows of that
+    length never reaches it, with gradients or without. (Tensors that only say that they are on a GPU.)"""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cosmos_rl_b200.ops import functional as F
+    seen = []
+
+    def launch(x2, weight, eps, res2, rstd):
+        seen.append(tuple(res2.shape))
+        return torch.empty_like(x2), torch.empty_like(x2)
+    monkeypatch.setattr(F, "_rmsnorm_fwd", launch)
+    with FakeTensorMode():
+        make = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda")
+        x, weight = make(4, 512), make(512)
+        for w in (weight, weight.clone().requires_grad_(True)):
+            for shape in ((4, 512), (2, 2, 512), (2, 1024), (2048,)):
+                F.rms_norm(x, w, residual=make(*shape))
+            for shape in ((3, 500), (4, 511), (3, 2, 500)):
+                with pytest.raises(RuntimeError):
+                    F.rms_norm(x, w, residual=make(*shape))
+    assert seen == [(4, 512)] * 8
