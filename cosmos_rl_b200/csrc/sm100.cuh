@@ -556,12 +556,13 @@ __device__ __forceinline__ float exp2_approx(float x) {
   return y;
 }
 // 2^x of two values on the fp32 pipe, for a share of the exponentials where the special-function unit is what a kernel waits
-// for. x <= 126; below -126 it is taken as -126, NaN stays NaN. x = n + f with n the nearest integer: the sum with 1.5 * 2^23
-// holds n in its low bits. 2^f is the polynomial of degree 5 whose largest relative error on [-1/2, 1/2] is least (7.5e-8,
-// found by Remez exchange); with the rounding of the Horner steps 2.1e-7, ex2.approx has 2^-22.
+// for. x <= 126; below -126.5 the result is 0, minus infinity (a hidden key's score) among it, and NaN stays NaN. x = n + f with
+// n the nearest integer: the sum with 1.5 * 2^23 holds n in its low bits, and x is held at -127, whose 2^n has no bit set. 2^f is
+// the polynomial of degree 5 whose largest relative error on [-1/2, 1/2] is least (7.5e-8, found by Remez exchange); with the
+// rounding of the Horner steps 2.1e-7, ex2.approx has 2^-22.
 __device__ __forceinline__ float2 exp2_poly2(float2 x) {
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-126.f));
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-126.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-127.f));
   const float2 t = add2(x, make_float2(12582912.f, 12582912.f));
   const float2 n = add2(t, make_float2(-12582912.f, -12582912.f));
   const float2 f = fma2(n, make_float2(-1.f, -1.f), x);

@@ -1474,6 +1474,32 @@ def test_flash_attention_forward_forms_agree(hq, hkv, causal):
     native.read_status(q.device)
 
 
+@pytest.mark.parametrize("n,hq,hkv", [(200, 4, 2), (1300, 16, 4)])     # the one-tile form; two tiles an item
+def test_flash_attention_hidden_keys_have_no_weight(n, hq, hkv):
+    """Values of later tokens and of the next sequence leave no trace, however large they are, and a query that sees no key
+    has a zero row and an infinite log-sum-exp."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(80)
+    d, scale = 128, 1.0 / math.sqrt(128)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    cu = i32([0, n, n + 77])
+    q, k, v = _bf16(n + 77, hq, d), _bf16(n + 77, hkv, d), _bf16(n + 77, hkv, d)
+    assert ((n + 127) // 128 * hq * 2 > native.num_sms(0)) == (n > 1000)
+    for causal in (True, False):
+        want, want_lse = attention.flash_fwd(q, k, v, cu, cu, n, scale, causal)
+        for first in (n // 3, n - 1, n) if causal else (n,):        # the first value that is changed
+            big = v.clone()
+            big[first:] = 3e38
+            got, got_lse = attention.flash_fwd(q, k, big, cu, cu, n, scale, causal)
+            assert torch.equal(got[:first], want[:first]) and torch.equal(got_lse, want_lse), (causal, first)
+    more = 60                                                       # queries without a key, in front
+    out, lse = attention.flash_fwd(q[:n], k[:n - more], v[:n - more], i32([0, n]), i32([0, n - more]), n, scale, True)
+    native.read_status(q.device)
+    assert (out[:more] == 0).all() and (lse[:, :more] == math.inf).all()
+    ref = R.varlen_attention(q[more:n].float(), k[:n - more].float(), v[:n - more].float(), i32([0, n - more]), scale, True)
+    assert torch.allclose(out[more:].float(), ref, atol=2e-2, rtol=2e-2)     # bf16 result and probabilities
+
+
 @pytest.mark.parametrize("hq,hkv,longest,copies", [(2, 2, 128, 1), (4, 2, 64, 1), (14, 2, 64, 5), (3, 3, 65, 1)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_flash_attention_backward_forms_agree(dirty_allocations, hq, hkv, longest, copies, causal):
