@@ -434,9 +434,10 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __
 // ------------------------------------------------------------------------------------------------
 // Positions are found with 32-bit divisions unless the tensor is too large for them. row_tiles (nullable, device): only the
 // first row_tiles[0] * 128 rows are in use. A thread of the forward works on ITEMS vectors of 8 columns whose loads are all in
-// flight before the first is used. The quotient is a product with the correctly rounded reciprocal: a division by 1 + e^-x takes
-// more instructions, and its path for special operands where x is zero (padding rows). 8192 x 18944: 162 us, 153; all zero
-// 299 and 152.
+// flight before the first is used. The quotient is a division, as in the epilogues that form SwiGLU elsewhere: the same gate and
+// up values give the same bits there and here, which a product with the reciprocal (one rounding more, 8192 x 18944 in 153 us)
+// does not. A zero gate, as in padding rows, would send it through its path for special operands and is not divided:
+// 8192 x 18944 169 us, all zero too; divided 164 and 300. (One test for eight gates: 174 and 134.)
 template <class Index, int ITEMS>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I,
@@ -462,7 +463,12 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
     unpack8(g[k], a);
     unpack8(u[k], b);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = a[j] * __frcp_rn(1.f + __expf(-a[j])) * b[j];
+    for (int j = 0; j < 8; ++j) {
+      float x = a[j] == 0.f ? 1.f : a[j];
+      asm("" : "+f"(x));   // or the compiler, which sees that the quotient is not used for a zero, divides the zero
+      const float silu = x / (1.f + __expf(-x));
+      o[j] = (a[j] == 0.f ? a[j] : silu) * b[j];
+    }
     reinterpret_cast<uint4*>(out)[idx] = pack8(o);
   }
 }

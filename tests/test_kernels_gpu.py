@@ -1500,6 +1500,21 @@ def test_flash_attention_hidden_keys_have_no_weight(n, hq, hkv):
     assert torch.allclose(out[more:].float(), ref, atol=2e-2, rtol=2e-2)     # bf16 result and probabilities
 
 
+@pytest.mark.parametrize("M", [256, 1024])      # the weight-streaming epilogue, that of the CTA pairs
+def test_swiglu_gives_the_same_bits_wherever_it_is_formed(M):
+    """Each weight row picks one input, so that the products give the gate and up values exactly: the epilogues and the kernel
+    that takes them from memory round the same way, saturated and zero gates among them."""
+    torch.manual_seed(81)
+    n = 4096
+    x = _bf16(M, n) * 4
+    x[:, ::9], x[:, 1::9], x[:, 2::9] = 0, -100, 100
+    eye = torch.eye(n, device=DEV, dtype=torch.bfloat16)
+    w = torch.cat([eye, eye.roll(5, 0)])
+    got = F.skinny_gate_up_swiglu(x, w) if M <= 256 else F.gemm(x, w, swiglu=True)
+    native.read_status(x.device)
+    assert torch.equal(got, F.swiglu(torch.cat([x, x.roll(5, 1)], 1)))
+
+
 @pytest.mark.parametrize("hq,hkv,longest,copies", [(2, 2, 128, 1), (4, 2, 64, 1), (14, 2, 64, 5), (3, 3, 65, 1)])
 @pytest.mark.parametrize("causal", [True, False])
 def test_flash_attention_backward_forms_agree(dirty_allocations, hq, hkv, longest, copies, causal):
