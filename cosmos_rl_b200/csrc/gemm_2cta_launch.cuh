@@ -81,26 +81,38 @@ gemm2_sum_shares_kernel(const float* __restrict__ ws, void* __restrict__ C, long
   }
 }
 
-// How many CTA pairs can be resident at once (asked once per kernel and device; <= num_sms / 2).
+// How many CTA pairs of `kern` run at once on `num_sms` SMs: a caller may reserve some for kernels on other streams. `whole` is
+// the kernel's own (per device): what the device has room for, asked once and whatever the first call's num_sms is. Also makes
+// the kernel's shared memory available. 0 or an error code.
 template <class Kern>
-static int max_pairs(Kern kern, int smem_bytes, int num_sms, int threads = G2_THREADS) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * (num_sms / 2), 1, 1);
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem_bytes;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-    (void)cudaGetLastError();
-    n = num_sms / 2;
+static int resident_pairs(Kern kern, int (&whole)[16], int smem_bytes, int threads, int num_sms, int& np) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return B200_ERR_RUNTIME;
+  if (whole[dev] == 0) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return B200_ERR_RUNTIME;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return B200_ERR_LAUNCH;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (sms / 2), 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem_bytes;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = sms / 2;
+    }
+    whole[dev] = n < sms / 2 ? n : sms / 2;
   }
-  return n < num_sms / 2 ? n : num_sms / 2;
+  np = whole[dev] < num_sms / 2 ? whole[dev] : num_sms / 2;
+  if (np < 1) np = 1;
+  return 0;
 }
 
 // Contraction blocks that a cut has to save a pair: the shares' way through memory and the kernel that adds them. Weight
@@ -129,19 +141,11 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   const int n_cols = EPI == G2_EPI_SWIGLU ? N / 2 : N;
   using SM = Gemm2Smem<BN, STAGES>;
   auto kern = gemm2_bf16_kernel<BN, STAGES, A_MN, B_MN, EPI>;
-  static int pairs[16] = {0};  // per device
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return B200_ERR_RUNTIME;
-  if (pairs[dev] == 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL) != cudaSuccess)
-      return B200_ERR_LAUNCH;
-    pairs[dev] = max_pairs(kern, SM::TOTAL, num_sms);
-  }
+  static int whole[16] = {0};
+  int np = 0;
+  if (const int rc = resident_pairs(kern, whole, SM::TOTAL, G2_THREADS, num_sms, np)) return rc;
   constexpr int OUT_BN = EPI == G2_EPI_SWIGLU ? BN / 2 : BN;
   const int tiles = ((M + G2_BM - 1) / G2_BM) * ((n_cols + OUT_BN - 1) / OUT_BN);
-  int np = pairs[dev];
-  if (num_sms / 2 < np) np = num_sms / 2;  // the caller may reserve SMs for kernels on other streams
-  if (np < 1) np = 1;
   ep.rest = EPI == G2_EPI_STORE && allow_cut ? g2_rest(tiles, np, (K + G2_BK - 1) / G2_BK, ep.splits) : (ep.splits = 0);
   if (ep.rest > 0 && ep.ws == nullptr) return B200_NEED_WORKSPACE;
   const int a_rows = !A_MN && M < G2_BM_CTA ? M : G2_BM_CTA;

@@ -126,6 +126,15 @@ static bool narrow_tiles(int M, int N, int K, int pairs) {
   return wide <= pairs && 2 * wide > pairs && narrow > pairs && 3 * (narrow - pairs) <= pairs && K >= 64 * G2_BK;
 }
 
+// The CTA pairs that the rules below reckon with: as many as run at once.
+static int gemm_pairs(int num_sms) {
+  static int whole[16] = {0};
+  int np = 0;
+  const int rc = resident_pairs(gemm2_bf16_kernel<256, 6, false, false, G2_EPI_STORE>, whole, Gemm2Smem<256, 6>::TOTAL, G2_THREADS,
+                                num_sms, np);
+  return rc ? num_sms / 2 : np;
+}
+
 template <bool A_MN, bool B_MN>
 static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                           long long ldc, const Gemm2Params& ep, int epi, bool cut, uint32_t* status, int num_sms,
@@ -136,7 +145,7 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
     else
       return B200_ERR_ARG;
   }
-  if (N > 128 && !(cut && narrow_tiles(M, N, K, num_sms / 2)))
+  if (N > 128 && !(cut && narrow_tiles(M, N, K, gemm_pairs(num_sms))))
     return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
   return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
 }
@@ -150,7 +159,7 @@ static bool pair_kernel_usable(const void* C, int M, long long ldc, int out_fp32
 // CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56). It is usable where the
 // rows of C are whole 16 bytes, which is what its stores write.
 static bool pair_kernel_for_few_rows(const void* C, int M, int N, long long ldc, int out_fp32, int num_sms) {
-  return M <= 128 && (N + 255) / 256 <= num_sms / 2 && pair_kernel_usable(C, 129, ldc, out_fp32) &&
+  return M <= 128 && (N + 255) / 256 <= gemm_pairs(num_sms) && pair_kernel_usable(C, 129, ldc, out_fp32) &&
          ((N * (out_fp32 ? 4 : 2)) & 15) == 0;
 }
 
@@ -202,14 +211,14 @@ extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, i
                            path, 0, nullptr, status, num_sms, stream);
 }
 
-// Whether a call of b200_gemm_bf16_ws with `cut` will want its workspace, by the sizes alone and if every pair of SMs can be
-// had: a caller that asks saves the call that only finds out.
+// Whether a call of b200_gemm_bf16_ws with `cut` will want its workspace, by the sizes alone: a caller that asks saves the call
+// that only finds out.
 extern "C" int b200_gemm_cuts(int M, int N, int K, int num_sms) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2) return 0;
-  const int bn = N > 128 && !narrow_tiles(M, N, K, num_sms / 2) ? 256 : 128;
+  const int pairs = gemm_pairs(num_sms), bn = N > 128 && !narrow_tiles(M, N, K, pairs) ? 256 : 128;
   int splits = 0;
-  return g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), num_sms / 2, (K + G2_BK - 1) / G2_BK, splits) > 0;
+  return g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), pairs, (K + G2_BK - 1) / G2_BK, splits) > 0;
 }
 
 // Scratch of b200_gemm_bf16_ws, in elements.

@@ -507,20 +507,17 @@ extern "C" int b200_gemm_fp8_block(const void* A, const float* sa, const void* B
   // x 4096 67 and 50, 1500 x 4096 x 14336 111 and 91. Half of a pair would stand idle up to 128 rows.
   auto rounds = [](long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
   auto tiles = [&](int rows, int cols) { return (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
-  if (num_sms >= 2 && M > F8_BM && 9 * rounds(tiles(2 * F8_BM, FP_BN), num_sms / 2) <= 5 * rounds(tiles(F8_BM, F8_BN), num_sms)) {
-    if (make_tmap_2d(&tmB, B, N, K, ldb, F8_BN / 2, F8_BK, 1)) return B200_ERR_TENSORMAP;
-    static int pairs[16] = {0};   // per device
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return B200_ERR_RUNTIME;
-    if (pairs[dev] == 0) {
-      if (cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FP_SMEM) != cudaSuccess)
-        return B200_ERR_LAUNCH;
-      pairs[dev] = max_pairs(gemm_fp8_pair_kernel, FP_SMEM, num_sms, FP_THREADS);
+  if (num_sms >= 2 && M > F8_BM) {
+    static int whole[16] = {0};
+    int np = 0;
+    if (const int rc = resident_pairs(gemm_fp8_pair_kernel, whole, FP_SMEM, FP_THREADS, num_sms, np)) return rc;
+    const long long pair_tiles = tiles(2 * F8_BM, FP_BN);
+    if (9 * rounds(pair_tiles, np) <= 5 * rounds(tiles(F8_BM, F8_BN), num_sms)) {
+      if (make_tmap_2d(&tmB, B, N, K, ldb, F8_BN / 2, F8_BK, 1)) return B200_ERR_TENSORMAP;
+      const int grid = 2 * (pair_tiles < np ? (int)pair_tiles : np);
+      gemm_fp8_pair_kernel<<<grid, FP_THREADS, FP_SMEM, stream>>>(tmA, tmB, tmC, p);
+      return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
     }
-    int np = pairs[dev] < num_sms / 2 ? pairs[dev] : num_sms / 2;
-    if (tiles(2 * F8_BM, FP_BN) < np) np = (int)tiles(2 * F8_BM, FP_BN);
-    gemm_fp8_pair_kernel<<<2 * np, FP_THREADS, FP_SMEM, stream>>>(tmA, tmB, tmC, p);
-    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
   }
   static bool attr_set = false;
   if (!attr_set) {

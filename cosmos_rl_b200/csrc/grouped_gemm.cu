@@ -262,26 +262,22 @@ int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, in
   // there is room for, up to 128 rows an expert more than there are. A bf16 result that is added to keeps its one rounding in
   // the other kernel.
   const long long pair_tiles = (long long)num_experts * ((N + G2_BM - 1) / G2_BM) * ((K + 255) / 256);
-  if (!(accumulate && !out_fp32) && num_sms >= 2 && pair_tiles >= num_sms / 2 &&
-      pair_tiles < (1ll << 31) && max_rows >= 320ll * num_experts) {
+  if (!(accumulate && !out_fp32) && num_sms >= 2 && pair_tiles < (1ll << 31) && max_rows >= 320ll * num_experts) {
     auto kern = gemm2_bf16_kernel<256, 6, true, true, G2_EPI_EXPERTS>;
     using SM = Gemm2Smem<256, 6>;
-    static int pairs[16] = {0};   // per device
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return B200_ERR_RUNTIME;
-    if (pairs[dev] == 0) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL) != cudaSuccess) return B200_ERR_LAUNCH;
-      pairs[dev] = max_pairs(kern, SM::TOTAL, num_sms);
+    static int whole[16] = {0};
+    int np = 0;
+    if (const int rc = resident_pairs(kern, whole, SM::TOTAL, G2_THREADS, num_sms, np)) return rc;
+    if (pair_tiles >= np) {
+      Gemm2Params ep2{};
+      ep2.out_fp32 = out_fp32;
+      ep2.accumulate = accumulate;
+      ep2.a_bytes = SM::A_BYTES;
+      ep2.offsets = expert_offsets;
+      ep2.experts = num_experts;
+      kern<<<2 * np, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, tmC, N, K, 0, ep2, status);
+      return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
     }
-    Gemm2Params ep2{};
-    ep2.out_fp32 = out_fp32;
-    ep2.accumulate = accumulate;
-    ep2.a_bytes = SM::A_BYTES;
-    ep2.offsets = expert_offsets;
-    ep2.experts = num_experts;
-    const int np = pairs[dev] < num_sms / 2 ? pairs[dev] : num_sms / 2;
-    kern<<<2 * np, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, tmC, N, K, 0, ep2, status);
-    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
   }
   static bool s2 = false;
   if (set_smem(grouped_wgrad_kernel, s2)) return B200_ERR_LAUNCH;

@@ -1,5 +1,8 @@
 """Numerics of every sm_100a kernel against the fp32 PyTorch statements in ops/reference.py."""
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -1593,3 +1596,25 @@ def test_flash_attention_running_maximum_in_both_forms(h):
         ref, ref_lse = R.varlen_attention(q.float(), k.float(), v.float(), cu, 1.0 / math.sqrt(d), causal, return_lse=True)
         assert torch.allclose(out.float(), ref, atol=2e-2, rtol=2e-2)      # bf16 result and probabilities
         assert torch.allclose(lse, ref_lse, atol=1e-2, rtol=1e-4)
+
+
+def test_few_sms_in_the_first_call_do_not_bind_the_later_ones():
+    """How many CTA pairs run at once is the device's affair: a process whose first product leaves SMs to other streams gets
+    all of them in the next call, whose tiles then leave pairs idle and want scratch to be cut."""
+    code = """
+import torch
+from cosmos_rl_b200.ops import native
+L, st = native.lib(), native.status_word(torch.device("cuda", 0))
+def call(M, N, K, sms):
+    a, b = (torch.randn(n, K, device="cuda").to(torch.bfloat16) for n in (M, N))
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    return L.b200_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 0, 0, 0, 0, None, 0, 0, 0, 0, 1, None,
+                               st.data_ptr(), sms, native.stream())
+assert call(256, 2048, 512, 8) == 0
+assert call(100, 4096, 8192, native.num_sms(0)) == native.NEED_WORKSPACE
+torch.cuda.synchronize()
+native.read_status(st.device)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
