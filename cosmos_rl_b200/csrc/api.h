@@ -37,14 +37,14 @@ int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, int N, int K
                       int bias_bf16, int epilogue, int up_row0, int path, uint32_t* status, int num_sms,
                       cudaStream_t stream);
 
-// Same. With `cut` a call whose tiles leave half of their last round of CTA pairs idle cuts that round along the contraction;
-// ws: fp32 scratch of b200_gemm_ws_floats(num_sms) elements (null: B200_NEED_WORKSPACE from a call that would use it).
+// Same. With `cut` a call whose tiles leave half of their last round of CTA pairs idle cuts that round along the contraction.
+// ws: fp32 scratch of ws_floats elements; B200_NEED_WORKSPACE from a call that would use more. b200_gemm_scratch: how many such
+// a call uses (0: it is not cut), rows16: C and its row stride are multiples of 16 bytes.
 int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                       long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate, const void* bias,
-                      int bias_bf16, int epilogue, int up_row0, int path, int cut, float* ws, uint32_t* status,
-                      int num_sms, cudaStream_t stream);
-long long b200_gemm_ws_floats(int num_sms);
-int b200_gemm_cuts(int M, int N, int K, int num_sms);   // whether such a call will want it, by its sizes
+                      int bias_bf16, int epilogue, int up_row0, int path, int cut, float* ws, long long ws_floats,
+                      uint32_t* status, int num_sms, cudaStream_t stream);
+long long b200_gemm_scratch(int M, int N, int K, int rows16, int out_fp32, int bias, int epilogue, int path, int num_sms);
 
 // Weight-streaming GEMM for decode-sized batches (M <= 256) and the reductions that finish a decode-layer step
 // (gemm_skinny.cu). x [M, K] bf16, W [rows, K] bf16. ws == NULL: out (bf16) = x W^T (+ bias), splits = 1; swiglu: W is a

@@ -119,9 +119,6 @@ static int resident_pairs(Kern kern, int (&whole)[16], int smem_bytes, int threa
 // gradients, us, uncut and cut: 1500 tokens (24 blocks), 6144 x 4096 57 and 61; 2048 tokens (32 blocks) 74 and 77. Of 64 blocks
 // and more every cut pays: 300 x 4096 x 28672 141 and 89, 1500 x 4096 x 14336 149 and 125, 1500 x 4096 x 4096 49 and 44.
 constexpr int G2_CUT_BLOCKS = 30;
-// Scratch of a launch whose last round is cut (Gemm2Params::ws) for `num_sms` SMs.
-constexpr long long g2_ws_floats(int num_sms) { return (long long)(num_sms / 2) * G2_BM * 256; }
-
 // Tiles of the last round that are cut along the contraction, into how many shares; 0: none.
 inline int g2_rest(long long tiles, int pairs, int num_kb, int& splits) {
   const int rest = (int)(tiles % pairs);
@@ -132,11 +129,14 @@ inline int g2_rest(long long tiles, int pairs, int num_kb, int& splits) {
   return rest;
 }
 
-// allow_cut: a launch that would gain from a workspace and has none (ep.ws null) returns B200_NEED_WORKSPACE
+// Scratch of a launch that cuts `rest` tiles (Gemm2Params::ws), in elements.
+constexpr long long g2_ws_floats(int rest, int splits, int bn) { return (long long)rest * splits * G2_BM * bn; }
+
+// allow_cut: a launch that would gain from a workspace and has too little (ep.ws, ws_floats) returns B200_NEED_WORKSPACE
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
 static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                         long long ldc, Gemm2Params ep, uint32_t* status, int num_sms, cudaStream_t stream,
-                        bool allow_cut = false) {
+                        bool allow_cut = false, long long ws_floats = 0) {
   CUtensorMap tmA, tmB, tmC, tmW;
   const int n_cols = EPI == G2_EPI_SWIGLU ? N / 2 : N;
   using SM = Gemm2Smem<BN, STAGES>;
@@ -147,7 +147,7 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
   constexpr int OUT_BN = EPI == G2_EPI_SWIGLU ? BN / 2 : BN;
   const int tiles = ((M + G2_BM - 1) / G2_BM) * ((n_cols + OUT_BN - 1) / OUT_BN);
   ep.rest = EPI == G2_EPI_STORE && allow_cut ? g2_rest(tiles, np, (K + G2_BK - 1) / G2_BK, ep.splits) : (ep.splits = 0);
-  if (ep.rest > 0 && ep.ws == nullptr) return B200_NEED_WORKSPACE;
+  if (ep.rest > 0 && (ep.ws == nullptr || ws_floats < g2_ws_floats(ep.rest, ep.splits, BN))) return B200_NEED_WORKSPACE;
   const int a_rows = !A_MN && M < G2_BM_CTA ? M : G2_BM_CTA;
   ep.a_bytes = a_rows * G2_BK * 2;
   if (A_MN ? make_tmap_2d(&tmA, A, K, M, lda, 64, 64, 2) : make_tmap_2d(&tmA, A, M, K, lda, a_rows, G2_BK, 2))
@@ -156,7 +156,7 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
     return B200_ERR_TENSORMAP;
   if (make_tmap_out(&tmC, C, M, n_cols, ldc, ep.out_fp32)) return B200_ERR_TENSORMAP;
   tmW = tmC;
-  if (ep.rest > 0 && make_tmap_out(&tmW, ep.ws, (uint64_t)np * G2_BM, BN, BN, 1)) return B200_ERR_TENSORMAP;
+  if (ep.rest > 0 && make_tmap_out(&tmW, ep.ws, (uint64_t)ep.rest * ep.splits * G2_BM, BN, BN, 1)) return B200_ERR_TENSORMAP;
   const int grid = 2 * (ep.rest > 0 || tiles >= np ? np : tiles);
   kern<<<grid, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, tmW, M, N, K, ep, status);
   if (cudaGetLastError() != cudaSuccess) return B200_ERR_LAUNCH;

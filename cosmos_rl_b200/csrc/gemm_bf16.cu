@@ -135,32 +135,36 @@ static int gemm_pairs(int num_sms) {
   return rc ? num_sms / 2 : np;
 }
 
+static int pair_tile_width(int M, int N, int K, bool cut, int num_sms) {
+  return N > 128 && !(cut && narrow_tiles(M, N, K, gemm_pairs(num_sms))) ? 256 : 128;
+}
+
 template <bool A_MN, bool B_MN>
 static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                          long long ldc, const Gemm2Params& ep, int epi, bool cut, uint32_t* status, int num_sms,
-                          cudaStream_t stream) {
+                          long long ldc, const Gemm2Params& ep, int epi, bool cut, long long ws_floats, uint32_t* status,
+                          int num_sms, cudaStream_t stream) {
   if (epi == G2_EPI_SWIGLU) {
     if constexpr (!A_MN && !B_MN)
       return launch_gemm2<256, 6, false, false, G2_EPI_SWIGLU>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream);
     else
       return B200_ERR_ARG;
   }
-  if (N > 128 && !(cut && narrow_tiles(M, N, K, gemm_pairs(num_sms))))
-    return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
-  return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut);
-}
-
-static bool pair_kernel_usable(const void* C, int M, long long ldc, int out_fp32) {
-  const int eb = out_fp32 ? 4 : 2;
-  return M > 128 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ((ldc * eb) & 15) == 0;
+  if (pair_tile_width(M, N, K, cut, num_sms) == 256)
+    return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut, ws_floats);
+  return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut, ws_floats);
 }
 
 // Up to 128 rows the pair kernel is the faster one when all its tiles run at once, with or without a cut (100 rows, us, single
 // CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56). It is usable where the
 // rows of C are whole 16 bytes, which is what its stores write.
-static bool pair_kernel_for_few_rows(const void* C, int M, int N, long long ldc, int out_fp32, int num_sms) {
-  return M <= 128 && (N + 255) / 256 <= gemm_pairs(num_sms) && pair_kernel_usable(C, 129, ldc, out_fp32) &&
-         ((N * (out_fp32 ? 4 : 2)) & 15) == 0;
+static bool pairs_for_few_rows(int M, int N, int out_fp32, int num_sms) {
+  return M <= 128 && (N + 255) / 256 <= gemm_pairs(num_sms) && ((N * (out_fp32 ? 4 : 2)) & 15) == 0;
+}
+
+// Whether a call takes the CTA-pair kernel. rows16: the rows of C start on 16-byte boundaries; without that there is none.
+static bool takes_pairs(bool rows16, int M, int N, int out_fp32, bool bias, int epilogue, int path, bool cut, int num_sms) {
+  if (epilogue == G2_EPI_SWIGLU || bias || path == 2) return true;   // what only this kernel has
+  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, out_fp32, num_sms)));
 }
 
 }  // namespace b200
@@ -173,29 +177,30 @@ static bool pair_kernel_for_few_rows(const void* C, int M, int N, long long ldc,
 // (reason << 24) | CUresult of the last tensor-map encode that failed in this process (0: none); see gemm_core.cuh
 extern "C" int b200_last_tmap_error() { return b200::last_tmap_error(); }
 
-// cut: a call whose tiles leave half of their last round of CTA pairs idle cuts it along the contraction. ws: scratch for that
-// (b200_gemm_ws_floats); null: such a call returns B200_NEED_WORKSPACE and has launched nothing.
+// cut: a call whose tiles leave half of their last round of CTA pairs idle cuts it along the contraction. ws: scratch of
+// ws_floats elements for that; with less than b200_gemm_scratch says such a call returns B200_NEED_WORKSPACE and has launched
+// nothing.
 extern "C" int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                                  long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate,
                                  const void* bias, int bias_bf16, int epilogue, int up_row0, int path, int cut, float* ws,
-                                 uint32_t* status, int num_sms, cudaStream_t stream) {
+                                 long long ws_floats, uint32_t* status, int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return B200_ERR_ARG;
   // TMA needs 16-byte aligned row strides; MN-major tiles are fetched in 64-element columns
   if ((lda & 7) || (ldb & 7)) return B200_ERR_ARG;
   using namespace b200;
-  const bool want_pair = path != 1 && (pair_kernel_usable(C, M, ldc, out_fp32) ||
-                                       (cut && pair_kernel_for_few_rows(C, M, N, ldc, out_fp32, num_sms)));
-  if (epilogue == G2_EPI_SWIGLU || bias != nullptr || path == 2) {
-    // epilogues that only the CTA-pair kernel has
-    if (!pair_kernel_usable(C, 129, ldc, out_fp32)) return B200_ERR_ARG;
+  const bool rows16 = !(reinterpret_cast<uintptr_t>(C) & 15) && !((ldc * (out_fp32 ? 4 : 2)) & 15);
+  if (takes_pairs(rows16, M, N, out_fp32, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
+    if (!rows16) return B200_ERR_ARG;
     if (epilogue == G2_EPI_SWIGLU && (a_mn || b_mn || (N & 1) || accumulate)) return B200_ERR_ARG;
-  }
-  if (want_pair || epilogue == G2_EPI_SWIGLU || bias != nullptr || path == 2) {
     Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, {}};
-    if (!a_mn && !b_mn) return dispatch_gemm2<false, false>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
-    if (!a_mn && b_mn) return dispatch_gemm2<false, true>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
-    if (a_mn && b_mn) return dispatch_gemm2<true, true>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
-    return dispatch_gemm2<true, false>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0, status, num_sms, stream);
+    auto go = [&](auto am, auto bm) {
+      return dispatch_gemm2<decltype(am)::value, decltype(bm)::value>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0,
+                                                                      ws_floats, status, num_sms, stream);
+    };
+    if (!a_mn && !b_mn) return go(std::false_type{}, std::false_type{});
+    if (!a_mn && b_mn) return go(std::false_type{}, std::true_type{});
+    if (a_mn && b_mn) return go(std::true_type{}, std::true_type{});
+    return go(std::true_type{}, std::false_type{});
   }
   if (!a_mn && !b_mn) return dispatch_bn<false, false>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
   if (!a_mn && b_mn) return dispatch_bn<false, true>(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, status, num_sms, stream);
@@ -208,21 +213,21 @@ extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, i
                                  const void* bias, int bias_bf16, int epilogue, int up_row0, int path,
                                  uint32_t* status, int num_sms, cudaStream_t stream) {
   return b200_gemm_bf16_ws(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, bias, bias_bf16, epilogue, up_row0,
-                           path, 0, nullptr, status, num_sms, stream);
+                           path, 0, nullptr, 0, status, num_sms, stream);
 }
 
-// Whether a call of b200_gemm_bf16_ws with `cut` will want its workspace, by the sizes alone: a caller that asks saves the call
-// that only finds out.
-extern "C" int b200_gemm_cuts(int M, int N, int K, int num_sms) {
+// Scratch that such a call with `cut` wants, in elements; 0: it is not cut. rows16: C and its row stride are multiples of 16 bytes.
+extern "C" long long b200_gemm_scratch(int M, int N, int K, int rows16, int out_fp32, int bias, int epilogue, int path,
+                                       int num_sms) {
   using namespace b200;
-  if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2) return 0;
-  const int pairs = gemm_pairs(num_sms), bn = N > 128 && !narrow_tiles(M, N, K, pairs) ? 256 : 128;
+  if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2 || epilogue == G2_EPI_SWIGLU || !rows16) return 0;
+  if (!takes_pairs(true, M, N, out_fp32, bias != 0, epilogue, path, true, num_sms)) return 0;
+  const int bn = pair_tile_width(M, N, K, true, num_sms);
   int splits = 0;
-  return g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), pairs, (K + G2_BK - 1) / G2_BK, splits) > 0;
+  const int rest = g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), gemm_pairs(num_sms),
+                           (K + G2_BK - 1) / G2_BK, splits);
+  return g2_ws_floats(rest, splits, bn);
 }
-
-// Scratch of b200_gemm_bf16_ws, in elements.
-extern "C" long long b200_gemm_ws_floats(int num_sms) { return b200::g2_ws_floats(num_sms); }
 
 extern "C" int b200_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                               long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate,

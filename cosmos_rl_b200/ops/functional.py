@@ -260,13 +260,8 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_cuts(M: int, N: int, K: int, sms: int) -> bool:
-    return native.lib().b200_gemm_cuts(M, N, K, sms) != 0
-
-
-@functools.lru_cache(maxsize=8)
-def _gemm_ws_floats(sms: int) -> int:
-    return native.lib().b200_gemm_ws_floats(sms)
+def _gemm_scratch(M: int, N: int, K: int, rows16: bool, out_fp32: bool, bias: bool, swiglu: bool, path: int, sms: int) -> int:
+    return native.lib().b200_gemm_scratch(M, N, K, rows16, out_fp32, bias, swiglu, path, sms)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = False,
@@ -288,21 +283,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = Fals
     if bias is not None:
         assert bias.is_contiguous() and bias.numel() == N and bias.dtype in (torch.bfloat16, torch.float32)
     dev = a.device.index if a.device.index is not None else torch.cuda.current_device()
-    sms, strm, L = native.num_sms(dev), native.stream(), native.lib()
+    sms, out_fp32 = native.num_sms(dev), out.dtype == torch.float32
+    rows16 = (out.data_ptr() | out.stride(0) * out.element_size()) % 16 == 0
+    floats, ws = _gemm_scratch(M, N, K, rows16, out_fp32, bias is not None, swiglu, path, sms), None
 
-    def call(ws):
-        return L.b200_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-                                   int(a_mn), int(b_mn), 1 if out.dtype == torch.float32 else 0, 1 if accumulate else 0,
-                                   native.ptr(bias), 1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
-                                   1 if swiglu else 0, N // 2 if swiglu else 0, path, 1, native.ptr(ws),
-                                   native.status_word(a.device).data_ptr(), sms, strm)
+    def call(cut):
+        return native.lib().b200_gemm_bf16_ws(
+            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+            int(out_fp32), int(accumulate), native.ptr(bias), int(bias is not None and bias.dtype == torch.bfloat16), int(swiglu),
+            N // 2 if swiglu else 0, path, cut, native.ptr(ws), floats, native.status_word(a.device).data_ptr(), sms,
+            native.stream())
 
-    def scratch():      # the last round of tiles is cut along the contraction
-        return torch.empty(_gemm_ws_floats(sms), dtype=torch.float32, device=a.device)
-
-    rc = call(scratch() if not swiglu and _gemm_cuts(M, N, K, sms) else None)
+    if floats:      # the last round of tiles is cut along the contraction; it stays whole where there is no room for that
+        try:
+            ws = torch.empty(floats, dtype=torch.float32, device=a.device)
+        except torch.cuda.OutOfMemoryError:
+            floats = 0
+    rc = call(1)
     if rc == native.NEED_WORKSPACE:
-        rc = call(scratch())
+        rc = call(0)
     native.check(rc, "gemm_bf16")
     return out
 

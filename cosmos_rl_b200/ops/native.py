@@ -55,10 +55,9 @@ _SIGS = {
     "b200_gemm_bf16_ex": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                           c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_gemm_bf16_ws": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-                          c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                          c_int, c_void_p],
-    "b200_gemm_ws_floats": [c_int],
-    "b200_gemm_cuts": [c_int, c_int, c_int, c_int],
+                          c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong,
+                          c_void_p, c_int, c_void_p],
+    "b200_gemm_scratch": [c_int] * 9,
     "b200_gemm_skinny_splits": [c_int, c_int, c_int, c_int, c_int],
     "b200_gemm_skinny": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                          c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
@@ -143,7 +142,7 @@ def lib() -> ctypes.CDLL:
         if hasattr(handle, name):
             fn = getattr(handle, name)
             fn.argtypes = args
-            fn.restype = c_longlong if name == "b200_gemm_ws_floats" else c_int
+            fn.restype = c_longlong if name == "b200_gemm_scratch" else c_int
     return handle
 
 

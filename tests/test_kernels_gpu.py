@@ -1608,7 +1608,7 @@ L, st = native.lib(), native.status_word(torch.device("cuda", 0))
 def call(M, N, K, sms):
     a, b = (torch.randn(n, K, device="cuda").to(torch.bfloat16) for n in (M, N))
     out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
-    return L.b200_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 0, 0, 0, 0, None, 0, 0, 0, 0, 1, None,
+    return L.b200_gemm_bf16_ws(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 0, 0, 0, 0, None, 0, 0, 0, 0, 1, None, 0,
                                st.data_ptr(), sms, native.stream())
 assert call(256, 2048, 512, 8) == 0
 assert call(100, 4096, 8192, native.num_sms(0)) == native.NEED_WORKSPACE
@@ -1618,3 +1618,40 @@ native.read_status(st.device)
     r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_gemm_scratch_is_what_the_call_uses():
+    """A call that is not cut takes no scratch, one that is takes the room of its shares, and where that cannot be had the
+    tiles stay whole."""
+    torch.manual_seed(84)
+    N, K = 3840, 4104
+    a, b, buf = _bf16(1300, K), _bf16(N, K), torch.empty(1300, N + 8, dtype=torch.bfloat16, device=DEV)
+    ref = a.double() @ b.double().t()
+    native.status_word(a.device)
+
+    def check(out):
+        native.read_status(a.device)
+        # one rounding to bf16 and fp32 sums of K products
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -20 * a.double().norm(dim=1, keepdim=True)
+                * b.double().norm(dim=1) + 1e-5).all()
+
+    def taken(out, path):
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        F.gemm(a, b, out=out, path=path)
+        return torch.cuda.max_memory_allocated() - before
+    tiles, pairs = 6 * 15, native.num_sms(0) // 2
+    shares = tiles % pairs * (pairs // (tiles % pairs))
+    # four bytes a value of each share of 256 x 256; single CTAs; rows that do not start on 16-byte boundaries
+    for out, path, want in ((buf[:, :N], 0, shares * 256 * 256 * 4), (buf[:, :N], 1, 0), (buf[:, 1:N + 1], 0, 0)):
+        assert taken(out, path) == want
+        check(out)
+    torch.cuda.empty_cache()
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (1 << 20)) /
+                                                   torch.cuda.get_device_properties(0).total_memory)
+        buf.zero_()
+        assert taken(buf[:, :N], 0) == 0
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    check(buf[:, :N])
