@@ -156,15 +156,21 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
 
 // Up to 128 rows the pair kernel is the faster one when all its tiles run at once, with or without a cut (100 rows, us, single
 // CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56). It is usable where the
-// rows of C are whole 16 bytes, which is what its stores write.
-static bool pairs_for_few_rows(int M, int N, int out_fp32, int num_sms) {
-  return M <= 128 && (N + 255) / 256 <= gemm_pairs(num_sms) && ((N * (out_fp32 ? 4 : 2)) & 15) == 0;
+// rows of C are whole 16 bytes, which is what its stores write. A product that is added to bf16 values is rounded once, with the
+// sum, in the single-CTA kernel and where a tile is cut; the TMA adds of whole tiles would round it before, too.
+static bool pairs_for_few_rows(int M, int N, int K, int out_fp32, int accumulate, int num_sms) {
+  if (M > 128 || (N + 255) / 256 > gemm_pairs(num_sms) || ((N * (out_fp32 ? 4 : 2)) & 15)) return false;
+  if (out_fp32 || !accumulate) return true;
+  const int bn = pair_tile_width(M, N, K, true, num_sms), tiles = (N + bn - 1) / bn;
+  int splits = 0;
+  return g2_rest(tiles, gemm_pairs(num_sms), (K + G2_BK - 1) / G2_BK, splits) == tiles;
 }
 
 // Whether a call takes the CTA-pair kernel. rows16: the rows of C start on 16-byte boundaries; without that there is none.
-static bool takes_pairs(bool rows16, int M, int N, int out_fp32, bool bias, int epilogue, int path, bool cut, int num_sms) {
+static bool takes_pairs(bool rows16, int M, int N, int K, int out_fp32, int accumulate, bool bias, int epilogue, int path, bool cut,
+                        int num_sms) {
   if (epilogue == G2_EPI_SWIGLU || bias || path == 2) return true;   // what only this kernel has
-  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, out_fp32, num_sms)));
+  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, K, out_fp32, accumulate, num_sms)));
 }
 
 }  // namespace b200
@@ -189,7 +195,7 @@ extern "C" int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, i
   if ((lda & 7) || (ldb & 7)) return B200_ERR_ARG;
   using namespace b200;
   const bool rows16 = !(reinterpret_cast<uintptr_t>(C) & 15) && !((ldc * (out_fp32 ? 4 : 2)) & 15);
-  if (takes_pairs(rows16, M, N, out_fp32, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
+  if (takes_pairs(rows16, M, N, K, out_fp32, accumulate, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
     if (!rows16) return B200_ERR_ARG;
     if (epilogue == G2_EPI_SWIGLU && (a_mn || b_mn || (N & 1) || accumulate)) return B200_ERR_ARG;
     Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, {}};
@@ -217,11 +223,11 @@ extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, i
 }
 
 // Scratch that such a call with `cut` wants, in elements; 0: it is not cut. rows16: C and its row stride are multiples of 16 bytes.
-extern "C" long long b200_gemm_scratch(int M, int N, int K, int rows16, int out_fp32, int bias, int epilogue, int path,
-                                       int num_sms) {
+extern "C" long long b200_gemm_scratch(int M, int N, int K, int rows16, int out_fp32, int accumulate, int bias, int epilogue,
+                                       int path, int num_sms) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2 || epilogue == G2_EPI_SWIGLU || !rows16) return 0;
-  if (!takes_pairs(true, M, N, out_fp32, bias != 0, epilogue, path, true, num_sms)) return 0;
+  if (!takes_pairs(true, M, N, K, out_fp32, accumulate, bias != 0, epilogue, path, true, num_sms)) return 0;
   const int bn = pair_tile_width(M, N, K, true, num_sms);
   int splits = 0;
   const int rest = g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), gemm_pairs(num_sms),

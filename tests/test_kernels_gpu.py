@@ -1655,3 +1655,15 @@ def test_gemm_scratch_is_what_the_call_uses():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     check(buf[:, :N])
+
+
+@pytest.mark.parametrize("M,N,K", [(100, 4096, 512), (128, 520, 256), (77, 4096, 8192), (16, 104, 4096)])
+def test_gemm_few_rows_added_to_bf16_are_rounded_once(M, N, K):
+    """Sums of whole numbers, which fp32 holds exactly: what was there and the product make one bf16 value with one rounding."""
+    torch.manual_seed(85)
+    a, b = (torch.randint(-3, 4, (n, K), device=DEV).to(torch.bfloat16) for n in (M, N))
+    out = (torch.randn(M, N, device=DEV) * 16).to(torch.bfloat16)
+    want = (out.float() + a.float() @ b.float().t()).to(torch.bfloat16)
+    F.gemm(a, b, out=out, accumulate=True)
+    native.read_status(a.device)
+    assert torch.equal(out, want)
