@@ -14,7 +14,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 }
 
 // C of the cut tiles: the sum of their shares (+ bias) (+ C). A warp has one row of a tile, a lane eight columns; rows of C
-// start on 16-byte boundaries. Grid (rest, 256 / 8).
+// start on 16-byte boundaries. Above 128 rows the sum is added to C in memory, like the tiles that are not cut: whatever else
+// adds to C at that time, no value is lost. Fewer rows are all cut, or added by the single-CTA kernel, and read C and write it.
+// Grid (rest, 256 / 8).
 template <int BN>
 __global__ void __launch_bounds__(256)
 gemm2_sum_shares_kernel(const float* __restrict__ ws, void* __restrict__ C, long long ldc, int M, int N, Gemm2Params ep) {
@@ -52,13 +54,35 @@ gemm2_sum_shares_kernel(const float* __restrict__ ws, void* __restrict__ C, long
           v[j] += ep.bias_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(ep.bias)[col + j])
                                : reinterpret_cast<const float*>(ep.bias)[col + j];
     }
+    const bool add = ep.accumulate && M > 128;
     if (ep.out_fp32) {
       float* dst = reinterpret_cast<float*>(C) + row * ldc + col;
+      if (add) {
+        if (col + 8 <= N) {
+          red_add(dst, v[0], v[1], v[2], v[3]);
+          red_add(dst + 4, v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (col + j < N) atomicAdd(dst + j, v[j]);
+        }
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         if (col + j < N) dst[j] = ep.accumulate ? dst[j] + v[j] : v[j];
     } else {
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + row * ldc + col;
+      if (add) {
+        if (col + 8 <= N) {
+          red_add(dst, pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (col + j < N) atomicAdd(dst + j, __float2bfloat16(v[j]));
+        }
+        continue;
+      }
       if (col + 8 <= N) {
         if (ep.accumulate) {
           const uint4 old = *reinterpret_cast<const uint4*>(dst);

@@ -1667,3 +1667,26 @@ def test_gemm_few_rows_added_to_bf16_are_rounded_once(M, N, K):
     F.gemm(a, b, out=out, accumulate=True)
     native.read_status(a.device)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,N", [(300, 4096), (264, 1032)])
+def test_gemm_cut_tiles_added_from_two_streams(dtype, M, N):
+    """Products of small whole numbers that two streams add to one result at the same time: no addend is lost, in tiles that
+    are cut as in those that are not, and every sum is exact in either type."""
+    torch.manual_seed(86)
+    K, times = 8192, 8
+    a, b = ((torch.rand(n, K, device=DEV) < 1 / 64).to(torch.bfloat16) for n in (M, N))
+    want = a.float() @ b.float().t()
+    assert want.max() * 2 * times <= 256
+    assert F._gemm_scratch(M, N, K, True, dtype == torch.float32, True, False, False, 0, native.num_sms(0)) > 0
+    out = torch.zeros(M, N, dtype=dtype, device=DEV)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(times):
+        for s in streams:
+            with torch.cuda.stream(s):
+                F.gemm(a, b, out=out, accumulate=True)
+    torch.cuda.synchronize()
+    native.read_status(a.device)
+    assert torch.equal(out.float(), 2 * times * want)
