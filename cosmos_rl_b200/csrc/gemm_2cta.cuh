@@ -11,7 +11,8 @@
 //
 // Epilogue: the four epilogue warps of each CTA read their TMEM lane quadrant with tcgen05.ld, convert, write
 // 32-row x 128-byte slabs into swizzled staging buffers and hand them to TMA stores (or TMA reduce-adds when
-// the result is accumulated into C). TMA clips rows and columns outside C, so no edge code exists.
+// the result is accumulated into C). TMA clips rows and columns outside C; the columns of a last, incomplete 16 bytes of C's rows
+// are left to the threads (store_tail).
 //
 // Last round. Tiles rarely fill their last round of CTA pairs, and calls of few rows have fewer tiles than pairs. If at most
 // half of the pairs would have a tile in that round, its tiles come first, each cut along the contraction into as many equal
@@ -91,6 +92,8 @@ struct Gemm2Params {
   int a_bytes;       // bytes of A that the leader fetches a stage: all its 128 rows, or those there are
   int rest, splits;  // tiles 0 .. rest - 1 are cut into `splits` shares along the contraction (see "Last round"), 0: none
   float* ws;         // shares, [pairs][256][BN]
+  void* C;           // the result and its row stride, for what the tensor map leaves out
+  long long ldc;
   DlogitsParams dl;  // G2_EPI_DLOGITS
   // G2_EPI_EXPERTS: C is [experts, M, N], and expert e contracts over rows [offsets[e], offsets[e + 1]) of A and B (multiples
   // of 64; both MN-major)
@@ -422,9 +425,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         }
         fence_proxy_async_smem();
         __syncwarp();
+        const int gc = col_base + c;
         if (elect_one()) {
-          const int gc = col_base + c;
-          if (gc < n_cols && row0 < M) {
+          if (gc < (cut ? n_cols : whole16(n_cols, ep.out_fp32)) && row0 < M) {
             if constexpr (EPI == G2_EPI_EXPERTS) {
               if (ep.accumulate) tma_reduce_add_3d(tmC, slab, gc, row0, unit.batch);
               else tma_store_3d(tmC, slab, gc, row0, unit.batch);
@@ -433,6 +436,13 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
             else tma_store_2d(tmC, slab, gc, row0);
           }
           tma_store_commit();
+        }
+        if constexpr (EPI != G2_EPI_EXPERTS) {
+          const long long at = (long long)(row0 + lane) * ep.ldc;
+          if (!cut && row0 + lane < M) {
+            if (ep.out_fp32) store_tail((float*)ep.C + at, slab, gc, n_cols, ep.accumulate);
+            else store_tail((__nv_bfloat16*)ep.C + at, slab, gc, n_cols, ep.accumulate);
+          }
         }
         ++slab_idx;
       }

@@ -178,7 +178,10 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
     return B200_ERR_TENSORMAP;
   if (B_MN ? make_tmap_2d(&tmB, B, K, N, ldb, 64, 64, 2) : make_tmap_2d(&tmB, B, N, K, ldb, BN / 2, G2_BK, 2))
     return B200_ERR_TENSORMAP;
-  if (make_tmap_out(&tmC, C, M, n_cols, ldc, ep.out_fp32)) return B200_ERR_TENSORMAP;
+  ep.C = C;
+  ep.ldc = ldc;
+  const int whole_cols = whole16(n_cols, ep.out_fp32);   // 0: nothing is stored through the map
+  if (make_tmap_out(&tmC, C, M, whole_cols ? whole_cols : (ep.out_fp32 ? 4 : 8), ldc, ep.out_fp32)) return B200_ERR_TENSORMAP;
   tmW = tmC;
   if (ep.rest > 0 && make_tmap_out(&tmW, ep.ws, (uint64_t)ep.rest * ep.splits * G2_BM, BN, BN, 1)) return B200_ERR_TENSORMAP;
   const int grid = 2 * (ep.rest > 0 || tiles >= np ? np : tiles);

@@ -155,8 +155,8 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
 }
 
 // Up to 128 rows the pair kernel is the faster one when all its tiles run at once, with or without a cut (100 rows, us, single
-// CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56). It is usable where the
-// rows of C are whole 16 bytes, which is what its stores write. A product that is added to bf16 values is rounded once, with the
+// CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56), and the rows of C are
+// whole 16 bytes, which is what its stores write. A product that is added to bf16 values is rounded once, with the
 // sum, in the single-CTA kernel and where a tile is cut; the TMA adds of whole tiles would round it before, too.
 static bool pairs_for_few_rows(int M, int N, int K, int out_fp32, int accumulate, int num_sms) {
   if (M > 128 || (N + 255) / 256 > gemm_pairs(num_sms) || ((N * (out_fp32 ? 4 : 2)) & 15)) return false;
@@ -198,7 +198,7 @@ extern "C" int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, i
   if (takes_pairs(rows16, M, N, K, out_fp32, accumulate, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
     if (!rows16) return B200_ERR_ARG;
     if (epilogue == G2_EPI_SWIGLU && (a_mn || b_mn || (N & 1) || accumulate)) return B200_ERR_ARG;
-    Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, {}};
+    Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, nullptr, 0, {}};
     auto go = [&](auto am, auto bm) {
       return dispatch_gemm2<decltype(am)::value, decltype(bm)::value>(A, B, C, M, N, K, lda, ldb, ldc, ep, epilogue, cut != 0,
                                                                       ws_floats, status, num_sms, stream);

@@ -41,6 +41,24 @@ struct GemmSmem {
   static constexpr int TOTAL_WITH_EPI = EPI_OFFSET + EPI_BYTES + 1024;
 };
 
+// A TMA store or add writes whole 16 bytes, so the tensor map of a result ends where its rows have no whole 16 bytes left, and the
+// threads write the columns from there on.
+__host__ __device__ constexpr int whole16(int cols, int out_fp32) { return cols & ~(out_fp32 ? 3 : 7); }
+// Those columns of the row `c` of a result of `cols` columns, from this thread's row of a slab (32 rows x 128 bytes, 128-byte
+// swizzle) that begins at column col0.
+template <class T>
+__device__ __forceinline__ void store_tail(T* c, const uint8_t* slab, int col0, int cols, bool add) {
+  constexpr int PER = 16 / sizeof(T);
+  const int tail = cols & ~(PER - 1), in = tail - col0;
+  if (tail == cols || in < 0 || in >= 8 * PER) return;
+  const uint32_t lane = threadIdx.x & 31;
+  const T* v = reinterpret_cast<const T*>(slab + lane * 128 + (((uint32_t)(in / PER) ^ (lane & 7)) << 4));
+  for (int k = 0; k < cols - tail; ++k) {
+    if (add) atomicAdd(c + tail + k, v[k]);
+    else c[tail + k] = v[k];
+  }
+}
+
 // One output tile as seen by every role of the pipeline.
 struct TileInfo {
   int m_blk, n_blk;  // tile indices handed to the epilogue

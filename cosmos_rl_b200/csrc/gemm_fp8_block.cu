@@ -145,16 +145,6 @@ __device__ __forceinline__ void f8_fill_slab(uint8_t* slab, const float2* acc) {
                    pack_bf16x2(acc[4 * j + 2].x, acc[4 * j + 2].y), pack_bf16x2(acc[4 * j + 3].x, acc[4 * j + 3].y));
 }
 
-// The columns of the last, incomplete 16 bytes of a row, from the thread's row of its slab: a TMA store writes whole ones, so
-// the tensor map ends before them.
-__device__ __forceinline__ void f8_store_tail(const F8Params& p, const uint8_t* slab, long long row, int col0) {
-  const int tail = p.N & ~7, in = tail - col0;
-  if (tail == p.N || in < 0 || in >= 64 || row >= p.M) return;
-  const uint32_t lane = threadIdx.x & 31;
-  const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(slab + lane * 128 + (((uint32_t)(in >> 3) ^ (lane & 7)) << 4));
-  for (int c = tail; c < p.N; ++c) p.C[row * p.ldc + c] = v[c - tail];
-}
-
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmC, F8Params p) {
@@ -280,11 +270,11 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (elect_one()) tma_store_wait_read<0>();   // the store of the tile before has read the slab
       __syncwarp();
       f8_fill_slab(slab, acc);
-      f8_store_tail(p, slab, row0 + lane, col0);
+      if (row0 + lane < p.M) store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab, col0, p.N, false);
       fence_proxy_async_smem();
       __syncwarp();
       if (elect_one()) {
-        if (row0 < p.M && col0 < (p.N & ~7)) tma_store_2d(&tmC, slab, col0, row0);
+        if (row0 < p.M && col0 < whole16(p.N, 0)) tma_store_2d(&tmC, slab, col0, row0);
         tma_store_commit();
       }
     }
@@ -402,14 +392,16 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       __syncwarp();
       f8_fill_slab(slab, acc);
       f8_fill_slab(slab + 4096, acc + 32);
-      f8_store_tail(p, slab, row0 + lane, col0);
-      f8_store_tail(p, slab + 4096, row0 + lane, col0 + 64);
+      if (row0 + lane < p.M) {
+        store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab, col0, p.N, false);
+        store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab + 4096, col0 + 64, p.N, false);
+      }
       fence_proxy_async_smem();
       __syncwarp();
       if (elect_one()) {
         if (row0 < p.M) {
-          if (col0 < (p.N & ~7)) tma_store_2d(&tmC, slab, col0, row0);
-          if (col0 + 64 < (p.N & ~7)) tma_store_2d(&tmC, slab + 4096, col0 + 64, row0);
+          if (col0 < whole16(p.N, 0)) tma_store_2d(&tmC, slab, col0, row0);
+          if (col0 + 64 < whole16(p.N, 0)) tma_store_2d(&tmC, slab + 4096, col0 + 64, row0);
         }
         tma_store_commit();
       }
@@ -499,7 +491,7 @@ extern "C" int b200_gemm_fp8_block(const void* A, const float* sa, const void* B
   CUtensorMap tmA, tmB, tmC;
   if (make_tmap_2d(&tmA, A, M, K, lda, a_rows, F8_BK, 1)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, B, N, K, ldb, F8_BN, F8_BK, 1)) return B200_ERR_TENSORMAP;
-  if (make_tmap_out(&tmC, C, M, N < 8 ? 8 : N & ~7, ldc, 0)) return B200_ERR_TENSORMAP;
+  if (make_tmap_out(&tmC, C, M, N < 8 ? 8 : whole16(N, 0), ldc, 0)) return B200_ERR_TENSORMAP;
   const bool vec_scales = !((ldsa | ldsb) & 3) && !(((uintptr_t)sa | (uintptr_t)sb) & 15);
   const F8Params p{sa, sb, (__nv_bfloat16*)C, ldc, M, N, K, ldsa, ldsb, a_rows, vec_scales, status};
   // Rounds of tiles decide: a pair's round takes 1.8 times as long as one of single CTAs and does twice the work at most.

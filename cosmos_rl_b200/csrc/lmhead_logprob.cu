@@ -241,7 +241,7 @@ int b200_lmhead_dlogits(const void* hidden, const void* weight, const long long*
   // The logits are formed at the rate of the dense GEMM: CTA pairs once there are rows for their 256-row tiles (2048 x
   // 16384 x 3584: 147 us against 182 us with one CTA a tile, whose operand traffic bounds it).
   if (T > 128 && !(reinterpret_cast<uintptr_t>(dlogits) & 15) && !(ldd & 7)) {
-    const Gemm2Params ep{nullptr, 0, 0, 0, 0, 8, 0, 0, 0, nullptr, dl};
+    const Gemm2Params ep{nullptr, 0, 0, 0, 0, 8, 0, 0, 0, nullptr, nullptr, 0, dl};
     return launch_gemm2<256, 6, false, false, G2_EPI_DLOGITS>(hidden, wchunk, dlogits, T, Vc, H, ldh, ldw, ldd, ep, status,
                                                               num_sms, stream);
   }

@@ -1689,3 +1689,35 @@ def test_gemm_cut_tiles_added_from_two_streams(dtype, M, N):
     torch.cuda.synchronize()
     native.read_status(a.device)
     assert torch.equal(out.float(), 2 * times * want)
+
+
+# columns that end inside 16 bytes: fewer than those; several tiles; one tile of 128 columns; few rows; tiles that are cut; SwiGLU,
+# whose result has half of the columns
+@pytest.mark.parametrize("M,N,K,swiglu", [(200, 5, 192, False), (300, 1001, 200, False), (130, 99, 128, False),
+                                          (64, 1002, 128, False), (1300, 3843, 4104, False), (300, 2002, 200, True)])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, False),
+                                              (torch.float32, True)])
+def test_gemm_leaves_the_values_beside_its_result(M, N, K, swiglu, dtype, accumulate):
+    if swiglu and (accumulate or dtype == torch.float32):
+        pytest.skip("the SwiGLU epilogue writes bf16 and does not add")
+    torch.manual_seed(87)
+    a, b = _bf16(M, K), _bf16(N, K)
+    bias = None if swiglu else _bf16(N)                            # keeps few rows on the CTA pairs, too
+    cols = N // 2 if swiglu else N
+    buf = torch.randn(M + 1, (cols + 7) // 8 * 8 + 8, device=DEV).to(dtype)
+    before = buf.clone()
+    F.gemm(a, b, out=buf[:M, :cols], accumulate=accumulate, bias=bias, swiglu=swiglu)
+    native.read_status(a.device)
+    assert torch.equal(buf[:, cols:], before[:, cols:]) and torch.equal(buf[M], before[M])
+    h = a.double() @ b.double().t()
+    ref = torch.nn.functional.silu(h[:, :cols]) * h[:, cols:] if swiglu else h + bias.double()
+    # fp32 sums of K products (through the gate's slope of at most 1.1, times the other factor), and for bf16 one rounding of
+    # the product and one of the sum with what was there
+    size = a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=1)
+    bound = 2.0 ** -20 * (size[:, :cols] * h[:, cols:].abs() * 1.1 + size[:, cols:] * h[:, :cols].abs() if swiglu else size) + 1e-5
+    if dtype == torch.bfloat16:
+        bound = bound + 2.0 ** -8 * ref.abs()
+    if accumulate:
+        ref = ref + before[:M, :cols].double()
+        bound = bound + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22) * ref.abs()
+    assert ((buf[:M, :cols].double() - ref).abs() <= bound).all()
