@@ -42,7 +42,7 @@ struct SkinnyParams {
   int to_ws;                  // 1: fp32 partials through the 3-D map; 0: bf16 result through the 2-D map
   int M, N;                   // N = columns of the output (for SwiGLU: the intermediate size)
   int splits;
-  __nv_bfloat16* out;         // direct output of the row-store epilogue
+  __nv_bfloat16* out;         // direct output: the row-store epilogue, and what the tensor map leaves out
   long long ldo;
   int up_row0;                // SwiGLU: first "up" row of W
   int b_rows;                 // rows of W per tile (BN, or the width chosen at launch)
@@ -89,8 +89,9 @@ struct SkinnySchedule {
 };
 
 // Epilogue: each warp turns its 32 accumulator rows into slabs of 32 rows x 128 bytes (32 fp32 or 64 bf16 columns) in
-// swizzled shared memory and hands them to TMA stores, which clip rows >= M and columns >= N.
-template <int BN, bool SWIGLU>
+// swizzled shared memory and hands them to TMA stores, which clip rows >= M and columns >= N; the columns of a last, incomplete 16
+// bytes of a bf16 row are left to the threads (TAIL: there are any; a test in the loop took 0.5 us of a decode block's 115).
+template <int BN, bool SWIGLU, bool TAIL>
 struct SkinnyEpilogue {
   using Params = SkinnyParams;
   static constexpr bool CUSTOM_TILE = true;
@@ -161,14 +162,16 @@ struct SkinnyEpilogue {
       }
       fence_proxy_async_smem();
       __syncwarp();
+      const int gc = t.n_blk * OUT_BN + c;
       if (elect_one()) {
-        const int gc = t.n_blk * OUT_BN + c;
-        if (gc < p.N && row0 < p.M) {
+        if (gc < (TAIL ? whole16(p.N, 0) : p.N) && row0 < p.M) {
           if (p.to_ws) tma_store_3d(p.tm_out, slab, gc, row0, t.batch);
           else tma_store_2d(p.tm_out, slab, gc, row0);
         }
         tma_store_commit();
       }
+      if constexpr (TAIL)
+        if (row0 + lane < p.M) store_tail(p.out + (long long)(row0 + lane) * p.ldo, slab, gc, p.N, false);
       ++slab_idx;
     }
   }
@@ -218,13 +221,13 @@ struct SwigluRowsEpilogue {
   }
 };
 
-template <int BN, bool SWIGLU, int A_ROWS>
+template <int BN, bool SWIGLU, int A_ROWS, bool TAIL>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmO, int M, int N, int K, SkinnyParams ep, uint32_t* status) {
   ep.tm_out = &tmO;
   if (threadIdx.x == 0) tma_prefetch_desc(&tmO);
-  gemm_mainloop<BN, SkinnyCfg<BN, A_ROWS>::STAGES, SkinnyEpilogue<BN, SWIGLU>, SkinnySchedule<BN, SWIGLU>,
+  gemm_mainloop<BN, SkinnyCfg<BN, A_ROWS>::STAGES, SkinnyEpilogue<BN, SWIGLU, TAIL>, SkinnySchedule<BN, SWIGLU>,
                 GemmTraits<false, false, false, false, 0, false, SWIGLU, true, A_ROWS, false, true>>(&tmA, &tmB, M, N, K, ep, status);
 }
 
@@ -511,12 +514,12 @@ static int launch_skinny_kernel(Kern kern, bool& attr_set, int smem, int units, 
   return units < num_sms ? units : num_sms;   // grid
 }
 
-template <int BN, bool SWIGLU, int A_ROWS>
+template <int BN, bool SWIGLU, int A_ROWS, bool TAIL>
 static int launch_skinny(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmO, int M, int N, int K,
                          const b200::SkinnyParams& ep, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   using SM = GemmSmem<BN, SkinnyCfg<BN, A_ROWS>::STAGES, A_ROWS>;
-  auto kern = gemm_skinny_kernel<BN, SWIGLU, A_ROWS>;
+  auto kern = gemm_skinny_kernel<BN, SWIGLU, A_ROWS, TAIL>;
   static bool attr_set = false;
   constexpr int OUT_BN = SWIGLU ? BN / 2 : BN;
   const int units = ((M + GEMM_BM - 1) / GEMM_BM) * ((N + OUT_BN - 1) / OUT_BN) * ep.splits;
@@ -578,24 +581,28 @@ int b200_gemm_skinny(const void* x, const void* W, void* out, float* ws, int M, 
   CUtensorMap tmA, tmB, tmO;
   if (make_tmap_2d(&tmA, x, M, K, ldx, box_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, W, n_rows_w, K, ldw, swiglu ? b_rows / 2 : b_rows, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
-  if (ws ? make_tmap_ws(&tmO, ws, splits, M, N) : make_tmap_out16(&tmO, out, M, N, ldo)) return B200_ERR_TENSORMAP;
+  if (ws ? make_tmap_ws(&tmO, ws, splits, M, N) : make_tmap_out16(&tmO, out, M, N < 8 ? 8 : whole16(N, 0), ldo)) return B200_ERR_TENSORMAP;
   // Blocks of weights that a CTA brings into L2 ahead of its predecessor's end: a decode block of five sequences (8B) takes
   // 135.5 us without, 131.7 with half or all of this, 134.4 with twice as much; at 128 sequences (7B) 180.2, 179.7, 180.3 and
   // 182.3: more than the pipeline's own depth competes with the kernel that still runs.
   SkinnyParams ep{nullptr, ws ? nullptr : bias, bias_bf16, ws ? 1 : 0, M, N, splits, (__nv_bfloat16*)out, ldo, up_row0,
                   b_rows, box_rows * GEMM_BK * 2, pdl_enabled() ? (bn == 256 ? 8 : 16) : 0};
-  auto launch = [&](auto rows) -> int {
+  auto launch = [&](auto rows, auto tail) -> int {
     constexpr int R = decltype(rows)::value;
+    constexpr bool T = decltype(tail)::value;
     if (width) return launch_swiglu_rows<R>(tmA, tmB, M, N, K, ep, status, num_sms, stream);
     if (bn == 256)
-      return swiglu ? launch_skinny<256, true, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream)
-                    : launch_skinny<256, false, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
-    return swiglu ? launch_skinny<128, true, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream)
-                  : launch_skinny<128, false, R>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
+      return swiglu ? launch_skinny<256, true, R, T>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream)
+                    : launch_skinny<256, false, R, T>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
+    return swiglu ? launch_skinny<128, true, R, T>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream)
+                  : launch_skinny<128, false, R, T>(tmA, tmB, tmO, M, N, K, ep, status, num_sms, stream);
   };
-  if (a_rows == 16) return launch(std::integral_constant<int, 16>{});
-  if (a_rows == 64) return launch(std::integral_constant<int, 64>{});
-  return launch(std::integral_constant<int, GEMM_BM>{});
+  auto launch_rows = [&](auto tail) -> int {
+    if (a_rows == 16) return launch(std::integral_constant<int, 16>{}, tail);
+    if (a_rows == 64) return launch(std::integral_constant<int, 64>{}, tail);
+    return launch(std::integral_constant<int, GEMM_BM>{}, tail);
+  };
+  return !ws && whole16(N, 0) != N ? launch_rows(std::true_type{}) : launch_rows(std::false_type{});
 }
 
 int b200_splitk_reduce(const float* ws, int splits, int M, int N, const void* bias, int bias_bf16, void* out,

@@ -1721,3 +1721,20 @@ def test_gemm_leaves_the_values_beside_its_result(M, N, K, swiglu, dtype, accumu
         ref = ref + before[:M, :cols].double()
         bound = bound + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22) * ref.abs()
     assert ((buf[:M, :cols].double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 5, 64), (33, 1001, 256), (130, 4099, 128), (256, 20003, 64)])
+def test_skinny_leaves_the_values_beside_its_result(M, N, K):
+    """Columns that end inside 16 bytes, in rows with a stride of their own (too short a contraction to be split)."""
+    torch.manual_seed(88)
+    x, w, bias = _bf16(M, K), _bf16(N, K), _bf16(N)
+    assert native.lib().b200_gemm_skinny_splits(M, N, K, 0, native.num_sms(0)) == 1
+    buf = _bf16(M + 1, (N + 7) // 8 * 8 + 8)
+    before = buf.clone()
+    F.gemm_skinny(x, w, bias=bias, out=buf[:M, :N])
+    native.read_status(x.device)
+    assert torch.equal(buf[:, N:], before[:, N:]) and torch.equal(buf[M], before[M])
+    ref = x.double() @ w.double().t() + bias.double()
+    # one rounding to bf16 and fp32 sums of K products
+    bound = 2.0 ** -8 * ref.abs() + 2.0 ** -20 * x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=1) + 1e-5
+    assert ((buf[:M, :N].double() - ref).abs() <= bound).all()
