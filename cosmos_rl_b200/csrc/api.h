@@ -265,6 +265,7 @@ int b200_ep_combine_push(const void* y, int H, int E, int ep, int rank, const in
 int b200_gemm_fp8_block(const void* A, const float* sa, const void* B, const float* sb, void* C, int M, int N, int K,
                         long long lda, long long ldb, long long ldc, int ldsa, int ldsb, uint32_t* status, int num_sms,
                         cudaStream_t stream);
+int b200_gemm_fp8_block_pairs(int M, int N, int num_sms);   // whether such a call takes CTA pairs
 
 // Column-parallel GEMM fused with the tensor-parallel all-gather of its input rows (ag_gemm.cu).
 int b200_ag_gemm(const void* x, const void* W, void* out, int M, int N, int K, long long ldx, long long ldw,

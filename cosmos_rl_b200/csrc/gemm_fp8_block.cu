@@ -474,6 +474,23 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   }
 }
 
+static long long f8_tiles(int M, int N, int rows, int cols) { return (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols); }
+
+// CTA pairs of a call, 0: single CTAs, or an error code. Rounds of tiles decide: a pair's round takes 1.8 times as long as one of
+// single CTAs and does twice the work at most. us, pairs and single CTAs: 8192^3 488 and 514, 1000 x 28672 x 4096 119 and 122,
+// 129 x 37888 x 3584 35 and 38; 300 x 28672 x 4096 67 and 50, 1500 x 4096 x 14336 111 and 91. Half of a pair would stand idle up to
+// 128 rows.
+static int f8_pairs(int M, int N, int num_sms) {
+  if (num_sms < 2 || M <= F8_BM) return 0;
+  static int whole[16] = {0};
+  int np = 0;
+  if (const int rc = resident_pairs(gemm_fp8_pair_kernel, whole, FP_SMEM, FP_THREADS, num_sms, np)) return rc;
+  auto rounds = [](long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
+  const long long pair_tiles = f8_tiles(M, N, 2 * F8_BM, FP_BN);
+  if (9 * rounds(pair_tiles, np) > 5 * rounds(f8_tiles(M, N, F8_BM, F8_BN), num_sms)) return 0;
+  return pair_tiles < np ? (int)pair_tiles : np;
+}
+
 }  // namespace b200
 
 // A [M,K] e4m3 (row stride lda bytes = elements), sa [M, ldsa] fp32; B [N,K] e4m3, sb [ceil(N/128), ldsb] fp32;
@@ -494,22 +511,12 @@ extern "C" int b200_gemm_fp8_block(const void* A, const float* sa, const void* B
   if (make_tmap_out(&tmC, C, M, N < 8 ? 8 : whole16(N, 0), ldc, 0)) return B200_ERR_TENSORMAP;
   const bool vec_scales = !((ldsa | ldsb) & 3) && !(((uintptr_t)sa | (uintptr_t)sb) & 15);
   const F8Params p{sa, sb, (__nv_bfloat16*)C, ldc, M, N, K, ldsa, ldsb, a_rows, vec_scales, status};
-  // Rounds of tiles decide: a pair's round takes 1.8 times as long as one of single CTAs and does twice the work at most.
-  // us, pairs and single CTAs: 8192^3 488 and 514, 1000 x 28672 x 4096 119 and 122, 129 x 37888 x 3584 35 and 38; 300 x 28672
-  // x 4096 67 and 50, 1500 x 4096 x 14336 111 and 91. Half of a pair would stand idle up to 128 rows.
-  auto rounds = [](long long tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
-  auto tiles = [&](int rows, int cols) { return (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
-  if (num_sms >= 2 && M > F8_BM) {
-    static int whole[16] = {0};
-    int np = 0;
-    if (const int rc = resident_pairs(gemm_fp8_pair_kernel, whole, FP_SMEM, FP_THREADS, num_sms, np)) return rc;
-    const long long pair_tiles = tiles(2 * F8_BM, FP_BN);
-    if (9 * rounds(pair_tiles, np) <= 5 * rounds(tiles(F8_BM, F8_BN), num_sms)) {
-      if (make_tmap_2d(&tmB, B, N, K, ldb, F8_BN / 2, F8_BK, 1)) return B200_ERR_TENSORMAP;
-      const int grid = 2 * (pair_tiles < np ? (int)pair_tiles : np);
-      gemm_fp8_pair_kernel<<<grid, FP_THREADS, FP_SMEM, stream>>>(tmA, tmB, tmC, p);
-      return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
-    }
+  const int np = f8_pairs(M, N, num_sms);
+  if (np < 0) return np;
+  if (np > 0) {
+    if (make_tmap_2d(&tmB, B, N, K, ldb, F8_BN / 2, F8_BK, 1)) return B200_ERR_TENSORMAP;
+    gemm_fp8_pair_kernel<<<2 * np, FP_THREADS, FP_SMEM, stream>>>(tmA, tmB, tmC, p);
+    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
   }
   static bool attr_set = false;
   if (!attr_set) {
@@ -517,7 +524,11 @@ extern "C" int b200_gemm_fp8_block(const void* A, const float* sa, const void* B
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  const int grid = tiles(F8_BM, F8_BN) < num_sms ? (int)tiles(F8_BM, F8_BN) : num_sms;
+  const long long tiles = f8_tiles(M, N, F8_BM, F8_BN);
+  const int grid = tiles < num_sms ? (int)tiles : num_sms;
   gemm_fp8_block_kernel<<<grid, F8_THREADS, F8_SMEM, stream>>>(tmA, tmB, tmC, p);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
+
+// Whether such a call takes CTA pairs.
+extern "C" int b200_gemm_fp8_block_pairs(int M, int N, int num_sms) { return b200::f8_pairs(M, N, num_sms) > 0; }

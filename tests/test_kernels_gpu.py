@@ -602,33 +602,46 @@ def test_grouped_wgrad_forms(E, N, K, rows, out_dtype, accumulate):
 
 
 @pytest.mark.gpu
-# (rows, columns, contraction): one tile and few rows; ragged everything; 128-wide tiles; one tile past a full round; two shares
-# of uneven length; a contraction too short to be cut
-@pytest.mark.parametrize("M,N,K", [(3, 256, 4096), (127, 1032, 4200), (129, 520, 8200), (300, 104, 4096), (1300, 3840, 4104),
-                                   (900, 2304, 4160), (256, 512, 512)])
-@pytest.mark.parametrize("out_dtype,accumulate,bias,mn", [(torch.bfloat16, False, True, False), (torch.float32, True, False, False),
-                                                          (torch.bfloat16, True, False, True)])
-def test_gemm_cut_last_round(M, N, K, out_dtype, accumulate, bias, mn):
+# (rows, columns, contraction): one tile and few rows; ragged everything; tiles of 128 columns because there are no more of them;
+# tiles of 128 columns, of which ten are left for a second round; 256 columns and a second round; two shares of uneven length;
+# columns that end inside 16 bytes; a contraction too short to be cut
+@pytest.mark.parametrize("M,N,K", [(3, 256, 4096), (127, 1032, 4200), (129, 520, 8200), (300, 104, 4096), (700, 3584, 4104),
+                                   (1300, 3840, 4104), (900, 2304, 4160), (300, 1001, 4096), (256, 512, 512)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("out_dtype,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True),
+                                                  (torch.float32, True)])
+def test_gemm_cut_last_round(M, N, K, a_mn, b_mn, out_dtype, accumulate):
     torch.manual_seed(M + N)
     a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, K, device="cuda").to(torch.bfloat16)
-    bv = torch.randn(N, device="cuda").to(torch.bfloat16) if bias else None
-    if mn and M % 8:
-        pytest.skip("rows of a transposed operand are 16 bytes")
-    buf = torch.randn(M + 1, N, device="cuda").to(out_dtype)
-    out, before = buf[:M], buf.clone()
-    ops = (a.t().contiguous(), b.t().contiguous()) if mn else (a, b)
-    F.gemm(*ops, a_mn=mn, b_mn=mn, out=out, accumulate=accumulate, bias=bv)
+    bv = None if accumulate else torch.randn(N, device="cuda").to(torch.bfloat16)
+    sms, few = native.num_sms(0), M <= 128
+    width = 128 if N <= 128 or (M, N) == (700, 3584) else 256
+    left = -(-M // 256) * -(-N // width) % (sms // 2)
+    scratch = F._gemm_scratch(M, N, K, True, out_dtype == torch.float32, accumulate, bv is not None, False, 0, sms)
+    assert scratch == (0 if K == 512 else left * min(sms // 2 // left, 8) * 256 * width)
+
+    def stored(t):          # [K, rows], rows of whole 16 bytes
+        buf = torch.zeros(K, (t.shape[0] + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")
+        buf[:, :t.shape[0]] = t.t()
+        return buf[:, :t.shape[0]]
+    ops = stored(a) if a_mn else a, stored(b) if b_mn else b
+    buf = torch.randn(M + 1, (N + 7) // 8 * 8, device="cuda").to(out_dtype)
+    before = buf.clone()
+    F.gemm(*ops, a_mn=a_mn, b_mn=b_mn, out=buf[:M, :N], accumulate=accumulate, bias=bv)
     torch.cuda.synchronize()
     assert native.read_status(a.device) == 0
-    ref = a.double() @ b.double().t() + (bv.double() if bias else 0) + (before[:M].double() if accumulate else 0)
-    # fp32 sums of K products, and for bf16 one rounding of the product and one of the sum with what was there
-    bound = 2.0 ** -20 * K ** 0.5 * a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=1) / K ** 0.5 + 1e-5
-    if out_dtype == torch.bfloat16:
-        bound = bound + 2.0 ** -8 * ref.abs() + (2.0 ** -8 * (ref - before[:M].double()).abs() if accumulate else 0)
-    assert ((out.double() - ref).abs() <= bound).all()
-    assert torch.equal(buf[M], before[M])
+    ref = a.double() @ b.double().t() + (0 if accumulate else bv.double())
+    # fp32 sums of K products, and for bf16 one rounding of the product (not for few rows) and one of the sum with what was there
+    bound = 2.0 ** -20 * a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=1) + 1e-5
+    if out_dtype == torch.bfloat16 and not (accumulate and few):
+        bound = bound + 2.0 ** -8 * ref.abs()
+    if accumulate:
+        ref = ref + before[:M, :N].double()
+        bound = bound + (2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -22) * ref.abs()
+    assert ((buf[:M, :N].double() - ref).abs() <= bound).all()
+    assert torch.equal(buf[M], before[M]) and torch.equal(buf[:M, N:], before[:M, N:])
     again = before.clone()
-    F.gemm(*ops, a_mn=mn, b_mn=mn, out=again[:M], accumulate=accumulate, bias=bv)
+    F.gemm(*ops, a_mn=a_mn, b_mn=b_mn, out=again[:M, :N], accumulate=accumulate, bias=bv)
     assert torch.equal(again, buf)
 
 
@@ -671,11 +684,14 @@ def test_attention_far_apart_scores(n, hq, hkv, causal):
 
 
 @pytest.mark.gpu
-# one row; K of one block, of less than one, of 4 n + 1 blocks; columns that end inside 16 bytes; CTA pairs (enough tiles for
-# two rounds of single CTAs) with ragged rows and columns, and with more tiles than pairs
-@pytest.mark.parametrize("M,N,K", [(1, 264, 128), (3, 5, 144), (1, 4096, 640), (127, 1001, 112), (129, 19000, 128),
-                                   (257, 19197, 656), (2000, 12300, 400)])
-def test_gemm_fp8_block_forms(M, N, K):
+# one row; K of one block, of less than one, of 4 n + 1 blocks; columns that end inside 16 bytes. CTA pairs: one block, an odd
+# number of blocks, more of them than stages, with a second CTA that has one row or none and in one round of tiles and several
+@pytest.mark.parametrize("M,N,K,pairs", [(1, 264, 128, False), (3, 5, 144, False), (1, 4096, 640, False), (127, 1001, 112, False),
+                                         (129, 19000, 128, False), (257, 19197, 656, False), (129, 18900, 128, True),
+                                         (129, 18901, 656, True), (384, 9470, 640, True), (2000, 12300, 400, True),
+                                         (2000, 12300, 640, True), (1930, 12299, 1408, True)])
+def test_gemm_fp8_block_forms(M, N, K, pairs):
+    assert native.lib().b200_gemm_fp8_block_pairs(M, N, native.num_sms(0)) == pairs
     torch.manual_seed(M)
     a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
     b = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
