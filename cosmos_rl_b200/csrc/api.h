@@ -44,8 +44,8 @@ int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K
                       long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate, const void* bias,
                       int bias_bf16, int epilogue, int up_row0, int path, int cut, float* ws, long long ws_floats,
                       uint32_t* status, int num_sms, cudaStream_t stream);
-long long b200_gemm_scratch(int M, int N, int K, int rows16, int out_fp32, int accumulate, int bias, int epilogue, int path,
-                            int num_sms);
+long long b200_gemm_scratch(int M, int N, int K, int a_mn, int rows16, int out_fp32, int accumulate, int bias, int epilogue,
+                            int path, int num_sms);
 
 // Weight-streaming GEMM for decode-sized batches (M <= 256) and the reductions that finish a decode-layer step
 // (gemm_skinny.cu). x [M, K] bf16, W [rows, K] bf16. ws == NULL: out (bf16) = x W^T (+ bias), splits = 1; swiglu: W is a

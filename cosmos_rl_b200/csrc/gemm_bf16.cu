@@ -119,11 +119,14 @@ static int dispatch_bn(const void* A, const void* B, void* C, int M, int N, int 
 
 // 128-wide tiles, whose product takes 0.6 of the time of a 256-wide one, where those would fill more than half of one round of
 // pairs (so that it is not cut) and these one round and at most a third of the next, which is cut then. us, 256 and 128 wide:
-// 700 x 3584 x 18944 (42 tiles) 99 and 80, 600 x 4096 x 14336 (48) 79 and 70; 1003 x 4096 x 14336 (64) 84 and 91.
-static bool narrow_tiles(int M, int N, int K, int pairs) {
+// 700 x 3584 x 18944 (42 tiles) 99 and 80, 600 x 4096 x 14336 (48) 79 and 70, the same with B stored [K, N]; 1003 x 4096 x 14336
+// (64) 84 and 91. Narrow tiles fetch A twice as often. Stored [K, M] with M no multiple of 64, it has boxes that lie partly
+// outside, which take longer: 600 x 4096 x 14336 86 and 101, 648 x 3584 x 8192 52 and 52 to 54, 704 x 3584 x 18944 102 and 79.
+static bool narrow_tiles(int M, int N, int K, bool a_mn, int pairs) {
   const int num_m = (M + G2_BM - 1) / G2_BM;
   const long long wide = (long long)num_m * ((N + 255) / 256), narrow = (long long)num_m * ((N + 127) / 128);
-  return wide <= pairs && 2 * wide > pairs && narrow > pairs && 3 * (narrow - pairs) <= pairs && K >= 64 * G2_BK;
+  return wide <= pairs && 2 * wide > pairs && narrow > pairs && 3 * (narrow - pairs) <= pairs && K >= 64 * G2_BK &&
+         !(a_mn && M % 64);
 }
 
 // The CTA pairs that the rules below reckon with: as many as run at once.
@@ -135,8 +138,8 @@ static int gemm_pairs(int num_sms) {
   return rc ? num_sms / 2 : np;
 }
 
-static int pair_tile_width(int M, int N, int K, bool cut, int num_sms) {
-  return N > 128 && !(cut && narrow_tiles(M, N, K, gemm_pairs(num_sms))) ? 256 : 128;
+static int pair_tile_width(int M, int N, int K, bool a_mn, bool cut, int num_sms) {
+  return N > 128 && !(cut && narrow_tiles(M, N, K, a_mn, gemm_pairs(num_sms))) ? 256 : 128;
 }
 
 template <bool A_MN, bool B_MN>
@@ -149,7 +152,7 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
     else
       return B200_ERR_ARG;
   }
-  if (pair_tile_width(M, N, K, cut, num_sms) == 256)
+  if (pair_tile_width(M, N, K, A_MN, cut, num_sms) == 256)
     return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut, ws_floats);
   return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut, ws_floats);
 }
@@ -158,19 +161,19 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
 // CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56), and the rows of C are
 // whole 16 bytes, which is what its stores write. A product that is added to bf16 values is rounded once, with the
 // sum, in the single-CTA kernel and where a tile is cut; the TMA adds of whole tiles would round it before, too.
-static bool pairs_for_few_rows(int M, int N, int K, int out_fp32, int accumulate, int num_sms) {
+static bool pairs_for_few_rows(int M, int N, int K, bool a_mn, int out_fp32, int accumulate, int num_sms) {
   if (M > 128 || (N + 255) / 256 > gemm_pairs(num_sms) || ((N * (out_fp32 ? 4 : 2)) & 15)) return false;
   if (out_fp32 || !accumulate) return true;
-  const int bn = pair_tile_width(M, N, K, true, num_sms), tiles = (N + bn - 1) / bn;
+  const int bn = pair_tile_width(M, N, K, a_mn, true, num_sms), tiles = (N + bn - 1) / bn;
   int splits = 0;
   return g2_rest(tiles, gemm_pairs(num_sms), (K + G2_BK - 1) / G2_BK, splits) == tiles;
 }
 
 // Whether a call takes the CTA-pair kernel. rows16: the rows of C start on 16-byte boundaries; without that there is none.
-static bool takes_pairs(bool rows16, int M, int N, int K, int out_fp32, int accumulate, bool bias, int epilogue, int path, bool cut,
-                        int num_sms) {
+static bool takes_pairs(bool rows16, int M, int N, int K, bool a_mn, int out_fp32, int accumulate, bool bias, int epilogue, int path,
+                        bool cut, int num_sms) {
   if (epilogue == G2_EPI_SWIGLU || bias || path == 2) return true;   // what only this kernel has
-  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, K, out_fp32, accumulate, num_sms)));
+  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, K, a_mn, out_fp32, accumulate, num_sms)));
 }
 
 }  // namespace b200
@@ -195,7 +198,7 @@ extern "C" int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, i
   if ((lda & 7) || (ldb & 7)) return B200_ERR_ARG;
   using namespace b200;
   const bool rows16 = !(reinterpret_cast<uintptr_t>(C) & 15) && !((ldc * (out_fp32 ? 4 : 2)) & 15);
-  if (takes_pairs(rows16, M, N, K, out_fp32, accumulate, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
+  if (takes_pairs(rows16, M, N, K, a_mn != 0, out_fp32, accumulate, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
     if (!rows16) return B200_ERR_ARG;
     if (epilogue == G2_EPI_SWIGLU && (a_mn || b_mn || (N & 1) || accumulate)) return B200_ERR_ARG;
     Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, nullptr, 0, {}};
@@ -223,12 +226,12 @@ extern "C" int b200_gemm_bf16_ex(const void* A, const void* B, void* C, int M, i
 }
 
 // Scratch that such a call with `cut` wants, in elements; 0: it is not cut. rows16: C and its row stride are multiples of 16 bytes.
-extern "C" long long b200_gemm_scratch(int M, int N, int K, int rows16, int out_fp32, int accumulate, int bias, int epilogue,
+extern "C" long long b200_gemm_scratch(int M, int N, int K, int a_mn, int rows16, int out_fp32, int accumulate, int bias, int epilogue,
                                        int path, int num_sms) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2 || epilogue == G2_EPI_SWIGLU || !rows16) return 0;
-  if (!takes_pairs(true, M, N, K, out_fp32, accumulate, bias != 0, epilogue, path, true, num_sms)) return 0;
-  const int bn = pair_tile_width(M, N, K, true, num_sms);
+  if (!takes_pairs(true, M, N, K, a_mn != 0, out_fp32, accumulate, bias != 0, epilogue, path, true, num_sms)) return 0;
+  const int bn = pair_tile_width(M, N, K, a_mn != 0, true, num_sms);
   int splits = 0;
   const int rest = g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), gemm_pairs(num_sms),
                            (K + G2_BK - 1) / G2_BK, splits);

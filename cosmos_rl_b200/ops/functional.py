@@ -260,9 +260,9 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_scratch(M: int, N: int, K: int, rows16: bool, out_fp32: bool, accumulate: bool, bias: bool, swiglu: bool, path: int,
-                  sms: int) -> int:
-    return native.lib().b200_gemm_scratch(M, N, K, rows16, out_fp32, accumulate, bias, swiglu, path, sms)
+def _gemm_scratch(M: int, N: int, K: int, a_mn: bool, rows16: bool, out_fp32: bool, accumulate: bool, bias: bool, swiglu: bool,
+                  path: int, sms: int) -> int:
+    return native.lib().b200_gemm_scratch(M, N, K, a_mn, rows16, out_fp32, accumulate, bias, swiglu, path, sms)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = False,
@@ -286,7 +286,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = Fals
     dev = a.device.index if a.device.index is not None else torch.cuda.current_device()
     sms, out_fp32 = native.num_sms(dev), out.dtype == torch.float32
     rows16 = (out.data_ptr() | out.stride(0) * out.element_size()) % 16 == 0
-    floats, ws = _gemm_scratch(M, N, K, rows16, out_fp32, accumulate, bias is not None, swiglu, path, sms), None
+    floats, ws = _gemm_scratch(M, N, K, a_mn, rows16, out_fp32, accumulate, bias is not None, swiglu, path, sms), None
 
     def call(cut):
         return native.lib().b200_gemm_bf16_ws(

@@ -57,7 +57,7 @@ _SIGS = {
     "b200_gemm_bf16_ws": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                           c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong,
                           c_void_p, c_int, c_void_p],
-    "b200_gemm_scratch": [c_int] * 10,
+    "b200_gemm_scratch": [c_int] * 11,
     "b200_gemm_skinny_splits": [c_int, c_int, c_int, c_int, c_int],
     "b200_gemm_skinny": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                          c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],

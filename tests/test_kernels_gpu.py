@@ -603,10 +603,11 @@ def test_grouped_wgrad_forms(E, N, K, rows, out_dtype, accumulate):
 
 @pytest.mark.gpu
 # (rows, columns, contraction): one tile and few rows; ragged everything; tiles of 128 columns because there are no more of them;
-# tiles of 128 columns, of which ten are left for a second round; 256 columns and a second round; two shares of uneven length;
+# tiles of 128 columns, of which ten are left for a second round (not where A is stored transposed with rows that fill no box, as
+# the first of the two has them); 256 columns and a second round; two shares of uneven length;
 # columns that end inside 16 bytes; a contraction too short to be cut
 @pytest.mark.parametrize("M,N,K", [(3, 256, 4096), (127, 1032, 4200), (129, 520, 8200), (300, 104, 4096), (700, 3584, 4104),
-                                   (1300, 3840, 4104), (900, 2304, 4160), (300, 1001, 4096), (256, 512, 512)])
+                                   (704, 3584, 4104), (1300, 3840, 4104), (900, 2304, 4160), (300, 1001, 4096), (256, 512, 512)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
 @pytest.mark.parametrize("out_dtype,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True),
                                                   (torch.float32, True)])
@@ -615,10 +616,11 @@ def test_gemm_cut_last_round(M, N, K, a_mn, b_mn, out_dtype, accumulate):
     a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, K, device="cuda").to(torch.bfloat16)
     bv = None if accumulate else torch.randn(N, device="cuda").to(torch.bfloat16)
     sms, few = native.num_sms(0), M <= 128
-    width = 128 if N <= 128 or (M, N) == (700, 3584) else 256
+    width = 128 if N <= 128 or (N == 3584 and not (a_mn and M % 64)) else 256
     left = -(-M // 256) * -(-N // width) % (sms // 2)
-    scratch = F._gemm_scratch(M, N, K, True, out_dtype == torch.float32, accumulate, bv is not None, False, 0, sms)
-    assert scratch == (0 if K == 512 else left * min(sms // 2 // left, 8) * 256 * width)
+    scratch = F._gemm_scratch(M, N, K, a_mn, True, out_dtype == torch.float32, accumulate, bv is not None, False, 0, sms)
+    shares = min(sms // 2 // left, 8)
+    assert scratch == (0 if K == 512 or shares < 2 else left * shares * 256 * width)
 
     def stored(t):          # [K, rows], rows of whole 16 bytes
         buf = torch.zeros(K, (t.shape[0] + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")
@@ -1694,7 +1696,7 @@ def test_gemm_cut_tiles_added_from_two_streams(dtype, M, N):
     a, b = ((torch.rand(n, K, device=DEV) < 1 / 64).to(torch.bfloat16) for n in (M, N))
     want = a.float() @ b.float().t()
     assert want.max() * 2 * times <= 256
-    assert F._gemm_scratch(M, N, K, True, dtype == torch.float32, True, False, False, 0, native.num_sms(0)) > 0
+    assert F._gemm_scratch(M, N, K, False, True, dtype == torch.float32, True, False, False, 0, native.num_sms(0)) > 0
     out = torch.zeros(M, N, dtype=dtype, device=DEV)
     streams = [torch.cuda.Stream() for _ in range(2)]
     torch.cuda.synchronize()
