@@ -14,7 +14,8 @@
 // they are listed by the length of their sequence, the longest first, and dealt out forwards and backwards in turn: an SM
 // that gets the longest of one round gets the shortest of the next. 128 sequences of 384 to 1536 tokens, 4 kv heads: the
 // busiest SM has 31.6 pages' work instead of 42.6 in the order of the sequences, the mean is 28.5: 61
-// and 65 us; 64 sequences of 1000 to 4000 tokens, 8 kv heads: 120 and 133.
+// and 65 us; 64 sequences of 1000 to 4000 tokens, 8 kv heads: 120 and 133. Short sequences and those of like length gain nothing and
+// are left as they come: 208 of 198 tokens, 1 kv head 9.2 us, 15.5 when everything was sorted; 237 of 232, 4 kv heads 26.5 and 33.3.
 //   warp 0   : TMA producer (Q tile per item, K / V^T slabs per page through a 3-stage ring)
 //   warp 1   : MMA issuer (one thread), owns the TMEM allocation (S^T: 16 columns, O^T: 16 columns)
 //   warps 2-5: softmax. Thread <-> TMEM lane: a token row of S^T, a head-dim row of O^T. Column (head)
@@ -43,6 +44,7 @@ constexpr int PDT_P_BYTES = 2 * PDT_N * 64 * 2;             // two 16 x 64-token
 constexpr int PDT_SMEM = PDT_STAGES * PDT_STAGE_BYTES + 2 * PDT_Q_BYTES + 2 * PDT_P_BYTES + 2048 /*barriers, reductions, order*/ + 1024;
 constexpr int PDT_THREADS = 192;
 constexpr int PDT_SORT_MAX = 256;  // sequences that are sorted: each CTA compares all of them with each other
+constexpr int PDT_UNEVEN = 3;      // they are if an item of one has so many pages more or less than one of the first sequence
 constexpr float PDT_LOG2E = 1.4426950408889634f;
 
 struct PdtParams {
@@ -114,8 +116,8 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_ready + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* red = reinterpret_cast<float*>(bars + 24);      // [2 buffers][4 warps][8 heads], 16-byte aligned
-  uint16_t* pages_sh = reinterpret_cast<uint16_t*>(red + 64);   // [PDT_SORT_MAX] pages of each sequence
-  uint8_t* order = reinterpret_cast<uint8_t*>(pages_sh + PDT_SORT_MAX);   // [PDT_SORT_MAX] sequences by length
+  uint32_t* keys = reinterpret_cast<uint32_t*>(red + 64);             // [PDT_SORT_MAX], 16-byte aligned
+  uint8_t* order = reinterpret_cast<uint8_t*>(keys + PDT_SORT_MAX);   // [PDT_SORT_MAX] sequences by length
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = p.hq / p.hkv;
@@ -154,26 +156,31 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   const uint32_t tmem_o = tmem_base + 32;   // S^T: columns [0,16) and [16,32) (even / odd tile); O^T: [32,48)
   pdl_wait();  // the set-up above is CTA-local; queries, cache pages and lengths are global memory
 
-  const bool sorted = n_items > (int)gridDim.x && p.B <= PDT_SORT_MAX;
-  if (sorted) {
-    for (int b = threadIdx.x; b < PDT_SORT_MAX; b += PDT_THREADS) {
-      int pages = 0;
-      if (b < p.B) pages = (p.seq_lens[b] + PDT_PAGE - 1) / PDT_PAGE - (p.prefix_pages ? p.prefix_pages[b] : 0);
-      pages_sh[b] = (uint16_t)min(max(pages, 0), 65535);
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < p.B; b += PDT_THREADS) {
-      const int mine = pages_sh[b];
-      int rank = 0;
+  bool sorted = n_items > (int)gridDim.x && p.B <= PDT_SORT_MAX && p.max_pages >= PDT_UNEVEN * p.nsplit;
+  if (sorted) {   // every warp finds out by itself: a barrier takes longer
+    auto pages_of = [&](int b) { return max((p.seq_lens[b] + PDT_PAGE - 1) / PDT_PAGE - (p.prefix_pages ? p.prefix_pages[b] : 0), 0); };
+    const int first = pages_of(0);
+    bool uneven = false;
+#pragma unroll
+    for (int b = lane; b < PDT_SORT_MAX; b += 32)
+      if (b < p.B) uneven |= abs(pages_of(b) - first) >= PDT_UNEVEN * p.nsplit;
+    sorted = __any_sync(0xffffffffu, uneven);
+    if (sorted) {   // one key a sequence: pages, and among equals the earlier sequence first; there is nothing past the last
+      for (int b = threadIdx.x; b < PDT_SORT_MAX; b += PDT_THREADS)
+        keys[b] = b < p.B ? ((uint32_t)min(pages_of(b), 0xffffff) << 8) + (PDT_SORT_MAX - 1 - b) : 0u;
+      __syncthreads();
+      for (int b = threadIdx.x; b < p.B; b += PDT_THREADS) {
+        const uint32_t mine = keys[b];
+        int rank = 0;
 #pragma unroll 4
-      for (int o = 0; o < p.B; o += 4) {   // past the end there is nothing longer
-        const ushort4 x = *reinterpret_cast<const ushort4*>(pages_sh + o);
-        rank += (x.x > mine || (x.x == mine && o < b)) + (x.y > mine || (x.y == mine && o + 1 < b)) +
-                (x.z > mine || (x.z == mine && o + 2 < b)) + (x.w > mine || (x.w == mine && o + 3 < b));
+        for (int o = 0; o < p.B; o += 4) {
+          const uint4 x = *reinterpret_cast<const uint4*>(keys + o);
+          rank += (x.x > mine) + (x.y > mine) + (x.z > mine) + (x.w > mine);
+        }
+        order[rank] = (uint8_t)b;
       }
-      order[rank] = (uint8_t)b;
+      __syncthreads();
     }
-    __syncthreads();
   }
   // the k-th item of this CTA; rises with k
   auto nth = [&](int k) -> int {

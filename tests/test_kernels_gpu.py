@@ -1756,3 +1756,19 @@ def test_skinny_leaves_the_values_beside_its_result(M, N, K):
     # one rounding to bf16 and fp32 sums of K products
     bound = 2.0 ** -8 * ref.abs() + 2.0 ** -20 * x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=1) + 1e-5
     assert ((buf[:M, :N].double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,hq,hkv,length", [(256, 7, 1, 130), (40, 32, 8, 600), (80, 4, 2, 1)])
+def test_paged_decode_many_equal_sequences(B, hq, hkv, length):
+    """More items than SMs and nothing to sort: the items come in the order of the sequences."""
+    torch.manual_seed(89)
+    per = (length + 127) // 128
+    table = torch.randperm(B * per).int().view(B, per)
+    cache, q = _bf16(B * per, 2, hkv, 128, 128), _bf16(B, hq, 128)
+    lens = torch.full((B,), length, dtype=torch.int32)
+    out = F.paged_decode(q, cache, table.cuda(), lens.cuda(), v_transposed=True)
+    native.read_status(q.device)
+    ref = R.paged_decode(q.cpu(), cache.cpu(), table, lens, v_transposed=True)
+    # probabilities and the result are rounded to bf16 (2^-9 each)
+    assert (out.cpu().float() - ref.float()).norm() <= 2.0 ** -7 * ref.float().norm()
+    assert (out.cpu().float() - ref.float()).abs().max() <= 2.0 ** -6 * ref.float().abs().max()
