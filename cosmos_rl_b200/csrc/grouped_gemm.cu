@@ -213,6 +213,30 @@ static int set_smem(Kern k, bool& done) {
   return 0;
 }
 
+// CTA pairs of a call of expert weight gradients, 0: single CTAs, or an error code. Single CTAs are bound by operands out of L2 (4.9
+// blocks of 48 KB for 64 KB of result, 4096 tokens on 128 experts), and a pair on a 256 x 256 tile fetches two thirds of that. us,
+// single CTAs and pairs, 1536 x 2048 a gradient: 256 rows for each of 128 experts 290 and 260, 512 rows 465 and 400, 2048 rows for
+// each of 16 165 and 143; few rows are bound by the epilogue, of which a pair has the less: 44 rows 190 and 216, 6 rows 166 and
+// 191. max_rows is what there is room for, up to 128 rows an expert more than there are. What the larger tiles waste at the edges
+// and in the last round counts against them: with a fifth more rounds than single CTAs have they are still no slower (58 experts of
+// 640 x 1144 58.1 and 58.3), with more they are (101 of 360 x 688, 1334 rows, 104 and 118; 8 of 1112 x 352, two rounds for one, 9.8
+// and 13.1). A result in fp32 that is added to is bound by its way through memory up to twice as many rows (92 of 504 x 4064, 537
+// rows, 356 and 418). A bf16 result that is added to keeps its one rounding in the other kernel.
+using WG_SMEM = Gemm2Smem<256, 6>;
+static int wgrad_pairs(int max_rows, int N, int K, int num_experts, int out_fp32, int accumulate, int num_sms) {
+  if ((accumulate && !out_fp32) || num_sms < 2 || max_rows < (accumulate ? 640ll : 320ll) * num_experts) return 0;
+  static int whole[16] = {0};
+  int np = 0;
+  if (const int rc = resident_pairs(gemm2_bf16_kernel<256, 6, true, true, G2_EPI_EXPERTS>, whole, WG_SMEM::TOTAL, G2_THREADS,
+                                    num_sms, np))
+    return rc;
+  auto tiles = [&](int rows) { return (long long)num_experts * ((N + rows - 1) / rows) * ((K + 255) / 256); };
+  auto rounds = [](long long n, int at_once) { return (n + at_once - 1) / at_once; };
+  const long long pair_tiles = tiles(G2_BM);
+  if (pair_tiles < np || pair_tiles >= (1ll << 31)) return 0;
+  return 5 * rounds(pair_tiles, np) <= 6 * rounds(tiles(GEMM_BM), num_sms) ? np : 0;
+}
+
 }  // namespace b200
 
 extern "C" {
@@ -245,6 +269,11 @@ int b200_grouped_gemm(const void* X, const void* W, void* Y, int max_rows, int N
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 
+// Whether such a call of expert weight gradients takes CTA pairs.
+int b200_grouped_wgrad_pairs(int max_rows, int N, int K, int num_experts, int out_fp32, int accumulate, int num_sms) {
+  return b200::wgrad_pairs(max_rows, N, K, num_experts, out_fp32, accumulate, num_sms) > 0;
+}
+
 // dW[e][N, K] (+)= dY[rows of e, N]^T . X[rows of e, K]; rows of e = [expert_offsets[e], expert_offsets[e+1])
 int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, int N, int K, int num_experts,
                        long long lddy, long long ldx, const int* expert_offsets, int out_fp32, int accumulate,
@@ -255,29 +284,18 @@ int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, in
   if (make_tmap_grouped_out(&tmC, dW, num_experts, N, K, K, (uint64_t)N * K, out_fp32)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmA, dY, max_rows, N, lddy, 64, 64, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmB, X, max_rows, K, ldx, 64, 64, 2)) return B200_ERR_TENSORMAP;
-  // CTA pairs on 256 x 256 tiles once every pair has one: the single CTAs are bound by operands out of L2 (4.9 blocks of 48 KB
-  // for 64 KB of result, 4096 tokens on 128 experts), and a pair fetches two thirds of that. us, single CTAs and pairs, 1536 x
-  // 2048 a gradient: 256 rows for each of 128 experts 290 and 260, 512 rows 465 and 400, 2048 rows for each of 16 165 and 143;
-  // few rows are bound by the epilogue, of which a pair has the less: 44 rows 190 and 216, 6 rows 166 and 191. max_rows is what
-  // there is room for, up to 128 rows an expert more than there are. A bf16 result that is added to keeps its one rounding in
-  // the other kernel.
-  const long long pair_tiles = (long long)num_experts * ((N + G2_BM - 1) / G2_BM) * ((K + 255) / 256);
-  if (!(accumulate && !out_fp32) && num_sms >= 2 && pair_tiles < (1ll << 31) && max_rows >= 320ll * num_experts) {
-    auto kern = gemm2_bf16_kernel<256, 6, true, true, G2_EPI_EXPERTS>;
-    using SM = Gemm2Smem<256, 6>;
-    static int whole[16] = {0};
-    int np = 0;
-    if (const int rc = resident_pairs(kern, whole, SM::TOTAL, G2_THREADS, num_sms, np)) return rc;
-    if (pair_tiles >= np) {
-      Gemm2Params ep2{};
-      ep2.out_fp32 = out_fp32;
-      ep2.accumulate = accumulate;
-      ep2.a_bytes = SM::A_BYTES;
-      ep2.offsets = expert_offsets;
-      ep2.experts = num_experts;
-      kern<<<2 * np, G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmC, tmC, N, K, 0, ep2, status);
-      return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
-    }
+  const int np = wgrad_pairs(max_rows, N, K, num_experts, out_fp32, accumulate, num_sms);
+  if (np < 0) return np;
+  if (np > 0) {
+    Gemm2Params ep2{};
+    ep2.out_fp32 = out_fp32;
+    ep2.accumulate = accumulate;
+    ep2.a_bytes = WG_SMEM::A_BYTES;
+    ep2.offsets = expert_offsets;
+    ep2.experts = num_experts;
+    gemm2_bf16_kernel<256, 6, true, true, G2_EPI_EXPERTS><<<2 * np, G2_THREADS, WG_SMEM::TOTAL, stream>>>(
+        tmA, tmB, tmC, tmC, N, K, 0, ep2, status);
+    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
   }
   static bool s2 = false;
   if (set_smem(grouped_wgrad_kernel, s2)) return B200_ERR_LAUNCH;

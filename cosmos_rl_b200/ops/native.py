@@ -119,6 +119,7 @@ _SIGS = {
     "b200_moe_combine_dprob": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "b200_grouped_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p,
                           c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
+    "b200_grouped_wgrad_pairs": [c_int] * 7,
     "b200_grouped_wgrad": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong,
                            c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_quant_mxfp4": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],

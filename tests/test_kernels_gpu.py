@@ -575,12 +575,16 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
-# ragged result rows and columns; experts without rows; fp32 sums; too few rows for CTA pairs
-@pytest.mark.parametrize("E,N,K,rows", [(10, 1032, 520, [128, 0, 640, 384, 0, 256, 1024, 128, 512, 768]),
-                                        (6, 1536, 768, [512] * 6), (40, 256, 520, [128] * 40)])
+# ragged result rows and columns; experts without rows; fp32 sums; too few rows for CTA pairs; a round more than single CTAs have
+@pytest.mark.parametrize("E,N,K,rows,pairs", [(10, 1000, 520, [256, 0, 1280, 768, 0, 512, 2048, 256, 1024, 1536], True),
+                                              (6, 1536, 768, [768] * 6, True), (40, 256, 520, [128] * 40, False),
+                                              (10, 1032, 520, [256, 0, 1280, 768, 0, 512, 2048, 256, 1024, 1536], False)])
 @pytest.mark.parametrize("out_dtype,accumulate", [(torch.bfloat16, False), (torch.bfloat16, True), (torch.float32, True)])
-def test_grouped_wgrad_forms(E, N, K, rows, out_dtype, accumulate):
+def test_grouped_wgrad_forms(E, N, K, rows, pairs, out_dtype, accumulate):
     torch.manual_seed(E)
+    fp32 = out_dtype == torch.float32
+    assert native.lib().b200_grouped_wgrad_pairs(sum(rows), N, K, E, int(fp32), int(accumulate), native.num_sms(0)) == \
+        (pairs and (fp32 or not accumulate))
     off = torch.tensor([0] + rows, device="cuda").cumsum(0).to(torch.int32)
     Mp = int(off[-1])
     dy, x = torch.randn(Mp, N, device="cuda").to(torch.bfloat16), torch.randn(Mp, K, device="cuda").to(torch.bfloat16)
