@@ -178,7 +178,8 @@ struct G2ExpertWork {
   }
 };
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
+// TAIL: the rows of C end inside 16 bytes (a test in the epilogue of all kernels took 0.6 us of 33 x 3832 x 712 in fp32, 9.9).
+template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool TAIL>
 __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmC,
                                                const CUtensorMap* tmW, int M, int N, int K, const Gemm2Params& ep,
                                                uint32_t* status) {
@@ -427,7 +428,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         __syncwarp();
         const int gc = col_base + c;
         if (elect_one()) {
-          if (gc < (cut ? n_cols : whole16(n_cols, ep.out_fp32)) && row0 < M) {
+          if (gc < (TAIL && !cut ? whole16(n_cols, ep.out_fp32) : n_cols) && row0 < M) {
             if constexpr (EPI == G2_EPI_EXPERTS) {
               if (ep.accumulate) tma_reduce_add_3d(tmC, slab, gc, row0, unit.batch);
               else tma_store_3d(tmC, slab, gc, row0, unit.batch);
@@ -437,7 +438,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
           }
           tma_store_commit();
         }
-        if constexpr (EPI != G2_EPI_EXPERTS) {
+        if constexpr (TAIL) {
           const long long at = (long long)(row0 + lane) * ep.ldc;
           if (!cut && row0 + lane < M) {
             if (ep.out_fp32) store_tail((float*)ep.C + at, slab, gc, n_cols, ep.accumulate);

@@ -5,17 +5,18 @@
 
 namespace b200 {
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
+template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool TAIL = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, int M, int N, int K,
                   Gemm2Params ep, uint32_t* status) {
-  gemm2_mainloop<BN, STAGES, A_MN, B_MN, EPI>(&tmA, &tmB, &tmC, &tmW, M, N, K, ep, status);
+  gemm2_mainloop<BN, STAGES, A_MN, B_MN, EPI, TAIL>(&tmA, &tmB, &tmC, &tmW, M, N, K, ep, status);
 }
 
 // C of the cut tiles: the sum of their shares (+ bias) (+ C). A warp has one row of a tile, a lane eight columns; rows of C
 // start on 16-byte boundaries. Above 128 rows the sum is added to C in memory, like the tiles that are not cut: whatever else
-// adds to C at that time, no value is lost. Fewer rows are all cut, or added by the single-CTA kernel, and read C and write it.
+// adds to C at that time, no value is lost. Fewer rows, all of whose tiles come this way, read C and write it like the single-CTA
+// kernel, and round once.
 // Grid (rest, 256 / 8).
 template <int BN>
 __global__ void __launch_bounds__(256)
@@ -153,24 +154,38 @@ inline int g2_rest(long long tiles, int pairs, int num_kb, int& splits) {
   return rest;
 }
 
+// The same, but with `all` every tile, in one share if there is nothing to cut: sums that are to be rounded once pass through the
+// kernel that adds the shares. All tiles run at once then.
+inline int g2_shared_tiles(long long tiles, int pairs, int num_kb, bool all, int& splits) {
+  const int rest = g2_rest(tiles, pairs, num_kb, splits);
+  if (!all || rest == tiles) return rest;
+  splits = 1;
+  return (int)tiles;
+}
+
+// Few rows that are added to bf16 values: the single-CTA kernel rounds the sum only, TMA adds round the product before it as well.
+inline bool g2_round_once(int M, int out_fp32, int accumulate) { return M <= G2_BM_CTA && accumulate && !out_fp32; }
+
 // Scratch of a launch that cuts `rest` tiles (Gemm2Params::ws), in elements.
 constexpr long long g2_ws_floats(int rest, int splits, int bn) { return (long long)rest * splits * G2_BM * bn; }
 
 // allow_cut: a launch that would gain from a workspace and has too little (ep.ws, ws_floats) returns B200_NEED_WORKSPACE
-template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
-static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                        long long ldc, Gemm2Params ep, uint32_t* status, int num_sms, cudaStream_t stream,
-                        bool allow_cut = false, long long ws_floats = 0) {
+template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool TAIL>
+static int launch_gemm2_form(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                             long long ldc, Gemm2Params ep, uint32_t* status, int num_sms, cudaStream_t stream,
+                             bool allow_cut, long long ws_floats) {
   CUtensorMap tmA, tmB, tmC, tmW;
   const int n_cols = EPI == G2_EPI_SWIGLU ? N / 2 : N;
   using SM = Gemm2Smem<BN, STAGES>;
-  auto kern = gemm2_bf16_kernel<BN, STAGES, A_MN, B_MN, EPI>;
+  auto kern = gemm2_bf16_kernel<BN, STAGES, A_MN, B_MN, EPI, TAIL>;
   static int whole[16] = {0};
   int np = 0;
   if (const int rc = resident_pairs(kern, whole, SM::TOTAL, G2_THREADS, num_sms, np)) return rc;
   constexpr int OUT_BN = EPI == G2_EPI_SWIGLU ? BN / 2 : BN;
   const int tiles = ((M + G2_BM - 1) / G2_BM) * ((n_cols + OUT_BN - 1) / OUT_BN);
-  ep.rest = EPI == G2_EPI_STORE && allow_cut ? g2_rest(tiles, np, (K + G2_BK - 1) / G2_BK, ep.splits) : (ep.splits = 0);
+  const bool all = g2_round_once(M, ep.out_fp32, ep.accumulate) && tiles <= np;
+  ep.rest = EPI == G2_EPI_STORE && allow_cut ? g2_shared_tiles(tiles, np, (K + G2_BK - 1) / G2_BK, all, ep.splits)
+                                             : (ep.splits = 0);
   if (ep.rest > 0 && (ep.ws == nullptr || ws_floats < g2_ws_floats(ep.rest, ep.splits, BN))) return B200_NEED_WORKSPACE;
   const int a_rows = !A_MN && M < G2_BM_CTA ? M : G2_BM_CTA;
   ep.a_bytes = a_rows * G2_BK * 2;
@@ -192,6 +207,16 @@ static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int
                                   (const float*)ep.ws, C, ldc, M, N, ep) != cudaSuccess)
       return B200_ERR_LAUNCH;
   return 0;
+}
+
+template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI>
+static int launch_gemm2(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                        long long ldc, const Gemm2Params& ep, uint32_t* status, int num_sms, cudaStream_t stream,
+                        bool allow_cut = false, long long ws_floats = 0) {
+  const int n_cols = EPI == G2_EPI_SWIGLU ? N / 2 : N;
+  auto launch = whole16(n_cols, ep.out_fp32) == n_cols ? launch_gemm2_form<BN, STAGES, A_MN, B_MN, EPI, false>
+                                                       : launch_gemm2_form<BN, STAGES, A_MN, B_MN, EPI, true>;
+  return launch(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, allow_cut, ws_floats);
 }
 
 }  // namespace b200

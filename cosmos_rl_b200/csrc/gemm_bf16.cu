@@ -138,8 +138,8 @@ static int gemm_pairs(int num_sms) {
   return rc ? num_sms / 2 : np;
 }
 
-static int pair_tile_width(int M, int N, int K, bool a_mn, bool cut, int num_sms) {
-  return N > 128 && !(cut && narrow_tiles(M, N, K, a_mn, gemm_pairs(num_sms))) ? 256 : 128;
+static int pair_tile_width(int M, int N, int K, bool a_mn, int out_fp32, int accumulate, bool cut, int num_sms) {
+  return N > 128 && (g2_round_once(M, out_fp32, accumulate) || !(cut && narrow_tiles(M, N, K, a_mn, gemm_pairs(num_sms)))) ? 256 : 128;
 }
 
 template <bool A_MN, bool B_MN>
@@ -152,29 +152,27 @@ static int dispatch_gemm2(const void* A, const void* B, void* C, int M, int N, i
     else
       return B200_ERR_ARG;
   }
-  if (pair_tile_width(M, N, K, A_MN, cut, num_sms) == 256)
+  if (pair_tile_width(M, N, K, A_MN, ep.out_fp32, ep.accumulate, cut, num_sms) == 256)
     return launch_gemm2<256, 6, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut, ws_floats);
   return launch_gemm2<128, 8, A_MN, B_MN, G2_EPI_STORE>(A, B, C, M, N, K, lda, ldb, ldc, ep, status, num_sms, stream, cut, ws_floats);
 }
 
 // Up to 128 rows the pair kernel is the faster one when all its tiles run at once, with or without a cut (100 rows, us, single
 // CTAs and pairs: 4096 x 28672 165 and 51, 14336 x 4096 36 and 29; 28672 x 4096, 112 tiles, 51 and 56), and the rows of C are
-// whole 16 bytes, which is what its stores write. A product that is added to bf16 values is rounded once, with the
-// sum, in the single-CTA kernel and where a tile is cut; the TMA adds of whole tiles would round it before, too. A pair's only tile
-// that is not cut has twice the columns to write of a single CTA's (7 x 184 x 960 11.0 us and 9.1).
-static bool pairs_for_few_rows(int M, int N, int K, bool a_mn, int out_fp32, int accumulate, int num_sms) {
+// whole 16 bytes, which is what its stores write. With 129 to 255 columns a pair has one tile of 256 where single CTAs have two of
+// 128, and unless it is cut its results take longer to write (7 x 184 x 960 11.0 us and 9.1; 8 x 112 x 1280 7.8 and 9.4).
+static bool pairs_for_few_rows(int M, int N, int K, int out_fp32, int num_sms) {
   if (M > 128 || (N + 255) / 256 > gemm_pairs(num_sms) || ((N * (out_fp32 ? 4 : 2)) & 15)) return false;
-  const int bn = pair_tile_width(M, N, K, a_mn, true, num_sms), tiles = (N + bn - 1) / bn;
+  if (N <= 128 || N >= 256) return true;
   int splits = 0;
-  if (g2_rest(tiles, gemm_pairs(num_sms), (K + G2_BK - 1) / G2_BK, splits) == tiles) return true;
-  return N >= 256 && (out_fp32 || !accumulate);
+  return g2_rest(1, gemm_pairs(num_sms), (K + G2_BK - 1) / G2_BK, splits) > 0;
 }
 
 // Whether a call takes the CTA-pair kernel. rows16: the rows of C start on 16-byte boundaries; without that there is none.
-static bool takes_pairs(bool rows16, int M, int N, int K, bool a_mn, int out_fp32, int accumulate, bool bias, int epilogue, int path,
+static bool takes_pairs(bool rows16, int M, int N, int K, int out_fp32, bool bias, int epilogue, int path,
                         bool cut, int num_sms) {
   if (epilogue == G2_EPI_SWIGLU || bias || path == 2) return true;   // what only this kernel has
-  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, K, a_mn, out_fp32, accumulate, num_sms)));
+  return path != 1 && rows16 && (M > 128 || (cut && pairs_for_few_rows(M, N, K, out_fp32, num_sms)));
 }
 
 }  // namespace b200
@@ -199,7 +197,7 @@ extern "C" int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, i
   if ((lda & 7) || (ldb & 7)) return B200_ERR_ARG;
   using namespace b200;
   const bool rows16 = !(reinterpret_cast<uintptr_t>(C) & 15) && !((ldc * (out_fp32 ? 4 : 2)) & 15);
-  if (takes_pairs(rows16, M, N, K, a_mn != 0, out_fp32, accumulate, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
+  if (takes_pairs(rows16, M, N, K, out_fp32, bias != nullptr, epilogue, path, cut != 0, num_sms)) {
     if (!rows16) return B200_ERR_ARG;
     if (epilogue == G2_EPI_SWIGLU && (a_mn || b_mn || (N & 1) || accumulate)) return B200_ERR_ARG;
     Gemm2Params ep{bias, bias_bf16, out_fp32, accumulate, up_row0, 8, 0, 0, 0, ws, nullptr, 0, {}};
@@ -231,11 +229,13 @@ extern "C" long long b200_gemm_scratch(int M, int N, int K, int a_mn, int rows16
                                        int path, int num_sms) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || num_sms < 2 || epilogue == G2_EPI_SWIGLU || !rows16) return 0;
-  if (!takes_pairs(true, M, N, K, a_mn != 0, out_fp32, accumulate, bias != 0, epilogue, path, true, num_sms)) return 0;
-  const int bn = pair_tile_width(M, N, K, a_mn != 0, true, num_sms);
+  if (!takes_pairs(true, M, N, K, out_fp32, bias != 0, epilogue, path, true, num_sms)) return 0;
+  const int bn = pair_tile_width(M, N, K, a_mn != 0, out_fp32, accumulate, true, num_sms);
+  const int pairs = gemm_pairs(num_sms);
+  const long long tiles = (long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn);
   int splits = 0;
-  const int rest = g2_rest((long long)((M + G2_BM - 1) / G2_BM) * ((N + bn - 1) / bn), gemm_pairs(num_sms),
-                           (K + G2_BK - 1) / G2_BK, splits);
+  const int rest = g2_shared_tiles(tiles, pairs, (K + G2_BK - 1) / G2_BK, g2_round_once(M, out_fp32, accumulate) && tiles <= pairs,
+                                   splits);
   return g2_ws_floats(rest, splits, bn);
 }
 

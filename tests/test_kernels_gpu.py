@@ -1678,7 +1678,9 @@ def test_gemm_scratch_is_what_the_call_uses(monkeypatch):
     check(buf[:, :N])
 
 
-@pytest.mark.parametrize("M,N,K", [(100, 4096, 512), (128, 520, 256), (77, 4096, 8192), (16, 104, 4096)])
+# all columns in one share, single CTAs (129 to 255 columns, not cut), several shares, tiles of 128 columns in several and in one
+@pytest.mark.parametrize("M,N,K", [(100, 4096, 512), (128, 520, 256), (7, 184, 504), (77, 4096, 8192), (16, 104, 4096),
+                                   (5, 72, 200)])
 def test_gemm_few_rows_added_to_bf16_are_rounded_once(M, N, K):
     """Sums of whole numbers, which fp32 holds exactly: what was there and the product make one bf16 value with one rounding."""
     torch.manual_seed(85)
