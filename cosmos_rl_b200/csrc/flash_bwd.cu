@@ -231,7 +231,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t tm_dp = tmem_base + 256, tm_dq = tmem_base + 384;
 
   if (warp == 0) {
-    // ---- scheduler and TMA producer (whole warp, lane 0 issues)
+    // ---- scheduler and TMA producer (the whole warp, one elected lane issues)
     FlashWork work;
     work.list.init(p.cu_q, p.B, FB_B, p.hq, p.levels_q, !p.causal);
     work.init(reinterpret_cast<uint4*>(bars + 32), bars + 23);
@@ -594,7 +594,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   bool ok = true;
   if (warp == 0) {
-    // the whole warp: lane 0 issues the tile loads, all lanes fetch the 128 rows' lse and delta with plain loads
+    // the whole warp: one elected lane issues the tile loads, all lanes fetch the 128 rows' lse and delta with plain loads
     // (their addresses have no 16-byte alignment, so they cannot be a bulk copy)
     for (int i = 0; i < n && !*abort_flag; ++i) {
       const int s = i & 1;

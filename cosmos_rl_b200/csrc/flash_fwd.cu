@@ -270,7 +270,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else {
     setmaxnreg_dec<88>();
     if (warp == 0) {
-      // ------------------------------------------------ scheduler and TMA producer (whole warp, lane 0 issues)
+      // ------------------------------------------------ scheduler and TMA producer (the whole warp, one elected lane issues)
       FlashWork work;
       work.list.init(p.cu_q, p.B, 2 * FA_B, p.hq, p.levels, !p.causal);
       work.init(reinterpret_cast<uint4*>(bars + 30), bars + 32);

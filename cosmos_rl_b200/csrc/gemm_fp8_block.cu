@@ -11,11 +11,13 @@
 //   one CTA, 128 x 128 tiles: four buffers, six 32 KB stages, two warps a TMEM lane quadrant with 64 columns each
 //   CTA pair, 256 x 256 tiles: half the operand bytes of a product from L2 and shared memory; each CTA has two buffers of
 //   its 128 rows x 256 columns, handed over by halves of 128 columns
-// What bounds them: cycles are few enough that the clock falls (4096 x 37888 x 3584: 830 000 cycles of either form, at 1.5 to
-// 1.7 GHz), and within them the hand-over of a buffer: release, wait, products, commit, wait, four loads, 1100 cycles for the
-// two k-blocks in flight (products: 1024). What counted, at this size: a form that waits for its scales, writes rows from
-// registers and issues from one thread 845 us; scales multiplied when they are used 667; results through TMA stores and two
-// issuers 613; loads in flight under the multiplications 539; CTA pairs 488 us, 2282 TFLOP/s.
+// What bounds them, 4096 x 37888 x 3584 on pairs: 32 tiles of 28 k-blocks a pair, 896 k-blocks of 512 cycles of products. In the
+// steady state the hand-over of a buffer (release, wait, products, commit, wait, four loads) takes 1100 cycles for the two
+// k-blocks in flight, 650 a k-block where it was traced, which is 490 000 to 580 000 of the 830 000 cycles of a call; where the
+// others go, between tiles or in waits for operands, has not been measured. The clock falls under such calls: ten of them after a
+// pause 506 us each, 590 us in a loop of a second. What counted, ten calls at a time: a form that waits for its scales, writes
+// rows from registers and issues from one thread 845 us; scales multiplied when they are used 667; results through TMA stores and
+// two issuers 613; loads in flight under the multiplications 539; CTA pairs 488 to 506 (2198 to 2282 TFLOP/s; 1885 in the loop).
 // Operands arrive by TMA (128-byte swizzle, a 128-byte row = 128 fp8 elements). Persistent CTAs, bounded waits.
 #include "gemm_core.cuh"
 #include "gemm_2cta_launch.cuh"
@@ -270,7 +272,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (elect_one()) tma_store_wait_read<0>();   // the store of the tile before has read the slab
       __syncwarp();
       f8_fill_slab(slab, acc);
-      if (row0 + lane < p.M) store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab, col0, p.N, false);
+      if ((p.N & 7) && row0 + lane < p.M) store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab, col0, p.N, false);
       fence_proxy_async_smem();
       __syncwarp();
       if (elect_one()) {
@@ -392,7 +394,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       __syncwarp();
       f8_fill_slab(slab, acc);
       f8_fill_slab(slab + 4096, acc + 32);
-      if (row0 + lane < p.M) {
+      if ((p.N & 7) && row0 + lane < p.M) {
         store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab, col0, p.N, false);
         store_tail(p.C + (long long)(row0 + lane) * p.ldc, slab + 4096, col0 + 64, p.N, false);
       }

@@ -273,7 +273,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = Fals
     ``a_mn``: ``a`` is stored ``[K, M]`` instead of ``[M, K]``; ``b_mn``: ``b`` is stored ``[K, N]`` instead of
     ``[N, K]``. ``bias [N]`` (bf16 or fp32) is added in the epilogue. ``swiglu``: ``b`` is a fused gate/up weight
     ``[2 I, K]`` and the result is ``silu(A Bg^T) * (A Bu^T)`` of shape ``[M, I]``. ``path``: 0 lets the library choose
-    between the CTA-pair kernel (256-row tiles over two SMs) and the single-CTA kernel, 1 / 2 force one of them."""
+    between the CTA-pair kernel (256-row tiles over two SMs) and the single-CTA kernel, 1 / 2 force one of them.
+
+    The same call gives the same bits again. Which values are summed in one go and which in shares depends on M, N, K and the
+    number of SMs, so a row may come out different in the last place in a call of another size. ``accumulate`` adds value by
+    value in memory above 128 rows; with fewer ``out`` is read and written, and nothing else may add to it meanwhile."""
     assert a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     assert a.stride(-1) == 1 and b.stride(-1) == 1 and a.dim() == 2 and b.dim() == 2
     K, M = (a.shape[0], a.shape[1]) if a_mn else (a.shape[1], a.shape[0])
