@@ -436,8 +436,8 @@ __global__ void rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __
 // first row_tiles[0] * 128 rows are in use. A thread of the forward works on ITEMS vectors of 8 columns whose loads are all in
 // flight before the first is used. The quotient is a division, as in the epilogues that form SwiGLU elsewhere: the same gate and
 // up values give the same bits there and here, which a product with the reciprocal (one rounding more, 8192 x 18944 in 153 us)
-// does not. A zero gate, as in padding rows, would send it through its path for special operands and is not divided:
-// 8192 x 18944 169 us, all zero too; divided 164 and 300. (One test for eight gates: 174 and 134.)
+// does not. Zero gates would send it through its path for special operands, so a thread that has nothing else (rows of padding)
+// does not divide: 8192 x 18944 165 us, all zero 135 (163 and 300 if it does).
 template <class Index, int ITEMS>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T, int I,
@@ -449,28 +449,31 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
     const Index idx = first + k * 256;
+    g[k] = make_uint4(0, 0, 0, 0);
     if (idx >= total) continue;
     const Index t = idx / nvec, v = idx - t * nvec;
     const uint4* row = reinterpret_cast<const uint4*>(gu + (long long)t * 2 * I);
     g[k] = row[v];
     u[k] = row[nvec + v];
   }
+  uint32_t any = 0;
 #pragma unroll
-  for (int k = 0; k < ITEMS; ++k) {
-    const Index idx = first + k * 256;
-    if (idx >= total) continue;
-    float a[8], b[8], o[8];
-    unpack8(g[k], a);
-    unpack8(u[k], b);
+  for (int k = 0; k < ITEMS; ++k) any |= g[k].x | g[k].y | g[k].z | g[k].w;
+  auto write = [&](auto silu) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float x = a[j] == 0.f ? 1.f : a[j];
-      asm("" : "+f"(x));   // or the compiler, which sees that the quotient is not used for a zero, divides the zero
-      const float silu = x / (1.f + __expf(-x));
-      o[j] = (a[j] == 0.f ? a[j] : silu) * b[j];
+    for (int k = 0; k < ITEMS; ++k) {
+      const Index idx = first + k * 256;
+      if (idx >= total) continue;
+      float a[8], b[8], o[8];
+      unpack8(g[k], a);
+      unpack8(u[k], b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = silu(a[j]) * b[j];
+      reinterpret_cast<uint4*>(out)[idx] = pack8(o);
     }
-    reinterpret_cast<uint4*>(out)[idx] = pack8(o);
-  }
+  };
+  if (any & 0x7fff7fffu) write([](float x) { return x / (1.f + __expf(-x)); });
+  else write([](float x) { return x; });
 }
 
 template <class Index>
