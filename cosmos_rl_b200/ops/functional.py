@@ -24,12 +24,11 @@ def _c(t: torch.Tensor) -> torch.Tensor:
     return t if t.is_contiguous() else t.contiguous()
 
 
-def _rows(t: torch.Tensor, columns: Optional[int] = None) -> torch.Tensor:
-    """Contiguous ``[rows, columns]`` (default: the last dimension). A tensor that is that already is not viewed again, which
-    costs a small call as much as its launch; one that cannot be raises."""
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous ``[rows, last dimension]``; a tensor that is that already is not viewed again, which costs a small call as
+    much as its launch."""
     t = _c(t)
-    columns = t.shape[-1] if columns is None else columns
-    return t if t.dim() == 2 and t.shape[1] == columns else t.view(-1, columns)
+    return t if t.dim() == 2 else t.view(-1, t.shape[-1])
 
 
 def needs_graph(*tensors: Optional[torch.Tensor]) -> bool:
@@ -98,8 +97,12 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual:
         if x.dtype != torch.bfloat16:
             raise TypeError("rms_norm on CUDA expects bf16 activations")
         if not needs_graph(x, weight, residual):
-            y, res_out = _rmsnorm_fwd(_rows(x), weight, eps,
-                                      _rows(residual, x.shape[-1]) if residual is not None else None, None)
+            x2 = _rows(x)
+            if residual is not None:
+                residual = _c(residual)
+                if residual.shape != x2.shape:
+                    residual = residual.view(-1, x2.shape[1])     # raises unless it has rows of this length
+            y, res_out = _rmsnorm_fwd(x2, weight, eps, residual, None)
             if x.dim() == 2:
                 return y, res_out
             return y.view(x.shape), res_out.view(x.shape) if res_out is not None else None
