@@ -160,14 +160,19 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_cache, const __gri
   if (sorted) {   // every warp finds out by itself: a barrier takes longer
     auto pages_of = [&](int b) { return max((p.seq_lens[b] + PDT_PAGE - 1) / PDT_PAGE - (p.prefix_pages ? p.prefix_pages[b] : 0), 0); };
     const int first = pages_of(0);
+    int pages[PDT_SORT_MAX / 32];
     bool uneven = false;
 #pragma unroll
-    for (int b = lane; b < PDT_SORT_MAX; b += 32)
-      if (b < p.B) uneven |= abs(pages_of(b) - first) >= PDT_UNEVEN * p.nsplit;
+    for (int i = 0; i < PDT_SORT_MAX / 32; ++i) {
+      pages[i] = 32 * i + lane < p.B ? pages_of(32 * i + lane) : -1;
+      uneven |= pages[i] >= 0 && abs(pages[i] - first) >= PDT_UNEVEN * p.nsplit;
+    }
     sorted = __any_sync(0xffffffffu, uneven);
     if (sorted) {   // one key a sequence: pages, and among equals the earlier sequence first; there is nothing past the last
-      for (int b = threadIdx.x; b < PDT_SORT_MAX; b += PDT_THREADS)
-        keys[b] = b < p.B ? ((uint32_t)min(pages_of(b), 0xffffff) << 8) + (PDT_SORT_MAX - 1 - b) : 0u;
+#pragma unroll
+      for (int i = 0; i < PDT_SORT_MAX / 32; ++i)
+        if (i % (PDT_THREADS / 32) == warp)
+          keys[32 * i + lane] = pages[i] < 0 ? 0u : ((uint32_t)min(pages[i], 0xffffff) << 8) + (PDT_SORT_MAX - 1 - 32 * i - lane);
       __syncthreads();
       for (int b = threadIdx.x; b < p.B; b += PDT_THREADS) {
         const uint32_t mine = keys[b];
