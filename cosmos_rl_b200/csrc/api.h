@@ -102,13 +102,17 @@ int b200_moe_permute(const void* x, const int* idx, const int* offsets, int* cur
                      int k, int H, cudaStream_t stream);
 // clears the rows of xp between an expert's last filled row (filled: rows claimed by the permutation, its cursor) and the
 // next expert's first; none at or past max_rows
-int b200_moe_zero_padding(const int* filled, const int* offsets, void* xp, int E, int max_rows, int H, cudaStream_t stream);
-int b200_moe_scatter_scaled(const void* src, const float* probs, const int* row_map, void* dst, int T, int k, int H,
-                            cudaStream_t stream);
+int b200_moe_zero_padding(const int* filled, const int* offsets, void* xp, void* row_info, int E, int max_rows, int H,
+                          cudaStream_t stream);
+// dst[row_map[t, j]] = src[t]. row_info (8 bytes a row): (t * k + j, probs[t, j]) here, (-1, 0) in the rows of padding (above)
+int b200_moe_spread(const void* src, const float* probs, const int* row_map, void* dst, void* row_info, int T, int k, int H,
+                    cudaStream_t stream);
 int b200_moe_combine(const void* y, const float* probs, const int* row_map, void* out, int T, int k, int H,
                      cudaStream_t stream);
-int b200_moe_combine_dprob(const void* dout, const void* y, const int* row_map, float* dprob, int T, int k, int H,
-                           cudaStream_t stream);
+// Backward between the two expert projections: dact [max_rows, I] without the weights -> dh1 [max_rows, 2I], ap = prob * act
+// [max_rows, I] (both zero in rows of padding below n_tiles * 128), dprob [T, k]
+int b200_moe_swiglu_bwd(const void* dact, const void* h1, const void* row_info, const int* n_tiles, void* dh1, void* ap,
+                        float* dprob, int max_rows, int I, cudaStream_t stream);
 // Grouped GEMMs over the padded, expert-sorted token buffer (see grouped_gemm.cu for the three forms).
 int b200_grouped_gemm(const void* X, const void* W, void* Y, int max_rows, int N, int K, int num_experts,
                       long long ldx, long long ldy, const int* tile_expert, const int* n_tiles, int mode,

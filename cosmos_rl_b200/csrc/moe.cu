@@ -128,14 +128,17 @@ permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx,
   }
 }
 
-// the rows between an expert's last filled row and the next expert's first: the GEMMs contract over them
+// the rows between an expert's last filled row and the next expert's first: the GEMMs contract over them. row_info (nullable) says
+// that they belong to no (token, choice).
 __global__ void __launch_bounds__(ROW_MAX_THREADS)
 zero_padding_kernel(const int* __restrict__ filled, const int* __restrict__ offsets, __nv_bfloat16* __restrict__ xp,
-                    int max_rows, int H) {
+                    int2* __restrict__ row_info, int max_rows, int H) {
   const int e = blockIdx.x, end = min(offsets[e + 1], max_rows);   // counts that are only an upper bound may add up to more
-  for (int r = offsets[e] + filled[e] + blockIdx.y; r < end; r += gridDim.y)
+  for (int r = offsets[e] + filled[e] + blockIdx.y; r < end; r += gridDim.y) {
     for (int i = threadIdx.x; i < H / 8; i += blockDim.x)
       reinterpret_cast<uint4*>(xp + (long long)r * H)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (row_info && threadIdx.x == 0) row_info[r] = make_int2(-1, 0);
+  }
 }
 
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
@@ -155,22 +158,18 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return u;
 }
 
-// spread rows through an existing row_map (backward of combine: dy[pos] = prob * dout[t])
+// Backward of combine, without the weights (expert_swiglu_bwd_kernel brings them in): the k rows of a token get its gradient, and
+// row_info says which (token, choice) a row belongs to and what its weight is.
 __global__ void __launch_bounds__(ROW_MAX_THREADS)
-scatter_scaled_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ probs,
-                      const int* __restrict__ row_map, __nv_bfloat16* __restrict__ dst, int k, int H) {
+spread_kernel(const __nv_bfloat16* __restrict__ src, const float* __restrict__ probs, const int* __restrict__ row_map,
+              __nv_bfloat16* __restrict__ dst, int2* __restrict__ row_info, int k, int H) {
   const long long t = blockIdx.x;
+  for (int j = threadIdx.x; j < k; j += blockDim.x)
+    row_info[row_map[t * k + j]] = make_int2((int)(t * k + j), __float_as_int(probs[t * k + j]));
   for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
-    float f[8];
-    unpack8(reinterpret_cast<const uint4*>(src + t * H)[i], f);
+    const uint4 v = reinterpret_cast<const uint4*>(src + t * H)[i];
 #pragma unroll 4
-    for (int j = 0; j < k; ++j) {
-      const float p = probs ? probs[t * k + j] : 1.f;
-      float o[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) o[c] = f[c] * p;
-      reinterpret_cast<uint4*>(dst + (long long)row_map[t * k + j] * H)[i] = pack8(o);
-    }
+    for (int j = 0; j < k; ++j) reinterpret_cast<uint4*>(dst + (long long)row_map[t * k + j] * H)[i] = v;
   }
 }
 
@@ -193,42 +192,52 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ pr
   }
 }
 
-// dprob[t,j] = <dout[t], y[row_map[t,j]]>, eight choices at a time
-__global__ void __launch_bounds__(ROW_MAX_THREADS)
-combine_dprob_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
-                     const int* __restrict__ row_map, float* __restrict__ dprob, int k, int H) {
-  __shared__ float sh[ROW_MAX_THREADS / 32][8];
-  const long long t = blockIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int j0 = 0; j0 < k; j0 += 8) {
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
-      float f[8];
-      unpack8(reinterpret_cast<const uint4*>(dout + t * H)[i], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (j0 + j < k) {
-          float g[8];
-          unpack8(reinterpret_cast<const uint4*>(y + (long long)row_map[t * k + j0 + j] * H)[i], g);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) s[j] += f[c] * g[c];
-        }
-      }
-    }
+// Backward of the experts' middle. With a = silu(g) o u, the row's output is p (a Wd^T) and dact = dout Wd lacks the weight p:
+//   dprob = <a, dact>,  dh1 = p dact d(a)/d(g, u),  ap = p a (what the gradient of Wd contracts with the unweighted dout).
+// So the weights' gradient needs neither the experts' output nor a pass over it, a is not formed in a pass of its own, and the
+// gradient is spread as it is. Bound by HBM (12 bytes an element of a; 4096 tokens on 128 experts of 768, 8 each: 61 us, 0.85 of
+// copy speed; the passes it stands for, a, the gradient of a and dprob, took 126). One warp a row, since dprob is the row's sum;
+// 40 warps an SM hide the way from a row's number to its data better than three vectors a lane on their way with 16 or 24 warps
+// (73 and 64 us), and several warps a row add a barrier (80).
+__global__ void __launch_bounds__(256, 5)
+expert_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bfloat16* __restrict__ h1,
+                         const int2* __restrict__ row_info, const int* __restrict__ n_tiles, __nv_bfloat16* __restrict__ dh1,
+                         __nv_bfloat16* __restrict__ ap, float* __restrict__ dprob, int I) {
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);   // there is room for whole blocks of rows
+  const int2 info = row_info[row];
+  if (row >= (long long)n_tiles[0] * MOE_ALIGN) return;
+  const int lane = threadIdx.x & 31, nvec = I >> 3;
+  uint4* out = reinterpret_cast<uint4*>(dh1 + row * 2 * I);
+  uint4* out_a = reinterpret_cast<uint4*>(ap + row * I);
+  if (info.x < 0) {   // padding
+    for (int v = lane; v < nvec; v += 32) out[v] = out[nvec + v] = out_a[v] = make_uint4(0u, 0u, 0u, 0u);
+    return;
+  }
+  const uint4* in = reinterpret_cast<const uint4*>(h1 + row * 2 * I);
+  const uint4* in_d = reinterpret_cast<const uint4*>(dact + row * I);
+  const float p = __int_as_float(info.y);
+  float dot = 0.f;
+  for (int v = lane; v < nvec; v += 32) {
+    const uint4 gv = in[v], uv = in[nvec + v], dv = in_d[v];
+    float a[8], b[8], c[8], dg[8], du[8];
+    unpack8(gv, a);
+    unpack8(uv, b);
+    unpack8(dv, c);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
-      if (lane == 0) sh[warp][j] = s[j];
+      const float s = 1.f / (1.f + __expf(-a[j])), silu = a[j] * s, act = silu * b[j], pd = p * c[j];
+      dot += act * c[j];
+      dg[j] = pd * b[j] * (s + silu * (1.f - s));
+      du[j] = pd * silu;
+      a[j] = p * act;
     }
-    __syncthreads();
-    if (threadIdx.x < 8 && j0 + (int)threadIdx.x < k) {
-      float r = 0.f;
-      for (int w = 0; w < (int)blockDim.x / 32; ++w) r += sh[w][threadIdx.x];
-      dprob[t * k + j0 + threadIdx.x] = r;
-    }
-    __syncthreads();
+    out[v] = pack8(dg);
+    out[nvec + v] = pack8(du);
+    out_a[v] = pack8(a);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if (lane == 0) dprob[info.x] = dot;
 }
 
 // threads of a block that moves rows of H elements
@@ -266,19 +275,21 @@ int b200_moe_permute(const void* x, const int* idx, const int* offsets, int* cur
   return ok();
 }
 
-int b200_moe_zero_padding(const int* filled, const int* offsets, void* xp, int E, int max_rows, int H, cudaStream_t stream) {
+int b200_moe_zero_padding(const int* filled, const int* offsets, void* xp, void* row_info, int E, int max_rows, int H,
+                          cudaStream_t stream) {
   if (E <= 0) return 0;
   if (H & 7) return B200_ERR_ARG;
-  zero_padding_kernel<<<dim3(E, E < 64 ? 32 : 16), row_threads(H), 0, stream>>>(filled, offsets, (__nv_bfloat16*)xp, max_rows, H);
+  zero_padding_kernel<<<dim3(E, E < 64 ? 32 : 16), row_threads(H), 0, stream>>>(filled, offsets, (__nv_bfloat16*)xp,
+                                                                                (int2*)row_info, max_rows, H);
   return ok();
 }
 
-int b200_moe_scatter_scaled(const void* src, const float* probs, const int* row_map, void* dst, int T, int k, int H,
-                            cudaStream_t stream) {
+int b200_moe_spread(const void* src, const float* probs, const int* row_map, void* dst, void* row_info, int T, int k, int H,
+                    cudaStream_t stream) {
   if (T <= 0) return 0;
   if (H & 7) return B200_ERR_ARG;
-  scatter_scaled_kernel<<<T, row_threads(H), 0, stream>>>((const __nv_bfloat16*)src, probs, row_map, (__nv_bfloat16*)dst,
-                                                          k, H);
+  spread_kernel<<<T, row_threads(H), 0, stream>>>((const __nv_bfloat16*)src, probs, row_map, (__nv_bfloat16*)dst,
+                                                  (int2*)row_info, k, H);
   return ok();
 }
 
@@ -290,12 +301,13 @@ int b200_moe_combine(const void* y, const float* probs, const int* row_map, void
   return ok();
 }
 
-int b200_moe_combine_dprob(const void* dout, const void* y, const int* row_map, float* dprob, int T, int k, int H,
-                           cudaStream_t stream) {
-  if (T <= 0) return 0;
-  if (H & 7) return B200_ERR_ARG;
-  combine_dprob_kernel<<<T, row_threads(H), 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)y, row_map,
-                                                         dprob, k, H);
+int b200_moe_swiglu_bwd(const void* dact, const void* h1, const void* row_info, const int* n_tiles, void* dh1, void* ap,
+                        float* dprob, int max_rows, int I, cudaStream_t stream) {
+  if (max_rows <= 0) return 0;
+  if ((I & 7) || (max_rows & 7)) return B200_ERR_ARG;
+  expert_swiglu_bwd_kernel<<<max_rows / 8, 256, 0, stream>>>((const __nv_bfloat16*)dact, (const __nv_bfloat16*)h1,
+                                                                   (const int2*)row_info, n_tiles, (__nv_bfloat16*)dh1,
+                                                                   (__nv_bfloat16*)ap, dprob, I);
   return ok();
 }
 

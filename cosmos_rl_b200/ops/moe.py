@@ -89,13 +89,13 @@ class _Dispatch:
                                                    native.ptr(self.cursor), self.max_tiles, native.stream()),
                      "moe_offsets")
 
-    def zero_padding(self, buf: torch.Tensor) -> None:
-        """Clears the rows of an expert-sorted buffer that no (token, choice) fills. After the permutation ``cursor`` holds
-        how many rows each expert got; the caller's histogram is read for the offsets only, since the caller may clear or
-        refill it before backward runs."""
+    def zero_padding(self, buf: torch.Tensor, row_info: Optional[torch.Tensor] = None) -> None:
+        """Clears the rows of an expert-sorted buffer that no (token, choice) fills, and marks them in ``row_info``. After the
+        permutation ``cursor`` holds how many rows each expert got; the caller's histogram is read for the offsets only, since
+        the caller may clear or refill it before backward runs."""
         native.check(native.lib().b200_moe_zero_padding(native.ptr(self.cursor), native.ptr(self.offsets),
-                                                        native.ptr(buf), self.E, buf.shape[0], buf.shape[1],
-                                                        native.stream()), "moe_zero_padding")
+                                                        native.ptr(buf), native.ptr(row_info), self.E, buf.shape[0],
+                                                        buf.shape[1], native.stream()), "moe_zero_padding")
 
 
 def _rows16(x: torch.Tensor) -> torch.Tensor:
@@ -155,33 +155,34 @@ class _MoEExperts(torch.autograd.Function):
         probs = probs.float().contiguous()
         native.check(L.b200_moe_combine(native.ptr(y), native.ptr(probs), native.ptr(disp.row_map), native.ptr(out), T,
                                         k, H, native.stream()), "moe_combine")
-        ctx.save_for_backward(xp, h1, y, probs, w_gate_up, w_down)
+        ctx.save_for_backward(xp, h1, probs, w_gate_up, w_down)
         ctx.disp = disp
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        xp, h1, y, probs, w_gate_up, w_down = ctx.saved_tensors
+        xp, h1, probs, w_gate_up, w_down = ctx.saved_tensors
         disp = ctx.disp
         T, k, E = disp.T, disp.k, disp.E
         H = xp.shape[1]
-        I2 = h1.shape[1]
+        I = h1.shape[1] // 2
         L = native.lib()
         dout = _rows16(dout)
-        dprob = torch.empty(T, k, dtype=torch.float32, device=dout.device)
-        native.check(L.b200_moe_combine_dprob(native.ptr(dout), native.ptr(y), native.ptr(disp.row_map),
-                                              native.ptr(dprob), T, k, H, native.stream()), "moe_dprob")
+        # the gradient goes to the experts' rows without its weights; they come in between the two projections
         dy = torch.empty(disp.max_rows, H, dtype=torch.bfloat16, device=dout.device)
-        disp.zero_padding(dy)
-        native.check(L.b200_moe_scatter_scaled(native.ptr(dout), native.ptr(probs), native.ptr(disp.row_map),
-                                               native.ptr(dy), T, k, H, native.stream()), "moe_scatter")
-        act = _swiglu_rows(h1, disp)                        # recomputed: cheaper than keeping [Mp, I] alive
-        dact = _grouped(dy, w_down, disp, 1, I2 // 2)       # dY . W_down[e]   (W_down [E, H, I])
-        dw_down = torch.empty_like(w_down)
-        _grouped_wgrad(dy, act, disp, dw_down, False)
+        row_info = torch.empty(disp.max_rows, 2, dtype=torch.int32, device=dout.device)
+        disp.zero_padding(dy, row_info)
+        native.check(L.b200_moe_spread(native.ptr(dout), native.ptr(probs), native.ptr(disp.row_map), native.ptr(dy),
+                                       native.ptr(row_info), T, k, H, native.stream()), "moe_spread")
+        dact = _grouped(dy, w_down, disp, 1, I)             # dY . W_down[e]   (W_down [E, H, I])
         dh1 = torch.empty_like(h1)
-        native.check(L.b200_swiglu_bwd(native.ptr(dact), native.ptr(h1), native.ptr(dh1), h1.shape[0], I2 // 2,
-                                       native.ptr(disp.n_tiles), native.stream()), "swiglu_bwd")
+        ap = torch.empty(disp.max_rows, I, dtype=torch.bfloat16, device=dout.device)
+        dprob = torch.empty(T, k, dtype=torch.float32, device=dout.device)
+        native.check(L.b200_moe_swiglu_bwd(native.ptr(dact), native.ptr(h1), native.ptr(row_info), native.ptr(disp.n_tiles),
+                                           native.ptr(dh1), native.ptr(ap), native.ptr(dprob), disp.max_rows, I,
+                                           native.stream()), "moe_swiglu_bwd")
+        dw_down = torch.empty_like(w_down)
+        _grouped_wgrad(dy, ap, disp, dw_down, False)
         dxp = _grouped(dh1, w_gate_up, disp, 1, H)          # dH1 . W_gu[e]     (W_gu [E, 2I, H])
         dw_gu = torch.empty_like(w_gate_up)
         _grouped_wgrad(dh1, xp, disp, dw_gu, False)

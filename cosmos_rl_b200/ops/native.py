@@ -113,10 +113,10 @@ _SIGS = {
     "b200_moe_route_topk": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "b200_moe_offsets": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "b200_moe_permute": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
-    "b200_moe_zero_padding": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
-    "b200_moe_scatter_scaled": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "b200_moe_zero_padding": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "b200_moe_spread": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "b200_moe_combine": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
-    "b200_moe_combine_dprob": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "b200_moe_swiglu_bwd": [c_void_p] * 7 + [c_int, c_int, c_void_p],
     "b200_grouped_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p,
                           c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_grouped_wgrad_pairs": [c_int] * 7,

@@ -1778,3 +1778,37 @@ def test_paged_decode_many_equal_sequences(B, hq, hkv, length):
     # probabilities and the result are rounded to bf16 (2^-9 each)
     assert (out.cpu().float() - ref.float()).norm() <= 2.0 ** -7 * ref.float().norm()
     assert (out.cpu().float() - ref.float()).abs().max() <= 2.0 ** -6 * ref.float().abs().max()
+
+
+@pytest.mark.parametrize("I", [8, 248, 256, 264, 1536])
+def test_moe_swiglu_bwd_rows(I):
+    """The backward between the experts' projections: a vector less and more than a warp's 32, rows of padding, and tiles past the
+    last one in use, which stay as they are."""
+    torch.manual_seed(85)
+    rows, used, k = 512, 256, 2
+    h1, dact = _bf16(rows, 2 * I), _bf16(rows, I)
+    probs = torch.rand(rows, device=DEV)
+    live = torch.rand(rows, device=DEV) < 0.7
+    src = torch.where(live, torch.randperm(rows, device=DEV), -1).to(torch.int32)
+    info = torch.stack([src, torch.where(live, probs, 0.).view(torch.int32)], dim=1).contiguous()
+    h1[:used][~live[:used]] = float("nan")                       # what padding holds must not show
+    dh1, ap = (torch.full((rows, n), 7., dtype=torch.bfloat16, device=DEV) for n in (2 * I, I))
+    dprob = torch.full((rows,), 7., device=DEV)
+    n_tiles = torch.tensor([used // 128], dtype=torch.int32, device=DEV)
+    native.check(native.lib().b200_moe_swiglu_bwd(native.ptr(dact), native.ptr(h1), native.ptr(info), native.ptr(n_tiles),
+                                                  native.ptr(dh1), native.ptr(ap), native.ptr(dprob), rows, I,
+                                                  native.stream()), "moe_swiglu_bwd")
+    torch.cuda.synchronize()
+    gu = h1[:used].double().requires_grad_(True)
+    act = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+    p, d, on = probs[:used, None].double(), dact[:used].double(), live[:used, None]
+    want, = torch.autograd.grad(torch.where(on, act, 0.), gu, p * d)
+    want, act = torch.where(on, want, 0.), torch.where(on, act.detach(), 0.)
+    # one rounding to bf16; the factors in fp32 with the fast exponential (2 ulp, and its argument's rounding)
+    assert torch.allclose(dh1[:used].double(), want, rtol=2 ** -8, atol=1e-5)
+    assert torch.allclose(ap[:used].double(), p * act, rtol=2 ** -8, atol=1e-5)
+    at = src[:used][live[:used]].long()
+    ref = (act * d).sum(-1)[live[:used]]
+    # I fp32 products with a rounding of 2^-20 each at most
+    assert ((dprob[at].double() - ref).abs() <= 2 ** -20 * (act * d).abs().sum(-1)[live[:used]] + 1e-6).all()
+    assert (dh1[used:] == 7).all() and (ap[used:] == 7).all() and (dprob == 7).sum() == rows - at.numel()
