@@ -1812,3 +1812,17 @@ def test_moe_swiglu_bwd_rows(I):
     # I fp32 products with a rounding of 2^-20 each at most
     assert ((dprob[at].double() - ref).abs() <= 2 ** -20 * (act * d).abs().sum(-1)[live[:used]] + 1e-6).all()
     assert (dh1[used:] == 7).all() and (ap[used:] == 7).all() and (dprob == 7).sum() == rows - at.numel()
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 2, 2), (16, 33, 1), (17, 256, 8), (4099, 16, 8)])
+def test_moe_router_counts(T, E, k):
+    """Choices counted a block at a time: one token, a full block, one more, and experts that every block has."""
+    from cosmos_rl_b200.ops import moe
+    torch.manual_seed(86)
+    logits = torch.randn(T, E, device=DEV)
+    counts = torch.full((E,), 5, dtype=torch.int32, device=DEV)      # added to
+    p, i = moe.route_topk(logits, k, False, counts)
+    pr, ir = torch.softmax(logits.double(), -1).topk(k, dim=-1)
+    assert torch.equal(i.long(), ir)
+    assert torch.allclose(p.double(), pr, rtol=2 ** -19, atol=1e-30)   # the exponential's argument is good to 2^-22 of up to 8
+    assert torch.equal(counts.long() - 5, torch.bincount(ir.flatten(), minlength=E))
