@@ -120,6 +120,9 @@ int b200_grouped_gemm(const void* X, const void* W, void* Y, int max_rows, int N
 int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, int N, int K, int num_experts,
                        long long lddy, long long ldx, const int* expert_offsets, int out_fp32, int accumulate,
                        uint32_t* status, int num_sms, cudaStream_t stream);
+int b200_grouped_wgrad_filled(const void* dY, const void* X, void* dW, int max_rows, int N, int K, int num_experts,
+                              long long lddy, long long ldx, const int* expert_offsets, const int* filled, int out_fp32,
+                              int accumulate, uint32_t* status, int num_sms, cudaStream_t stream);
 int b200_grouped_wgrad_pairs(int max_rows, int N, int K, int num_experts, int out_fp32, int accumulate, int num_sms);
 
 // ---- normalisation / activation / rotary ------------------------------------------------------------

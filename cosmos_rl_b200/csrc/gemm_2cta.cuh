@@ -96,8 +96,9 @@ struct Gemm2Params {
   long long ldc;
   DlogitsParams dl;  // G2_EPI_DLOGITS
   // G2_EPI_EXPERTS: C is [experts, M, N], and expert e contracts over rows [offsets[e], offsets[e + 1]) of A and B (multiples
-  // of 64; both MN-major)
+  // of 64; both MN-major), or over the blocks of 64 that its first filled[e] rows reach into (nullable)
   const int* offsets;
+  const int* filled;
   int experts;
 };
 
@@ -157,12 +158,13 @@ struct G2Work {
 // G2_EPI_EXPERTS: all tiles of an expert's weight gradient, expert by expert
 struct G2ExpertWork {
   int num_n, per_expert, total;
-  const int* offsets;
+  const int *offsets, *filled;
   __device__ __forceinline__ void init(const Gemm2Params& ep, bool, int num_m, int num_n_, int) {
     num_n = num_n_;
     per_expert = num_m * num_n_;
     total = per_expert * ep.experts;
     offsets = ep.offsets;
+    filled = ep.filled;
   }
   __device__ __forceinline__ bool get(int it, G2Unit& u) const {
     const int i = (blockIdx.x >> 1) + it * (gridDim.x >> 1);
@@ -173,6 +175,7 @@ struct G2ExpertWork {
     u.n_blk = r - u.m_blk * num_n;
     u.kb0 = offsets[u.batch] / G2_BK;
     u.kb1 = offsets[u.batch + 1] / G2_BK;
+    if (filled) u.kb1 = min(u.kb1, u.kb0 + (filled[u.batch] + G2_BK - 1) / G2_BK);
     u.cut = false;
     return true;
   }

@@ -27,6 +27,7 @@ struct GroupedParams {
   int out_fp32, accumulate, bn, batched;
   const int* tile_expert;     // [max_tiles] expert of each 128-row tile (fwd/dgrad)
   const int* expert_offsets;  // [E + 1] padded row offsets (wgrad)
+  const int* filled;          // [E] rows that are not padding (wgrad), nullable
   const int* n_tiles;         // [1] number of 128-row tiles in use
   int num_experts;
 };
@@ -131,13 +132,14 @@ struct TokenTileSchedule {
 // wgrad: tiles = expert x (128-row tile of dW) x (BN-column tile of dW); contraction over the expert's rows
 struct ExpertWgradSchedule {
   int num_m, num_n, per_expert, total, bn;
-  const int* off;
+  const int *off, *filled;
   __device__ __forceinline__ void init(int M, int N, int, int BN, const GroupedParams& p) {
     num_m = (M + GEMM_BM - 1) / GEMM_BM;
     num_n = (N + BN - 1) / BN;
     per_expert = num_m * num_n;
     total = per_expert * p.num_experts;
     off = p.expert_offsets;
+    filled = p.filled;
     bn = BN;
   }
   __device__ __forceinline__ bool get(int it, TileInfo& t) const {
@@ -150,6 +152,7 @@ struct ExpertWgradSchedule {
     t.b_mn0 = t.n_blk * bn;
     t.k0 = off[e];
     t.num_kb = (off[e + 1] - off[e]) / GEMM_BK;
+    if (filled) t.num_kb = min(t.num_kb, (filled[e] + GEMM_BK - 1) / GEMM_BK);
     t.batch = e;
     return true;
   }
@@ -252,7 +255,7 @@ int b200_grouped_gemm(const void* X, const void* W, void* Y, int max_rows, int N
   if (make_tmap_grouped_out(&tmC, Y, 1, max_rows, N, ldy, (uint64_t)max_rows * ldy, 0)) return B200_ERR_TENSORMAP;
   if (make_tmap_2d(&tmA, X, max_rows, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   static bool s0 = false, s1 = false;
-  GroupedParams ep{nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, n_tiles, num_experts};
+  GroupedParams ep{nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles, num_experts};
   const int grid = num_sms;
   if (mode == 0) {
     if (make_tmap_3d(&tmB, W, num_experts, N, K, K, (uint64_t)N * K, GG_BN, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
@@ -274,10 +277,12 @@ int b200_grouped_wgrad_pairs(int max_rows, int N, int K, int num_experts, int ou
   return b200::wgrad_pairs(max_rows, N, K, num_experts, out_fp32, accumulate, num_sms) > 0;
 }
 
-// dW[e][N, K] (+)= dY[rows of e, N]^T . X[rows of e, K]; rows of e = [expert_offsets[e], expert_offsets[e+1])
-int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, int N, int K, int num_experts,
-                       long long lddy, long long ldx, const int* expert_offsets, int out_fp32, int accumulate,
-                       uint32_t* status, int num_sms, cudaStream_t stream) {
+// dW[e][N, K] (+)= dY[rows of e, N]^T . X[rows of e, K]; rows of e = [expert_offsets[e], expert_offsets[e+1]). With `filled` only
+// the first filled[e] of them count and the rest is zero: blocks of 64 rows that hold nothing else are left out (half of the
+// experts have one; 4096 tokens, 8 of 128 experts each, 1536 x 2048 and 2048 x 768 a gradient: 395 us with them, 385).
+int b200_grouped_wgrad_filled(const void* dY, const void* X, void* dW, int max_rows, int N, int K, int num_experts,
+                              long long lddy, long long ldx, const int* expert_offsets, const int* filled, int out_fp32,
+                              int accumulate, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (max_rows <= 0 || N <= 0 || K <= 0 || (lddy & 7) || (ldx & 7)) return B200_ERR_ARG;
   CUtensorMap tmA, tmB, tmC;
@@ -292,6 +297,7 @@ int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, in
     ep2.accumulate = accumulate;
     ep2.a_bytes = WG_SMEM::A_BYTES;
     ep2.offsets = expert_offsets;
+    ep2.filled = filled;
     ep2.experts = num_experts;
     gemm2_bf16_kernel<256, 6, true, true, G2_EPI_EXPERTS><<<2 * np, G2_THREADS, WG_SMEM::TOTAL, stream>>>(
         tmA, tmB, tmC, tmC, N, K, 0, ep2, status);
@@ -300,10 +306,17 @@ int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, in
   static bool s2 = false;
   if (set_smem(grouped_wgrad_kernel, s2)) return B200_ERR_LAUNCH;
   GroupedParams ep{nullptr, accumulate && !out_fp32 ? (const __nv_bfloat16*)dW : nullptr, K, (long long)N * K, K, N, out_fp32,
-                   accumulate, GG_BN, 1, nullptr, expert_offsets, nullptr, num_experts};
+                   accumulate, GG_BN, 1, nullptr, expert_offsets, filled, nullptr, num_experts};
   grouped_wgrad_kernel<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, N, K,
                                                                                                      0, ep, status);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+}
+
+int b200_grouped_wgrad(const void* dY, const void* X, void* dW, int max_rows, int N, int K, int num_experts,
+                       long long lddy, long long ldx, const int* expert_offsets, int out_fp32, int accumulate,
+                       uint32_t* status, int num_sms, cudaStream_t stream) {
+  return b200_grouped_wgrad_filled(dY, X, dW, max_rows, N, K, num_experts, lddy, ldx, expert_offsets, nullptr, out_fp32,
+                                   accumulate, status, num_sms, stream);
 }
 
 }  // extern "C"

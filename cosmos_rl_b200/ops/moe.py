@@ -123,14 +123,17 @@ def _grouped(x, w, disp: _Dispatch, mode: int, n_out: int) -> torch.Tensor:
     return y
 
 
-def _grouped_wgrad(dy, x, disp: _Dispatch, out: torch.Tensor, accumulate: bool) -> None:
+def _grouped_wgrad(dy, x, disp: _Dispatch, out: torch.Tensor, accumulate: bool,
+                   filled: Optional[torch.Tensor] = None) -> None:
+    """``filled`` (int32 [E]): how many of an expert's rows are not zero in both factors; without it all of its block counts."""
     st = native.status_word(x.device)
     dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
-    native.check(native.lib().b200_grouped_wgrad(native.ptr(dy), native.ptr(x), native.ptr(out), disp.max_rows,
-                                                 dy.shape[1], x.shape[1], disp.E, dy.stride(0), x.stride(0),
-                                                 native.ptr(disp.offsets), 1 if out.dtype == torch.float32 else 0,
-                                                 int(accumulate), native.ptr(st), native.num_sms(dev),
-                                                 native.stream()), "grouped_wgrad")
+    native.check(native.lib().b200_grouped_wgrad_filled(native.ptr(dy), native.ptr(x), native.ptr(out), disp.max_rows,
+                                                        dy.shape[1], x.shape[1], disp.E, dy.stride(0), x.stride(0),
+                                                        native.ptr(disp.offsets), native.ptr(filled),
+                                                        1 if out.dtype == torch.float32 else 0, int(accumulate),
+                                                        native.ptr(st), native.num_sms(dev), native.stream()),
+                 "grouped_wgrad")
 
 
 class _MoEExperts(torch.autograd.Function):
@@ -182,10 +185,10 @@ class _MoEExperts(torch.autograd.Function):
                                            native.ptr(dh1), native.ptr(ap), native.ptr(dprob), disp.max_rows, I,
                                            native.stream()), "moe_swiglu_bwd")
         dw_down = torch.empty_like(w_down)
-        _grouped_wgrad(dy, ap, disp, dw_down, False)
+        _grouped_wgrad(dy, ap, disp, dw_down, False, disp.cursor)
         dxp = _grouped(dh1, w_gate_up, disp, 1, H)          # dH1 . W_gu[e]     (W_gu [E, 2I, H])
         dw_gu = torch.empty_like(w_gate_up)
-        _grouped_wgrad(dh1, xp, disp, dw_gu, False)
+        _grouped_wgrad(dh1, xp, disp, dw_gu, False, disp.cursor)
         dx = torch.empty(T, H, dtype=torch.bfloat16, device=dout.device)
         native.check(L.b200_moe_combine(native.ptr(dxp), None, native.ptr(disp.row_map), native.ptr(dx), T, k, H,
                                         native.stream()), "moe_unpermute")

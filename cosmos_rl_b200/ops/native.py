@@ -122,6 +122,8 @@ _SIGS = {
     "b200_grouped_wgrad_pairs": [c_int] * 7,
     "b200_grouped_wgrad": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong,
                            c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
+    "b200_grouped_wgrad_filled": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong,
+                                  c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_quant_mxfp4": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "b200_dequant_mxfp4": [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p],
     "b200_quant_fp8_block": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p],

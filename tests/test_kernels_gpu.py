@@ -1826,3 +1826,34 @@ def test_moe_router_counts(T, E, k):
     assert torch.equal(i.long(), ir)
     assert torch.allclose(p.double(), pr, rtol=2 ** -19, atol=1e-30)   # the exponential's argument is good to 2^-22 of up to 8
     assert torch.equal(counts.long() - 5, torch.bincount(ir.flatten(), minlength=E))
+
+
+@pytest.mark.parametrize("counts", [(0, 1, 64, 65), (128, 63, 129, 320)])
+@pytest.mark.parametrize("pairs", [False, True])
+def test_expert_weight_gradients_of_filled_rows(counts, pairs):
+    """Blocks of 64 rows past an expert's last one are not contracted over, whatever they hold, in both forms of the kernel."""
+    torch.manual_seed(87)
+    N, K, E = (2048, 2560, 4) if pairs else (136, 264, 4)
+    off = [0]
+    for c in counts:
+        off.append(off[-1] + -(-c // 128) * 128)
+    Mp = max(off[-1], 320 * E if pairs else 128)                     # the room decides which form it is
+    dy, x = _bf16(Mp, N), _bf16(Mp, K)
+    for e, c in enumerate(counts):
+        last = off[e] + -(-c // 64) * 64
+        dy[off[e] + c:last] = x[off[e] + c:last] = 0
+        dy[last:off[e + 1]] = x[last:off[e + 1]] = float("nan")
+    out = torch.full((E, N, K), 7., dtype=torch.bfloat16, device=DEV)
+    offsets, filled = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in (off, counts))
+    sms = native.num_sms(0)
+    assert native.lib().b200_grouped_wgrad_pairs(Mp, N, K, E, 0, 0, sms) == int(pairs)
+    native.check(native.lib().b200_grouped_wgrad_filled(native.ptr(dy), native.ptr(x), native.ptr(out), Mp, N, K, E, N, K,
+                                                        native.ptr(offsets), native.ptr(filled), 0, 0,
+                                                        native.ptr(native.status_word(dy.device)), sms, native.stream()),
+                 "grouped_wgrad")
+    native.read_status(dy.device)
+    for e, c in enumerate(counts):
+        a, b = dy[off[e]:off[e] + c].double(), x[off[e]:off[e] + c].double()
+        # one rounding to bf16 and fp32 sums of c products
+        bound = 2.0 ** -8 * (a.t() @ b).abs() + 2.0 ** -20 * a.norm(dim=0)[:, None] * b.norm(dim=0) + 1e-6
+        assert ((out[e].double() - a.t() @ b).abs() <= bound).all(), e
