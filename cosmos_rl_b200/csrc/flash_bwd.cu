@@ -10,7 +10,8 @@
 //          dP = dO V^T         M=queries N=keys K=d        TMEM dP
 //          dS = exp2(S c - lse) o (dP - delta)             softmax warps, bf16 into the columns of S
 //          dQ += dS K          M=queries N=d K=keys        A = dS out of TMEM, B = the K tile read MN-major
-//          delta = rowsum(O o dO) of its rows is formed first and left in memory for the second kernel.
+//          delta = rowsum(O o dO) of its rows is formed first (O fetched under the end of the item before) and left in memory
+//          for the second kernel.
 //          K has three slots: a block is needed from S until dQ, and with two the load of block j + 1 starts when dQ of block
 //          j - 1 is through and S of j + 1 waits for it (3600 and 2340 tokens, 16 heads, no mask: 296 us, 244 with
 //          three). The result passes through the K slot that the item read last, since there is no room for staging of
@@ -48,7 +49,7 @@ constexpr int FB_D = 128;
 constexpr int FB_TILE = FB_B * FB_D * 2;             // 32 KiB, two boxes of 128 rows x 64 elements
 constexpr int FB_STATS = 2 * 2 * FB_B * 4;           // dK/dV kernel: lse and delta of two query blocks
 constexpr int FB_SMEM = 6 * FB_TILE + FB_STATS + 256 + 1024;          // dK/dV kernel
-constexpr int FB_SMEM_DQ = 7 * FB_TILE + 512 + 1024;                  // dQ kernel: Q, dO, K x3, V x2
+constexpr int FB_SMEM_DQ = 7 * FB_TILE + 512 + 2 * FB_B * 4 + 1024;   // dQ kernel: Q, dO, K x3, V x2, delta of two items
 constexpr int FB_THREADS = 320;                      // TMA warp, MMA warp, 8 softmax warps
 constexpr float FB_LOG2E = 1.4426950408889634f;
 // One pair of exponentials in so many runs on the fp32 pipe (exp2_poly2): the two warps of a scheduler are in their exponentials
@@ -183,19 +184,21 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint64_t* ds_ready = bars + 17;
   uint64_t* done = bars + 18;
   uint64_t* dp_free = bars + 36;     // dP has been read
+  uint64_t* dlt_full = bars + 37;    // [4] delta of a quadrant's rows, from its two warps
   uint64_t* item_full = bars + 19;   // [2] slots of the work queue
   uint64_t* item_empty = bars + 21;  // [2] read by the MMA thread and the eight softmax warps
   FlashItem* items = reinterpret_cast<FlashItem*>(bars + 24);   // [2]
   // bars + 32: 16 bytes and bars + 23: barrier of cluster launch control
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 34);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  float* dlt_sh = reinterpret_cast<float*>(bars + 64);          // [2][128] -delta of the item's rows
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
     mbar_init(do_full, 1);
-    mbar_init(do_empty, 1);
+    mbar_init(do_empty, 9);
     for (int s = 0; s < 3; ++s) {
       mbar_init(&k_full[s], 1);
       mbar_init(&k_empty[s], 1);
@@ -207,6 +210,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_init(&item_full[s], 1);
       mbar_init(&item_empty[s], 9);
     }
+    for (int s = 0; s < 4; ++s) mbar_init(&dlt_full[s], 2);
     mbar_init(bars + 23, 1);
     mbar_init(dp_ready, 1);
     mbar_init(ds_ready, 8);
@@ -364,56 +368,80 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
     const float2 c2 = make_float2(p.scale_log2, p.scale_log2);
-    uint32_t kv = 0, finished = 0;
+    uint32_t kv = 0, nq = 0, finished = 0;
     bool ok = true;
-    for (uint32_t it = 0; ok; ++it) {
+    // An item's statistics: delta is rowsum(O o dO), 16 rows a warp. O (a row is one coalesced 256-byte read) and the lane's lse are
+    // fetched before the result of the item before is written, dO is read from the tile that dP takes. Loads of both where the
+    // sums are used, and by both warps of a quadrant, held up every item: 32 x 256 tokens, 28 heads, 92.8 us and 72.1 so (38 are
+    // the bytes); 5 x 1536 tokens 147 and 133; 1 x 8192 517 and 506. (Two more warps for it: 107, 167 and 558. Their waits are
+    // not free, and they had two blocks' time for 64 rows each.) Rows past the end are read at the last row and dropped: no branch
+    // keeps the loads apart.
+    uint2 o2[16];
+    float lse = 0.f;
+    bool valid = false;
+    auto fetch = [&](uint32_t it) -> bool {
+      if (!fb_wait(&item_full[it & 1], (it >> 1) & 1, ST_TIMEOUT_FULL, p.status, abort_flag)) return false;
+      const FlashItem& w = items[it & 1];
+      if (!(valid = w.valid)) return true;
+      const int first = w.row0 + quad * 32 + half_id * 16, own = w.row0 + row;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const long long t = w.q_beg + min(first + i, w.len_q - 1);
+        o2[i] = *reinterpret_cast<const uint2*>(p.out + t * p.ldo + w.head * FB_D + lane * 4);
+      }
+      lse = own < w.len_q ? p.lse[(long long)w.head * p.Tq + w.q_beg + own] : INFINITY;
+      return true;
+    };
+    ok = fetch(0);
+    for (uint32_t it = 0; ok && valid; ++it) {
       const uint32_t slot = it & 1;
-      if (!(ok = fb_wait(&item_full[slot], (it >> 1) & 1, ST_TIMEOUT_FULL, p.status, abort_flag))) break;
       const FlashItem& w = items[slot];                  // read where it is needed: registers are short in the loop
-      if (!w.valid) break;
       const int n = fb_key_blocks(w, p.causal);
       const int q_idx = w.row0 + row;
-      const bool live = q_idx < w.len_q;
       const int k_limit = p.causal ? min(w.len_k, q_idx + w.len_k - w.len_q + 1) : w.len_k;   // keys [0, k_limit) are visible
-      const long long at = (long long)w.head * p.Tq + w.q_beg + q_idx;
-      const float nlse = live ? -p.lse[at] * FB_LOG2E : -INFINITY;
-      // delta of the quadrant's 32 rows: a row is one coalesced 256-byte read of O and of dO; the sums of 32 rows are
-      // reduced together (each shuffle step halves the rows that a lane carries) and row r ends up in lane r. Rows past
-      // the end are read at the last row and dropped: no branch keeps the loads apart.
-      float delta;
-      {
-        float v[32];
-#pragma unroll
-        for (int i0 = 0; i0 < 32; i0 += 16) {
-          uint2 o2[16], g2[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const long long t = w.q_beg + min(w.row0 + quad * 32 + i0 + i, w.len_q - 1);
-            o2[i] = *reinterpret_cast<const uint2*>(p.out + t * p.ldo + w.head * FB_D + lane * 4);
-            g2[i] = *reinterpret_cast<const uint2*>(p.dout + t * p.lddo + w.head * FB_D + lane * 4);
-          }
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].x));
-            const float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].y));
-            const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].x));
-            const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2[i].y));
-            v[i0 + i] = (x0.x * y0.x + x0.y * y0.y) + (x1.x * y1.x + x1.y * y1.y);
-          }
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {   // lane distance d: d rows stay with each lane
-          const bool hi = lane & d;
-#pragma unroll
-          for (int i = 0; i < d; ++i) {
-            const float send = hi ? v[i] : v[i + d], keep = hi ? v[i + d] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-          }
-        }
-        delta = v[0];
+      const float nlse = -lse * FB_LOG2E;
+      // The sums of the 16 rows are reduced together (each shuffle step but the first halves the rows that a lane carries): row r
+      // ends up in the lanes r and r + 16. The quadrant's two warps exchange theirs.
+      float v[16];
+      if (n > 0) {
+        if (!(ok = fb_wait(do_full, nq & 1, ST_TIMEOUT_FULL, p.status, abort_flag))) break;
+        ++nq;
       }
-      if (live && half_id == 0) p.delta[at] = delta;
-      const float2 nl2 = make_float2(nlse, nlse), nd2 = make_float2(-delta, -delta);
+      // the lane's four columns: 8 of the 16 bytes of chunk (lane / 2) & 7 in the half tile lane / 16
+      const uint8_t* g_row = do_sh + (lane >> 4) * (FB_TILE / 2) + (quad * 32 + half_id * 16) * 128 + (lane & 1) * 8;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint2 g2 = *reinterpret_cast<const uint2*>(g_row + i * 128 + ((((lane >> 1) & 7) ^ (i & 7)) << 4));
+        const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].x));
+        const float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o2[i].y));
+        const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2.x));
+        const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2.y));
+        v[i] = (x0.x * y0.x + x0.y * y0.y) + (x1.x * y1.x + x1.y * y1.y);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) {   // lane distance d: d rows stay with each lane
+        const bool hi = lane & d;
+#pragma unroll
+        for (int i = 0; i < d; ++i) {
+          const float send = hi ? v[i] : v[i + d], keep = hi ? v[i + d] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+        }
+      }
+      if (lane < 16) {
+        const int r = quad * 32 + half_id * 16 + lane;
+        if (w.row0 + r < w.len_q && n > 0) p.delta[(long long)w.head * p.Tq + w.q_beg + w.row0 + r] = v[0];
+        dlt_sh[slot * FB_B + r] = -v[0];   // two items' worth: a warp that has got to the next item's has read this one's
+      }
+      __syncwarp();
+      if (lane == 0) {
+        if (n > 0) mbar_arrive(do_empty);
+        mbar_arrive(&dlt_full[quad]);
+      }
+      if (!(ok = fb_wait(&dlt_full[quad], it & 1, ST_TIMEOUT_FULL, p.status, abort_flag))) break;
+      const float nd = dlt_sh[slot * FB_B + row];
+      const float2 nl2 = make_float2(nlse, nlse), nd2 = make_float2(nd, nd);
       for (int j = 0; j < n; ++j, ++kv) {
         const uint32_t s = kv & 1;
         if (!(ok = fb_wait(&s_ready[s], (kv >> 1) & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
@@ -458,7 +486,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(ds_ready);
       }
-      if (!ok) break;
+      if (!ok || !(ok = fetch(it + 1))) break;
       if (n > 0) {
         if (!(ok = fb_wait(done, finished & 1, ST_TIMEOUT_TMEM_FULL, p.status, abort_flag))) break;
         ++finished;

@@ -1857,3 +1857,23 @@ def test_expert_weight_gradients_of_filled_rows(counts, pairs):
         # one rounding to bf16 and fp32 sums of c products
         bound = 2.0 ** -8 * (a.t() @ b).abs() + 2.0 ** -20 * a.norm(dim=0)[:, None] * b.norm(dim=0) + 1e-6
         assert ((out[e].double() - a.t() @ b).abs() <= bound).all(), e
+
+
+def test_flash_attention_backward_items_without_keys_between_others():
+    """CTAs take items one after the other and fetch the next one's rows early: items without a key block, of one and of several,
+    last blocks of 2 and 60 rows, in one call of more items than there are SMs."""
+    from cosmos_rl_b200.ops import attention
+    torch.manual_seed(88)
+    d, hq, hkv, lens_q, lens_k = 128, 28, 4, [300, 130, 700, 1], [200, 0, 64, 129]
+    cu_q, cu_k = (torch.tensor([0] + n, dtype=torch.int32, device=DEV).cumsum(0).to(torch.int32) for n in (lens_q, lens_k))
+    q, k, v = _bf16(sum(lens_q), hq, d), _bf16(sum(lens_k), hkv, d), _bf16(sum(lens_k), hkv, d)
+    go, scale = _bf16(*q.shape), 1 / math.sqrt(d)
+    out, lse = attention.flash_fwd(q, k, v, cu_q, cu_k, max(lens_q), scale, False)
+    got = attention.flash_bwd(go, q, k, v, out, lse, cu_q, max(lens_q), scale, cu_k=cu_k, max_k=max(lens_k), causal=False)
+    native.read_status(q.device)
+    ref_in = [t.float().requires_grad_(True) for t in (q, k, v)]
+    ref = R.varlen_attention(*ref_in, cu_q, scale, False, cu_k)
+    want = torch.autograd.grad(ref, ref_in, go.float())
+    for g, w in zip(got, want):   # P and dS are rounded to bf16 (2^-9 each) on the way, the result once more
+        assert (g.float() - w).norm() <= 4 * 2 ** -9 * w.norm()
+        assert (g.float() - w).abs().max() <= 2e-2 * w.abs().max()
