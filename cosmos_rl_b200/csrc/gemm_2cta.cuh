@@ -36,7 +36,7 @@ constexpr int G2_BM = 256;      // rows of the pair's tile
 constexpr int G2_BK = 64;
 constexpr int G2_THREADS = 192;
 
-enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3 };
+enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3, G2_EPI_LOGPROB = 4 };
 
 template <int BN, int STAGES>
 struct Gemm2Smem {
@@ -82,6 +82,55 @@ struct DlogitsRow {
   }
 };
 
+// G2_EPI_LOGPROB: the accumulator is a tile of logits (before the temperature), of which only four sums a row remain.
+struct LogprobParams {
+  const long long* labels;
+  float* partial;     // [T, nsplit, 4]
+  int T, V, nsplit;
+  float scale_log2;   // inv_temperature * log2(e): logits are tracked in the log2 domain
+};
+
+// One row's running maximum, sum of exponentials, label logit and sum of exponential * logit over the tiles of a unit.
+struct LogprobRow {
+  float m, l, z, e;
+  long long label;
+  __device__ __forceinline__ void begin(const LogprobParams& p, long long r) {
+    m = -INFINITY; l = 0.f; z = -INFINITY; e = 0.f;
+    label = r < p.T ? p.labels[r] : -1;
+  }
+  __device__ __forceinline__ void chunk(const LogprobParams& p, int c, const float (&v)[32]) {   // columns [c, c + 32)
+    if (c >= p.V) return;
+    float x[32];
+    float cmax = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      x[i] = (c + i < p.V) ? v[i] * p.scale_log2 : -INFINITY;
+      cmax = fmaxf(cmax, x[i]);
+    }
+    const float nm = fmaxf(m, cmax);
+    const float corr = exp2f(m - nm);  // m = -inf on the first chunk -> 0
+    float sl = 0.f, se = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      float pexp = exp2f(x[i] - nm);
+      sl += pexp;
+      se += (c + i < p.V) ? pexp * x[i] : 0.f;
+    }
+    l = l * corr + sl;
+    e = e * corr + se;
+    m = nm;
+    const long long off = label - c;
+    if (off >= 0 && off < 32) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (i == (int)off) z = x[i];
+    }
+  }
+  __device__ __forceinline__ void store(const LogprobParams& p, long long r, int split) const {
+    if (r < p.T) *reinterpret_cast<float4*>(p.partial + (r * p.nsplit + split) * 4) = make_float4(m, l, z, e);
+  }
+};
+
 struct Gemm2Params {
   const void* bias;  // [N] added to every row (nullable); bf16 when bias_bf16 else fp32
   int bias_bf16;
@@ -100,6 +149,7 @@ struct Gemm2Params {
   const int* offsets;
   const int* filled;
   int experts;
+  LogprobParams lg;  // G2_EPI_LOGPROB
 };
 
 // tile index -> (m_blk, n_blk): groups of `G` row blocks sweep all column blocks before the next group starts, so
@@ -181,6 +231,34 @@ struct G2ExpertWork {
   }
 };
 
+// G2_EPI_LOGPROB: a unit is a block of 256 rows and one of nsplit equal ranges of column tiles (batch), walked tile by tile. The
+// row blocks of a range run side by side, so that the weights of a tile come from HBM once.
+struct G2LogprobWork {
+  int num_m, num_n, num_kb, nsplit;
+  __device__ __forceinline__ void init(const Gemm2Params& ep, bool, int num_m_, int num_n_, int num_kb_) {
+    num_m = num_m_;
+    num_n = num_n_;
+    num_kb = num_kb_;
+    nsplit = ep.lg.nsplit;
+  }
+  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
+    for (int i = blockIdx.x >> 1; i < num_m * nsplit; i += gridDim.x >> 1) {
+      const int s = i / num_m, n0 = (int)((long long)s * num_n / nsplit), n1 = (int)((long long)(s + 1) * num_n / nsplit);
+      if (it < n1 - n0) {
+        u.m_blk = i - s * num_m;
+        u.n_blk = n0 + it;
+        u.batch = s;
+        u.kb0 = 0;
+        u.kb1 = num_kb;
+        u.cut = false;
+        return true;
+      }
+      it -= n1 - n0;
+    }
+    return false;
+  }
+};
+
 // TAIL: the rows of C end inside 16 bytes (a test in the epilogue of all kernels took 0.6 us of 33 x 3832 x 712 in fp32, 9.9).
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool TAIL>
 __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmC,
@@ -233,7 +311,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   constexpr int OUT_BN = (EPI == G2_EPI_SWIGLU) ? BN / 2 : BN;  // columns of C per tile
   const int n_cols = (EPI == G2_EPI_SWIGLU) ? N / 2 : N;        // columns of C
   const int num_n = (n_cols + OUT_BN - 1) / OUT_BN;
-  std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork, G2Work> work;
+  std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork, std::conditional_t<EPI == G2_EPI_LOGPROB, G2LogprobWork, G2Work>> work;
   work.init(ep, EPI == G2_EPI_STORE, num_m, num_n, (K + G2_BK - 1) / G2_BK);
   G2Unit unit;
 
@@ -342,6 +420,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
     uint32_t acc = 0, acc_phase = 0;
     uint32_t slab_idx = 0;
     const uint32_t sw = (uint32_t)(lane & 7);  // 128-byte swizzle: 16-byte chunk j of row r sits at chunk j ^ (r & 7)
+    LogprobRow lgr;
+    long long lg_row = -1;   // the row and the range that lgr is about
+    int lg_split = -1;
     for (int it = 0; work.get(it, unit) && !*abort_flag; ++it) {
       const int m_blk = unit.m_blk, n_blk = unit.n_blk;
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
@@ -359,6 +440,24 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       if constexpr (EPI == G2_EPI_DLOGITS) dlr.load(ep.dl, min(row0 + lane, M - 1));
       // a slab = 32 rows x 128 bytes of C: 64 bf16 or 32 fp32 columns
       const int slab_cols = out_fp32 ? 32 : 64;
+      if constexpr (EPI == G2_EPI_LOGPROB) {
+        if (row0 + lane != lg_row || unit.batch != lg_split) {
+          if (lg_split >= 0) lgr.store(ep.lg, lg_row, lg_split);
+          lg_row = row0 + lane;
+          lg_split = unit.batch;
+          lgr.begin(ep.lg, lg_row);
+        }
+#pragma unroll 1
+        for (int c = 0; c < BN; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(taddr + c, r);
+          tmem_ld_wait();
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          lgr.chunk(ep.lg, col_base + c, v);
+        }
+      } else
 #pragma unroll 1
       for (int c = 0; c < OUT_BN; c += slab_cols) {
         uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
@@ -454,6 +553,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc ? tempty_leader1 : tempty_leader0);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+    }
+    if constexpr (EPI == G2_EPI_LOGPROB) {
+      if (lg_split >= 0) lgr.store(ep.lg, lg_row, lg_split);
     }
     if (elect_one()) tma_store_wait<0>();
   }

@@ -3,7 +3,7 @@
 // reference (cosmos_rl/utils/util.py:314-366, 899-994) and feeds the GRPO loss
 // (cosmos_rl/policy/trainer/llm_trainer/grpo_trainer.py:113-353).
 //
-// Forward: work unit = (128-row block of tokens, vocabulary split). The CTA that owns a unit walks its
+// Forward: work unit = (block of tokens, vocabulary range). The CTA pair (up to 128 tokens: CTA) that owns a unit walks its
 // vocabulary tiles; each epilogue thread owns one token row and keeps an online-softmax state
 // (running max, sum of exp, label logit, sum exp*logit) in registers across tiles, written once per unit
 // to a [T, nsplit, 4] fp32 scratch that b200_logprob_combine reduces.
@@ -20,122 +20,81 @@ constexpr int LP_STAGES = 4;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 
+// Up to 128 rows: one CTA a tile, the vocabulary in as many ranges as there are CTAs (the pair form for more is an epilogue of
+// gemm_2cta.cuh).
 struct LogprobEpilogue {
-  struct Params {
-    const long long* labels;
-    float* partial;  // [T, nsplit, 4]
-    int T, V, nsplit, tps;
-    float scale_log2;  // inv_temperature * log2(e): logits are tracked in the log2 domain
-  };
-  float m, l, z, e;
-  int cur_unit_m = -1, cur_split = -1;
-  long long label;
-
-  __device__ __forceinline__ void flush(const Params& p, int row) {
-    if (cur_unit_m < 0) return;
-    long long r = (long long)cur_unit_m * GEMM_BM + row;
-    if (r < p.T) {
-      float4 o = make_float4(m, l, z, e);
-      *reinterpret_cast<float4*>(p.partial + (r * p.nsplit + cur_split) * 4) = o;
-    }
-  }
+  using Params = LogprobParams;
+  LogprobRow st;
+  int cur_split = -1;
   __device__ __forceinline__ void tile_begin(const Params& p, const TileInfo& t, int row) {
-    const int m_blk = t.m_blk, n_blk = t.n_blk;
-    int split = n_blk / p.tps;
-    if (m_blk != cur_unit_m || split != cur_split) {
-      flush(p, row);
-      cur_unit_m = m_blk;
-      cur_split = split;
-      m = -INFINITY; l = 0.f; z = -INFINITY; e = 0.f;
-      long long r = (long long)m_blk * GEMM_BM + row;
-      label = r < p.T ? p.labels[r] : -1;
-    }
+    if (t.batch == cur_split) return;
+    if (cur_split >= 0) st.store(p, row, cur_split);
+    cur_split = t.batch;
+    st.begin(p, row);
   }
-  __device__ __forceinline__ void chunk(const Params& p, const TileInfo& t, int row, int col0,
-                                        const float (&v)[32]) {
-    const int c = t.n_blk * LP_BN + col0;
-    if (c >= p.V) return;
-    float x[32];
-    float cmax = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      x[i] = (c + i < p.V) ? v[i] * p.scale_log2 : -INFINITY;
-      cmax = fmaxf(cmax, x[i]);
-    }
-    const float nm = fmaxf(m, cmax);
-    const float corr = exp2f(m - nm);  // m = -inf on the first chunk -> 0
-    float sl = 0.f, se = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      float pexp = exp2f(x[i] - nm);
-      sl += pexp;
-      se += (c + i < p.V) ? pexp * x[i] : 0.f;
-    }
-    l = l * corr + sl;
-    e = e * corr + se;
-    m = nm;
-    const long long off = label - c;
-    if (off >= 0 && off < 32) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (i == (int)off) z = x[i];
-    }
+  __device__ __forceinline__ void chunk(const Params& p, const TileInfo& t, int, int col0, const float (&v)[32]) {
+    st.chunk(p, t.n_blk * LP_BN + col0, v);
   }
   __device__ __forceinline__ void tile_end(const Params&, const TileInfo&, int) {}
   __device__ __forceinline__ void finish(const Params& p) {
-    const int quad = (threadIdx.x >> 5) & 3;
-    flush(p, quad * 32 + (threadIdx.x & 31));
+    if (cur_split >= 0) st.store(p, ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31), cur_split);
   }
 };
 
-// Work unit u = (token block, vocabulary split); CTA b owns units b, b+grid, ... and walks the tps
-// vocabulary tiles of each. n_blk may run past the last real tile in the final split: those tiles read
-// zero-filled weights and the epilogue masks every column >= V.
+// Range s (TileInfo::batch) of the vocabulary's tiles belongs to CTA s, s + grid, ...
 struct LogprobSched {
-  int num_m, tps, units, num_kb;
-  __device__ __forceinline__ void init(int M, int, int K, int, const LogprobEpilogue::Params& p) {
-    num_m = (M + GEMM_BM - 1) / GEMM_BM;
-    tps = p.tps;
-    units = num_m * p.nsplit;
+  int num_n, nsplit, num_kb;
+  __device__ __forceinline__ void init(int, int N, int K, int BN, const LogprobParams& p) {
+    num_n = (N + BN - 1) / BN;
+    nsplit = p.nsplit;
     num_kb = (K + GEMM_BK - 1) / GEMM_BK;
   }
   __device__ __forceinline__ bool get(int it, TileInfo& t) const {
-    int j = it / tps, i = it - j * tps;
-    int u = blockIdx.x + j * gridDim.x;
-    if (u >= units) return false;
-    t.m_blk = u % num_m;
-    t.n_blk = (u / num_m) * tps + i;
-    t.a_mn0 = t.m_blk * GEMM_BM;
-    t.b_mn0 = t.n_blk * LP_BN;
-    t.k0 = 0;
-    t.num_kb = num_kb;
-    t.batch = 0;
-    return true;
+    for (int s = blockIdx.x; s < nsplit; s += gridDim.x) {
+      const int n0 = (int)((long long)s * num_n / nsplit), n1 = (int)((long long)(s + 1) * num_n / nsplit);
+      if (it < n1 - n0) {
+        t.m_blk = 0;
+        t.n_blk = n0 + it;
+        t.a_mn0 = 0;
+        t.b_mn0 = t.n_blk * LP_BN;
+        t.k0 = 0;
+        t.num_kb = num_kb;
+        t.batch = s;
+        return true;
+      }
+      it -= n1 - n0;
+    }
+    return false;
   }
 };
 
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 lmhead_logprob_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int T, int V,
-                      int H, LogprobEpilogue::Params ep, uint32_t* status) {
+                      int H, LogprobParams ep, uint32_t* status) {
   gemm_mainloop<LP_BN, LP_STAGES, LogprobEpilogue, LogprobSched>(&tmA, &tmB, T, V, H, ep, status);
 }
 
+// One warp a row.
 __global__ void logprob_combine_kernel(const float* __restrict__ partial, const long long* __restrict__ labels,
                                        float* __restrict__ logprob, float* __restrict__ lse_out,
                                        float* __restrict__ entropy, int T, int nsplit) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= T) return;
   const float4* p = reinterpret_cast<const float4*>(partial) + (long long)r * nsplit;
-  float M = -INFINITY;
-  for (int s = 0; s < nsplit; ++s) M = fmaxf(M, p[s].x);
-  float L = 0.f, E = 0.f, Z = -INFINITY;
-  for (int s = 0; s < nsplit; ++s) {
-    float4 q = p[s];
-    float c = exp2f(q.x - M);
-    L += q.y * c;
-    E += q.w * c;
+  float M = -INFINITY, L = 0.f, E = 0.f, Z = -INFINITY;
+  auto add = [&](const float4& q) {   // the larger maximum stays as it is, whoever has it
+    const float nm = fmaxf(M, q.x), a = M == nm ? 1.f : exp2f(M - nm), c = q.x == nm ? 1.f : exp2f(q.x - nm);
+    L = L * a + q.y * c;
+    E = E * a + q.w * c;
     Z = fmaxf(Z, q.z);
-  }
+    M = nm;
+  };
+  for (int s = lane; s < nsplit; s += 32) add(p[s]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    add(make_float4(__shfl_xor_sync(0xffffffffu, M, o), __shfl_xor_sync(0xffffffffu, L, o), __shfl_xor_sync(0xffffffffu, Z, o),
+                    __shfl_xor_sync(0xffffffffu, E, o)));
+  if (lane != 0) return;
   // convert from the log2 domain back to natural log
   const float lse2 = M + log2f(L);
   if (lse_out) lse_out[r] = lse2 * LN2;
@@ -202,8 +161,27 @@ int b200_lmhead_logprob_partial(const void* hidden, const void* weight, const lo
                                 int nsplit, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (T <= 0 || V <= 0 || H <= 0 || (H & 7) || nsplit <= 0) return B200_ERR_ARG;
+  const int num_n = (V + LP_BN - 1) / LP_BN;
+  if (nsplit > num_n) return B200_ERR_ARG;
+  const LogprobParams lg{labels, partial, T, V, nsplit, inv_temperature * LOG2E};
   CUtensorMap tmA, tmB;
   if (make_tmap_2d(&tmA, hidden, T, H, ldh, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  // The logits are formed at the rate of the dense GEMM: CTA pairs once there are rows for their 256-row tiles. 2048 x 152064 x
+  // 3584: 1458 us, with one CTA a tile, whose operand traffic bounds it, 1666; 200 rows 221 and 268.
+  if (T > GEMM_BM) {
+    using SM = Gemm2Smem<LP_BN, 6>;
+    if (make_tmap_2d(&tmB, weight, V, H, ldw, LP_BN / 2, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+    auto kern = gemm2_bf16_kernel<LP_BN, 6, false, false, G2_EPI_LOGPROB>;
+    static int whole[16] = {0};
+    int np = 0;
+    if (const int rc = resident_pairs(kern, whole, SM::TOTAL, G2_THREADS, num_sms, np)) return rc;
+    Gemm2Params ep{};
+    ep.a_bytes = SM::A_BYTES;
+    ep.lg = lg;
+    const long long units = (long long)((T + G2_BM - 1) / G2_BM) * nsplit;
+    kern<<<2 * (int)(units < np ? units : np), G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmB, tmB, T, V, H, ep, status);
+    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  }
   if (make_tmap_2d(&tmB, weight, V, H, ldw, LP_BN, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   using SM = GemmSmem<LP_BN, LP_STAGES>;
   static bool attr_set = false;
@@ -213,20 +191,14 @@ int b200_lmhead_logprob_partial(const void* hidden, const void* weight, const lo
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  const int num_m = (T + GEMM_BM - 1) / GEMM_BM;
-  const int num_n = (V + LP_BN - 1) / LP_BN;
-  if (nsplit > num_n) return B200_ERR_ARG;
-  LogprobEpilogue::Params ep{labels, partial, T, V, nsplit, (num_n + nsplit - 1) / nsplit, inv_temperature * LOG2E};
-  int units = num_m * nsplit;
-  int grid = units < num_sms ? units : num_sms;
-  lmhead_logprob_kernel<<<grid, GEMM_THREADS, SM::TOTAL, stream>>>(tmA, tmB, T, V, H, ep, status);
+  lmhead_logprob_kernel<<<nsplit < num_sms ? nsplit : num_sms, GEMM_THREADS, SM::TOTAL, stream>>>(tmA, tmB, T, V, H, lg, status);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 
 int b200_logprob_combine(const float* partial, const long long* labels, float* logprob, float* lse, float* entropy,
                          int T, int nsplit, cudaStream_t stream) {
   if (T <= 0) return 0;
-  b200::logprob_combine_kernel<<<(T + 127) / 128, 128, 0, stream>>>(partial, labels, logprob, lse, entropy, T, nsplit);
+  b200::logprob_combine_kernel<<<(T + 7) / 8, 256, 0, stream>>>(partial, labels, logprob, lse, entropy, T, nsplit);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 

@@ -512,14 +512,17 @@ def skinny_qkv_rope_append(x2: torch.Tensor, qkv_weight: torch.Tensor, bias: Opt
 # --------------------------------------------------------------------------------------------------
 # fused lm_head + log-prob + entropy
 # --------------------------------------------------------------------------------------------------
+@functools.lru_cache(maxsize=1024)
 def _pick_nsplit(T: int, V: int, sms: int) -> int:
-    num_m = (T + 127) // 128
+    """Ranges of the vocabulary: CTA pairs (up to 128 rows: CTAs) take units of a row block and a range one after the other."""
+    rows, slots = (256, max(1, sms // 2)) if T > 128 else (128, sms)
+    num_m = (T + rows - 1) // rows
     num_n = (V + 255) // 256
     best, best_score = 1, -1.0
-    for ns in range(1, min(num_n, 64) + 1):
+    for ns in range(1, min(num_n, max(64, slots)) + 1):
         units = num_m * ns
-        waves = math.ceil(units / sms)
-        eff = units / (waves * sms)
+        waves = math.ceil(units / slots)
+        eff = units / (waves * slots)
         # prefer full waves, then fewer splits (less scratch, fewer partial merges)
         score = eff - 0.002 * ns
         if score > best_score:

@@ -1877,3 +1877,23 @@ def test_flash_attention_backward_items_without_keys_between_others():
     for g, w in zip(got, want):   # P and dS are rounded to bf16 (2^-9 each) on the way, the result once more
         assert (g.float() - w).norm() <= 4 * 2 ** -9 * w.norm()
         assert (g.float() - w).abs().max() <= 2e-2 * w.abs().max()
+
+
+@pytest.mark.parametrize("T,V,H", [(1, 40009, 64), (128, 1500, 136), (129, 257, 64), (256, 40009, 72), (300, 20001, 64), (777, 255, 64)])
+def test_fused_logprob_ranges(T, V, H):
+    """Rows around the tiles of both forms; a vocabulary with fewer tiles than CTAs, with more, and with a last tile of one column;
+    a CTA pair whose ranges belong to two row blocks."""
+    torch.manual_seed(89)
+    h, w = _bf16(T, H), _bf16(V, H, scale=0.3)
+    labels = torch.randint(0, V, (T,), device=DEV)
+    labels[-1], labels[0] = V - 1, -100 if T > 1 else 0
+    lp, ent = F.fused_logprob(h, w, labels, 0.8)
+    native.read_status(h.device)
+    logits = h.double() @ w.double().t() / 0.8
+    lse = logits.logsumexp(-1)
+    want = torch.where(labels >= 0, logits.gather(-1, labels.clamp_min(0)[:, None])[:, 0] - lse, 0.)
+    want_ent = lse - ((logits - lse[:, None]).exp() * logits).sum(-1)
+    # a logit is an fp32 sum of H products; the sums over the vocabulary are relative to their largest term
+    logit = 2.0 ** -20 * (h.double().norm(dim=1) * w.double().norm(dim=1).max()) / 0.8
+    assert ((lp.double() - want).abs() <= 2 * logit + 1e-5 * (1 + lse.abs())).all()
+    assert ((ent.double() - want_ent).abs() <= (2 + logits.abs().amax(-1)) * (2 * logit + 1e-5)).all()
