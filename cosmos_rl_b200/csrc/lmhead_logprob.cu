@@ -82,18 +82,22 @@ __global__ void logprob_combine_kernel(const float* __restrict__ partial, const 
   if (r >= T) return;
   const float4* p = reinterpret_cast<const float4*>(partial) + (long long)r * nsplit;
   float M = -INFINITY, L = 0.f, E = 0.f, Z = -INFINITY;
-  auto add = [&](const float4& q) {   // the larger maximum stays as it is, whoever has it
-    const float nm = fmaxf(M, q.x), a = M == nm ? 1.f : exp2f(M - nm), c = q.x == nm ? 1.f : exp2f(q.x - nm);
-    L = L * a + q.y * c;
-    E = E * a + q.w * c;
-    Z = fmaxf(Z, q.z);
-    M = nm;
-  };
-  for (int s = lane; s < nsplit; s += 32) add(p[s]);
+  for (int s = lane; s < nsplit; s += 32) M = fmaxf(M, p[s].x);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    add(make_float4(__shfl_xor_sync(0xffffffffu, M, o), __shfl_xor_sync(0xffffffffu, L, o), __shfl_xor_sync(0xffffffffu, Z, o),
-                    __shfl_xor_sync(0xffffffffu, E, o)));
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  for (int s = lane; s < nsplit; s += 32) {
+    const float4 q = p[s];
+    const float c = exp2f(q.x - M);
+    L += q.y * c;
+    E += q.w * c;
+    Z = fmaxf(Z, q.z);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    L += __shfl_xor_sync(0xffffffffu, L, o);
+    E += __shfl_xor_sync(0xffffffffu, E, o);
+    Z = fmaxf(Z, __shfl_xor_sync(0xffffffffu, Z, o));
+  }
   if (lane != 0) return;
   // convert from the log2 domain back to natural log
   const float lse2 = M + log2f(L);
