@@ -17,26 +17,15 @@ from .functional import needs_graph
 
 
 def native_flash_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
-    return (q.is_cuda and q.dtype == torch.bfloat16 and q.shape[-1] == 128 and q.stride(-1) == 1
-            and k.stride(-1) == 1 and v.stride(-1) == 1 and q.stride(1) == 128 and k.stride(1) == 128
-            and v.stride(1) == 128 and q.stride(0) % 8 == 0 and k.stride(0) % 8 == 0 and v.stride(0) % 8 == 0
-            and q.shape[1] % k.shape[1] == 0)
+    return q.is_cuda and native.host().flash_ok(q, k, v)
 
 
 def flash_fwd(q, k, v, cu_q, cu_k, max_q: int, scale: float, causal: bool = True
               ) -> Tuple[torch.Tensor, torch.Tensor]:
     """q [Tq, hq, 128], k / v [Tk, hkv, 128] (token-strided views are fine). Returns (out [Tq, hq, 128] bf16,
     lse [hq, Tq] fp32)."""
-    Tq, hq, d = q.shape
-    Tk, hkv = k.shape[0], k.shape[1]
-    out = torch.empty(Tq, hq, d, dtype=q.dtype, device=q.device)
-    lse = torch.empty(hq, Tq, dtype=torch.float32, device=q.device)
-    native.check(native.lib().b200_flash_fwd(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), cu_q.data_ptr(), cu_k.data_ptr(),
-        cu_q.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0), v.stride(0), hq * d, int(max_q),
-        1 if causal else 0, float(scale), native.status_word(q.device).data_ptr(), native.num_sms(q.device.index),
-        native.stream()), "flash_fwd")
-    return out, lse
+    return native.tensors(native.host().flash_fwd(q, k, v, cu_q, cu_k, max_q, causal, scale, native.status_word(q.device),
+                                                  native.num_sms(q.device.index), native.stream()), "flash_fwd")
 
 
 class _FlashAttn(torch.autograd.Function):
@@ -83,12 +72,11 @@ def flash_bwd(dout, q, k, v, out, lse, cu, max_seqlen: int, scale: float, cu_k=N
     dv = torch.empty(Tk, hkv, d, dtype=v.dtype, device=q.device)
     delta = torch.empty(hq, Tq, dtype=torch.float32, device=q.device)
     st = native.status_word(q.device)
-    native.check(native.lib().b200_flash_bwd(
-        native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(out), native.ptr(dout), native.ptr(lse),
-        native.ptr(dq), native.ptr(dk), native.ptr(dv), native.ptr(delta), native.ptr(cu), native.ptr(cu_k),
-        cu.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0), v.stride(0), out.stride(0), dout.stride(0),
-        dq.stride(0), dk.stride(0), dv.stride(0), int(max_seqlen), int(max_k if max_k is not None else max_seqlen),
-        1 if causal else 0, float(scale), native.ptr(st), native.num_sms(q.device.index), native.stream()), "flash_bwd")
+    native.check(native.host().b200_flash_bwd(
+        q, k, v, out, dout, lse, dq, dk, dv, delta, cu, cu_k, cu.numel() - 1, Tq, Tk, hq, hkv, d, q.stride(0), k.stride(0),
+        v.stride(0), out.stride(0), dout.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), int(max_seqlen),
+        int(max_k if max_k is not None else max_seqlen), 1 if causal else 0, scale, st, native.num_sms(q.device.index),
+        native.stream()), "flash_bwd")
     return dq, dk, dv
 
 

@@ -1,8 +1,9 @@
-"""In-tree build of the sm_100a kernel library (``libb200rl.so``).
+"""In-tree build of the sm_100a kernel library (``libb200rl.so``) and of its entry points that take tensors (``_host.so``).
 
 Every ``csrc/*.cu`` is compiled with ``nvcc -gencode arch=compute_100a,code=sm_100a`` into an object file and
 linked into one shared library next to this module, so the library travels with the source tree and is
-loaded with ``ctypes`` (no torch C++ headers are involved, a full rebuild takes well under a minute).
+loaded with ``ctypes``; no torch C++ headers are involved. ``csrc/host.cpp`` is one file against torch's headers and becomes a
+Python extension beside it, built again when torch or Python change. A full rebuild takes well under a minute.
 Run ``python -m cosmos_rl_b200.ops.build`` or call :func:`build`.
 """
 from __future__ import annotations
@@ -13,11 +14,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent.parent / "csrc"
 OUT_DIR = Path(__file__).resolve().parent
 LIB_NAME = "libb200rl.so"
+HOST_NAME = "_host.so"
 OBJ_DIR = OUT_DIR / "build"
 
 NVCC_FLAGS = [
@@ -34,13 +37,18 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or put it on PATH")
 
 
-def _digest(paths) -> str:
+def _digest(paths, flags) -> str:
     h = hashlib.sha256()
     for p in sorted(paths):
         h.update(p.name.encode())
         h.update(p.read_bytes())
-    h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(" ".join(flags).encode())
     return h.hexdigest()
+
+
+def _fresh(target: Path, digest: str) -> bool:
+    stamp = OUT_DIR / (target.name + ".sha256")
+    return target.exists() and stamp.exists() and stamp.read_text().strip() == digest
 
 
 def sources():
@@ -56,9 +64,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     srcs = sources()
     headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h"))
     stamp = OUT_DIR / (LIB_NAME + ".sha256")
-    digest = _digest(srcs + headers)
+    digest = _digest(srcs + headers, NVCC_FLAGS)
     lib = lib_path()
-    if not force and lib.exists() and stamp.exists() and stamp.read_text().strip() == digest:
+    if not force and _fresh(lib, digest):
+        build_host(force)
         return lib
     OBJ_DIR.mkdir(exist_ok=True)
     nvcc = _nvcc()
@@ -82,7 +91,33 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     stamp.write_text(digest)
+    build_host(force)
     return lib
+
+
+def host_path() -> Path:
+    return OUT_DIR / HOST_NAME
+
+
+def build_host(force: bool = False) -> Path:
+    """Compile (if stale) the extension of ``csrc/host.cpp``; the kernel library has been built."""
+    import torch
+    src, ext = CSRC / "host.cpp", host_path()
+    root = Path(torch.__file__).resolve().parent
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    digest = _digest([src, CSRC / "api.h"], flags + [torch.__version__, sys.version])
+    if not force and _fresh(ext, digest):
+        return ext
+    cuda = Path(_nvcc()).resolve().parent.parent
+    include = [root / "include", root / "include/torch/csrc/api/include", sysconfig.get_paths()["include"], cuda / "include", CSRC]
+    cmd = ["g++", *flags, *(f"-I{d}" for d in include), str(src), "-o", str(ext), f"-L{root / 'lib'}", "-ltorch_python",
+           "-ltorch_cpu", "-ltorch", "-lc10", f"-L{OUT_DIR}", f"-l:{LIB_NAME}", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+    (OUT_DIR / (HOST_NAME + ".sha256")).write_text(digest)
+    return ext
 
 
 if __name__ == "__main__":

@@ -45,50 +45,38 @@ def needs_graph(*tensors: Optional[torch.Tensor]) -> bool:
 # RMSNorm
 # --------------------------------------------------------------------------------------------------
 def _rmsnorm_fwd(x2, weight, eps, res2, rstd):
-    y = torch.empty_like(x2)
-    res_out = torch.empty_like(x2) if res2 is not None else None
-    T, H = x2.shape
-    native.check(native.lib().b200_rmsnorm_fwd(x2.data_ptr(), native.ptr(res2), weight.data_ptr(), y.data_ptr(),
-                                               native.ptr(res_out), native.ptr(rstd), T, H, eps, native.stream()),
-                 "rmsnorm_fwd")
-    return y, res_out
+    return native.tensors(native.host().rmsnorm_fwd(x2, weight, eps, res2, rstd, native.stream()), "rmsnorm_fwd")
+
+
+def _rows_like(residual, x2):
+    """``residual`` as contiguous rows of x2's length; raises unless it has such."""
+    residual = _c(residual)
+    return residual if residual.shape == x2.shape else residual.view(-1, x2.shape[1])
 
 
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps, residual):
         shape = x.shape
-        H = shape[-1]
-        x2 = _c(x).view(-1, H)
-        T = x2.shape[0]
-        res2 = _c(residual).view(-1, H) if residual is not None else None
-        rstd = torch.empty(T, dtype=torch.float32, device=x.device)
+        x2 = _rows(x)
+        res2 = _rows_like(residual, x2) if residual is not None else None
+        rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
         y, res_out = _rmsnorm_fwd(x2, weight, eps, res2, rstd)
-        h = res_out if residual is not None else x2
-        ctx.save_for_backward(h, weight, rstd)
-        ctx.has_res = residual is not None
+        ctx.save_for_backward(res_out if res2 is not None else x2, weight, rstd)
+        ctx.has_res = res2 is not None
         ctx.shape = shape
-        if residual is not None:
-            return y.view(shape), res_out.view(shape)
-        return y.view(shape), None
+        if len(shape) == 2:
+            return y, res_out
+        return y.view(shape), (res_out.view(shape) if res2 is not None else None)
 
     @staticmethod
     def backward(ctx, dy, dres_out):
         h, weight, rstd = ctx.saved_tensors
-        H = h.shape[-1]
-        T = h.shape[0]
-        dy2 = _c(dy).view(-1, H)
-        dres2 = _c(dres_out).view(-1, H) if dres_out is not None else None
-        dx = torch.empty_like(h)
-        dw = ws = None
-        if ctx.needs_input_grad[1]:
-            dw = torch.empty(H, dtype=torch.bfloat16, device=h.device)
-            ws = torch.empty(_NORM_WS_ROWS * max(H, 1024), dtype=torch.float32, device=h.device)
-        native.check(native.lib().b200_rmsnorm_bwd2(native.ptr(dy2), native.ptr(h), native.ptr(weight),
-                                                    native.ptr(rstd), native.ptr(dres2), native.ptr(dx),
-                                                    native.ptr(dw), native.ptr(ws), T, H, native.stream()), "rmsnorm_bwd")
-        dxv = dx.view(ctx.shape)
-        return dxv, dw, None, (dxv if ctx.has_res else None)
+        dx, dw = native.tensors(native.host().rmsnorm_bwd(dy, h, weight, rstd, dres_out, ctx.needs_input_grad[1], _NORM_WS_ROWS,
+                                                          native.stream()), "rmsnorm_bwd")
+        if len(ctx.shape) != 2:
+            dx = dx.view(ctx.shape)
+        return dx, dw, None, (dx if ctx.has_res else None)
 
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: Optional[torch.Tensor] = None):
@@ -99,9 +87,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual:
         if not needs_graph(x, weight, residual):
             x2 = _rows(x)
             if residual is not None:
-                residual = _c(residual)
-                if residual.shape != x2.shape:
-                    residual = residual.view(-1, x2.shape[1])     # raises unless it has rows of this length
+                residual = _rows_like(residual, x2)
             y, res_out = _rmsnorm_fwd(x2, weight, eps, residual, None)
             if x.dim() == 2:
                 return y, res_out
@@ -119,10 +105,20 @@ def _rope_native(q, k, positions, theta, backward):
     assert q.stride(-1) == 1 and q.stride(1) == d
     if k is not None:
         assert k.stride(-1) == 1 and k.stride(1) == d
-    L = native.lib()
-    native.check(L.b200_rope_inplace(native.ptr(q), native.ptr(k), native.ptr(positions), T, hq, hkv, d, q.stride(0),
-                                     k.stride(0) if k is not None else 0, float(theta), 1 if backward else 0,
-                                     native.stream()), "rope")
+    native.check(native.host().b200_rope_inplace(q, k, positions, T, hq, hkv, d, q.stride(0),
+                                                 k.stride(0) if k is not None else 0, theta, 1 if backward else 0,
+                                                 native.stream()), "rope")
+
+
+def _rope_qkv_native(qkv, positions, hq, hkv, d, theta, backward):
+    """The q and k columns of a fused projection, in place."""
+    rc = native.host().rope_qkv(qkv, positions, hq, hkv, d, theta, backward, native.stream())
+    if rc is not None:
+        native.check(rc, "rope")
+        return
+    q = qkv[:, : hq * d].unflatten(-1, (hq, d))
+    k = qkv[:, hq * d: (hq + hkv) * d].unflatten(-1, (hkv, d))
+    _rope_native(q, k, positions, theta, backward)
 
 
 class _RoPE(torch.autograd.Function):
@@ -161,10 +157,7 @@ class _RoPEQKV(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, positions, hq, hkv, d, theta):
-        T = qkv.shape[0]
-        q = qkv[:, : hq * d].unflatten(-1, (hq, d))
-        k = qkv[:, hq * d: (hq + hkv) * d].unflatten(-1, (hkv, d))
-        _rope_native(q, k, positions, theta, False)
+        _rope_qkv_native(qkv, positions, hq, hkv, d, theta, False)
         ctx.mark_dirty(qkv)
         ctx.save_for_backward(positions)
         ctx.cfg = (hq, hkv, d, theta)
@@ -175,9 +168,7 @@ class _RoPEQKV(torch.autograd.Function):
         (positions,) = ctx.saved_tensors
         hq, hkv, d, theta = ctx.cfg
         dqkv = dqkv.clone(memory_format=torch.contiguous_format)
-        q = dqkv[:, : hq * d].unflatten(-1, (hq, d))
-        k = dqkv[:, hq * d: (hq + hkv) * d].unflatten(-1, (hkv, d))
-        _rope_native(q, k, positions, theta, True)
+        _rope_qkv_native(dqkv, positions, hq, hkv, d, theta, True)
         return dqkv, None, None, None, None, None
 
 
@@ -188,13 +179,7 @@ def rope_qkv_(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: 
         positions = positions.to(torch.int64)
         if torch.is_grad_enabled() and qkv.requires_grad:
             return _RoPEQKV.apply(qkv, positions, hq, hkv, d, theta)
-        if qkv.shape[1] == (hq + 2 * hkv) * d and qkv.is_contiguous():
-            heads = qkv.view(qkv.shape[0], hq + 2 * hkv, d)
-            q, k = heads[:, :hq], heads[:, hq: hq + hkv]
-        else:
-            q = qkv[:, : hq * d].unflatten(-1, (hq, d))
-            k = qkv[:, hq * d: (hq + hkv) * d].unflatten(-1, (hkv, d))
-        _rope_native(q, k, positions, theta, False)
+        _rope_qkv_native(qkv, positions, hq, hkv, d, theta, False)
         return qkv
     T = qkv.shape[0]
     q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=-1)
@@ -206,30 +191,23 @@ def rope_qkv_(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: 
 # SwiGLU
 # --------------------------------------------------------------------------------------------------
 def _swiglu_fwd(gu):
-    out = torch.empty(gu.shape[0], gu.shape[1] // 2, dtype=gu.dtype, device=gu.device)
-    native.check(native.lib().b200_swiglu_fwd(native.ptr(gu), native.ptr(out), gu.shape[0], gu.shape[1] // 2, None,
-                                              native.stream()), "swiglu_fwd")
-    return out
+    return native.tensors(native.host().swiglu_fwd(gu, native.stream()), "swiglu_fwd")
 
 
 class _SwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate_up):
-        I2 = gate_up.shape[-1]
-        gu = _c(gate_up).view(-1, I2)
+        gu = _rows(gate_up)
         out = _swiglu_fwd(gu)
         ctx.save_for_backward(gu)
         ctx.shape = gate_up.shape
-        return out.view(*gate_up.shape[:-1], I2 // 2)
+        return out if gate_up.dim() == 2 else out.view(*gate_up.shape[:-1], out.shape[1])
 
     @staticmethod
     def backward(ctx, dout):
         (gu,) = ctx.saved_tensors
-        d2 = _c(dout).view(-1, gu.shape[1] // 2)
-        dgu = torch.empty_like(gu)
-        native.check(native.lib().b200_swiglu_bwd(native.ptr(d2), native.ptr(gu), native.ptr(dgu), gu.shape[0],
-                                                  gu.shape[1] // 2, None, native.stream()), "swiglu_bwd")
-        return dgu.view(ctx.shape)
+        dgu = native.tensors(native.host().swiglu_bwd(dout, gu, native.stream()), "swiglu_bwd")
+        return dgu if len(ctx.shape) == 2 else dgu.view(ctx.shape)
 
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
@@ -262,9 +240,9 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     return out
 
 
-@functools.lru_cache(maxsize=4096)
 def _gemm_scratch(M: int, N: int, K: int, a_mn: bool, rows16: bool, out_fp32: bool, accumulate: bool, bias: bool, swiglu: bool,
                   path: int, sms: int) -> int:
+    """Values of fp32 scratch that such a call of :func:`gemm` takes while it runs."""
     return native.lib().b200_gemm_scratch(M, N, K, a_mn, rows16, out_fp32, accumulate, bias, swiglu, path, sms)
 
 
@@ -281,44 +259,28 @@ def gemm(a: torch.Tensor, b: torch.Tensor, a_mn: bool = False, b_mn: bool = Fals
     The same call gives the same bits again. Which values are summed in one go and which in shares depends on M, N, K and the
     number of SMs, so a row may come out different in the last place in a call of another size. ``accumulate`` adds value by
     value in memory above 128 rows; with fewer ``out`` is read and written, and nothing else may add to it meanwhile."""
-    assert a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    assert a.stride(-1) == 1 and b.stride(-1) == 1 and a.dim() == 2 and b.dim() == 2
-    K, M = (a.shape[0], a.shape[1]) if a_mn else (a.shape[1], a.shape[0])
-    Kb, N = (b.shape[0], b.shape[1]) if b_mn else (b.shape[1], b.shape[0])
-    assert K == Kb, (a.shape, b.shape, a_mn, b_mn)
-    if out is None:
-        out = torch.empty(M, N // 2 if swiglu else N, dtype=out_dtype, device=a.device)
-    if bias is not None:
-        assert bias.is_contiguous() and bias.numel() == N and bias.dtype in (torch.bfloat16, torch.float32)
-    dev = a.device.index if a.device.index is not None else torch.cuda.current_device()
-    sms, out_fp32 = native.num_sms(dev), out.dtype == torch.float32
-    rows16 = (out.data_ptr() | out.stride(0) * out.element_size()) % 16 == 0
-    floats, ws = _gemm_scratch(M, N, K, a_mn, rows16, out_fp32, accumulate, bias is not None, swiglu, path, sms), None
+    assert a.is_cuda
+    dev = a.device
+    st, sms = native.status_word(dev), native.num_sms(dev.index)
 
-    def call(cut):
-        return native.lib().b200_gemm_bf16_ws(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), int(a_mn), int(b_mn),
-            int(out_fp32), int(accumulate), native.ptr(bias), int(bias is not None and bias.dtype == torch.bfloat16), int(swiglu),
-            N // 2 if swiglu else 0, path, cut, native.ptr(ws), floats, native.status_word(a.device).data_ptr(), sms,
-            native.stream())
+    def call(ws, floats):
+        return native.host().gemm(a, b, a_mn, b_mn, out, out_dtype == torch.float32, accumulate, bias, swiglu, path, ws, floats, st,
+                                  sms, native.stream())
 
-    if floats:      # the last round of tiles is cut along the contraction; it stays whole where there is no room for that
+    r = call(None, -1)
+    if type(r) is int and r > native.NEED_WORKSPACE:
+        # the last round of tiles is cut along the contraction, in so many values of scratch; it stays whole where there is no room
         try:
-            ws = torch.empty(floats, dtype=torch.float32, device=a.device)
+            ws, floats = torch.empty(r, dtype=torch.float32, device=dev), r
         except torch.cuda.OutOfMemoryError:
-            floats = 0
-    rc = call(1)
-    if rc == native.NEED_WORKSPACE:
-        rc = call(0)
-    native.check(rc, "gemm_bf16")
-    return out
+            ws, floats = None, 0
+        r = call(ws, floats)
+    return native.tensors(r, "gemm_bf16")
 
 
 def _tc_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """The tensor-core GEMMs move rows with TMA: feature dimensions must give 16-byte rows."""
-    return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
-            and weight.stride(-1) == 1 and weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0
-            and weight.stride(0) % 8 == 0)
+    return x.is_cuda and native.host().linear_ok(x, weight)
 
 
 class _LinearTC(torch.autograd.Function):
@@ -328,11 +290,11 @@ class _LinearTC(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias):
-        x2 = _c(x).view(-1, x.shape[-1])
+        x2 = _rows(x)
         # the result is allocated in its final shape: callers rotate / scale it in place, which autograd forbids on
         # a view returned by a custom function
         y = torch.empty(*x.shape[:-1], weight.shape[0], dtype=torch.bfloat16, device=x.device)
-        y2 = y.view(-1, weight.shape[0])
+        y2 = y if y.dim() == 2 else y.view(-1, weight.shape[0])
         gemm(x2, weight, out=y2, bias=bias if (bias is not None and x2.shape[0] > 128) else None)
         if bias is not None and x2.shape[0] <= 128:
             y2 += bias
@@ -344,7 +306,7 @@ class _LinearTC(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x2, weight = ctx.saved_tensors
-        dy2 = _c(dy).view(-1, weight.shape[0])
+        dy2 = _rows(dy)
         dx = gemm(dy2, weight, b_mn=True) if ctx.needs_input_grad[0] else None
         dw = None
         if ctx.needs_input_grad[1]:
@@ -355,7 +317,7 @@ class _LinearTC(torch.autograd.Function):
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True)
         db = dy2.sum(0) if ctx.has_bias and ctx.needs_input_grad[2] else None
-        return (dx.view(ctx.shape) if dx is not None else None), dw, db
+        return (dx.view(ctx.shape) if dx is not None and len(ctx.shape) != 2 else dx), dw, db
 
 
 def linear_tc(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -429,17 +391,15 @@ def _skinny_launch(x2, weight, N, swiglu, out, use_ws, bias=None):
     assert x2.stride(-1) == 1 and weight.stride(-1) == 1
     dev = x2.device.index if x2.device.index is not None else torch.cuda.current_device()
     sms = native.num_sms(dev)
-    L = native.lib()
+    L = native.host()
     splits = 1 if swiglu else L.b200_gemm_skinny_splits(M, N, K, 0, sms)
     ws = _skinny_workspace(x2.device) if (use_ws or splits > 1) else None
     if ws is not None:
         assert splits * M * N <= ws.numel()
-    st = native.status_word(x2.device)
-    native.check(L.b200_gemm_skinny(native.ptr(x2), native.ptr(weight), native.ptr(out) if ws is None else None,
-                                    native.ptr(ws), M, N, K, x2.stride(0), weight.stride(0),
-                                    out.stride(0) if out is not None else 0, native.ptr(bias),
+    native.check(L.b200_gemm_skinny(x2, weight, out if ws is None else None, ws, M, N, K, x2.stride(0), weight.stride(0),
+                                    out.stride(0) if out is not None else 0, bias,
                                     1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
-                                    1 if swiglu else 0, N if swiglu else 0, splits, native.ptr(st), sms,
+                                    1 if swiglu else 0, N if swiglu else 0, splits, native.status_word(x2.device), sms,
                                     native.stream()), "gemm_skinny")
     return ws, splits
 
@@ -447,25 +407,17 @@ def _skinny_launch(x2, weight, N, swiglu, out, use_ws, bias=None):
 def gemm_skinny(x2: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x2 [M <= 256, K] @ weight [N, K]^T (+ bias)`` in bf16 on the weight-streaming kernel."""
-    (M, K), N = x2.shape, weight.shape[0]
-    assert x2.is_cuda and x2.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and M <= _SKINNY_MAX_M
-    assert x2.stride(-1) == 1 and weight.stride(-1) == 1
-    if out is None:
-        out = torch.empty(M, N, dtype=torch.bfloat16, device=x2.device)
-    dev, strm = x2.device.index, native.stream()
+    assert x2.is_cuda
+    dev, strm = x2.device, native.stream()
+    st, sms = native.status_word(dev), native.num_sms(dev.index)
 
     def call(ws):
-        return native.lib().b200_skinny_linear(x2.data_ptr(), weight.data_ptr(), native.ptr(bias),
-                                               1 if bias is not None and bias.dtype == torch.bfloat16 else 0,
-                                               out.data_ptr(), native.ptr(ws), 0 if ws is None else _SKINNY_WS_FLOATS, M, N,
-                                               K, x2.stride(0), weight.stride(0), out.stride(0),
-                                               native.status_word(x2.device).data_ptr(), native.num_sms(dev), strm)
+        return native.host().skinny_linear(x2, weight, bias, out, ws, _SKINNY_MAX_M, st, sms, strm)
 
-    rc = call(_skinny_ws.get((dev, strm)))
-    if rc == native.NEED_WORKSPACE:     # the first shape on this stream whose contraction is split
-        rc = call(_skinny_workspace(x2.device))
-    native.check(rc, "gemm_skinny")
-    return out
+    r = call(_skinny_ws.get((dev.index, strm)))
+    if type(r) is int and r == native.NEED_WORKSPACE:     # the first shape on this stream whose contraction is split
+        r = call(_skinny_workspace(dev))
+    return native.tensors(r, "gemm_skinny")
 
 
 def skinny_gate_up_swiglu(x2: torch.Tensor, gate_up_weight: torch.Tensor) -> torch.Tensor:
@@ -485,10 +437,8 @@ def skinny_linear_residual_rmsnorm(x2: torch.Tensor, weight: torch.Tensor, resid
     y = torch.empty(M, H, dtype=torch.bfloat16, device=x2.device)
     res_out = torch.empty_like(y)
     assert norm_weight.dtype == torch.bfloat16 and (residual is None or residual.is_contiguous())
-    native.check(native.lib().b200_splitk_reduce_residual_rmsnorm(native.ptr(ws), splits, M, H, native.ptr(residual),
-                                                                  native.ptr(norm_weight), float(eps),
-                                                                  native.ptr(res_out), native.ptr(y), native.stream()),
-                 "splitk_reduce_residual_rmsnorm")
+    native.check(native.host().b200_splitk_reduce_residual_rmsnorm(ws, splits, M, H, residual, norm_weight, eps, res_out, y,
+                                                                   native.stream()), "splitk_reduce_residual_rmsnorm")
     return y, res_out
 
 
@@ -501,11 +451,9 @@ def skinny_qkv_rope_append(x2: torch.Tensor, qkv_weight: torch.Tensor, bias: Opt
     assert N == (hq + 2 * hkv) * d and positions.dtype == torch.int64 and slot_mapping.dtype == torch.int32
     ws, splits = _skinny_launch(x2, qkv_weight, N, False, None, True)
     q = torch.empty(M, hq, d, dtype=torch.bfloat16, device=x2.device)
-    native.check(native.lib().b200_splitk_reduce_qkv_rope_append(
-        native.ptr(ws), splits, M, hq, hkv, d, native.ptr(bias),
-        1 if bias is not None and bias.dtype == torch.bfloat16 else 0, native.ptr(positions), native.ptr(slot_mapping),
-        float(theta), native.ptr(q), native.ptr(cache), cache.shape[3], 1 if v_transposed else 0, native.stream()),
-        "splitk_reduce_qkv_rope_append")
+    native.check(native.host().b200_splitk_reduce_qkv_rope_append(
+        ws, splits, M, hq, hkv, d, bias, 1 if bias is not None and bias.dtype == torch.bfloat16 else 0, positions, slot_mapping,
+        theta, q, cache, cache.shape[3], 1 if v_transposed else 0, native.stream()), "splitk_reduce_qkv_rope_append")
     return q
 
 
@@ -556,13 +504,11 @@ class _FusedLogprob(torch.autograd.Function):
         lse = torch.empty_like(lp)
         ent = torch.empty_like(lp)
         st = native.status_word(hidden.device)
-        L = native.lib()
-        native.check(L.b200_lmhead_logprob_partial(native.ptr(hidden), native.ptr(weight), native.ptr(labels),
-                                                   native.ptr(partial), T, V, H, hidden.stride(0), weight.stride(0),
-                                                   1.0 / temperature, nsplit, native.ptr(st), sms, native.stream()),
+        L = native.host()
+        native.check(L.b200_lmhead_logprob_partial(hidden, weight, labels, partial, T, V, H, hidden.stride(0), weight.stride(0),
+                                                   1.0 / temperature, nsplit, st, sms, native.stream()),
                      "lmhead_logprob_partial")
-        native.check(L.b200_logprob_combine(native.ptr(partial), native.ptr(labels), native.ptr(lp), native.ptr(lse),
-                                            native.ptr(ent), T, nsplit, native.stream()), "logprob_combine")
+        native.check(L.b200_logprob_combine(partial, labels, lp, lse, ent, T, nsplit, native.stream()), "logprob_combine")
         ctx.save_for_backward(hidden, weight, labels, lse, ent)
         ctx.temperature = temperature
         ctx.want_entropy = want_entropy
@@ -578,7 +524,7 @@ class _FusedLogprob(torch.autograd.Function):
         use_ent = ctx.want_entropy and g_ent is not None
         g_ent_t = _c(g_ent.float()) if use_ent else None
         st = native.status_word(hidden.device)
-        L = native.lib()
+        L = native.host()
         need_dh = ctx.needs_input_grad[0]
         need_dw = ctx.needs_input_grad[1]
         dh = torch.zeros(T, H, dtype=torch.float32, device=hidden.device) if need_dh else None
@@ -588,12 +534,9 @@ class _FusedLogprob(torch.autograd.Function):
         for v0 in range(0, V, chunk):
             vc = min(chunk, V - v0)
             dl = buf[:, :vc]
-            native.check(L.b200_lmhead_dlogits(native.ptr(hidden), native.ptr(weight), native.ptr(labels),
-                                               native.ptr(lse), native.ptr(g_lp), native.ptr(g_ent_t),
-                                               native.ptr(ent) if use_ent else None, native.ptr(buf), T, V, H,
+            native.check(L.b200_lmhead_dlogits(hidden, weight, labels, lse, g_lp, g_ent_t, ent if use_ent else None, buf, T, V, H,
                                                hidden.stride(0), weight.stride(0), v0, vc, buf.stride(0),
-                                               1.0 / ctx.temperature, native.ptr(st), ctx.sms, native.stream()),
-                         "lmhead_dlogits")
+                                               1.0 / ctx.temperature, st, ctx.sms, native.stream()), "lmhead_dlogits")
             # both products on this library's GEMM: dh accumulates in fp32 through the epilogue's reduce-add,
             # dW of this vocabulary slice contracts dlogits^T and hidden over the token axis as stored
             if need_dh:
@@ -694,10 +637,9 @@ def paged_decode(q, cache, block_table, seq_lens, scale: Optional[float] = None,
         return out
     if v_transposed:
         st = native.status_word(q.device)
-        native.check(native.lib().b200_paged_decode_tc(
-            native.ptr(qc), native.ptr(cache), cache.shape[0], native.ptr(block_table), native.ptr(seq_lens),
-            native.ptr(out), native.ptr(scratch), B, hq, hkv, d, page_size, block_table.shape[1], nsplit, scale,
-            native.ptr(st), sms, native.stream()), "paged_decode_tc")
+        native.check(native.host().b200_paged_decode_tc(qc, cache, cache.shape[0], block_table, seq_lens, out, scratch, B, hq, hkv, d,
+                                                        page_size, block_table.shape[1], nsplit, scale, st, sms,
+                                                        native.stream()), "paged_decode_tc")
         return out
     native.check(native.lib().b200_paged_decode(native.ptr(qc), native.ptr(cache), native.ptr(block_table),
                                                 native.ptr(seq_lens), native.ptr(out), native.ptr(scratch), B, hq,
@@ -737,8 +679,7 @@ def quant_fp8_block(w: torch.Tensor, block_rows: int = 128):
     assert w.stride(-1) == 1 and w.dtype == torch.bfloat16
     q = torch.empty(R, C, dtype=torch.float8_e4m3fn, device=w.device)
     scales = torch.empty((R + block_rows - 1) // block_rows, (C + 127) // 128, dtype=torch.float32, device=w.device)
-    native.check(native.lib().b200_quant_fp8_block(native.ptr(w), w.stride(0), native.ptr(q), q.stride(0),
-                                                   native.ptr(scales), R, C, block_rows, native.stream()),
+    native.check(native.host().b200_quant_fp8_block(w, w.stride(0), q, q.stride(0), scales, R, C, block_rows, native.stream()),
                  "quant_fp8_block")
     return q, scales
 
@@ -758,10 +699,9 @@ def gemm_fp8_block(aq: torch.Tensor, sa: torch.Tensor, bq: torch.Tensor, sb: tor
         out = torch.empty(M, N, dtype=torch.bfloat16, device=aq.device)
     st = native.status_word(aq.device)
     dev = aq.device.index if aq.device.index is not None else torch.cuda.current_device()
-    native.check(native.lib().b200_gemm_fp8_block(native.ptr(aq), native.ptr(sa), native.ptr(bq), native.ptr(sb),
-                                                  native.ptr(out), M, N, K, aq.stride(0), bq.stride(0), out.stride(0),
-                                                  sa.stride(0), sb.stride(0), native.ptr(st), native.num_sms(dev),
-                                                  native.stream()), "gemm_fp8_block")
+    native.check(native.host().b200_gemm_fp8_block(aq, sa, bq, sb, out, M, N, K, aq.stride(0), bq.stride(0), out.stride(0),
+                                                   sa.stride(0), sb.stride(0), st, native.num_sms(dev), native.stream()),
+                 "gemm_fp8_block")
     return out
 
 

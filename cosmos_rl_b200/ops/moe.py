@@ -62,8 +62,7 @@ def route_topk(logits: torch.Tensor, k: int, renorm: bool = True, counts: Option
     lg = logits.float().contiguous()
     probs = torch.empty(T, k, dtype=torch.float32, device=logits.device)
     idx = torch.empty(T, k, dtype=torch.int32, device=logits.device)
-    native.check(native.lib().b200_moe_route_topk(native.ptr(lg), T, E, k, int(renorm), native.ptr(probs),
-                                                  native.ptr(idx), native.ptr(counts), native.stream()), "moe_route")
+    native.check(native.host().b200_moe_route_topk(lg, T, E, k, int(renorm), probs, idx, counts, native.stream()), "moe_route")
     return probs, idx
 
 
@@ -84,18 +83,15 @@ class _Dispatch:
         self.n_tiles = torch.empty(1, dtype=torch.int32, device=dev)
         self.cursor = torch.empty(E, dtype=torch.int32, device=dev)
         self.row_map = torch.empty(T, k, dtype=torch.int32, device=dev)
-        native.check(native.lib().b200_moe_offsets(native.ptr(counts), E, native.ptr(self.offsets),
-                                                   native.ptr(self.tile_expert), native.ptr(self.n_tiles),
-                                                   native.ptr(self.cursor), self.max_tiles, native.stream()),
-                     "moe_offsets")
+        native.check(native.host().b200_moe_offsets(counts, E, self.offsets, self.tile_expert, self.n_tiles, self.cursor,
+                                                    self.max_tiles, native.stream()), "moe_offsets")
 
     def zero_padding(self, buf: torch.Tensor, row_info: Optional[torch.Tensor] = None) -> None:
         """Clears the rows of an expert-sorted buffer that no (token, choice) fills, and marks them in ``row_info``. After the
         permutation ``cursor`` holds how many rows each expert got; the caller's histogram is read for the offsets only, since
         the caller may clear or refill it before backward runs."""
-        native.check(native.lib().b200_moe_zero_padding(native.ptr(self.cursor), native.ptr(self.offsets),
-                                                        native.ptr(buf), native.ptr(row_info), self.E, buf.shape[0],
-                                                        buf.shape[1], native.stream()), "moe_zero_padding")
+        native.check(native.host().b200_moe_zero_padding(self.cursor, self.offsets, buf, row_info, self.E, buf.shape[0],
+                                                         buf.shape[1], native.stream()), "moe_zero_padding")
 
 
 def _rows16(x: torch.Tensor) -> torch.Tensor:
@@ -106,8 +102,7 @@ def _rows16(x: torch.Tensor) -> torch.Tensor:
 
 def _swiglu_rows(h1: torch.Tensor, disp: _Dispatch) -> torch.Tensor:
     out = torch.empty(h1.shape[0], h1.shape[1] // 2, dtype=h1.dtype, device=h1.device)
-    native.check(native.lib().b200_swiglu_fwd(native.ptr(h1), native.ptr(out), h1.shape[0], h1.shape[1] // 2,
-                                              native.ptr(disp.n_tiles), native.stream()), "swiglu_fwd")
+    native.check(native.host().b200_swiglu_fwd(h1, out, h1.shape[0], h1.shape[1] // 2, disp.n_tiles, native.stream()), "swiglu_fwd")
     return out
 
 
@@ -116,10 +111,9 @@ def _grouped(x, w, disp: _Dispatch, mode: int, n_out: int) -> torch.Tensor:
     y = torch.empty(disp.max_rows, n_out, dtype=torch.bfloat16, device=x.device)
     st = native.status_word(x.device)
     dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
-    native.check(native.lib().b200_grouped_gemm(native.ptr(x), native.ptr(w), native.ptr(y), disp.max_rows, n_out, K,
-                                                disp.E, x.stride(0), y.stride(0), native.ptr(disp.tile_expert),
-                                                native.ptr(disp.n_tiles), mode, 0, native.ptr(st),
-                                                native.num_sms(dev), native.stream()), "grouped_gemm")
+    native.check(native.host().b200_grouped_gemm(x, w, y, disp.max_rows, n_out, K, disp.E, x.stride(0), y.stride(0),
+                                                 disp.tile_expert, disp.n_tiles, mode, 0, st, native.num_sms(dev),
+                                                 native.stream()), "grouped_gemm")
     return y
 
 
@@ -128,12 +122,10 @@ def _grouped_wgrad(dy, x, disp: _Dispatch, out: torch.Tensor, accumulate: bool,
     """``filled`` (int32 [E]): how many of an expert's rows are not zero in both factors; without it all of its block counts."""
     st = native.status_word(x.device)
     dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
-    native.check(native.lib().b200_grouped_wgrad_filled(native.ptr(dy), native.ptr(x), native.ptr(out), disp.max_rows,
-                                                        dy.shape[1], x.shape[1], disp.E, dy.stride(0), x.stride(0),
-                                                        native.ptr(disp.offsets), native.ptr(filled),
-                                                        1 if out.dtype == torch.float32 else 0, int(accumulate),
-                                                        native.ptr(st), native.num_sms(dev), native.stream()),
-                 "grouped_wgrad")
+    native.check(native.host().b200_grouped_wgrad_filled(dy, x, out, disp.max_rows, dy.shape[1], x.shape[1], disp.E, dy.stride(0),
+                                                         x.stride(0), disp.offsets, filled,
+                                                         1 if out.dtype == torch.float32 else 0, int(accumulate), st,
+                                                         native.num_sms(dev), native.stream()), "grouped_wgrad")
 
 
 class _MoEExperts(torch.autograd.Function):
@@ -143,21 +135,19 @@ class _MoEExperts(torch.autograd.Function):
         E, I2, _ = w_gate_up.shape
         I = I2 // 2
         k = idx.shape[1]
-        L = native.lib()
+        L = native.host()
         disp = _Dispatch(idx, E, counts)
         # rows of the permuted buffers beyond the last tile in use are never read and stay uninitialised
         xp = torch.empty(disp.max_rows, H, dtype=torch.bfloat16, device=x.device)
-        native.check(L.b200_moe_permute(native.ptr(_rows16(x)), native.ptr(idx), native.ptr(disp.offsets),
-                                        native.ptr(disp.cursor), native.ptr(disp.row_map), native.ptr(xp), T, k, H,
-                                        native.stream()), "moe_permute")
+        native.check(L.b200_moe_permute(_rows16(x), idx, disp.offsets, disp.cursor, disp.row_map, xp, T, k, H, native.stream()),
+                     "moe_permute")
         disp.zero_padding(xp)
         h1 = _grouped(xp, w_gate_up, disp, 0, I2)
         act = _swiglu_rows(h1, disp)
         y = _grouped(act, w_down, disp, 0, H)
         out = torch.empty(T, H, dtype=torch.bfloat16, device=x.device)
         probs = probs.float().contiguous()
-        native.check(L.b200_moe_combine(native.ptr(y), native.ptr(probs), native.ptr(disp.row_map), native.ptr(out), T,
-                                        k, H, native.stream()), "moe_combine")
+        native.check(L.b200_moe_combine(y, probs, disp.row_map, out, T, k, H, native.stream()), "moe_combine")
         ctx.save_for_backward(xp, h1, probs, w_gate_up, w_down)
         ctx.disp = disp
         return out
@@ -169,29 +159,26 @@ class _MoEExperts(torch.autograd.Function):
         T, k, E = disp.T, disp.k, disp.E
         H = xp.shape[1]
         I = h1.shape[1] // 2
-        L = native.lib()
+        L = native.host()
         dout = _rows16(dout)
         # the gradient goes to the experts' rows without its weights; they come in between the two projections
         dy = torch.empty(disp.max_rows, H, dtype=torch.bfloat16, device=dout.device)
         row_info = torch.empty(disp.max_rows, 2, dtype=torch.int32, device=dout.device)
         disp.zero_padding(dy, row_info)
-        native.check(L.b200_moe_spread(native.ptr(dout), native.ptr(probs), native.ptr(disp.row_map), native.ptr(dy),
-                                       native.ptr(row_info), T, k, H, native.stream()), "moe_spread")
+        native.check(L.b200_moe_spread(dout, probs, disp.row_map, dy, row_info, T, k, H, native.stream()), "moe_spread")
         dact = _grouped(dy, w_down, disp, 1, I)             # dY . W_down[e]   (W_down [E, H, I])
         dh1 = torch.empty_like(h1)
         ap = torch.empty(disp.max_rows, I, dtype=torch.bfloat16, device=dout.device)
         dprob = torch.empty(T, k, dtype=torch.float32, device=dout.device)
-        native.check(L.b200_moe_swiglu_bwd(native.ptr(dact), native.ptr(h1), native.ptr(row_info), native.ptr(disp.n_tiles),
-                                           native.ptr(dh1), native.ptr(ap), native.ptr(dprob), disp.max_rows, I,
-                                           native.stream()), "moe_swiglu_bwd")
+        native.check(L.b200_moe_swiglu_bwd(dact, h1, row_info, disp.n_tiles, dh1, ap, dprob, disp.max_rows, I, native.stream()),
+                     "moe_swiglu_bwd")
         dw_down = torch.empty_like(w_down)
         _grouped_wgrad(dy, ap, disp, dw_down, False, disp.cursor)
         dxp = _grouped(dh1, w_gate_up, disp, 1, H)          # dH1 . W_gu[e]     (W_gu [E, 2I, H])
         dw_gu = torch.empty_like(w_gate_up)
         _grouped_wgrad(dh1, xp, disp, dw_gu, False, disp.cursor)
         dx = torch.empty(T, H, dtype=torch.bfloat16, device=dout.device)
-        native.check(L.b200_moe_combine(native.ptr(dxp), None, native.ptr(disp.row_map), native.ptr(dx), T, k, H,
-                                        native.stream()), "moe_unpermute")
+        native.check(L.b200_moe_combine(dxp, None, disp.row_map, dx, T, k, H, native.stream()), "moe_unpermute")
         return dx, dprob, None, dw_gu, dw_down, None
 
 

@@ -150,6 +150,19 @@ def lib() -> ctypes.CDLL:
     return handle
 
 
+@functools.lru_cache(maxsize=1)
+def host():
+    """The entry points that take tensors (``csrc/host.cpp``): launchers of :func:`lib` with tensors for their pointers, and calls
+    that allocate their results as well."""
+    lib()
+    try:
+        from . import _host
+    except ImportError as e:
+        raise NativeError(f"{_LIB_PATH.parent / '_host.so'} is missing or was built for another torch: build it with "
+                          "`python -m cosmos_rl_b200.ops.build`") from e
+    return _host
+
+
 def ptr(t):
     """Device (or host) address of a tensor, ``None`` -> NULL."""
     return None if t is None else t.data_ptr()
@@ -189,6 +202,14 @@ def check(rc: int, what: str) -> None:
             except Exception:
                 pass
         raise NativeError(f"{what}: {names.get(rc, rc)}{detail}")
+
+
+def tensors(r, what: str):
+    """The answer of one of :func:`host`'s calls: its tensors, or the code of a launcher that failed."""
+    if type(r) is int:
+        check(r, what)
+    LAUNCHES[0] += 1
+    return r
 
 
 @functools.lru_cache(maxsize=8)

@@ -57,3 +57,28 @@ def test_rms_norm_refuses_a_residual_of_other_rows(monkeypatch):
                 with pytest.raises(RuntimeError):
                     F.rms_norm(x, w, residual=make(*shape))
     assert seen == [(4, 512)] * 8
+
+
+def test_launchers_refuse_what_cannot_be_launched():
+    """Wrong counts and types, sizes beyond the argument's, and tensors that have no memory end in an exception before a launch."""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cosmos_rl_b200.ops import build, native
+    if not (native.available() and build.host_path().exists()):
+        pytest.skip("the kernel library is not built")
+    H, x = native.host(), torch.zeros(4, 8, dtype=torch.bfloat16)
+    for args in ((x,), (x, 0, 0), (1, 0), (None, 0)):
+        with pytest.raises(TypeError):
+            H.swiglu_fwd(*args)
+    with pytest.raises(TypeError):
+        H.b200_swiglu_fwd(x, "out", 4, 4, None, 0)
+    with pytest.raises(ValueError):
+        H.b200_swiglu_fwd(x, x, 4, 1 << 31, None, 0)
+    with pytest.raises(AssertionError):
+        H.swiglu_fwd(x[0], 0)
+    with pytest.raises(AssertionError):
+        H.gemm(x, x, False, False, None, False, False, None, False, 0, None, -1, 0, 148, 0)      # not on a GPU
+    with FakeTensorMode(), pytest.raises(RuntimeError, match="without memory"):
+        H.swiglu_fwd(torch.empty(4, 8, dtype=torch.bfloat16, device="cuda"), 0)
