@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "api.h"
+#include "sm100.cuh"
 
 namespace {
 
@@ -42,8 +43,6 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
-// Makes the compiler unpack `u` again after this point instead of keeping the eight fp32 values alive in registers.
-__device__ __forceinline__ void keep_packed(uint4& u) { asm volatile("" : "+r"(u.x), "+r"(u.y), "+r"(u.z), "+r"(u.w)); }
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   uint4 u;
   __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&u);
@@ -151,17 +150,42 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-// RMSNorm backward of wide rows: dx (+ dres) and the weight gradient in one pass over dy and x. Persistent CTAs walk
-// groups of ROWS rows; a thread keeps the weight-gradient sums of its own columns in registers and writes them once, to
-// its block's row of dw_partial (null: no weight gradient).
-template <int VPT, int ROWS, int MIN_CTAS>
+// RMSNorm backward of wide rows: dx (+ dres) and the weight gradient in one pass over dy and x. Persistent CTAs walk pairs of
+// adjacent rows; a thread keeps the weight-gradient sums of its own columns in registers and writes them once, to its block's row
+// of dw_partial (null: no weight gradient).
+// Bound by HBM, if enough rows are on their way: a row is dy, x and dres, and rows come through a ring of NORM_STAGES in shared
+// memory as bulk copies, three rows ahead of the one that is worked on. 8192 x 3584: 40.2 us, with the loads of two rows in
+// registers, whose way the CTA waited for, 49.7 (36 are the bytes); 16384 x 5120 122 and 164; 64 x 3584 3.6 and 3.4.
+constexpr int NORM_STAGES = 4;
+template <int VPT, int MIN_CTAS>
 __global__ void __launch_bounds__(NORM_MAX_THREADS, MIN_CTAS)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ dw_partial, long long T, int H) {
-  __shared__ float sh[2][ROWS][16];
+  extern __shared__ __align__(16) uint8_t ring[];   // [NORM_STAGES][dy, x, dres][H]
+  __shared__ float sh[2][1][16];
+  __shared__ uint64_t full[NORM_STAGES];
   const int nvec = H >> 3;
+  const uint32_t row_bytes = (uint32_t)H * 2;
+  // the it-th row of this CTA: both rows of a pair, then the pair a grid further
+  auto row_of = [&](int it) { return ((long long)blockIdx.x + (long long)(it >> 1) * gridDim.x) * 2 + (it & 1); };
+  auto fetch = [&](int it) {
+    const long long row = row_of(it);
+    if (row >= T) return;
+    uint8_t* dst = ring + (it % NORM_STAGES) * 3 * row_bytes;
+    uint64_t* bar = &full[it % NORM_STAGES];
+    b200::mbar_arrive_expect_tx(bar, (dres ? 3 : 2) * row_bytes);
+    b200::bulk_load(dst, dy + row * H, row_bytes, bar);
+    b200::bulk_load(dst + row_bytes, x + row * H, row_bytes, bar);
+    if (dres) b200::bulk_load(dst + 2 * row_bytes, dres + row * H, row_bytes, bar);
+  };
+  b200::pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NORM_STAGES; ++s) b200::mbar_init(&full[s], 1);
+    b200::mbar_fence_init();
+    for (int s = 0; s < NORM_STAGES - 1; ++s) fetch(s);
+  }
   uint4 wv[VPT];
   float dw[VPT][8];
 #pragma unroll
@@ -172,69 +196,50 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 #pragma unroll
     for (int j = 0; j < 8; ++j) dw[i][j] = 0.f;
   }
-  int buf = 0;
-  for (long long row0 = (long long)blockIdx.x * ROWS; row0 < T; row0 += (long long)gridDim.x * ROWS, buf ^= 1) {
-    uint4 a[ROWS][VPT], b[ROWS][VPT];
-    float rs[ROWS], dot[ROWS];
+  __syncthreads();
+  for (int it = 0;; ++it) {
+    const long long row = row_of(it);
+    if (row >= T) break;   // the pair's second row is the tensor's last row but one pair: nothing follows
+    float rs = rstd[row];
+    const uint4* in = reinterpret_cast<const uint4*>(ring + (it % NORM_STAGES) * 3 * row_bytes);
+    if (!b200::mbar_wait(&full[it % NORM_STAGES], (it / NORM_STAGES) & 1)) rs = __int_as_float(0x7fffffff);   // NaN shows it
+    uint4 a[VPT], b[VPT];
+    float dot[1] = {0.f};
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      const bool in = row0 + r < T;
-      rs[r] = in ? rstd[row0 + r] : 0.f;
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
+      a[i] = b[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (v < nvec) {
+        a[i] = in[v];
+        b[i] = in[nvec + v];
+      }
+      float fa[8], fb[8], g[8];
+      unpack8(a[i], fa);
+      unpack8(b[i], fb);
+      unpack8(wv[i], g);
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int v = threadIdx.x + i * blockDim.x;
-        a[r][i] = b[r][i] = make_uint4(0u, 0u, 0u, 0u);
-        if (in && v < nvec) {
-          a[r][i] = reinterpret_cast<const uint4*>(dy + (row0 + r) * H)[v];
-          b[r][i] = reinterpret_cast<const uint4*>(x + (row0 + r) * H)[v];
-        }
+      for (int j = 0; j < 8; ++j) {
+        const float xh = fb[j] * rs;
+        dw[i][j] += fa[j] * xh;
+        dot[0] += fa[j] * g[j] * xh;
       }
     }
+    block_sums<1>(dot, sh[it & 1]);
+    // its barrier says that every thread is through with the row before, whose stage takes the row three ahead
+    if (threadIdx.x == 0) fetch(it + NORM_STAGES - 1);
+    dot[0] /= (float)H;
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      dot[r] = 0.f;
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
+      if (v >= nvec) continue;
+      float fa[8], fb[8], g[8], o[8];
+      unpack8(a[i], fa);
+      unpack8(b[i], fb);
+      unpack8(wv[i], g);
+      unpack8(dres ? in[2 * nvec + v] : make_uint4(0u, 0u, 0u, 0u), o);
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        float fa[8], fb[8], g[8];
-        unpack8(a[r][i], fa);
-        unpack8(b[r][i], fb);
-        unpack8(wv[i], g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xh = fb[j] * rs[r];
-          dw[i][j] += fa[j] * xh;
-          dot[r] += fa[j] * g[j] * xh;
-        }
-      }
-    }
-    uint4 d[ROWS][VPT];   // in flight across the barrier
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int v = threadIdx.x + i * blockDim.x;
-        d[r][i] = make_uint4(0u, 0u, 0u, 0u);
-        if (dres && row0 + r < T && v < nvec) d[r][i] = reinterpret_cast<const uint4*>(dres + (row0 + r) * H)[v];
-      }
-    block_sums<ROWS>(dot, sh[buf]);
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-      dot[r] /= (float)H;
-#pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int v = threadIdx.x + i * blockDim.x;
-        float fa[8], fb[8], g[8], o[8];
-        keep_packed(a[r][i]);
-        keep_packed(b[r][i]);
-        keep_packed(wv[i]);
-        unpack8(a[r][i], fa);
-        unpack8(b[r][i], fb);
-        unpack8(wv[i], g);
-        unpack8(d[r][i], o);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += rs[r] * (fa[j] * g[j] - fb[j] * rs[r] * dot[r]);
-        if (row0 + r < T && v < nvec) reinterpret_cast<uint4*>(dx + (row0 + r) * H)[v] = pack8(o);
-      }
+      for (int j = 0; j < 8; ++j) o[j] += rs * (fa[j] * g[j] - fb[j] * rs * dot[0]);
+      reinterpret_cast<uint4*>(dx + row * H)[v] = pack8(o);
     }
   }
   if (dw_partial) {
@@ -250,11 +255,13 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// dw[c] = sum of the rows of partial [rows, H], as bf16: a warp takes every eighth row of 32 columns
+// dw[c] = sum of the rows of partial [rows, H], as bf16: a warp takes every eighth row of 32 columns. Its CTAs are there when the
+// kernel before ends (8192 x 3584, both: 43.0 us, one after the other 45.1).
 __global__ void __launch_bounds__(256)
 rmsnorm_dw_sum_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, int rows, int H) {
   __shared__ float sh[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  b200::pdl_wait();
   float s = 0.f;
   if (c < H) {
 #pragma unroll 8
@@ -650,16 +657,28 @@ int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float*
     }
   } else {
     const NormShape n(H);
-    auto go = [&](auto kern, int group, int ctas) {
-      const long long groups = (T + group - 1) / group;
-      rows = (int)(groups < ctas ? groups : ctas);
-      kern<<<rows, n.threads, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                           rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, ws, T, H);
+    if (((uintptr_t)dy | (uintptr_t)x | (uintptr_t)dres) & 15) return B200_ERR_ARG;
+    const int smem = NORM_STAGES * 3 * H * 2;
+    auto go = [&](auto kern, int ctas) {
+      const long long pairs = (T + 1) / 2;
+      rows = (int)(pairs < ctas ? pairs : ctas);
+      kern<<<rows, n.threads, smem, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
+                                              (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, ws, T, H);
     };
-    if (n.vpt == 1) go(rmsnorm_bwd_kernel<1, 2, 2>, 2, RMSNORM_WS_ROWS);
-    else go(rmsnorm_bwd_kernel<2, 2, 1>, 2, RMSNORM_WS_ROWS / 2);
+    static bool attr_set = false;
+    if (!attr_set) {
+      constexpr int most = NORM_STAGES * 3 * NORM_MAX_H * 2;
+      if (cudaFuncSetAttribute(rmsnorm_bwd_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most / 2) != cudaSuccess ||
+          cudaFuncSetAttribute(rmsnorm_bwd_kernel<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+        return B200_ERR_LAUNCH;
+      attr_set = true;
+    }
+    if (n.vpt == 1) go(rmsnorm_bwd_kernel<1, 2>, RMSNORM_WS_ROWS);
+    else go(rmsnorm_bwd_kernel<2, 1>, RMSNORM_WS_ROWS / 2);
   }
-  if (dw) rmsnorm_dw_sum_kernel<<<(H + 31) / 32, 256, 0, stream>>>(ws, (__nv_bfloat16*)dw, rows, H);
+  if (dw && b200::launch_pdl(rmsnorm_dw_sum_kernel, dim3((H + 31) / 32), dim3(256), 0, stream, (const float*)ws,
+                             (__nv_bfloat16*)dw, rows, H) != cudaSuccess)
+    return B200_ERR_LAUNCH;
   return ok();
 }
 

@@ -1897,3 +1897,25 @@ def test_fused_logprob_ranges(T, V, H):
     logit = 2.0 ** -20 * (h.double().norm(dim=1) * w.double().norm(dim=1).max()) / 0.8
     assert ((lp.double() - want).abs() <= 2 * logit + 1e-5 * (1 + lse.abs())).all()
     assert ((ent.double() - want_ent).abs() <= (2 + logits.abs().amax(-1)) * (2 * logit + 1e-5)).all()
+
+
+@pytest.mark.parametrize("H", [1032, 4096, 4104, 8192])
+@pytest.mark.parametrize("T,residual", [(1, True), (2, False), (593, True), (1187, False), (2380, True)])
+def test_rms_norm_backward_rows_through_a_ring(T, H, residual):
+    """Fewer rows than stages, one row left of a pair, as many pairs as CTAs and one more, several times round the ring; a whole row
+    of threads and one vector more."""
+    torch.manual_seed(90)
+    x, w = _bf16(T, H).requires_grad_(True), _bf16(H).requires_grad_(True)
+    res = _bf16(T, H) if residual else None
+    y, total = F.rms_norm(x, w, 1e-6, residual=res)
+    dy, dres = _bf16(T, H), _bf16(T, H)
+    dx, dw = torch.autograd.grad([y, total] if residual else [y], [x, w], [dy, dres] if residual else [dy])
+    h = (total if residual else x).detach().double().requires_grad_(True)
+    wd = w.detach().double().requires_grad_(True)
+    ref = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-6) * wd
+    want, want_w = torch.autograd.grad(ref, [h, wd], dy.double())
+    if residual:
+        want = want + dres.double()
+    # one rounding to bf16; sums of H (rows: T) fp32 products in between
+    assert ((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -16 * dy.double().norm(dim=1, keepdim=True)).all()
+    assert ((dw.double() - want_w).abs() <= 2 ** -8 * want_w.abs() + 2 ** -18 * T ** 0.5 * dy.double().norm(dim=0)).all()
