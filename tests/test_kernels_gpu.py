@@ -1919,3 +1919,18 @@ def test_rms_norm_backward_rows_through_a_ring(T, H, residual):
     # one rounding to bf16; sums of H (rows: T) fp32 products in between
     assert ((dx.double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -16 * dy.double().norm(dim=1, keepdim=True)).all()
     assert ((dw.double() - want_w).abs() <= 2 ** -8 * want_w.abs() + 2 ** -18 * T ** 0.5 * dy.double().norm(dim=0)).all()
+
+
+@pytest.mark.parametrize("M", [1, 129])
+@pytest.mark.parametrize("N,K,pad", [(136, 64, 0), (1032, 1024, 8), (1032, 1032, 0), (264, 1000, 4)])
+def test_skinny_short_contractions(M, N, K, pad):
+    """Up to 16 blocks in one kernel, one value more in two; rows that only the second kernel can write."""
+    torch.manual_seed(91)
+    x, w, bias = _bf16(M, K), _bf16(N, K, scale=0.1), _bf16(N)
+    buf = torch.full((M, N + pad), 7., dtype=torch.bfloat16, device=DEV)
+    F.gemm_skinny(x, w, bias=bias, out=buf[:, :N])
+    native.read_status(x.device)
+    ref = x.double() @ w.double().t() + bias.double()
+    # one rounding to bf16, fp32 sums of K products
+    bound = 2.0 ** -8 * ref.abs() + 2.0 ** -20 * x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=1) + 1e-6
+    assert ((buf[:, :N].double() - ref).abs() <= bound).all() and (buf[:, N:] == 7).all()
