@@ -485,11 +485,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
             uint32_t u[32];
             tmem_ld_32x32b_x32(taddr + BN / 2 + cc, u);
             tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float g = __uint_as_float(r[j]);
-              v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
-            }
+            swiglu_values(reinterpret_cast<const float(&)[32]>(r), reinterpret_cast<const float(&)[32]>(u), v);
           } else if constexpr (EPI == G2_EPI_DLOGITS) {
             tmem_ld_wait();
             const long long off = dlr.label - (ep.dl.v0 + col_base + cc);

@@ -126,10 +126,8 @@ struct SkinnyEpilogue {
           tmem_ld_32x32b_x32(taddr + BN / 2 + cc, u);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float g = row0 + lane < p.M ? __uint_as_float(a[j]) : SKINNY_NO_ROW;
-            v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
-          }
+          for (int j = 0; j < 32; ++j) v[j] = row0 + lane < p.M ? __uint_as_float(a[j]) : SKINNY_NO_ROW;
+          swiglu_values(v, reinterpret_cast<const float(&)[32]>(u), v);
         } else {
           tmem_ld_wait();
 #pragma unroll
@@ -195,10 +193,8 @@ struct SwigluRowsEpilogue {
       tmem_ld_wait();
       float v[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float g = r < p.M ? __uint_as_float(a[j]) : SKINNY_NO_ROW;
-        v[j] = g / (1.f + __expf(-g)) * __uint_as_float(u[j]);
-      }
+      for (int j = 0; j < 16; ++j) v[j] = r < p.M ? __uint_as_float(a[j]) : SKINNY_NO_ROW;
+      swiglu_values(v, reinterpret_cast<const float(&)[16]>(u), v);
       if (r >= p.M) continue;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {

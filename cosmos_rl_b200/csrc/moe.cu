@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "api.h"
+#include "sm100.cuh"
 
 namespace {
 
@@ -209,7 +210,7 @@ combine_kernel(const __nv_bfloat16* __restrict__ y, const float* __restrict__ pr
 // Backward of the experts' middle. With a = silu(g) o u, the row's output is p (a Wd^T) and dact = dout Wd lacks the weight p:
 //   dprob = <a, dact>,  dh1 = p dact d(a)/d(g, u),  ap = p a (what the gradient of Wd contracts with the unweighted dout).
 // So the weights' gradient needs neither the experts' output nor a pass over it, a is not formed in a pass of its own, and the
-// gradient is spread as it is. Bound by HBM (12 bytes an element of a; 4096 tokens on 128 experts of 768, 8 each: 61 us, 0.85 of
+// gradient is spread as it is. Bound by HBM (12 bytes an element of a; 4096 tokens on 128 experts of 768, 8 each: 59 us, 0.88 of
 // copy speed; the passes it stands for, a, the gradient of a and dprob, took 126). One warp a row, since dprob is the row's sum;
 // 40 warps an SM hide the way from a row's number to its data better than three vectors a lane on their way with 16 or 24 warps
 // (73 and 64 us), and several warps a row add a barrier (80).
@@ -233,21 +234,22 @@ expert_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dact, const __nv_bflo
   float dot = 0.f;
   for (int v = lane; v < nvec; v += 32) {
     const uint4 gv = in[v], uv = in[nvec + v], dv = in_d[v];
-    float a[8], b[8], c[8], dg[8], du[8];
+    float a[8], b[8], c[8], s[8];
     unpack8(gv, a);
     unpack8(uv, b);
     unpack8(dv, c);
+    b200::sigmoids(a, s);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float s = 1.f / (1.f + __expf(-a[j])), silu = a[j] * s, act = silu * b[j], pd = p * c[j];
+      const float silu = a[j] * s[j], act = silu * b[j], pd = p * c[j];
       dot += act * c[j];
-      dg[j] = pd * b[j] * (s + silu * (1.f - s));
-      du[j] = pd * silu;
-      a[j] = p * act;
+      a[j] = pd * b[j] * (s[j] + silu * (1.f - s[j]));
+      b[j] = pd * silu;
+      c[j] = p * act;
     }
-    out[v] = pack8(dg);
-    out[nvec + v] = pack8(du);
-    out_a[v] = pack8(a);
+    out[v] = pack8(a);
+    out[nvec + v] = pack8(b);
+    out_a[v] = pack8(c);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);

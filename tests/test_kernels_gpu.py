@@ -1934,3 +1934,27 @@ def test_skinny_short_contractions(M, N, K, pad):
     # one rounding to bf16, fp32 sums of K products
     bound = 2.0 ** -8 * ref.abs() + 2.0 ** -20 * x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=1) + 1e-6
     assert ((buf[:, :N].double() - ref).abs() <= bound).all() and (buf[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("M", [5, 100, 300])
+def test_swiglu_epilogues_of_special_gates(M):
+    """Gates whose exponential overflows, zeros, infinities and NaN beside ordinary ones, in the tiles of few, some and many rows."""
+    special = torch.tensor([0., -0., 1., -1., 20., -20., -85.5, -86., -86.5, -88., -88.75, -100., -3e38, 3e38, 1e38, float("inf"),
+                            float("-inf"), float("nan"), 1e-38, -1e-38], device=DEV)
+    torch.manual_seed(92)
+    I, K = 264, 64
+    gates = torch.randn(I, device=DEV) * 8
+    gates[:len(special)] = special
+    gates[150:150 + len(special)] = special.flip(0)
+    x, w = torch.zeros(M, K, dtype=torch.bfloat16, device=DEV), torch.zeros(2 * I, K, dtype=torch.bfloat16, device=DEV)
+    x[:, 0], w[:I, 0], w[I:, 0] = 1., gates.to(torch.bfloat16), torch.randn(I, device=DEV).to(torch.bfloat16)
+    got = F.skinny_gate_up_swiglu(x, w) if M <= 256 else F.gemm(x, w, swiglu=True)
+    native.read_status(x.device)
+    g, u = w[:I, 0].float(), w[I:, 0].float()
+    want = (g / (1 + torch.exp(-g)) * u).to(torch.bfloat16)
+    bad = torch.isnan(g) | torch.isinf(g)
+    assert torch.equal(torch.isnan(got[:, bad]), torch.isnan(want[bad]).expand(M, -1))
+    assert torch.equal(torch.isinf(got), torch.isinf(want).expand(M, -1))
+    ok = torch.isfinite(want)
+    # __expf is good to 2^-21 of a result of up to 2^6 in its exponent; one rounding to bf16
+    assert torch.allclose(got[:, ok].float(), want[ok].float().expand(M, -1), rtol=2 ** -7, atol=1e-30)
