@@ -47,6 +47,16 @@ int b200_gemm_bf16_ws(const void* A, const void* B, void* C, int M, int N, int K
 long long b200_gemm_scratch(int M, int N, int K, int a_mn, int rows16, int out_fp32, int accumulate, int bias, int epilogue,
                             int path, int num_sms);
 
+// A gated MLP in training (gemm_mlp.cu), M > 128: gate_up [M, 2 I] = x W^T and act [M, I] = silu(gate) * up, as its pass over the
+// stored values makes it; and dgate_up [M, 2 I], the gradient of gate_up where the gradient of act is dy W (W [K, I] as stored).
+// I % 8 == 0; gate_up, act and dgate_up contiguous and 16-byte aligned. ws: fp32 scratch of ws_floats elements for a last round that
+// is cut along the contraction (b200_gemm_gated_scratch: how many; with less it stays whole).
+int b200_gemm_gate_up(const void* x, const void* W, void* gate_up, void* act, int M, int I, int K, long long ldx, long long ldw,
+                      float* ws, long long ws_floats, uint32_t* status, int num_sms, cudaStream_t stream);
+int b200_gemm_dgate_up(const void* dy, const void* W, const void* gate_up, void* dgate_up, int M, int I, int K, long long lddy,
+                       long long ldw, float* ws, long long ws_floats, uint32_t* status, int num_sms, cudaStream_t stream);
+long long b200_gemm_gated_scratch(int M, int I, int K, int backward, int num_sms);
+
 // Weight-streaming GEMM for decode-sized batches (M <= 256) and the reductions that finish a decode-layer step
 // (gemm_skinny.cu). x [M, K] bf16, W [rows, K] bf16. ws == NULL: out (bf16) = x W^T (+ bias), splits = 1; swiglu: W is a
 // fused gate/up weight with up rows at up_row0 and out = silu(x Wg^T) * (x Wu^T) of N columns. ws != NULL: fp32

@@ -36,14 +36,20 @@ constexpr int G2_BM = 256;      // rows of the pair's tile
 constexpr int G2_BK = 64;
 constexpr int G2_THREADS = 192;
 
-enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3, G2_EPI_LOGPROB = 4 };
+enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3, G2_EPI_LOGPROB = 4, G2_EPI_GATE_UP = 5,
+       G2_EPI_DGATE_UP = 6 };
 
-template <int BN, int STAGES>
+// Epilogue warps of a CTA: two a TMEM lane quadrant where the epilogue computes (8192 x 18944 x 3584, backward: 1084
+// us with one, 911)
+__host__ __device__ constexpr int g2_epilogue_warps(int epi) { return epi == G2_EPI_GATE_UP || epi == G2_EPI_DGATE_UP ? 8 : 4; }
+__host__ __device__ constexpr int g2_threads(int epi) { return 64 + 32 * g2_epilogue_warps(epi); }
+
+template <int BN, int STAGES, int EPI = G2_EPI_STORE>
 struct Gemm2Smem {
   static constexpr int A_BYTES = G2_BM_CTA * G2_BK * 2;
   static constexpr int B_BYTES = (BN / 2) * G2_BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGING_BYTES = 4 * 2 * 4096;  // 4 epilogue warps x 2 slabs of 32 rows x 128 bytes
+  static constexpr int STAGING_BYTES = g2_epilogue_warps(EPI) * 2 * 4096;  // 2 slabs of 32 rows x 128 bytes a warp
   static constexpr int BAR_BYTES = 256;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING_BYTES + BAR_BYTES + 1024;
 };
@@ -264,7 +270,8 @@ template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool TAIL>
 __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUtensorMap* tmB, const CUtensorMap* tmC,
                                                const CUtensorMap* tmW, int M, int N, int K, const Gemm2Params& ep,
                                                uint32_t* status) {
-  using SM = Gemm2Smem<BN, STAGES>;
+  using SM = Gemm2Smem<BN, STAGES, EPI>;
+  constexpr int EW = g2_epilogue_warps(EPI);
   static_assert(BN == 128 || BN == 256, "BN");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -275,6 +282,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   uint64_t* tempty_bar = tfull_bar + 2;      // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  uint64_t* in_full = full_bar + 16;         // [8 epilogue warps][2], G2_EPI_DGATE_UP: gates and ups of a chunk
+  static_assert(EPI != G2_EPI_DGATE_UP || (2 * STAGES + 5 <= 16 && SM::BAR_BYTES >= 256), "barriers");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -289,8 +298,10 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 8);  // 4 epilogue warps of each CTA of the pair
+      mbar_init(&tempty_bar[a], 2 * EW);  // the epilogue warps of both CTAs of the pair
     }
+    if constexpr (EPI == G2_EPI_DGATE_UP)
+      for (int i = 0; i < 2 * EW; ++i) mbar_init(&in_full[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(tmA);
@@ -308,11 +319,12 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   const uint32_t tmem_base = *tmem_slot;
 
   const int num_m = (M + G2_BM - 1) / G2_BM;
-  constexpr int OUT_BN = (EPI == G2_EPI_SWIGLU) ? BN / 2 : BN;  // columns of C per tile
-  const int n_cols = (EPI == G2_EPI_SWIGLU) ? N / 2 : N;        // columns of C
+  constexpr bool GATED = EPI == G2_EPI_SWIGLU || EPI == G2_EPI_GATE_UP;   // half of a tile's columns are gates, half ups
+  constexpr int OUT_BN = GATED ? BN / 2 : BN;  // columns of C per tile
+  const int n_cols = GATED ? N / 2 : N;        // columns of C
   const int num_n = (n_cols + OUT_BN - 1) / OUT_BN;
   std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork, std::conditional_t<EPI == G2_EPI_LOGPROB, G2LogprobWork, G2Work>> work;
-  work.init(ep, EPI == G2_EPI_STORE, num_m, num_n, (K + G2_BK - 1) / G2_BK);
+  work.init(ep, EPI == G2_EPI_STORE || EPI == G2_EPI_GATE_UP || EPI == G2_EPI_DGATE_UP, num_m, num_n, (K + G2_BK - 1) / G2_BK);
   G2Unit unit;
 
   if (warp == 0) {
@@ -328,7 +340,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         // rows of B that this CTA feeds: its half of the tile's columns; with the SwiGLU epilogue the leader
         // feeds the gate rows and the other CTA the matching up rows, so a thread sees both in its TMEM lane
         int b_row0;
-        if constexpr (EPI == G2_EPI_SWIGLU) b_row0 = n_blk * (BN / 2) + (cta_rank ? ep.up_row0 : 0);
+        if constexpr (GATED) b_row0 = n_blk * (BN / 2) + (cta_rank ? ep.up_row0 : 0);
         else b_row0 = n_blk * BN + (int)cta_rank * (BN / 2);
         for (int kb = unit.kb0; kb < unit.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
@@ -414,7 +426,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   } else {
     // ------------------------------ epilogue (warps 2..5 of both CTAs) --------------------
     const int quad = warp & 3;  // TMEM lane quadrant this warp may access
-    uint8_t* slab0 = staging + quad * 8192;
+    const int half = EW == 8 ? (warp - 2) >> 2 : 0;   // of a tile's columns, where a quadrant has two warps
+    uint8_t* slab0 = staging + (quad + 4 * half) * 8192;
     const uint32_t tempty_leader0 = mapa_shared(smem_u32(&tempty_bar[0]), 0);
     const uint32_t tempty_leader1 = mapa_shared(smem_u32(&tempty_bar[1]), 0);
     uint32_t acc = 0, acc_phase = 0;
@@ -423,6 +436,26 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
     LogprobRow lgr;
     long long lg_row = -1;   // the row and the range that lgr is about
     int lg_split = -1;
+    // G2_EPI_DGATE_UP: chunks so far, and the one whose gates and ups are fetched next (unit in_it, chunk in_i of it)
+    uint32_t in_count = 0;
+    int in_it = 0, in_i = 0;
+    auto in_fetch = [&](uint32_t count) {   // one elected lane
+      G2Unit t;
+      for (; work.get(in_it, t); ++in_it, in_i = 0) {
+        const int row = t.m_blk * G2_BM + (int)cta_rank * G2_BM_CTA + quad * 32, col = t.n_blk * BN + half * 128 + 32 * in_i;
+        if (t.cut || row >= M || in_i == 4 || col >= n_cols) continue;
+        ++in_i;
+        uint64_t* bar = &in_full[2 * (warp - 2) + (count & 1)];
+        uint8_t* slab = slab0 + (count & 1) * 4096;
+        mbar_arrive_expect_tx(bar, 4096);
+        tma_load_3d(slab, tmC, bar, col, 0, row);
+        tma_load_3d(slab + 2048, tmC, bar, col, 1, row);
+        return;
+      }
+    };
+    if constexpr (EPI == G2_EPI_DGATE_UP) {
+      if (elect_one()) in_fetch(0);
+    }
     for (int it = 0; work.get(it, unit) && !*abort_flag; ++it) {
       const int m_blk = unit.m_blk, n_blk = unit.n_blk;
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) {
@@ -456,6 +489,113 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
           lgr.chunk(ep.lg, col_base + c, v);
+        }
+      } else if constexpr (EPI == G2_EPI_GATE_UP || EPI == G2_EPI_DGATE_UP) {
+        auto pair = [](uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); };
+        if (unit.cut) {   // fp32 into the pair's part of the workspace; gemm2_sum_gated_kernel does the rest
+          float* dst = ep.ws + ((long long)(blockIdx.x >> 1) * G2_BM + (row0 - m_blk * G2_BM) + lane) * BN;
+#pragma unroll 1
+          for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(taddr + c, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+          }
+        } else if constexpr (EPI == G2_EPI_GATE_UP) {
+          // The gate and up values as they are stored, and what the SwiGLU kernel makes of them: the same bits as its pass over them.
+          const int c = half * 64, gc = col_base + c;
+          if (gc < n_cols && row0 < M) {
+            auto put = [&](const uint32_t (&v)[32], auto store) {   // 64 columns as bf16 pairs, through the next staging slab
+              uint8_t* slab = slab0 + (slab_idx++ & 1) * 4096;
+              if (elect_one()) tma_store_wait_read<1>();
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                *reinterpret_cast<uint4*>(slab + lane * 128 + ((((uint32_t)j) ^ sw) << 4)) =
+                    make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (elect_one()) {
+                store(slab);
+                tma_store_commit();
+              }
+            };
+            auto fetch = [&](uint32_t col, uint32_t (&v)[32]) {   // accumulator columns col .. col + 63, rounded
+              uint32_t r[2][32];
+              tmem_ld_32x32b_x32(taddr + col, r[0]);
+              tmem_ld_32x32b_x32(taddr + col + 32, r[1]);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                v[j] = pack_bf16x2(__uint_as_float(r[j >> 4][2 * (j & 15)]), __uint_as_float(r[j >> 4][2 * (j & 15) + 1]));
+            };
+            uint32_t g[32], u[32];
+            fetch(c, g);
+            put(g, [&](uint8_t* slab) { tma_store_3d(tmW, slab, gc, 0, row0); });
+            fetch(BN / 2 + c, u);
+            put(u, [&](uint8_t* slab) { tma_store_3d(tmW, slab, gc, 1, row0); });
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              float a[8], b[8];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 x = pair(g[4 * q + j]), y = pair(u[4 * q + j]);
+                a[2 * j] = x.x; a[2 * j + 1] = x.y;
+                b[2 * j] = y.x; b[2 * j + 1] = y.y;
+              }
+              swiglu_values(a, b, a);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) g[4 * q + j] = pack_bf16x2(a[2 * j], a[2 * j + 1]);
+            }
+            put(g, [&](uint8_t* slab) { tma_store_2d(tmC, slab, gc, row0); });
+          }
+        } else if (row0 < M) {
+          // The accumulators are the gradient of the product. Gates and ups come by TMA, a chunk of 32 columns ahead, into the
+          // slab (two halves of 32 rows x 64 bytes) from which their gradients leave.
+#pragma unroll 1
+          for (int i = 0; i < 4 && col_base + half * 128 + 32 * i < n_cols; ++i, ++in_count) {
+            uint8_t* slab = slab0 + (in_count & 1) * 4096;
+            if (elect_one()) {
+              tma_store_wait_read<0>();   // the other slab's results have left
+              in_fetch(in_count + 1);
+            }
+            __syncwarp();
+            if (!mbar_wait(&in_full[2 * (warp - 2) + (in_count & 1)], (in_count >> 1) & 1)) {
+              atomicCAS(status, ST_OK, ST_TIMEOUT_FULL);
+              *abort_flag = 1;
+            }
+            const int gc = col_base + half * 128 + 32 * i;
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(taddr + half * 128 + 32 * i, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {   // 64-byte swizzle: chunk q of row r sits at chunk q ^ ((r >> 1) & 3)
+              uint4* at = reinterpret_cast<uint4*>(slab + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4));
+              const uint4 gv = at[0], uv = at[2048 / 16];
+              const uint32_t gs[4] = {gv.x, gv.y, gv.z, gv.w}, us[4] = {uv.x, uv.y, uv.z, uv.w};
+              float a[8], b[8], d[8];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 x = pair(gs[j]), y = pair(us[j]);
+                // rounded as it was when it was stored
+                const float2 z = pair(pack_bf16x2(__uint_as_float(r[8 * q + 2 * j]), __uint_as_float(r[8 * q + 2 * j + 1])));
+                a[2 * j] = x.x; a[2 * j + 1] = x.y;
+                b[2 * j] = y.x; b[2 * j + 1] = y.y;
+                d[2 * j] = z.x; d[2 * j + 1] = z.y;
+              }
+              swiglu_grads(a, b, d);
+              at[0] = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
+              at[2048 / 16] = make_uint4(pack_bf16x2(b[0], b[1]), pack_bf16x2(b[2], b[3]), pack_bf16x2(b[4], b[5]), pack_bf16x2(b[6], b[7]));
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (elect_one()) {
+              tma_store_3d(tmW, slab, gc, 0, row0);
+              tma_store_3d(tmW, slab + 2048, gc, 1, row0);
+              tma_store_commit();
+            }
+          }
         }
       } else
 #pragma unroll 1

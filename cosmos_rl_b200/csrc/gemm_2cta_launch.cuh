@@ -6,7 +6,7 @@
 namespace b200 {
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int EPI, bool TAIL = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2_threads(EPI), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, int M, int N, int K,
                   Gemm2Params ep, uint32_t* status) {

@@ -92,18 +92,18 @@ void want(Py_ssize_t n, Py_ssize_t count) {
 }
 
 // ---- one entry for a launcher ------------------------------------------------------------------------------------
-template <class... A, size_t... I>
-PyObject* launch(int (*fn)(A...), PyObject* const* args, std::index_sequence<I...>) {
+template <class R, class... A, size_t... I>
+PyObject* launch(R (*fn)(A...), PyObject* const* args, std::index_sequence<I...>) {
   const std::tuple<A...> a{Arg<A>::of(args[I])...};
-  int rc;
+  R rc;
   {
     Unlocked unlocked;
     rc = std::apply(fn, a);
   }
-  return PyLong_FromLong(rc);
+  return PyLong_FromLongLong(rc);
 }
-template <class... A>
-PyObject* launch_all(int (*fn)(A...), PyObject* const* args, Py_ssize_t n) {
+template <class R, class... A>
+PyObject* launch_all(R (*fn)(A...), PyObject* const* args, Py_ssize_t n) {
   want(n, sizeof...(A));
   return launch(fn, args, std::index_sequence_for<A...>{});
 }
@@ -384,6 +384,9 @@ PyMethodDef methods[] = {
     LAUNCHER(b200_swiglu_fwd),
     LAUNCHER(b200_rope_inplace),
     LAUNCHER(b200_flash_bwd),
+    LAUNCHER(b200_gemm_gate_up),
+    LAUNCHER(b200_gemm_dgate_up),
+    LAUNCHER(b200_gemm_gated_scratch),
     LAUNCHER(b200_gemm_skinny_splits),
     LAUNCHER(b200_gemm_skinny),
     LAUNCHER(b200_splitk_reduce_residual_rmsnorm),

@@ -151,6 +151,11 @@ def _linear(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor] = None) 
     return y if lora is None else lora.apply(x, y)
 
 
+def _plain(w: torch.Tensor) -> bool:
+    """A weight that ``_linear`` gives to the bf16 GEMM and nothing else."""
+    return not (hasattr(w, "_lora") or hasattr(w, "_fp8") or getattr(w, "_fp8_train", False))
+
+
 class Attention(nn.Module):
     def __init__(self, a: GPTArgs):
         super().__init__()
@@ -233,7 +238,10 @@ class FeedForward(nn.Module):
 
     def forward(self, x, tp=None):
         if tp is None:
-            return _linear(F.swiglu(_linear(x, self.gate_up_proj.weight)), self.down_proj.weight)
+            w_in, w_out = self.gate_up_proj.weight, self.down_proj.weight
+            if _plain(w_in) and _plain(w_out):
+                return F.gated_mlp(x, w_in, w_out)
+            return _linear(F.swiglu(_linear(x, w_in)), w_out)
         return tp.row_linear(F.swiglu(tp.col_linear(x, self.gate_up_proj.weight)), self.down_proj.weight)
 
 

@@ -283,6 +283,14 @@ def _tc_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     return x.is_cuda and native.host().linear_ok(x, weight)
 
 
+def _weight_grad(weight: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor) -> Optional[torch.Tensor]:
+    """``dy2^T x2``, or None if it was accumulated into ``weight.grad``."""
+    if weight.grad is not None and weight.grad.dtype in (torch.bfloat16, torch.float32) and weight.grad.stride(-1) == 1:
+        gemm(dy2, x2, a_mn=True, b_mn=True, out=weight.grad, accumulate=True)
+        return None
+    return gemm(dy2, x2, a_mn=True, b_mn=True)
+
+
 class _LinearTC(torch.autograd.Function):
     """``y = x W^T (+ b)`` with forward, dgrad and wgrad on the tcgen05 GEMM. The bias is added in the forward
     epilogue; when ``W.grad`` already exists the weight gradient is accumulated into it by the GEMM epilogue itself
@@ -308,14 +316,7 @@ class _LinearTC(torch.autograd.Function):
         x2, weight = ctx.saved_tensors
         dy2 = _rows(dy)
         dx = gemm(dy2, weight, b_mn=True) if ctx.needs_input_grad[0] else None
-        dw = None
-        if ctx.needs_input_grad[1]:
-            if weight.grad is not None and weight.grad.dtype in (torch.bfloat16, torch.float32) \
-                    and weight.grad.stride(-1) == 1:
-                gemm(dy2, x2, a_mn=True, b_mn=True, out=weight.grad, accumulate=True)
-                dw = None  # accumulated in place
-            else:
-                dw = gemm(dy2, x2, a_mn=True, b_mn=True)
+        dw = _weight_grad(weight, dy2, x2) if ctx.needs_input_grad[1] else None
         db = dy2.sum(0) if ctx.has_bias and ctx.needs_input_grad[2] else None
         return (dx.view(ctx.shape) if dx is not None and len(ctx.shape) != 2 else dx), dw, db
 
@@ -329,6 +330,75 @@ def linear_tc(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
         y = linear_infer(_rows(x), weight, bias)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], weight.shape[0])
     return torch.nn.functional.linear(x, weight, bias)
+
+
+def _gated_workspace(a: torch.Tensor, I: int, backward: bool, sms: int):
+    """Scratch of such a GEMM on ``a`` (none where there is no room: its last round stays whole) and its size."""
+    floats = native.host().b200_gemm_gated_scratch(a.shape[0], I, a.shape[1], backward, sms)
+    if floats:
+        try:
+            return torch.empty(floats, dtype=torch.float32, device=a.device), floats
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return None, 0
+
+
+# Fewer rows have passes of a few microseconds, and tiles too few to hide an epilogue that computes. us, projection and pass, and
+# one kernel, forward and backward: 300 x 4096 x 14336 98 and 104, 73 and 74; 640 x 3584 x 18944 180 and 176, 119 and 109; 1003 x
+# 4096 x 14336 205 and 194, 136 and 126; 8192 x 3584 x 18944 (under the power cap) 1820 and 1610, 1120 and 930.
+_GATED_MLP_ROWS = 512
+
+
+class _GatedMLP(torch.autograd.Function):
+    """``(silu(x Wg^T) * (x Wu^T)) Wd^T`` for a fused ``[2 I, H]`` weight. The product and its gradient are formed in the epilogues
+    of the GEMMs around them; the bits are those of the separate passes (``linear_tc`` and ``swiglu``)."""
+
+    @staticmethod
+    def forward(ctx, x, w_gate_up, w_down):
+        x2 = _rows(x)
+        M, I = x2.shape[0], w_gate_up.shape[0] // 2
+        gu = torch.empty(M, 2 * I, dtype=torch.bfloat16, device=x.device)
+        act = torch.empty(M, I, dtype=torch.bfloat16, device=x.device)
+        sms = native.num_sms(x.device.index)
+        ws, floats = _gated_workspace(x2, I, False, sms)
+        native.check(native.host().b200_gemm_gate_up(x2, w_gate_up, gu, act, M, I, x2.shape[1], x2.stride(0), w_gate_up.stride(0),
+                                                     ws, floats, native.status_word(x.device), sms, native.stream()),
+                     "gemm_gate_up")
+        ctx.save_for_backward(x2, w_gate_up, w_down, gu, act)
+        ctx.shape = x.shape
+        y = gemm(act, w_down)
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[1])
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, w_gate_up, w_down, gu, act = ctx.saved_tensors
+        dy2 = _rows(dy)
+        dx = dgu = dw_gate_up = dw_down = None
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
+            dgu, sms = torch.empty_like(gu), native.num_sms(dy.device.index)
+            ws, floats = _gated_workspace(dy2, act.shape[1], True, sms)
+            native.check(native.host().b200_gemm_dgate_up(dy2, w_down, gu, dgu, gu.shape[0], act.shape[1], dy2.shape[1],
+                                                          dy2.stride(0), w_down.stride(0), ws, floats,
+                                                          native.status_word(dy.device), sms, native.stream()), "gemm_dgate_up")
+        if ctx.needs_input_grad[2]:
+            dw_down = _weight_grad(w_down, dy2, act)
+        if ctx.needs_input_grad[0]:
+            dx = gemm(dgu, w_gate_up, b_mn=True)
+            if len(ctx.shape) != 2:
+                dx = dx.view(ctx.shape)
+        if ctx.needs_input_grad[1]:
+            dw_gate_up = _weight_grad(w_gate_up, dgu, x2)
+        return dx, dw_gate_up, dw_down
+
+
+def gated_mlp(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> torch.Tensor:
+    """``linear(swiglu(linear(x, w_gate_up)), w_down)``; in training on CUDA (bf16, from _GATED_MLP_ROWS rows) without passes over the
+    activation of their own."""
+    rows = x.numel() // max(1, x.shape[-1])
+    if needs_graph(x, w_gate_up, w_down) and rows >= _GATED_MLP_ROWS and _tc_ok(x, w_gate_up) and _tc_ok(x, w_down) \
+            and w_gate_up.shape[0] == 2 * w_down.shape[1] and w_down.shape[1] % 8 == 0:
+        return _GatedMLP.apply(x, w_gate_up, w_down)
+    return linear_tc(swiglu(linear_tc(x, w_gate_up)), w_down)
 
 
 def _dims_ok(*ts: torch.Tensor) -> bool:

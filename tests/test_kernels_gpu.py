@@ -1958,3 +1958,54 @@ def test_swiglu_epilogues_of_special_gates(M):
     ok = torch.isfinite(want)
     # __expf is good to 2^-21 of a result of up to 2^6 in its exponent; one rounding to bf16
     assert torch.allclose(got[:, ok].float(), want[ok].float().expand(M, -1), rtol=2 ** -7, atol=1e-30)
+
+
+@pytest.mark.parametrize("M,H,I", [(512, 64, 8), (513, 264, 136), (700, 256, 1000), (1100, 4104, 1160), (640, 3584, 2432)])
+def test_gated_mlp_matches_its_separate_passes(M, H, I):
+    """Blocks of 128 and 32 columns that end early, a last row block of one row, last rounds that are cut and that are not; gradients
+    new and added to."""
+    torch.manual_seed(93)
+    x = _bf16(M, H).requires_grad_(True)
+    wg, wd = _bf16(2 * I, H, scale=0.05).requires_grad_(True), _bf16(H, I, scale=0.05).requires_grad_(True)
+    dy, before = _bf16(M, H), _bf16(2 * I, H)
+    y = F.gated_mlp(x, wg, wd)
+    assert "GatedMLP" in type(y.grad_fn).__name__
+    wg.grad = before.clone()
+    y.backward(dy)
+    native.read_status(x.device)
+    got = [y.detach(), x.grad, wg.grad, wd.grad]
+    xs, ws, ds = (t.detach().clone().requires_grad_(True) for t in (x, wg, wd))
+    ws.grad = before.clone()
+    z = F.linear_tc(F.swiglu(F.linear_tc(xs, ws)), ds)
+    z.backward(dy)
+    native.read_status(x.device)
+    for a, b in zip(got, (z.detach(), xs.grad, ws.grad, ds.grad)):
+        # the same roundings; sums of cut tiles in another order turn some of them, and what follows sums over those
+        assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
+    # one side of the gradients at a time
+    for needs in ((True, False, False), (False, True, False), (False, False, True)):
+        ins = [t.detach().clone().requires_grad_(n) for t, n in zip((x, wg, wd), needs)]
+        F.gated_mlp(*ins).backward(dy)
+        for t, n, ref in zip(ins, needs, (xs.grad, None, ds.grad)):
+            assert (t.grad is not None) == n
+            if n and ref is not None:
+                assert (t.grad.float() - ref.float()).norm() <= 2 ** -8 * ref.float().norm()
+    native.read_status(x.device)
+
+
+def test_gated_mlp_without_room_for_scratch(monkeypatch):
+    """Shares of a last round need scratch; without it the round stays whole."""
+    from cosmos_rl_b200.ops import functional
+    torch.manual_seed(94)
+    M, H, I = 600, 4096, 3840
+    assert native.host().b200_gemm_gated_scratch(M, I, H, False, native.num_sms(0)) > 0
+    x, wg, wd = _bf16(M, H).requires_grad_(True), _bf16(2 * I, H, scale=0.02), _bf16(H, I, scale=0.02)
+    dy, outs = _bf16(M, H), []
+    for room in (True, False):
+        if not room:
+            monkeypatch.setattr(functional, "_gated_workspace", lambda *a: (None, 0))
+        y = F.gated_mlp(x, wg, wd)
+        outs.append((y.detach(), torch.autograd.grad(y, x, dy)[0]))
+        native.read_status(x.device)
+    for a, b in zip(*outs):
+        assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
