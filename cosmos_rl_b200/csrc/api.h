@@ -143,6 +143,9 @@ int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float*
                       void* dw, float* ws, long long T, int H, cudaStream_t stream);
 int b200_rope_inplace(void* q, void* k, const long long* positions, int T, int hq, int hkv, int d, long long q_stride,
                       long long k_stride, float theta, int backward, cudaStream_t stream);
+// The same from one [T, (hq + 2 hkv) d] tensor into another, values copied; d a multiple of 16 up to 512, rows on 16-byte boundaries
+int b200_rope_qkv(const void* src, void* dst, const long long* positions, int T, int hq, int hkv, int d, long long src_stride,
+                  long long dst_stride, float theta, int backward, cudaStream_t stream);
 // row_tiles (device, nullable): only the first row_tiles[0] * 128 of the T rows are in use.
 int b200_swiglu_fwd(const void* gate_up, void* out, long long T, int I, const int* row_tiles, cudaStream_t stream);
 int b200_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, long long T, int I, const int* row_tiles,

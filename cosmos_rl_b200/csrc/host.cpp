@@ -251,6 +251,30 @@ PyObject* rope_qkv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// (qkv [T, (hq + 2 hkv) d], positions, hq, hkv, d, theta, backward, stream) -> a new tensor, q and k columns rotated. None: not a
+// matrix that the kernel takes.
+PyObject* rope_qkv_new(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  want(n, 8);
+  const Tensor &qkv = tensor(a[0]), &pos = tensor(a[1]);
+  const int hq = Arg<int>::of(a[2]), hkv = Arg<int>::of(a[3]), d = Arg<int>::of(a[4]), backward = flag(a[6]);
+  const float theta = (float)real(a[5]);
+  const cudaStream_t s = stream_of(a[7]);
+  if (qkv.dim() != 2 || !bf16(qkv) || qkv.stride(1) != 1 || hq <= 0 || hkv <= 0 || d <= 0 || d % 16 || d > 512 ||
+      qkv.size(1) != (int64_t)(hq + 2 * hkv) * d || qkv.stride(0) % 8 || ((uintptr_t)mem(qkv) & 15))
+    Py_RETURN_NONE;
+  Tensor out;
+  int rc;
+  {
+    Unlocked unlocked;
+    out = like(qkv, qkv.sizes());
+    rc = b200_rope_qkv(mem(qkv), mem(out), (const long long*)mem(pos), i32(qkv.size(0)), hq, hkv, d, qkv.stride(0), out.stride(0), theta,
+                       backward, s);
+  }
+  return rc ? PyLong_FromLong(rc) : give(out);
+  END_HANDLE_TH_ERRORS
+}
+
 // whether the tensor-core GEMMs take x and weight: they move rows with TMA, feature dimensions must give 16-byte rows
 PyObject* linear_ok(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -376,6 +400,7 @@ PyMethodDef methods[] = {
     ENTRY("swiglu_fwd", swiglu_fwd),
     ENTRY("swiglu_bwd", swiglu_bwd),
     ENTRY("rope_qkv", rope_qkv),
+    ENTRY("rope_qkv_new", rope_qkv_new),
     ENTRY("linear_ok", linear_ok),
     ENTRY("skinny_linear", skinny_linear),
     ENTRY("gemm", gemm),

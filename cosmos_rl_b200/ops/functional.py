@@ -167,9 +167,13 @@ class _RoPEQKV(torch.autograd.Function):
     def backward(ctx, dqkv):
         (positions,) = ctx.saved_tensors
         hq, hkv, d, theta = ctx.cfg
-        dqkv = dqkv.clone(memory_format=torch.contiguous_format)
-        _rope_qkv_native(dqkv, positions, hq, hkv, d, theta, True)
-        return dqkv, None, None, None, None, None
+        out = native.host().rope_qkv_new(dqkv, positions, hq, hkv, d, theta, True, native.stream())
+        if out is None:
+            out = dqkv.clone(memory_format=torch.contiguous_format)
+            _rope_qkv_native(out, positions, hq, hkv, d, theta, True)
+        else:
+            native.tensors(out, "rope")
+        return out, None, None, None, None, None
 
 
 def rope_qkv_(qkv: torch.Tensor, positions: torch.Tensor, hq: int, hkv: int, d: int, theta: float) -> torch.Tensor:

@@ -2009,3 +2009,26 @@ def test_gated_mlp_without_room_for_scratch(monkeypatch):
         native.read_status(x.device)
     for a, b in zip(*outs):
         assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
+
+
+@pytest.mark.parametrize("T,hq,hkv,d", [(1, 1, 1, 16), (7, 3, 1, 48), (593, 4, 2, 128), (1184, 62, 5, 128), (601, 2, 1, 512)])
+def test_rope_rows_in_place_and_into_a_new_tensor(T, hq, hkv, d):
+    """One token a CTA and two, a token left over, tokens of one part and of two; the backward's new tensor has the rotated columns of
+    the in-place form and the values as they were."""
+    torch.manual_seed(95)
+    qkv, pos = _bf16(T, (hq + 2 * hkv) * d), torch.randint(0, 40000, (T,), device=DEV)
+    for back in (False, True):
+        inplace = qkv.clone()
+        F._rope_qkv_native(inplace, pos, hq, hkv, d, 1e6, back)
+        new = native.host().rope_qkv_new(qkv, pos, hq, hkv, d, 1e6, back, native.stream())
+        assert torch.equal(new, inplace) and torch.equal(new[:, (hq + hkv) * d:], qkv[:, (hq + hkv) * d:])
+        inv = 1e6 ** (-torch.arange(0, d, 2, device=DEV, dtype=torch.float64) / d)
+        ang = pos.double()[:, None] * inv * (-1 if back else 1)
+        x = qkv[:, :(hq + hkv) * d].double().view(T, hq + hkv, d)
+        a, b, c, s = x[..., :d // 2], x[..., d // 2:], ang.cos()[:, None], ang.sin()[:, None]
+        want = torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+        # angles of up to 40000 with an fp32 rounding and a power good to 2 ulp: 40000 * 2^-22; one rounding to bf16
+        size = torch.cat([(a.square() + b.square()).sqrt()] * 2, dim=-1)
+        assert ((new[:, :(hq + hkv) * d].double().view_as(want) - want).abs() <= 2 ** -8 * want.abs() + 40000 * 2.0 ** -22 * size).all()
+    for bad in (qkv[:, ::2], qkv[:, :-1], qkv[:, 1:]):
+        assert native.host().rope_qkv_new(bad, pos, hq, hkv, d, 1e6, True, native.stream()) is None
