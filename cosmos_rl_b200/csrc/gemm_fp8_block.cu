@@ -11,13 +11,16 @@
 //   one CTA, 128 x 128 tiles: four buffers, six 32 KB stages, two warps a TMEM lane quadrant with 64 columns each
 //   CTA pair, 256 x 256 tiles: half the operand bytes of a product from L2 and shared memory; each CTA has two buffers of
 //   its 128 rows x 256 columns, handed over by halves of 128 columns
-// What bounds them, 4096 x 37888 x 3584 on pairs: 32 tiles of 28 k-blocks a pair, 896 k-blocks of 512 cycles of products. In the
-// steady state the hand-over of a buffer (release, wait, products, commit, wait, four loads) takes 1100 cycles for the two
-// k-blocks in flight, 650 a k-block where it was traced, which is 490 000 to 580 000 of the 830 000 cycles of a call; where the
-// others go, between tiles or in waits for operands, has not been measured. The clock falls under such calls: ten of them after a
-// pause 506 us each, 590 us in a loop of a second. What counted, ten calls at a time: a form that waits for its scales, writes
-// rows from registers and issues from one thread 845 us; scales multiplied when they are used 667; results through TMA stores and
-// two issuers 613; loads in flight under the multiplications 539; CTA pairs 488 to 506 (2198 to 2282 TFLOP/s; 1885 in the loop).
+// What bounds them, 4096 x 37888 x 3584 on pairs: 32 tiles of 28 k-blocks a pair, 896 k-blocks of 512 cycles of products; 458 752
+// of the 624 000 cycles of a call the tensor pipe is busy. A k-block takes 634 cycles, 524 in a form that hands the buffers over
+// and scales nothing, 541 with its TMEM loads alone and 550 with its products alone; a tile's end takes the promotion warps 1700
+// more (the next tile's place and scales 535, bf16 into the slabs 600), of which the two k-blocks ahead hide part. Fewer cycles
+// buy less than their share of time, for the clock falls under such calls: 777 000 cycles at 1.57 GHz became 624 000 at 1.41, ten
+// calls after a pause 494 us and then 440, 544 and 488 in a loop of a second; products without hand-over are 372 and 410.
+// What counted before, ten calls at a time: a form that waits for its scales, writes rows from registers and issues from one
+// thread 845 us; scales multiplied when they are used 667; results through TMA stores and two issuers 613; loads in flight under
+// the multiplications 539; CTA pairs 488 to 506. One issuer with 256-column products 490, one that takes the halves in turn 467,
+// the next tile's scales fetched inside the loop 449: slower than 440.
 // Operands arrive by TMA (128-byte swizzle, a 128-byte row = 128 fp8 elements). Persistent CTAs, bounded waits.
 #include "gemm_core.cuh"
 #include "gemm_2cta_launch.cuh"
@@ -81,16 +84,16 @@ struct F8Scales {
   }
 };
 
-// One warp's share of a tile: 32 rows x 32 NCH columns. acc = sum over the k-blocks of scale x accumulator; `it` counts the
-// k-blocks of all tiles. The next 32 columns are on their way out of TMEM while the present ones are multiplied, and the
-// barrier of the next k-block is asked before the answer is needed: a warp that does one after the other takes 400 cycles
-// for 64 columns. taddr(it): first column of the accumulator; wait / ready(it): it is complete; release(it): it has been read.
-template <int NCH, class Addr, class Wait, class Ready, class Release>
-__device__ __forceinline__ bool f8_promote(float2 (&acc)[16 * NCH], F8Scales& sc, uint32_t& it, Addr taddr, Wait wait, Ready ready,
-                                           Release release) {
-  static_assert(NCH % 2 == 0, "the two register buffers alternate");
+// One warp's share of a tile: acc = sum over the k-blocks of scale x accumulator; `it` counts the k-blocks of all tiles.
+// taddr(it): first column of the accumulator; wait / ready(it): it is complete; release(it): it has been read. The barrier of
+// the next k-block is asked before the answer is needed.
+// 64 columns (single CTAs): 32 at a time, the next 32 on their way out of TMEM while the present ones are multiplied. A warp
+// that does one after the other takes 400 cycles a k-block.
+template <class Addr, class Wait, class Ready, class Release>
+__device__ __forceinline__ bool f8_promote64(float2 (&acc)[32], F8Scales& sc, uint32_t& it, Addr taddr, Wait wait, Ready ready,
+                                             Release release) {
 #pragma unroll
-  for (int c = 0; c < 16 * NCH; ++c) acc[c] = make_float2(0.f, 0.f);
+  for (int c = 0; c < 32; ++c) acc[c] = make_float2(0.f, 0.f);
   const int num_kb = sc.num_kb;
   uint32_t r[2][32];
   if (!wait(it)) return false;
@@ -106,32 +109,89 @@ __device__ __forceinline__ bool f8_promote(float2 (&acc)[16 * NCH], F8Scales& sc
     cur[2] = cur[3];
     const bool more = kb + 1 < num_kb;
     bool rdy = false;
+    auto multiply = [&](float2* to, const uint32_t (&v)[32]) {
 #pragma unroll
-    for (int c = 0; c < NCH; ++c) {
-      uint32_t(&v)[32] = r[c & 1];
-      tmem_ld_wait(v);
-      if (c + 1 < NCH) {
-        tmem_ld_32x32b_x32(taddr(it) + (c + 1) * 32, r[(c + 1) & 1]);
-        if (c + 2 == NCH && more) rdy = ready(it + 1);
-      } else {
-        tc_fence_before_sync();
-        __syncwarp();
-        release(it);
-        rdy = __all_sync(0xffffffffu, rdy);
-        if (rdy) {
-          tc_fence_after_sync();
-          tmem_ld_32x32b_x32(taddr(it + 1), r[0]);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        acc[16 * c + j] = fma2(s, make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), acc[16 * c + j]);
+      for (int j = 0; j < 16; ++j) to[j] = fma2(s, make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), to[j]);
+    };
+    tmem_ld_wait(r[0]);
+    tmem_ld_32x32b_x32(taddr(it) + 32, r[1]);
+    if (more) rdy = ready(it + 1);
+    multiply(acc, r[0]);
+    tmem_ld_wait(r[1]);
+    tc_fence_before_sync();
+    __syncwarp();
+    release(it);
+    rdy = __all_sync(0xffffffffu, rdy);
+    if (rdy) {
+      tc_fence_after_sync();
+      tmem_ld_32x32b_x32(taddr(it + 1), r[0]);
     }
+    multiply(acc + 16, r[1]);
     ++it;
     if (more && !rdy) {
       if (!wait(it)) return false;
       tc_fence_after_sync();
       tmem_ld_32x32b_x32(taddr(it), r[0]);
+    }
+  }
+  return true;
+}
+
+// 128 columns (CTA pairs): 64 are read out of TMEM and waited for at once, and each 32 registers are loaded again as soon as
+// they have been multiplied. By 32 columns as above a k-block meets four waits instead of two: 494 us, not 440, for
+// 4096 x 37888 x 3584. (64 columns at once in single CTAs leave nothing to overlap: 102 us, not 97, for 1500 x 4096 x 14336.)
+template <class Addr, class Wait, class Ready, class Release>
+__device__ __forceinline__ bool f8_promote128(float2 (&acc)[64], F8Scales& sc, uint32_t& it, Addr taddr, Wait wait, Ready ready,
+                                              Release release) {
+#pragma unroll
+  for (int c = 0; c < 64; ++c) acc[c] = make_float2(0.f, 0.f);
+  const int num_kb = sc.num_kb;
+  uint32_t r[2][32];
+  auto load = [&](uint32_t t) {
+    tmem_ld_32x32b_x32(t, r[0]);
+    tmem_ld_32x32b_x32(t + 32, r[1]);
+  };
+  if (!wait(it)) return false;
+  tc_fence_after_sync();
+  load(taddr(it));
+  float cur[4];
+#pragma unroll 1
+  for (int kb = 0; kb < num_kb; ++kb) {
+    if ((kb & 3) == 0) sc.next(kb, cur);
+    const float2 s = make_float2(cur[0], cur[0]);
+    cur[0] = cur[1];
+    cur[1] = cur[2];
+    cur[2] = cur[3];
+    const bool more = kb + 1 < num_kb;
+#pragma unroll
+    for (int c = 0; c < 4; c += 2) {
+      tmem_ld_wait(r[0]);
+      tmem_ld_wait(r[1]);
+      if (c + 2 == 4) {
+        tc_fence_before_sync();
+        __syncwarp();
+        release(it);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          acc[16 * (c + h) + j] =
+              fma2(s, make_float2(__uint_as_float(r[h][2 * j]), __uint_as_float(r[h][2 * j + 1])), acc[16 * (c + h) + j]);
+        if (c + 2 < 4) tmem_ld_32x32b_x32(taddr(it) + (c + 2 + h) * 32, r[h]);
+      }
+    }
+    bool rdy = more && ready(it + 1);
+    rdy = __all_sync(0xffffffffu, rdy);
+    if (rdy) {
+      tc_fence_after_sync();
+      load(taddr(it + 1));
+    }
+    ++it;
+    if (more && !rdy) {
+      if (!wait(it)) return false;
+      tc_fence_after_sync();
+      load(taddr(it));
     }
   }
   return true;
@@ -261,7 +321,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     for (int i = blockIdx.x; i < total; i += gridDim.x) {
       float2 acc[32];
-      if (!f8_promote<2>(acc, sc, it, taddr, wait, ready, release)) break;
+      if (!f8_promote64(acc, sc, it, taddr, wait, ready, release)) break;
       const int row0 = m_blk * F8_BM + quad * 32, col0 = n_blk * F8_BN + chalf * 64;
       if (i + (int)gridDim.x < total) {   // the next tile's first scales come under the stores
         tile_of(i + gridDim.x, m_blk, n_blk);
@@ -383,7 +443,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
     for (int i = pair0; i < total; i += pairs) {
       float2 acc[64];
-      if (!f8_promote<4>(acc, sc, it, taddr, wait, ready, release)) break;
+      if (!f8_promote128(acc, sc, it, taddr, wait, ready, release)) break;
       const int row0 = m_blk * 2 * F8_BM + row_in, col0 = n_blk * FP_BN + col_in;
       if (i + pairs < total) {   // the next tile's first scales come under the stores
         tile_of(i + pairs, m_blk, n_blk);
@@ -478,10 +538,11 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 static long long f8_tiles(int M, int N, int rows, int cols) { return (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols); }
 
-// CTA pairs of a call, 0: single CTAs, or an error code. Rounds of tiles decide: a pair's round takes 1.8 times as long as one of
-// single CTAs and does twice the work at most. us, pairs and single CTAs: 8192^3 488 and 514, 1000 x 28672 x 4096 119 and 122,
-// 129 x 37888 x 3584 35 and 38; 300 x 28672 x 4096 67 and 50, 1500 x 4096 x 14336 111 and 91. Half of a pair would stand idle up to
-// 128 rows.
+// CTA pairs of a call, 0: single CTAs, or an error code. Rounds of tiles decide: a pair does at most twice the work of a single
+// CTA in its round, which takes 1.5 to 1.7 times as long, up to 1.9 times with K = 512; the line lies at 1.8, where no K loses.
+// us, pairs and single CTAs (a cold L2): 8192^3 406 and 507, 1000 x 28672 x 4096 106 and 123, 129 x 37888 x 3584 42 and 49;
+// 300 x 28672 x 4096 66 and 60; below the line 640 x 28672 (5 rounds and 8) 81 and 84 with K = 4096, 24.6 and 23.5 with 512. Half
+// of a pair would stand idle up to 128 rows.
 static int f8_pairs(int M, int N, int num_sms) {
   if (num_sms < 2 || M <= F8_BM) return 0;
   static int whole[16] = {0};
