@@ -37,7 +37,7 @@ constexpr int G2_BK = 64;
 constexpr int G2_THREADS = 192;
 
 enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3, G2_EPI_LOGPROB = 4, G2_EPI_GATE_UP = 5,
-       G2_EPI_DGATE_UP = 6 };
+       G2_EPI_DGATE_UP = 6, G2_EPI_GROUPED = 7 };
 
 // Epilogue warps of a CTA: two a TMEM lane quadrant where the epilogue computes (8192 x 18944 x 3584, backward: 1084
 // us with one, 911)
@@ -152,6 +152,7 @@ struct Gemm2Params {
   DlogitsParams dl;  // G2_EPI_DLOGITS
   // G2_EPI_EXPERTS: C is [experts, M, N], and expert e contracts over rows [offsets[e], offsets[e + 1]) of A and B (multiples
   // of 64; both MN-major), or over the blocks of 64 that its first filled[e] rows reach into (nullable)
+  // G2_EPI_GROUPED: rows [offsets[e], offsets[e + 1]) of A and C belong to B[e] (multiples of 32)
   const int* offsets;
   const int* filled;
   int experts;
@@ -173,6 +174,7 @@ __device__ __forceinline__ void g2_tile_coords(int i, int num_m, int num_n, int 
 // What a pair works on, one unit after the other: its share of a cut tile, then whole tiles.
 struct G2Unit {
   int m_blk, n_blk, batch, kb0, kb1;
+  int row, row_end;   // G2_EPI_GROUPED: first row of the tile, end of the expert's
   bool cut;
 };
 struct G2Work {
@@ -232,6 +234,45 @@ struct G2ExpertWork {
     u.kb0 = offsets[u.batch] / G2_BK;
     u.kb1 = offsets[u.batch + 1] / G2_BK;
     if (filled) u.kb1 = min(u.kb1, u.kb0 + (filled[u.batch] + G2_BK - 1) / G2_BK);
+    u.cut = false;
+    return true;
+  }
+};
+
+// G2_EPI_GROUPED: the tiles of every expert's rows, which start anew with each; up to 16 row blocks of an expert run side by side,
+// so that a tile of its weights comes from HBM once (columns first: 470 -> 607 us, 8 experts of 28672 x 4096, 256 rows each).
+// `get` is called with rising `it` and walks on from expert to expert.
+struct G2GroupedWork {
+  int num_n, num_kb, experts, e, base, row, row_end;   // the expert under way, its first unit and its rows
+  const int* offsets;
+  __device__ __forceinline__ void init(const Gemm2Params& ep, bool, int, int num_n_, int num_kb_) {
+    num_n = num_n_;
+    num_kb = num_kb_;
+    experts = ep.experts;
+    offsets = ep.offsets;
+    e = base = 0;
+    row = offsets[0];
+    row_end = offsets[1];
+  }
+  __device__ __forceinline__ bool get(int it, G2Unit& u) {
+    const int i = (blockIdx.x >> 1) + it * (gridDim.x >> 1);
+    int num_m = (row_end - row + G2_BM - 1) / G2_BM;
+    while (i - base >= num_m * num_n) {
+      if (++e >= experts) {
+        e = experts - 1;
+        return false;
+      }
+      base += num_m * num_n;
+      row = row_end;
+      row_end = offsets[e + 1];
+      num_m = (row_end - row + G2_BM - 1) / G2_BM;
+    }
+    g2_tile_coords(i - base, num_m, num_n, 16, u.m_blk, u.n_blk);
+    u.row = row + u.m_blk * G2_BM;
+    u.row_end = row_end;
+    u.batch = e;
+    u.kb0 = 0;
+    u.kb1 = num_kb;
     u.cut = false;
     return true;
   }
@@ -323,7 +364,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   constexpr int OUT_BN = GATED ? BN / 2 : BN;  // columns of C per tile
   const int n_cols = GATED ? N / 2 : N;        // columns of C
   const int num_n = (n_cols + OUT_BN - 1) / OUT_BN;
-  std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork, std::conditional_t<EPI == G2_EPI_LOGPROB, G2LogprobWork, G2Work>> work;
+  std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork,
+                     std::conditional_t<EPI == G2_EPI_LOGPROB, G2LogprobWork,
+                                        std::conditional_t<EPI == G2_EPI_GROUPED, G2GroupedWork, G2Work>>> work;
   work.init(ep, EPI == G2_EPI_STORE || EPI == G2_EPI_GATE_UP || EPI == G2_EPI_DGATE_UP, num_m, num_n, (K + G2_BK - 1) / G2_BK);
   G2Unit unit;
 
@@ -333,10 +376,11 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int it = 0; work.get(it, unit) && ok && !*abort_flag; ++it) {
-        const int m_blk = unit.m_blk, n_blk = unit.n_blk;
-        // rows of A that lie outside the tensor are not fetched: it takes longer than fetching rows that exist
-        const bool peer_rows = m_blk * G2_BM + G2_BM_CTA < M;
-        const int a_row0 = m_blk * G2_BM + (int)cta_rank * G2_BM_CTA;
+        const int n_blk = unit.n_blk;
+        // rows of A that lie outside the tensor (or the expert) are not fetched: it takes longer than fetching rows that exist
+        const int tile_row = EPI == G2_EPI_GROUPED ? unit.row : unit.m_blk * G2_BM;
+        const bool peer_rows = tile_row + G2_BM_CTA < (EPI == G2_EPI_GROUPED ? unit.row_end : M);
+        const int a_row0 = tile_row + (int)cta_rank * G2_BM_CTA;
         // rows of B that this CTA feeds: its half of the tile's columns; with the SwiGLU epilogue the leader
         // feeds the gate rows and the other CTA the matching up rows, so a thread sees both in its TMEM lane
         int b_row0;
@@ -361,7 +405,12 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
 #pragma unroll
             for (int j = 0; j < G2_BM_CTA / 64; ++j) tma_load_2d_pair(sa + j * 8192, tmA, bar, a_row0 + j * 64, k);
           }
-          if constexpr (!B_MN) {
+          if constexpr (EPI == G2_EPI_GROUPED && !B_MN) {
+            tma_load_3d_pair(sb, tmB, bar, k, b_row0, unit.batch);
+          } else if constexpr (EPI == G2_EPI_GROUPED) {
+#pragma unroll
+            for (int j = 0; j < (BN / 2) / 64; ++j) tma_load_3d_pair(sb + j * 8192, tmB, bar, b_row0 + j * 64, k, unit.batch);
+          } else if constexpr (!B_MN) {
             tma_load_2d_pair(sb, tmB, bar, k, b_row0);
           } else {
 #pragma unroll
@@ -465,7 +514,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       }
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
-      const int row0 = m_blk * G2_BM + (int)cta_rank * G2_BM_CTA + quad * 32;  // first row of this warp's slabs
+      // first row of this warp's slabs, and where the rows of C end
+      const int row0 = (EPI == G2_EPI_GROUPED ? unit.row : m_blk * G2_BM) + (int)cta_rank * G2_BM_CTA + quad * 32;
+      const int row_end = EPI == G2_EPI_GROUPED ? unit.row_end : M;
       const int col_base = n_blk * OUT_BN;
       const bool cut = EPI == G2_EPI_STORE && unit.cut;             // fp32 into the pair's part of the workspace
       const bool out_fp32 = cut || ep.out_fp32;
@@ -609,7 +660,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         // epilogue (28672 x 4096 over 64 rows: 70 us, 54). Two warps a quadrant in place of a stage: 45 there, but 73 and 69
         // over 300 rows.
         uint32_t plain[2][32];
-        if constexpr (EPI == G2_EPI_STORE || EPI == G2_EPI_EXPERTS) {
+        if constexpr (EPI == G2_EPI_STORE || EPI == G2_EPI_EXPERTS || EPI == G2_EPI_GROUPED) {
           tmem_ld_32x32b_x32(taddr + c, plain[0]);
           if (!out_fp32) tmem_ld_32x32b_x32(taddr + c + 32, plain[1]);
           tmem_ld_wait();
@@ -666,7 +717,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
         __syncwarp();
         const int gc = col_base + c;
         if (elect_one()) {
-          if (gc < (TAIL && !cut ? whole16(n_cols, ep.out_fp32) : n_cols) && row0 < M) {
+          if (gc < (TAIL && !cut ? whole16(n_cols, ep.out_fp32) : n_cols) && row0 < row_end) {
             if constexpr (EPI == G2_EPI_EXPERTS) {
               if (ep.accumulate) tma_reduce_add_3d(tmC, slab, gc, row0, unit.batch);
               else tma_store_3d(tmC, slab, gc, row0, unit.batch);

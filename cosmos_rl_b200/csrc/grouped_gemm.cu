@@ -5,8 +5,8 @@
 // Tokens routed to the local experts are stored sorted by expert in one [Mp, *] buffer in which every
 // expert's block starts on a multiple of 128 rows (padding rows are zero). Then a 128-row output tile belongs
 // to exactly one expert and a 64-row contraction block never straddles two experts, so all three GEMMs run on
-// the dense pipeline of gemm_core.cuh with a different tile schedule and 3-D tensor maps over the stacked
-// expert weights [E, N, K]:
+// the dense pipelines of gemm_core.cuh and, on CTA pairs, gemm_2cta.cuh with a different tile schedule and 3-D tensor maps
+// over the stacked expert weights [E, N, K]:
 //   forward  Y[Mp, N]   = X[Mp, K] . W[e]^T                      (A 2-D K-major, B 3-D K-major, z = expert)
 //   dgrad    dX[Mp, K]  = dY[Mp, N] . W[e]                       (A 2-D K-major, B 3-D MN-major)
 //   wgrad    dW[e][N,K] (+)= dY[rows of e]^T . X[rows of e]      (A, B 2-D MN-major, contraction = the expert's rows)
@@ -240,36 +240,81 @@ static int wgrad_pairs(int max_rows, int N, int K, int num_experts, int out_fp32
   return 5 * rounds(pair_tiles, np) <= 6 * rounds(tiles(GEMM_BM), num_sms) ? np : 0;
 }
 
+// CTA pairs of a call of grouped GEMMs, 0: single CTAs, or an error code. A single CTA fetches 48 KB out of L2 for a block of
+// 128 x 256 x 64, and that bounds it (770 cycles a block, products 512); a pair fetches 64 KB for twice the work. us, single CTAs
+// and pairs (a cold L2), rows an expert in brackets: 16 experts of 1536 x 2048 94 and 80 (1024), 155 and 140 (2048); 16 of 1024 x 512
+// 44 and 38 (2048); 8 of 28672 x 4096 2028 and 1398 (1024); input gradient of 8 of 14336 x 4096 905 and 699 (1024).
+// Up to 128 rows half of a pair stands idle: 153 and 159 (64). Tiles of 256 rows are rounded up once an expert: with a tenth more
+// rounds than single CTAs have pairs are no slower (64 of 1408 x 2048 151 and 143 (384)), with more it varies (128 of 1536 x 2048,
+// 1.2, 224 and 226; of 2048 x 768 126 and 120; 5 rounds for 4, 413 and 433; 3 for 2, 19.4 and 23.6). Short contractions and few tiles
+// are bound by what a tile costs beside its products (16 of 256 x 256 15.3 and 17.4 (2048)). max_rows is what there is room for,
+// about 64 rows an expert more than the padded rows there are, from which both numbers of tiles are estimated.
+using GR_SMEM = Gemm2Smem<256, 6, G2_EPI_GROUPED>;
+template <bool B_MN>
+constexpr auto grouped_pair_kernel = gemm2_bf16_kernel<256, 6, false, B_MN, G2_EPI_GROUPED>;
+static int grouped_pairs(int max_rows, int N, int K, int num_experts, int mode, int num_sms) {
+  if (num_sms < 2 || (N & 7) || K < 512 || max_rows < 320ll * num_experts) return 0;
+  static int whole[2][16] = {};
+  int np = 0;
+  if (const int rc = resident_pairs(mode == 0 ? grouped_pair_kernel<false> : grouped_pair_kernel<true>, whole[mode != 0],
+                                    GR_SMEM::TOTAL, G2_THREADS, num_sms, np))
+    return rc;
+  const long long num_n = (N + 255) / 256, pair_tiles = max_rows * num_n / G2_BM;
+  const long long tiles = (max_rows - 64ll * num_experts) * num_n / GEMM_BM;
+  if (pair_tiles < 2 * np || pair_tiles >= (1ll << 30)) return 0;
+  return 10 * ((pair_tiles + np - 1) / np) <= 11 * ((tiles + num_sms - 1) / num_sms) ? np : 0;
+}
+
 }  // namespace b200
 
 extern "C" {
 
 // mode 0: Y[Mp, N] = X[Mp, K] . W[e]^T with W [E, N, K]
 // mode 1: dX[Mp, N] = dY[Mp, K] . W[e]   with W [E, K, N]   (K is the contraction = rows of W[e])
+// expert_offsets [E + 1] (nullable): the experts' first rows, for tiles of 256 rows that begin with each
+int b200_grouped_gemm_rows(const void* X, const void* W, void* Y, int max_rows, int N, int K, int num_experts,
+                           long long ldx, long long ldy, const int* expert_offsets, const int* tile_expert, const int* n_tiles,
+                           int mode, int accumulate, uint32_t* status, int num_sms, cudaStream_t stream) {
+  using namespace b200;
+  if (max_rows <= 0 || N <= 0 || K <= 0 || (ldx & 7) || (max_rows % GEMM_BM)) return B200_ERR_ARG;
+  const int np = expert_offsets && !accumulate ? grouped_pairs(max_rows, N, K, num_experts, mode, num_sms) : 0;
+  if (np < 0) return np;
+  CUtensorMap tmA, tmB, tmC;
+  if (np > 0 ? make_tmap_out(&tmC, Y, max_rows, N, ldy, 0)
+             : make_tmap_grouped_out(&tmC, Y, 1, max_rows, N, ldy, (uint64_t)max_rows * ldy, 0))
+    return B200_ERR_TENSORMAP;
+  if (make_tmap_2d(&tmA, X, max_rows, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  // W[e] stored [K(contraction), N(out)]: MN-major B, boxes of 64 contraction rows x 64 output columns
+  if (mode == 0 ? make_tmap_3d(&tmB, W, num_experts, N, K, K, (uint64_t)N * K, np > 0 ? 128 : GG_BN, GEMM_BK, 2)
+                : make_tmap_3d(&tmB, W, num_experts, K, N, N, (uint64_t)N * K, 64, 64, 2))
+    return B200_ERR_TENSORMAP;
+  if (np > 0) {
+    Gemm2Params ep2{};
+    ep2.a_bytes = GR_SMEM::A_BYTES;
+    ep2.offsets = expert_offsets;
+    ep2.experts = num_experts;
+    const auto pair_kern = mode == 0 ? grouped_pair_kernel<false> : grouped_pair_kernel<true>;
+    pair_kern<<<2 * np, G2_THREADS, GR_SMEM::TOTAL, stream>>>(tmA, tmB, tmC, tmC, max_rows, N, K, ep2, status);
+    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  }
+  static bool s0 = false, s1 = false;
+  GroupedParams ep{nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles, num_experts};
+  if (mode == 0 ? set_smem(grouped_fwd_kernel, s0) : set_smem(grouped_dgrad_kernel, s1)) return B200_ERR_LAUNCH;
+  const auto kern = mode == 0 ? grouped_fwd_kernel : grouped_dgrad_kernel;
+  kern<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, max_rows, N, K, ep, status);
+  return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+}
+
+// Whether such a call that is given the experts' first rows takes CTA pairs.
+int b200_grouped_gemm_pairs(int max_rows, int N, int K, int num_experts, int mode, int num_sms) {
+  return b200::grouped_pairs(max_rows, N, K, num_experts, mode, num_sms) > 0;
+}
+
 int b200_grouped_gemm(const void* X, const void* W, void* Y, int max_rows, int N, int K, int num_experts,
                       long long ldx, long long ldy, const int* tile_expert, const int* n_tiles, int mode,
                       int accumulate, uint32_t* status, int num_sms, cudaStream_t stream) {
-  using namespace b200;
-  if (max_rows <= 0 || N <= 0 || K <= 0 || (ldx & 7) || (max_rows % GEMM_BM)) return B200_ERR_ARG;
-  CUtensorMap tmA, tmB, tmC;
-  if (make_tmap_grouped_out(&tmC, Y, 1, max_rows, N, ldy, (uint64_t)max_rows * ldy, 0)) return B200_ERR_TENSORMAP;
-  if (make_tmap_2d(&tmA, X, max_rows, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
-  static bool s0 = false, s1 = false;
-  GroupedParams ep{nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles, num_experts};
-  const int grid = num_sms;
-  if (mode == 0) {
-    if (make_tmap_3d(&tmB, W, num_experts, N, K, K, (uint64_t)N * K, GG_BN, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
-    if (set_smem(grouped_fwd_kernel, s0)) return B200_ERR_LAUNCH;
-    grouped_fwd_kernel<<<grid, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, max_rows, N,
-                                                                                                   K, ep, status);
-  } else {
-    // W[e] stored [K(contraction), N(out)]: MN-major B, boxes of 64 contraction rows x 64 output columns
-    if (make_tmap_3d(&tmB, W, num_experts, K, N, N, (uint64_t)N * K, 64, 64, 2)) return B200_ERR_TENSORMAP;
-    if (set_smem(grouped_dgrad_kernel, s1)) return B200_ERR_LAUNCH;
-    grouped_dgrad_kernel<<<grid, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, max_rows,
-                                                                                                     N, K, ep, status);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  return b200_grouped_gemm_rows(X, W, Y, max_rows, N, K, num_experts, ldx, ldy, nullptr, tile_expert, n_tiles, mode, accumulate,
+                                status, num_sms, stream);
 }
 
 // Whether such a call of expert weight gradients takes CTA pairs.

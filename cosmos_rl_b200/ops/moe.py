@@ -111,9 +111,9 @@ def _grouped(x, w, disp: _Dispatch, mode: int, n_out: int) -> torch.Tensor:
     y = torch.empty(disp.max_rows, n_out, dtype=torch.bfloat16, device=x.device)
     st = native.status_word(x.device)
     dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
-    native.check(native.host().b200_grouped_gemm(x, w, y, disp.max_rows, n_out, K, disp.E, x.stride(0), y.stride(0),
-                                                 disp.tile_expert, disp.n_tiles, mode, 0, st, native.num_sms(dev),
-                                                 native.stream()), "grouped_gemm")
+    native.check(native.host().b200_grouped_gemm_rows(x, w, y, disp.max_rows, n_out, K, disp.E, x.stride(0), y.stride(0),
+                                                      disp.offsets, disp.tile_expert, disp.n_tiles, mode, 0, st,
+                                                      native.num_sms(dev), native.stream()), "grouped_gemm")
     return y
 
 

@@ -575,6 +575,41 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
+# rows an expert: none, one, a whole pair of row blocks, one row more, the second block's last row; columns and contractions that
+# end inside a tile; more row blocks than run side by side
+@pytest.mark.parametrize("E,N,K,rows", [(40, 1032, 520, [0, 1, 256, 257, 511, 640, 129, 384]), (3, 1280, 512, [4500, 0, 4200]),
+                                        (64, 512, 840, [255, 513, 300])])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_grouped_gemm_on_pairs(E, N, K, rows, mode):
+    rows = [rows[e % len(rows)] for e in range(E)]
+    padded = [(r + 127) // 128 * 128 for r in rows]
+    Mp = sum(padded) + 128 * E
+    assert native.lib().b200_grouped_gemm_pairs(Mp, N, K, E, mode, native.num_sms(0)) == 1
+    torch.manual_seed(E)
+    offsets = torch.tensor([0] + padded, dtype=torch.int32).cumsum(0).to(torch.int32)
+    x = torch.zeros(Mp, K, dtype=torch.bfloat16, device="cuda")
+    for e, r in enumerate(rows):
+        x[offsets[e]:offsets[e] + r] = torch.randn(r, K, device="cuda").to(torch.bfloat16)
+    w = torch.randn((E, N, K) if mode == 0 else (E, K, N), device="cuda").to(torch.bfloat16)
+    out = torch.full((Mp, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    tiles = torch.repeat_interleave(torch.arange(E, dtype=torch.int32), torch.tensor(padded) // 128).cuda()
+    n_tiles, first = torch.tensor([tiles.numel()], dtype=torch.int32, device="cuda"), offsets.cuda()
+    st = native.status_word(x.device)
+    native.check(native.lib().b200_grouped_gemm_rows(native.ptr(x), native.ptr(w), native.ptr(out), Mp, N, K, E, K, N,
+                                                     native.ptr(first), native.ptr(tiles), native.ptr(n_tiles), mode, 0,
+                                                     native.ptr(st), native.num_sms(0), native.stream()), "grouped_gemm")
+    torch.cuda.synchronize()
+    assert native.read_status(x.device) == 0
+    for e in range(E):
+        lo, hi = int(offsets[e]), int(offsets[e + 1])
+        a, b = x[lo:hi].double(), (w[e].t() if mode == 0 else w[e]).double()
+        # one rounding to bf16 (2^-9) and fp32 sums of K products, which a 64-bit sum bounds by 2^-24 K |a| |b|
+        bound = (a @ b).abs() * 2.0 ** -8 + 2.0 ** -24 * K * (a.abs() @ b.abs()) + 1e-30
+        assert ((out[lo:hi].double() - a @ b).abs() <= bound).all()
+    assert (out[offsets[E]:] == 7.0).all()
+
+
+@pytest.mark.gpu
 # ragged result rows and columns; experts without rows; fp32 sums; too few rows for CTA pairs; a round more than single CTAs have
 @pytest.mark.parametrize("E,N,K,rows,pairs", [(10, 1000, 520, [256, 0, 1280, 768, 0, 512, 2048, 256, 1024, 1536], True),
                                               (6, 1536, 768, [768] * 6, True), (40, 256, 520, [128] * 40, False),
