@@ -124,6 +124,9 @@ int b200_moe_combine(const void* y, const float* probs, const int* row_map, void
 int b200_moe_swiglu_bwd(const void* dact, const void* h1, const void* row_info, const int* n_tiles, void* dh1, void* ap,
                         float* dprob, int max_rows, int I, cudaStream_t stream);
 // Grouped GEMMs over the padded, expert-sorted token buffer (see grouped_gemm.cu for the three forms).
+int b200_grouped_gate_up(const void* X, const void* W, void* h1, void* act, int max_rows, int I, int K, int num_experts,
+                         long long ldx, const int* expert_offsets, const int* tile_expert, const int* n_tiles, uint32_t* status,
+                         int num_sms, cudaStream_t stream);
 int b200_grouped_gemm_pairs(int max_rows, int N, int K, int num_experts, int mode, int num_sms);
 int b200_grouped_gemm_rows(const void* X, const void* W, void* Y, int max_rows, int N, int K, int num_experts,
                            long long ldx, long long ldy, const int* expert_offsets, const int* tile_expert, const int* n_tiles,

@@ -78,7 +78,7 @@ struct TileInfo {
 // Epi::side() concurrently with the pipeline (used by the fused GEMM + cross-GPU reduction kernel).
 // PRODUCER_HOOK: the TMA producer calls sched.before_tile_load(tile, ep, status) before the first load of a tile
 // and gives up (abort) when it returns false (used to wait for operand rows that another GPU is still sending).
-// B_TWO_BOXES (K-major 2-D B only): the B tile is fetched as two boxes of BN / 2 rows starting at rows t.b_mn0 and
+// B_TWO_BOXES (K-major B only): the B tile is fetched as two boxes of BN / 2 rows starting at rows t.b_mn0 and
 // t.b_mn1 (gate and up rows of a fused gate/up weight, so that one accumulator row holds both).
 // L2_PREFETCH (B not MN-major, 2-D): before the CTA waits for the previous kernel of the stream it brings the first
 // ep.prefetch_kb contraction blocks of its B tiles into L2. The schedule's init() may then read nothing but Params.
@@ -248,8 +248,13 @@ __device__ __forceinline__ void gemm_mainloop(const CUtensorMap* tmA, const CUte
             }
           }
           if constexpr (Traits::B_TWO_BOXES) {
-            tma_load_2d(sb, tmB, &full_bar[stage], k, t.b_mn0);
-            tma_load_2d(sb + b_half, tmB, &full_bar[stage], k, t.b_mn1);
+            if constexpr (Traits::B_3D) {
+              tma_load_3d(sb, tmB, &full_bar[stage], k, t.b_mn0, t.batch);
+              tma_load_3d(sb + b_half, tmB, &full_bar[stage], k, t.b_mn1, t.batch);
+            } else {
+              tma_load_2d(sb, tmB, &full_bar[stage], k, t.b_mn0);
+              tma_load_2d(sb + b_half, tmB, &full_bar[stage], k, t.b_mn1);
+            }
           } else if constexpr (!Traits::B_MN) {
             if constexpr (Traits::B_3D) tma_load_3d(sb, tmB, &full_bar[stage], k, t.b_mn0, t.batch);
             else tma_load_2d(sb, tmB, &full_bar[stage], k, t.b_mn0);

@@ -10,22 +10,6 @@ namespace b200 {
 
 constexpr int MLP_STAGES = 5;   // with the staging slabs of eight warps
 
-// gate and up halves of a contiguous [rows, 2 I] tensor as [rows][2][I]: boxes of 32 rows x `cols` columns of one half
-static int make_tmap_halves(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t I, int cols, CUtensorMapSwizzle swizzle) {
-  PFN_encodeTiled enc = get_encode_tiled();
-  if (!enc) { last_tmap_error() = 1 << 24; return -1; }
-  cuuint64_t gdim[3] = {I, 2, rows};
-  cuuint64_t gstr[2] = {I * 2, I * 4};
-  cuuint32_t box[3] = {(cuuint32_t)cols, 1, 32};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = encode_with_context([&] {
-    return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstr, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  });
-  if (r != CUDA_SUCCESS) last_tmap_error() = (3 << 24) | 0x50000 | (int)r;
-  return r == CUDA_SUCCESS ? 0 : -3;
-}
-
 // Tiles that were cut along the contraction: the sum of their shares, in the order of the contraction, and the epilogue on it. A
 // warp has one row of a tile. Grid (rest, 256 / 8).
 template <int EPI>

@@ -20,6 +20,7 @@ namespace b200 {
 
 struct GroupedParams {
   const CUtensorMap* tm_out;  // output as [batches, rows, N] (batches = experts for wgrad, else 1): boxes of 32 rows x 128 bytes
+  const CUtensorMap* tm_act;  // gate/up projection: [rows, N / 2] activation, and tm_out is [rows][2][N / 2]
   const __nv_bfloat16* old;   // bf16 output that is accumulated into: its values are added in fp32 before the one rounding
   long long ld_old, batch_old;
   int N;                      // output columns
@@ -103,6 +104,74 @@ struct GroupedEpilogue {
   }
 };
 
+// Gate/up projection: 128 gate columns and the 128 up columns that go with them; they leave as they are, and with their
+// activation, which is formed from the rounded values and has the bits of a pass over them. The pass read and wrote 12 bytes an
+// element of it at memory speed; here it is 4, written under the next tile's products (4096 tokens, 8 of 128 experts of 768 each:
+// 217 us for the product and 36 for the pass, 232).
+struct GroupedGateUpEpilogue {
+  using Params = GroupedParams;
+  static constexpr bool CUSTOM_TILE = true;
+  uint32_t slab_idx = 0;
+  __device__ __forceinline__ void finish(const Params&) {
+    if (elect_one()) tma_store_wait<0>();
+  }
+  __device__ __forceinline__ void tile(const Params& p, const TileInfo& t, int, uint32_t taddr, uint8_t* epi_smem) {
+    const int lane = threadIdx.x & 31, quad = (threadIdx.x >> 5) & 3;
+    uint8_t* slab0 = epi_smem + quad * 8192;
+    const uint32_t sw = (uint32_t)(lane & 7);
+    const int row0 = t.m_blk * GEMM_BM + quad * 32, inter = p.N / 2;
+    auto put = [&](const uint32_t (&v)[32], auto store) {   // 64 columns as bf16 pairs, through the next staging slab
+      uint8_t* slab = slab0 + (slab_idx++ & 1) * 4096;
+      if (elect_one()) tma_store_wait_read<1>();   // the store issued two slabs ago has finished reading this buffer
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(slab + lane * 128 + ((((uint32_t)j) ^ sw) << 4)) =
+            make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (elect_one()) {
+        store(slab);
+        tma_store_commit();
+      }
+    };
+    auto fetch = [&](uint32_t col, uint32_t (&v)[32]) {   // accumulator columns col .. col + 63, rounded
+      uint32_t r[2][32];
+      tmem_ld_32x32b_x32(taddr + col, r[0]);
+      tmem_ld_32x32b_x32(taddr + col + 32, r[1]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        v[j] = pack_bf16x2(__uint_as_float(r[j >> 4][2 * (j & 15)]), __uint_as_float(r[j >> 4][2 * (j & 15) + 1]));
+    };
+#pragma unroll 1
+    for (int c = 0; c < 128; c += 64) {
+      const int gc = t.n_blk * 128 + c;
+      if (gc >= inter) break;
+      uint32_t g[32], u[32];
+      fetch(c, g);
+      put(g, [&](uint8_t* slab) { tma_store_3d(p.tm_out, slab, gc, 0, row0); });
+      fetch(128 + c, u);
+      put(u, [&](uint8_t* slab) { tma_store_3d(p.tm_out, slab, gc, 1, row0); });
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        float a[8], b[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          a[2 * j] = __uint_as_float(g[4 * q + j] << 16);
+          a[2 * j + 1] = __uint_as_float(g[4 * q + j] & 0xffff0000u);
+          b[2 * j] = __uint_as_float(u[4 * q + j] << 16);
+          b[2 * j + 1] = __uint_as_float(u[4 * q + j] & 0xffff0000u);
+        }
+        swiglu_values(a, b, a);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g[4 * q + j] = pack_bf16x2(a[2 * j], a[2 * j + 1]);
+      }
+      put(g, [&](uint8_t* slab) { tma_store_2d(p.tm_act, slab, gc, row0); });
+    }
+  }
+};
+
 // forward / dgrad: tiles = (128-row tile of the padded token buffer) x (BN-column tile)
 struct TokenTileSchedule {
   int num_n, total, num_kb, bn;
@@ -125,6 +194,20 @@ struct TokenTileSchedule {
     t.k0 = 0;
     t.num_kb = num_kb;
     t.batch = tile_expert[t.m_blk];
+    return true;
+  }
+};
+
+// gate/up projection: the same with 128 columns of either half of N
+struct GateUpTileSchedule : TokenTileSchedule {
+  int inter;
+  __device__ __forceinline__ void init(int M, int N, int K, int BN, const GroupedParams& p) {
+    TokenTileSchedule::init(M, N / 2, K, BN / 2, p);
+    inter = N / 2;
+  }
+  __device__ __forceinline__ bool get(int it, TileInfo& t) const {
+    if (!TokenTileSchedule::get(it, t)) return false;
+    t.b_mn1 = inter + t.b_mn0;
     return true;
   }
 };
@@ -165,6 +248,15 @@ grouped_fwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                    const __grid_constant__ CUtensorMap tmC, int M, int N, int K, GroupedParams ep, uint32_t* status) {
   ep.tm_out = &tmC;
   gemm_mainloop<GG_BN, GG_STAGES, GroupedEpilogue, TokenTileSchedule, GemmTraits<false, false, false, true>>(
+      &tmA, &tmB, M, N, K, ep, status);
+}
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+grouped_gate_up_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                       const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD, int M, int N, int K,
+                       GroupedParams ep, uint32_t* status) {
+  ep.tm_out = &tmC;
+  ep.tm_act = &tmD;
+  gemm_mainloop<GG_BN, GG_STAGES, GroupedGateUpEpilogue, GateUpTileSchedule, GemmTraits<false, false, false, true, 0, false, true>>(
       &tmA, &tmB, M, N, K, ep, status);
 }
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -298,10 +390,39 @@ int b200_grouped_gemm_rows(const void* X, const void* W, void* Y, int max_rows, 
     return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
   }
   static bool s0 = false, s1 = false;
-  GroupedParams ep{nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles, num_experts};
+  GroupedParams ep{nullptr, nullptr, accumulate ? (const __nv_bfloat16*)Y : nullptr, ldy, 0, N, max_rows, 0, accumulate, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles, num_experts};
   if (mode == 0 ? set_smem(grouped_fwd_kernel, s0) : set_smem(grouped_dgrad_kernel, s1)) return B200_ERR_LAUNCH;
   const auto kern = mode == 0 ? grouped_fwd_kernel : grouped_dgrad_kernel;
   kern<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, max_rows, N, K, ep, status);
+  return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+}
+
+// h1[Mp, 2 I] = X[Mp, K] . W[e]^T with W [E, 2 I, K] (gate rows, then up rows), act[Mp, I] = silu(gate) o up of the rounded h1.
+// Where the product takes CTA pairs the activation is a pass over it: pairs save more than the pass costs.
+int b200_grouped_gate_up(const void* X, const void* W, void* h1, void* act, int max_rows, int I, int K, int num_experts,
+                         long long ldx, const int* expert_offsets, const int* tile_expert, const int* n_tiles, uint32_t* status,
+                         int num_sms, cudaStream_t stream) {
+  using namespace b200;
+  if (max_rows <= 0 || I <= 0 || I > (1 << 30) || (I & 7) || K <= 0 || (ldx & 7) || (max_rows % GEMM_BM)) return B200_ERR_ARG;
+  const int np = grouped_pairs(max_rows, 2 * I, K, num_experts, 0, num_sms);
+  if (np < 0) return np;
+  if (np > 0) {
+    if (const int rc = b200_grouped_gemm_rows(X, W, h1, max_rows, 2 * I, K, num_experts, ldx, 2 * I, expert_offsets, tile_expert,
+                                              n_tiles, 0, 0, status, num_sms, stream))
+      return rc;
+    return b200_swiglu_fwd(h1, act, max_rows, I, n_tiles, stream);
+  }
+  CUtensorMap tmA, tmB, tmC, tmD;
+  if (make_tmap_2d(&tmA, X, max_rows, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_3d(&tmB, W, num_experts, 2 * I, K, K, (uint64_t)2 * I * K, GG_BN / 2, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
+  if (make_tmap_halves(&tmC, h1, max_rows, I, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return B200_ERR_TENSORMAP;
+  if (make_tmap_out(&tmD, act, max_rows, I, I, 0)) return B200_ERR_TENSORMAP;
+  static bool done = false;
+  if (set_smem(grouped_gate_up_kernel, done)) return B200_ERR_LAUNCH;
+  GroupedParams ep{nullptr, nullptr, nullptr, 2 * I, 0, 2 * I, max_rows, 0, 0, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles,
+                   num_experts};
+  grouped_gate_up_kernel<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, tmD, max_rows,
+                                                                                                       2 * I, K, ep, status);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 
@@ -350,7 +471,7 @@ int b200_grouped_wgrad_filled(const void* dY, const void* X, void* dW, int max_r
   }
   static bool s2 = false;
   if (set_smem(grouped_wgrad_kernel, s2)) return B200_ERR_LAUNCH;
-  GroupedParams ep{nullptr, accumulate && !out_fp32 ? (const __nv_bfloat16*)dW : nullptr, K, (long long)N * K, K, N, out_fp32,
+  GroupedParams ep{nullptr, nullptr, accumulate && !out_fp32 ? (const __nv_bfloat16*)dW : nullptr, K, (long long)N * K, K, N, out_fp32,
                    accumulate, GG_BN, 1, nullptr, expert_offsets, filled, nullptr, num_experts};
   grouped_wgrad_kernel<<<num_sms, GEMM_THREADS, GemmSmem<GG_BN, GG_STAGES>::TOTAL_WITH_EPI, stream>>>(tmA, tmB, tmC, N, K,
                                                                                                      0, ep, status);

@@ -429,6 +429,7 @@ PyMethodDef methods[] = {
     LAUNCHER(b200_moe_spread),
     LAUNCHER(b200_moe_swiglu_bwd),
     LAUNCHER(b200_moe_combine),
+    LAUNCHER(b200_grouped_gate_up),
     LAUNCHER(b200_grouped_gemm_rows),
     LAUNCHER(b200_grouped_wgrad_filled),
     {nullptr, nullptr, 0, nullptr},

@@ -100,10 +100,17 @@ def _rows16(x: torch.Tensor) -> torch.Tensor:
     return x if x.data_ptr() % 16 == 0 else x.clone()
 
 
-def _swiglu_rows(h1: torch.Tensor, disp: _Dispatch) -> torch.Tensor:
-    out = torch.empty(h1.shape[0], h1.shape[1] // 2, dtype=h1.dtype, device=h1.device)
-    native.check(native.host().b200_swiglu_fwd(h1, out, h1.shape[0], h1.shape[1] // 2, disp.n_tiles, native.stream()), "swiglu_fwd")
-    return out
+def _gate_up(x, w, disp: _Dispatch) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Gate and up values of the sorted rows, and their activation."""
+    I2, K = w.shape[1], x.shape[1]
+    h1 = torch.empty(disp.max_rows, I2, dtype=torch.bfloat16, device=x.device)
+    act = torch.empty(disp.max_rows, I2 // 2, dtype=torch.bfloat16, device=x.device)
+    st = native.status_word(x.device)
+    dev = x.device.index if x.device.index is not None else torch.cuda.current_device()
+    native.check(native.host().b200_grouped_gate_up(x, w, h1, act, disp.max_rows, I2 // 2, K, disp.E, x.stride(0), disp.offsets,
+                                                    disp.tile_expert, disp.n_tiles, st, native.num_sms(dev), native.stream()),
+                 "grouped_gate_up")
+    return h1, act
 
 
 def _grouped(x, w, disp: _Dispatch, mode: int, n_out: int) -> torch.Tensor:
@@ -142,8 +149,7 @@ class _MoEExperts(torch.autograd.Function):
         native.check(L.b200_moe_permute(_rows16(x), idx, disp.offsets, disp.cursor, disp.row_map, xp, T, k, H, native.stream()),
                      "moe_permute")
         disp.zero_padding(xp)
-        h1 = _grouped(xp, w_gate_up, disp, 0, I2)
-        act = _swiglu_rows(h1, disp)
+        h1, act = _gate_up(xp, w_gate_up, disp)
         y = _grouped(act, w_down, disp, 0, H)
         out = torch.empty(T, H, dtype=torch.bfloat16, device=x.device)
         probs = probs.float().contiguous()

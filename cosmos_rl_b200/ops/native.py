@@ -120,6 +120,7 @@ _SIGS = {
     "b200_grouped_gemm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p,
                           c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_grouped_gemm_pairs": [c_int] * 6,
+    "b200_grouped_gate_up": [c_void_p] * 4 + [c_int] * 4 + [c_longlong] + [c_void_p] * 4 + [c_int, c_void_p],
     "b200_grouped_gemm_rows": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p,
                                c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_grouped_wgrad_pairs": [c_int] * 7,

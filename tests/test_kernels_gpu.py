@@ -575,6 +575,39 @@ def test_gemm_fp8_block_scaled(M, N, K):
 
 
 @pytest.mark.gpu
+# half a box of activation columns, one tile and eight columns, the layer's; a contraction of less than a block, and of a ragged
+# number of them; enough rows for CTA pairs, and all other numbers that are not
+@pytest.mark.parametrize("I,K,rows", [(8, 40, [1, 0, 130]), (136, 264, [128, 300, 0, 5]), (768, 512, [0, 257, 64]),
+                                      (640, 512, [4500, 0, 4200])])
+def test_grouped_gate_up_has_the_bits_of_two_passes(I, K, rows):
+    E, lib, st = len(rows), native.lib(), native.status_word(torch.device("cuda"))
+    padded = [(r + 127) // 128 * 128 for r in rows]
+    Mp = sum(padded) + 128 * E
+    sms = native.num_sms(0)
+    assert lib.b200_grouped_gemm_pairs(Mp, 2 * I, K, E, 0, sms) == int(max(rows) > 4000)
+    torch.manual_seed(I)
+    first = torch.tensor([0] + padded, dtype=torch.int32).cumsum(0).to(torch.int32)
+    x = torch.zeros(Mp, K, dtype=torch.bfloat16, device="cuda")
+    for e, r in enumerate(rows):
+        x[first[e]:first[e] + r] = torch.randn(r, K, device="cuda").to(torch.bfloat16)
+    w = torch.randn(E, 2 * I, K, device="cuda").to(torch.bfloat16)
+    w[0, :I] *= 40.0                                         # gates whose exponential overflows
+    tiles = torch.repeat_interleave(torch.arange(E, dtype=torch.int32), torch.tensor(padded) // 128).cuda()
+    n_tiles, offsets = torch.tensor([tiles.numel()], dtype=torch.int32, device="cuda"), first.cuda()
+    h1, act = (torch.full((Mp, n), 7.0, dtype=torch.bfloat16, device="cuda") for n in (2 * I, I))
+    native.check(native.host().b200_grouped_gate_up(x, w, h1, act, Mp, I, K, E, K, offsets, tiles, n_tiles, st, sms, native.stream()),
+                 "grouped_gate_up")
+    want_h1, want = torch.full_like(h1, 7.0), torch.full_like(act, 7.0)
+    native.check(lib.b200_grouped_gemm(native.ptr(x), native.ptr(w), native.ptr(want_h1), Mp, 2 * I, K, E, K, 2 * I,
+                                       native.ptr(tiles), native.ptr(n_tiles), 0, 0, native.ptr(st), sms, native.stream()),
+                 "grouped_gemm")
+    native.check(lib.b200_swiglu_fwd(native.ptr(want_h1), native.ptr(want), Mp, I, native.ptr(n_tiles), native.stream()), "swiglu_fwd")
+    torch.cuda.synchronize()
+    assert native.read_status(x.device) == 0
+    assert torch.equal(h1, want_h1) and torch.equal(act.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.gpu
 # rows an expert: none, one, a whole pair of row blocks, one row more, the second block's last row; columns and contractions that
 # end inside a tile; more row blocks than run side by side
 @pytest.mark.parametrize("E,N,K,rows", [(40, 1032, 520, [0, 1, 256, 257, 511, 640, 129, 384]), (3, 1280, 512, [4500, 0, 4200]),
