@@ -37,11 +37,13 @@ constexpr int G2_BK = 64;
 constexpr int G2_THREADS = 192;
 
 enum { G2_EPI_STORE = 0, G2_EPI_SWIGLU = 1, G2_EPI_DLOGITS = 2, G2_EPI_EXPERTS = 3, G2_EPI_LOGPROB = 4, G2_EPI_GATE_UP = 5,
-       G2_EPI_DGATE_UP = 6, G2_EPI_GROUPED = 7 };
+       G2_EPI_DGATE_UP = 6, G2_EPI_GROUPED = 7, G2_EPI_GROUPED_GATE_UP = 8 };
 
 // Epilogue warps of a CTA: two a TMEM lane quadrant where the epilogue computes (8192 x 18944 x 3584, backward: 1084
 // us with one, 911)
-__host__ __device__ constexpr int g2_epilogue_warps(int epi) { return epi == G2_EPI_GATE_UP || epi == G2_EPI_DGATE_UP ? 8 : 4; }
+__host__ __device__ constexpr int g2_epilogue_warps(int epi) {
+  return epi == G2_EPI_GATE_UP || epi == G2_EPI_DGATE_UP || epi == G2_EPI_GROUPED_GATE_UP ? 8 : 4;
+}
 __host__ __device__ constexpr int g2_threads(int epi) { return 64 + 32 * g2_epilogue_warps(epi); }
 
 template <int BN, int STAGES, int EPI = G2_EPI_STORE>
@@ -152,7 +154,7 @@ struct Gemm2Params {
   DlogitsParams dl;  // G2_EPI_DLOGITS
   // G2_EPI_EXPERTS: C is [experts, M, N], and expert e contracts over rows [offsets[e], offsets[e + 1]) of A and B (multiples
   // of 64; both MN-major), or over the blocks of 64 that its first filled[e] rows reach into (nullable)
-  // G2_EPI_GROUPED: rows [offsets[e], offsets[e + 1]) of A and C belong to B[e] (multiples of 32)
+  // G2_EPI_GROUPED, _GROUPED_GATE_UP: rows [offsets[e], offsets[e + 1]) of A and C belong to B[e] (multiples of 32)
   const int* offsets;
   const int* filled;
   int experts;
@@ -360,13 +362,15 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
   const uint32_t tmem_base = *tmem_slot;
 
   const int num_m = (M + G2_BM - 1) / G2_BM;
-  constexpr bool GATED = EPI == G2_EPI_SWIGLU || EPI == G2_EPI_GATE_UP;   // half of a tile's columns are gates, half ups
+  constexpr bool GROUPED = EPI == G2_EPI_GROUPED || EPI == G2_EPI_GROUPED_GATE_UP;
+  constexpr bool GATE_UP = EPI == G2_EPI_GATE_UP || EPI == G2_EPI_GROUPED_GATE_UP;
+  constexpr bool GATED = EPI == G2_EPI_SWIGLU || GATE_UP;   // half of a tile's columns are gates, half ups
   constexpr int OUT_BN = GATED ? BN / 2 : BN;  // columns of C per tile
   const int n_cols = GATED ? N / 2 : N;        // columns of C
   const int num_n = (n_cols + OUT_BN - 1) / OUT_BN;
   std::conditional_t<EPI == G2_EPI_EXPERTS, G2ExpertWork,
                      std::conditional_t<EPI == G2_EPI_LOGPROB, G2LogprobWork,
-                                        std::conditional_t<EPI == G2_EPI_GROUPED, G2GroupedWork, G2Work>>> work;
+                                        std::conditional_t<GROUPED, G2GroupedWork, G2Work>>> work;
   work.init(ep, EPI == G2_EPI_STORE || EPI == G2_EPI_GATE_UP || EPI == G2_EPI_DGATE_UP, num_m, num_n, (K + G2_BK - 1) / G2_BK);
   G2Unit unit;
 
@@ -378,8 +382,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       for (int it = 0; work.get(it, unit) && ok && !*abort_flag; ++it) {
         const int n_blk = unit.n_blk;
         // rows of A that lie outside the tensor (or the expert) are not fetched: it takes longer than fetching rows that exist
-        const int tile_row = EPI == G2_EPI_GROUPED ? unit.row : unit.m_blk * G2_BM;
-        const bool peer_rows = tile_row + G2_BM_CTA < (EPI == G2_EPI_GROUPED ? unit.row_end : M);
+        const int tile_row = GROUPED ? unit.row : unit.m_blk * G2_BM;
+        const bool peer_rows = tile_row + G2_BM_CTA < (GROUPED ? unit.row_end : M);
         const int a_row0 = tile_row + (int)cta_rank * G2_BM_CTA;
         // rows of B that this CTA feeds: its half of the tile's columns; with the SwiGLU epilogue the leader
         // feeds the gate rows and the other CTA the matching up rows, so a thread sees both in its TMEM lane
@@ -405,9 +409,9 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
 #pragma unroll
             for (int j = 0; j < G2_BM_CTA / 64; ++j) tma_load_2d_pair(sa + j * 8192, tmA, bar, a_row0 + j * 64, k);
           }
-          if constexpr (EPI == G2_EPI_GROUPED && !B_MN) {
+          if constexpr (GROUPED && !B_MN) {
             tma_load_3d_pair(sb, tmB, bar, k, b_row0, unit.batch);
-          } else if constexpr (EPI == G2_EPI_GROUPED) {
+          } else if constexpr (GROUPED) {
 #pragma unroll
             for (int j = 0; j < (BN / 2) / 64; ++j) tma_load_3d_pair(sb + j * 8192, tmB, bar, b_row0 + j * 64, k, unit.batch);
           } else if constexpr (!B_MN) {
@@ -515,8 +519,8 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
       // first row of this warp's slabs, and where the rows of C end
-      const int row0 = (EPI == G2_EPI_GROUPED ? unit.row : m_blk * G2_BM) + (int)cta_rank * G2_BM_CTA + quad * 32;
-      const int row_end = EPI == G2_EPI_GROUPED ? unit.row_end : M;
+      const int row0 = (GROUPED ? unit.row : m_blk * G2_BM) + (int)cta_rank * G2_BM_CTA + quad * 32;
+      const int row_end = GROUPED ? unit.row_end : M;
       const int col_base = n_blk * OUT_BN;
       const bool cut = EPI == G2_EPI_STORE && unit.cut;             // fp32 into the pair's part of the workspace
       const bool out_fp32 = cut || ep.out_fp32;
@@ -541,7 +545,7 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
           lgr.chunk(ep.lg, col_base + c, v);
         }
-      } else if constexpr (EPI == G2_EPI_GATE_UP || EPI == G2_EPI_DGATE_UP) {
+      } else if constexpr (GATE_UP || EPI == G2_EPI_DGATE_UP) {
         auto pair = [](uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); };
         if (unit.cut) {   // fp32 into the pair's part of the workspace; gemm2_sum_gated_kernel does the rest
           float* dst = ep.ws + ((long long)(blockIdx.x >> 1) * G2_BM + (row0 - m_blk * G2_BM) + lane) * BN;
@@ -553,10 +557,10 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
 #pragma unroll
             for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
           }
-        } else if constexpr (EPI == G2_EPI_GATE_UP) {
+        } else if constexpr (GATE_UP) {
           // The gate and up values as they are stored, and what the SwiGLU kernel makes of them: the same bits as its pass over them.
           const int c = half * 64, gc = col_base + c;
-          if (gc < n_cols && row0 < M) {
+          if (gc < n_cols && row0 < row_end) {
             auto put = [&](const uint32_t (&v)[32], auto store) {   // 64 columns as bf16 pairs, through the next staging slab
               uint8_t* slab = slab0 + (slab_idx++ & 1) * 4096;
               if (elect_one()) tma_store_wait_read<1>();

@@ -107,7 +107,8 @@ struct GroupedEpilogue {
 // Gate/up projection: 128 gate columns and the 128 up columns that go with them; they leave as they are, and with their
 // activation, which is formed from the rounded values and has the bits of a pass over them. The pass read and wrote 12 bytes an
 // element of it at memory speed; here it is 4, written under the next tile's products (4096 tokens, 8 of 128 experts of 768 each:
-// 217 us for the product and 36 for the pass, 232).
+// 217 us for the product and 36 for the pass, 232). On CTA pairs G2_EPI_GROUPED_GATE_UP does the same (16 experts, 4096 tokens: the
+// layer forward and backward 1040 us with the pass, 1018).
 struct GroupedGateUpEpilogue {
   using Params = GroupedParams;
   static constexpr bool CUSTOM_TILE = true;
@@ -398,25 +399,31 @@ int b200_grouped_gemm_rows(const void* X, const void* W, void* Y, int max_rows, 
 }
 
 // h1[Mp, 2 I] = X[Mp, K] . W[e]^T with W [E, 2 I, K] (gate rows, then up rows), act[Mp, I] = silu(gate) o up of the rounded h1.
-// Where the product takes CTA pairs the activation is a pass over it: pairs save more than the pass costs.
 int b200_grouped_gate_up(const void* X, const void* W, void* h1, void* act, int max_rows, int I, int K, int num_experts,
                          long long ldx, const int* expert_offsets, const int* tile_expert, const int* n_tiles, uint32_t* status,
                          int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (max_rows <= 0 || I <= 0 || I > (1 << 30) || (I & 7) || K <= 0 || (ldx & 7) || (max_rows % GEMM_BM)) return B200_ERR_ARG;
-  const int np = grouped_pairs(max_rows, 2 * I, K, num_experts, 0, num_sms);
+  int np = grouped_pairs(max_rows, 2 * I, K, num_experts, 0, num_sms);
   if (np < 0) return np;
-  if (np > 0) {
-    if (const int rc = b200_grouped_gemm_rows(X, W, h1, max_rows, 2 * I, K, num_experts, ldx, 2 * I, expert_offsets, tile_expert,
-                                              n_tiles, 0, 0, status, num_sms, stream))
-      return rc;
-    return b200_swiglu_fwd(h1, act, max_rows, I, n_tiles, stream);
-  }
-  CUtensorMap tmA, tmB, tmC, tmD;
+  CUtensorMap tmA, tmB, tmC, tmD;   // both take boxes of 128 rows of A and of 128 gate or up rows
   if (make_tmap_2d(&tmA, X, max_rows, K, ldx, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_3d(&tmB, W, num_experts, 2 * I, K, K, (uint64_t)2 * I * K, GG_BN / 2, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
   if (make_tmap_halves(&tmC, h1, max_rows, I, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return B200_ERR_TENSORMAP;
   if (make_tmap_out(&tmD, act, max_rows, I, I, 0)) return B200_ERR_TENSORMAP;
+  if (np > 0) {
+    using SM = Gemm2Smem<256, 5, G2_EPI_GROUPED_GATE_UP>;
+    auto kern = gemm2_bf16_kernel<256, 5, false, false, G2_EPI_GROUPED_GATE_UP>;
+    static int whole[16] = {0};
+    if (const int rc = resident_pairs(kern, whole, SM::TOTAL, g2_threads(G2_EPI_GROUPED_GATE_UP), num_sms, np)) return rc;
+    Gemm2Params ep2{};
+    ep2.up_row0 = I;
+    ep2.a_bytes = SM::A_BYTES;
+    ep2.offsets = expert_offsets;
+    ep2.experts = num_experts;
+    kern<<<2 * np, g2_threads(G2_EPI_GROUPED_GATE_UP), SM::TOTAL, stream>>>(tmA, tmB, tmD, tmC, max_rows, 2 * I, K, ep2, status);
+    return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
+  }
   static bool done = false;
   if (set_smem(grouped_gate_up_kernel, done)) return B200_ERR_LAUNCH;
   GroupedParams ep{nullptr, nullptr, nullptr, 2 * I, 0, 2 * I, max_rows, 0, 0, GG_BN, 0, tile_expert, nullptr, nullptr, n_tiles,
