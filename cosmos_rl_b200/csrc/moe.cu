@@ -48,6 +48,10 @@ route_topk_kernel(const float* __restrict__ logits, int T, int E, int k, int ren
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    // A logit that is not a number leaves that in the token's weights; to the choice it is the least of values, so that every token
+    // has k experts of its own that exist, whatever its logits are: the kernels that follow address memory with them.
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = (lane + 32 * i) < E ? fmaxf(v[i], 0.f) : -1.f;
     const float inv = 1.f / s;
     float prob = 0.f, tsum = 0.f;
     int choice = 0;
@@ -75,7 +79,7 @@ route_topk_kernel(const float* __restrict__ logits, int T, int E, int k, int ren
     if (lane < k) {
       probs[(long long)token * k + lane] = prob * (renorm ? 1.f / tsum : 1.f);
       idx[(long long)token * k + lane] = choice;
-      if (choice < E) atomicAdd(&hist[choice], 1);   // logits that are not numbers have no choice
+      atomicAdd(&hist[choice], 1);
     }
   }
   if (counts) {

@@ -2100,3 +2100,28 @@ def test_rope_rows_in_place_and_into_a_new_tensor(T, hq, hkv, d):
         assert ((new[:, :(hq + hkv) * d].double().view_as(want) - want).abs() <= 2 ** -8 * want.abs() + 40000 * 2.0 ** -22 * size).all()
     for bad in (qkv[:, ::2], qkv[:, :-1], qkv[:, 1:]):
         assert native.host().rope_qkv_new(bad, pos, hq, hkv, d, 1e6, True, native.stream()) is None
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 8, 8), (40, 16, 8), (17, 33, 2), (33, 128, 8), (16, 256, 1)])
+@pytest.mark.parametrize("renorm", [False, True])
+def test_moe_router_of_logits_that_are_not_numbers(T, E, k, renorm):
+    """Rows that hold NaN or infinities, all over or here and there: k experts that exist, none twice, all of them counted, and
+    weights that show it. What the other rows get does not change."""
+    from cosmos_rl_b200.ops import moe
+    torch.manual_seed(96)
+    logits = torch.randn(T, E, device=DEV)
+    plain_p, plain_i = moe.route_topk(logits, k, renorm)
+    bad = torch.arange(T, device=DEV) % 5 != 4
+    kinds = torch.arange(T, device=DEV) % 5
+    logits[kinds == 0] = float("nan")
+    logits[kinds == 1, E - 1] = float("nan")
+    logits[kinds == 2] = float("-inf")
+    logits[kinds == 3, 0] = float("inf")
+    counts = torch.zeros(E, dtype=torch.int32, device=DEV)
+    p, i = moe.route_topk(logits, k, renorm, counts)
+    torch.cuda.synchronize()
+    assert int(i.min()) >= 0 and int(i.max()) < E
+    assert (i.sort(dim=-1).values.diff(dim=-1) > 0).all()
+    assert torch.equal(counts.long(), torch.bincount(i.flatten().long(), minlength=E)) and int(counts.sum()) == T * k
+    assert torch.isnan(p[bad]).all()
+    assert torch.equal(p[~bad], plain_p[~bad]) and torch.equal(i[~bad], plain_i[~bad])
