@@ -400,7 +400,7 @@ def gated_mlp(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) ->
     activation of their own."""
     rows = x.numel() // max(1, x.shape[-1])
     if needs_graph(x, w_gate_up, w_down) and rows >= _GATED_MLP_ROWS and _tc_ok(x, w_gate_up) and _tc_ok(x, w_down) \
-            and w_gate_up.shape[0] == 2 * w_down.shape[1] and w_down.shape[1] % 8 == 0:
+            and x.shape[-1] == w_gate_up.shape[1] and w_gate_up.shape[0] == 2 * w_down.shape[1] and w_down.shape[1] % 8 == 0:
         return _GatedMLP.apply(x, w_gate_up, w_down)
     return linear_tc(swiglu(linear_tc(x, w_gate_up)), w_down)
 

@@ -82,3 +82,29 @@ def test_launchers_refuse_what_cannot_be_launched():
         H.gemm(x, x, False, False, None, False, False, None, False, 0, None, -1, 0, 148, 0)      # not on a GPU
     with FakeTensorMode(), pytest.raises(RuntimeError, match="without memory"):
         H.swiglu_fwd(torch.empty(4, 8, dtype=torch.bfloat16, device="cuda"), 0)
+
+
+def test_gated_mlp_of_mismatched_shapes_goes_through_the_checked_calls(monkeypatch):
+    """The fused form hands the launcher one contraction for the activations and the weight: shapes that do not fit never reach it,
+    with few rows or many. (Tensors that only say that they are on a GPU.)"""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cosmos_rl_b200.ops import build, native
+    from cosmos_rl_b200.ops import functional as F
+    if not (native.available() and build.host_path().exists()):
+        pytest.skip("the kernel library is not built")
+    fused, separate = [], []
+    monkeypatch.setattr(F._GatedMLP, "apply", lambda x, *w: fused.append(tuple(x.shape)))
+    monkeypatch.setattr(F, "linear_tc", lambda x, w, *b: separate.append(tuple(x.shape)))
+    monkeypatch.setattr(F, "swiglu", lambda gu: torch.empty(1))
+    with FakeTensorMode():
+        make = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda", requires_grad=True)
+        for rows in (8, 512, 1000):
+            for width, gate_up, down in ((72, (96, 64), (64, 48)), (56, (96, 64), (64, 48)), (64, (96, 64), (64, 56))):
+                F.gated_mlp(make(rows, width), make(*gate_up), make(*down))
+                assert not fused and separate.pop(0) == (rows, width) and len(separate) == 1
+                separate.clear()
+        F.gated_mlp(make(512, 64), make(96, 64), make(64, 48))
+    assert fused == [(512, 64)] and not separate

@@ -2125,3 +2125,12 @@ def test_moe_router_of_logits_that_are_not_numbers(T, E, k, renorm):
     assert torch.equal(counts.long(), torch.bincount(i.flatten().long(), minlength=E)) and int(counts.sum()) == T * k
     assert torch.isnan(p[bad]).all()
     assert torch.equal(p[~bad], plain_p[~bad]) and torch.equal(i[~bad], plain_i[~bad])
+
+
+@pytest.mark.parametrize("M", [8, 511, 512, 1000])
+def test_gated_mlp_refuses_a_contraction_of_two_lengths(M):
+    """Activations that are wider or narrower than the weight raise, on either side of the rows that take the fused form."""
+    w_gate_up, w_down = _bf16(96, 64).requires_grad_(True), _bf16(64, 48)
+    for width in (56, 72):
+        with pytest.raises(AssertionError):
+            F.gated_mlp(_bf16(M, width), w_gate_up, w_down)
