@@ -370,8 +370,10 @@ class _GatedMLP(torch.autograd.Function):
                      "gemm_gate_up")
         ctx.save_for_backward(x2, w_gate_up, w_down, gu, act)
         ctx.shape = x.shape
-        y = gemm(act, w_down)
-        return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[1])
+        # in its final shape: a view that a custom function returns may not be changed in place
+        y = torch.empty(*x.shape[:-1], w_down.shape[0], dtype=torch.bfloat16, device=x.device)
+        gemm(act, w_down, out=_rows(y))
+        return y
 
     @staticmethod
     def backward(ctx, dy):

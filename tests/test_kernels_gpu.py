@@ -2134,3 +2134,19 @@ def test_gated_mlp_refuses_a_contraction_of_two_lengths(M):
     for width in (56, 72):
         with pytest.raises(AssertionError):
             F.gated_mlp(_bf16(M, width), w_gate_up, w_down)
+
+
+@pytest.mark.parametrize("shape", [(1, 600), (2, 3, 100), (600,)])
+def test_gated_mlp_result_may_be_changed_in_place(shape):
+    """Activations of any number of dimensions; what comes back is no view, which autograd would not let a caller change."""
+    torch.manual_seed(97)
+    x, wg, wd = _bf16(*shape, 64).requires_grad_(True), _bf16(96, 64, scale=0.1), _bf16(64, 48, scale=0.1)
+    y = F.gated_mlp(x, wg, wd)
+    assert "GatedMLP" in type(y.grad_fn).__name__ and y.shape == x.shape
+    before = y.detach().clone()
+    y.mul_(2.0)
+    dx, = torch.autograd.grad(y, x, torch.ones_like(y))
+    x2 = x.detach().reshape(-1, 64).requires_grad_(True)
+    z = F.gated_mlp(x2, wg, wd)
+    want, = torch.autograd.grad(z, x2, torch.full_like(z, 2.0))
+    assert torch.equal(before.view_as(z), z) and torch.equal(dx.view_as(want), want)
