@@ -353,12 +353,12 @@ def _gated_workspace(a: torch.Tensor, I: int, backward: bool, sms: int):
 _GATED_MLP_ROWS = 512
 
 
-class _GatedMLP(torch.autograd.Function):
-    """``(silu(x Wg^T) * (x Wu^T)) Wd^T`` for a fused ``[2 I, H]`` weight. The product and its gradient are formed in the epilogues
-    of the GEMMs around them; the bits are those of the separate passes (``linear_tc`` and ``swiglu``)."""
+class _GatedMLPIn(torch.autograd.Function):
+    """``x Wg^T`` and ``x Wu^T`` for a fused ``[2 I, H]`` weight, side by side, and ``silu`` of the one times the other, formed in the
+    epilogue of the GEMM. The product has no gradient of its own: :class:`_GatedMLPOut` gives that of the projections."""
 
     @staticmethod
-    def forward(ctx, x, w_gate_up, w_down):
+    def forward(ctx, x, w_gate_up):
         x2 = _rows(x)
         M, I = x2.shape[0], w_gate_up.shape[0] // 2
         gu = torch.empty(M, 2 * I, dtype=torch.bfloat16, device=x.device)
@@ -368,42 +368,57 @@ class _GatedMLP(torch.autograd.Function):
         native.check(native.host().b200_gemm_gate_up(x2, w_gate_up, gu, act, M, I, x2.shape[1], x2.stride(0), w_gate_up.stride(0),
                                                      ws, floats, native.status_word(x.device), sms, native.stream()),
                      "gemm_gate_up")
-        ctx.save_for_backward(x2, w_gate_up, w_down, gu, act)
+        ctx.save_for_backward(x2, w_gate_up)
         ctx.shape = x.shape
+        ctx.mark_non_differentiable(act)
+        ctx.set_materialize_grads(False)
+        return gu, act
+
+    @staticmethod
+    def backward(ctx, dgu, _):
+        x2, w_gate_up = ctx.saved_tensors
+        dx = gemm(dgu, w_gate_up, b_mn=True) if ctx.needs_input_grad[0] else None
+        dw = _weight_grad(w_gate_up, dgu, x2) if ctx.needs_input_grad[1] else None
+        return (dx.view(ctx.shape) if dx is not None and len(ctx.shape) != 2 else dx), dw
+
+
+class _GatedMLPOut(torch.autograd.Function):
+    """``act Wd^T`` in ``shape``; its backward goes through the activation, in the epilogue of the product's gradient, and gives the
+    gradient of the gate and up values. A function of its own, so that what it saves is gone when _GatedMLPIn's gradients are
+    formed: as one function both halves' five rows of I values a token live until the last of them is (8192 x 18944: 0.9 GB)."""
+
+    @staticmethod
+    def forward(ctx, gu, act, w_down, shape):
         # in its final shape: a view that a custom function returns may not be changed in place
-        y = torch.empty(*x.shape[:-1], w_down.shape[0], dtype=torch.bfloat16, device=x.device)
+        y = torch.empty(*shape, w_down.shape[0], dtype=torch.bfloat16, device=gu.device)
         gemm(act, w_down, out=_rows(y))
+        ctx.save_for_backward(gu, act, w_down)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w_gate_up, w_down, gu, act = ctx.saved_tensors
+        gu, act, w_down = ctx.saved_tensors
         dy2 = _rows(dy)
-        dx = dgu = dw_gate_up = dw_down = None
-        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
+        dgu = None
+        if ctx.needs_input_grad[0]:
             dgu, sms = torch.empty_like(gu), native.num_sms(dy.device.index)
             ws, floats = _gated_workspace(dy2, act.shape[1], True, sms)
             native.check(native.host().b200_gemm_dgate_up(dy2, w_down, gu, dgu, gu.shape[0], act.shape[1], dy2.shape[1],
                                                           dy2.stride(0), w_down.stride(0), ws, floats,
                                                           native.status_word(dy.device), sms, native.stream()), "gemm_dgate_up")
-        if ctx.needs_input_grad[2]:
-            dw_down = _weight_grad(w_down, dy2, act)
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dgu, w_gate_up, b_mn=True)
-            if len(ctx.shape) != 2:
-                dx = dx.view(ctx.shape)
-        if ctx.needs_input_grad[1]:
-            dw_gate_up = _weight_grad(w_gate_up, dgu, x2)
-        return dx, dw_gate_up, dw_down
+        dw = _weight_grad(w_down, dy2, act) if ctx.needs_input_grad[2] else None
+        return dgu, None, dw, None
 
 
 def gated_mlp(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> torch.Tensor:
     """``linear(swiglu(linear(x, w_gate_up)), w_down)``; in training on CUDA (bf16, from _GATED_MLP_ROWS rows) without passes over the
-    activation of their own."""
+    activation of their own, otherwise by those three calls. The sums are theirs but where a last round of tiles is cut: the two
+    GEMMs cut other tiles than the plain ones do, so shares come in another order there."""
     rows = x.numel() // max(1, x.shape[-1])
     if needs_graph(x, w_gate_up, w_down) and rows >= _GATED_MLP_ROWS and _tc_ok(x, w_gate_up) and _tc_ok(x, w_down) \
             and x.shape[-1] == w_gate_up.shape[1] and w_gate_up.shape[0] == 2 * w_down.shape[1] and w_down.shape[1] % 8 == 0:
-        return _GatedMLP.apply(x, w_gate_up, w_down)
+        gu, act = _GatedMLPIn.apply(x, w_gate_up)
+        return _GatedMLPOut.apply(gu, act, w_down, x.shape[:-1])
     return linear_tc(swiglu(linear_tc(x, w_gate_up)), w_down)
 
 

@@ -96,7 +96,8 @@ def test_gated_mlp_of_mismatched_shapes_goes_through_the_checked_calls(monkeypat
     if not (native.available() and build.host_path().exists()):
         pytest.skip("the kernel library is not built")
     fused, separate = [], []
-    monkeypatch.setattr(F._GatedMLP, "apply", lambda x, *w: fused.append(tuple(x.shape)))
+    monkeypatch.setattr(F._GatedMLPIn, "apply", lambda x, w: (fused.append(tuple(x.shape)), None))
+    monkeypatch.setattr(F._GatedMLPOut, "apply", lambda *a: None)
     monkeypatch.setattr(F, "linear_tc", lambda x, w, *b: separate.append(tuple(x.shape)))
     monkeypatch.setattr(F, "swiglu", lambda gu: torch.empty(1))
     with FakeTensorMode():

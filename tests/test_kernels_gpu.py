@@ -2150,3 +2150,27 @@ def test_gated_mlp_result_may_be_changed_in_place(shape):
     z = F.gated_mlp(x2, wg, wd)
     want, = torch.autograd.grad(z, x2, torch.full_like(z, 2.0))
     assert torch.equal(before.view_as(z), z) and torch.equal(dx.view_as(want), want)
+
+
+def test_gated_mlp_backward_holds_no_more_than_its_separate_passes():
+    """What the activation's gradient was formed from is given back before the gate/up projection's gradients are formed."""
+    torch.manual_seed(98)
+    M, H, I = 2048, 2048, 4096
+    x, wg, wd = _bf16(M, H).requires_grad_(True), _bf16(2 * I, H, scale=0.02).requires_grad_(True), _bf16(H, I, scale=0.02).requires_grad_(True)
+    dy = _bf16(M, H)
+
+    def peak(fn):
+        for _ in range(2):      # the second time with what the first keeps
+            y = fn()
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            grads = torch.autograd.grad(y, (x, wg, wd), dy)
+            most = torch.cuda.max_memory_allocated() - before
+            del y, grads
+        return most
+
+    separate = peak(lambda: F.linear_tc(F.swiglu(F.linear_tc(x, wg)), wd))
+    fused = peak(lambda: F.gated_mlp(x, wg, wd))
+    scratch = 4 * native.host().b200_gemm_gated_scratch(M, I, H, True, native.num_sms(0))
+    assert scratch < 2 * M * I and fused <= separate + scratch      # one row of I values more a token would show
