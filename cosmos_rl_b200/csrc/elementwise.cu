@@ -700,13 +700,16 @@ int b200_rmsnorm_bwd2(const void* dy, const void* x, const void* w, const float*
       kern<<<rows, n.threads, smem, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                               (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, ws, T, H);
     };
-    static bool attr_set = false;
-    if (!attr_set) {
+    // the limit is the device's, not the process's
+    static bool raised[16] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return B200_ERR_RUNTIME;
+    if (!raised[dev]) {
       constexpr int most = NORM_STAGES * 3 * NORM_MAX_H * 2;
       if (cudaFuncSetAttribute(rmsnorm_bwd_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most / 2) != cudaSuccess ||
           cudaFuncSetAttribute(rmsnorm_bwd_kernel<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
         return B200_ERR_LAUNCH;
-      attr_set = true;
+      raised[dev] = true;
     }
     if (n.vpt == 1) go(rmsnorm_bwd_kernel<1, 2>, RMSNORM_WS_ROWS);
     else go(rmsnorm_bwd_kernel<2, 1>, RMSNORM_WS_ROWS / 2);

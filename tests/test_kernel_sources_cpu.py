@@ -109,3 +109,13 @@ def test_gated_mlp_of_mismatched_shapes_goes_through_the_checked_calls(monkeypat
                 separate.clear()
         F.gated_mlp(make(512, 64), make(96, 64), make(64, 48))
     assert fused == [(512, 64)] and not separate
+
+
+def test_shared_memory_of_the_norms_is_raised_on_every_device():
+    """The limit of a kernel's dynamic shared memory belongs to a device: what remembers that it has been raised is kept per device,
+    or the first launch on a second one fails."""
+    src = (CSRC / "elementwise.cu").read_text()
+    calls = [m.start() for m in re.finditer(r"cudaFuncSetAttribute\(", src)]
+    assert calls and not re.search(r"static bool \w+ =", src)
+    for at in calls:
+        assert re.search(r"if \(!(\w+)\[dev\]\)", src[:at]) and "cudaGetDevice(&dev)" in src[:at]

@@ -2174,3 +2174,17 @@ def test_gated_mlp_backward_holds_no_more_than_its_separate_passes():
     fused = peak(lambda: F.gated_mlp(x, wg, wd))
     scratch = 4 * native.host().b200_gemm_gated_scratch(M, I, H, True, native.num_sms(0))
     assert scratch < 2 * M * I and fused <= separate + scratch      # one row of I values more a token would show
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+@pytest.mark.parametrize("H", [3584, 8192])
+def test_rms_norm_backward_on_a_second_gpu(H):
+    grads = []
+    torch.manual_seed(99)
+    host = [torch.randn(n, H).to(torch.bfloat16) for n in (5, 1, 5)]
+    for dev in (0, 1):
+        with torch.cuda.device(dev):
+            x, w, dy = (t.to(f"cuda:{dev}") for t in host)
+            x, w = x.requires_grad_(True), w[0].requires_grad_(True)
+            grads.append([g.cpu() for g in torch.autograd.grad(F.rms_norm(x, w)[0], [x, w], dy)])
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
