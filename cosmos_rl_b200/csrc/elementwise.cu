@@ -397,13 +397,14 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
 // sines and cosines are formed once, in shared memory, while those are on their way. `plain` heads behind the rotated ones are
 // copied (the values of a gradient that is not rotated in place). 32 heads of 128, in place: 8192 tokens 26.1 us, with the
 // angles formed again for every four heads 28.8 (20 are the bytes); 57 tokens, 6 heads 2.3 and 4.0. Persistent CTAs that
-// fetch a token ahead have the angles of one token after the other: 40.
+// fetch a token ahead have the angles of one token after the other: 40. In place q_out is q and k_out is k, so neither is
+// __restrict__: a thread reads its vectors before it writes them, and nobody else touches them.
 constexpr int ROPE_MAX_D = 512, ROPE_MAX_THREADS = 512;
 template <int ROWS>
 __global__ void __launch_bounds__(ROPE_MAX_THREADS)
-rope_vec_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ q_out,
-                __nv_bfloat16* __restrict__ k_out, const long long* __restrict__ pos, int T, int hq, int hkv, int plain, int d,
-                long long q_stride, long long k_stride, long long q_out_stride, long long k_out_stride, float log2_theta, float sign) {
+rope_vec_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k, __nv_bfloat16* q_out, __nv_bfloat16* k_out,
+                const long long* __restrict__ pos, int T, int hq, int hkv, int plain, int d, long long q_stride, long long k_stride,
+                long long q_out_stride, long long k_out_stride, float log2_theta, float sign) {
   __shared__ float2 sc[ROWS][ROPE_MAX_D / 2];   // sine, cosine
   const int half = d >> 1, vecs = half >> 3, items = (hq + hkv + plain) * vecs;
   const long long t0 = (long long)blockIdx.x * ROWS;

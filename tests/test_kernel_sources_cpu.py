@@ -119,3 +119,13 @@ def test_shared_memory_of_the_norms_is_raised_on_every_device():
     assert calls and not re.search(r"static bool \w+ =", src)
     for at in calls:
         assert re.search(r"if \(!(\w+)\[dev\]\)", src[:at]) and "cudaGetDevice(&dev)" in src[:at]
+
+
+def test_kernels_that_work_in_place_promise_no_separate_memory():
+    """Where a launcher may pass one buffer as source and as destination, a kernel's parameters for the two are not __restrict__:
+    the compiler could read what has been overwritten."""
+    src = (CSRC / "elementwise.cu").read_text()
+    assert "launch_rope_vec(q, k, q, k," in src
+    params = re.search(r"^rope_vec_kernel\((.*?)\) \{", src, flags=re.M | re.S).group(1)
+    for name in ("q", "k", "q_out", "k_out"):
+        assert re.search(r"__nv_bfloat16\* %s\b" % name, params), name
