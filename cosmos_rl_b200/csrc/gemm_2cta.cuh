@@ -653,8 +653,10 @@ __device__ __forceinline__ void gemm2_mainloop(const CUtensorMap* tmA, const CUt
           }
         }
       } else
+      // Rows past the end hold what shared memory held, and quotients of that take the slow way: a warp that has only such rows
+      // forms none (304 x 12704 x 1000 105 us with them, 28; 311 x 72 x 896 37 and 11).
 #pragma unroll 1
-      for (int c = 0; c < OUT_BN; c += slab_cols) {
+      for (int c = EPI == G2_EPI_SWIGLU && row0 >= M ? OUT_BN : 0; c < OUT_BN; c += slab_cols) {
         uint8_t* slab = slab0 + (slab_idx & 1) * 4096;
         // the store issued two slabs ago has finished reading this buffer
         if (elect_one()) tma_store_wait_read<1>();
