@@ -617,10 +617,13 @@ int b200_skinny_linear(const void* x, const void* W, const void* bias, int bias_
                        long long ws_floats, int M, int N, int K, long long ldx, long long ldw, long long ldo,
                        uint32_t* status, int num_sms, cudaStream_t stream) {
   const int splits = b200_gemm_skinny_splits(M, N, K, 0, num_sms);
-  // Short contractions stay whole: the second kernel costs more than shares save up to 16 blocks. us, split and whole: 57 rows,
-  // 1024 x 512 5.9 and 4.6, 512 x 1024 6.2 and 5.7, 8192 x 1024 8.9 and 6.9; one row 6.0 and 5.7 (1024 x 1024); of 32 blocks 57 x
-  // 2048 x 2048 8.6 and 8.8, one row 7.7 and 8.7. What only the reduction can write (rows off the 16-byte grid) is split.
-  const bool whole = K <= 16 * b200::GEMM_BK && !(N & 7) && !(ldo & 7) && !(reinterpret_cast<uintptr_t>(out) & 15);
+  // Short contractions stay whole: the second kernel costs more than shares save up to 16 blocks of rows on the 128-byte grid. us,
+  // split and whole: 57 rows, 1024 x 512 5.9 and 4.6, 512 x 1024 6.2 and 5.7, 8192 x 1024 8.9 and 6.9; one row 6.0 and 5.7 (1024 x
+  // 1024); of 32 blocks 57 x 2048 x 2048 8.6 and 8.8, one row 7.7 and 8.7. Rows off that grid take half as long again to fetch, and
+  // there the line is at 11 blocks: 118 rows, 1024 x 648 7.8 and 7.6, x 712 7.3 and 7.9, x 1000 7.7 and 9.5. What only the reduction
+  // can write (results off the 16-byte grid) is split.
+  const int most = (K | ldx | ldw) & 63 ? 11 : 16;
+  const bool whole = K <= most * b200::GEMM_BK && !(N & 7) && !(ldo & 7) && !(reinterpret_cast<uintptr_t>(out) & 15);
   if (splits == 1 || whole)
     return b200_gemm_skinny(x, W, out, nullptr, M, N, K, ldx, ldw, ldo, bias, bias_bf16, 0, 0, 1, status, num_sms, stream);
   if (ws == nullptr) return B200_NEED_WORKSPACE;

@@ -129,3 +129,27 @@ def test_kernels_that_work_in_place_promise_no_separate_memory():
     params = re.search(r"^rope_vec_kernel\((.*?)\) \{", src, flags=re.M | re.S).group(1)
     for name in ("q", "k", "q_out", "k_out"):
         assert re.search(r"__nv_bfloat16\* %s\b" % name, params), name
+
+
+def test_short_contractions_stay_whole_where_their_rows_are_on_the_128_byte_grid():
+    """Whether a projection of few rows is cut is known before anything is launched: a call that is, and has no workspace, says so."""
+    import pytest
+
+    from cosmos_rl_b200.ops import native
+    if not native.available():
+        pytest.skip("the kernel library is not built")
+    L = native.lib()
+
+    def asks(M, N, K, ldx, ldw):
+        return L.b200_skinny_linear(None, None, None, 0, None, None, 0, M, N, K, ldx, ldw, N, None, 148, None) == native.NEED_WORKSPACE
+
+    for M in (1, 57, 256):
+        for N in (72, 1024):
+            assert L.b200_gemm_skinny_splits(M, N, 712, 0, 148) > 1
+            for K in (704, 1000, 1032, 1088):
+                assert asks(M, N, K, K, K) == (K > 704)
+            for K, ldx, ldw in ((768, 776, 768), (1024, 1024, 1032), (712, 768, 768)):
+                assert asks(M, N, K, ldx, ldw)
+            for K in (704, 768, 1024):
+                assert not asks(M, N, K, K, K) and not asks(M, N, K, K + 64, K)
+            assert not asks(M, N, 696, 776, 696)
