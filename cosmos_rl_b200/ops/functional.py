@@ -621,7 +621,9 @@ class _FusedLogprob(torch.autograd.Function):
         dh = torch.zeros(T, H, dtype=torch.float32, device=hidden.device) if need_dh else None
         dw = torch.empty_like(weight) if need_dw else None
         chunk = _dlogits_chunk(T, V)
-        buf = torch.empty(T, chunk, dtype=torch.bfloat16, device=hidden.device)
+        # rows on the 16-byte grid, whatever the vocabulary is: all products move them with TMA
+        buf = torch.empty(T, (chunk + 7) // 8 * 8, dtype=torch.bfloat16, device=hidden.device)
+        direct = _dims_ok(hidden, weight)
         for v0 in range(0, V, chunk):
             vc = min(chunk, V - v0)
             dl = buf[:, :vc]
@@ -631,12 +633,15 @@ class _FusedLogprob(torch.autograd.Function):
             # both products on this library's GEMM: dh accumulates in fp32 through the epilogue's reduce-add,
             # dW of this vocabulary slice contracts dlogits^T and hidden over the token axis as stored
             if need_dh:
-                if _dims_ok(dl, weight):
+                if direct:
                     gemm(dl, weight[v0:v0 + vc], b_mn=True, out=dh, accumulate=True)
                 else:
                     dh.add_(torch.mm(dl, weight[v0:v0 + vc]))
             if need_dw:
-                mm_tn(dl, hidden, out=dw[v0:v0 + vc])
+                if direct:
+                    gemm(dl, hidden, a_mn=True, b_mn=True, out=dw[v0:v0 + vc])
+                else:
+                    mm_tn(dl, hidden, out=dw[v0:v0 + vc])
         return (dh.to(hidden.dtype) if need_dh else None), dw, None, None, None
 
 

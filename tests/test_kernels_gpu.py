@@ -2188,3 +2188,29 @@ def test_rms_norm_backward_on_a_second_gpu(H):
             x, w = x.requires_grad_(True), w[0].requires_grad_(True)
             grads.append([g.cpu() for g in torch.autograd.grad(F.rms_norm(x, w)[0], [x, w], dy)])
     assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+@pytest.mark.parametrize("T,V,H", [(1, 20001, 64), (129, 20001, 136), (300, 65539, 64), (777, 16387, 72), (1100, 1031, 64)])
+def test_fused_logprob_gradients_of_a_ragged_vocabulary(monkeypatch, T, V, H):
+    """A vocabulary that is no multiple of 8: the logit gradients' rows start on 16 bytes all the same, so both products take this
+    library's GEMM, in one chunk of few rows and in several of many."""
+    calls, real = [], F.gemm
+
+    def gemm(a, b, **kw):
+        calls.append(a.stride(0))
+        return real(a, b, **kw)
+
+    monkeypatch.setattr(F, "gemm", gemm)
+    torch.manual_seed(100)
+    h, w = _bf16(T, H).requires_grad_(True), _bf16(V, H, scale=0.3).requires_grad_(True)
+    labels, g, ge = torch.randint(0, V, (T,), device=DEV), torch.randn(T, device=DEV), torch.randn(T, device=DEV) * 0.1
+    labels[0] = V - 1
+    lp, ent = F.fused_logprob(h, w, labels, 1.0)
+    got = torch.autograd.grad([lp, ent], [h, w], [g, ge])
+    native.read_status(h.device)
+    assert len(calls) == 2 * -(-V // F._dlogits_chunk(T, V)) and all(s % 8 == 0 for s in calls)
+    hd, wd = h.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    logp = torch.log_softmax(hd @ wd.t(), -1)
+    want = torch.autograd.grad([logp.gather(-1, labels[:, None])[:, 0], -(logp.exp() * logp).sum(-1)], [hd, wd], [g.double(), ge.double()])
+    for a, b in zip(got, want):     # the logits' gradient is rounded to bf16 (2^-9), and the result once more
+        assert (a.double() - b).norm() <= 2 ** -7 * b.norm()
