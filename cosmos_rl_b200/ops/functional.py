@@ -570,15 +570,17 @@ def _pick_nsplit(T: int, V: int, sms: int) -> int:
 
 
 _DLOGITS_CHUNK = int(os.environ.get("B200RL_DLOGITS_CHUNK", "16384"))
+_DLOGITS_MOST = 1 if "B200RL_DLOGITS_CHUNK" in os.environ else 4      # times as many for few rows; a number that was asked for stays
 
 
 def _dlogits_chunk(T: int, V: int) -> int:
-    """Vocabulary columns whose logit gradients are held at a time: _DLOGITS_CHUNK, and up to four times as many where few rows
-    make up for it (rows x columns as for 2048), since a chunk of few rows is no work for the whole machine (64 x 152064 x 3584,
-    backward: 972 us in ten chunks, 675 in three; 700 x 128256 x 4096: 1860 in eight, 1770 in four). Longer chunks are faster yet
-    (627 in one), but the hidden states' gradient would be summed over them in one go: its error, 2.2e-3 from bf16 alone, is the
-    same within 5e-4 of it up to four times, and grows by 2e-3 of it beyond."""
-    return min(_DLOGITS_CHUNK * max(1, min(4, 2048 // T)), V)
+    """Vocabulary columns whose logit gradients are held at a time: as many as B200RL_DLOGITS_CHUNK says, or _DLOGITS_CHUNK, and up
+    to four times as many where few rows make up for it (rows x columns as for 2048), since a chunk of few rows is no work for the
+    whole machine (64 x 152064 x 3584, backward: 972 us in ten chunks, 675 in three; 700 x 128256 x 4096: 1860 in eight, 1770 in
+    four). Longer chunks are faster yet (627 in one), but the hidden states' gradient is summed over them in one go: its error,
+    2.2e-3 from bf16 alone, does not change up to four times (between 0.993 and 1.010 of it, 1.0000 over 42 cases of 1 to 1024
+    rows), and grows by 2e-3 of it beyond."""
+    return min(_DLOGITS_CHUNK * max(1, min(_DLOGITS_MOST, 2048 // T)), V)
 
 
 class _FusedLogprob(torch.autograd.Function):

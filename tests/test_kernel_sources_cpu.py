@@ -153,3 +153,16 @@ def test_short_contractions_stay_whole_where_their_rows_are_on_the_128_byte_grid
             for K in (704, 768, 1024):
                 assert not asks(M, N, K, K, K) and not asks(M, N, K, K + 64, K)
             assert not asks(M, N, 696, 776, 696)
+
+
+def test_the_output_heads_chunk_is_what_was_asked_for():
+    """B200RL_DLOGITS_CHUNK bounds the memory of the head's backward: for any number of rows it is the number of columns held."""
+    import os
+    import subprocess
+    import sys
+    show = "from cosmos_rl_b200.ops import functional as F; print([F._dlogits_chunk(T, 152064) for T in (1, 700, 2048, 8192)])"
+    env = {k: v for k, v in os.environ.items() if k != "B200RL_DLOGITS_CHUNK"}
+    for extra, want in (({}, [65536, 32768, 16384, 16384]), ({"B200RL_DLOGITS_CHUNK": "4096"}, [4096] * 4),
+                        ({"B200RL_DLOGITS_CHUNK": "16384"}, [16384] * 4), ({"B200RL_DLOGITS_CHUNK": "200000"}, [152064] * 4)):
+        out = subprocess.run([sys.executable, "-c", show], env={**env, **extra}, cwd=CSRC.parent.parent, capture_output=True, text=True)
+        assert out.returncode == 0 and out.stdout.strip() == str(want), (extra, out.stdout, out.stderr)
