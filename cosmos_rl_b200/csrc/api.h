@@ -85,11 +85,12 @@ int b200_last_tmap_error(void);
 
 // Fused lm_head GEMM + per-token log-prob statistics, never materialising [T, V] logits.
 //   hidden [T, H] bf16, weight [V, H] bf16, labels [T] int64 (label < 0: row ignored)
-//   partial [T, nsplit, 4] fp32 scratch: (max, sumexp, label_logit, sum p_unnorm*logit)
+//   partial [T, nsplit, 4] fp32 scratch: (max, sumexp, label_logit, sum p_unnorm*logit), nsplit <= tiles of 256 vocabulary columns
+//   pairs: CTA pairs on tiles of 256 rows, else CTAs on tiles of 128
 // followed by b200_logprob_combine -> logprob [T], lse [T], entropy [T] (fp32).
 int b200_lmhead_logprob_partial(const void* hidden, const void* weight, const long long* labels, float* partial,
                                 int T, int V, int H, long long ldh, long long ldw, float inv_temperature,
-                                int nsplit, uint32_t* status, int num_sms, cudaStream_t stream);
+                                int nsplit, int pairs, uint32_t* status, int num_sms, cudaStream_t stream);
 int b200_logprob_combine(const float* partial, const long long* labels, float* logprob, float* lse, float* entropy,
                          int T, int nsplit, cudaStream_t stream);
 // Backward helper: dlogits[T, Vc] (bf16) = (softmax(logits/temp) * (g_lp_total) - onehot * g_lp) * inv_temp for a vocab

@@ -280,31 +280,44 @@ struct G2GroupedWork {
   }
 };
 
-// G2_EPI_LOGPROB: a unit is a block of 256 rows and one of nsplit equal ranges of column tiles (batch), walked tile by tile. The
-// row blocks of a range run side by side, so that the weights of a tile come from HBM once.
-struct G2LogprobWork {
-  int num_m, num_n, num_kb, nsplit;
-  __device__ __forceinline__ void init(const Gemm2Params& ep, bool, int num_m_, int num_n_, int num_kb_) {
+// G2_EPI_LOGPROB (and the form of lmhead_logprob.cu with one CTA a tile): a unit is a block of rows and one of nsplit ranges of
+// column tiles, of which the first take one tile more where they cannot all be equal. The units of a CTA or pair, `first` and every
+// `step` further, are walked tile by tile; the row blocks of a range run side by side, so that a tile's weights come from HBM once.
+struct LogprobTiles {
+  int num_m, units, len, longer;
+  __device__ __forceinline__ void init(int num_m_, int num_n, int nsplit) {
     num_m = num_m_;
-    num_n = num_n_;
-    num_kb = num_kb_;
-    nsplit = ep.lg.nsplit;
+    units = num_m_ * nsplit;
+    len = num_n / nsplit;
+    longer = num_n - len * nsplit;
   }
-  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
-    for (int i = blockIdx.x >> 1; i < num_m * nsplit; i += gridDim.x >> 1) {
-      const int s = i / num_m, n0 = (int)((long long)s * num_n / nsplit), n1 = (int)((long long)(s + 1) * num_n / nsplit);
-      if (it < n1 - n0) {
-        u.m_blk = i - s * num_m;
-        u.n_blk = n0 + it;
-        u.batch = s;
-        u.kb0 = 0;
-        u.kb1 = num_kb;
-        u.cut = false;
+  __device__ __forceinline__ bool get(int it, int first, int step, int& m_blk, int& n_blk, int& range) const {
+    for (int i = first; i < units; i += step) {
+      range = i / num_m;
+      const int n = len + (range < longer);
+      if (it < n) {
+        m_blk = i - range * num_m;
+        n_blk = range * len + min(range, longer) + it;
         return true;
       }
-      it -= n1 - n0;
+      it -= n;
     }
     return false;
+  }
+};
+struct G2LogprobWork {
+  LogprobTiles tiles;
+  int num_kb;
+  __device__ __forceinline__ void init(const Gemm2Params& ep, bool, int num_m, int num_n, int num_kb_) {
+    tiles.init(num_m, num_n, ep.lg.nsplit);
+    num_kb = num_kb_;
+  }
+  __device__ __forceinline__ bool get(int it, G2Unit& u) const {
+    if (!tiles.get(it, blockIdx.x >> 1, gridDim.x >> 1, u.m_blk, u.n_blk, u.batch)) return false;
+    u.kb0 = 0;
+    u.kb1 = num_kb;
+    u.cut = false;
+    return true;
   }
 };
 

@@ -3,7 +3,7 @@
 // reference (cosmos_rl/utils/util.py:314-366, 899-994) and feeds the GRPO loss
 // (cosmos_rl/policy/trainer/llm_trainer/grpo_trainer.py:113-353).
 //
-// Forward: work unit = (block of tokens, vocabulary range). The CTA pair (up to 128 tokens: CTA) that owns a unit walks its
+// Forward: work unit = (block of tokens, vocabulary range). The CTA or, on blocks of 256, the CTA pair that owns a unit walks its
 // vocabulary tiles; each epilogue thread owns one token row and keeps an online-softmax state
 // (running max, sum of exp, label logit, sum exp*logit) in registers across tiles, written once per unit
 // to a [T, nsplit, 4] fp32 scratch that b200_logprob_combine reduces.
@@ -20,51 +20,42 @@ constexpr int LP_STAGES = 4;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 
-// Up to 128 rows: one CTA a tile, the vocabulary in as many ranges as there are CTAs (the pair form for more is an epilogue of
-// gemm_2cta.cuh).
+// One CTA a tile of 128 rows (the pair form is an epilogue of gemm_2cta.cuh).
 struct LogprobEpilogue {
   using Params = LogprobParams;
   LogprobRow st;
-  int cur_split = -1;
+  int cur_m = 0, cur_range = -1;
+  __device__ __forceinline__ void store(const Params& p, int row) const {
+    if (cur_range >= 0) st.store(p, (long long)cur_m * GEMM_BM + row, cur_range);
+  }
   __device__ __forceinline__ void tile_begin(const Params& p, const TileInfo& t, int row) {
-    if (t.batch == cur_split) return;
-    if (cur_split >= 0) st.store(p, row, cur_split);
-    cur_split = t.batch;
-    st.begin(p, row);
+    if (t.batch == cur_range && t.m_blk == cur_m) return;
+    store(p, row);
+    cur_m = t.m_blk;
+    cur_range = t.batch;
+    st.begin(p, (long long)cur_m * GEMM_BM + row);
   }
   __device__ __forceinline__ void chunk(const Params& p, const TileInfo& t, int, int col0, const float (&v)[32]) {
     st.chunk(p, t.n_blk * LP_BN + col0, v);
   }
   __device__ __forceinline__ void tile_end(const Params&, const TileInfo&, int) {}
-  __device__ __forceinline__ void finish(const Params& p) {
-    if (cur_split >= 0) st.store(p, ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31), cur_split);
-  }
+  __device__ __forceinline__ void finish(const Params& p) { store(p, ((threadIdx.x >> 5) & 3) * 32 + (threadIdx.x & 31)); }
 };
 
-// Range s (TileInfo::batch) of the vocabulary's tiles belongs to CTA s, s + grid, ...
 struct LogprobSched {
-  int num_n, nsplit, num_kb;
-  __device__ __forceinline__ void init(int, int N, int K, int BN, const LogprobParams& p) {
-    num_n = (N + BN - 1) / BN;
-    nsplit = p.nsplit;
+  LogprobTiles tiles;
+  int num_kb;
+  __device__ __forceinline__ void init(int M, int N, int K, int BN, const LogprobParams& p) {
+    tiles.init((M + GEMM_BM - 1) / GEMM_BM, (N + BN - 1) / BN, p.nsplit);
     num_kb = (K + GEMM_BK - 1) / GEMM_BK;
   }
   __device__ __forceinline__ bool get(int it, TileInfo& t) const {
-    for (int s = blockIdx.x; s < nsplit; s += gridDim.x) {
-      const int n0 = (int)((long long)s * num_n / nsplit), n1 = (int)((long long)(s + 1) * num_n / nsplit);
-      if (it < n1 - n0) {
-        t.m_blk = 0;
-        t.n_blk = n0 + it;
-        t.a_mn0 = 0;
-        t.b_mn0 = t.n_blk * LP_BN;
-        t.k0 = 0;
-        t.num_kb = num_kb;
-        t.batch = s;
-        return true;
-      }
-      it -= n1 - n0;
-    }
-    return false;
+    if (!tiles.get(it, blockIdx.x, gridDim.x, t.m_blk, t.n_blk, t.batch)) return false;
+    t.a_mn0 = t.m_blk * GEMM_BM;
+    t.b_mn0 = t.n_blk * LP_BN;
+    t.k0 = 0;
+    t.num_kb = num_kb;
+    return true;
   }
 };
 
@@ -162,17 +153,16 @@ extern "C" {
 
 int b200_lmhead_logprob_partial(const void* hidden, const void* weight, const long long* labels, float* partial,
                                 int T, int V, int H, long long ldh, long long ldw, float inv_temperature,
-                                int nsplit, uint32_t* status, int num_sms, cudaStream_t stream) {
+                                int nsplit, int pairs, uint32_t* status, int num_sms, cudaStream_t stream) {
   using namespace b200;
   if (T <= 0 || V <= 0 || H <= 0 || (H & 7) || nsplit <= 0) return B200_ERR_ARG;
-  const int num_n = (V + LP_BN - 1) / LP_BN;
-  if (nsplit > num_n) return B200_ERR_ARG;
+  const int num_n = (V + LP_BN - 1) / LP_BN, rows = pairs ? G2_BM : GEMM_BM;
+  const long long units = (long long)((T + rows - 1) / rows) * nsplit;
+  if (nsplit > num_n || units > INT_MAX / 2) return B200_ERR_ARG;
   const LogprobParams lg{labels, partial, T, V, nsplit, inv_temperature * LOG2E};
   CUtensorMap tmA, tmB;
   if (make_tmap_2d(&tmA, hidden, T, H, ldh, GEMM_BM, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
-  // The logits are formed at the rate of the dense GEMM: CTA pairs once there are rows for their 256-row tiles. 2048 x 152064 x
-  // 3584: 1458 us, with one CTA a tile, whose operand traffic bounds it, 1666; 200 rows 221 and 268.
-  if (T > GEMM_BM) {
+  if (pairs) {
     using SM = Gemm2Smem<LP_BN, 6>;
     if (make_tmap_2d(&tmB, weight, V, H, ldw, LP_BN / 2, GEMM_BK, 2)) return B200_ERR_TENSORMAP;
     auto kern = gemm2_bf16_kernel<LP_BN, 6, false, false, G2_EPI_LOGPROB>;
@@ -182,7 +172,6 @@ int b200_lmhead_logprob_partial(const void* hidden, const void* weight, const lo
     Gemm2Params ep{};
     ep.a_bytes = SM::A_BYTES;
     ep.lg = lg;
-    const long long units = (long long)((T + G2_BM - 1) / G2_BM) * nsplit;
     kern<<<2 * (int)(units < np ? units : np), G2_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmB, tmB, T, V, H, ep, status);
     return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
   }
@@ -195,7 +184,7 @@ int b200_lmhead_logprob_partial(const void* hidden, const void* weight, const lo
       return B200_ERR_LAUNCH;
     attr_set = true;
   }
-  lmhead_logprob_kernel<<<nsplit < num_sms ? nsplit : num_sms, GEMM_THREADS, SM::TOTAL, stream>>>(tmA, tmB, T, V, H, lg, status);
+  lmhead_logprob_kernel<<<(int)(units < num_sms ? units : num_sms), GEMM_THREADS, SM::TOTAL, stream>>>(tmA, tmB, T, V, H, lg, status);
   return cudaGetLastError() == cudaSuccess ? 0 : B200_ERR_LAUNCH;
 }
 

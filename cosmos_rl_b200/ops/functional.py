@@ -551,12 +551,8 @@ def skinny_qkv_rope_append(x2: torch.Tensor, qkv_weight: torch.Tensor, bias: Opt
 # --------------------------------------------------------------------------------------------------
 # fused lm_head + log-prob + entropy
 # --------------------------------------------------------------------------------------------------
-@functools.lru_cache(maxsize=1024)
-def _pick_nsplit(T: int, V: int, sms: int) -> int:
-    """Ranges of the vocabulary: CTA pairs (up to 128 rows: CTAs) take units of a row block and a range one after the other."""
-    rows, slots = (256, max(1, sms // 2)) if T > 128 else (128, sms)
-    num_m = (T + rows - 1) // rows
-    num_n = (V + 255) // 256
+def _pick_nsplit(num_m: int, num_n: int, slots: int) -> int:
+    """Ranges of ``num_n`` column tiles, of which ``slots`` CTAs or pairs take units of a row block and a range in turn."""
     best, best_score = 1, -1.0
     for ns in range(1, min(num_n, max(64, slots)) + 1):
         units = num_m * ns
@@ -567,6 +563,26 @@ def _pick_nsplit(T: int, V: int, sms: int) -> int:
         if score > best_score:
             best, best_score = ns, score
     return best
+
+
+@functools.lru_cache(maxsize=1024)
+def _logprob_form(T: int, V: int, H: int, sms: int) -> Tuple[int, bool]:
+    """Ranges of the vocabulary, and whether CTA pairs take them.
+
+    A pair's tile has 256 rows, a single CTA's 128, so pairs have more of them to do where the last 256 are not full; in return a
+    pair's contraction block takes 0.4 us and a single CTA's a quarter more, unless the epilogue, 21 blocks' worth of time for
+    either, covers them. us, single CTAs and pairs: 152064 x 3584, 2048 rows 1620 to 1780 and 1400 to 1450, 640
+    rows 550 and 562, 384 rows 354 and 402, 200 rows 261 and 232; 32000 x 512, 640 rows 49 and 56, 384 rows 33 and 41, 2048 rows
+    121 and 119; 1000 rows of 128256 x 1024 264 and 253."""
+    num_n, kb = (V + 255) // 256, (H + 63) // 64
+    forms = []
+    for pairs, rows, slots in ((True, 256, max(1, sms // 2)), (False, 128, sms)):
+        num_m = (T + rows - 1) // rows
+        ns = _pick_nsplit(num_m, num_n, slots)
+        rounds = math.ceil(num_m * ns / slots) * math.ceil(num_n / ns)
+        if T > 128 or not pairs:
+            forms.append((rounds * max(21, kb) + 2 if pairs else rounds * max(21.2, 1.25 * kb), ns, pairs))
+    return min(forms, key=lambda f: f[0])[1:]
 
 
 _DLOGITS_CHUNK = int(os.environ.get("B200RL_DLOGITS_CHUNK", "16384"))
@@ -591,7 +607,7 @@ class _FusedLogprob(torch.autograd.Function):
         hidden = _c(hidden)
         dev = hidden.device.index if hidden.device.index is not None else torch.cuda.current_device()
         sms = native.num_sms(dev)
-        nsplit = _pick_nsplit(T, V, sms)
+        nsplit, pairs = _logprob_form(T, V, H, sms)
         partial = torch.empty(T, nsplit, 4, dtype=torch.float32, device=hidden.device)
         lp = torch.empty(T, dtype=torch.float32, device=hidden.device)
         lse = torch.empty_like(lp)
@@ -599,7 +615,7 @@ class _FusedLogprob(torch.autograd.Function):
         st = native.status_word(hidden.device)
         L = native.host()
         native.check(L.b200_lmhead_logprob_partial(hidden, weight, labels, partial, T, V, H, hidden.stride(0), weight.stride(0),
-                                                   1.0 / temperature, nsplit, st, sms, native.stream()),
+                                                   1.0 / temperature, nsplit, pairs, st, sms, native.stream()),
                      "lmhead_logprob_partial")
         native.check(L.b200_logprob_combine(partial, labels, lp, lse, ent, T, nsplit, native.stream()), "logprob_combine")
         ctx.save_for_backward(hidden, weight, labels, lse, ent)

@@ -69,7 +69,7 @@ _SIGS = {
     "b200_splitk_reduce_qkv_rope_append": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p,
                                            c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "b200_lmhead_logprob_partial": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong,
-                                    c_longlong, c_float, c_int, c_void_p, c_int, c_void_p],
+                                    c_longlong, c_float, c_int, c_int, c_void_p, c_int, c_void_p],
     "b200_logprob_combine": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
     "b200_lmhead_dlogits": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                             c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_longlong, c_float, c_void_p, c_int,

@@ -166,3 +166,14 @@ def test_the_output_heads_chunk_is_what_was_asked_for():
                         ({"B200RL_DLOGITS_CHUNK": "16384"}, [16384] * 4), ({"B200RL_DLOGITS_CHUNK": "200000"}, [152064] * 4)):
         out = subprocess.run([sys.executable, "-c", show], env={**env, **extra}, cwd=CSRC.parent.parent, capture_output=True, text=True)
         assert out.returncode == 0 and out.stdout.strip() == str(want), (extra, out.stdout, out.stderr)
+
+
+def test_output_head_forms():
+    """CTA pairs of the output head have tiles of 256 rows: not for rows that fill half of their last one, unless the contraction is
+    long enough to make up for it, and never for 128 rows or fewer."""
+    from cosmos_rl_b200.ops import functional as F
+    for T, V, H, pairs in ((1, 152064, 3584, False), (128, 152064, 3584, False), (129, 152064, 3584, True), (384, 152064, 3584, False),
+                           (384, 32000, 512, False), (640, 32000, 512, False), (1024, 128256, 512, True), (800, 152064, 4096, True),
+                           (2048, 152064, 3584, True), (300, 1500, 512, False), (5000, 152064, 3584, True)):
+        ns, got = F._logprob_form(T, V, H, 148)
+        assert got is pairs and 1 <= ns <= -(-V // 256), (T, V, H)

@@ -2214,3 +2214,25 @@ def test_fused_logprob_gradients_of_a_ragged_vocabulary(monkeypatch, T, V, H):
     want = torch.autograd.grad([logp.gather(-1, labels[:, None])[:, 0], -(logp.exp() * logp).sum(-1)], [hd, wd], [g.double(), ge.double()])
     for a, b in zip(got, want):     # the logits' gradient is rounded to bf16 (2^-9), and the result once more
         assert (a.double() - b).norm() <= 2 ** -7 * b.norm()
+
+
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("T,V,H,ranges", [(129, 40009, 64, 7), (300, 20001, 72, 79), (1153, 1025, 64, 5), (513, 3000, 136, 1), (2100, 9000, 64, 20)])
+def test_fused_logprob_row_blocks_and_ranges(monkeypatch, pairs, T, V, H, ranges):
+    """Both forms on several row blocks: ranges of unequal length, one range, a range a tile, more units than CTAs, and a last row
+    block of one row."""
+    monkeypatch.setattr(F, "_logprob_form", lambda *a: (ranges, pairs))
+    torch.manual_seed(101)
+    h, w = _bf16(T, H), _bf16(V, H, scale=0.3)
+    labels = torch.randint(0, V, (T,), device=DEV)
+    labels[-1], labels[0] = V - 1, -100
+    lp, ent = F.fused_logprob(h, w, labels, 1.0)
+    native.read_status(h.device)
+    logits = h.double() @ w.double().t()
+    lse = logits.logsumexp(-1)
+    want = torch.where(labels >= 0, logits.gather(-1, labels.clamp_min(0)[:, None])[:, 0] - lse, 0.)
+    want_ent = lse - ((logits - lse[:, None]).exp() * logits).sum(-1)
+    # a logit is an fp32 sum of H products; the sums over the vocabulary are relative to their largest term
+    logit = 2.0 ** -20 * (h.double().norm(dim=1) * w.double().norm(dim=1).max())
+    assert ((lp.double() - want).abs() <= 2 * logit + 1e-5 * (1 + lse.abs())).all()
+    assert ((ent.double() - want_ent).abs() <= (2 + logits.abs().amax(-1)) * (2 * logit + 1e-5)).all()
