@@ -644,7 +644,9 @@ static int launch_rope_vec(const void* q, const void* k, void* q_out, void* k_ou
                            int plain, int d, long long q_stride, long long k_stride, long long q_out_stride, long long k_out_stride,
                            float theta, int backward, cudaStream_t stream) {
   // a token that is more than 512 vectors is taken in equal parts
-  const int items = (hq + hkv + plain) * (d / 16), parts = (items + ROPE_MAX_THREADS - 1) / ROPE_MAX_THREADS;
+  const int items = (hq + hkv + plain) * (d / 16);
+  if (items <= 0) return B200_ERR_ARG;
+  const int parts = (items + ROPE_MAX_THREADS - 1) / ROPE_MAX_THREADS;
   const int threads = ((items + parts - 1) / parts + 31) / 32 * 32, rows = T >= 148 * 4 ? ROPE_ROWS : 1;
   auto kern = rows == 1 ? rope_vec_kernel<1> : rope_vec_kernel<ROPE_ROWS>;
   kern<<<(unsigned)((T + rows - 1) / rows), threads, 0, stream>>>(

@@ -177,3 +177,24 @@ def test_output_head_forms():
                            (2048, 152064, 3584, True), (300, 1500, 512, False), (5000, 152064, 3584, True)):
         ns, got = F._logprob_form(T, V, H, 148)
         assert got is pairs and 1 <= ns <= -(-V // 256), (T, V, H)
+
+
+def _in_a_child(code):
+    """What ``code`` prints in a process of its own, which a fault on the host would end."""
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", code], cwd=CSRC.parent.parent, capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
+    return r.stdout.strip()
+
+
+def test_rotary_embedding_of_no_heads_is_refused():
+    """Without heads, or of no columns, there is nothing to divide among threads: the launcher says so."""
+    import pytest
+
+    from cosmos_rl_b200.ops import native
+    if not native.available():
+        pytest.skip("the kernel library is not built")
+    for hq, d in ((0, 16), (0, 128), (2, 0)):
+        assert int(_in_a_child("from cosmos_rl_b200.ops import native\n"
+                               f"print(native.lib().b200_rope_inplace(4096, None, 4096, 4, {hq}, 0, {d}, 64, 0, 1e4, 0, None))")) < 0
