@@ -362,6 +362,10 @@ PyObject* flash_ok(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor& q = *t[0];
   bool ok = q.is_cuda() && bf16(q) && q.size(-1) == 128;
   for (int i = 0; i < 3 && ok; ++i) ok = t[i]->stride(-1) == 1 && t[i]->stride(1) == 128 && t[i]->stride(0) % 8 == 0;
+  if (ok && t[1]->size(1) == 0) {
+    PyErr_SetString(PyExc_ZeroDivisionError, "attention without kv heads");
+    throw python_error();
+  }
   return PyBool_FromLong(ok && q.size(1) % t[1]->size(1) == 0);
   END_HANDLE_TH_ERRORS
 }

@@ -198,3 +198,24 @@ def test_rotary_embedding_of_no_heads_is_refused():
     for hq, d in ((0, 16), (0, 128), (2, 0)):
         assert int(_in_a_child("from cosmos_rl_b200.ops import native\n"
                                f"print(native.lib().b200_rope_inplace(4096, None, 4096, 4, {hq}, 0, {d}, 64, 0, 1e4, 0, None))")) < 0
+
+
+def test_attention_without_kv_heads_raises():
+    """Keys of no heads, on tensors that only say that they are on a GPU: an exception, as Python's own division has it."""
+    import pytest
+
+    from cosmos_rl_b200.ops import build, native
+    if not (native.available() and build.host_path().exists()):
+        pytest.skip("the kernel library is not built")
+    assert _in_a_child("""
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from cosmos_rl_b200.ops import attention
+with FakeTensorMode():
+    make = lambda heads: torch.empty(4, heads, 128, dtype=torch.bfloat16, device="cuda")
+    print(attention.native_flash_supported(make(8), make(4), make(4)), attention.native_flash_supported(make(8), make(3), make(3)))
+    try:
+        attention.native_flash_supported(make(8), make(0), make(0))
+    except ZeroDivisionError:
+        print("raised")
+""").split() == ["True", "False", "raised"]
