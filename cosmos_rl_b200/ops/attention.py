@@ -24,7 +24,7 @@ def flash_fwd(q, k, v, cu_q, cu_k, max_q: int, scale: float, causal: bool = True
               ) -> Tuple[torch.Tensor, torch.Tensor]:
     """q [Tq, hq, 128], k / v [Tk, hkv, 128] (token-strided views are fine). Returns (out [Tq, hq, 128] bf16,
     lse [hq, Tq] fp32)."""
-    return native.tensors(native.host().flash_fwd(q, k, v, cu_q, cu_k, max_q, causal, scale, native.status_word(q.device),
+    return native.tensors(native.host().flash_fwd(q, k, v, cu_q, cu_k, int(max_q), causal, scale, native.status_word(q.device),
                                                   native.num_sms(q.device.index), native.stream()), "flash_fwd")
 
 

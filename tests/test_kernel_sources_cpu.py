@@ -219,3 +219,21 @@ with FakeTensorMode():
     except ZeroDivisionError:
         print("raised")
 """).split() == ["True", "False", "raised"]
+
+
+def test_flash_fwd_takes_its_longest_sequence_as_a_number_of_any_kind(monkeypatch):
+    import types
+
+    import numpy as np
+    import torch
+
+    from cosmos_rl_b200.ops import attention, native
+    seen = []
+    monkeypatch.setattr(native, "host", lambda: types.SimpleNamespace(flash_fwd=lambda *a: seen.append(a[5]) or (None, None)))
+    for name in ("status_word", "num_sms"):
+        monkeypatch.setattr(native, name, lambda d: 0)
+    monkeypatch.setattr(native, "stream", lambda: 0)
+    t = torch.zeros(1)
+    for longest in (7, 7.0, np.float32(7.0), np.int64(7), torch.tensor(7), torch.tensor(7.0)):
+        attention.flash_fwd(t, t, t, t, t, longest, 1.0)
+    assert seen == [7] * 6 and all(type(n) is int for n in seen)
