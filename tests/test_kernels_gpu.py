@@ -2236,3 +2236,63 @@ def test_fused_logprob_row_blocks_and_ranges(monkeypatch, pairs, T, V, H, ranges
     logit = 2.0 ** -20 * (h.double().norm(dim=1) * w.double().norm(dim=1).max())
     assert ((lp.double() - want).abs() <= 2 * logit + 1e-5 * (1 + lse.abs())).all()
     assert ((ent.double() - want_ent).abs() <= (2 + logits.abs().amax(-1)) * (2 * logit + 1e-5)).all()
+
+
+def _same_bits(a, b):
+    nan = torch.isnan(b)
+    return torch.equal(torch.isnan(a), nan) and torch.equal(a.view(torch.int16)[~nan], b.view(torch.int16)[~nan])
+
+
+def _all_gates(M, H=64):
+    """Activations and a fused weight whose gates are all the bf16 values there are, beside random ups, without a rounding."""
+    torch.manual_seed(102)
+    gates = torch.arange(1 << 16, device=DEV).to(torch.int32).to(torch.int16).view(torch.bfloat16)
+    I = len(gates)
+    x, w = torch.zeros(M, H, dtype=torch.bfloat16, device=DEV), torch.zeros(2 * I, H, dtype=torch.bfloat16, device=DEV)
+    x[:, 0], w[:I, 0], w[I:, 0] = 1.0, gates, _bf16(I)
+    return x, w, I
+
+
+@pytest.mark.parametrize("M", [1, 5, 100, 200, 300])
+def test_swiglu_epilogues_have_the_divisions_bits(M):
+    """Every bf16 gate, infinities and NaN among them, in the epilogues of inference: what the pass over stored values makes of it,
+    which divides. (A product's zeros have no sign.)"""
+    x, w, I = _all_gates(M)
+    want = F.swiglu(w[:, 0][None] + 0.0).expand(M, -1)
+    got = F.skinny_gate_up_swiglu(x, w) if M <= 256 else F.gemm(x, w, swiglu=True)
+    native.read_status(x.device)
+    assert _same_bits(got, want.contiguous())
+
+
+def test_gated_mlp_epilogues_have_the_bits_of_the_passes():
+    """Every bf16 gate in training, and gates so small that they are stored as zeros of both signs, where nothing is cut: stored
+    values, activation and gradients are those of the separate passes."""
+    M = 300
+    x, w, I = _all_gates(M)
+    x[1::2, 0], w[:I][w[:I, 0].abs() < 2.0 ** -60] = 2.0 ** -70, -2.0 ** -66
+    w_down, dy = _bf16(64, I), _bf16(M, 64)
+    H, st, sms = native.host(), native.status_word(x.device), native.num_sms(0)
+    assert not H.b200_gemm_gated_scratch(M, I, 64, False, sms) and not H.b200_gemm_gated_scratch(M, I, 64, True, sms)
+    gu, act, dgu = (torch.empty(M, n, dtype=torch.bfloat16, device=DEV) for n in (2 * I, I, 2 * I))
+    native.check(H.b200_gemm_gate_up(x, w, gu, act, M, I, 64, 64, 64, None, 0, st, sms, native.stream()), "gate_up")
+    native.check(H.b200_gemm_dgate_up(dy, w_down, gu, dgu, M, I, 64, 64, I, None, 0, st, sms, native.stream()), "dgate_up")
+    native.read_status(x.device)
+    want_gu = F.gemm(x, w)
+    assert ((want_gu[1, :I] == 0) & torch.signbit(want_gu[1, :I])).any()
+    dact = F.gemm(dy, w_down, b_mn=True)
+    want = native.tensors(H.swiglu_bwd(dact, want_gu, native.stream()), "swiglu_bwd")
+    assert _same_bits(gu, want_gu) and _same_bits(act, F.swiglu(want_gu)) and _same_bits(dgu, want)
+
+
+def test_expert_swiglu_backward_has_the_bits_of_its_pass():
+    """Every bf16 gate between the experts' projections: with weights of one, the gradients of the pass that divides."""
+    rows = 128
+    _, w, I = _all_gates(1)
+    h1, dact = w[:, 0][None].expand(rows, -1).contiguous(), _bf16(rows, I)
+    info = torch.stack([torch.arange(rows, device=DEV, dtype=torch.int32), torch.ones(rows, device=DEV).view(torch.int32)], 1).contiguous()
+    dh1, ap, dprob = torch.empty_like(h1), torch.empty_like(dact), torch.empty(rows, device=DEV)
+    n_tiles = torch.ones(1, dtype=torch.int32, device=DEV)
+    native.check(native.host().b200_moe_swiglu_bwd(dact, h1, info, n_tiles, dh1, ap, dprob, rows, I, native.stream()), "moe_swiglu_bwd")
+    want = native.tensors(native.host().swiglu_bwd(dact, h1, native.stream()), "swiglu_bwd")
+    torch.cuda.synchronize()
+    assert _same_bits(dh1, want)
