@@ -136,7 +136,7 @@ _SIGS = {
 
 
 def available() -> bool:
-    return _LIB_PATH.exists()
+    return _LIB_PATH.exists() and (_LIB_PATH.parent / "_host.so").exists()
 
 
 @functools.lru_cache(maxsize=1)

@@ -237,3 +237,15 @@ def test_flash_fwd_takes_its_longest_sequence_as_a_number_of_any_kind(monkeypatc
     for longest in (7, 7.0, np.float32(7.0), np.int64(7), torch.tensor(7), torch.tensor(7.0)):
         attention.flash_fwd(t, t, t, t, t, longest, 1.0)
     assert seen == [7] * 6 and all(type(n) is int for n in seen)
+
+
+def test_native_code_is_available_when_both_libraries_are(monkeypatch, tmp_path):
+    """The kernels' library alone runs nothing: its entry points are in the extension beside it."""
+    from cosmos_rl_b200.ops import build, native
+    assert native._LIB_PATH.parent / build.HOST_NAME == build.host_path()
+    monkeypatch.setattr(native, "_LIB_PATH", tmp_path / build.LIB_NAME)
+    assert not native.available()
+    (tmp_path / build.LIB_NAME).touch()
+    assert not native.available()
+    (tmp_path / build.HOST_NAME).touch()
+    assert native.available()
