@@ -49,9 +49,13 @@ def _rmsnorm_fwd(x2, weight, eps, res2, rstd):
 
 
 def _rows_like(residual, x2):
-    """``residual`` as contiguous rows of x2's length; raises unless it has such."""
+    """``residual`` as contiguous rows of x2's length; raises unless it has such, and as many as x2: the kernel reads them."""
     residual = _c(residual)
-    return residual if residual.shape == x2.shape else residual.view(-1, x2.shape[1])
+    if residual.shape != x2.shape:
+        residual = residual.view(-1, x2.shape[1])
+        if residual.shape[0] < x2.shape[0]:
+            raise RuntimeError(f"a residual of {residual.shape[0]} rows for {x2.shape[0]} rows of activations")
+    return residual
 
 
 class _RMSNorm(torch.autograd.Function):

@@ -249,3 +249,23 @@ def test_native_code_is_available_when_both_libraries_are(monkeypatch, tmp_path)
     assert not native.available()
     (tmp_path / build.HOST_NAME).touch()
     assert native.available()
+
+
+def test_rms_norm_refuses_a_residual_of_fewer_rows(monkeypatch):
+    """Rows of the right length that are too few would be read past their end, with gradients or without. (Tensors that only say
+    that they are on a GPU.)"""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cosmos_rl_b200.ops import functional as F
+    monkeypatch.setattr(F, "_rmsnorm_fwd", lambda x2, weight, eps, res2, rstd: (torch.empty_like(x2), torch.empty_like(x2)))
+    with FakeTensorMode():
+        make = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda")
+        for w in (make(512), make(512).requires_grad_(True)):
+            for shape in ((1, 512), (3, 512), (0, 512), (512,), (1, 3, 512)):
+                with pytest.raises(RuntimeError):
+                    F.rms_norm(make(4, 512), w, residual=make(*shape))
+                with pytest.raises(RuntimeError):
+                    F.rms_norm(make(2, 2, 512), w, residual=make(*shape))
+            F.rms_norm(make(2, 2, 512), w, residual=make(4, 512))
