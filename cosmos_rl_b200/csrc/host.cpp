@@ -295,7 +295,8 @@ PyObject* skinny_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   uint32_t* status = (uint32_t*)address(a[6]);
   const cudaStream_t s = stream_of(a[8]);
   REQUIRE(x.dim() == 2 && x.is_cuda() && bf16(x) && bf16(w) && x.size(0) <= max_m);
-  REQUIRE(x.stride(1) == 1 && w.stride(-1) == 1);
+  REQUIRE(w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1);
+  REQUIRE(x.size(1) == w.size(1));
   int rc;
   {
     Unlocked unlocked;

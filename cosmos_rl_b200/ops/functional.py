@@ -483,7 +483,7 @@ def _skinny_workspace(device: torch.device) -> torch.Tensor:
 def _skinny_launch(x2, weight, N, swiglu, out, use_ws, bias=None):
     M, K = x2.shape
     assert x2.is_cuda and x2.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and M <= _SKINNY_MAX_M
-    assert x2.stride(-1) == 1 and weight.stride(-1) == 1
+    assert x2.stride(-1) == 1 and weight.stride(-1) == 1 and K == weight.shape[1]
     dev = x2.device.index if x2.device.index is not None else torch.cuda.current_device()
     sms = native.num_sms(dev)
     L = native.host()

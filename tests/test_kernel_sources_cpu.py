@@ -269,3 +269,29 @@ def test_rms_norm_refuses_a_residual_of_fewer_rows(monkeypatch):
                 with pytest.raises(RuntimeError):
                     F.rms_norm(make(2, 2, 512), w, residual=make(*shape))
             F.rms_norm(make(2, 2, 512), w, residual=make(4, 512))
+
+
+def test_projections_of_few_rows_refuse_a_contraction_of_two_lengths(monkeypatch):
+    """The launchers are told one contraction: activations that are wider than the weight would be read past its rows. (Tensors that
+    only say that they are on a GPU.)"""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cosmos_rl_b200.ops import build, native
+    from cosmos_rl_b200.ops import functional as F
+    if not (native.available() and build.host_path().exists()):
+        pytest.skip("the kernel library is not built")
+    for name, value in (("status_word", None), ("num_sms", 148)):
+        monkeypatch.setattr(native, name, lambda d, value=value: value)
+    monkeypatch.setattr(native, "stream", lambda: 0)
+    with FakeTensorMode():
+        make = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda")
+        pos, slots = (torch.empty(4, dtype=t, device="cuda") for t in (torch.int64, torch.int32))
+        for width in (56, 72):
+            for call in (lambda x: F.gemm_skinny(x, make(96, 64)), lambda x: F.linear_infer(x, make(96, 64)),
+                         lambda x: F.skinny_gate_up_swiglu(x, make(96, 64)),
+                         lambda x: F.skinny_linear_residual_rmsnorm(x, make(96, 64), None, make(96), 1e-6),
+                         lambda x: F.skinny_qkv_rope_append(x, make(96, 64), None, pos, slots, 1e4, 4, 1, 16, make(1, 2, 1, 128, 16), True)):
+                with pytest.raises(AssertionError):
+                    call(make(4, width))
