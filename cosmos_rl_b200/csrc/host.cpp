@@ -280,7 +280,7 @@ PyObject* linear_ok(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   want(n, 2);
   const Tensor &x = tensor(a[0]), &w = tensor(a[1]);
-  return PyBool_FromLong(x.is_cuda() && bf16(x) && bf16(w) && w.dim() == 2 && w.stride(1) == 1 && w.size(0) % 8 == 0 &&
+  return PyBool_FromLong(x.is_cuda() && w.device() == x.device() && bf16(x) && bf16(w) && w.dim() == 2 && w.stride(1) == 1 && w.size(0) % 8 == 0 &&
                          w.size(1) % 8 == 0 && w.stride(0) % 8 == 0);
   END_HANDLE_TH_ERRORS
 }

@@ -295,3 +295,22 @@ def test_projections_of_few_rows_refuse_a_contraction_of_two_lengths(monkeypatch
                          lambda x: F.skinny_qkv_rope_append(x, make(96, 64), None, pos, slots, 1e4, 4, 1, 16, make(1, 2, 1, 128, 16), True)):
                 with pytest.raises(AssertionError):
                     call(make(4, width))
+
+
+def test_weights_elsewhere_are_not_given_to_a_kernel():
+    """A weight that was left on the host, or is on another GPU, goes to torch's own product, which says so."""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cosmos_rl_b200.ops import build, native
+    from cosmos_rl_b200.ops import functional as F
+    if not (native.available() and build.host_path().exists()):
+        pytest.skip("the kernel library is not built")
+    with FakeTensorMode():
+        make = lambda device, *shape: torch.empty(*shape, dtype=torch.bfloat16, device=device)
+        assert F._tc_ok(make("cuda:0", 4, 64), make("cuda:0", 96, 64))
+        for device in ("cpu", "cuda:1"):
+            assert not F._tc_ok(make("cuda:0", 4, 64), make(device, 96, 64))
+            with pytest.raises(RuntimeError, match="device"):
+                F.linear_tc(make("cuda:0", 4, 64), make(device, 96, 64))
