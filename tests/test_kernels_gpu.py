@@ -2296,3 +2296,22 @@ def test_expert_swiglu_backward_has_the_bits_of_its_pass():
     want = native.tensors(native.host().swiglu_bwd(dact, h1, native.stream()), "swiglu_bwd")
     torch.cuda.synchronize()
     assert _same_bits(dh1, want)
+
+
+@pytest.mark.parametrize("T,hq,hkv,d", [(5, 2, 1, 128), (601, 4, 2, 64)])
+def test_rope_gradients_in_rows_apart_and_expanded(T, hq, hkv, d):
+    """The new tensor of the backward from rows that are further apart than they are long, that share one row's memory, or that start
+    off the 16-byte grid or lie in columns, which are copied first."""
+    torch.manual_seed(103)
+    n, pos = (hq + 2 * hkv) * d, torch.arange(T, device=DEV) * 7
+    qkv = _bf16(T, n).requires_grad_(True)
+    wide, row = _bf16(T, n + 24), _bf16(1, n)
+    for g in (wide[:, 8:8 + n], wide[:, 16:16 + n], row.expand(T, -1), wide[:, 3:3 + n], _bf16(n, T).t()):
+        z = F.rope_qkv_(qkv * 1.0, pos, hq, hkv, d, 1e6)
+        dx, = torch.autograd.grad(z, qkv, g)
+        want = g.clone(memory_format=torch.contiguous_format)
+        F._rope_qkv_native(want, pos, hq, hkv, d, 1e6, True)
+        assert torch.equal(dx, want) and dx.is_contiguous()
+    taken = [native.host().rope_qkv_new(g, pos, hq, hkv, d, 1e6, True, native.stream()) is not None
+             for g in (wide[:, 8:8 + n], row.expand(T, -1), wide[:, 3:3 + n], _bf16(n, T).t())]
+    assert taken == [True, True, False, False]
