@@ -241,7 +241,7 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
 // (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), which
 // rounds it correctly: the bits of `/` for every bf16 gate and for 5e8 random fp32 gates. Threads with a gate whose exponential
 // overflows, or that is not finite, divide. It pays in epilogues, which have one or two warps a scheduler (gate/up of 14336 x
-// 4096 in inference, 1003 rows 270 us with `/` and 193, 300 rows 165 and 120, 1003 x 1024 x 512 30.7 and 12.3); a pass over
+// 4096 in inference, 1003 rows 270 us with `/` and 193, 300 rows 165 and 100, 1003 x 1024 x 512 30.7 and 12.3); a pass over
 // stored values has the warps to hide the branch and would pay for the check (8192 x 18944 165 us, 203).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float rcp_ge1(float d) {
